@@ -471,6 +471,18 @@ int lia_window_attn_masked(const void* q, int ldq, int q_f32, int act_f32, const
                            int gate_mode, int ldg, void* out, int out_f32, float* workspace, int M, int H, int G, int v_div, int dim, int vdim,
                            int window, int chunk, float scale, float softcap, int heads_per_block, int rows_per_block, int nsplit,
                            lia_stream_t stream);
+/* 1 if lia_window_attn_mma takes these head sizes (64 or 128 query/key channels, 64, 128 or 256 value channels), addresses (16-byte aligned)
+ * and strides (elements; whole 16 bytes) */
+int lia_window_attn_mma_takes(const void* q, int ldq, int q_f32, const void* kcache, long long k_slot_stride, const void* vcache,
+                              long long v_slot_stride, const void* out, int H, int G, int v_div, int dim, int vdim);
+/* lia_window_attn_masked on the tensor cores, for bf16 caches.  prompt != 0: the rows belong to nseg portions, segs[s] = {slot, first position,
+ * first row, rows} on the device (NULL: all rows are one portion that continues from meta's first row); prompt == 0: every row by itself,
+ * its keys in nsplit ranges (workspace as for lia_window_attn). */
+int lia_window_attn_mma(const void* q, int ldq, int q_f32, const void* kcache, long long k_slot_stride, const void* vcache,
+                        long long v_slot_stride, const int* meta, const int* segs, int nseg, const float* temp, const float* slopes,
+                        const float* sink, const void* gate, int gate_mode, int ldg, void* out, int out_f32, float* workspace, int M, int H, int G,
+                        int v_div, int dim, int vdim, int window, int chunk, float scale, float softcap, int prompt, int nsplit,
+                        lia_stream_t stream);
 /* lia_qkv_prep with Gv value heads beside G key heads */
 int lia_qkv_prep_heads(const void* y, int act_f32, int ld, int q_off, int k_off, int v_off, const float* bias, const float* wconv,
                        const float* conv_state, int taps, int norm_mode, const float* qnorm_w, const float* knorm_w, float eps, float temp_coef,

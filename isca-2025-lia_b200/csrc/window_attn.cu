@@ -5,7 +5,7 @@
 //
 //   kv_store:     the new tokens' keys go into the key cache as they are; each value head is divided by its root mean square
 //                 (fp32) and cached so.
-//   window_attn:  one block per (group of token rows, group of up to 8 query heads, range of keys); a warp owns (row, head)
+//   window_attn:  (bf16 caches with heads of 64, 128 or 256 channels: window_attn_mma.cu)  one block per (group of token rows, group of up to 8 query heads, range of keys); a warp owns (row, head)
 //                 pairs.  32 cached positions at a time are staged in shared memory as fp32 for the key/value heads the
 //                 block's query heads use, once for all rows of the block that continue one sequence; lane j scores key j,
 //                     s = cap * tanh((q . k) * scale * temp_h / cap) - slopes[h] * (pos - j)     (cap <= 0: no cap)
@@ -21,16 +21,9 @@
 //                 that an earlier layer published for the same token; q goes out in fp32, k and v into the caches.
 #include <math.h>
 
-#include "common.cuh"
+#include "window_attn.cuh"
 
 namespace {
-
-template <typename T> __device__ __forceinline__ float ldf(const T* p);
-template <> __device__ __forceinline__ float ldf<float>(const float* p) { return *p; }
-template <> __device__ __forceinline__ float ldf<bf16>(const bf16* p) { return __bfloat162float(*p); }
-template <typename T> __device__ __forceinline__ void stf(T* p, float v);
-template <> __device__ __forceinline__ void stf<float>(float* p, float v) { *p = v; }
-template <> __device__ __forceinline__ void stf<bf16>(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
 
 // meta[row] = {slot, position}.  Block per row, warp per value head in turn.
 template <typename T>
@@ -176,45 +169,6 @@ __global__ void __launch_bounds__(256) qkv_prep_kernel(const T* __restrict__ y, 
 
 constexpr int TK = 32;     // cached positions per stage (= lanes: lane j scores key j)
 constexpr int NWARP = 8;
-
-struct WindowArgs {
-  int H, G, dim, vdim, window;
-  int HB, NG, QR, nsplit;      // query heads per block (spanning at most NG key/value heads), rows per block, key ranges per row
-  float scale, softcap;
-  int q_f32, gate_mode, ldg;   // queries in fp32; gate: 0 none, 1 fp32 [M][H] as is, 2 sigmoid of the activations' type [M][ldg], per channel
-  int chunk = 0;               // > 0: a position sees only the keys of its own block of `chunk` positions (counted from the sequence's start)
-  int v_div = 1;               // key head g reads value head g / v_div (the value cache holds G / v_div heads)
-  int out_f32 = 0;             // the output in fp32 whatever the caches hold
-};
-
-// first position a query at `pos` sees: the window's start, and the start of its chunk if the mask is chunked
-__device__ __forceinline__ int first_key(const WindowArgs& a, int pos) {
-  int lo = max(0, pos - a.window + 1);
-  if (a.chunk > 0) lo = max(lo, pos - pos % a.chunk);
-  return lo;
-}
-
-// the output in the caches' type or, `out_f32`, in fp32
-template <typename T>
-__device__ __forceinline__ void store_out(T* out, size_t at, float v, const WindowArgs& a) {
-  if (a.out_f32) reinterpret_cast<float*>(out)[at] = v;
-  else stf(out + at, v);
-}
-
-// what the scores and the output take besides q, k, v (each may be null)
-struct WindowExtras {
-  const float* temp;     // [H] multiplies the scaled score
-  const float* slopes;   // [H] slopes[h] * (pos - j) is taken off the score
-  const float* sink;     // [H] exp(sink_h) joins the softmax's denominator
-  const void* gate;      // see WindowArgs::gate_mode
-};
-
-template <typename T>
-__device__ __forceinline__ float gate_of(const WindowExtras& x, const WindowArgs& a, size_t row, int h, int ch) {
-  if (a.gate_mode == 1) return reinterpret_cast<const float*>(x.gate)[row * a.H + h];
-  if (a.gate_mode == 2) return 1.0f / (1.0f + expf(-ldf(reinterpret_cast<const T*>(x.gate) + row * a.ldg + (size_t)h * a.vdim + ch)));
-  return 1.0f;
-}
 
 __host__ __device__ inline int key_stride(int dim) { return dim % 4 == 0 ? dim + 4 : (dim | 1); }   // conflict-free rows (128-bit or scalar reads)
 
@@ -515,6 +469,18 @@ __global__ void __launch_bounds__(128) diff_combine_kernel(const float* __restri
   for (int c = lane; c < vdim; c += 32) stf(out + (row * H + h) * vdim + c, (a1[c] - lambda * a2[c]) * inv);
 }
 
+}  // namespace
+
+int window_combine(const float* part, const float2* part_ml, void* out, int act_f32, int M, const WindowExtras& x, const WindowArgs& a, cudaStream_t stream) {
+  const unsigned grid = (unsigned)((size_t)M * a.H);
+  if (act_f32) window_combine_kernel<float><<<grid, 128, 0, stream>>>(part, part_ml, reinterpret_cast<float*>(out), a.vdim, a.nsplit, x, a);
+  else window_combine_kernel<bf16><<<grid, 128, 0, stream>>>(part, part_ml, reinterpret_cast<bf16*>(out), a.vdim, a.nsplit, x, a);
+  LIA_LAUNCH_CHECK();
+  return LIA_OK;
+}
+
+namespace {
+
 size_t attn_smem(const WindowArgs& a) {
   return ((size_t)(a.QR * a.HB * a.dim + 3) / 4 * 4 + (size_t)a.NG * TK * (key_stride(a.dim) + a.vdim)) * sizeof(float);
 }
@@ -532,10 +498,7 @@ int launch_attn(const void* q, int ldq, const void* kcache, long long kss, const
                                                                    reinterpret_cast<const T*>(vcache), vss, meta, x, reinterpret_cast<T*>(out), part,
                                                                    part_ml, M, a);
   LIA_LAUNCH_CHECK();
-  if (a.nsplit > 1) {
-    window_combine_kernel<T><<<(unsigned)((size_t)M * a.H), 128, 0, stream>>>(part, part_ml, reinterpret_cast<T*>(out), a.vdim, a.nsplit, x, a);
-    LIA_LAUNCH_CHECK();
-  }
+  if (a.nsplit > 1) return window_combine(part, part_ml, out, sizeof(T) == 4, M, x, a, stream);
   return LIA_OK;
 }
 

@@ -754,8 +754,16 @@ def window_attn_plan(M, nseg, H, G, dim, vdim, window, max_ctx, sms):
     return hb, qr, nsplit
 
 
+def window_decode_splits(M, H, G, span, max_ctx, sms):
+    """Key ranges per row of the tensor-core kernel for single tokens: as many as keep all blocks (one per row and up to 8 query heads of a
+    key head; two fit an SM) in one wave, none under 64 keys."""
+    rep = H // G
+    blocks = M * (H // max(d for d in range(1, 9) if rep % d == 0))
+    return max(1, min(2 * sms // blocks, window_attn_split_class(max_ctx, span))) if max_ctx > 0 else 1
+
+
 def window_attn(q, kcache, vcache, meta, temp, out, H, G, dim, vdim, window, scale, softcap, nseg=None, max_ctx=0, slopes=None, sink=None,
-                gate=None, gate_per_head=False, chunk=0, v_div=1):
+                gate=None, gate_per_head=False, chunk=0, v_div=1, segs=None):
     """Softmax attention of every row over the last ``window`` cached positions of its sequence (csrc/window_attn.cu);
     ``window`` <= 0: over its whole history.  ``nseg``: portions in the step (None: one row each); ``max_ctx``: an upper
     bound of the rows' history lengths (0: unknown, no split of the keys).  ``temp`` [H] multiplies the scores, ``slopes``
@@ -763,7 +771,9 @@ def window_attn(q, kcache, vcache, meta, temp, out, H, G, dim, vdim, window, sca
     as it is (``gate_per_head``), else sigmoid of a pre-activation per channel (a column slice of the activations' type).
     ``q`` may be fp32 while the caches are bf16, and so may ``out``.  ``chunk`` > 0: a position sees only the keys of its own
     block of ``chunk`` positions (blocks counted from the sequence's start).  ``v_div``: key head g reads value head g // v_div
-    (the value cache holds G // v_div heads: several attention maps over one set of values)."""
+    (the value cache holds G // v_div heads: several attention maps over one set of values).  ``segs`` int32 [nseg, 4] on the device
+    (slot, first position, first row, rows): the portions whose rows these are; with them, or with one portion, a step of prompts on
+    bf16 caches runs on the tensor cores (csrc/window_attn_mma.cu), and so does a step of single tokens."""
     ldq = _rowmajor(q, "q")
     _req(meta, "meta", I32)
     for t, n in ((temp, "temp"), (slopes, "slopes"), (sink, "sink")):
@@ -788,7 +798,22 @@ def window_attn(q, kcache, vcache, meta, temp, out, H, G, dim, vdim, window, sca
                 raise _lib.LiaError("window_attn: a per-channel gate must be an [M, H * vdim] slice of the activations' dtype")
     window = int(window) if window > 0 else 1 << 30
     span = min(window, int(chunk)) if chunk > 0 else window               # the most keys a row can see
-    hb, qr, nsplit = window_attn_plan(M, nseg if nseg is not None else M, H, G, dim, vdim, span, max_ctx, _sm_count(q.device))
+    portions = nseg if nseg is not None else M
+    if segs is not None and (tuple(_req(segs, "segs", I32).shape) != (portions, 4)):
+        raise _lib.LiaError("window_attn: segs must be int32 [nseg, 4]")
+    by_rows = M < 2 * portions
+    if kcache.dtype == BF16 and (by_rows or segs is not None or portions == 1) and _lib.load().lia_window_attn_mma_takes(
+            _p(q), ldq, _f32(q), _p(kcache), kcache.stride(0), _p(vcache), vcache.stride(0), _p(out), H, G, int(v_div), dim, vdim):
+        nsplit = window_decode_splits(M, H, G, span, max_ctx, _sm_count(q.device)) if by_rows else 1
+        ws = None
+        if nsplit > 1:
+            ws = torch.empty(_lib.load().lia_window_attn_workspace_floats(M, H, vdim, nsplit), dtype=F32, device=q.device)
+        check(_lib.load().lia_window_attn_mma(_p(q), ldq, _f32(q), _p(kcache), kcache.stride(0), _p(vcache), vcache.stride(0), _p(meta), _p(segs), portions,
+                                              _p(temp), _p(slopes), _p(sink), _p(gate), gate_mode, ldg, _p(out), _f32(out), _p(ws), M, H, G, int(v_div),
+                                              dim, vdim, window, int(chunk), float(scale), float(softcap), int(not by_rows), nsplit, _stream()), "lia_window_attn_mma")
+        count_launches(2 if nsplit > 1 else 1)
+        return out
+    hb, qr, nsplit = window_attn_plan(M, portions, H, G, dim, vdim, span, max_ctx, _sm_count(q.device))
     ws = None
     if nsplit > 1:
         ws = torch.empty(_lib.load().lia_window_attn_workspace_floats(M, H, vdim, nsplit), dtype=F32, device=q.device)

@@ -380,7 +380,7 @@ class WindowAttentionMixer:
         ops.kv_store(k, v, batch.meta, kc, vc, self.G, self.dim, self.vdim, self.eps, self.norm_values)
         o = torch.empty(M, self.H * self.vdim, dtype=self.dtype, device=h.device)
         ops.window_attn(q, kc, vc, batch.meta, self.temp, o, self.H, self.G, self.dim, self.vdim, self.window, self.scale, self.softcap,
-                        nseg=batch.segs.shape[0], max_ctx=batch.max_ctx)
+                        nseg=batch.segs.shape[0], segs=batch.segs, max_ctx=batch.max_ctx)
         return self.out(o)
 
 
@@ -478,7 +478,7 @@ class DifferentialAttentionMixer:
         ops.qkv_prep(y, self.proj.offsets, batch.meta, q, kc, vc, H2, G2, self.dim, self.vdim, self.eps, freq=self.freq, rot_dims=self.rot_dims,
                      v_heads=self.G)
         a = torch.empty(M, H2 * self.vdim, dtype=F32, device=h.device)
-        ops.window_attn(q, kc, vc, batch.meta, None, a, H2, G2, self.dim, self.vdim, self.window, self.scale, 0.0, nseg=batch.segs.shape[0],
+        ops.window_attn(q, kc, vc, batch.meta, None, a, H2, G2, self.dim, self.vdim, self.window, self.scale, 0.0, nseg=batch.segs.shape[0], segs=batch.segs,
                         max_ctx=batch.max_ctx, chunk=self.chunk, v_div=2)
         o = torch.empty(M, self.H * self.vdim, dtype=self.dtype, device=h.device)
         ops.diff_combine(a, o, self.H, self.G, self.vdim, self.lam, 1.0 - self.diff, self.eps)
@@ -597,7 +597,7 @@ class SinkAttentionMixer:
         if self.taps > 1:
             ops.conv_state_update(y, offs, H * self.dim, G * self.vdim, conv, batch.segs, self.taps, nk=G * self.dim)
         o = torch.empty(M, H * self.vdim, dtype=self.dtype, device=h.device)
-        ops.window_attn(q, kc, vc, batch.meta, None, o, H, G, self.dim, self.vdim, 0, self.scale, 0.0, nseg=batch.segs.shape[0],
+        ops.window_attn(q, kc, vc, batch.meta, None, o, H, G, self.dim, self.vdim, 0, self.scale, 0.0, nseg=batch.segs.shape[0], segs=batch.segs,
                         max_ctx=batch.max_ctx, slopes=self.slopes, sink=self.sink, gate=gate, gate_per_head=self.gate == "head")
         return self.out(o)
 
