@@ -516,6 +516,15 @@ int lia_latent_store(const void* dkv, int ldd, int act_f32, const float* c_norm_
 int lia_latent_attn_masked(const float* qa, const void* cache, int cache_f32, long long slot_stride, const int* meta, const float* gate,
                            const float* sink, float* out, float* workspace, int nsplit, int M, int H, int kv_rank, int rot, int window, float scale,
                            lia_stream_t stream);
+/* Latent attention of np portions, portions[i] = {slot, first position, first row, rows} on the HOST, with keys and values expanded per head first,
+ * on the tensor cores.  cache: bf16 rows of kv_rank + rot numbers, slots slot_stride elements apart.  q: rows of H heads of dim unrotated + rot
+ * rotated channels (the rotated ones as projected, not read); qr: [row][H][qr_stride] fp32, the rotated ones turned; w_ukv [2 H dim][kv_rank] bf16: Wuk's
+ * rows, then Wuv's (values of dim channels); gate [row][H], sink [H] fp32 or NULL; out [row][H dim]; workspace for the latents that any 16 neighbouring
+ * portions see (windows counted).  dim 64 or 128, rot 64; 16-byte aligned rows. */
+size_t lia_latent_expanded_workspace_bytes(long long latents, int H, int dim);
+int lia_latent_attn_expanded(const void* q, int ldq, const float* qr, int qr_stride, const void* cache, long long slot_stride, const int* portions, int np,
+                             const void* w_ukv, const float* gate, const float* sink, void* out, int out_f32, void* workspace, int H, int dim,
+                             int rot, int kv_rank, int window, float scale, lia_stream_t stream);
 /* lia_router_topk_ext on rows of ldl numbers whose first E are the logits; sigmoid != 0: an expert's score is the sigmoid of its logit */
 int lia_router_topk_scored(const float* logits, int ldl, const float* correction, int renorm, int sigmoid, int* idx, float* wt, int M, int E,
                            int top, lia_stream_t stream);

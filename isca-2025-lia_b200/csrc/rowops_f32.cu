@@ -11,6 +11,11 @@
 
 #include "common.cuh"
 
+// linear_mma.cu
+bool linear_mma_takes(const void* A, int a_f32, long long lda, long long sA, const void* W, int w_f32, long long ldw, long long sW, int M, int K, int batch);
+int linear_mma(const void* A, int a_f32, long long lda, long long sA, const void* W, int w_f32, long long ldw, long long sW, void* C, int c_f32, long long ldc,
+               long long sC, int M, int N, int K, int batch, float scale, cudaStream_t stream);
+
 namespace {
 
 template <typename T> __device__ __forceinline__ float ldf(const T* p);
@@ -732,6 +737,9 @@ int launch_plain(const void* A, long long lda, long long sA, const void* W, long
     LIA_LAUNCH_CHECK();
     return LIA_OK;
   }
+  // Tensor cores where rows and addresses are whole 16 bytes, CUDA cores for the rest.
+  if (linear_mma_takes(A, sizeof(TA) == 4, lda, sA, W, sizeof(TW) == 4, ldw, sW, M, K, batch))
+    return linear_mma(A, sizeof(TA) == 4, lda, sA, W, sizeof(TW) == 4, ldw, sW, C, c_f32, ldc, sC, M, N, K, batch, scale, stream);
   dim3 grid((N + 63) / 64, (M + 63) / 64, batch);
   if (c_f32)
     linear_plain_kernel<TA, TW, float><<<grid, 256, 0, stream>>>(reinterpret_cast<const TA*>(A), lda, sA, reinterpret_cast<const TW*>(W), ldw, sW,

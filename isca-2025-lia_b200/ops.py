@@ -488,6 +488,35 @@ def latent_attn(qa, cache, meta, gate, out, H, kv_rank, rot, scale, max_ctx=0, w
     return out
 
 
+def latent_attn_expanded(q, qr, cache, portions, w_ukv, gate, out, H, dim, rot, kv_rank, scale, window=0, sink=None):
+    """Attention of the rows of ``portions`` -- (slot, first position, first row, rows) each, host numbers -- over the latents they see, keys and values
+    expanded per head (csrc/latent_attn_mma.cu).  ``q`` [M, H * (dim + rot)] bf16; ``qr``: the turned query parts, a view [M, H, rot] of fp32;
+    ``cache`` [slots, capacity, kv_rank + rot] bf16; ``w_ukv`` [2 H dim, kv_rank]: Wuk above Wuv.  ``out`` [M, H * dim] bf16 or fp32: only the
+    portions' rows are written."""
+    _dev(q, "q", BF16); _req(cache, "cache"); _req(w_ukv, "w_ukv")
+    M = q.shape[0]
+    for t, m in ((gate, "gate"), (sink, "sink")):
+        if t is not None:
+            _req(t, m, F32)
+    if (qr.dtype != F32 or tuple(qr.shape) != (M, H, rot) or qr.stride(2) != 1 or qr.stride(0) != H * qr.stride(1) or q.shape[1] != H * (dim + rot)
+            or tuple(w_ukv.shape) != (2 * H * dim, kv_rank) or cache.shape[2] != kv_rank + rot or not out.is_contiguous() or tuple(out.shape) != (M, H * dim)
+            or (gate is not None and tuple(gate.shape) != (M, H)) or (sink is not None and sink.numel() != H)):
+        raise _lib.LiaError("latent_attn_expanded: shapes do not agree")
+    seen = []
+    for slot, p0, row, n in portions:
+        if not (0 <= slot < cache.shape[0] and 0 <= p0 and n > 0 and p0 + n <= cache.shape[1] and 0 <= row and row + n <= M):
+            raise _lib.LiaError(f"latent_attn_expanded: portion {(slot, p0, row, n)} outside {M} rows or the cache {tuple(cache.shape)}")
+        seen.append(p0 + n - (max(0, p0 - window + 1) if window > 0 else 0))
+    lib = _lib.load()
+    groups = range(0, len(seen), 16)
+    ws = torch.empty(lib.lia_latent_expanded_workspace_bytes(max(sum(seen[g:g + 16]) for g in groups), H, dim), dtype=torch.uint8, device=q.device)
+    table = (ctypes.c_int * (4 * len(portions)))(*[int(x) for p in portions for x in p])
+    check(lib.lia_latent_attn_expanded(_p(q), _rowmajor(q, "q"), _p(qr), qr.stride(1), _p(cache), cache.stride(0), table, len(portions), _p(w_ukv), _p(gate),
+                                       _p(sink), _p(out), _f32(out), _p(ws), H, dim, rot, kv_rank, int(window), float(scale), _stream()), "lia_latent_attn_expanded")
+    count_launches(2 * len(groups))
+    return out
+
+
 # ------------------------------------------------------------------------------------------------------------------
 # Models whose sublayers sit between layer norms on a 32-bit residual stream: decay / delta-rule recurrences, sliding-window
 # attention with grouped key/value heads, dense and mixture-of-experts feed-forwards.  (Not in the reference either.)

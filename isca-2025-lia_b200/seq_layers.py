@@ -143,6 +143,9 @@ class LatentAttentionMixer:
 
     EXPAND_ROWS = 64          # portions of at least this many rows may expand the latents they see ...
     EXPAND_RATIO = 4          # ... if these are at most this many times the rows
+    # The tensor-core form, which keeps expanded keys and values as exact as fp32 (csrc/latent_attn_mma.cu), for designs with a rotated part or a gate:
+    EXPAND_ROWS_EXACT = 16             # from here on expanding costs less than attention in the latent space on the CUDA cores
+    EXPAND_KEYS_EXACT = 1 << 20        # keys x heads whose expansion (1.5 KB each at 128 channels) a step may hold at a time
 
     def __init__(self, w, heads, dim, rot_dim, vdim, kv_rank, rot_dims, rot_base, scale, norm_eps, dtype, device, q_rank=None, rot_pairs=False,
                  rot_scaling=None, gate="head", window=0, sink=False, own_latent=True):
@@ -173,6 +176,10 @@ class LatentAttentionMixer:
         if not rot_dim and gate is None and dim + vdim < 2 * kv_rank and max(dim, vdim) <= 512:
             self.up_k, self.up_v = Linear([w["uk"]], dtype, device), Linear([w["uv"]], dtype, device)
             self.w_uv = self.up_v.weight
+        self.w_ukv = None
+        if self.up_k is None and dtype == BF16 and dim == vdim and dim in (64, 128) and rot_dim == 64 and kv_rank % 8 == 0:
+            self.w_ukv = torch.cat([w["uk"], w["uv"]], 0).to(device=device, dtype=dtype).contiguous()
+            self.w_uv = self.w_ukv[heads * dim:]
         self.out = Linear([w["o"]], dtype, device)
         self.rot_mag = 1.0
         if not rot_dim:
@@ -215,9 +222,18 @@ class LatentAttentionMixer:
         elif self.own_latent:
             ops.latent_store(dkv, self.c_norm_w, batch.meta, cache, self.rank, self.eps)
         done = 0                                          # rows before this one have their output
-        for i, (slot, p0, row, n) in enumerate(batch.portions if self.up_k is not None and batch.portions is not None else ()):
+        portions = batch.portions if batch.portions is not None else ()
+        exact = self._expands_exactly(q, portions, H)
+        if exact:
+            ops.latent_attn_expanded(q, qa.view(M, H, D)[:, :, self.rank:], cache, [portions[i] for i in exact], self.w_ukv, gate, o, H, self.dim, self.rot,
+                                     self.rank, self.scale, window=self.window, sink=self.sink)
+        for i, (slot, p0, row, n) in enumerate(portions if exact or self.up_k is not None else ()):
+            if i in exact:
+                self._in_latent_space(q, qa, cache, gate, batch, o, done, row)
+                done = row + n
+                continue
             base = max(0, p0 - self.window + 1) if self.window else 0
-            if n >= self.EXPAND_ROWS and p0 + n - base <= self.EXPAND_RATIO * n:
+            if self.up_k is not None and n >= self.EXPAND_ROWS and p0 + n - base <= self.EXPAND_RATIO * n:
                 self._in_latent_space(q, qa, cache, gate, batch, o, done, row)
                 self._expand(q[row:row + n], cache[slot, base:p0 + n], self._positions_from(batch, i, base), p0 + n - base, o[row:row + n])
                 done = row + n
@@ -226,6 +242,18 @@ class LatentAttentionMixer:
             og = torch.empty(M, H * self.vdim, dtype=self.dtype, device=h.device)
             o = ops.sigmoid_mul(o, self.proj.part(y, 2 if self.own_latent else 1), og)
         return self.out(o)
+
+    def _expands_exactly(self, q, portions, H):
+        """The portions (by number) whose latents are expanded to keys and values as exact as fp32: of some length, within the workspace's bound."""
+        if self.w_ukv is None or q.data_ptr() % 16 or q.stride(0) % 8:
+            return ()
+        found, seen = [], 0
+        for i, (_, p0, _, n) in enumerate(portions):
+            ctx = p0 + n - (max(0, p0 - self.window + 1) if self.window else 0)
+            if n >= self.EXPAND_ROWS_EXACT and (seen + ctx) * H <= self.EXPAND_KEYS_EXACT:
+                found.append(i)
+                seen += ctx
+        return found
 
     def _in_latent_space(self, q, qa, cache, gate, batch, o, r0, r1):
         """Rows [r0, r1) of ``o``: the query carried into the latent space, attention there, Wuv on what comes out."""
