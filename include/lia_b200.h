@@ -541,6 +541,17 @@ int lia_moe_gemm_weighted(const void* A, int a_f32, int lda, const void* W, int 
 int lia_moe_combine_gated(const void* ypair, int ypair_f32, const int* pos_of, const float* wt, int weighted, const void* shared, int act_f32,
                           const float* shared_gate, int ldg, const int* idx, int n_real, const void* h, float* y, int M, int W, int top,
                           lia_stream_t stream);
+/* lia_moe_plan with row tiles of tile_rows rows */
+int lia_moe_plan_rows(const int* idx, int pairs, int E, int tile_rows, int n_tiles, int* perm, int* tile_expert, int* pos_of, lia_stream_t stream);
+/* One projection of every expert over its own rows on the tensor cores (bf16 rows and weights), one launch.  perm / tile_expert: a plan with tiles of
+ * lia_moe_tc_rows() rows; A [n_tiles * rows][K]: the rows in the plan's order.  up: C [n_tiles * rows][N] bf16 = act(sum), or gated (weights [E][2N][K], gate
+ * rows before up rows): act(gate) * up, both sums in fp32; weigh_in: the sums are first multiplied by their pair's wt.  down: C bf16 in the plan's
+ * order, unweighted, or (c_f32) C [pairs][N] fp32 by pair, times wt unless weigh_in.  Tiles of experts >= E are skipped.  K, N multiples of 8.
+ * A wait inside that does not end within seconds ends the launch; lia_moe_timeouts() (synchronises) counts such launches. */
+int lia_moe_tc_rows(void);
+int lia_moe_timeouts(void);
+int lia_moe_gemm_tc(const void* A, const void* W, void* C, int c_f32, const int* perm, const int* tile_expert, int n_tiles, const float* wt, int N,
+                    int K, int E, int up, int act, int gated, float p0, float p1, int weigh_in, lia_stream_t stream);
 
 /* ---- Designs that keep several residual streams, run two mixers side by side and recur through a state-space dual or a gated linear
  * recurrent unit; routers that choose among groups of experts.  (ABI 11) ---- */

@@ -14,6 +14,7 @@
 // LN is (x - mean) / sqrt(mean((x - mean)^2) + eps) * w + b with fp32 statistics taken in two passes over a staged row.
 #include <math.h>
 
+#include "act.cuh"
 #include "common.cuh"
 
 namespace {
@@ -110,28 +111,6 @@ __global__ void __launch_bounds__(256) ln_gather_kernel(const float* __restrict_
 }
 
 // ---------------------------------------------------------------------------------------------------- activations
-__device__ __forceinline__ float act_apply(float z, int act) {
-  switch (act) {
-    case LIA_ACT_RELU: return fmaxf(z, 0.f);
-    case LIA_ACT_SILU: return z / (1.0f + expf(-z));
-    case LIA_ACT_GELU_ERF: return 0.5f * z * (1.0f + erff(z * 0.70710678118654752440f));
-    case LIA_ACT_GELU_TANH: return 0.5f * z * (1.0f + tanhf(0.79788456080286535588f * (z + 0.044715f * z * z * z)));
-    case LIA_ACT_RELU_SQUARED: return fmaxf(z, 0.f) * fmaxf(z, 0.f);
-    default: return z;
-  }
-}
-
-// the product of a gated feed-forward: act(g) * u, or (LIA_ACT_CLAMPED_SWISH, p0 = limit, p1 = alpha) with g' = min(g, limit) and
-// u' = clamp(u, -limit, limit): g' * sigmoid(alpha g') * (u' + 1)
-__device__ __forceinline__ float gated_apply(float g, float u, int act, float p0, float p1) {
-  if (act == LIA_ACT_CLAMPED_SWISH) {
-    g = fminf(g, p0);
-    u = fminf(fmaxf(u, -p0), p0);
-    return g / (1.0f + expf(-p1 * g)) * (u + 1.0f);
-  }
-  return act_apply(g, act) * u;
-}
-
 // out[m][f] = act(in[m][f]) * in[m][up_off + f]   (up_off < 0: no second factor)
 // perm (may be null): row m holds the projections of pair perm[m], whose routing weight multiplies both factors first (the
 // projection of a weighted input); rows of no pair (-1) become zero.
@@ -237,17 +216,17 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const float* __restric
 // ---------------------------------------------------------------------------------------------------- experts
 constexpr int TM = 64;        // rows of a tile of the grouped projection
 
-// One block.  pairs = M * top (token, choice) pairs; expert e gets ceil(count_e / TM) tiles, one after the other.
-//   perm[tile * TM + r] = pair index, or -1 in the padding of an expert's last tile
+// One block.  pairs = M * top (token, choice) pairs; expert e gets ceil(count_e / tile_rows) tiles, one after the other.
+//   perm[tile * tile_rows + r] = pair index, or -1 in the padding of an expert's last tile
 //   tile_expert[tile]   = expert of the tile, -1 for the unused tiles at the end (n_tiles of them exist in all)
 //   pos_of[pair]        = its place in perm (the row of the experts' intermediate buffer)
 __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ idx, int pairs, int E, int n_tiles, int* __restrict__ perm,
-                                                        int* __restrict__ tile_expert, int* __restrict__ pos_of) {
+                                                        int* __restrict__ tile_expert, int* __restrict__ pos_of, int tile_rows) {
   extern __shared__ int sh[];            // count[E] | offset[E]
   int* count = sh;
   int* offset = sh + E;
   for (int e = threadIdx.x; e < E; e += 1024) count[e] = 0;
-  for (int i = threadIdx.x; i < n_tiles * TM; i += 1024) perm[i] = -1;
+  for (int i = threadIdx.x; i < n_tiles * tile_rows; i += 1024) perm[i] = -1;
   for (int i = threadIdx.x; i < n_tiles; i += 1024) tile_expert[i] = -1;
   __syncthreads();
   for (int p = threadIdx.x; p < pairs; p += 1024) pos_of[p] = atomicAdd(&count[idx[p]], 1);      // rank inside its expert
@@ -255,8 +234,8 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
   if (threadIdx.x == 0) {
     int tile = 0;
     for (int e = 0; e < E; ++e) {
-      offset[e] = tile * TM;
-      const int nt = (count[e] + TM - 1) / TM;
+      offset[e] = tile * tile_rows;
+      const int nt = (count[e] + tile_rows - 1) / tile_rows;
       for (int t = 0; t < nt; ++t) tile_expert[tile + t] = e;
       tile += nt;
     }
@@ -415,6 +394,14 @@ __global__ void moe_gather_kernel(const T* __restrict__ src, const int* __restri
   }
 }
 
+// the same for rows of whole 16 bytes: block per place, `vecs` of them per row (number by number: 32 us for 4736 rows of 2048 bf16; 6 us so)
+__global__ void __launch_bounds__(128) moe_gather_vec_kernel(const uint4* __restrict__ src, const int* __restrict__ perm, uint4* __restrict__ dst, int vecs, int top) {
+  const int p = perm[blockIdx.x];
+  const uint4* from = src + (size_t)(p < 0 ? 0 : p / top) * vecs;
+  uint4* to = dst + (size_t)blockIdx.x * vecs;
+  for (int i = threadIdx.x; i < vecs; i += 128) to[i] = p < 0 ? make_uint4(0u, 0u, 0u, 0u) : from[i];
+}
+
 // y[m][c] = sum_t f(m * top + t)[c] (in the order of t) + sigmoid(sgate[m]) * shared[m][c] (sgate null: + shared[m][c]);
 // f(pair) = ypair[pair], or, with a plan, wt[pair] * ypair[pos_of[pair]] (the experts' outputs still in the plan's order and not
 // yet weighted; `weighted`: nor to be).  A pair whose expert
@@ -436,6 +423,48 @@ __global__ void moe_combine_kernel(const TY* __restrict__ ypair, const int* __re
     }
     if (shared) s += sgate ? ldf(shared + e) / (1.0f + expf(-sgate[m * ldg])) : ldf(shared + e);
     y[e] = s;
+  }
+}
+
+// the same, four columns per thread and one block per row: numbers and pairs of a row are read as whole vectors
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const bf16* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  float4 f;
+  unpack_bf16x2(u.x, f.x, f.y);
+  unpack_bf16x2(u.y, f.z, f.w);
+  return f;
+}
+template <typename TY, typename TS>
+__global__ void __launch_bounds__(256) moe_combine_vec_kernel(const TY* __restrict__ ypair, const int* __restrict__ pos_of, const float* __restrict__ wt,
+                                                              const TS* __restrict__ shared, float* __restrict__ y, int W, int top,
+                                                              const int* __restrict__ idx, int n_real, const TS* __restrict__ h, int weighted,
+                                                              const float* __restrict__ sgate, int ldg) {
+  const size_t m = blockIdx.x;
+  const float gate = sgate ? 1.0f + expf(-sgate[m * ldg]) : 1.0f;
+  for (int c = threadIdx.x * 4; c < W; c += 1024) {
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int t = 0; t < top; ++t) {
+      const size_t pair = m * top + t;
+      if (idx && idx[pair] >= n_real) {
+        const float w = wt[pair];
+        const float4 v = load4(h + m * W + c);
+        s.x = fmaf(w, v.x, s.x); s.y = fmaf(w, v.y, s.y); s.z = fmaf(w, v.z, s.z); s.w = fmaf(w, v.w, s.w);
+      } else if (pos_of) {
+        const float w = weighted ? 1.0f : wt[pair];
+        const float4 v = load4(ypair + (size_t)pos_of[pair] * W + c);
+        s.x = fmaf(w, v.x, s.x); s.y = fmaf(w, v.y, s.y); s.z = fmaf(w, v.z, s.z); s.w = fmaf(w, v.w, s.w);
+      } else {
+        const float4 v = load4(ypair + pair * W + c);
+        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+      }
+    }
+    if (shared) {
+      float4 v = load4(shared + m * W + c);
+      if (sgate) { v.x /= gate; v.y /= gate; v.z /= gate; v.w /= gate; }
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    *reinterpret_cast<float4*>(y + m * W + c) = s;
   }
 }
 
@@ -545,11 +574,15 @@ extern "C" int lia_router_topk_grouped(const float* logits, int ldl, const float
 extern "C" int lia_moe_tile_rows(void) { return TM; }
 
 extern "C" int lia_moe_plan(const int* idx, int pairs, int E, int n_tiles, int* perm, int* tile_expert, int* pos_of, lia_stream_t stream_) {
+  return lia_moe_plan_rows(idx, pairs, E, TM, n_tiles, perm, tile_expert, pos_of, stream_);
+}
+
+extern "C" int lia_moe_plan_rows(const int* idx, int pairs, int E, int tile_rows, int n_tiles, int* perm, int* tile_expert, int* pos_of, lia_stream_t stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-  LIA_CHECK_ARG(idx && perm && tile_expert && pos_of && pairs > 0 && E > 0 && E <= 4096, "lia_moe_plan: bad arguments");
-  LIA_CHECK_ARG(n_tiles >= (int)(((long long)pairs + (long long)(E < pairs ? E : pairs) * (TM - 1)) / TM),
+  LIA_CHECK_ARG(idx && perm && tile_expert && pos_of && pairs > 0 && E > 0 && E <= 4096 && tile_rows > 0, "lia_moe_plan: bad arguments");
+  LIA_CHECK_ARG(n_tiles >= (int)(((long long)pairs + (long long)(E < pairs ? E : pairs) * (tile_rows - 1)) / tile_rows),
                 "lia_moe_plan: %d tiles cannot hold %d pairs of %d experts", n_tiles, pairs, E);
-  moe_plan_kernel<<<1, 1024, (size_t)2 * E * sizeof(int), stream>>>(idx, pairs, E, n_tiles, perm, tile_expert, pos_of);
+  moe_plan_kernel<<<1, 1024, (size_t)2 * E * sizeof(int), stream>>>(idx, pairs, E, n_tiles, perm, tile_expert, pos_of, tile_rows);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -621,6 +654,12 @@ extern "C" int lia_moe_gemm_weighted(const void* A, int a_f32, int lda, const vo
 extern "C" int lia_moe_gather(const void* src, int act_f32, const int* perm, void* dst, int places, int W, int top, lia_stream_t stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LIA_CHECK_ARG(src && perm && dst && places > 0 && W > 0 && top > 0, "lia_moe_gather: bad arguments");
+  const size_t row_bytes = (size_t)W * (act_f32 ? 4 : 2);
+  if (row_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) % 16 == 0) {
+    moe_gather_vec_kernel<<<places, 128, 0, stream>>>(reinterpret_cast<const uint4*>(src), perm, reinterpret_cast<uint4*>(dst), (int)(row_bytes / 16), top);
+    LIA_LAUNCH_CHECK();
+    return LIA_OK;
+  }
   const unsigned blocks = capped_blocks((size_t)places * W);
   if (act_f32) moe_gather_kernel<float><<<blocks, 256, 0, stream>>>(reinterpret_cast<const float*>(src), perm, reinterpret_cast<float*>(dst), places, W, top);
   else moe_gather_kernel<bf16><<<blocks, 256, 0, stream>>>(reinterpret_cast<const bf16*>(src), perm, reinterpret_cast<bf16*>(dst), places, W, top);
@@ -668,6 +707,17 @@ extern "C" int lia_moe_combine_gated(const void* ypair, int ypair_f32, const int
   LIA_CHECK_ARG(!shared_gate || (shared && ldg >= 1), "lia_moe_combine: a gate without a shared expert");
   LIA_CHECK_ARG(!idx || (h && wt && n_real >= 0), "lia_moe_combine: identity experts need the routing weights and the experts' input");
   const unsigned blocks = capped_blocks((size_t)M * W);
+const uintptr_t addr = reinterpret_cast<uintptr_t>(ypair) | reinterpret_cast<uintptr_t>(shared) | reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(y);
+  if (W % 4 == 0 && addr % 16 == 0) {
+#define LIA_MCV(TY, TS) moe_combine_vec_kernel<TY, TS><<<M, 256, 0, stream>>>(reinterpret_cast<const TY*>(ypair), pos_of, wt, reinterpret_cast<const TS*>(shared), y, W, top, idx, n_real, reinterpret_cast<const TS*>(h), weighted, shared_gate, ldg)
+    if (ypair_f32 && act_f32) LIA_MCV(float, float);
+    else if (ypair_f32) LIA_MCV(float, bf16);
+    else if (act_f32) LIA_MCV(bf16, float);
+    else LIA_MCV(bf16, bf16);
+#undef LIA_MCV
+    LIA_LAUNCH_CHECK();
+    return LIA_OK;
+  }
 #define LIA_MC(TY, TS) moe_combine_kernel<TY, TS><<<blocks, 256, 0, stream>>>(reinterpret_cast<const TY*>(ypair), pos_of, wt, reinterpret_cast<const TS*>(shared), y, M, W, top, idx, n_real, reinterpret_cast<const TS*>(h), weighted, shared_gate, ldg)
   if (ypair_f32 && act_f32) LIA_MC(float, float);
   else if (ypair_f32) LIA_MC(float, bf16);

@@ -606,16 +606,38 @@ def router_topk(logits, top, idx, wt, correction=None, renorm=True, sigmoid=Fals
     count_launches()
 
 
-def moe_tiles(pairs, E):
-    """Row tiles that always hold ``pairs`` (token, choice) pairs grouped by expert."""
-    tm = _lib.load().lia_moe_tile_rows()
+def moe_tiles(pairs, E, tensor_core=False):
+    """Row tiles that always hold ``pairs`` (token, choice) pairs grouped by expert, and their rows (``tensor_core``: those of ``moe_gemm_tc``)."""
+    lib = _lib.load()
+    tm = lib.lia_moe_tc_rows() if tensor_core else lib.lia_moe_tile_rows()
     return (pairs + min(E, pairs) * (tm - 1)) // tm, tm
 
 
 def moe_plan(idx, E, perm, tile_expert, pos_of):
     _req(idx, "idx", I32); _req(perm, "perm", I32); _req(tile_expert, "tile_expert", I32); _req(pos_of, "pos_of", I32)
-    check(_lib.load().lia_moe_plan(_p(idx), idx.numel(), E, tile_expert.numel(), _p(perm), _p(tile_expert), _p(pos_of), _stream()), "lia_moe_plan")
+    tiles = tile_expert.numel()
+    if perm.numel() % tiles:
+        raise _lib.LiaError("moe_plan: perm must hold whole tiles")
+    check(_lib.load().lia_moe_plan_rows(_p(idx), idx.numel(), E, perm.numel() // tiles, tiles, _p(perm), _p(tile_expert), _p(pos_of), _stream()), "lia_moe_plan")
     count_launches()
+
+
+def moe_gemm_tc(a, w, out, perm, tile_expert, wt, up, act=ACT_NONE, gated=False, act_params=(0.0, 0.0), weigh_in=False):
+    """One projection of every expert over its own rows in one tensor-core launch (csrc/moe_sm100.cu): ``a`` [places, K] bf16 in the order of a plan with
+    tiles of ``moe_tiles(.., tensor_core=True)`` rows, ``w`` [E, N, K] (``gated``: [E, 2N, K]).  up: out [places, N] bf16 = act(sums), with
+    both factors of a gated activation in fp32; down: out bf16 [places, N] unweighted, or fp32 [pairs, N] by pair, times ``wt`` unless ``weigh_in``."""
+    _req(a, "a"); _req(w, "w"); _req(perm, "perm", I32); _req(tile_expert, "tile_expert", I32)
+    E, N, K = w.shape
+    if gated:
+        N //= 2
+    tm = _lib.load().lia_moe_tc_rows()
+    if (perm.numel() != tile_expert.numel() * tm or tuple(a.shape) != (perm.numel(), K) or not out.is_cuda or not out.is_contiguous() or out.dim() != 2
+            or out.shape[1] != N or (out.dtype == BF16 and out.shape[0] != perm.numel()) or (out.dtype == F32 and (up or out.shape[0] != wt.numel()))):
+        raise _lib.LiaError(f"moe_gemm_tc: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}, {perm.numel()} places")
+    check(_lib.load().lia_moe_gemm_tc(_p(a), _p(w), _p(out), _f32(out), _p(perm), _p(tile_expert), tile_expert.numel(), _p(_req(wt, "wt", F32)), N, K, E, int(up),
+                                      act, int(gated), float(act_params[0]), float(act_params[1]), int(weigh_in), _stream()), "lia_moe_gemm_tc")
+    count_launches()
+    return out
 
 
 def moe_gemm(a, w, out, idx, wt, top, up, act=ACT_NONE, perm=None, tile_expert=None, gated=False, act_params=(0.0, 0.0), weigh_in=False):

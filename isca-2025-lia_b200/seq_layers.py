@@ -796,8 +796,10 @@ class MoEFeedForward:
     grouped by expert on the device (no host round trip) and each projection runs as one grouped launch; a handful of pairs
     (decoding) take the form with one warp per output instead.  The result is fp32."""
 
-    FEW_PAIRS = 48            # up to here: one warp per output, no plan
-    TENSOR_CORE_PAIRS = 512   # from here (bf16, sizes that are multiples of 8): every expert's rows through the tensor-core GEMM
+    # Up to max(16, experts) pairs, FEW_PAIRS at most: one warp per output, whose weight reads grow with the pairs; above (bf16, sizes that are
+    # multiples of 8): tensor cores, which read every chosen expert once.  16 experts, width 4096: 16 pairs 266 | 270 us, 40 pairs 541 | 276 us.
+    FEW_PAIRS = 48
+    TENSOR_CORE_PAIRS = 512   # from here the experts' outputs are rounded to bf16 before they are weighted and added
 
     def __init__(self, router_w, experts_w, top, ff, act, shared, dtype, device, correction=None, renorm=True, identity=0, act_params=(0.0, 0.0),
                  score="softmax", weigh="output", shared_gate=None, groups=None):
@@ -829,44 +831,31 @@ class MoEFeedForward:
         W = self.w_up.shape[2]
         self.tensor_core = dtype == BF16 and W % 8 == 0 and ff % 8 == 0 and os.environ.get("LIA_PLAIN_LINEAR", "0") == "0"
 
-    def _workspace(self, rows, N, K, device):
-        """One split-K workspace large enough for every row count among the experts' launches."""
-        key = (device, "experts")
-        need = ops.GemmWorkspace.bytes_for([(m, N, K) for m in set(rows)])
-        ws = Linear._gemm_ws.get(key)
-        if ws is None or ws.buf.numel() < need:
-            ws = Linear._gemm_ws[key] = ops.GemmWorkspace(need, device)
-        return ws
-
     def _experts_tensor_core(self, h, idx, wt, y, shared_gate):
-        """Prompts: the pairs grouped by expert (tiles of 64 rows), the rows gathered into that order, then one tensor-core
-        GEMM per expert and projection on its contiguous rows (launched back to back from the library).  The tile table comes to the host once per call (the only
-        round trip; decode steps never take this path, so they stay capturable)."""
+        """The pairs grouped by expert (tiles of 128 rows), the rows gathered into that order, then one tensor-core launch per projection
+        over all experts (csrc/moe_sm100.cu).  The experts' outputs are kept by pair in fp32, or from TENSOR_CORE_PAIRS pairs on in the plan's order in bf16."""
         M, W = h.shape
-        E, R, top, ff, dev = self.E, self.R, self.top, self.ff, h.device
+        R, top, ff, dev = self.R, self.top, self.ff, h.device
         pairs = M * top
-        n_tiles, tm = ops.moe_tiles(pairs, R)
+        n_tiles, tm = ops.moe_tiles(pairs, R, tensor_core=True)
         perm = torch.empty(n_tiles * tm, dtype=torch.int32, device=dev)
         tile_expert = torch.empty(n_tiles, dtype=torch.int32, device=dev)
         pos_of = torch.empty(pairs, dtype=torch.int32, device=dev)
         ops.moe_plan(idx, R, perm, tile_expert, pos_of)
         xs = torch.empty(n_tiles * tm, W, dtype=self.dtype, device=dev)
         ops.moe_gather(h, perm, xs, top)
-        counts = torch.bincount(tile_expert.cpu().long() + 1, minlength=R + 1)[1:E + 1].tolist()     # tiles per expert that has weights (they come first)
-        used, rows = max(sum(counts), 1) * tm, [n * tm for n in counts if n]
-        n_up = self.w_up.shape[1]
-        up = torch.empty(used, n_up, dtype=self.dtype, device=dev)
-        mid = torch.empty(used, ff, dtype=self.dtype, device=dev)
-        ys = torch.empty(used, W, dtype=self.dtype, device=dev)
-        if rows:
-            ops.moe_expert_gemms(xs, self.w_up, up, counts, tm, self._workspace(rows, n_up, W, dev))
-            if self.act == ops.ACT_CLAMPED_SWISH:
-                ops.clamped_glu(up, ff, ff, mid, *self.act_params)
-            else:
-                ops.gated_act(up, ff, mid, self.act, up_off=ff if self.gated else -1, perm=perm if self.weigh_in else None, wt=wt)
-            ops.moe_expert_gemms(mid, self.w_down, ys, counts, tm, self._workspace(rows, W, ff, dev))
-        ops.moe_combine(ys, self.shared(h) if self.shared is not None else None, y, top, pos_of=pos_of, wt=None if self.weigh_in else wt,
-                        identity=(idx, E, h, wt) if self.identity else None, weighted=self.weigh_in, shared_gate=shared_gate)
+        mid = torch.empty(n_tiles * tm, ff, dtype=self.dtype, device=dev)
+        ops.moe_gemm_tc(xs, self.w_up, mid, perm, tile_expert, wt, True, self.act, gated=self.gated, act_params=self.act_params, weigh_in=self.weigh_in)
+        shared = self.shared(h) if self.shared is not None else None
+        identity = (idx, self.E, h, wt) if self.identity else None
+        if pairs >= self.TENSOR_CORE_PAIRS:
+            ys = torch.empty(n_tiles * tm, W, dtype=self.dtype, device=dev)
+            ops.moe_gemm_tc(mid, self.w_down, ys, perm, tile_expert, wt, False)
+            ops.moe_combine(ys, shared, y, top, pos_of=pos_of, wt=None if self.weigh_in else wt, identity=identity, weighted=self.weigh_in, shared_gate=shared_gate)
+        else:
+            ys = torch.empty(pairs, W, dtype=F32, device=dev)
+            ops.moe_gemm_tc(mid, self.w_down, ys, perm, tile_expert, wt, False, weigh_in=self.weigh_in)
+            ops.moe_combine(ys, shared, y, top, identity=identity, shared_gate=shared_gate)
         return y
 
     def __call__(self, h, router_input=None):
@@ -884,7 +873,7 @@ class MoEFeedForward:
         identity = (idx, self.E, h, wt) if self.identity else None
         pairs = M * top
         y = torch.empty(M, W, dtype=F32, device=dev)
-        if self.tensor_core and pairs >= self.TENSOR_CORE_PAIRS and h.is_contiguous() and not torch.cuda.is_current_stream_capturing():
+        if self.tensor_core and pairs > min(self.FEW_PAIRS, max(16, self.E)) and h.is_contiguous() and h.dtype == BF16 and h.data_ptr() % 16 == 0:
             return self._experts_tensor_core(h, idx, wt, y, shared_gate)
         ypair = torch.empty(pairs, W, dtype=F32, device=dev)
         if pairs <= self.FEW_PAIRS:

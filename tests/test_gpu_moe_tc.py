@@ -1,0 +1,83 @@
+"""The experts' projections in one tensor-core launch (csrc/moe_sm100.cu) against float64, at the edges of its tiles: experts with 0, 1, 127, 128, 129 and
+more rows, widths around 64, 128 and 256 columns, every form of the projections, pairs of experts without weights; and the vectorised gather
+and combination around them."""
+import pytest
+import torch
+
+import lia_b200  # noqa: F401
+from lia_b200 import _lib, ops
+
+pytestmark = pytest.mark.gpu
+BF16, F32, F64 = torch.bfloat16, torch.float32, torch.float64
+DEV = "cuda"
+
+
+def act64(z, act):
+    if act == ops.ACT_SILU:
+        return z * torch.sigmoid(z)
+    return torch.relu(z) ** 2 if act == ops.ACT_RELU_SQUARED else z
+
+
+@pytest.mark.parametrize("counts,top", [([128, 0, 1, 127], 1), ([129, 300, 64], 2), ([5], 1), ([60, 3, 0, 9, 30], 3), ([1] * 149, 1)])            # (149 row tiles: more than SMs, wide and narrow column tiles)
+@pytest.mark.parametrize("W,ff", [(64, 8), (72, 136), (264, 128), (136, 264)])
+@pytest.mark.parametrize("form", ["plain", "gated", "clamped", "gated weigh in"])
+def test_projections(counts, top, W, ff, form):
+    g = torch.Generator().manual_seed(W + ff + len(counts))
+    E, gated, weigh_in = len(counts) - (1 if len(counts) == 5 else 0), form != "plain", form == "gated weigh in"     # the last expert of five has no weights
+    act = {"plain": ops.ACT_RELU_SQUARED, "clamped": ops.ACT_CLAMPED_SWISH}.get(form, ops.ACT_SILU)
+    experts = torch.cat([torch.full((n,), e) for e, n in enumerate(counts)])
+    pairs = len(experts) // top * top
+    idx = experts[torch.randperm(len(experts), generator=g)][:pairs].to(torch.int32).view(-1, top).contiguous()
+    M = idx.shape[0]
+    wt = torch.rand(M, top, generator=g) + 0.1
+    h = torch.randn(M, W, generator=g).to(BF16)
+    w_up = (torch.randn(E, (2 if gated else 1) * ff, W, generator=g) * W ** -0.5).to(BF16)
+    w_down = (torch.randn(E, W, ff, generator=g) * ff ** -0.5).to(BF16)
+    R = len(counts)
+    n_tiles, tm = ops.moe_tiles(pairs, R, tensor_core=True)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    perm, tile_expert, pos_of = torch.empty(n_tiles * tm, **i32), torch.empty(n_tiles, **i32), torch.empty(pairs, **i32)
+    ops.moe_plan(idx.to(DEV), R, perm, tile_expert, pos_of)
+    xs = torch.empty(n_tiles * tm, W, dtype=BF16, device=DEV)
+    ops.moe_gather(h.to(DEV), perm, xs, top)
+    at = pos_of.cpu().long()
+    assert torch.equal(xs.cpu()[at], h.repeat_interleave(top, 0)) and bool((xs.cpu()[perm.cpu() < 0] == 0).all())
+    mid = torch.empty(n_tiles * tm, ff, dtype=BF16, device=DEV)
+    dwt = wt.to(DEV)
+    ops.moe_gemm_tc(xs, w_up.to(DEV), mid, perm, tile_expert, dwt, True, act, gated=gated, act_params=(1.5, 1.7), weigh_in=weigh_in)
+    # every pair in float64, from the bf16 numbers that the projections read
+    e = idx.reshape(-1).long()
+    real = e < E
+    x = h.to(F64).repeat_interleave(top, 0)
+    z = torch.stack([w_up.to(F64)[min(int(k), E - 1)] @ v for k, v in zip(e, x)]) * (wt.reshape(-1, 1).to(F64) if weigh_in else 1.0)
+    if form == "clamped":
+        a, u = z[:, :ff].clamp(max=1.5), z[:, ff:].clamp(-1.5, 1.5)
+        want = a * torch.sigmoid(1.7 * a) * (u + 1.0)
+    else:
+        want = act64(z[:, :ff], act) * (z[:, ff:] if gated else 1.0)
+    got = mid.cpu()[at][real].to(F64)
+    assert float(((got - want[real]).abs() - want[real].abs() * 2.0 ** -8).max()) < 1e-5        # one rounding of a result made in fp32
+    m64 = mid.cpu()[at].to(F64)
+    down = torch.stack([w_down.to(F64)[min(int(k), E - 1)] @ v for k, v in zip(e, m64)])
+    ys = torch.empty(n_tiles * tm, W, dtype=BF16, device=DEV)
+    ops.moe_gemm_tc(mid, w_down.to(DEV), ys, perm, tile_expert, dwt, False)
+    assert float(((ys.cpu()[at][real].to(F64) - down[real]).abs() - down[real].abs() * 2.0 ** -8).max()) < 1e-5
+    yp = torch.full((pairs, W), 3.0, device=DEV)
+    ops.moe_gemm_tc(mid, w_down.to(DEV), yp, perm, tile_expert, dwt, False, weigh_in=weigh_in)
+    weighed = down * (1.0 if weigh_in else wt.reshape(-1, 1).to(F64))
+    assert float((yp.cpu().to(F64)[real] - weighed[real]).abs().max()) < 1e-5 and bool((yp.cpu()[~real] == 3.0).all())
+    # both ways through the combination, beside a gated shared expert and experts that hand the token back
+    shared, gate = torch.randn(M, W, generator=g).to(BF16), torch.randn(M, 3, generator=g)
+    ident = (idx.to(DEV), E, h.to(DEV), dwt) if E < R else None
+    terms = torch.where(real[:, None], weighed, wt.reshape(-1, 1).to(F64) * x)
+    total = terms.view(M, top, W).sum(1) + shared.to(F64) * torch.sigmoid(gate[:, 1:2].to(F64))
+    for plan in (False, True):
+        y = torch.empty(M, W, device=DEV)
+        if plan:
+            ops.moe_combine(ys, shared.to(DEV), y, top, pos_of=pos_of, wt=None if weigh_in else dwt, identity=ident, weighted=weigh_in, shared_gate=gate.to(DEV)[:, 1:2])
+        else:
+            ops.moe_combine(yp, shared.to(DEV), y, top, identity=ident, shared_gate=gate.to(DEV)[:, 1:2])
+        # the plan's outputs are rounded to bf16 before they are weighted: half a unit of 2^-8 of each term
+        bound = 1e-5 + (terms.abs().view(M, top, W).sum(1) * 2.0 ** -8 if plan else 0.0)
+        assert bool(((y.cpu().to(F64) - total).abs() <= bound).all())
+    assert _lib.load().lia_moe_timeouts() == 0
