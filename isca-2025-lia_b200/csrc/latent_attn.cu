@@ -47,6 +47,8 @@ __global__ void __launch_bounds__(128) latent_prep_kernel(const T* __restrict__ 
                                                           const float* __restrict__ cw, const float* __restrict__ inv_freq, const int* __restrict__ meta,
                                                           T* __restrict__ cache, long long slot_stride, float* __restrict__ qa, int H, int dim, int rot,
                                                           int rot_dims, int kv_rank, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float sh[];                 // rot floats: one vector to rotate
   __shared__ float red[4];
   const int row = blockIdx.x;
@@ -84,6 +86,8 @@ __global__ void __launch_bounds__(128) latent_prep_pairs_kernel(const T* __restr
                                                                 const float* __restrict__ cw, const double* __restrict__ freq, float mag,
                                                                 const int* __restrict__ meta, T* __restrict__ cache, long long slot_stride,
                                                                 float* __restrict__ qa, int H, int dim, int rot, int rot_dims, int kv_rank, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float cs[];                 // cos | sin of the rot_dims / 2 pairs
   __shared__ float red[4];
   const int row = blockIdx.x;
@@ -145,6 +149,8 @@ __device__ __forceinline__ void store_vec(float* p, const float* f) { *reinterpr
 template <typename T>
 __global__ void __launch_bounds__(128) latent_store_kernel(const T* __restrict__ dkv, int ldd, const float* __restrict__ cw, const int* __restrict__ meta,
                                                            T* __restrict__ cache, long long slot_stride, int M, int kv_rank, float eps, int vec) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= M) return;
   const T* d = dkv + (size_t)row * ldd;
@@ -198,6 +204,8 @@ __global__ void __launch_bounds__(256) latent_attn_kernel(const float* __restric
                                                           const int* __restrict__ meta, const float* __restrict__ gate,
                                                           const float* __restrict__ sink, float* __restrict__ out, float* __restrict__ part,
                                                           float2* __restrict__ part_ml, int H, int kv_rank, int rot, int window, float scale) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float sm[];
   const int D = kv_rank + rot, DS = padded_row(D), G4 = (DS - 4) / 4;
   float* qs = sm;                    // [HG][DS]
@@ -356,6 +364,8 @@ __global__ void __launch_bounds__(256) latent_attn_kernel(const float* __restric
 __global__ void __launch_bounds__(128) latent_combine_kernel(const float* __restrict__ part, const float2* __restrict__ part_ml,
                                                              const float* __restrict__ gate, const float* __restrict__ sink, float* __restrict__ out,
                                                              int H, int kv_rank, int nsplit) {
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t rh = blockIdx.x;
   float m = -INFINITY;
   for (int z = 0; z < nsplit; ++z) m = fmaxf(m, part_ml[rh * nsplit + z].x);
@@ -379,11 +389,11 @@ int launch_attn(const float* qa, const void* cache, long long slot_stride, const
   dim3 grid(M, (H + HG - 1) / HG, nsplit);
   float* part = ws;
   float2* part_ml = reinterpret_cast<float2*>(ws + (size_t)M * H * nsplit * kv_rank);
-  latent_attn_kernel<T, RM><<<grid, 256, smem, stream>>>(qa, reinterpret_cast<const T*>(cache), slot_stride, meta, gate, sink, out, part, part_ml,
+  lia_launch(latent_attn_kernel<T, RM>, dim3(grid), dim3(256), smem, stream, qa, reinterpret_cast<const T*>(cache), slot_stride, meta, gate, sink, out, part, part_ml,
                                                          H, kv_rank, rot, window, scale);
   LIA_LAUNCH_CHECK();
   if (nsplit > 1) {
-    latent_combine_kernel<<<(unsigned)((size_t)M * H), 128, 0, stream>>>(part, part_ml, gate, sink, out, H, kv_rank, nsplit);
+    lia_launch(latent_combine_kernel, dim3((unsigned)((size_t)M * H)), dim3(128), 0, stream, part, part_ml, gate, sink, out, H, kv_rank, nsplit);
     LIA_LAUNCH_CHECK();
   }
   return LIA_OK;
@@ -408,10 +418,10 @@ extern "C" int lia_latent_prep(const void* q, int ldq, const void* dkv, int ldd,
                 "lia_latent_prep: bad shape H=%d dim=%d rot=%d rot_dims=%d kv_rank=%d", H, dim, rot, rot_dims, kv_rank);
   const size_t smem = (size_t)rot * sizeof(float);
   if (act_f32)
-    latent_prep_kernel<float><<<M, 128, smem, stream>>>(reinterpret_cast<const float*>(q), ldq, reinterpret_cast<const float*>(dkv), ldd, c_norm_w, inv_freq,
+    lia_launch(latent_prep_kernel<float>, dim3(M), dim3(128), smem, stream, reinterpret_cast<const float*>(q), ldq, reinterpret_cast<const float*>(dkv), ldd, c_norm_w, inv_freq,
                                                         meta, reinterpret_cast<float*>(cache), slot_stride, qa, H, dim, rot, rot_dims, kv_rank, eps);
   else
-    latent_prep_kernel<bf16><<<M, 128, smem, stream>>>(reinterpret_cast<const bf16*>(q), ldq, reinterpret_cast<const bf16*>(dkv), ldd, c_norm_w, inv_freq,
+    lia_launch(latent_prep_kernel<bf16>, dim3(M), dim3(128), smem, stream, reinterpret_cast<const bf16*>(q), ldq, reinterpret_cast<const bf16*>(dkv), ldd, c_norm_w, inv_freq,
                                                        meta, reinterpret_cast<bf16*>(cache), slot_stride, qa, H, dim, rot, rot_dims, kv_rank, eps);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
@@ -426,10 +436,10 @@ extern "C" int lia_latent_prep_pairs(const void* q, int ldq, const void* dkv, in
                 "lia_latent_prep_pairs: bad shape H=%d dim=%d rot=%d rot_dims=%d kv_rank=%d", H, dim, rot, rot_dims, kv_rank);
   const size_t smem = (size_t)(rot_dims > 0 ? rot_dims : 2) * sizeof(float);
   if (act_f32)
-    latent_prep_pairs_kernel<float><<<M, 128, smem, stream>>>(reinterpret_cast<const float*>(q), ldq, reinterpret_cast<const float*>(dkv), ldd, c_norm_w,
+    lia_launch(latent_prep_pairs_kernel<float>, dim3(M), dim3(128), smem, stream, reinterpret_cast<const float*>(q), ldq, reinterpret_cast<const float*>(dkv), ldd, c_norm_w,
                                                               freq, mag, meta, reinterpret_cast<float*>(cache), slot_stride, qa, H, dim, rot, rot_dims, kv_rank, eps);
   else
-    latent_prep_pairs_kernel<bf16><<<M, 128, smem, stream>>>(reinterpret_cast<const bf16*>(q), ldq, reinterpret_cast<const bf16*>(dkv), ldd, c_norm_w,
+    lia_launch(latent_prep_pairs_kernel<bf16>, dim3(M), dim3(128), smem, stream, reinterpret_cast<const bf16*>(q), ldq, reinterpret_cast<const bf16*>(dkv), ldd, c_norm_w,
                                                              freq, mag, meta, reinterpret_cast<bf16*>(cache), slot_stride, qa, H, dim, rot, rot_dims, kv_rank, eps);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
@@ -467,10 +477,10 @@ extern "C" int lia_latent_store(const void* dkv, int ldd, int act_f32, const flo
   const int vec = kv_rank % n == 0 && kv_rank <= 4 * 32 * n && ldd % n == 0 && slot_stride % n == 0 && reinterpret_cast<uintptr_t>(dkv) % 16 == 0 &&
                   reinterpret_cast<uintptr_t>(cache) % 16 == 0;
   if (act_f32)
-    latent_store_kernel<float><<<grid, 128, 0, stream>>>(reinterpret_cast<const float*>(dkv), ldd, c_norm_w, meta, reinterpret_cast<float*>(cache),
+    lia_launch(latent_store_kernel<float>, dim3(grid), dim3(128), 0, stream, reinterpret_cast<const float*>(dkv), ldd, c_norm_w, meta, reinterpret_cast<float*>(cache),
                                                          slot_stride, M, kv_rank, eps, vec);
   else
-    latent_store_kernel<bf16><<<grid, 128, 0, stream>>>(reinterpret_cast<const bf16*>(dkv), ldd, c_norm_w, meta, reinterpret_cast<bf16*>(cache),
+    lia_launch(latent_store_kernel<bf16>, dim3(grid), dim3(128), 0, stream, reinterpret_cast<const bf16*>(dkv), ldd, c_norm_w, meta, reinterpret_cast<bf16*>(cache),
                                                         slot_stride, M, kv_rank, eps, vec);
   LIA_LAUNCH_CHECK();
   return LIA_OK;

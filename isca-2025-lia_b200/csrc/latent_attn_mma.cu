@@ -47,6 +47,8 @@ template <int DN, int DR> constexpr int expanded_smem() { return (BM * DN + 3 * 
 
 template <int DN, int DR>
 __global__ void __launch_bounds__(128, 2) latent_expanded_kernel(const __grid_constant__ ExpandedArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int QC = DN / 8, RC = DR / 8, NT = BK / 8;
   extern __shared__ __align__(128) unsigned char smem[];
   const uint32_t qn = smem_u32(smem), qr = qn + BM * DN * 2, kn = qr + 3 * BM * DR * 2, kr = kn + 3 * BK * DN * 2, vs = kr + BK * DR * 2;
@@ -266,7 +268,7 @@ __global__ void __launch_bounds__(128, 2) latent_expanded_kernel(const __grid_co
 template <int DN, int DR> int run(const ExpandedArgs& a, int tiles, cudaStream_t stream) {
   constexpr int smem = expanded_smem<DN, DR>();
   LIA_CUDA(cudaFuncSetAttribute(latent_expanded_kernel<DN, DR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  latent_expanded_kernel<DN, DR><<<dim3(a.H, tiles), 128, smem, stream>>>(a);
+  lia_launch(latent_expanded_kernel<DN, DR>, dim3(dim3(a.H, tiles)), dim3(128), smem, stream, a);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }

@@ -75,6 +75,8 @@ template <int NA, int NW, int NT, int OUT>
 __global__ void __launch_bounds__(256) linear_mma_kernel(const void* __restrict__ A, long long lda, long long sA, const void* __restrict__ Wt, long long ldw,
                                                          long long sW, void* __restrict__ C, long long ldc, long long sC, int M, int N, int K, float scale,
                                                          int part, const std::conditional_t<OUT == OUT_PARTS, RowRanges, NoRanges> ranges) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int TN = 16 * NT, AB = Tile<NA, TM>::BYTES, WB = Tile<NW, TN>::BYTES;
   constexpr bool SPLIT = NA * NW > 1;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -218,7 +220,7 @@ int run(const void* A, long long lda, long long sA, const void* W, long long ldw
   constexpr int smem = 2 * (Tile<NA, TM>::BYTES + Tile<NW, 16 * NT>::BYTES);
   if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(linear_mma_kernel<NA, NW, NT, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const dim3 grid((N + 16 * NT - 1) / (16 * NT), (M + TM - 1) / TM, batch);
-  linear_mma_kernel<NA, NW, NT, OUT><<<grid, 256, smem, stream>>>(A, lda, sA, W, ldw, sW, C, ldc, sC, M, N, K, scale, 0, NoRanges{});
+  lia_launch(linear_mma_kernel<NA, NW, NT, OUT>, dim3(grid), dim3(256), smem, stream, A, lda, sA, W, ldw, sW, C, ldc, sC, M, N, K, scale, 0, NoRanges{});
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -262,7 +264,7 @@ int linear_mma_parts(const bf16* const* src, const int* rows, int n, long long l
   }
   LIA_CHECK_ARG(tiles <= 65535, "linear_mma_parts: too many rows (%d)", out);
   constexpr int NT = 8, smem = 2 * (Tile<1, TM>::BYTES + Tile<1, 16 * NT>::BYTES);
-  linear_mma_kernel<1, 1, NT, OUT_PARTS><<<dim3((N + 16 * NT - 1) / (16 * NT), tiles, 1), 256, smem, stream>>>(nullptr, lda, 0, W, K, 0, C, 3ll * N, 0, 0, N, K,
+  lia_launch(linear_mma_kernel<1, 1, NT, OUT_PARTS>, dim3(dim3((N + 16 * NT - 1) / (16 * NT), tiles, 1)), dim3(256), smem, stream, nullptr, lda, 0, W, K, 0, C, 3ll * N, 0, 0, N, K,
                                                                                                               1.0f, part, r);
   LIA_LAUNCH_CHECK();
   return LIA_OK;

@@ -56,6 +56,8 @@ __global__ void __launch_bounds__(256) conv_prep_kernel(const T* __restrict__ y,
                                                         const float* __restrict__ a_log, const float* __restrict__ dt_bias, float* __restrict__ qk,
                                                         float* __restrict__ v, int G, int H, int dim, int vdim, int taps, float q_scale,
                                                         float unit_eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float ch[];                 // C channels after convolution and SiLU
   const int row = blockIdx.x;
   const int slot = meta[2 * row], pos = meta[2 * row + 1];
@@ -97,6 +99,8 @@ __global__ void __launch_bounds__(256) conv_prep_kernel(const T* __restrict__ y,
 template <typename T>
 __global__ void __launch_bounds__(256) conv_state_update_kernel(const T* __restrict__ y, int ld, ConvCols cc, float* __restrict__ state,
                                                                 const int* __restrict__ segs, int taps) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int seg = blockIdx.y;
   const int slot = segs[4 * seg], row0 = segs[4 * seg + 2], len = segs[4 * seg + 3];
   const int C = cc.nq + cc.nk + cc.nv;
@@ -123,6 +127,8 @@ __global__ void __launch_bounds__(256) conv_state_update_kernel(const T* __restr
 template <typename T>
 __global__ void forget_gate_prep_kernel(const T* __restrict__ y, int ld, int q_off, int f_off, int v_off, const float* __restrict__ f_bias,
                                         const float* __restrict__ low, float* __restrict__ out, int M, int nq, int nv) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int C = 2 * nq + nv;
   const size_t n = (size_t)M * C;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
@@ -202,6 +208,8 @@ __global__ void __launch_bounds__(NW * 32, 2) linear_scan_kernel(const T* __rest
                                                               int in_silu, const float* __restrict__ decay, const float* __restrict__ gates,
                                                               float* __restrict__ St, const int* __restrict__ segs, int H, int G, int dim, int vdim,
                                                               float* __restrict__ o) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr bool DELTA = MODE == 1, FORGET = MODE == 2;
   constexpr int DP = DR * 32;                    // dim padded to whole warps
   constexpr int ROWF = 2 * DP + CB + 4;          // floats of one staged token: q | k | v (this block's columns) | beta | g | 2 pad
@@ -391,7 +399,7 @@ int launch_scan_mode(const void* q, const void* k, int ldqk, const void* v, int 
   const size_t smem = (size_t)2 * TB * (2 * DR * 32 + CB + 4) * sizeof(float);
   dim3 grid((vdim + CB - 1) / CB, H, nseg);
   if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(linear_scan_kernel<T, DR, MODE, VL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  linear_scan_kernel<T, DR, MODE, VL><<<grid, NW * 32, smem, stream>>>(reinterpret_cast<const T*>(q), reinterpret_cast<const T*>(k), ldqk,
+  lia_launch_after(linear_scan_kernel<T, DR, MODE, VL>, dim3(grid), dim3(NW * 32), smem, stream, reinterpret_cast<const T*>(q), reinterpret_cast<const T*>(k), ldqk,
                                                                        reinterpret_cast<const T*>(v), ldv, in_silu, decay, gates, St, segs, H, G, dim, vdim, o);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
@@ -448,6 +456,8 @@ __global__ void __launch_bounds__(256) conv_act_kernel(const T* __restrict__ y, 
                                                        const float* __restrict__ bias, float* __restrict__ state, const int* __restrict__ meta,
                                                        float* __restrict__ out, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
                                                        float* __restrict__ gates, ConvActArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int c = blockIdx.x * 256 + threadIdx.x;
   const int r0 = blockIdx.y * a.strip, r1 = min(a.M, r0 + a.strip);
   if (c >= a.C + a.H) return;
@@ -543,6 +553,8 @@ template <int NJ, int RG, int TG, bool VL>
 __global__ void __launch_bounds__(128, TG > 1 ? 1 : (NJ <= 2 ? 5 : (NJ <= 4 ? 3 : 1))) ssd_scan_kernel(const float* __restrict__ B, const float* __restrict__ C, const float* __restrict__ x, int ld,
                                                        const float* __restrict__ gates, const float* __restrict__ D, float* __restrict__ St,
                                                        const int* __restrict__ segs, int H, int G, int N, int vdim, float* __restrict__ o) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int SSD_COLS = 4 * 4 * 32 / RG, NP = NJ * 4 * RG, ROWF = 2 * NP + SSD_COLS + 4;
   extern __shared__ __align__(16) float stage[];       // [2][SSD_TB][ROWF]
   const int seg = blockIdx.z, h = blockIdx.y, colb = blockIdx.x * SSD_COLS, g = h / (H / G);
@@ -721,7 +733,7 @@ int launch_ssd_as(const float* B, const float* C, const float* x, int ld, const 
   const size_t smem = (size_t)2 * SSD_TB * (2 * NJ * 4 * RG + COLS + 4) * sizeof(float);
   if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(ssd_scan_kernel<NJ, RG, TG, VL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((vdim + COLS - 1) / COLS, H, nseg);
-  ssd_scan_kernel<NJ, RG, TG, VL><<<grid, 128, smem, stream>>>(B, C, x, ld, gates, D, St, segs, H, G, N, vdim, o);
+  lia_launch_after(ssd_scan_kernel<NJ, RG, TG, VL>, dim3(grid), dim3(128), smem, stream, B, C, x, ld, gates, D, St, segs, H, G, N, vdim, o);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -749,6 +761,8 @@ template <typename T, int LRU_W>
 __global__ void __launch_bounds__(LRU_W * 32) rglru_scan_kernel(const float* __restrict__ u, const float* __restrict__ z, const float* __restrict__ z_bias,
                                                                 const float* __restrict__ c, const T* __restrict__ y, int ldy, const float* __restrict__ y_bias,
                                                                 float* __restrict__ St, const int* __restrict__ segs, int width, int n, T* __restrict__ out) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int SWEEP = LRU_W * 2 * LRU_T;
   __shared__ float2 maps[2][LRU_W][LRU_CH];   // a warp's eight tokens as S -> x S + y
   const int seg = blockIdx.y, slot = segs[4 * seg], row0 = segs[4 * seg + 2], len = segs[4 * seg + 3];
@@ -827,10 +841,10 @@ extern "C" int lia_conv_prep(const void* y, int y_f32, int ld, int q_off, int k_
   LIA_CHECK_ARG(smem <= 160 * 1024, "lia_conv_prep: %d channels do not fit shared memory", cc.nq + cc.nk + cc.nv);
   if (y_f32) {
     if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(conv_prep_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    conv_prep_kernel<float><<<M, 256, smem, stream>>>(reinterpret_cast<const float*>(y), ld, cc, wconv, conv_state, meta, gates, a_log, dt_bias, qk, v, G, H, dim, vdim, taps, q_scale, unit_eps);
+    lia_launch(conv_prep_kernel<float>, dim3(M), dim3(256), smem, stream, reinterpret_cast<const float*>(y), ld, cc, wconv, conv_state, meta, gates, a_log, dt_bias, qk, v, G, H, dim, vdim, taps, q_scale, unit_eps);
   } else {
     if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(conv_prep_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    conv_prep_kernel<bf16><<<M, 256, smem, stream>>>(reinterpret_cast<const bf16*>(y), ld, cc, wconv, conv_state, meta, gates, a_log, dt_bias, qk, v, G, H, dim, vdim, taps, q_scale, unit_eps);
+    lia_launch(conv_prep_kernel<bf16>, dim3(M), dim3(256), smem, stream, reinterpret_cast<const bf16*>(y), ld, cc, wconv, conv_state, meta, gates, a_log, dt_bias, qk, v, G, H, dim, vdim, taps, q_scale, unit_eps);
   }
   LIA_LAUNCH_CHECK();
   return LIA_OK;
@@ -843,8 +857,8 @@ extern "C" int lia_conv_state_update(const void* y, int y_f32, int ld, int q_off
   if (taps == 1) return LIA_OK;
   ConvCols cc{q_off, k_off, v_off, nq, nk, nv};
   dim3 grid((nq + nk + nv + 255) / 256, nseg);
-  if (y_f32) conv_state_update_kernel<float><<<grid, 256, 0, stream>>>(reinterpret_cast<const float*>(y), ld, cc, conv_state, segs, taps);
-  else conv_state_update_kernel<bf16><<<grid, 256, 0, stream>>>(reinterpret_cast<const bf16*>(y), ld, cc, conv_state, segs, taps);
+  if (y_f32) lia_launch(conv_state_update_kernel<float>, dim3(grid), dim3(256), 0, stream, reinterpret_cast<const float*>(y), ld, cc, conv_state, segs, taps);
+  else lia_launch(conv_state_update_kernel<bf16>, dim3(grid), dim3(256), 0, stream, reinterpret_cast<const bf16*>(y), ld, cc, conv_state, segs, taps);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -869,8 +883,8 @@ extern "C" int lia_forget_gate_prep(const void* y, int y_f32, int ld, int q_off,
   size_t blocks = (n + 255) / 256;
   const size_t capb = (size_t)lia_sm_count() * 16;
   if (blocks > capb) blocks = capb;
-  if (y_f32) forget_gate_prep_kernel<float><<<(unsigned)blocks, 256, 0, stream>>>(reinterpret_cast<const float*>(y), ld, q_off, f_off, v_off, f_bias, low, out, M, nq, nv);
-  else forget_gate_prep_kernel<bf16><<<(unsigned)blocks, 256, 0, stream>>>(reinterpret_cast<const bf16*>(y), ld, q_off, f_off, v_off, f_bias, low, out, M, nq, nv);
+  if (y_f32) lia_launch(forget_gate_prep_kernel<float>, dim3((unsigned)blocks), dim3(256), 0, stream, reinterpret_cast<const float*>(y), ld, q_off, f_off, v_off, f_bias, low, out, M, nq, nv);
+  else lia_launch(forget_gate_prep_kernel<bf16>, dim3((unsigned)blocks), dim3(256), 0, stream, reinterpret_cast<const bf16*>(y), ld, q_off, f_off, v_off, f_bias, low, out, M, nq, nv);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -898,7 +912,7 @@ extern "C" int lia_conv_act(const void* y, int y_f32, int ld, int col0, int C, c
   ConvActArgs a{ld, col0, C, taps, act, single, ldo, M, M <= 64 ? 1 : CONV_STRIP, dt_col, H};
   dim3 grid((C + H + 255) / 256, (M + a.strip - 1) / a.strip);
   LIA_CHECK_ARG(grid.y <= 65535, "lia_conv_act: too many rows (%d)", M);
-#define LIA_CA(T, TM) conv_act_kernel<T, TM><<<grid, 256, 0, stream>>>(reinterpret_cast<const T*>(y), in_bias, wconv, bias, state, meta, out, dt_bias, a_log, gates, a)
+#define LIA_CA(T, TM) lia_launch(conv_act_kernel<T, TM>, dim3(grid), dim3(256), 0, stream, reinterpret_cast<const T*>(y), in_bias, wconv, bias, state, meta, out, dt_bias, a_log, gates, a)
   if (y_f32) {
     if (taps <= 4) LIA_CA(float, 4);
     else LIA_CA(float, MAX_TAPS);
@@ -911,8 +925,8 @@ extern "C" int lia_conv_act(const void* y, int y_f32, int ld, int col0, int C, c
   if (taps > 1 && !single) {
     ConvCols cc{col0, 0, 0, C, 0, 0};
     dim3 g2((C + 255) / 256, nseg);
-    if (y_f32) conv_state_update_kernel<float><<<g2, 256, 0, stream>>>(reinterpret_cast<const float*>(y), ld, cc, state, segs, taps);
-    else conv_state_update_kernel<bf16><<<g2, 256, 0, stream>>>(reinterpret_cast<const bf16*>(y), ld, cc, state, segs, taps);
+    if (y_f32) lia_launch(conv_state_update_kernel<float>, dim3(g2), dim3(256), 0, stream, reinterpret_cast<const float*>(y), ld, cc, state, segs, taps);
+    else lia_launch(conv_state_update_kernel<bf16>, dim3(g2), dim3(256), 0, stream, reinterpret_cast<const bf16*>(y), ld, cc, state, segs, taps);
     LIA_LAUNCH_CHECK();
   }
   return LIA_OK;
@@ -938,7 +952,7 @@ extern "C" int lia_rglru_scan(const float* u, const float* z, const float* z_bia
   LIA_CHECK_ARG(u && z && z_bias && c && y && state && segs && out, "lia_rglru_scan: null pointer");
   LIA_CHECK_ARG(nseg > 0 && nseg <= 65535 && rows >= nseg && width > 0 && blocks > 0 && width % blocks == 0 && ldy >= width, "lia_rglru_scan: bad shape width=%d blocks=%d", width, blocks);
   dim3 grid((width + LRU_CH - 1) / LRU_CH, nseg);
-#define LIA_RS(T, W_) rglru_scan_kernel<T, W_><<<grid, W_ * 32, 0, stream>>>(u, z, z_bias, c, reinterpret_cast<const T*>(y), ldy, y_bias, state, segs, width, width / blocks, reinterpret_cast<T*>(out))
+#define LIA_RS(T, W_) lia_launch_after(rglru_scan_kernel<T, W_>, dim3(grid), dim3(W_ * 32), 0, stream, u, z, z_bias, c, reinterpret_cast<const T*>(y), ldy, y_bias, state, segs, width, width / blocks, reinterpret_cast<T*>(out))
   if (y_f32 && rows == nseg) LIA_RS(float, 1);
   else if (y_f32) LIA_RS(float, 16);
   else if (rows == nseg) LIA_RS(bf16, 1);

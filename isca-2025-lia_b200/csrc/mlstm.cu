@@ -18,6 +18,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "rowvec.cuh"
 
 namespace {
 
@@ -84,6 +85,8 @@ __global__ void __launch_bounds__(NW * 32, 2) mlstm_scan_kernel(const T* __restr
                                                              const float* __restrict__ gates, float* __restrict__ St, float* __restrict__ nst,
                                                              float* __restrict__ mst, const int* __restrict__ segs, int H, int dim, int vdim,
                                                              float q_scale, float den_eps, float* __restrict__ o) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int DP = DR * 32;                    // dim padded to whole warps
   constexpr int ROWF = 2 * DP + CB + 4;          // floats of one staged token: q | k | v (this block's columns) | i | f | 2 pad (16-byte rows)
   constexpr int VEC = Vec128<T>::N;
@@ -242,6 +245,8 @@ __global__ void __launch_bounds__(NW * 32, 2) mlstm_scan_kernel(const T* __restr
 template <typename T>
 __global__ void __launch_bounds__(128) headnorm_gate_kernel(const float* __restrict__ o, const float* __restrict__ w, const T* __restrict__ gate, int ldg,
                                                             T* __restrict__ out, int M, int H, int vdim, float eps, int gate_silu) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int pair = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (pair >= M * H) return;
   const int row = pair / H, h = pair - row * H;
@@ -261,13 +266,66 @@ __global__ void __launch_bounds__(128) headnorm_gate_kernel(const float* __restr
   }
 }
 
+// The same with whole vectors of 4.  WIDE: one block per (row, head), for norms over many channels (all heads together: one warp per row took 15 us for
+// 4 rows of 1024 and 32 us for 2048 rows of 2048); else one warp per (row, head).
+template <typename T, bool WIDE>
+__global__ void __launch_bounds__(256) headnorm_gate_vec_kernel(const float* __restrict__ o, const float* __restrict__ w, const T* __restrict__ gate, int ldg,
+                                                                T* __restrict__ out, long long pairs, int H, int vdim, float eps, int gate_silu) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ __align__(16) float red[8];
+  constexpr int N = WIDE ? 256 : 32;
+  const int t = WIDE ? threadIdx.x : threadIdx.x & 31;
+  const long long pair = WIDE ? blockIdx.x : (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (pair >= pairs) return;
+  const long long row = pair / H;
+  const int h = (int)(pair - row * H);
+  const float* orow = o + pair * vdim;
+  constexpr int KEEP = 4;                                   // vectors per thread that stay in registers between the two passes
+  float4 v[KEEP];
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < KEEP; ++i) {
+    const int c = (t + i * N) * 4;
+    if (c < vdim) {
+      v[i] = load4(orow + c);
+      ss += dot4(v[i], v[i]);
+    }
+  }
+  for (int c = (t + KEEP * N) * 4; c < vdim; c += N * 4) {
+    const float4 u = load4(orow + c);
+    ss += dot4(u, u);
+  }
+  ss = WIDE ? block_sum256(ss, red) : warp_sum(ss);
+  const float inv = 1.0f / sqrtf(ss / (float)vdim + eps);
+  auto finish = [&](int c, const float4& u) {
+    const float4 g = load4(w + (size_t)h * vdim + c);
+    float4 y = make_float4(u.x * inv * g.x, u.y * inv * g.y, u.z * inv * g.z, u.w * inv * g.w);
+    if (gate != nullptr) {
+      const float4 z = load4(gate + row * ldg + (size_t)h * vdim + c);
+      const float4 s = make_float4(1.0f / (1.0f + expf(-z.x)), 1.0f / (1.0f + expf(-z.y)), 1.0f / (1.0f + expf(-z.z)), 1.0f / (1.0f + expf(-z.w)));
+      y.x *= gate_silu ? z.x * s.x : s.x;
+      y.y *= gate_silu ? z.y * s.y : s.y;
+      y.z *= gate_silu ? z.z * s.z : s.z;
+      y.w *= gate_silu ? z.w * s.w : s.w;
+    }
+    store4(out + pair * vdim + c, y);
+  };
+#pragma unroll
+  for (int i = 0; i < KEEP; ++i) {
+    const int c = (t + i * N) * 4;
+    if (c < vdim) finish(c, v[i]);
+  }
+  for (int c = (t + KEEP * N) * 4; c < vdim; c += N * 4) finish(c, load4(orow + c));
+}
+
 template <typename T, int DR, bool VL>
 int launch_scan_as(const void* q, const void* k, const void* v, int ld, const float* gates, float* St, float* nst, float* mst, const int* segs,
                 int nseg, int H, int dim, int vdim, float q_scale, float den_eps, float* o, cudaStream_t stream) {
   const size_t smem = (size_t)2 * TB * (2 * DR * 32 + CB + 4) * sizeof(float);
   if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(mlstm_scan_kernel<T, DR, VL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((vdim + CB - 1) / CB, H, nseg);
-  mlstm_scan_kernel<T, DR, VL><<<grid, NW * 32, smem, stream>>>(reinterpret_cast<const T*>(q), reinterpret_cast<const T*>(k), reinterpret_cast<const T*>(v),
+  lia_launch_after(mlstm_scan_kernel<T, DR, VL>, dim3(grid), dim3(NW * 32), smem, stream, reinterpret_cast<const T*>(q), reinterpret_cast<const T*>(k), reinterpret_cast<const T*>(v),
                                                             ld, gates, St, nst, mst, segs, H, dim, vdim, q_scale, den_eps, o);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
@@ -310,9 +368,21 @@ extern "C" int lia_headnorm_gate(const float* o, const float* w, const void* gat
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LIA_CHECK_ARG(o && w && out && M > 0 && H > 0 && vdim > 0 && (!gate || ldg >= H * vdim), "lia_headnorm_gate: bad arguments");
   const long long pairs = (long long)M * H;
+  const int sz = act_f32 ? 4 : 2;
+  if (vdim % 4 == 0 && rows_of_4(o, 4) && rows_of_4(w, 4) && reinterpret_cast<uintptr_t>(out) % (4 * sz) == 0 &&
+      (gate == nullptr || (ldg % 4 == 0 && reinterpret_cast<uintptr_t>(gate) % (4 * sz) == 0))) {
+    const bool wide = vdim > 512;
+    const unsigned g = (unsigned)(wide ? pairs : (pairs + 7) / 8);
+#define LIA_HN(T, WIDE) lia_launch(headnorm_gate_vec_kernel<T, WIDE>, dim3(g), dim3(256), 0, stream, o, w, reinterpret_cast<const T*>(gate), ldg, reinterpret_cast<T*>(out), pairs, H, vdim, eps, gate_silu)
+    if (act_f32) wide ? LIA_HN(float, true) : LIA_HN(float, false);
+    else wide ? LIA_HN(bf16, true) : LIA_HN(bf16, false);
+#undef LIA_HN
+    LIA_LAUNCH_CHECK();
+    return LIA_OK;
+  }
   const unsigned grid = (unsigned)((pairs + 3) / 4);
-  if (act_f32) headnorm_gate_kernel<float><<<grid, 128, 0, stream>>>(o, w, reinterpret_cast<const float*>(gate), ldg, reinterpret_cast<float*>(out), M, H, vdim, eps, gate_silu);
-  else headnorm_gate_kernel<bf16><<<grid, 128, 0, stream>>>(o, w, reinterpret_cast<const bf16*>(gate), ldg, reinterpret_cast<bf16*>(out), M, H, vdim, eps, gate_silu);
+  if (act_f32) lia_launch(headnorm_gate_kernel<float>, dim3(grid), dim3(128), 0, stream, o, w, reinterpret_cast<const float*>(gate), ldg, reinterpret_cast<float*>(out), M, H, vdim, eps, gate_silu);
+  else lia_launch(headnorm_gate_kernel<bf16>, dim3(grid), dim3(128), 0, stream, o, w, reinterpret_cast<const bf16*>(gate), ldg, reinterpret_cast<bf16*>(out), M, H, vdim, eps, gate_silu);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }

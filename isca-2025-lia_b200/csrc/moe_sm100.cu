@@ -66,6 +66,8 @@ enum { UP, UP_GATED, DOWN_PLAN, DOWN_PAIR };
 
 template <int MODE, int COLS>
 __global__ void __launch_bounds__(256, 1) moe_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const MoeArgs p) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr bool GATED = MODE == UP_GATED;
   constexpr int OUT_COLS = GATED ? COLS / 2 : COLS;                // output columns of a tile
   constexpr int STAGES = Shape<COLS>::STAGES, A_BYTES = Shape<COLS>::A_BYTES, B_BYTES = Shape<COLS>::B_BYTES, STAGE_BYTES = Shape<COLS>::STAGE_BYTES,
@@ -261,7 +263,7 @@ __global__ void __launch_bounds__(256, 1) moe_tc_kernel(const __grid_constant__ 
 template <int MODE, int COLS> int launch_as(const CUtensorMap& tmA, const CUtensorMap& tmB, const MoeArgs& a, long long tiles, cudaStream_t stream) {
   LIA_CUDA(cudaFuncSetAttribute(moe_tc_kernel<MODE, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<COLS>::SMEM));
   const int sms = lia_sm_count();
-  moe_tc_kernel<MODE, COLS><<<(unsigned)(tiles < sms ? tiles : sms), 256, Shape<COLS>::SMEM, stream>>>(tmA, tmB, a);
+  lia_launch(moe_tc_kernel<MODE, COLS>, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(256), Shape<COLS>::SMEM, stream, tmA, tmB, a);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }

@@ -43,6 +43,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) embed_rmsnorm_kernel(const int64_t* __restrict__ ids, const T* __restrict__ table,
                                                             const float* __restrict__ w, int w_n, float* __restrict__ x, int W,
                                                             int vocab, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[8];
   const int row = blockIdx.x;
   long long id = ids[row];
@@ -65,6 +67,8 @@ template <typename TY, typename TH>
 __global__ void __launch_bounds__(256) rms_add_norm_kernel(float* __restrict__ x, const TY* __restrict__ y, const float* __restrict__ w_post,
                                                            int w_post_n, const float* __restrict__ w_pre, int w_pre_n, TH* __restrict__ h,
                                                            int W, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float xs[];
   __shared__ float red[8];
   const size_t base = (size_t)blockIdx.x * W;
@@ -100,6 +104,8 @@ template <typename T, typename TC>
 __global__ void __launch_bounds__(256) embed_scale_pos_kernel(const int64_t* __restrict__ ids, const T* __restrict__ table, float scale,
                                                               const T* __restrict__ pos_table, const int* __restrict__ meta, float* __restrict__ x,
                                                               TC* __restrict__ cat, int W, int vocab, int max_pos) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.x;
   long long id = ids[row];
   if (id < 0 || id >= vocab) id = 0;     // the host checks the range; never read outside the table
@@ -130,6 +136,8 @@ __global__ void __launch_bounds__(256) embed_bigram_pos_kernel(const int64_t* __
                                                                long long token_stride, const double* __restrict__ freq, const int* __restrict__ meta,
                                                                float* __restrict__ x, const float* __restrict__ w, TH* __restrict__ h, int W, int vocab,
                                                                float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float xs[];
   __shared__ float red[8];
   const int row = blockIdx.x, slot = meta[2 * row], p = meta[2 * row + 1];
@@ -179,6 +187,8 @@ __global__ void __launch_bounds__(256) embed_bigram_pos_kernel(const int64_t* __
 template <typename TY, typename TH>
 __global__ void __launch_bounds__(256) residual_norm_kernel(float* __restrict__ x, const TY* __restrict__ y, int replace, const float* __restrict__ bias,
                                                             const float* __restrict__ w, TH* __restrict__ h, long long ldh, int W, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float xs[];
   __shared__ float red[8];
   const size_t base = (size_t)blockIdx.x * W;
@@ -204,6 +214,8 @@ __global__ void __launch_bounds__(256) residual_norm_kernel(float* __restrict__ 
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(128) rms_norm_rows_kernel(const TI* __restrict__ in, long long ld, const float* __restrict__ w, TO* __restrict__ out,
                                                             int M, int N, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= M) return;
   const TI* z = in + (size_t)row * ld;
@@ -219,6 +231,8 @@ __global__ void __launch_bounds__(128) rms_norm_rows_kernel(const TI* __restrict
 // out = a * sigmoid(g), element by element over [M][F]; a and g are row-major views with their own row strides
 template <typename TA, typename TG, typename TO>
 __global__ void sigmoid_mul_kernel(const TA* __restrict__ a, long long lda, const TG* __restrict__ g, long long ldg, TO* __restrict__ out, int M, int F) {
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t n = (size_t)M * F;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     const size_t m = e / F;
@@ -229,6 +243,8 @@ __global__ void sigmoid_mul_kernel(const TA* __restrict__ a, long long lda, cons
 
 // x = cap * tanh(x / cap) in place
 __global__ void softcap_kernel(float* __restrict__ x, size_t n, float cap) {
+  pdl_launch_dependents();
+  pdl_wait();
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) x[e] = cap * tanhf(x[e] / cap);
 }
 
@@ -245,6 +261,8 @@ __global__ void __launch_bounds__(256) gated_rms_add_kernel(float* __restrict__ 
                                                             const float* __restrict__ rb, const float* __restrict__ w, float* __restrict__ stack,
                                                             long long stack_stride, int n_mix, const float* __restrict__ mix, TH* __restrict__ h,
                                                             int W, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float gs[];
   __shared__ float red[8];
   const size_t row = blockIdx.x, base = row * W;
@@ -314,6 +332,8 @@ __global__ void __launch_bounds__(256) streams_kernel(float* __restrict__ x, con
                                                       const float* __restrict__ w_out, const float* __restrict__ w_in, const float* __restrict__ w,
                                                       TH* __restrict__ h, const int64_t* __restrict__ ids, const TH* __restrict__ table, int vocab, int S,
                                                       int W, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float us[];
   __shared__ float red[8];
   __shared__ float cmix[SM * SM], cout[SM], cin[SM];
@@ -435,6 +455,8 @@ __global__ void __launch_bounds__(256) streams_kernel(float* __restrict__ x, con
 template <typename TH>
 __global__ void __launch_bounds__(256) streams_gather_kernel(const float* __restrict__ x, const int* __restrict__ rows, const float* __restrict__ w,
                                                              TH* __restrict__ h, int S, int W, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float us[];
   __shared__ float red[8];
   const float* xr = x + (size_t)rows[blockIdx.x] * S * W;
@@ -454,6 +476,8 @@ __global__ void __launch_bounds__(256) streams_gather_kernel(const float* __rest
 template <typename T, int VEC>
 __global__ void __launch_bounds__(128) silu_gate_norm_kernel(const float* __restrict__ o, const T* __restrict__ z, int ldz, const float* __restrict__ w,
                                                              T* __restrict__ out, int F, int groups, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float us[];
   __shared__ float red[4];
   const size_t row = blockIdx.x / groups;
@@ -488,6 +512,8 @@ __global__ void __launch_bounds__(128) silu_gate_norm_kernel(const float* __rest
 template <typename T>
 __global__ void __launch_bounds__(256) poly_norm_kernel(const T* __restrict__ in, int ld, const float* __restrict__ coef, T* __restrict__ out, int F,
                                                         float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[8];
   const T* z = in + (size_t)blockIdx.x * ld;
   float s1 = 0.f, s2 = 0.f, s3 = 0.f;
@@ -512,6 +538,8 @@ __global__ void __launch_bounds__(256) poly_norm_kernel(const T* __restrict__ in
 template <typename TH>
 __global__ void __launch_bounds__(256) rms_gather_kernel(const float* __restrict__ x, const int* __restrict__ rows, const float* __restrict__ w,
                                                          int w_n, TH* __restrict__ h, int W, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[8];
   const size_t src = (size_t)rows[blockIdx.x] * W, dst = (size_t)blockIdx.x * W;
   float ss = 0.f;
@@ -525,6 +553,8 @@ __global__ void __launch_bounds__(256) rms_gather_kernel(const float* __restrict
 // column ranges of one projection's output row (row stride ld; up starts at column up_off)
 template <typename T>
 __global__ void clamped_glu_kernel(const T* __restrict__ gu, int ld, int up_off, T* __restrict__ out, int M, int F, float limit, float alpha) {
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t n = (size_t)M * F;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     const size_t m = e / F;
@@ -562,50 +592,65 @@ template <typename T> __device__ __forceinline__ bool vec_ok(const T* p, long lo
 
 // out[m][n] = act(sum_k a[m][k] w[n][k] + bias[n]) for a handful of outputs (gates: one per head), fp32 out.
 // mode 0: identity; 1: n < N/2 -> cap*tanh(z/cap), n >= N/2 -> logsigmoid(cap*tanh(z/cap)); 2: sigmoid.
-// One block of 4 warps per row: the warps split k (8 numbers per lane and sweep, 128-bit loads), 8 outputs per sweep,
-// partial sums meet in shared memory in a fixed order.
-template <typename TA, typename TW>
+// One block of 4 warps per R rows and 8 outputs: the warps split k (8 numbers per lane and sweep, 128-bit loads), partial sums meet in shared
+// memory in a fixed order.  Four rows per block share a read of the weights where the rows alone fill the GPU (2048 rows, 16 outputs of 2048
+// channels took 28 us with a row per block); a block per 8 outputs where they do not (16 rows took 18 us with one block for all of them).
+template <typename TA, typename TW, int R>
 __global__ void __launch_bounds__(128) linear_small_kernel(const TA* __restrict__ a, int lda, const TW* __restrict__ w, const float* __restrict__ bias,
                                                            float* __restrict__ out, int M, int N, int K, int mode, float cap) {
-  __shared__ float part[4][8];
-  const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const TA* ar = a + (size_t)row * lda;
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ float part[4][R][8];
+  const int row0 = blockIdx.x * R, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool va = vec_ok(a, lda), vw = vec_ok(w, K);
-  for (int n0 = 0; n0 < N; n0 += 8) {
-    float acc[8];
+  for (int n0 = blockIdx.y * 8; n0 < N; n0 += gridDim.y * 8) {
+  float acc[R][8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-    for (int k = threadIdx.x * 8; k < K; k += 128 * 8) {
-      float av[8], wv[8];
-      load8(ar, k, K, va, av);
+  for (int r = 0; r < R; ++r)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (n0 + j < N) {
-          load8(w + (size_t)(n0 + j) * K, k, K, vw, wv);
+    for (int j = 0; j < 8; ++j) acc[r][j] = 0.f;
+  for (int k = threadIdx.x * 8; k < K; k += 128 * 8) {
+    float av[R][8], wv[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) acc[j] = fmaf(av[i], wv[i], acc[j]);
-        }
+    for (int r = 0; r < R; ++r) {
+      if (row0 + r < M) {
+        load8(a + (size_t)(row0 + r) * lda, k, K, va, av[r]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) av[r][i] = 0.f;
       }
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = warp_sum(acc[j]);
-    __syncthreads();
-    if (lane == 0) {
+    for (int j = 0; j < 8; ++j) {
+      if (n0 + j < N) {
+        load8(w + (size_t)(n0 + j) * K, k, K, vw, wv);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) part[warp][j] = acc[j];
-    }
-    __syncthreads();
-    const int n = n0 + threadIdx.x;
-    if (threadIdx.x < 8 && n < N) {
-      float z = ((part[0][threadIdx.x] + part[1][threadIdx.x]) + (part[2][threadIdx.x] + part[3][threadIdx.x])) + (bias ? bias[n] : 0.f);
-      if (mode == 1) {
-        z = cap * tanhf(z / cap);
-        if (n >= N / 2) z = log_sigmoid(z);
-      } else if (mode == 2) {
-        z = 1.0f / (1.0f + expf(-z));
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[r][j] = fmaf(av[r][i], wv[i], acc[r][j]);
       }
-      out[(size_t)row * N + n] = z;
     }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      acc[r][j] = warp_sum(acc[r][j]);
+      if (lane == 0) part[warp][r][j] = acc[r][j];
+    }
+  __syncthreads();
+  const int r = threadIdx.x >> 3, n = n0 + (threadIdx.x & 7), j = threadIdx.x & 7;
+  if (r < R && row0 + r < M && n < N) {
+    float z = ((part[0][r][j] + part[1][r][j]) + (part[2][r][j] + part[3][r][j])) + (bias ? bias[n] : 0.f);
+    if (mode == 1) {
+      z = cap * tanhf(z / cap);
+      if (n >= N / 2) z = log_sigmoid(z);
+    } else if (mode == 2) {
+      z = 1.0f / (1.0f + expf(-z));
+    }
+    out[(size_t)(row0 + r) * N + n] = z;
+  }
+  __syncthreads();                          // `part` may be overwritten
   }
 }
 
@@ -616,6 +661,8 @@ template <typename TA, typename TW, typename TC>
 __global__ void __launch_bounds__(128) linear_fewrows_kernel(const TA* __restrict__ A, long long lda, long long sA, const TW* __restrict__ Wt,
                                                              long long ldw, long long sW, TC* __restrict__ C, long long ldc, long long sC, int M,
                                                              int N, int K, float scale) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int b = blockIdx.y;
   A += (size_t)b * sA;
   Wt += (size_t)b * sW;
@@ -654,6 +701,8 @@ template <typename TA, typename TW, typename TC>
 __global__ void __launch_bounds__(256) linear_plain_kernel(const TA* __restrict__ A, long long lda, long long sA, const TW* __restrict__ Wt,
                                                            long long ldw, long long sW, TC* __restrict__ C, long long ldc, long long sC, int M,
                                                            int N, int K, float scale) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float As[16][64 + 4];
   __shared__ float Ws[16][64 + 4];
   const int b = blockIdx.z;
@@ -699,6 +748,8 @@ __global__ void __launch_bounds__(256) linear_plain_kernel(const TA* __restrict_
 }
 
 __global__ void __launch_bounds__(256) argmax_f32_kernel(const float* __restrict__ logits, int64_t* __restrict__ next, int V, int suppress) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float sv[8];
   __shared__ int si[8];
   const float* row = logits + (size_t)blockIdx.x * V;
@@ -729,10 +780,10 @@ int launch_plain(const void* A, long long lda, long long sA, const void* W, long
   if (M <= 64) {
     dim3 g2((N + 3) / 4, batch);
     if (c_f32)
-      linear_fewrows_kernel<TA, TW, float><<<g2, 128, 0, stream>>>(reinterpret_cast<const TA*>(A), lda, sA, reinterpret_cast<const TW*>(W), ldw, sW,
+      lia_launch(linear_fewrows_kernel<TA, TW, float>, dim3(g2), dim3(128), 0, stream, reinterpret_cast<const TA*>(A), lda, sA, reinterpret_cast<const TW*>(W), ldw, sW,
                                                                    reinterpret_cast<float*>(C), ldc, sC, M, N, K, scale);
     else
-      linear_fewrows_kernel<TA, TW, bf16><<<g2, 128, 0, stream>>>(reinterpret_cast<const TA*>(A), lda, sA, reinterpret_cast<const TW*>(W), ldw, sW,
+      lia_launch(linear_fewrows_kernel<TA, TW, bf16>, dim3(g2), dim3(128), 0, stream, reinterpret_cast<const TA*>(A), lda, sA, reinterpret_cast<const TW*>(W), ldw, sW,
                                                                   reinterpret_cast<bf16*>(C), ldc, sC, M, N, K, scale);
     LIA_LAUNCH_CHECK();
     return LIA_OK;
@@ -742,10 +793,10 @@ int launch_plain(const void* A, long long lda, long long sA, const void* W, long
     return linear_mma(A, sizeof(TA) == 4, lda, sA, W, sizeof(TW) == 4, ldw, sW, C, c_f32, ldc, sC, M, N, K, batch, scale, stream);
   dim3 grid((N + 63) / 64, (M + 63) / 64, batch);
   if (c_f32)
-    linear_plain_kernel<TA, TW, float><<<grid, 256, 0, stream>>>(reinterpret_cast<const TA*>(A), lda, sA, reinterpret_cast<const TW*>(W), ldw, sW,
+    lia_launch(linear_plain_kernel<TA, TW, float>, dim3(grid), dim3(256), 0, stream, reinterpret_cast<const TA*>(A), lda, sA, reinterpret_cast<const TW*>(W), ldw, sW,
                                                                  reinterpret_cast<float*>(C), ldc, sC, M, N, K, scale);
   else
-    linear_plain_kernel<TA, TW, bf16><<<grid, 256, 0, stream>>>(reinterpret_cast<const TA*>(A), lda, sA, reinterpret_cast<const TW*>(W), ldw, sW,
+    lia_launch(linear_plain_kernel<TA, TW, bf16>, dim3(grid), dim3(256), 0, stream, reinterpret_cast<const TA*>(A), lda, sA, reinterpret_cast<const TW*>(W), ldw, sW,
                                                                 reinterpret_cast<bf16*>(C), ldc, sC, M, N, K, scale);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
@@ -759,9 +810,9 @@ extern "C" int lia_embed_rmsnorm(const int64_t* ids, const void* table, int tabl
   LIA_CHECK_ARG(ids && table && w && x, "lia_embed_rmsnorm: null pointer");
   LIA_CHECK_ARG(rows > 0 && W > 0 && vocab > 0 && (w_n == 1 || w_n == W), "lia_embed_rmsnorm: bad shape rows=%d W=%d w_n=%d", rows, W, w_n);
   if (table_f32)
-    embed_rmsnorm_kernel<float><<<rows, 256, 0, stream>>>(ids, reinterpret_cast<const float*>(table), w, w_n, x, W, vocab, eps);
+    lia_launch(embed_rmsnorm_kernel<float>, dim3(rows), dim3(256), 0, stream, ids, reinterpret_cast<const float*>(table), w, w_n, x, W, vocab, eps);
   else
-    embed_rmsnorm_kernel<bf16><<<rows, 256, 0, stream>>>(ids, reinterpret_cast<const bf16*>(table), w, w_n, x, W, vocab, eps);
+    lia_launch(embed_rmsnorm_kernel<bf16>, dim3(rows), dim3(256), 0, stream, ids, reinterpret_cast<const bf16*>(table), w, w_n, x, W, vocab, eps);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -777,7 +828,7 @@ extern "C" int lia_rms_add_norm(float* x, const void* y, int y_f32, const float*
 #define LIA_RAN(TY, TH)                                                                                                      \
   do {                                                                                                                       \
     if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(rms_add_norm_kernel<TY, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    rms_add_norm_kernel<TY, TH><<<rows, 256, smem, stream>>>(x, reinterpret_cast<const TY*>(y), w_post, w_post_n, w_pre, w_pre_n,        \
+    lia_launch(rms_add_norm_kernel<TY, TH>, dim3(rows), dim3(256), smem, stream, x, reinterpret_cast<const TY*>(y), w_post, w_post_n, w_pre, w_pre_n,        \
                                                              reinterpret_cast<TH*>(h), W, eps);                              \
   } while (0)
   if (y_f32 && h_f32) LIA_RAN(float, float);
@@ -802,7 +853,7 @@ extern "C" int lia_gated_rms_add(float* x, const void* y, int y_f32, const void*
 #define LIA_GRA(TY, TH)                                                                                                      \
   do {                                                                                                                       \
     if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(gated_rms_add_kernel<TY, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    gated_rms_add_kernel<TY, TH><<<rows, 256, smem, stream>>>(x, reinterpret_cast<const TY*>(y), reinterpret_cast<const TH*>(r), ldr, rb, w, stack, \
+    lia_launch(gated_rms_add_kernel<TY, TH>, dim3(rows), dim3(256), smem, stream, x, reinterpret_cast<const TY*>(y), reinterpret_cast<const TH*>(r), ldr, rb, w, stack, \
                                                               stack_stride, n_mix, mix, reinterpret_cast<TH*>(h), W, eps);    \
   } while (0)
   if (y_f32 && act_f32) LIA_GRA(float, float);
@@ -817,8 +868,8 @@ extern "C" int lia_gated_rms_add(float* x, const void* y, int y_f32, const void*
 extern "C" int lia_poly_norm(const void* in, int ld, const float* coef, void* out, int act_f32, int M, int F, float eps, lia_stream_t stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LIA_CHECK_ARG(in && coef && out && M > 0 && F > 0 && ld >= F, "lia_poly_norm: bad arguments");
-  if (act_f32) poly_norm_kernel<float><<<M, 256, 0, stream>>>(reinterpret_cast<const float*>(in), ld, coef, reinterpret_cast<float*>(out), F, eps);
-  else poly_norm_kernel<bf16><<<M, 256, 0, stream>>>(reinterpret_cast<const bf16*>(in), ld, coef, reinterpret_cast<bf16*>(out), F, eps);
+  if (act_f32) lia_launch(poly_norm_kernel<float>, dim3(M), dim3(256), 0, stream, reinterpret_cast<const float*>(in), ld, coef, reinterpret_cast<float*>(out), F, eps);
+  else lia_launch(poly_norm_kernel<bf16>, dim3(M), dim3(256), 0, stream, reinterpret_cast<const bf16*>(in), ld, coef, reinterpret_cast<bf16*>(out), F, eps);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -827,8 +878,8 @@ extern "C" int lia_rms_gather(const float* x, const int* rows, const float* w, i
                               lia_stream_t stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LIA_CHECK_ARG(x && rows && w && h && n > 0 && W > 0 && (w_n == 1 || w_n == W), "lia_rms_gather: bad arguments");
-  if (h_f32) rms_gather_kernel<float><<<n, 256, 0, stream>>>(x, rows, w, w_n, reinterpret_cast<float*>(h), W, eps);
-  else rms_gather_kernel<bf16><<<n, 256, 0, stream>>>(x, rows, w, w_n, reinterpret_cast<bf16*>(h), W, eps);
+  if (h_f32) lia_launch(rms_gather_kernel<float>, dim3(n), dim3(256), 0, stream, x, rows, w, w_n, reinterpret_cast<float*>(h), W, eps);
+  else lia_launch(rms_gather_kernel<bf16>, dim3(n), dim3(256), 0, stream, x, rows, w, w_n, reinterpret_cast<bf16*>(h), W, eps);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -841,8 +892,8 @@ extern "C" int lia_clamped_glu(const void* gate_up, int ld, int up_off, void* ou
   size_t blocks = (n + 255) / 256;
   const size_t capb = (size_t)lia_sm_count() * 16;
   if (blocks > capb) blocks = capb;
-  if (act_f32) clamped_glu_kernel<float><<<(unsigned)blocks, 256, 0, stream>>>(reinterpret_cast<const float*>(gate_up), ld, up_off, reinterpret_cast<float*>(out), M, F, limit, alpha);
-  else clamped_glu_kernel<bf16><<<(unsigned)blocks, 256, 0, stream>>>(reinterpret_cast<const bf16*>(gate_up), ld, up_off, reinterpret_cast<bf16*>(out), M, F, limit, alpha);
+  if (act_f32) lia_launch(clamped_glu_kernel<float>, dim3((unsigned)blocks), dim3(256), 0, stream, reinterpret_cast<const float*>(gate_up), ld, up_off, reinterpret_cast<float*>(out), M, F, limit, alpha);
+  else lia_launch(clamped_glu_kernel<bf16>, dim3((unsigned)blocks), dim3(256), 0, stream, reinterpret_cast<const bf16*>(gate_up), ld, up_off, reinterpret_cast<bf16*>(out), M, F, limit, alpha);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -852,11 +903,16 @@ extern "C" int lia_linear_small(const void* a, int a_f32, int lda, const void* w
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LIA_CHECK_ARG(a && w && out && M > 0 && N > 0 && K > 0 && lda >= K, "lia_linear_small: bad arguments");
   LIA_CHECK_ARG(mode >= 0 && mode <= 2 && (mode != 1 || (N % 2 == 0 && cap > 0.f)), "lia_linear_small: bad mode %d (N=%d cap=%f)", mode, N, cap);
-  const int grid = M;
-  if (a_f32 && w_f32) linear_small_kernel<float, float><<<grid, 128, 0, stream>>>(reinterpret_cast<const float*>(a), lda, reinterpret_cast<const float*>(w), bias, out, M, N, K, mode, cap);
-  else if (a_f32) linear_small_kernel<float, bf16><<<grid, 128, 0, stream>>>(reinterpret_cast<const float*>(a), lda, reinterpret_cast<const bf16*>(w), bias, out, M, N, K, mode, cap);
-  else if (w_f32) linear_small_kernel<bf16, float><<<grid, 128, 0, stream>>>(reinterpret_cast<const bf16*>(a), lda, reinterpret_cast<const float*>(w), bias, out, M, N, K, mode, cap);
-  else linear_small_kernel<bf16, bf16><<<grid, 128, 0, stream>>>(reinterpret_cast<const bf16*>(a), lda, reinterpret_cast<const bf16*>(w), bias, out, M, N, K, mode, cap);
+  const bool four = M >= 8 * lia_sm_count();
+  const dim3 grid(four ? (M + 3) / 4 : M, (N + 7) / 8 < 65535 ? (N + 7) / 8 : 65535);
+#define LIA_LS(TA, TW)                                                                                                                                      \
+  (four ? lia_launch(linear_small_kernel<TA, TW, 4>, grid, dim3(128), 0, stream, reinterpret_cast<const TA*>(a), lda, reinterpret_cast<const TW*>(w), bias, out, M, N, K, mode, cap) \
+        : lia_launch(linear_small_kernel<TA, TW, 1>, grid, dim3(128), 0, stream, reinterpret_cast<const TA*>(a), lda, reinterpret_cast<const TW*>(w), bias, out, M, N, K, mode, cap))
+  if (a_f32 && w_f32) LIA_LS(float, float);
+  else if (a_f32) LIA_LS(float, bf16);
+  else if (w_f32) LIA_LS(bf16, float);
+  else LIA_LS(bf16, bf16);
+#undef LIA_LS
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -877,7 +933,7 @@ extern "C" int lia_linear_plain(const void* A, int a_f32, long long lda, long lo
 extern "C" int lia_argmax_f32(const float* logits, int64_t* next, int B, int V, int suppress_id, lia_stream_t stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LIA_CHECK_ARG(logits && next && B > 0 && V > 0, "lia_argmax_f32: bad arguments");
-  argmax_f32_kernel<<<B, 256, 0, stream>>>(logits, next, V, suppress_id);
+  lia_launch(argmax_f32_kernel, dim3(B), dim3(256), 0, stream, logits, next, V, suppress_id);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -886,7 +942,7 @@ extern "C" int lia_embed_scale_pos(const int64_t* ids, const void* table, const 
                                    float* x, void* cat, int cat_f32, int rows, int W, int vocab, int max_pos, lia_stream_t stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LIA_CHECK_ARG(ids && table && meta && x && rows > 0 && W > 0 && vocab > 0 && (!pos_table || max_pos > 0), "lia_embed_scale_pos: bad arguments");
-#define LIA_ESP(T, TC) embed_scale_pos_kernel<T, TC><<<rows, 256, 0, stream>>>(ids, reinterpret_cast<const T*>(table), scale, reinterpret_cast<const T*>(pos_table), meta, x, reinterpret_cast<TC*>(cat), W, vocab, max_pos)
+#define LIA_ESP(T, TC) lia_launch(embed_scale_pos_kernel<T, TC>, dim3(rows), dim3(256), 0, stream, ids, reinterpret_cast<const T*>(table), scale, reinterpret_cast<const T*>(pos_table), meta, x, reinterpret_cast<TC*>(cat), W, vocab, max_pos)
   if (table_f32 && cat_f32) LIA_ESP(float, float);
   else if (table_f32) LIA_ESP(float, bf16);
   else if (cat_f32) LIA_ESP(bf16, float);
@@ -906,7 +962,7 @@ extern "C" int lia_residual_norm(float* x, const void* y, int y_f32, int replace
 #define LIA_RN(TY, TH)                                                                                                       \
   do {                                                                                                                       \
     if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(residual_norm_kernel<TY, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    residual_norm_kernel<TY, TH><<<rows, 256, smem, stream>>>(x, reinterpret_cast<const TY*>(y), replace, bias, w, reinterpret_cast<TH*>(h), ldh, W, eps); \
+    lia_launch(residual_norm_kernel<TY, TH>, dim3(rows), dim3(256), smem, stream, x, reinterpret_cast<const TY*>(y), replace, bias, w, reinterpret_cast<TH*>(h), ldh, W, eps); \
   } while (0)
   if (y_f32 && h_f32) LIA_RN(float, float);
   else if (y_f32) LIA_RN(float, bf16);
@@ -922,7 +978,7 @@ extern "C" int lia_rms_norm_rows(const void* in, int in_f32, long long ld, const
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LIA_CHECK_ARG(in && w && out && M > 0 && N > 0 && ld >= N, "lia_rms_norm_rows: bad arguments");
   const unsigned grid = (unsigned)((M + 3) / 4);
-#define LIA_RNR(TI, TO) rms_norm_rows_kernel<TI, TO><<<grid, 128, 0, stream>>>(reinterpret_cast<const TI*>(in), ld, w, reinterpret_cast<TO*>(out), M, N, eps)
+#define LIA_RNR(TI, TO) lia_launch(rms_norm_rows_kernel<TI, TO>, dim3(grid), dim3(128), 0, stream, reinterpret_cast<const TI*>(in), ld, w, reinterpret_cast<TO*>(out), M, N, eps)
   if (in_f32 && out_f32) LIA_RNR(float, float);
   else if (in_f32) LIA_RNR(float, bf16);
   else if (out_f32) LIA_RNR(bf16, float);
@@ -941,7 +997,7 @@ extern "C" int lia_sigmoid_mul(const void* a, int a_f32, long long lda, const vo
   size_t blocks = (n + 255) / 256;
   const size_t capb = (size_t)lia_sm_count() * 16;
   if (blocks > capb) blocks = capb;
-#define LIA_SM(TA, TG) sigmoid_mul_kernel<TA, TG, TG><<<(unsigned)blocks, 256, 0, stream>>>(reinterpret_cast<const TA*>(a), lda, reinterpret_cast<const TG*>(gate), ldg, reinterpret_cast<TG*>(out), M, F)
+#define LIA_SM(TA, TG) lia_launch(sigmoid_mul_kernel<TA, TG, TG>, dim3((unsigned)blocks), dim3(256), 0, stream, reinterpret_cast<const TA*>(a), lda, reinterpret_cast<const TG*>(gate), ldg, reinterpret_cast<TG*>(out), M, F)
   if (a_f32 && gate_f32) LIA_SM(float, float);
   else if (a_f32) LIA_SM(float, bf16);
   else if (gate_f32) LIA_SM(bf16, float);
@@ -957,7 +1013,7 @@ extern "C" int lia_softcap_f32(float* x, long long n, float cap, lia_stream_t st
   size_t blocks = ((size_t)n + 255) / 256;
   const size_t capb = (size_t)lia_sm_count() * 16;
   if (blocks > capb) blocks = capb;
-  softcap_kernel<<<(unsigned)blocks, 256, 0, stream>>>(x, (size_t)n, cap);
+  lia_launch(softcap_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, x, (size_t)n, cap);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -973,7 +1029,7 @@ extern "C" int lia_embed_bigram_pos(const int64_t* ids, const void* table, const
 #define LIA_EBP(T, TH)                                                                                                       \
   do {                                                                                                                       \
     if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(embed_bigram_pos_kernel<T, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    embed_bigram_pos_kernel<T, TH><<<rows, 256, smem, stream>>>(ids, reinterpret_cast<const T*>(table), reinterpret_cast<const T*>(bigram), buckets, \
+    lia_launch(embed_bigram_pos_kernel<T, TH>, dim3(rows), dim3(256), smem, stream, ids, reinterpret_cast<const T*>(table), reinterpret_cast<const T*>(bigram), buckets, \
                                                                 mul_prev, mul_cur, tokens, token_stride, freq, meta, x, w, reinterpret_cast<TH*>(h), \
                                                                 W, vocab, eps);                                              \
   } while (0)
@@ -994,7 +1050,7 @@ int launch_streams(float* x, const void* y, const float* w_y, const void* y2, co
                    cudaStream_t stream) {
   const size_t smem = h ? (size_t)W * sizeof(float) : 0;
   if (smem > 40 * 1024) LIA_CUDA(cudaFuncSetAttribute(streams_kernel<TY, TH, SM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  streams_kernel<TY, TH, SM, VEC><<<rows, 256, smem, stream>>>(x, reinterpret_cast<const TY*>(y), w_y, reinterpret_cast<const TY*>(y2), w_y2, scale, mix, w_out,
+  lia_launch(streams_kernel<TY, TH, SM, VEC>, dim3(rows), dim3(256), smem, stream, x, reinterpret_cast<const TY*>(y), w_y, reinterpret_cast<const TY*>(y2), w_y2, scale, mix, w_out,
                                                                w_in, w, reinterpret_cast<TH*>(h), ids, reinterpret_cast<const TH*>(table), vocab, S, W, eps);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
@@ -1052,10 +1108,10 @@ extern "C" int lia_streams_gather(const float* x, const int* rows, const float* 
   const size_t smem = (size_t)W * sizeof(float);
   if (h_f32) {
     if (smem > 40 * 1024) LIA_CUDA(cudaFuncSetAttribute(streams_gather_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    streams_gather_kernel<float><<<n, 256, smem, stream>>>(x, rows, w, reinterpret_cast<float*>(h), S, W, eps);
+    lia_launch(streams_gather_kernel<float>, dim3(n), dim3(256), smem, stream, x, rows, w, reinterpret_cast<float*>(h), S, W, eps);
   } else {
     if (smem > 40 * 1024) LIA_CUDA(cudaFuncSetAttribute(streams_gather_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    streams_gather_kernel<bf16><<<n, 256, smem, stream>>>(x, rows, w, reinterpret_cast<bf16*>(h), S, W, eps);
+    lia_launch(streams_gather_kernel<bf16>, dim3(n), dim3(256), smem, stream, x, rows, w, reinterpret_cast<bf16*>(h), S, W, eps);
   }
   LIA_LAUNCH_CHECK();
   return LIA_OK;
@@ -1072,7 +1128,7 @@ extern "C" int lia_silu_gate_norm(const float* o, const void* z, int ldz, const 
 #define LIA_SGN(T, VEC)                                                                                                      \
   do {                                                                                                                       \
     if (smem > 40 * 1024) LIA_CUDA(cudaFuncSetAttribute(silu_gate_norm_kernel<T, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    silu_gate_norm_kernel<T, VEC><<<grid, 128, smem, stream>>>(o, reinterpret_cast<const T*>(z), ldz, w, reinterpret_cast<T*>(out), F, groups, eps); \
+    lia_launch(silu_gate_norm_kernel<T, VEC>, dim3(grid), dim3(128), smem, stream, o, reinterpret_cast<const T*>(z), ldz, w, reinterpret_cast<T*>(out), F, groups, eps); \
   } while (0)
   if (act_f32 && vec) LIA_SGN(float, 4);
   else if (act_f32) LIA_SGN(float, 1);

@@ -16,6 +16,7 @@
 
 #include "act.cuh"
 #include "common.cuh"
+#include "rowvec.cuh"
 
 namespace {
 
@@ -55,6 +56,8 @@ __device__ __forceinline__ void row_stats(const float* row, int W, float eps, fl
 template <typename T>
 __global__ void __launch_bounds__(256) embed_rows_kernel(const int64_t* __restrict__ ids, const T* __restrict__ table, float* __restrict__ x,
                                                          float* __restrict__ x_copy, int W, int vocab) {
+  pdl_launch_dependents();
+  pdl_wait();
   long long id = ids[blockIdx.x];
   if (id < 0 || id >= vocab) id = 0;     // the host checks the range; never read outside the table
   const T* e = table + (size_t)id * W;
@@ -70,6 +73,8 @@ __global__ void __launch_bounds__(256) ln_add_norm_kernel(float* __restrict__ x,
                                                           const float* __restrict__ b_post, float mult, const float* __restrict__ extra,
                                                           const float* __restrict__ w_pre, const float* __restrict__ b_pre, TH* __restrict__ h, int W,
                                                           float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float xs[];
   __shared__ float red[8];
   const size_t base = (size_t)blockIdx.x * W;
@@ -98,9 +103,79 @@ __global__ void __launch_bounds__(256) ln_add_norm_kernel(float* __restrict__ x,
   for (int i = threadIdx.x; i < W; i += 256) stf(h + base + i, (xs[i] - mean) * inv * w_pre[i] + b_pre[i]);
 }
 
+// The same for rows of up to 1024 V numbers that come as whole vectors of 4: a row stays in registers between its passes and a statistic costs one
+// barrier.  A decoded token's rows are a handful, so what counts is the chain of four reductions.
+__device__ __forceinline__ float4 normed4(const float4& v, float mean, float inv, const float* w, const float* b) {
+  const float4 g = load4(w), c = load4(b);
+  return make_float4((v.x - mean) * inv * g.x + c.x, (v.y - mean) * inv * g.y + c.y, (v.z - mean) * inv * g.z + c.z, (v.w - mean) * inv * g.w + c.w);
+}
+template <int V>
+__device__ __forceinline__ void row_stats4(const float4 (&v)[V], int W, float eps, float* red, float& mean, float& inv) {
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < V; ++i)
+    if ((int)(threadIdx.x + i * 256) * 4 < W) s += sum4(v[i]);
+  mean = block_sum256(s, red) / (float)W;
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < V; ++i)
+    if ((int)(threadIdx.x + i * 256) * 4 < W) {
+      const float4 d = make_float4(v[i].x - mean, v[i].y - mean, v[i].z - mean, v[i].w - mean);
+      ss += dot4(d, d);
+    }
+  inv = 1.0f / sqrtf(block_sum256(ss, red + 8) / (float)W + eps);
+}
+template <typename TY, typename TH, int V>
+__global__ void __launch_bounds__(256) ln_add_norm_vec_kernel(float* __restrict__ x, const TY* __restrict__ y, const float* __restrict__ w_post,
+                                                              const float* __restrict__ b_post, float mult, const float* __restrict__ extra,
+                                                              const float* __restrict__ w_pre, const float* __restrict__ b_pre, TH* __restrict__ h, int W,
+                                                              float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ __align__(16) float red[32];
+  const size_t base = (size_t)blockIdx.x * W;
+  float4 xv[V], yv[V];
+  float mean, inv;
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const int c = (threadIdx.x + i * 256) * 4;
+    if (c < W) {
+      xv[i] = load4(x + base + c);
+      if (y != nullptr) yv[i] = load4(y + base + c);
+    }
+  }
+  if (y != nullptr) row_stats4(yv, W, eps, red, mean, inv);
+  if (y != nullptr || extra != nullptr) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int c = (threadIdx.x + i * 256) * 4;
+      if (c < W) {
+        if (y != nullptr) {
+          const float4 n = normed4(yv[i], mean, inv, w_post + c, b_post + c);
+          xv[i].x += mult * n.x; xv[i].y += mult * n.y; xv[i].z += mult * n.z; xv[i].w += mult * n.w;
+        }
+        if (extra != nullptr) {
+          const float4 e = load4(extra + base + c);
+          xv[i].x += e.x; xv[i].y += e.y; xv[i].z += e.z; xv[i].w += e.w;
+        }
+        store4(x + base + c, xv[i]);
+      }
+    }
+  }
+  if (h == nullptr) return;
+  row_stats4(xv, W, eps, red + 16, mean, inv);
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const int c = (threadIdx.x + i * 256) * 4;
+    if (c < W) store4(h + base + c, normed4(xv[i], mean, inv, w_pre + c, b_pre + c));
+  }
+}
+
 template <typename TH>
 __global__ void __launch_bounds__(256) ln_gather_kernel(const float* __restrict__ x, const int* __restrict__ rows, const float* __restrict__ w,
                                                         const float* __restrict__ b, TH* __restrict__ h, int W, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float xs[];
   __shared__ float red[8];
   const size_t src = (size_t)rows[blockIdx.x] * W, dst = (size_t)blockIdx.x * W;
@@ -117,6 +192,8 @@ __global__ void __launch_bounds__(256) ln_gather_kernel(const float* __restrict_
 template <typename T>
 __global__ void gated_act_kernel(const T* __restrict__ in, int ld, int up_off, T* __restrict__ out, int M, int F, int act,
                                  const int* __restrict__ perm, const float* __restrict__ wt) {
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t n = (size_t)M * F;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     const size_t m = e / F;
@@ -129,6 +206,27 @@ __global__ void gated_act_kernel(const T* __restrict__ in, int ld, int up_off, T
   }
 }
 
+// the same, four columns per thread
+template <typename T>
+__global__ void __launch_bounds__(256) gated_act_vec_kernel(const T* __restrict__ in, int ld, int up_off, T* __restrict__ out, unsigned quads, int F, int act,
+                                                            const int* __restrict__ perm, const float* __restrict__ wt) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const unsigned e = blockIdx.x * 256 + threadIdx.x;
+  if (e >= quads) return;
+  const unsigned per = (unsigned)F / 4, m = e / per, f = (e - m * per) * 4;
+  float ws = 1.0f;
+  if (perm != nullptr) ws = perm[m] < 0 ? 0.f : wt[perm[m]];
+  const T* row = in + (size_t)m * ld + f;
+  const float4 a = load4(row);
+  float4 v = make_float4(act_apply(ws * a.x, act), act_apply(ws * a.y, act), act_apply(ws * a.z, act), act_apply(ws * a.w, act));
+  if (up_off >= 0) {
+    const float4 u = load4(row + up_off);
+    v.x *= ws * u.x; v.y *= ws * u.y; v.z *= ws * u.z; v.w *= ws * u.w;
+  }
+  store4(out + (size_t)e * 4, v);
+}
+
 // ---------------------------------------------------------------------------------------------------- router
 // One warp per token: softmax over E logits (fp32), or a sigmoid of each (`sigmoid`), then `top` rounds of arg-max (lowest
 // index on ties) over the scores plus an optional per-expert correction that takes part in the choice only; a chosen expert's
@@ -138,6 +236,8 @@ __global__ void gated_act_kernel(const T* __restrict__ in, int ld, int up_off, T
 __global__ void __launch_bounds__(128) router_topk_kernel(const float* __restrict__ logits, int ldl, const float* __restrict__ correction,
                                                           int* __restrict__ idx, float* __restrict__ wt, int M, int E, int top, int renorm,
                                                           int sigmoid, int groups, int keep) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float sc[];          // [4 warps][2][E]: scores, choice scores; then [4 warps][groups]: the groups' best
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * 4 + warp;
@@ -222,6 +322,8 @@ constexpr int TM = 64;        // rows of a tile of the grouped projection
 //   pos_of[pair]        = its place in perm (the row of the experts' intermediate buffer)
 __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ idx, int pairs, int E, int n_tiles, int* __restrict__ perm,
                                                         int* __restrict__ tile_expert, int* __restrict__ pos_of, int tile_rows) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ int sh[];            // count[E] | offset[E]
   int* count = sh;
   int* offset = sh + E;
@@ -260,6 +362,8 @@ __global__ void __launch_bounds__(256) moe_gemm_kernel(const TA* __restrict__ A,
                                                        int ldc, const int* __restrict__ perm, const int* __restrict__ tile_expert,
                                                        const float* __restrict__ wt, int top, int N, int K, int act, int n_real, float p0, float p1,
                                                        int weigh_in) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int e = tile_expert[blockIdx.y];
   if (e < 0 || e >= n_real) return;
   __shared__ float As[16][TM + 4];
@@ -355,6 +459,8 @@ template <typename TA, typename TW, typename TC, bool UP>
 __global__ void __launch_bounds__(128) moe_fewrows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ Wt, long long sW, TC* __restrict__ C,
                                                           int ldc, const int* __restrict__ idx, const float* __restrict__ wt, int top, int N, int K,
                                                           int act, int gated, int n_real, float p0, float p1, int weigh_in) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int p = blockIdx.y, n = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (n >= N || idx[p] >= n_real) return;
   const TW* wr = Wt + (size_t)idx[p] * sW + (size_t)n * K;
@@ -385,6 +491,8 @@ __global__ void __launch_bounds__(128) moe_fewrows_kernel(const TA* __restrict__
 // dst[place] = src[perm[place] / top] for every place of the plan, zeros in the padding: the experts' inputs, expert by expert
 template <typename T>
 __global__ void moe_gather_kernel(const T* __restrict__ src, const int* __restrict__ perm, T* __restrict__ dst, int places, int W, int top) {
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t n = (size_t)places * W;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     const size_t r = e / W;
@@ -396,6 +504,8 @@ __global__ void moe_gather_kernel(const T* __restrict__ src, const int* __restri
 
 // the same for rows of whole 16 bytes: block per place, `vecs` of them per row (number by number: 32 us for 4736 rows of 2048 bf16; 6 us so)
 __global__ void __launch_bounds__(128) moe_gather_vec_kernel(const uint4* __restrict__ src, const int* __restrict__ perm, uint4* __restrict__ dst, int vecs, int top) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int p = perm[blockIdx.x];
   const uint4* from = src + (size_t)(p < 0 ? 0 : p / top) * vecs;
   uint4* to = dst + (size_t)blockIdx.x * vecs;
@@ -410,6 +520,8 @@ template <typename TY, typename TS>
 __global__ void moe_combine_kernel(const TY* __restrict__ ypair, const int* __restrict__ pos_of, const float* __restrict__ wt,
                                    const TS* __restrict__ shared, float* __restrict__ y, int M, int W, int top, const int* __restrict__ idx,
                                    int n_real, const TS* __restrict__ h, int weighted, const float* __restrict__ sgate, int ldg) {
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t n = (size_t)M * W;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     const size_t m = e / W;
@@ -427,19 +539,13 @@ __global__ void moe_combine_kernel(const TY* __restrict__ ypair, const int* __re
 }
 
 // the same, four columns per thread and one block per row: numbers and pairs of a row are read as whole vectors
-__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 load4(const bf16* p) {
-  const uint2 u = *reinterpret_cast<const uint2*>(p);
-  float4 f;
-  unpack_bf16x2(u.x, f.x, f.y);
-  unpack_bf16x2(u.y, f.z, f.w);
-  return f;
-}
 template <typename TY, typename TS>
 __global__ void __launch_bounds__(256) moe_combine_vec_kernel(const TY* __restrict__ ypair, const int* __restrict__ pos_of, const float* __restrict__ wt,
                                                               const TS* __restrict__ shared, float* __restrict__ y, int W, int top,
                                                               const int* __restrict__ idx, int n_real, const TS* __restrict__ h, int weighted,
                                                               const float* __restrict__ sgate, int ldg) {
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t m = blockIdx.x;
   const float gate = sgate ? 1.0f + expf(-sgate[m * ldg]) : 1.0f;
   for (int c = threadIdx.x * 4; c < W; c += 1024) {
@@ -480,8 +586,8 @@ extern "C" int lia_embed_rows(const int64_t* ids, const void* table, int table_f
                               lia_stream_t stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LIA_CHECK_ARG(ids && table && x && rows > 0 && W > 0 && vocab > 0, "lia_embed_rows: bad arguments");
-  if (table_f32) embed_rows_kernel<float><<<rows, 256, 0, stream>>>(ids, reinterpret_cast<const float*>(table), x, x_copy, W, vocab);
-  else embed_rows_kernel<bf16><<<rows, 256, 0, stream>>>(ids, reinterpret_cast<const bf16*>(table), x, x_copy, W, vocab);
+  if (table_f32) lia_launch(embed_rows_kernel<float>, dim3(rows), dim3(256), 0, stream, ids, reinterpret_cast<const float*>(table), x, x_copy, W, vocab);
+  else lia_launch(embed_rows_kernel<bf16>, dim3(rows), dim3(256), 0, stream, ids, reinterpret_cast<const bf16*>(table), x, x_copy, W, vocab);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -494,10 +600,25 @@ extern "C" int lia_ln_add_norm(float* x, const void* y, int y_f32, const float* 
   LIA_CHECK_ARG(!h || (w_pre && b_pre), "lia_ln_add_norm: the norm before the sublayer needs a weight and a bias");
   LIA_CHECK_ARG(rows > 0 && W > 0 && (size_t)W * 4 <= 160 * 1024, "lia_ln_add_norm: bad shape rows=%d W=%d", rows, W);
   const size_t smem = (size_t)W * sizeof(float);
+  const bool vec = W % 4 == 0 && W <= 4096 && rows_of_4(x, W) && rows_of_4(reinterpret_cast<const float*>(y), W) && rows_of_4(reinterpret_cast<float*>(h), W) &&
+                   rows_of_4(w_post, 4) && rows_of_4(b_post, 4) && rows_of_4(extra, W) && rows_of_4(w_pre, 4) && rows_of_4(b_pre, 4);
+#define LIA_LANV(TY, TH, V) \
+  lia_launch(ln_add_norm_vec_kernel<TY, TH, V>, dim3(rows), dim3(256), 0, stream, x, reinterpret_cast<const TY*>(y), w_post, b_post, mult, extra, w_pre, b_pre, reinterpret_cast<TH*>(h), W, eps)
+#define LIA_LANT(TY, TH) (W <= 1024 ? (void)LIA_LANV(TY, TH, 1) : W <= 2048 ? (void)LIA_LANV(TY, TH, 2) : (void)LIA_LANV(TY, TH, 4))
+  if (vec) {
+    if (y_f32 && h_f32) LIA_LANT(float, float);
+    else if (y_f32) LIA_LANT(float, bf16);
+    else if (h_f32) LIA_LANT(bf16, float);
+    else LIA_LANT(bf16, bf16);
+    LIA_LAUNCH_CHECK();
+    return LIA_OK;
+  }
+#undef LIA_LANT
+#undef LIA_LANV
 #define LIA_LAN(TY, TH)                                                                                                     \
   do {                                                                                                                      \
     if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(ln_add_norm_kernel<TY, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    ln_add_norm_kernel<TY, TH><<<rows, 256, smem, stream>>>(x, reinterpret_cast<const TY*>(y), w_post, b_post, mult, extra, w_pre, b_pre, \
+    lia_launch(ln_add_norm_kernel<TY, TH>, dim3(rows), dim3(256), smem, stream, x, reinterpret_cast<const TY*>(y), w_post, b_post, mult, extra, w_pre, b_pre, \
                                                             reinterpret_cast<TH*>(h), W, eps);                              \
   } while (0)
   if (y_f32 && h_f32) LIA_LAN(float, float);
@@ -516,10 +637,10 @@ extern "C" int lia_ln_gather(const float* x, const int* rows, const float* w, co
   const size_t smem = (size_t)W * sizeof(float);
   if (h_f32) {
     if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(ln_gather_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    ln_gather_kernel<float><<<n, 256, smem, stream>>>(x, rows, w, b, reinterpret_cast<float*>(h), W, eps);
+    lia_launch(ln_gather_kernel<float>, dim3(n), dim3(256), smem, stream, x, rows, w, b, reinterpret_cast<float*>(h), W, eps);
   } else {
     if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(ln_gather_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    ln_gather_kernel<bf16><<<n, 256, smem, stream>>>(x, rows, w, b, reinterpret_cast<bf16*>(h), W, eps);
+    lia_launch(ln_gather_kernel<bf16>, dim3(n), dim3(256), smem, stream, x, rows, w, b, reinterpret_cast<bf16*>(h), W, eps);
   }
   LIA_LAUNCH_CHECK();
   return LIA_OK;
@@ -535,9 +656,19 @@ extern "C" int lia_gated_act_weighted(const void* in, int ld, int up_off, void* 
   LIA_CHECK_ARG(in && out && M > 0 && F > 0 && ld >= F && (up_off < 0 || (up_off >= F && ld >= up_off + F)), "lia_gated_act: bad arguments");
   LIA_CHECK_ARG((perm == nullptr) == (wt == nullptr), "lia_gated_act: a row order and routing weights go together");
   LIA_CHECK_ARG((act >= LIA_ACT_NONE && act <= LIA_ACT_GELU_TANH) || act == LIA_ACT_RELU_SQUARED, "lia_gated_act: unknown activation %d", act);
+  const long long quads = (long long)M * (F / 4);
+  const int sz = act_f32 ? 4 : 2;
+  if (F % 4 == 0 && ld % 4 == 0 && (up_off < 0 || up_off % 4 == 0) && reinterpret_cast<uintptr_t>(in) % (4 * sz) == 0 && reinterpret_cast<uintptr_t>(out) % (4 * sz) == 0 &&
+      quads < (1ll << 31)) {
+    const unsigned g = (unsigned)((quads + 255) / 256);
+    if (act_f32) lia_launch(gated_act_vec_kernel<float>, dim3(g), dim3(256), 0, stream, reinterpret_cast<const float*>(in), ld, up_off, reinterpret_cast<float*>(out), (unsigned)quads, F, act, perm, wt);
+    else lia_launch(gated_act_vec_kernel<bf16>, dim3(g), dim3(256), 0, stream, reinterpret_cast<const bf16*>(in), ld, up_off, reinterpret_cast<bf16*>(out), (unsigned)quads, F, act, perm, wt);
+    LIA_LAUNCH_CHECK();
+    return LIA_OK;
+  }
   const unsigned blocks = capped_blocks((size_t)M * F);
-  if (act_f32) gated_act_kernel<float><<<blocks, 256, 0, stream>>>(reinterpret_cast<const float*>(in), ld, up_off, reinterpret_cast<float*>(out), M, F, act, perm, wt);
-  else gated_act_kernel<bf16><<<blocks, 256, 0, stream>>>(reinterpret_cast<const bf16*>(in), ld, up_off, reinterpret_cast<bf16*>(out), M, F, act, perm, wt);
+  if (act_f32) lia_launch(gated_act_kernel<float>, dim3(blocks), dim3(256), 0, stream, reinterpret_cast<const float*>(in), ld, up_off, reinterpret_cast<float*>(out), M, F, act, perm, wt);
+  else lia_launch(gated_act_kernel<bf16>, dim3(blocks), dim3(256), 0, stream, reinterpret_cast<const bf16*>(in), ld, up_off, reinterpret_cast<bf16*>(out), M, F, act, perm, wt);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -566,7 +697,7 @@ extern "C" int lia_router_topk_grouped(const float* logits, int ldl, const float
                 "lia_router_topk: %d experts, %d of %d groups, %d chosen", E, keep, groups, top);
   const size_t smem = ((size_t)8 * E + 4 * groups) * sizeof(float);
   if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(router_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  router_topk_kernel<<<(M + 3) / 4, 128, smem, stream>>>(logits, ldl, correction, idx, wt, M, E, top, renorm, sigmoid, groups, keep);
+  lia_launch(router_topk_kernel, dim3((M + 3) / 4), dim3(128), smem, stream, logits, ldl, correction, idx, wt, M, E, top, renorm, sigmoid, groups, keep);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -582,7 +713,7 @@ extern "C" int lia_moe_plan_rows(const int* idx, int pairs, int E, int tile_rows
   LIA_CHECK_ARG(idx && perm && tile_expert && pos_of && pairs > 0 && E > 0 && E <= 4096 && tile_rows > 0, "lia_moe_plan: bad arguments");
   LIA_CHECK_ARG(n_tiles >= (int)(((long long)pairs + (long long)(E < pairs ? E : pairs) * (tile_rows - 1)) / tile_rows),
                 "lia_moe_plan: %d tiles cannot hold %d pairs of %d experts", n_tiles, pairs, E);
-  moe_plan_kernel<<<1, 1024, (size_t)2 * E * sizeof(int), stream>>>(idx, pairs, E, n_tiles, perm, tile_expert, pos_of, tile_rows);
+  lia_launch(moe_plan_kernel, dim3(1), dim3(1024), (size_t)2 * E * sizeof(int), stream, idx, pairs, E, n_tiles, perm, tile_expert, pos_of, tile_rows);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -625,18 +756,18 @@ extern "C" int lia_moe_gemm_weighted(const void* A, int a_f32, int lda, const vo
     LIA_CHECK_ARG(pairs <= 65535, "lia_moe_gemm: too many pairs for the few-rows form");
     dim3 grid((N + 3) / 4, pairs);
     if (a_f32) {
-      if (up) moe_fewrows_kernel<float, float, float, true><<<grid, 128, 0, stream>>>((const float*)A, lda, (const float*)W, w_expert_stride, (float*)C, ldc, idx, wt, top, N, K, act, gated, n_real, p0, p1, weigh_in);
-      else moe_fewrows_kernel<float, float, float, false><<<grid, 128, 0, stream>>>((const float*)A, lda, (const float*)W, w_expert_stride, (float*)C, ldc, idx, wt, top, N, K, act, gated, n_real, p0, p1, weigh_in);
+      if (up) lia_launch(moe_fewrows_kernel<float, float, float, true>, dim3(grid), dim3(128), 0, stream, (const float*)A, lda, (const float*)W, w_expert_stride, (float*)C, ldc, idx, wt, top, N, K, act, gated, n_real, p0, p1, weigh_in);
+      else lia_launch(moe_fewrows_kernel<float, float, float, false>, dim3(grid), dim3(128), 0, stream, (const float*)A, lda, (const float*)W, w_expert_stride, (float*)C, ldc, idx, wt, top, N, K, act, gated, n_real, p0, p1, weigh_in);
     } else {
-      if (up) moe_fewrows_kernel<bf16, bf16, bf16, true><<<grid, 128, 0, stream>>>((const bf16*)A, lda, (const bf16*)W, w_expert_stride, (bf16*)C, ldc, idx, wt, top, N, K, act, gated, n_real, p0, p1, weigh_in);
-      else moe_fewrows_kernel<bf16, bf16, float, false><<<grid, 128, 0, stream>>>((const bf16*)A, lda, (const bf16*)W, w_expert_stride, (float*)C, ldc, idx, wt, top, N, K, act, gated, n_real, p0, p1, weigh_in);
+      if (up) lia_launch(moe_fewrows_kernel<bf16, bf16, bf16, true>, dim3(grid), dim3(128), 0, stream, (const bf16*)A, lda, (const bf16*)W, w_expert_stride, (bf16*)C, ldc, idx, wt, top, N, K, act, gated, n_real, p0, p1, weigh_in);
+      else lia_launch(moe_fewrows_kernel<bf16, bf16, float, false>, dim3(grid), dim3(128), 0, stream, (const bf16*)A, lda, (const bf16*)W, w_expert_stride, (float*)C, ldc, idx, wt, top, N, K, act, gated, n_real, p0, p1, weigh_in);
     }
     LIA_LAUNCH_CHECK();
     return LIA_OK;
   }
   LIA_CHECK_ARG(tile_expert && n_tiles > 0 && n_tiles <= 65535, "lia_moe_gemm: bad tile plan");
   dim3 grid((N + 63) / 64, n_tiles);
-#define LIA_MG(TA, TC, UP_, GATED_) moe_gemm_kernel<TA, TA, TC, UP_, GATED_><<<grid, 256, 0, stream>>>((const TA*)A, lda, (const TA*)W, w_expert_stride, (TC*)C, ldc, perm, tile_expert, wt, top, N, K, act, n_real, p0, p1, weigh_in)
+#define LIA_MG(TA, TC, UP_, GATED_) lia_launch(moe_gemm_kernel<TA, TA, TC, UP_, GATED_>, dim3(grid), dim3(256), 0, stream, (const TA*)A, lda, (const TA*)W, w_expert_stride, (TC*)C, ldc, perm, tile_expert, wt, top, N, K, act, n_real, p0, p1, weigh_in)
   if (a_f32) {
     if (up && gated) LIA_MG(float, float, true, true);
     else if (up) LIA_MG(float, float, true, false);
@@ -656,13 +787,13 @@ extern "C" int lia_moe_gather(const void* src, int act_f32, const int* perm, voi
   LIA_CHECK_ARG(src && perm && dst && places > 0 && W > 0 && top > 0, "lia_moe_gather: bad arguments");
   const size_t row_bytes = (size_t)W * (act_f32 ? 4 : 2);
   if (row_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) % 16 == 0) {
-    moe_gather_vec_kernel<<<places, 128, 0, stream>>>(reinterpret_cast<const uint4*>(src), perm, reinterpret_cast<uint4*>(dst), (int)(row_bytes / 16), top);
+    lia_launch(moe_gather_vec_kernel, dim3(places), dim3(128), 0, stream, reinterpret_cast<const uint4*>(src), perm, reinterpret_cast<uint4*>(dst), (int)(row_bytes / 16), top);
     LIA_LAUNCH_CHECK();
     return LIA_OK;
   }
   const unsigned blocks = capped_blocks((size_t)places * W);
-  if (act_f32) moe_gather_kernel<float><<<blocks, 256, 0, stream>>>(reinterpret_cast<const float*>(src), perm, reinterpret_cast<float*>(dst), places, W, top);
-  else moe_gather_kernel<bf16><<<blocks, 256, 0, stream>>>(reinterpret_cast<const bf16*>(src), perm, reinterpret_cast<bf16*>(dst), places, W, top);
+  if (act_f32) lia_launch(moe_gather_kernel<float>, dim3(blocks), dim3(256), 0, stream, reinterpret_cast<const float*>(src), perm, reinterpret_cast<float*>(dst), places, W, top);
+  else lia_launch(moe_gather_kernel<bf16>, dim3(blocks), dim3(256), 0, stream, reinterpret_cast<const bf16*>(src), perm, reinterpret_cast<bf16*>(dst), places, W, top);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -709,7 +840,7 @@ extern "C" int lia_moe_combine_gated(const void* ypair, int ypair_f32, const int
   const unsigned blocks = capped_blocks((size_t)M * W);
 const uintptr_t addr = reinterpret_cast<uintptr_t>(ypair) | reinterpret_cast<uintptr_t>(shared) | reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(y);
   if (W % 4 == 0 && addr % 16 == 0) {
-#define LIA_MCV(TY, TS) moe_combine_vec_kernel<TY, TS><<<M, 256, 0, stream>>>(reinterpret_cast<const TY*>(ypair), pos_of, wt, reinterpret_cast<const TS*>(shared), y, W, top, idx, n_real, reinterpret_cast<const TS*>(h), weighted, shared_gate, ldg)
+#define LIA_MCV(TY, TS) lia_launch(moe_combine_vec_kernel<TY, TS>, dim3(M), dim3(256), 0, stream, reinterpret_cast<const TY*>(ypair), pos_of, wt, reinterpret_cast<const TS*>(shared), y, W, top, idx, n_real, reinterpret_cast<const TS*>(h), weighted, shared_gate, ldg)
     if (ypair_f32 && act_f32) LIA_MCV(float, float);
     else if (ypair_f32) LIA_MCV(float, bf16);
     else if (act_f32) LIA_MCV(bf16, float);
@@ -718,7 +849,7 @@ const uintptr_t addr = reinterpret_cast<uintptr_t>(ypair) | reinterpret_cast<uin
     LIA_LAUNCH_CHECK();
     return LIA_OK;
   }
-#define LIA_MC(TY, TS) moe_combine_kernel<TY, TS><<<blocks, 256, 0, stream>>>(reinterpret_cast<const TY*>(ypair), pos_of, wt, reinterpret_cast<const TS*>(shared), y, M, W, top, idx, n_real, reinterpret_cast<const TS*>(h), weighted, shared_gate, ldg)
+#define LIA_MC(TY, TS) lia_launch(moe_combine_kernel<TY, TS>, dim3(blocks), dim3(256), 0, stream, reinterpret_cast<const TY*>(ypair), pos_of, wt, reinterpret_cast<const TS*>(shared), y, M, W, top, idx, n_real, reinterpret_cast<const TS*>(h), weighted, shared_gate, ldg)
   if (ypair_f32 && act_f32) LIA_MC(float, float);
   else if (ypair_f32) LIA_MC(float, bf16);
   else if (act_f32) LIA_MC(bf16, float);

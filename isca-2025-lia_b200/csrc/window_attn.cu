@@ -30,6 +30,8 @@ template <typename T>
 __global__ void __launch_bounds__(128) kv_store_kernel(const T* __restrict__ k, int ldk, const T* __restrict__ v, int ldv, const int* __restrict__ meta,
                                                        T* __restrict__ kcache, long long k_slot_stride, T* __restrict__ vcache, long long v_slot_stride,
                                                        int G, int dim, int vdim, float eps, int norm_values) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.x;
   const int slot = meta[2 * row], pos = meta[2 * row + 1];
   T* kr = kcache + (size_t)slot * k_slot_stride + (size_t)pos * G * dim;
@@ -74,6 +76,8 @@ __global__ void __launch_bounds__(256) qkv_prep_kernel(const T* __restrict__ y, 
                                                        const float* __restrict__ knorm_w, const double* __restrict__ freq, const int* __restrict__ meta,
                                                        float* __restrict__ v_first, float* __restrict__ q_out, T* __restrict__ kcache,
                                                        long long k_slot_stride, T* __restrict__ vcache, long long v_slot_stride, PrepArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float ch[];                 // C channels q | k | v, then cos | sin of the rotation's pairs
   __shared__ float red[8];
   const int row = blockIdx.x;
@@ -221,6 +225,8 @@ __global__ void __launch_bounds__(NWARP * 32) window_attn_kernel(const void* __r
                                                                 const T* __restrict__ vcache, long long v_slot_stride, const int* __restrict__ meta,
                                                                 WindowExtras x, T* __restrict__ out, float* __restrict__ part,
                                                                 float2* __restrict__ part_ml, int M, WindowArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float sm[];
   const int DKS = key_stride(a.dim);
   float* qs = sm;                                             // [QR * HB][dim]
@@ -424,6 +430,8 @@ __global__ void __launch_bounds__(NWARP * 32) window_attn_kernel(const void* __r
 template <typename T>
 __global__ void __launch_bounds__(128) window_combine_kernel(const float* __restrict__ part, const float2* __restrict__ part_ml, T* __restrict__ out,
                                                              int vdim, int nsplit, WindowExtras x, WindowArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t rh = blockIdx.x;
   const int h = (int)(rh % a.H);
   const size_t row = rh / a.H;
@@ -453,6 +461,8 @@ __global__ void __launch_bounds__(128) window_combine_kernel(const float* __rest
 template <typename T>
 __global__ void __launch_bounds__(128) diff_combine_kernel(const float* __restrict__ a, T* __restrict__ out, int M, int H, int G, int vdim,
                                                            float lambda, float mult, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   const long long pair = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (pair >= (long long)M * H) return;
@@ -473,8 +483,8 @@ __global__ void __launch_bounds__(128) diff_combine_kernel(const float* __restri
 
 int window_combine(const float* part, const float2* part_ml, void* out, int act_f32, int M, const WindowExtras& x, const WindowArgs& a, cudaStream_t stream) {
   const unsigned grid = (unsigned)((size_t)M * a.H);
-  if (act_f32) window_combine_kernel<float><<<grid, 128, 0, stream>>>(part, part_ml, reinterpret_cast<float*>(out), a.vdim, a.nsplit, x, a);
-  else window_combine_kernel<bf16><<<grid, 128, 0, stream>>>(part, part_ml, reinterpret_cast<bf16*>(out), a.vdim, a.nsplit, x, a);
+  if (act_f32) lia_launch(window_combine_kernel<float>, dim3(grid), dim3(128), 0, stream, part, part_ml, reinterpret_cast<float*>(out), a.vdim, a.nsplit, x, a);
+  else lia_launch(window_combine_kernel<bf16>, dim3(grid), dim3(128), 0, stream, part, part_ml, reinterpret_cast<bf16*>(out), a.vdim, a.nsplit, x, a);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -494,7 +504,7 @@ int launch_attn(const void* q, int ldq, const void* kcache, long long kss, const
   dim3 grid((M + a.QR - 1) / a.QR, (a.H + a.HB - 1) / a.HB, a.nsplit);
   float* part = ws;
   float2* part_ml = reinterpret_cast<float2*>(ws + (size_t)M * a.H * a.nsplit * a.vdim);
-  window_attn_kernel<T, VR, PP><<<grid, NWARP * 32, smem, stream>>>(q, ldq, reinterpret_cast<const T*>(kcache), kss,
+  lia_launch(window_attn_kernel<T, VR, PP>, dim3(grid), dim3(NWARP * 32), smem, stream, q, ldq, reinterpret_cast<const T*>(kcache), kss,
                                                                    reinterpret_cast<const T*>(vcache), vss, meta, x, reinterpret_cast<T*>(out), part,
                                                                    part_ml, M, a);
   LIA_LAUNCH_CHECK();
@@ -520,10 +530,10 @@ extern "C" int lia_kv_store(const void* k, int ldk, const void* v, int ldv, int 
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LIA_CHECK_ARG(k && v && meta && kcache && vcache && M > 0 && G > 0 && dim > 0 && vdim > 0 && ldk >= G * dim && ldv >= G * vdim, "lia_kv_store: bad arguments");
   if (act_f32)
-    kv_store_kernel<float><<<M, 128, 0, stream>>>(reinterpret_cast<const float*>(k), ldk, reinterpret_cast<const float*>(v), ldv, meta,
+    lia_launch(kv_store_kernel<float>, dim3(M), dim3(128), 0, stream, reinterpret_cast<const float*>(k), ldk, reinterpret_cast<const float*>(v), ldv, meta,
                                                   reinterpret_cast<float*>(kcache), k_slot_stride, reinterpret_cast<float*>(vcache), v_slot_stride, G, dim, vdim, eps, norm_values);
   else
-    kv_store_kernel<bf16><<<M, 128, 0, stream>>>(reinterpret_cast<const bf16*>(k), ldk, reinterpret_cast<const bf16*>(v), ldv, meta,
+    lia_launch(kv_store_kernel<bf16>, dim3(M), dim3(128), 0, stream, reinterpret_cast<const bf16*>(k), ldk, reinterpret_cast<const bf16*>(v), ldv, meta,
                                                  reinterpret_cast<bf16*>(kcache), k_slot_stride, reinterpret_cast<bf16*>(vcache), v_slot_stride, G, dim, vdim, eps, norm_values);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
@@ -560,11 +570,11 @@ extern "C" int lia_qkv_prep_heads(const void* y, int act_f32, int ld, int q_off,
   LIA_CHECK_ARG(smem <= 160 * 1024, "lia_qkv_prep: %d channels do not fit shared memory", (H + G) * dim + Gv * vdim);
   if (act_f32) {
     if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(qkv_prep_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    qkv_prep_kernel<float><<<M, 256, smem, stream>>>(reinterpret_cast<const float*>(y), ld, bias, wconv, conv_state, qnorm_w, knorm_w, freq, meta, v_first,
+    lia_launch(qkv_prep_kernel<float>, dim3(M), dim3(256), smem, stream, reinterpret_cast<const float*>(y), ld, bias, wconv, conv_state, qnorm_w, knorm_w, freq, meta, v_first,
                                                      q_out, reinterpret_cast<float*>(kcache), k_slot_stride, reinterpret_cast<float*>(vcache), v_slot_stride, a);
   } else {
     if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(qkv_prep_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    qkv_prep_kernel<bf16><<<M, 256, smem, stream>>>(reinterpret_cast<const bf16*>(y), ld, bias, wconv, conv_state, qnorm_w, knorm_w, freq, meta, v_first,
+    lia_launch(qkv_prep_kernel<bf16>, dim3(M), dim3(256), smem, stream, reinterpret_cast<const bf16*>(y), ld, bias, wconv, conv_state, qnorm_w, knorm_w, freq, meta, v_first,
                                                     q_out, reinterpret_cast<bf16*>(kcache), k_slot_stride, reinterpret_cast<bf16*>(vcache), v_slot_stride, a);
   }
   LIA_LAUNCH_CHECK();
@@ -634,8 +644,8 @@ extern "C" int lia_diff_combine(const float* a, void* out, int act_f32, int M, i
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LIA_CHECK_ARG(a && out && M > 0 && H > 0 && G > 0 && H % G == 0 && vdim > 0, "lia_diff_combine: bad arguments");
   const unsigned grid = (unsigned)(((long long)M * H + 3) / 4);
-  if (act_f32) diff_combine_kernel<float><<<grid, 128, 0, stream>>>(a, reinterpret_cast<float*>(out), M, H, G, vdim, lambda, mult, eps);
-  else diff_combine_kernel<bf16><<<grid, 128, 0, stream>>>(a, reinterpret_cast<bf16*>(out), M, H, G, vdim, lambda, mult, eps);
+  if (act_f32) lia_launch(diff_combine_kernel<float>, dim3(grid), dim3(128), 0, stream, a, reinterpret_cast<float*>(out), M, H, G, vdim, lambda, mult, eps);
+  else lia_launch(diff_combine_kernel<bf16>, dim3(grid), dim3(128), 0, stream, a, reinterpret_cast<bf16*>(out), M, H, G, vdim, lambda, mult, eps);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }

@@ -79,6 +79,8 @@ template <int DK, int DV, int NQ>
 __global__ void __launch_bounds__(128, (DV <= 128 && NQ == 1) ? 3 : 2) window_prompt_kernel(const void* __restrict__ q, int ldq, const bf16* __restrict__ kcache, long long k_slot_stride,
                                                             const bf16* __restrict__ vcache, long long v_slot_stride, const int* __restrict__ meta,
                                                             const int* __restrict__ segs, int nseg, WindowExtras x, bf16* __restrict__ out, int M, WindowArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int BK = PromptShape<DK, DV, NQ>::BK, QC = DK / 8, VC = DV / 8, NT = BK / 8;
   extern __shared__ __align__(128) unsigned char smem[];
   const uint32_t qs = smem_u32(smem), ks = qs + NQ * BM * DK * 2, vs = ks + 2 * BK * DK * 2;
@@ -281,6 +283,8 @@ __global__ void __launch_bounds__(128) window_decode_kernel(const void* __restri
                                                             const bf16* __restrict__ vcache, long long v_slot_stride, const int* __restrict__ meta,
                                                             WindowExtras x, bf16* __restrict__ out, float* __restrict__ part, float2* __restrict__ part_ml,
                                                             WindowArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int KC = DK / 32, VU = DV / 64;              // 16-byte chunks of a key row / value row per lane
   extern __shared__ __align__(16) float sums[];          // [4 warps][8 heads][DV]
   __shared__ float2 ml[4][8];
@@ -472,7 +476,7 @@ template <int DK, int DV, int NQ> int prompt_as(const Call& c) {
   constexpr int smem = PromptShape<DK, DV, NQ>::SMEM;
   LIA_CUDA(cudaFuncSetAttribute(window_prompt_kernel<DK, DV, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const dim3 grid(c.a.H, (c.M + BM - 1) / BM + (c.segs ? c.nseg - 1 : 0));     // at least as many tiles as the portions have
-  window_prompt_kernel<DK, DV, NQ><<<grid, 128, smem, c.stream>>>(c.q, c.ldq, c.kcache, c.kss, c.vcache, c.vss, c.meta, c.segs, c.nseg, c.x, c.out, c.M, c.a);
+  lia_launch(window_prompt_kernel<DK, DV, NQ>, dim3(grid), dim3(128), smem, c.stream, c.q, c.ldq, c.kcache, c.kss, c.vcache, c.vss, c.meta, c.segs, c.nseg, c.x, c.out, c.M, c.a);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -482,7 +486,7 @@ template <int DK, int DV, int NQ> int decode_as(const Call& c) {
   float* part = c.ws;
   float2* part_ml = reinterpret_cast<float2*>(c.ws + (size_t)c.M * c.a.H * c.a.nsplit * DV);
   const dim3 grid((unsigned)(c.M * (c.a.H / c.a.HB)), c.a.nsplit);
-  window_decode_kernel<DK, DV, NQ><<<grid, 128, smem, c.stream>>>(c.q, c.ldq, c.kcache, c.kss, c.vcache, c.vss, c.meta, c.x, c.out, part, part_ml, c.a);
+  lia_launch(window_decode_kernel<DK, DV, NQ>, dim3(grid), dim3(128), smem, c.stream, c.q, c.ldq, c.kcache, c.kss, c.vcache, c.vss, c.meta, c.x, c.out, part, part_ml, c.a);
   LIA_LAUNCH_CHECK();
   if (c.a.nsplit > 1) return window_combine(part, part_ml, c.out, 0, c.M, c.x, c.a, c.stream);
   return LIA_OK;
