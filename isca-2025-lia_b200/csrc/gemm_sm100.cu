@@ -679,6 +679,7 @@ static int gemm_impl(const void* A, const void* W, const void* bias, const void*
     if ((rc = make_tmap(&tmB, W, N, K, pl.pair ? pl.bn / 2 : pl.bn)) != LIA_OK) return rc;
     if (pl.pair) return launch_pair<256>(pl, tmA, tmB, ep, stream);
     if (pl.bn == 256) return launch<false, 256, 4>(pl, tmA, tmB, ep, ws, flags, stream);
+    if (pl.bn == 64) return launch_tp<false, 64, 8, false>(pl, tmA, tmB, ep, ws, flags, stream);
     return launch<false, 128, 6>(pl, tmA, tmB, ep, ws, flags, stream);
   }
 }
