@@ -286,6 +286,10 @@ int lia_argmax_f32(const float* logits, int64_t* next, int B, int V, int suppres
 int lia_mlstm_scan(const void* q, const void* k, const void* v, int act_f32, int ld, const float* gates, float* state_S, float* state_n,
                    float* state_m, const int* segs, int nseg, int H, int dim, int vdim, float q_scale, float den_eps, float* o,
                    lia_stream_t stream);
+/* the same with the caller's workspace of nseg * H * (dim + 1) floats, where the new n and m wait until every block has read the old ones */
+int lia_mlstm_scan_ws(const void* q, const void* k, const void* v, int act_f32, int ld, const float* gates, float* state_S, float* state_n,
+                      float* state_m, const int* segs, int nseg, int H, int dim, int vdim, float q_scale, float den_eps, float* o,
+                      float* ws, lia_stream_t stream);
 /* out[row][h] = o[row][h] / rms_over_vdim * w[h] * act(gate[row][h]), act = sigmoid (gate_silu == 0) or SiLU */
 int lia_headnorm_gate(const float* o, const float* w, const void* gate, int ldg, void* out, int act_f32, int M, int H, int vdim, float eps,
                       int gate_silu, lia_stream_t stream);

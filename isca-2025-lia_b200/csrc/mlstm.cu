@@ -83,7 +83,7 @@ constexpr int CB = CW * NW;      // columns per block
 template <typename T, int DR, bool VL>
 __global__ void __launch_bounds__(NW * 32, 2) mlstm_scan_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, int ld,
                                                              const float* __restrict__ gates, float* __restrict__ St, float* __restrict__ nst,
-                                                             float* __restrict__ mst, const int* __restrict__ segs, int H, int dim, int vdim,
+                                                             float* __restrict__ mst, float* __restrict__ ws, const int* __restrict__ segs, int H, int dim, int vdim,
                                                              float q_scale, float den_eps, float* __restrict__ o) {
   pdl_launch_dependents();
   pdl_wait();
@@ -227,17 +227,31 @@ __global__ void __launch_bounds__(NW * 32, 2) mlstm_scan_kernel(const T* __restr
     __syncthreads();
   }
 
+  // Every block of a head starts from the same n and m, and not all of them need be resident at once: the new n and m go to `ws` ([portion][head][dim + 1]),
+  // and the state takes them when all blocks are done (mlstm_state_kernel).  A head of one block writes them where they belong.
+  float* n_out = ws ? ws + ((size_t)seg * H + h) * (dim + 1) : np;
+  float* m_out = ws ? n_out + dim : mst + (size_t)slot * H + h;
 #pragma unroll
   for (int i = 0; i < DR; ++i) {
     const int r = lane + 32 * i;
     if (r < dim) {
-      if (colb == 0 && warp == 0) np[r] = n[i];
+      if (colb == 0 && warp == 0) n_out[r] = n[i];
 #pragma unroll
       for (int c = 0; c < CW; ++c)
         if (col0 + c < vdim) Sp[(size_t)(col0 + c) * dim + r] = S[i][c];
     }
   }
-  if (colb == 0 && threadIdx.x == 0) mst[(size_t)slot * H + h] = m;
+  if (colb == 0 && threadIdx.x == 0) *m_out = m;
+}
+
+__global__ void __launch_bounds__(128) mlstm_state_kernel(const float* __restrict__ ws, const int* __restrict__ segs, float* __restrict__ nst, float* __restrict__ mst, int H, int dim) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int h = blockIdx.x, seg = blockIdx.y;
+  const size_t head = (size_t)segs[4 * seg] * H + h;
+  const float* src = ws + ((size_t)seg * H + h) * (dim + 1);
+  for (int r = threadIdx.x; r < dim; r += 128) nst[head * dim + r] = src[r];
+  if (threadIdx.x == 0) mst[head] = src[dim];
 }
 
 // out[row][h][c] = o / sqrt(mean_c(o^2) + eps) * w[h*vdim + c] * act(gate[row][h*vdim + c]), act = sigmoid (gate_silu == 0) or
@@ -320,47 +334,63 @@ __global__ void __launch_bounds__(256) headnorm_gate_vec_kernel(const float* __r
 }
 
 template <typename T, int DR, bool VL>
-int launch_scan_as(const void* q, const void* k, const void* v, int ld, const float* gates, float* St, float* nst, float* mst, const int* segs,
+int launch_scan_as(const void* q, const void* k, const void* v, int ld, const float* gates, float* St, float* nst, float* mst, float* ws, const int* segs,
                 int nseg, int H, int dim, int vdim, float q_scale, float den_eps, float* o, cudaStream_t stream) {
   const size_t smem = (size_t)2 * TB * (2 * DR * 32 + CB + 4) * sizeof(float);
   if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(mlstm_scan_kernel<T, DR, VL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((vdim + CB - 1) / CB, H, nseg);
+  if (grid.x == 1) ws = nullptr;
   lia_launch_after(mlstm_scan_kernel<T, DR, VL>, dim3(grid), dim3(NW * 32), smem, stream, reinterpret_cast<const T*>(q), reinterpret_cast<const T*>(k), reinterpret_cast<const T*>(v),
-                                                            ld, gates, St, nst, mst, segs, H, dim, vdim, q_scale, den_eps, o);
+                                                            ld, gates, St, nst, mst, ws, segs, H, dim, vdim, q_scale, den_eps, o);
+  LIA_LAUNCH_CHECK();
+  if (ws != nullptr) lia_launch(mlstm_state_kernel, dim3(H, nseg), dim3(128), 0, stream, (const float*)ws, segs, nst, mst, H, dim);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
 
 template <typename T, int DR>
-int launch_scan(const void* q, const void* k, const void* v, int ld, const float* gates, float* St, float* nst, float* mst, const int* segs,
+int launch_scan(const void* q, const void* k, const void* v, int ld, const float* gates, float* St, float* nst, float* mst, float* ws, const int* segs,
                 int nseg, int H, int dim, int vdim, float q_scale, float den_eps, float* o, cudaStream_t stream) {
   constexpr int VEC = Vec128<T>::N;
   const bool aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) % 16 == 0) &&
                        ld % VEC == 0 && dim % VEC == 0 && vdim % VEC == 0;
-  if (aligned) return launch_scan_as<T, DR, true>(q, k, v, ld, gates, St, nst, mst, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
-  return launch_scan_as<T, DR, false>(q, k, v, ld, gates, St, nst, mst, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  if (aligned) return launch_scan_as<T, DR, true>(q, k, v, ld, gates, St, nst, mst, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  return launch_scan_as<T, DR, false>(q, k, v, ld, gates, St, nst, mst, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
 }
 
 template <typename T>
-int dispatch_scan(const void* q, const void* k, const void* v, int ld, const float* gates, float* St, float* nst, float* mst, const int* segs,
+int dispatch_scan(const void* q, const void* k, const void* v, int ld, const float* gates, float* St, float* nst, float* mst, float* ws, const int* segs,
                   int nseg, int H, int dim, int vdim, float q_scale, float den_eps, float* o, cudaStream_t stream) {
-  if (dim <= 32) return launch_scan<T, 1>(q, k, v, ld, gates, St, nst, mst, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
-  if (dim <= 64) return launch_scan<T, 2>(q, k, v, ld, gates, St, nst, mst, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
-  if (dim <= 128) return launch_scan<T, 4>(q, k, v, ld, gates, St, nst, mst, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
-  if (dim <= 256) return launch_scan<T, 8>(q, k, v, ld, gates, St, nst, mst, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
-  return launch_scan<T, 16>(q, k, v, ld, gates, St, nst, mst, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  if (dim <= 32) return launch_scan<T, 1>(q, k, v, ld, gates, St, nst, mst, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  if (dim <= 64) return launch_scan<T, 2>(q, k, v, ld, gates, St, nst, mst, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  if (dim <= 128) return launch_scan<T, 4>(q, k, v, ld, gates, St, nst, mst, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  if (dim <= 256) return launch_scan<T, 8>(q, k, v, ld, gates, St, nst, mst, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  return launch_scan<T, 16>(q, k, v, ld, gates, St, nst, mst, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
 }
 
 }  // namespace
 
+extern "C" int lia_mlstm_scan_ws(const void* q, const void* k, const void* v, int act_f32, int ld, const float* gates, float* state_S,
+                                 float* state_n, float* state_m, const int* segs, int nseg, int H, int dim, int vdim, float q_scale,
+                                 float den_eps, float* o, float* ws, lia_stream_t stream_) {
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  LIA_CHECK_ARG(q && k && v && gates && state_S && state_n && state_m && segs && o && ws, "lia_mlstm_scan: null pointer");
+  LIA_CHECK_ARG(nseg > 0 && nseg <= 65535 && H > 0 && H <= 65535 && dim > 0 && dim <= 512 && vdim > 0, "lia_mlstm_scan: bad shape nseg=%d H=%d dim=%d vdim=%d", nseg, H, dim, vdim);
+  if (act_f32) return dispatch_scan<float>(q, k, v, ld, gates, state_S, state_n, state_m, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  return dispatch_scan<bf16>(q, k, v, ld, gates, state_S, state_n, state_m, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+}
+
+// the same for a caller without a workspace
 extern "C" int lia_mlstm_scan(const void* q, const void* k, const void* v, int act_f32, int ld, const float* gates, float* state_S,
                               float* state_n, float* state_m, const int* segs, int nseg, int H, int dim, int vdim, float q_scale,
                               float den_eps, float* o, lia_stream_t stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-  LIA_CHECK_ARG(q && k && v && gates && state_S && state_n && state_m && segs && o, "lia_mlstm_scan: null pointer");
-  LIA_CHECK_ARG(nseg > 0 && nseg <= 65535 && H > 0 && H <= 65535 && dim > 0 && dim <= 512 && vdim > 0, "lia_mlstm_scan: bad shape nseg=%d H=%d dim=%d vdim=%d", nseg, H, dim, vdim);
-  if (act_f32) return dispatch_scan<float>(q, k, v, ld, gates, state_S, state_n, state_m, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
-  return dispatch_scan<bf16>(q, k, v, ld, gates, state_S, state_n, state_m, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  LIA_CHECK_ARG(nseg > 0 && nseg <= 65535 && H > 0 && H <= 65535 && dim > 0 && dim <= 512, "lia_mlstm_scan: bad shape nseg=%d H=%d dim=%d vdim=%d", nseg, H, dim, vdim);
+  float* ws = nullptr;
+  LIA_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&ws), (size_t)nseg * H * (dim + 1) * sizeof(float), stream));
+  const int rc = lia_mlstm_scan_ws(q, k, v, act_f32, ld, gates, state_S, state_n, state_m, segs, nseg, H, dim, vdim, q_scale, den_eps, o, ws, stream_);
+  LIA_CUDA(cudaFreeAsync(ws, stream));
+  return rc;
 }
 
 extern "C" int lia_headnorm_gate(const float* o, const float* w, const void* gate, int ldg, void* out, int act_f32, int M, int H, int vdim,

@@ -403,9 +403,11 @@ def mlstm_scan(q, k, v, gates, state_S, state_n, state_m, segs, H, dim, vdim, q_
     M = q.shape[0]
     if tuple(gates.shape) != (M, 2 * H) or tuple(o.shape) != (M, H * vdim) or tuple(state_S.shape[1:]) != (H, vdim, dim):
         raise _lib.LiaError("mlstm_scan: shapes do not agree")
-    check(_lib.load().lia_mlstm_scan(_p(q), _p(k), _p(v), _f32(q), ld, _p(gates), _p(state_S), _p(state_n), _p(state_m), _p(segs),
-                                     segs.shape[0], H, dim, vdim, float(q_scale), float(den_eps), _p(o), _stream()), "lia_mlstm_scan")
-    count_launches()
+    n = segs.shape[0]
+    ws = torch.empty(n * H * (dim + 1), dtype=F32, device=q.device)
+    check(_lib.load().lia_mlstm_scan_ws(_p(q), _p(k), _p(v), _f32(q), ld, _p(gates), _p(state_S), _p(state_n), _p(state_m), _p(segs),
+                                        n, H, dim, vdim, float(q_scale), float(den_eps), _p(o), _p(ws), _stream()), "lia_mlstm_scan_ws")
+    count_launches(2 if vdim > 16 else 1)
     return o
 
 
