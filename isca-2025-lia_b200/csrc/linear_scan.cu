@@ -1,5 +1,5 @@
 // Linear-attention recurrences with a matrix state per head, for prompts, portions of prompts and single decoded tokens
-// alike, and what prepares their inputs.
+// alike, and what prepares their inputs.  (DECAY with 128 dims in bf16, portions of 32 tokens and more: chunk_scan.cu.)
 //
 //   DECAY  (a fixed decay per head):     S_t = d_h S_{t-1} + k_t v_t^T                      o_t = S_t^T q_t
 //   DELTA  (gated delta rule):           S'  = g_t S_{t-1};  u_t = beta_t (v_t - S'^T k_t);  S_t = S' + k_t u_t^T;  o_t = S_t^T q_t
@@ -28,6 +28,7 @@
 //               read of B or C serves 16 cells, and the sums of several tokens meet in one round of exchanges.
 //   rglru_scan  (real-gated linear recurrent unit, one number per channel): S_t = a_t S_{t-1} + sqrt(1 - a_t^2) i_t u_t,  out_t = S_t gelu(y_t).
 //               128 tokens at a time: 32 half-warps fold 4 tokens each into one affine map, the maps are chained through shared memory.
+#include <limits.h>
 #include <math.h>
 
 #include "common.cuh"
@@ -206,7 +207,7 @@ constexpr int CB = CW * NW;      // columns per block
 template <typename T, int DR, int MODE, bool VL>
 __global__ void __launch_bounds__(NW * 32, 2) linear_scan_kernel(const T* __restrict__ q, const T* __restrict__ k, int ldqk, const T* __restrict__ v, int ldv,
                                                               int in_silu, const float* __restrict__ decay, const float* __restrict__ gates,
-                                                              float* __restrict__ St, const int* __restrict__ segs, int H, int G, int dim, int vdim,
+                                                              float* __restrict__ St, const int* __restrict__ segs, int below, int H, int G, int dim, int vdim,
                                                               float* __restrict__ o) {
   pdl_launch_dependents();
   pdl_wait();
@@ -220,6 +221,7 @@ __global__ void __launch_bounds__(NW * 32, 2) linear_scan_kernel(const T* __rest
   const int seg = blockIdx.z, h = blockIdx.y, colb = blockIdx.x * CB;
   const int hk = h / (H / G);
   const int slot = segs[4 * seg], row0 = segs[4 * seg + 2], len = segs[4 * seg + 3];
+  if (len >= below) return;                      // chunk_scan.cu has this portion
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col0 = colb + warp * CW;
 
@@ -395,12 +397,12 @@ __global__ void __launch_bounds__(NW * 32, 2) linear_scan_kernel(const T* __rest
 
 template <typename T, int DR, int MODE, bool VL>
 int launch_scan_mode(const void* q, const void* k, int ldqk, const void* v, int ldv, int in_silu, const float* decay, const float* gates, float* St,
-                     const int* segs, int nseg, int H, int G, int dim, int vdim, float* o, cudaStream_t stream) {
+                     const int* segs, int below, int nseg, int H, int G, int dim, int vdim, float* o, cudaStream_t stream) {
   const size_t smem = (size_t)2 * TB * (2 * DR * 32 + CB + 4) * sizeof(float);
   dim3 grid((vdim + CB - 1) / CB, H, nseg);
   if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(linear_scan_kernel<T, DR, MODE, VL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   lia_launch_after(linear_scan_kernel<T, DR, MODE, VL>, dim3(grid), dim3(NW * 32), smem, stream, reinterpret_cast<const T*>(q), reinterpret_cast<const T*>(k), ldqk,
-                                                                       reinterpret_cast<const T*>(v), ldv, in_silu, decay, gates, St, segs, H, G, dim, vdim, o);
+                                                                       reinterpret_cast<const T*>(v), ldv, in_silu, decay, gates, St, segs, below, H, G, dim, vdim, o);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -408,30 +410,30 @@ int launch_scan_mode(const void* q, const void* k, int ldqk, const void* v, int 
 // gates given: DELTA; decay given: DECAY; neither: FORGET
 template <typename T, int DR, bool VL>
 int launch_scan_as(const void* q, const void* k, int ldqk, const void* v, int ldv, int in_silu, const float* decay, const float* gates, float* St,
-                   const int* segs, int nseg, int H, int G, int dim, int vdim, float* o, cudaStream_t stream) {
-  if (gates != nullptr) return launch_scan_mode<T, DR, 1, VL>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, nseg, H, G, dim, vdim, o, stream);
-  if (decay != nullptr) return launch_scan_mode<T, DR, 0, VL>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, nseg, H, G, dim, vdim, o, stream);
-  return launch_scan_mode<T, DR, 2, VL>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, nseg, H, G, dim, vdim, o, stream);
+                   const int* segs, int below, int nseg, int H, int G, int dim, int vdim, float* o, cudaStream_t stream) {
+  if (gates != nullptr) return launch_scan_mode<T, DR, 1, VL>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, below, nseg, H, G, dim, vdim, o, stream);
+  if (decay != nullptr) return launch_scan_mode<T, DR, 0, VL>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, below, nseg, H, G, dim, vdim, o, stream);
+  return launch_scan_mode<T, DR, 2, VL>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, below, nseg, H, G, dim, vdim, o, stream);
 }
 
 template <typename T, int DR>
 int launch_scan(const void* q, const void* k, int ldqk, const void* v, int ldv, int in_silu, const float* decay, const float* gates, float* St,
-                const int* segs, int nseg, int H, int G, int dim, int vdim, float* o, cudaStream_t stream) {
+                const int* segs, int below, int nseg, int H, int G, int dim, int vdim, float* o, cudaStream_t stream) {
   constexpr int VEC = Vec128<T>::N;
   const bool aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) % 16 == 0) &&
                        ldqk % VEC == 0 && ldv % VEC == 0 && dim % VEC == 0 && vdim % VEC == 0;
-  if (aligned) return launch_scan_as<T, DR, true>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, nseg, H, G, dim, vdim, o, stream);
-  return launch_scan_as<T, DR, false>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, nseg, H, G, dim, vdim, o, stream);
+  if (aligned) return launch_scan_as<T, DR, true>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, below, nseg, H, G, dim, vdim, o, stream);
+  return launch_scan_as<T, DR, false>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, below, nseg, H, G, dim, vdim, o, stream);
 }
 
 template <typename T>
 int dispatch_scan(const void* q, const void* k, int ldqk, const void* v, int ldv, int in_silu, const float* decay, const float* gates, float* St,
-                  const int* segs, int nseg, int H, int G, int dim, int vdim, float* o, cudaStream_t stream) {
-  if (dim <= 32) return launch_scan<T, 1>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, nseg, H, G, dim, vdim, o, stream);
-  if (dim <= 64) return launch_scan<T, 2>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, nseg, H, G, dim, vdim, o, stream);
-  if (dim <= 128) return launch_scan<T, 4>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, nseg, H, G, dim, vdim, o, stream);
-  if (dim <= 256) return launch_scan<T, 8>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, nseg, H, G, dim, vdim, o, stream);
-  return launch_scan<T, 16>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, nseg, H, G, dim, vdim, o, stream);
+                  const int* segs, int below, int nseg, int H, int G, int dim, int vdim, float* o, cudaStream_t stream) {
+  if (dim <= 32) return launch_scan<T, 1>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, below, nseg, H, G, dim, vdim, o, stream);
+  if (dim <= 64) return launch_scan<T, 2>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, below, nseg, H, G, dim, vdim, o, stream);
+  if (dim <= 128) return launch_scan<T, 4>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, below, nseg, H, G, dim, vdim, o, stream);
+  if (dim <= 256) return launch_scan<T, 8>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, below, nseg, H, G, dim, vdim, o, stream);
+  return launch_scan<T, 16>(q, k, ldqk, v, ldv, in_silu, decay, gates, St, segs, below, nseg, H, G, dim, vdim, o, stream);
 }
 
 // ---------------------------------------------------------------------------------------------------- convolution of one column range
@@ -863,6 +865,12 @@ extern "C" int lia_conv_state_update(const void* y, int y_f32, int ld, int q_off
   return LIA_OK;
 }
 
+// the DECAY recurrence in bf16 over the portions of fewer than `below` tokens
+int decay_scan_tokens(const void* q, const void* k, int ldqk, const void* v, int ldv, const float* decay, float* St, const int* segs, int below, int nseg, int H, int G,
+                      int dim, int vdim, float* o, cudaStream_t stream) {
+  return dispatch_scan<bf16>(q, k, ldqk, v, ldv, 0, decay, nullptr, St, segs, below, nseg, H, G, dim, vdim, o, stream);
+}
+
 // gates == NULL: the DECAY recurrence with decay[H]; otherwise DELTA with gates[rows][2H] = beta | g.
 extern "C" int lia_linear_scan(const void* q, const void* k, int ldqk, const void* v, int ldv, int act_f32, int in_silu, const float* decay,
                                const float* gates, float* state_S, const int* segs, int nseg, int H, int G, int dim, int vdim, float* o,
@@ -871,8 +879,8 @@ extern "C" int lia_linear_scan(const void* q, const void* k, int ldqk, const voi
   LIA_CHECK_ARG(q && k && v && state_S && segs && o && (decay || gates), "lia_linear_scan: null pointer");
   LIA_CHECK_ARG(nseg > 0 && nseg <= 65535 && H > 0 && H <= 65535 && G > 0 && H % G == 0 && dim > 0 && dim <= 512 && vdim > 0,
                 "lia_linear_scan: bad shape nseg=%d H=%d G=%d dim=%d vdim=%d", nseg, H, G, dim, vdim);
-  if (act_f32) return dispatch_scan<float>(q, k, ldqk, v, ldv, in_silu, decay, gates, state_S, segs, nseg, H, G, dim, vdim, o, stream);
-  return dispatch_scan<bf16>(q, k, ldqk, v, ldv, in_silu, decay, gates, state_S, segs, nseg, H, G, dim, vdim, o, stream);
+  if (act_f32) return dispatch_scan<float>(q, k, ldqk, v, ldv, in_silu, decay, gates, state_S, segs, INT_MAX, nseg, H, G, dim, vdim, o, stream);
+  return dispatch_scan<bf16>(q, k, ldqk, v, ldv, in_silu, decay, gates, state_S, segs, INT_MAX, nseg, H, G, dim, vdim, o, stream);
 }
 
 extern "C" int lia_forget_gate_prep(const void* y, int y_f32, int ld, int q_off, int f_off, int v_off, const float* f_bias, const float* low,
@@ -896,7 +904,7 @@ extern "C" int lia_forget_scan(const float* q, const float* f, int ldqf, const f
   LIA_CHECK_ARG(q && f && v && state_S && segs && o, "lia_forget_scan: null pointer");
   LIA_CHECK_ARG(nseg > 0 && nseg <= 65535 && H > 0 && H <= 65535 && dim > 0 && dim <= 512 && vdim > 0,
                 "lia_forget_scan: bad shape nseg=%d H=%d dim=%d vdim=%d", nseg, H, dim, vdim);
-  return dispatch_scan<float>(q, f, ldqf, v, ldv, 0, nullptr, nullptr, state_S, segs, nseg, H, H, dim, vdim, o, stream);
+  return dispatch_scan<float>(q, f, ldqf, v, ldv, 0, nullptr, nullptr, state_S, segs, INT_MAX, nseg, H, H, dim, vdim, o, stream);
 }
 
 /* see lia_b200.h */

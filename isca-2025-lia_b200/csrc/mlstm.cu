@@ -1,5 +1,5 @@
 // Matrix-memory recurrence (mLSTM) with a running-maximum stabiliser, for prompts, portions of prompts and single decoded
-// tokens alike.  Per head, with log gates i_t, f_t (already capped / log-sigmoided by the gate projection's epilogue):
+// tokens alike (portions of 32 tokens and more in bf16, 128 or 256 dims: chunk_scan.cu).  Per head, with log gates i_t, f_t (already capped / log-sigmoided by the gate projection's epilogue):
 //     m_t = max(f_t + m_{t-1}, i_t)
 //     S_t = exp(f_t + m_{t-1} - m_t) S_{t-1} + exp(i_t - m_t) k_t v_t^T          (dim x vdim)
 //     n_t = exp(f_t + m_{t-1} - m_t) n_{t-1} + exp(i_t - m_t) k_t
@@ -15,10 +15,13 @@
 // 8 tokens are processed -- with 128-bit loads where the rows allow it: every block of a head re-reads that head's q and
 // k, and with one load instruction (and its address arithmetic) per number the fetch cost more issue slots than the
 // recurrence itself (2048 tokens, heads of 256 x 512: 1.24 -> 0.87 ms per layer).
+#include <limits.h>
 #include <math.h>
 
 #include "common.cuh"
 #include "rowvec.cuh"
+
+int mlstm_take_state(const float* ws, const int* segs, int nseg, float* nst, float* mst, int H, int dim, cudaStream_t stream);
 
 namespace {
 
@@ -83,7 +86,7 @@ constexpr int CB = CW * NW;      // columns per block
 template <typename T, int DR, bool VL>
 __global__ void __launch_bounds__(NW * 32, 2) mlstm_scan_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, int ld,
                                                              const float* __restrict__ gates, float* __restrict__ St, float* __restrict__ nst,
-                                                             float* __restrict__ mst, float* __restrict__ ws, const int* __restrict__ segs, int H, int dim, int vdim,
+                                                             float* __restrict__ mst, float* __restrict__ ws, const int* __restrict__ segs, int below, int H, int dim, int vdim,
                                                              float q_scale, float den_eps, float* __restrict__ o) {
   pdl_launch_dependents();
   pdl_wait();
@@ -95,6 +98,7 @@ __global__ void __launch_bounds__(NW * 32, 2) mlstm_scan_kernel(const T* __restr
   extern __shared__ __align__(16) float stage[]; // [2][TB][ROWF]
   const int seg = blockIdx.z, h = blockIdx.y, colb = blockIdx.x * CB;
   const int slot = segs[4 * seg], row0 = segs[4 * seg + 2], len = segs[4 * seg + 3];
+  if (len >= below) return;                      // chunk_scan.cu has this portion
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col0 = colb + warp * CW;
 
@@ -334,41 +338,52 @@ __global__ void __launch_bounds__(256) headnorm_gate_vec_kernel(const float* __r
 }
 
 template <typename T, int DR, bool VL>
-int launch_scan_as(const void* q, const void* k, const void* v, int ld, const float* gates, float* St, float* nst, float* mst, float* ws, const int* segs,
+int launch_scan_as(const void* q, const void* k, const void* v, int ld, const float* gates, float* St, float* nst, float* mst, float* ws, const int* segs, int below,
                 int nseg, int H, int dim, int vdim, float q_scale, float den_eps, float* o, cudaStream_t stream) {
   const size_t smem = (size_t)2 * TB * (2 * DR * 32 + CB + 4) * sizeof(float);
   if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(mlstm_scan_kernel<T, DR, VL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((vdim + CB - 1) / CB, H, nseg);
   if (grid.x == 1) ws = nullptr;
   lia_launch_after(mlstm_scan_kernel<T, DR, VL>, dim3(grid), dim3(NW * 32), smem, stream, reinterpret_cast<const T*>(q), reinterpret_cast<const T*>(k), reinterpret_cast<const T*>(v),
-                                                            ld, gates, St, nst, mst, ws, segs, H, dim, vdim, q_scale, den_eps, o);
+                                                            ld, gates, St, nst, mst, ws, segs, below, H, dim, vdim, q_scale, den_eps, o);
   LIA_LAUNCH_CHECK();
-  if (ws != nullptr) lia_launch(mlstm_state_kernel, dim3(H, nseg), dim3(128), 0, stream, (const float*)ws, segs, nst, mst, H, dim);
-  LIA_LAUNCH_CHECK();
-  return LIA_OK;
+  return ws ? mlstm_take_state(ws, segs, nseg, nst, mst, H, dim, stream) : LIA_OK;
 }
 
 template <typename T, int DR>
-int launch_scan(const void* q, const void* k, const void* v, int ld, const float* gates, float* St, float* nst, float* mst, float* ws, const int* segs,
+int launch_scan(const void* q, const void* k, const void* v, int ld, const float* gates, float* St, float* nst, float* mst, float* ws, const int* segs, int below,
                 int nseg, int H, int dim, int vdim, float q_scale, float den_eps, float* o, cudaStream_t stream) {
   constexpr int VEC = Vec128<T>::N;
   const bool aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) % 16 == 0) &&
                        ld % VEC == 0 && dim % VEC == 0 && vdim % VEC == 0;
-  if (aligned) return launch_scan_as<T, DR, true>(q, k, v, ld, gates, St, nst, mst, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
-  return launch_scan_as<T, DR, false>(q, k, v, ld, gates, St, nst, mst, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  if (aligned) return launch_scan_as<T, DR, true>(q, k, v, ld, gates, St, nst, mst, ws, segs, below, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  return launch_scan_as<T, DR, false>(q, k, v, ld, gates, St, nst, mst, ws, segs, below, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
 }
 
 template <typename T>
-int dispatch_scan(const void* q, const void* k, const void* v, int ld, const float* gates, float* St, float* nst, float* mst, float* ws, const int* segs,
+int dispatch_scan(const void* q, const void* k, const void* v, int ld, const float* gates, float* St, float* nst, float* mst, float* ws, const int* segs, int below,
                   int nseg, int H, int dim, int vdim, float q_scale, float den_eps, float* o, cudaStream_t stream) {
-  if (dim <= 32) return launch_scan<T, 1>(q, k, v, ld, gates, St, nst, mst, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
-  if (dim <= 64) return launch_scan<T, 2>(q, k, v, ld, gates, St, nst, mst, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
-  if (dim <= 128) return launch_scan<T, 4>(q, k, v, ld, gates, St, nst, mst, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
-  if (dim <= 256) return launch_scan<T, 8>(q, k, v, ld, gates, St, nst, mst, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
-  return launch_scan<T, 16>(q, k, v, ld, gates, St, nst, mst, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  if (dim <= 32) return launch_scan<T, 1>(q, k, v, ld, gates, St, nst, mst, ws, segs, below, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  if (dim <= 64) return launch_scan<T, 2>(q, k, v, ld, gates, St, nst, mst, ws, segs, below, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  if (dim <= 128) return launch_scan<T, 4>(q, k, v, ld, gates, St, nst, mst, ws, segs, below, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  if (dim <= 256) return launch_scan<T, 8>(q, k, v, ld, gates, St, nst, mst, ws, segs, below, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  return launch_scan<T, 16>(q, k, v, ld, gates, St, nst, mst, ws, segs, below, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
 }
 
 }  // namespace
+
+// the state takes the n and m that a scan left in its workspace
+int mlstm_take_state(const float* ws, const int* segs, int nseg, float* nst, float* mst, int H, int dim, cudaStream_t stream) {
+  lia_launch(mlstm_state_kernel, dim3(H, nseg), dim3(128), 0, stream, ws, segs, nst, mst, H, dim);
+  LIA_LAUNCH_CHECK();
+  return LIA_OK;
+}
+
+// bf16, the portions of fewer than `below` tokens; the state then takes every portion's n and m from the workspace
+int mlstm_scan_tokens(const void* q, const void* k, const void* v, int ld, const float* gates, float* St, float* nst, float* mst, float* ws, const int* segs, int below,
+                      int nseg, int H, int dim, int vdim, float q_scale, float den_eps, float* o, cudaStream_t stream) {
+  return dispatch_scan<bf16>(q, k, v, ld, gates, St, nst, mst, ws, segs, below, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+}
 
 extern "C" int lia_mlstm_scan_ws(const void* q, const void* k, const void* v, int act_f32, int ld, const float* gates, float* state_S,
                                  float* state_n, float* state_m, const int* segs, int nseg, int H, int dim, int vdim, float q_scale,
@@ -376,8 +391,8 @@ extern "C" int lia_mlstm_scan_ws(const void* q, const void* k, const void* v, in
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LIA_CHECK_ARG(q && k && v && gates && state_S && state_n && state_m && segs && o && ws, "lia_mlstm_scan: null pointer");
   LIA_CHECK_ARG(nseg > 0 && nseg <= 65535 && H > 0 && H <= 65535 && dim > 0 && dim <= 512 && vdim > 0, "lia_mlstm_scan: bad shape nseg=%d H=%d dim=%d vdim=%d", nseg, H, dim, vdim);
-  if (act_f32) return dispatch_scan<float>(q, k, v, ld, gates, state_S, state_n, state_m, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
-  return dispatch_scan<bf16>(q, k, v, ld, gates, state_S, state_n, state_m, ws, segs, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  if (act_f32) return dispatch_scan<float>(q, k, v, ld, gates, state_S, state_n, state_m, ws, segs, INT_MAX, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  return dispatch_scan<bf16>(q, k, v, ld, gates, state_S, state_n, state_m, ws, segs, INT_MAX, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
 }
 
 // the same for a caller without a workspace

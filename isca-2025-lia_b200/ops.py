@@ -392,9 +392,21 @@ def argmax_f32(logits, suppress_id=-1, out=None):
     return out
 
 
-def mlstm_scan(q, k, v, gates, state_S, state_n, state_m, segs, H, dim, vdim, q_scale, den_eps, o):
-    """Matrix-memory recurrence over every portion of the step (csrc/mlstm.cu).  q, k, v: column slices of one projection
-    output (same row stride); gates [rows, 2H] fp32 (log input, log forget); state tensors indexed by slot."""
+def _in_chunks(mlstm, q, k, v, ld, ldv, dim, vdim, state_S, o, n, lengths):
+    """Whether portions of a matrix-state recurrence are long enough for the form in chunks of tokens on the tensor cores (csrc/chunk_scan.cu), and it takes them;
+    and whether there are short ones as well.  A portion's own length decides how it is computed, whatever comes with it."""
+    if q.dtype != BF16:
+        return False, False
+    lib, M = _lib.load(), q.shape[0]
+    shortest, longest = lengths or (M if n == 1 else 1, M - n + 1)
+    fewest = lib.lia_chunk_scan_rows()
+    return (longest >= fewest and bool(lib.lia_chunk_scan_takes(mlstm, dim, vdim)) and ld % 8 == 0 and ldv % 8 == 0
+            and (q.data_ptr() | k.data_ptr() | v.data_ptr() | o.data_ptr()) % 16 == 0 and state_S.data_ptr() % 8 == 0), shortest < fewest
+
+
+def mlstm_scan(q, k, v, gates, state_S, state_n, state_m, segs, H, dim, vdim, q_scale, den_eps, o, lengths=None):
+    """Matrix-memory recurrence over every portion of the step (csrc/mlstm.cu; long portions csrc/chunk_scan.cu).  ``lengths``: tokens of the
+    shortest and of the longest portion, if known.  q, k, v: column slices of one projection output (same row stride); gates [rows, 2H] fp32 (log input, log forget); state tensors indexed by slot."""
     ld = _rowmajor(q, "q")
     if _rowmajor(k, "k") != ld or _rowmajor(v, "v") != ld or k.dtype != q.dtype or v.dtype != q.dtype:
         raise _lib.LiaError("mlstm_scan: q, k, v must be slices of one buffer")
@@ -405,6 +417,12 @@ def mlstm_scan(q, k, v, gates, state_S, state_n, state_m, segs, H, dim, vdim, q_
         raise _lib.LiaError("mlstm_scan: shapes do not agree")
     n = segs.shape[0]
     ws = torch.empty(n * H * (dim + 1), dtype=F32, device=q.device)
+    chunks, mixed = _in_chunks(1, q, k, v, ld, ld, dim, vdim, state_S, o, n, lengths)
+    if chunks:
+        check(_lib.load().lia_mlstm_scan_chunks(_p(q), _p(k), _p(v), ld, _p(gates), _p(state_S), _p(state_n), _p(state_m), _p(segs), n, int(mixed), H, dim, vdim,
+                                                float(q_scale), float(den_eps), _p(o), _p(ws), _stream()), "lia_mlstm_scan_chunks")
+        count_launches((2 if vdim > 16 else 1) + mixed)
+        return o
     check(_lib.load().lia_mlstm_scan_ws(_p(q), _p(k), _p(v), _f32(q), ld, _p(gates), _p(state_S), _p(state_n), _p(state_m), _p(segs),
                                         n, H, dim, vdim, float(q_scale), float(den_eps), _p(o), _p(ws), _stream()), "lia_mlstm_scan_ws")
     count_launches(2 if vdim > 16 else 1)
@@ -745,9 +763,10 @@ def conv_state_update(y, offs, nqk, nv, conv_state, segs, taps, nk=None):
         count_launches()
 
 
-def linear_scan(q, k, v, state_S, segs, H, G, dim, vdim, o, decay=None, gates=None, in_silu=False):
-    """Matrix-state recurrence over every portion of the step (csrc/linear_scan.cu): with ``decay`` [H] the fixed-decay form,
-    with ``gates`` [rows, 2H] = beta | g the gated delta rule.  q, k: column slices with one row stride, G heads."""
+def linear_scan(q, k, v, state_S, segs, H, G, dim, vdim, o, decay=None, gates=None, in_silu=False, lengths=None):
+    """Matrix-state recurrence over every portion of the step (csrc/linear_scan.cu; long portions with a fixed decay csrc/chunk_scan.cu): with ``decay`` [H] the fixed-decay form,
+    with ``gates`` [rows, 2H] = beta | g the gated delta rule.  q, k: column slices with one row stride, G heads.
+    ``lengths``: tokens of the shortest and of the longest portion, if known."""
     ld = _rowmajor(q, "q")
     if _rowmajor(k, "k") != ld or k.dtype != q.dtype or v.dtype != q.dtype:
         raise _lib.LiaError("linear_scan: q and k must be slices of one buffer, v of the same type")
@@ -759,6 +778,13 @@ def linear_scan(q, k, v, state_S, segs, H, G, dim, vdim, o, decay=None, gates=No
     if tuple(o.shape) != (M, H * vdim) or tuple(state_S.shape[1:]) != (H, vdim, dim) or (gates is not None and tuple(gates.shape) != (M, 2 * H)) \
             or (decay is not None and decay.numel() != H):
         raise _lib.LiaError("linear_scan: shapes do not agree")
+    n = segs.shape[0]
+    chunks, mixed = _in_chunks(0, q, k, v, ld, ldv, dim, vdim, state_S, o, n, lengths) if decay is not None and not in_silu else (False, False)
+    if chunks:
+        check(_lib.load().lia_decay_scan_chunks(_p(q), _p(k), ld, _p(v), ldv, _p(_req(decay, "decay", F32)), _p(state_S), _p(segs), n, int(mixed), H, G, dim, vdim, _p(o),
+                                                _stream()), "lia_decay_scan_chunks")
+        count_launches(1 + mixed)
+        return o
     check(_lib.load().lia_linear_scan(_p(q), _p(k), ld, _p(v), ldv, _f32(q), int(in_silu), _p(_req(decay, "decay", F32) if decay is not None else None),
                                       _p(_req(gates, "gates", F32) if gates is not None else None), _p(state_S), _p(segs), segs.shape[0], H, G, dim,
                                       vdim, _p(o), _stream()), "lia_linear_scan")

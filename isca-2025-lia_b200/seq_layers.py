@@ -35,6 +35,8 @@ class StepBatch:
 
     def __init__(self, rows, segs, meta, max_ctx=0, portions=None):
         self.rows, self.segs, self.meta, self.portions = rows, segs, meta, portions
+        lens = [n for _, _, _, n in portions] if portions else None
+        self.lengths = (min(lens), max(lens)) if lens else None      # of the shortest and the longest portion, if known
         self.max_ctx = max_ctx              # longest history (tokens cached after this step) among the step's sequences
         self.scratch = {}                   # what one layer of this step leaves for later layers (per-token tensors)
 
@@ -110,7 +112,7 @@ class MLSTMMixer:
         gates = torch.empty(M, 2 * H, dtype=F32, device=h.device)
         ops.linear_small(h, self.w_gates, self.b_gates, gates, ops.GATE_LOG_INPUT_FORGET, self.cap)
         o = torch.empty(M, H * self.vdim, dtype=F32, device=h.device)
-        ops.mlstm_scan(q, k, v, gates, S, n, m, batch.segs, H, self.dim, self.vdim, self.q_scale, self.den_eps, o)
+        ops.mlstm_scan(q, k, v, gates, S, n, m, batch.segs, H, self.dim, self.vdim, self.q_scale, self.den_eps, o, lengths=batch.lengths)
         on = torch.empty(M, H * self.vdim, dtype=self.dtype, device=h.device)
         ops.headnorm_gate(o, self.norm_w, g, on, H, self.vdim, self.eps)
         return self.out(on)
@@ -334,7 +336,7 @@ class DecayLinearAttentionMixer:
         ops.gated_act(y, F_, act, ops.ACT_SILU)
         q, k, v = act[:, offs[0]:offs[0] + H * self.dim], act[:, offs[1]:offs[1] + H * self.dim], act[:, offs[2]:offs[2] + H * self.vdim]
         o = torch.empty(M, H * self.vdim, dtype=F32, device=h.device)
-        ops.linear_scan(q, k, v, S, batch.segs, H, H, self.dim, self.vdim, o, decay=self.decay)
+        ops.linear_scan(q, k, v, S, batch.segs, H, H, self.dim, self.vdim, o, decay=self.decay, lengths=batch.lengths)
         on = torch.empty(M, H * self.vdim, dtype=self.dtype, device=h.device)
         ops.headnorm_gate(o, self.norm_w, g, on, 1, H * self.vdim, self.eps)       # one norm over all heads
         return self.out(on)
