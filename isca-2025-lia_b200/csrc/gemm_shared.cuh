@@ -719,6 +719,17 @@ Plan make_plan(int M, int N, int K, bool allow_pair = false) {
     long long g = total / 4;
     if (g < 1) g = 1;
     if (g > sms) g = sms;
+    // Small weights: handing partial sums over costs more than idle SMs do, and the more the more rows there are.  Up to 16 k-blocks a CTA takes a whole tile;
+    // else every tile is cut into the same 2 to 6 parts, if that occupies 5/8 of the SMs and leaves 5 to 32 k-blocks each: no CTA then works on two tiles, and
+    // 90 to 120 CTAs did better than all 148.  The line depends on the weights alone, so that a row's sums do not depend on the rows beside it.  1 / 16 /
+    // 128 rows in us, spans -> tiles or parts: 5632 x 1024 7.3 / 7.6 / 21 -> 5.8 / 6.1 / 12; 2560 x 2560 8.0 / 8.5 / 30 -> 6.5 / 7.6 / 23; 2048 x 5632
+    // 9.3 / 9.9 / 34 -> 8.2 / 8.9 / 26; 6144 x 4096 12.5 / 12.9 / 26 -> 12.3 / 12.5 / 23; worst of 35 shapes 1024 x 1024 5.4 / 6.3 / 17 -> 5.7 / 6.0 / 11.  Beyond
+    // the lines the chip's bandwidth decides: 4096 x 16384 24 us by spans, 25 in 4 parts; 12288 x 4096 18.7 and 19.3.
+    if (allow_pair) {
+      const int most = (sms * 13 / 16) / pl.tiles_a, parts = most < 6 ? most : 6;
+      if (pl.k_blocks <= 16 && pl.tiles_a <= sms) g = pl.tiles_a;
+      else if (parts >= 2 && (parts == 6 || pl.tiles_a * parts * 8 >= sms * 5) && pl.k_blocks >= 5 * parts && pl.k_blocks <= 32 * parts) g = (long long)pl.tiles_a * parts;
+    }
     pl.grid = (int)g;
     pl.streamk = (total % pl.grid != 0 || pl.tiles_a % pl.grid != 0) ? 1 : 0;
     const char* env = getenv("LIA_STREAMK");   // tuning/debug override: 0 = whole tiles per CTA

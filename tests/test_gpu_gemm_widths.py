@@ -42,3 +42,14 @@ def test_qkv_scatter(monkeypatch):
     for other in got[1:]:
         assert all(torch.equal(x, y) for x, y in zip(got[0], other))
     assert bool((got[0][1][0] == 0).all()) and bool((got[0][1][1] != 0).any())
+
+
+@pytest.mark.parametrize("N,K", [(8, 64), (136, 1024), (1024, 1032), (512, 1920), (2176, 1920), (2176, 1912), (2560, 2560), (7552, 640), (7560, 1280), (1024, 12288), (1024, 12296)])
+def test_few_rows_at_the_lines_between_tiles_parts_and_spans(N, K):
+    """Whole tiles, equal parts of tiles and spans: a row's result is right and does not depend on the rows beside it."""
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    a, w = torch.randn(100, K, generator=g, device="cuda").to(BF16), (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(BF16)
+    y = ops.gemm(a, w, None)
+    assert float((y.float() - a.float() @ w.float().T).abs().max()) < 0.035            # sums of size up to 5, rounded once to bf16
+    for M in (1, 16, 17, 33, 65):
+        assert torch.equal(ops.gemm(a[:M].contiguous(), w, None), y[:M])
