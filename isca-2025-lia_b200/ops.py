@@ -5,6 +5,7 @@ call into libliab200.so on ``torch.cuda.current_stream()``.  No op has a PyTorch
 fallback -- a missing library or a non-CUDA tensor raises.
 """
 import ctypes
+import functools
 import os
 
 import torch
@@ -392,21 +393,26 @@ def argmax_f32(logits, suppress_id=-1, out=None):
     return out
 
 
+@functools.lru_cache(maxsize=256)
+def _chunk_rows(mlstm, dim, vdim):
+    lib = _lib.load()
+    return lib.lia_chunk_scan_rows() if lib.lia_chunk_scan_takes(mlstm, dim, vdim) else 0
+
+
 def _in_chunks(mlstm, q, k, v, ld, ldv, dim, vdim, state_S, o, n, lengths):
     """Whether portions of a matrix-state recurrence are long enough for the form in chunks of tokens on the tensor cores (csrc/chunk_scan.cu), and it takes them;
     and whether there are short ones as well.  A portion's own length decides how it is computed, whatever comes with it."""
-    if q.dtype != BF16:
-        return False, False
-    lib, M = _lib.load(), q.shape[0]
+    fewest, M = _chunk_rows(mlstm, dim, vdim), q.shape[0]
     shortest, longest = lengths or (M if n == 1 else 1, M - n + 1)
-    fewest = lib.lia_chunk_scan_rows()
-    return (longest >= fewest and bool(lib.lia_chunk_scan_takes(mlstm, dim, vdim)) and ld % 8 == 0 and ldv % 8 == 0
-            and (q.data_ptr() | k.data_ptr() | v.data_ptr() | o.data_ptr()) % 16 == 0 and state_S.data_ptr() % 8 == 0), shortest < fewest
+    if q.dtype != BF16 or not fewest or longest < fewest:
+        return False, False
+    return (ld % 8 == 0 and ldv % 8 == 0 and (q.data_ptr() | k.data_ptr() | v.data_ptr() | o.data_ptr()) % 16 == 0 and state_S.data_ptr() % 8 == 0), shortest < fewest
 
 
 def mlstm_scan(q, k, v, gates, state_S, state_n, state_m, segs, H, dim, vdim, q_scale, den_eps, o, lengths=None):
     """Matrix-memory recurrence over every portion of the step (csrc/mlstm.cu; long portions csrc/chunk_scan.cu).  ``lengths``: tokens of the
-    shortest and of the longest portion, if known.  q, k, v: column slices of one projection output (same row stride); gates [rows, 2H] fp32 (log input, log forget); state tensors indexed by slot."""
+    shortest and of the longest portion, if known.  q, k, v: column slices of one projection output (same row
+    stride); gates [rows, 2H] fp32 (log input, log forget); state tensors indexed by slot."""
     ld = _rowmajor(q, "q")
     if _rowmajor(k, "k") != ld or _rowmajor(v, "v") != ld or k.dtype != q.dtype or v.dtype != q.dtype:
         raise _lib.LiaError("mlstm_scan: q, k, v must be slices of one buffer")

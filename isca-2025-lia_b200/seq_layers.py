@@ -798,8 +798,10 @@ class MoEFeedForward:
     grouped by expert on the device (no host round trip) and each projection runs as one grouped launch; a handful of pairs
     (decoding) take the form with one warp per output instead.  The result is fp32."""
 
-    # Up to max(16, experts) pairs, FEW_PAIRS at most: one warp per output, whose weight reads grow with the pairs; above (bf16, sizes that are
-    # multiples of 8): tensor cores, which read every chosen expert once.  16 experts, width 4096: 16 pairs 266 | 270 us, 40 pairs 541 | 276 us.
+    # Up to FEW_PAIRS pairs, and where these are more than max(16, experts) only if their weights are FEW_BYTES at most: one warp per output, whose weight reads grow
+    # with the pairs; above (bf16, sizes that are multiples of 8): tensor cores, which read every chosen expert once but take more launches.  16 experts,
+    # width 4096: 16 pairs 266 | 270 us, 40 pairs 541 | 276 us; width 1024, 18 pairs (78 MB): 75 | 107 us.
+    FEW_BYTES = 400 << 20
     FEW_PAIRS = 48
     TENSOR_CORE_PAIRS = 512   # from here the experts' outputs are rounded to bf16 before they are weighted and added
 
@@ -831,6 +833,7 @@ class MoEFeedForward:
         self.w_down = torch.stack([e["down"] for e in experts_w]).to(device=device, dtype=dtype).contiguous()     # [E, W, ff]
         self.shared = shared
         W = self.w_up.shape[2]
+        self.expert_bytes = (self.w_up[0].numel() + self.w_down[0].numel()) * self.w_up.element_size()
         self.tensor_core = dtype == BF16 and W % 8 == 0 and ff % 8 == 0 and os.environ.get("LIA_PLAIN_LINEAR", "0") == "0"
 
     def _experts_tensor_core(self, h, idx, wt, y, shared_gate):
@@ -875,7 +878,8 @@ class MoEFeedForward:
         identity = (idx, self.E, h, wt) if self.identity else None
         pairs = M * top
         y = torch.empty(M, W, dtype=F32, device=dev)
-        if self.tensor_core and pairs > min(self.FEW_PAIRS, max(16, self.E)) and h.is_contiguous() and h.dtype == BF16 and h.data_ptr() % 16 == 0:
+        few = pairs <= self.FEW_PAIRS and (pairs <= max(16, self.E) or pairs * self.expert_bytes <= self.FEW_BYTES)
+        if self.tensor_core and not few and h.is_contiguous() and h.dtype == BF16 and h.data_ptr() % 16 == 0:
             return self._experts_tensor_core(h, idx, wt, y, shared_gate)
         ypair = torch.empty(pairs, W, dtype=F32, device=dev)
         if pairs <= self.FEW_PAIRS:
