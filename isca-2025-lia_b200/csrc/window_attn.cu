@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(128) window_combine_kernel(const float* __rest
   float l = 0.f;
   for (int z = 0; z < nsplit; ++z) {
     const float2 ml = part_ml[rh * nsplit + z];
-    if (ml.y > 0.f) l += ml.y * expf(ml.x - m);
+    if (ml.y != 0.f) l += ml.y * expf(ml.x - m);          // a NaN score makes its part's sum NaN, and so the row
   }
   if (x.sink) l += expf(x.sink[h] - m);
   const float invl = 1.0f / l;
@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(128) window_combine_kernel(const float* __rest
     float s = 0.f;
     for (int z = 0; z < nsplit; ++z) {
       const float2 ml = part_ml[rh * nsplit + z];
-      if (ml.y > 0.f) s = fmaf(part[(rh * nsplit + z) * vdim + c], expf(ml.x - m), s);
+      if (ml.y != 0.f) s = fmaf(part[(rh * nsplit + z) * vdim + c], expf(ml.x - m), s);
     }
     store_out(out, rh * vdim + c, s * invl * gate_of<T>(x, a, row, h, c), a);
   }

@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(128) window_decode_kernel(const void* __restri
     for (int w = 0; w < 4; ++w) m = fmaxf(m, ml[w][hh].x);
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-      if (ml[w][hh].y > 0.f) {
+      if (ml[w][hh].y != 0.f) {                          // 0: the warp saw no key; a NaN is kept
         const float f = expf(ml[w][hh].x - m);
         l = fmaf(ml[w][hh].y, f, l);
         o = fmaf(sums[(w * 8 + hh) * DV + ch], f, o);
