@@ -15,6 +15,8 @@
 //            34 us (3.7 TB/s).
 // The tensor cores cut sums off below the 24th bit instead of rounding them.  Sums over one stage are therefore made apart and added to the
 // running ones in fp32: the error against 64 bits is 0.4 to 0.8 times that of the FMA chains (one running sum over 1700 keys: 5 times).
+// Numbers that are not finite do not survive this: a masked key of the stage has weight 0 and still meets its value, and a part of a split weight is 0 or has
+// the other sign.  Sums that are not finite stay so to the end, so it is there that such rows are found and formed again key by key (plain_row).
 #include "mma.cuh"
 #include "window_attn.cuh"
 
@@ -66,6 +68,48 @@ template <int D, int BK> __device__ __forceinline__ void load_tile(uint32_t dst,
     const bool in = j0 + j <= last;
     cp_async16(at_chunk<CH>(dst, j, c), rows + (size_t)(in ? j0 + j : last) * stride + c * 8, in ? 16 : 0);
   }
+}
+
+// One row and head over the keys [lo, hi] of its sequence, all of which it sees, by one warp on the CUDA cores: lane j scores every 32nd key, lane l owns the
+// value columns l, l + 32, ...  For the rows whose sums were not finite, so it is never worth being fast.
+template <int DV> struct PlainRow {
+  float m, l, o[DV / 32];
+};
+template <int DK, int DV, int NQ>
+__device__ __noinline__ PlainRow<DV> plain_row(const void* q, size_t q_at, const bf16* kc, size_t k_stride, const bf16* vc, size_t v_stride, int lo, int hi, int pos, float mul,
+                                               float slope, float softcap) {
+  const int lane = threadIdx.x & 31;
+  PlainRow<DV> y;
+  y.m = -INFINITY;
+  y.l = 0.f;
+#pragma unroll
+  for (int c = 0; c < DV / 32; ++c) y.o[c] = 0.f;
+  for (int j0 = lo; j0 <= hi; j0 += 32) {
+    const int nk = min(32, hi + 1 - j0);
+    float s = 0.f;
+    if (lane < nk) {
+      for (int d = 0; d < DK; ++d) {
+        const float x = NQ == 1 ? __bfloat162float(reinterpret_cast<const bf16*>(q)[q_at + d]) : reinterpret_cast<const float*>(q)[q_at + d];
+        s = fmaf(x, __bfloat162float(kc[(size_t)(j0 + lane) * k_stride + d]), s);
+      }
+      s *= mul;
+      if (softcap > 0.f) s = softcap * tanhf(s / softcap);
+      if (slope != 0.f) s -= slope * (float)(pos - j0 - lane);
+    } else {
+      s = -INFINITY;
+    }
+    const float m = fmaxf(y.m, warp_max(s)), base = m == -INFINITY ? 0.f : m, p = expf(s - base), al = expf(y.m - base);
+    y.m = m;
+    y.l = fmaf(y.l, al, warp_sum(p));
+#pragma unroll
+    for (int c = 0; c < DV / 32; ++c) y.o[c] *= al;
+    for (int j = 0; j < nk; ++j) {
+      const float w = __shfl_sync(0xffffffffu, p, j);
+#pragma unroll
+      for (int c = 0; c < DV / 32; ++c) y.o[c] = fmaf(w, __bfloat162float(vc[(size_t)(j0 + j) * v_stride + lane + 32 * c]), y.o[c]);
+    }
+  }
+  return y;
 }
 
 template <int DK, int DV, int NQ> struct PromptShape {
@@ -258,12 +302,17 @@ __global__ void __launch_bounds__(128, (DV <= 128 && NQ == 1) ? 3 : 2) window_pr
     __syncthreads();                                     // the stage may be overwritten
   }
 
+  unsigned again[2];                                     // lanes whose row's sums are not finite
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     l_run[u] += __shfl_xor_sync(0xffffffffu, l_run[u], 1);
     l_run[u] += __shfl_xor_sync(0xffffffffu, l_run[u], 2);
     const int r = warp * 16 + g + u * 8;
-    if (r >= rows) continue;
+    float probe = 0.f;                                   // NaN if a sum is not finite
+#pragma unroll
+    for (int n = 0; n < DV / 8; ++n) probe = fmaf(O[n][2 * u], 0.f, fmaf(O[n][2 * u + 1], 0.f, probe));
+    again[u] = __ballot_sync(0xffffffffu, r < rows && probe != 0.f);
+    if (r >= rows || ((again[u] >> (4 * g)) & 15u)) continue;
     const float invl = 1.0f / (l_run[u] + (x.sink ? expf(x.sink[h] - m_run[u]) : 0.f));
     const size_t row = row0 + r, at = (row * a.H + h) * DV;
 #pragma unroll
@@ -272,6 +321,18 @@ __global__ void __launch_bounds__(128, (DV <= 128 && NQ == 1) ? 3 : 2) window_pr
       const float y0 = O[n][2 * u] * invl * gate_of<bf16>(x, a, row, h, ch), y1 = O[n][2 * u + 1] * invl * gate_of<bf16>(x, a, row, h, ch + 1);
       if (a.out_f32) *reinterpret_cast<float2*>(reinterpret_cast<float*>(out) + at + ch) = make_float2(y0, y1);
       else *reinterpret_cast<uint32_t*>(out + at + ch) = pack_bf16x2(y0, y1);
+    }
+  }  if ((again[0] | again[1]) == 0u) return;
+#pragma unroll 1
+  for (int i = 0; i < 16; ++i) {
+    if ((((i < 8 ? again[0] : again[1]) >> (4 * (i & 7))) & 15u) == 0u) continue;
+    const size_t row = row0 + warp * 16 + i;
+    const PlainRow<DV> y = plain_row<DK, DV, NQ>(q, row * ldq + (size_t)h * DK, kc, k_stride, vc, v_stride, first_key(a, wpos + i), wpos + i, wpos + i, mul, slope, a.softcap);
+    const float invl = 1.0f / (y.l + (x.sink ? expf(x.sink[h] - y.m) : 0.f));
+#pragma unroll
+    for (int c = 0; c < DV / 32; ++c) {
+      const int ch = (int)(threadIdx.x & 31) + 32 * c;
+      store_out(out, (row * a.H + h) * DV + ch, y.o[c] * invl * gate_of<bf16>(x, a, row, h, ch), a);
     }
   }
 }
@@ -429,7 +490,27 @@ __global__ void __launch_bounds__(128) window_decode_kernel(const void* __restri
       dst[0] = make_float4(O[s * 8][i], O[s * 8 + 1][i], O[s * 8 + 2][i], O[s * 8 + 3][i]);
       dst[1] = make_float4(O[s * 8 + 4][i], O[s * 8 + 5][i], O[s * 8 + 6][i], O[s * 8 + 7][i]);
     }
-  __syncthreads();
+  float probe = 0.f;                                     // NaN if a sum is not finite
+#pragma unroll
+  for (int n = 0; n < VU * 8; ++n) probe = fmaf(O[n][0], 0.f, fmaf(O[n][1], 0.f, probe));
+  if (__syncthreads_or(probe != 0.f)) {                  // the whole range again, a head per warp
+#pragma unroll 1
+    for (int hh = warp; hh < a.HB; hh += 4) {
+      const int hq = h0 + hh;
+      const PlainRow<DV> y = plain_row<DK, DV, NQ>(q, (size_t)row * ldq + (size_t)hq * DK, kc, k_stride, vc, v_stride, lo + z * per * 16, min(pos, lo + t_end * 16 - 1), pos,
+                                                   a.scale * (x.temp ? x.temp[hq] : 1.0f), x.slopes ? x.slopes[hq] : 0.f, a.softcap);
+      const size_t rh = (size_t)row * a.H + hq;
+      const float invl = 1.0f / (y.l + (x.sink ? expf(x.sink[hq] - y.m) : 0.f));
+#pragma unroll
+      for (int c = 0; c < DV / 32; ++c) {
+        const int ch = lane + 32 * c;
+        if (a.nsplit == 1) store_out(out, rh * DV + ch, y.o[c] * invl * gate_of<bf16>(x, a, row, hq, ch), a);
+        else part[(rh * a.nsplit + z) * DV + ch] = y.o[c];
+      }
+      if (a.nsplit > 1 && lane == 0) part_ml[rh * a.nsplit + z] = make_float2(y.m, y.l);
+    }
+    return;
+  }
   for (int e = threadIdx.x; e < a.HB * DV; e += 128) {
     const int hh = e / DV, ch = e - hh * DV;
     float m = -INFINITY, l = 0.f, o = 0.f;
