@@ -9,6 +9,7 @@
 // are fetched in turn (the next keys while the values are taken in, the next values while the scores are made), so one stage of 52 KB
 // is enough and two blocks share an SM.  Bound: tensor cores and shared-memory reads about equally.  2048 tokens, 16 heads of 128 + 64 on latents
 // of 512: 4794 us in the latent space on the CUDA cores and 439 us for its two projections -> 329 and 67 us for the expansion.
+// Rows whose sums are not finite are formed again key by key at the end, as in window_attn_mma.cu: a masked key's weight of 0 still meets its value.
 #include <math.h>
 
 #include "mma.cuh"
@@ -42,6 +43,43 @@ struct ExpandedArgs {
   float scale;
   Portion p[MAX_PORTIONS];
 };
+
+// One row and head over the latents [lo, hi] by one warp on the CUDA cores: lane j scores every 32nd key, lane l owns the value columns l, l + 32, ...
+template <int DN> struct PlainRow {
+  float m, l, o[DN / 32];
+};
+template <int DN, int DR>
+__device__ __noinline__ PlainRow<DN> plain_row(const bf16* q, const float* qr, const bf16* keys, const bf16* vals, size_t stride, const bf16* key_rot, long long rot_stride, int lo,
+                                               int hi, float scale) {
+  const int lane = threadIdx.x & 31;
+  auto whole = [](const bf16* p) { return __bfloat162float(p[0]) + (__bfloat162float(p[DN]) + __bfloat162float(p[2 * DN])); };
+  PlainRow<DN> y;
+  y.m = -INFINITY;
+  y.l = 0.f;
+#pragma unroll
+  for (int c = 0; c < DN / 32; ++c) y.o[c] = 0.f;
+  for (int j0 = lo; j0 <= hi; j0 += 32) {
+    const int nk = min(32, hi + 1 - j0);
+    float s = -INFINITY;
+    if (lane < nk) {
+      s = 0.f;
+      for (int d = 0; d < DN; ++d) s = fmaf(__bfloat162float(q[d]), whole(keys + (size_t)(j0 + lane) * stride + d), s);
+      for (int d = 0; d < DR; ++d) s = fmaf(qr[d], __bfloat162float(key_rot[(size_t)(j0 + lane) * rot_stride + d]), s);
+      s *= scale;
+    }
+    const float m = fmaxf(y.m, warp_max(s)), base = m == -INFINITY ? 0.f : m, p = expf(s - base), al = expf(y.m - base);
+    y.m = m;
+    y.l = fmaf(y.l, al, warp_sum(p));
+#pragma unroll
+    for (int c = 0; c < DN / 32; ++c) y.o[c] *= al;
+    for (int j = 0; j < nk; ++j) {
+      const float w = __shfl_sync(0xffffffffu, p, j);
+#pragma unroll
+      for (int c = 0; c < DN / 32; ++c) y.o[c] = fmaf(w, whole(vals + (size_t)(j0 + j) * stride + lane + 32 * c), y.o[c]);
+    }
+  }
+  return y;
+}
 
 template <int DN, int DR> constexpr int expanded_smem() { return (BM * DN + 3 * BM * DR + 2 * 3 * BK * DN + BK * DR) * 2; }
 
@@ -241,26 +279,47 @@ __global__ void __launch_bounds__(128, 2) latent_expanded_kernel(const __grid_co
     cp_async_commit();
   }
 
+  // gate over the softmax's denominator, the sink among its terms: everything relative to the larger of maximum and sink
+  auto factor = [&](size_t row, float m, float l) {
+    const float f = a.gate ? a.gate[row * a.H + h] : 1.0f;
+    if (a.sink == nullptr) return f / l;
+    const float top = fmaxf(m, a.sink[h]), e = expf(m - top);
+    return f * (e / (l * e + expf(a.sink[h] - top)));
+  };
+  unsigned again[2];                                     // lanes whose row's sums are not finite
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     l_run[u] += __shfl_xor_sync(0xffffffffu, l_run[u], 1);
     l_run[u] += __shfl_xor_sync(0xffffffffu, l_run[u], 2);
     const int r = warp * 16 + g + u * 8;
-    if (r >= rows) continue;
+    float probe = 0.f;                                   // NaN if a sum is not finite
+#pragma unroll
+    for (int n = 0; n < DN / 8; ++n) probe = fmaf(O[n][2 * u], 0.f, fmaf(O[n][2 * u + 1], 0.f, probe));
+    again[u] = __ballot_sync(0xffffffffu, r < rows && probe != 0.f);
+    if (r >= rows || ((again[u] >> (4 * g)) & 15u)) continue;
     const size_t row = row0 + r, at = (row * a.H + h) * DN;
-    float f = a.gate ? a.gate[row * a.H + h] : 1.0f;
-    if (a.sink == nullptr) {
-      f /= l_run[u];
-    } else {                                             // everything relative to the larger of maximum and sink
-      const float top = fmaxf(m_run[u], a.sink[h]), e = expf(m_run[u] - top);
-      f *= e / (l_run[u] * e + expf(a.sink[h] - top));
-    }
+    const float f = factor(row, m_run[u], l_run[u]);
 #pragma unroll
     for (int n = 0; n < DN / 8; ++n) {
       const int ch = n * 8 + 2 * t;
       const float y0 = O[n][2 * u] * f, y1 = O[n][2 * u + 1] * f;
       if (a.out_f32) *reinterpret_cast<float2*>(reinterpret_cast<float*>(a.out) + at + ch) = make_float2(y0, y1);
       else *reinterpret_cast<uint32_t*>(reinterpret_cast<bf16*>(a.out) + at + ch) = pack_bf16x2(y0, y1);
+    }
+  }
+  if ((again[0] | again[1]) == 0u) return;
+#pragma unroll 1
+  for (int i = 0; i < 16; ++i) {
+    if ((((i < 8 ? again[0] : again[1]) >> (4 * (i & 7))) & 15u) == 0u) continue;
+    const size_t row = row0 + warp * 16 + i;
+    const PlainRow<DN> y = plain_row<DN, DR>(a.q + row * a.ldq + (size_t)h * (DN + DR), a.qr + (row * a.H + h) * a.qr_stride, keys, vals, key_stride, key_rot, a.kr_stride,
+                                             max(0, wpos + i - a.window + 1), wpos + i, a.scale);
+    const float f = factor(row, y.m, y.l);
+#pragma unroll
+    for (int c = 0; c < DN / 32; ++c) {
+      const size_t at = (row * a.H + h) * DN + lane + 32 * c;
+      if (a.out_f32) reinterpret_cast<float*>(a.out)[at] = y.o[c] * f;
+      else reinterpret_cast<bf16*>(a.out)[at] = __float2bfloat16_rn(y.o[c] * f);
     }
   }
 }

@@ -81,3 +81,24 @@ def test_single_token_weighs_an_infinite_value(max_ctx, H):
         o, c = o.clone(), c.clone()
         o[:H // 2, 9] = c[:H // 2, 9] = 0.0
         assert float((o - c).abs().max()) < TOL
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("window", [0, 40])
+@pytest.mark.parametrize("at", [3, 70, 129])
+def test_latent_rows_that_see_a_bad_key_and_those_that_do_not(dim, window, at):
+    H, n, past, rank, rot = 2, 130, 20, 64, 64
+    q, qr, lat = randn(n, H * (dim + rot), seed=1), randn(n, H, rot, seed=2).float(), randn(1, past + n, rank + rot, seed=3)
+    w = (randn(2 * H * dim, rank, seed=4).float() * rank ** -0.5).to(BF16)
+    sink = torch.linspace(-1.0, 1.0, H, device=DEV)
+
+    def run(lat):
+        out = torch.empty(n, H * dim, dtype=F32, device=DEV)
+        return ops.latent_attn_expanded(q, qr, lat, [(0, past, 0, n)], w, None, out, H, dim, rot, rank, 0.1, window=window, sink=sink)
+    clean, pos, key = run(lat), torch.arange(past, past + n), past + at
+    sees = ((pos >= key) & (pos - key < (window or 1 << 30))).to(DEV)
+    for c, bad in ((5, float("inf")), (5, float("nan")), (rank + 5, float("nan"))):         # in the latent, in the rotated part of the key
+        x = lat.clone()
+        x[0, key, c] = bad
+        out = run(x)
+        assert (float((out[~sees] - clean[~sees]).abs().max()) < TOL if bool((~sees).any()) else True) and bool((~torch.isfinite(out[sees])).all())
