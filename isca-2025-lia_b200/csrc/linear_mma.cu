@@ -4,7 +4,8 @@
 //
 // fp32 operands enter as three bf16 parts (mma.cuh): an fp32 x bf16 product is three bf16 products, fp32 x fp32 six (of the nine, those whose
 // factors together lie less than 24 bits below the highest).  Sums of 32 channels are made apart, the high products in one chain and the rest
-// in another, and added to the running ones in fp32, because the tensor cores cut sums off instead of rounding them.
+// in another, and added to the running ones in fp32, because the tensor cores cut sums off instead of rounding them.  An infinity has no parts (its
+// products with the other factor's parts, 0 or of the other sign, are NaN), so a sum that is not finite is formed again in one FMA chain.
 //
 // Bound: tensor cores (mma.sync m16n8k16).  128 x (16 NT) tile per block of 8 warps (4 x 2), a warp owns 32 x 8 NT; 32 channels per stage, two
 // stages; bf16 operands come by cp.async, fp32 ones through registers, where they are split.
@@ -70,6 +71,17 @@ struct RowRanges {
 struct NoRanges {};
 
 enum { OUT_F32, OUT_BF16, OUT_PARTS };     // OUT_PARTS: column n = group * part + c goes, as three bf16 parts, to [m][group][3][part]
+
+// sum_k a[k] w[k] in one chain, as far as it is not settled
+template <int NA, int NW> __device__ __noinline__ float plain_dot(const void* a, size_t a_at, const void* w, size_t w_at, int K) {
+  float s = 0.f;
+  for (int k = 0; k < K && s == s; ++k) {
+    const float x = NA == 3 ? reinterpret_cast<const float*>(a)[a_at + k] : __bfloat162float(reinterpret_cast<const bf16*>(a)[a_at + k]);
+    const float y = NW == 3 ? reinterpret_cast<const float*>(w)[w_at + k] : __bfloat162float(reinterpret_cast<const bf16*>(w)[w_at + k]);
+    s = fmaf(x, y, s);
+  }
+  return s;
+}
 
 template <int NA, int NW, int NT, int OUT>
 __global__ void __launch_bounds__(256) linear_mma_kernel(const void* __restrict__ A, long long lda, long long sA, const void* __restrict__ Wt, long long ldw,
@@ -184,6 +196,10 @@ __global__ void __launch_bounds__(256) linear_mma_kernel(const void* __restrict_
       for (int n = 0; n < NT; ++n) {
         const int col = n0 + wn + n * 8 + 2 * t;
         if (col >= N) continue;
+        if constexpr (SPLIT) {
+          if (!(fabsf(acc[i][n][2 * u]) < INFINITY)) acc[i][n][2 * u] = plain_dot<NA, NW>(A, (size_t)m * lda, Wt, (size_t)col * ldw, K);
+          if (col + 1 < N && !(fabsf(acc[i][n][2 * u + 1]) < INFINITY)) acc[i][n][2 * u + 1] = plain_dot<NA, NW>(A, (size_t)m * lda, Wt, (size_t)(col + 1) * ldw, K);
+        }
         const float x = acc[i][n][2 * u] * scale, y = acc[i][n][2 * u + 1] * scale;
         if constexpr (OUT == OUT_F32) {
           float* p = reinterpret_cast<float*>(C) + (size_t)b * sC + (size_t)m * ldc + col;

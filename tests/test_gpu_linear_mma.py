@@ -100,3 +100,27 @@ def test_latent_expanded_exactness(dim, rank, n, past, window, sink):
     want = torch.einsum("hns,shd->nhd", torch.softmax(sc, -1)[..., :ctx], kv[:, 1]).reshape(n, -1)
     # scores of size 3 within a few 2^-24 of their size, weights and values as exact: a few 1e-7 of the result
     assert float((out.cpu().to(F64) - want).norm() / want.norm()) < 2e-6
+
+
+@pytest.mark.parametrize("w_dt", [BF16, F32])
+@pytest.mark.parametrize("M,N,K", [(65, 24, 40), (130, 65, 520)])
+def test_linear_plain_with_numbers_that_are_not_finite(w_dt, M, N, K):
+    """An infinity times a finite weight is one, whatever the weight's low bits; largest finite numbers do not become one; a NaN stays in its row or column."""
+    g = torch.Generator().manual_seed(K)
+    a, w = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g).to(w_dt)
+    inf = float("inf")
+    w[1, 7] = 1.0                                               # no lower parts: 0 beside the infinity
+    a[3, 7], a[4, 0], a[5, K - 1] = inf, -inf, float("nan")
+    a[6, 2:4] = torch.tensor([inf, -inf])
+    a[7], a[8] = 0.0, 0.0
+    a[7, 1], w[:, 1] = 3.4e38, 0.5                              # the nearest bf16 number would be an infinity
+    a[8, 9], w[2, 9] = 1.0, inf
+    out = torch.empty(M, N, dtype=F32, device=DEV)
+    ops.linear_plain(a.to(DEV), w.to(DEV), out)
+    want = a.to(F64) @ w.to(F64).T                              # (float64 holds the finite sums; none of them overflows fp32)
+    got = out.cpu().to(F64)
+    fin = torch.isfinite(want)
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(got[~fin & ~torch.isnan(want)], want[~fin & ~torch.isnan(want)])
+    bound = torch.nan_to_num(a.to(F64).abs() @ w.to(F64).abs().T, nan=inf) * K * 2.0 ** -24
+    assert bool(((got - want).abs()[fin] <= bound[fin]).all())
+    assert not bool(fin[3].any()) and bool((~torch.isnan(want[3])).all()) and bool(fin[7, :2].all())
