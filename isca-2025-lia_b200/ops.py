@@ -640,11 +640,14 @@ def moe_tiles(pairs, E, tensor_core=False):
 
 
 def moe_plan(idx, E, perm, tile_expert, pos_of):
+    """Groups the pairs by expert in tiles of ``moe_tiles`` rows: those of the tensor-core form if ``perm`` holds exactly ``tile_expert.numel()`` of them, else
+    the others (``perm`` may then be larger than the plan)."""
     _req(idx, "idx", I32); _req(perm, "perm", I32); _req(tile_expert, "tile_expert", I32); _req(pos_of, "pos_of", I32)
-    tiles = tile_expert.numel()
-    if perm.numel() % tiles:
-        raise _lib.LiaError("moe_plan: perm must hold whole tiles")
-    check(_lib.load().lia_moe_plan_rows(_p(idx), idx.numel(), E, perm.numel() // tiles, tiles, _p(perm), _p(tile_expert), _p(pos_of), _stream()), "lia_moe_plan")
+    lib, tiles = _lib.load(), tile_expert.numel()
+    rows = lib.lia_moe_tc_rows() if perm.numel() == tiles * lib.lia_moe_tc_rows() else lib.lia_moe_tile_rows()
+    if perm.numel() < tiles * rows:
+        raise _lib.LiaError(f"moe_plan: {tiles} tiles of {rows} rows do not fit perm ({perm.numel()})")
+    check(lib.lia_moe_plan_rows(_p(idx), idx.numel(), E, rows, tiles, _p(perm), _p(tile_expert), _p(pos_of), _stream()), "lia_moe_plan")
     count_launches()
 
 

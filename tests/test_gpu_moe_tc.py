@@ -81,3 +81,21 @@ def test_projections(counts, top, W, ff, form):
         bound = 1e-5 + (terms.abs().view(M, top, W).sum(1) * 2.0 ** -8 if plan else 0.0)
         assert bool(((y.cpu().to(F64) - total).abs() <= bound).all())
     assert _lib.load().lia_moe_timeouts() == 0
+
+
+def test_a_plan_in_a_larger_buffer():
+    """The rows of a tile do not follow from how much room a caller has left behind the plan."""
+    E, idx = 3, torch.tensor([0, 2, 2, 0, 1] * 30, dtype=torch.int32, device=DEV)
+    n_tiles, tm = ops.moe_tiles(idx.numel(), E)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    plans = []
+    for room in (0, 1, 36 * n_tiles):
+        perm, tile_expert, pos_of = torch.full((n_tiles * tm + room,), 7, **i32), torch.empty(n_tiles, **i32), torch.empty(idx.numel(), **i32)
+        ops.moe_plan(idx, E, perm, tile_expert, pos_of)
+        place = perm[:n_tiles * tm].view(n_tiles, tm)
+        assert all(bool((idx[p[p >= 0].long()] == e).all()) for p, e in zip(place, tile_expert.tolist())) and bool((perm[n_tiles * tm:] == 7).all())
+        assert torch.equal(perm[pos_of.long()], torch.arange(idx.numel(), **i32))
+        plans.append(tile_expert)
+    assert torch.equal(plans[0], plans[1]) and torch.equal(plans[0], plans[2])
+    with pytest.raises(_lib.LiaError):
+        ops.moe_plan(idx, E, torch.empty(n_tiles * tm - 1, **i32), torch.empty(n_tiles, **i32), torch.empty(idx.numel(), **i32))
