@@ -403,7 +403,7 @@ def _in_chunks(mlstm, q, k, v, ld, ldv, dim, vdim, state_S, o, n, lengths):
     """Whether portions of a matrix-state recurrence are long enough for the form in chunks of tokens on the tensor cores (csrc/chunk_scan.cu), and it takes them;
     and whether there are short ones as well.  A portion's own length decides how it is computed, whatever comes with it."""
     fewest, M = _chunk_rows(mlstm, dim, vdim), q.shape[0]
-    shortest, longest = lengths or (M if n == 1 else 1, M - n + 1)
+    shortest, longest = lengths or (0, M - n + 1)        # unknown: there may be rows of no portion
     if q.dtype != BF16 or not fewest or longest < fewest:
         return False, False
     return (ld % 8 == 0 and ldv % 8 == 0 and (q.data_ptr() | k.data_ptr() | v.data_ptr() | o.data_ptr()) % 16 == 0 and state_S.data_ptr() % 8 == 0), shortest < fewest

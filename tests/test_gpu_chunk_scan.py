@@ -131,3 +131,24 @@ def test_a_portion_does_not_depend_on_its_company(gated):
     for slot, p0, row, n in segs:
         o, st = run(slice(row, row + n), [(slot, p0, 0, n)], (n, n))
         assert torch.equal(o, together[0][row:row + n]) and all(torch.equal(a[slot], b[slot]) for a, b in zip(st, together[1]))
+
+
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("lens", [[20], [70], [31]])
+def test_portions_of_unknown_lengths_in_a_larger_buffer(gated, lens):
+    """What the segments say counts, not how many rows the buffers have."""
+    H, dim, vdim, M, n = 2, 128, 64, 100, len(lens)
+    q, k, v, _, _, r = _step([M], H, H, dim, vdim)
+    segs = [(i, 0, 0, x) for i, x in enumerate(lens)]
+    dsegs = torch.tensor(segs, dtype=torch.int32, device="cuda")
+    gates, d = torch.cat([r(M, H), -r(M, H).abs()], 1).contiguous(), torch.tensor([0.99, 0.7], device="cuda")
+    start, got = (r(n, H, vdim, dim), r(n, H, dim), r(n, H)), []
+    for rows, lengths in ((M, None), (lens[0], (min(lens), max(lens)))):
+        st, o = [t.clone() for t in start], torch.full((rows, H * vdim), 7.0, device="cuda")
+        if gated:
+            ops.mlstm_scan(q[:rows], k[:rows], v[:rows], gates[:rows], *st, dsegs, H, dim, vdim, 0.1, 1e-6, o, lengths=lengths)
+        else:
+            ops.linear_scan(q[:rows], k[:rows], v[:rows], st[0], dsegs, H, H, dim, vdim, o, decay=d, lengths=lengths)
+        got.append((o, *st))
+    assert torch.equal(got[0][0][:lens[0]], got[1][0]) and bool((got[0][0][lens[0]:] == 7.0).all())
+    assert all(torch.equal(a, b) for a, b in zip(got[0][1:], got[1][1:])) and not torch.equal(got[0][1], start[0])
