@@ -642,7 +642,9 @@ extern "C" const unsigned long long* lia_debug_gemm_trace(void) {
 
 extern "C" size_t lia_gemm_workspace_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  return plan_workspace(make_plan(M, N, K));
+  // of the plan that a launch takes: with whole tiles or parts for small weights alone, by spans inside a fused exchange
+  const size_t alone = plan_workspace(make_plan(M, N, K, /*allow_pair=*/true)), spans = plan_workspace(make_plan(M, N, K));
+  return alone > spans ? alone : spans;
 }
 
 static int gemm_impl(const void* A, const void* W, const void* bias, const void* residual, void* out, int M, int N, int K,
