@@ -539,6 +539,11 @@ size_t lia_latent_expanded_workspace_bytes(long long latents, int H, int dim);
 int lia_latent_attn_expanded(const void* q, int ldq, const float* qr, int qr_stride, const void* cache, long long slot_stride, const int* portions, int np,
                              const void* w_ukv, const float* gate, const float* sink, void* out, int out_f32, void* workspace, int H, int dim,
                              int rot, int kv_rank, int window, float scale, lia_stream_t stream);
+/* the same in a workspace of any size that holds one head of the portion that sees most latents: portions, and heads of one portion, go in as many
+ * launches as it takes; the results are the same bits */
+int lia_latent_attn_expanded_in(const void* q, int ldq, const float* qr, int qr_stride, const void* cache, long long slot_stride, const int* portions, int np,
+                                const void* w_ukv, const float* gate, const float* sink, void* out, int out_f32, void* workspace, size_t workspace_bytes, int H,
+                                int dim, int rot, int kv_rank, int window, float scale, lia_stream_t stream);
 /* lia_router_topk_ext on rows of ldl numbers whose first E are the logits; sigmoid != 0: an expert's score is the sigmoid of its logit */
 int lia_router_topk_scored(const float* logits, int ldl, const float* correction, int renorm, int sigmoid, int* idx, float* wt, int M, int E,
                            int top, lia_stream_t stream);

@@ -175,6 +175,8 @@ _PROTOTYPES = {
     "lia_latent_expanded_workspace_bytes": (c_size_t, [c_longlong, c_int, c_int]),
     "lia_latent_attn_expanded": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                          c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p]),
+    "lia_latent_attn_expanded_in": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
+                                            c_int, c_void_p, c_size_t, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p]),
     "lia_moe_plan_rows": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "lia_moe_tc_rows": (c_int, []),
     "lia_moe_timeouts": (c_int, []),

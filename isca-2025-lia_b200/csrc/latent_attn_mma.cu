@@ -10,12 +10,14 @@
 // is enough and two blocks share an SM.  Bound: tensor cores and shared-memory reads about equally.  2048 tokens, 16 heads of 128 + 64 on latents
 // of 512: 4794 us in the latent space on the CUDA cores and 439 us for its two projections -> 329 and 67 us for the expansion.
 // Rows whose sums are not finite are formed again key by key at the end, as in window_attn_mma.cu: a masked key's weight of 0 still meets its value.
+#include <limits.h>
 #include <math.h>
+#include <stdint.h>
 
 #include "mma.cuh"
 
 // linear_mma.cu
-int linear_mma_parts(const bf16* const* src, const int* rows, int n, long long lda, const bf16* W, bf16* C, int N, int K, int part, cudaStream_t stream);
+int linear_mma_parts(const bf16* const* src, const int* rows, int n, long long lda, const bf16* W, bf16* C, long long ldc, int N, int K, int part, cudaStream_t stream);
 
 namespace {
 
@@ -34,12 +36,12 @@ struct Portion {
 struct ExpandedArgs {
   const bf16* q;        // rows of H heads of DN + DR channels, the first DN unrotated
   const float* qr;      // [row][H][qr_stride]: the rotated DR channels
-  const bf16* parts;    // [latent][2 H][3][DN]: keys of the heads, then values
+  const bf16* parts;    // [latent][2 nh][3][DN]: keys of the heads h0 .. h0 + nh - 1, then values
   const float* gate;    // [row][H] or null
   const float* sink;    // [H] or null
   void* out;            // [row][H * DN]
   long long kr_stride;
-  int ldq, qr_stride, H, window, out_f32, np;
+  int ldq, qr_stride, H, h0, nh, window, out_f32, np;
   float scale;
   Portion p[MAX_PORTIONS];
 };
@@ -91,16 +93,16 @@ __global__ void __launch_bounds__(128, 2) latent_expanded_kernel(const __grid_co
   extern __shared__ __align__(128) unsigned char smem[];
   const uint32_t qn = smem_u32(smem), qr = qn + BM * DN * 2, kn = qr + 3 * BM * DR * 2, kr = kn + 3 * BK * DN * 2, vs = kr + BK * DR * 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int h = blockIdx.x, tile = gridDim.y - 1 - blockIdx.y;                   // a portion's longest histories start first
+  const int h = a.h0 + blockIdx.x, tile = gridDim.y - 1 - blockIdx.y;            // a portion's longest histories start first
   int ip = 0;
   while (ip + 1 < a.np && tile >= a.p[ip + 1].tile0) ++ip;
   const Portion& pt = a.p[ip];
   const int skip = (tile - pt.tile0) * BM, row0 = pt.row0 + skip;
   const int rows = min(BM, pt.n - skip), pos0 = pt.pos0 + skip, pos_last = pos0 + rows - 1;
   const int jb = max(0, pos0 - a.window + 1);
-  const size_t key_stride = (size_t)a.H * 6 * DN;
-  const bf16* keys = a.parts + (size_t)pt.part0 * key_stride + (size_t)h * 3 * DN;
-  const bf16* vals = keys + (size_t)a.H * 3 * DN;
+  const size_t key_stride = (size_t)a.nh * 6 * DN;
+  const bf16* keys = a.parts + (size_t)pt.part0 * key_stride + (size_t)blockIdx.x * 3 * DN;
+  const bf16* vals = keys + (size_t)a.nh * 3 * DN;
   const bf16* key_rot = pt.kr;
 
   // three parts side by side in memory, three tiles in shared memory; keys behind the last are zero
@@ -327,7 +329,7 @@ __global__ void __launch_bounds__(128, 2) latent_expanded_kernel(const __grid_co
 template <int DN, int DR> int run(const ExpandedArgs& a, int tiles, cudaStream_t stream) {
   constexpr int smem = expanded_smem<DN, DR>();
   LIA_CUDA(cudaFuncSetAttribute(latent_expanded_kernel<DN, DR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  lia_launch(latent_expanded_kernel<DN, DR>, dim3(dim3(a.H, tiles)), dim3(128), smem, stream, a);
+  lia_launch(latent_expanded_kernel<DN, DR>, dim3(a.nh, tiles), dim3(128), smem, stream, a);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -340,6 +342,15 @@ extern "C" size_t lia_latent_expanded_workspace_bytes(long long latents, int H, 
 extern "C" int lia_latent_attn_expanded(const void* q, int ldq, const float* qr, int qr_stride, const void* cache, long long slot_stride, const int* portions, int np,
                                         const void* w_ukv, const float* gate, const float* sink, void* out, int out_f32, void* workspace, int H, int dim,
                                         int rot, int kv_rank, int window, float scale, lia_stream_t stream_) {
+  return lia_latent_attn_expanded_in(q, ldq, qr, qr_stride, cache, slot_stride, portions, np, w_ukv, gate, sink, out, out_f32, workspace, SIZE_MAX, H, dim, rot, kv_rank, window,
+                                     scale, stream_);
+}
+
+// Portions go together while they are at most MAX_PORTIONS and their expanded keys and values fit the workspace; a portion that does not fit by itself goes in
+// groups of heads.  Neither changes a bit of the result: every number is made by the same sums.
+extern "C" int lia_latent_attn_expanded_in(const void* q, int ldq, const float* qr, int qr_stride, const void* cache, long long slot_stride, const int* portions, int np,
+                                           const void* w_ukv, const float* gate, const float* sink, void* out, int out_f32, void* workspace, size_t workspace_bytes, int H,
+                                           int dim, int rot, int kv_rank, int window, float scale, lia_stream_t stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LIA_CHECK_ARG(q && qr && cache && portions && w_ukv && out && workspace && np > 0 && H > 0 && H <= 65535, "lia_latent_attn_expanded: bad arguments");
   LIA_CHECK_ARG((dim == 128 || dim == 64) && rot == 64 && kv_rank > 0 && kv_rank % 8 == 0, "lia_latent_attn_expanded: heads of %d + %d channels on latents of %d", dim, rot, kv_rank);
@@ -347,26 +358,44 @@ extern "C" int lia_latent_attn_expanded(const void* q, int ldq, const float* qr,
                          reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(workspace);
   LIA_CHECK_ARG(addr % 16 == 0 && ldq % 8 == 0 && ldq >= H * (dim + rot) && qr_stride % 4 == 0 && slot_stride % 8 == 0, "lia_latent_attn_expanded: addresses and rows must be whole 16 bytes");
   const int D = kv_rank + rot;
+  const size_t room = workspace_bytes / lia_latent_expanded_workspace_bytes(1, 1, dim);          // (latent, head) pairs
   if (window <= 0) window = 1 << 30;
-  for (int first = 0; first < np; first += MAX_PORTIONS) {
-    ExpandedArgs a{reinterpret_cast<const bf16*>(q), qr, reinterpret_cast<const bf16*>(workspace), gate, sink, out, D, ldq, qr_stride, H, window, out_f32,
-                   np - first < MAX_PORTIONS ? np - first : MAX_PORTIONS, scale, {}};
+  for (int first = 0; first < np;) {
+    ExpandedArgs a{reinterpret_cast<const bf16*>(q), qr, reinterpret_cast<const bf16*>(workspace), gate, sink, out, D, ldq, qr_stride, H, 0, 0, window, out_f32, 0, scale, {}};
     const bf16* src[MAX_PORTIONS];
-    int rows[MAX_PORTIONS], tiles = 0, latents = 0;
-    for (int i = 0; i < a.np; ++i) {
-      const int* p = portions + 4 * (first + i);                   // slot, first position, first row, rows
+    int rows[MAX_PORTIONS], tiles = 0;
+    long long latents = 0;
+    while (first < np && a.np < MAX_PORTIONS) {
+      const int* p = portions + 4 * first;                         // slot, first position, first row, rows
       LIA_CHECK_ARG(p[0] >= 0 && p[1] >= 0 && p[2] >= 0 && p[3] > 0, "lia_latent_attn_expanded: bad portion");
-      const int base = p[1] - window + 1 > 0 ? p[1] - window + 1 : 0;
+      const int base = p[1] - window + 1 > 0 ? p[1] - window + 1 : 0, seen = p[1] + p[3] - base, i = a.np;
+      if (i > 0 && ((size_t)(latents + seen) * H > room || latents + seen > INT_MAX)) break;
       src[i] = reinterpret_cast<const bf16*>(cache) + (size_t)p[0] * slot_stride + (size_t)base * D;
-      rows[i] = p[1] + p[3] - base;
-      a.p[i] = Portion{src[i] + kv_rank, p[2], p[3], p[1] - base, latents, tiles};
+      rows[i] = seen;
+      a.p[i] = Portion{src[i] + kv_rank, p[2], p[3], p[1] - base, (int)latents, tiles};
       tiles += (p[3] + BM - 1) / BM;
-      latents += rows[i];
+      latents += seen;
+      ++a.np;
+      ++first;
     }
     LIA_CHECK_ARG(tiles <= 65535, "lia_latent_attn_expanded: too many rows");
-    int rc = linear_mma_parts(src, rows, a.np, D, reinterpret_cast<const bf16*>(w_ukv), reinterpret_cast<bf16*>(workspace), 2 * H * dim, kv_rank, dim, stream);
-    if (rc == LIA_OK) rc = dim == 128 ? run<128, 64>(a, tiles, stream) : run<64, 64>(a, tiles, stream);
-    if (rc != LIA_OK) return rc;
+    LIA_CHECK_ARG((size_t)latents <= room, "lia_latent_attn_expanded: a workspace of %zu bytes does not hold one head of %lld latents", workspace_bytes, latents);
+    const int most = (size_t)latents * H <= room ? H : (int)(room / latents);
+    const bf16* wk = reinterpret_cast<const bf16*>(w_ukv);
+    bf16* ws = reinterpret_cast<bf16*>(workspace);
+    for (a.h0 = 0; a.h0 < H; a.h0 += a.nh) {
+      a.nh = most < H - a.h0 ? most : H - a.h0;
+      const long long ldc = 6ll * a.nh * dim;
+      int rc;
+      if (a.nh == H) {
+        rc = linear_mma_parts(src, rows, a.np, D, wk, ws, ldc, 2 * H * dim, kv_rank, dim, stream);
+      } else {
+        rc = linear_mma_parts(src, rows, a.np, D, wk + (size_t)a.h0 * dim * kv_rank, ws, ldc, a.nh * dim, kv_rank, dim, stream);
+        if (rc == LIA_OK) rc = linear_mma_parts(src, rows, a.np, D, wk + (size_t)(H + a.h0) * dim * kv_rank, ws + (size_t)3 * a.nh * dim, ldc, a.nh * dim, kv_rank, dim, stream);
+      }
+      if (rc == LIA_OK) rc = dim == 128 ? run<128, 64>(a, tiles, stream) : run<64, 64>(a, tiles, stream);
+      if (rc != LIA_OK) return rc;
+    }
   }
   return LIA_OK;
 }

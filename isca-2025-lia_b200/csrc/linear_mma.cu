@@ -264,8 +264,8 @@ int linear_mma(const void* A, int a_f32, long long lda, long long sA, const void
 }
 
 // bf16 x bf16 for up to 16 row ranges, the results one range after the other as three bf16 parts, `part` columns (a multiple of 2) at a
-// time: C [rows][N / part][3][part]
-int linear_mma_parts(const bf16* const* src, const int* rows, int n, long long lda, const bf16* W, bf16* C, int N, int K, int part, cudaStream_t stream) {
+// time: C [rows][N / part][3][part], rows ldc numbers apart
+int linear_mma_parts(const bf16* const* src, const int* rows, int n, long long lda, const bf16* W, bf16* C, long long ldc, int N, int K, int part, cudaStream_t stream) {
   LIA_CHECK_ARG(n > 0 && n <= RowRanges::MAX, "linear_mma_parts: %d row ranges", n);
   RowRanges r{};
   r.n = n;
@@ -280,7 +280,7 @@ int linear_mma_parts(const bf16* const* src, const int* rows, int n, long long l
   }
   LIA_CHECK_ARG(tiles <= 65535, "linear_mma_parts: too many rows (%d)", out);
   constexpr int NT = 8, smem = 2 * (Tile<1, TM>::BYTES + Tile<1, 16 * NT>::BYTES);
-  lia_launch(linear_mma_kernel<1, 1, NT, OUT_PARTS>, dim3(dim3((N + 16 * NT - 1) / (16 * NT), tiles, 1)), dim3(256), smem, stream, nullptr, lda, 0, W, K, 0, C, 3ll * N, 0, 0, N, K,
+  lia_launch(linear_mma_kernel<1, 1, NT, OUT_PARTS>, dim3(dim3((N + 16 * NT - 1) / (16 * NT), tiles, 1)), dim3(256), smem, stream, nullptr, lda, 0, W, K, 0, C, ldc, 0, 0, N, K,
                                                                                                               1.0f, part, r);
   LIA_LAUNCH_CHECK();
   return LIA_OK;

@@ -514,11 +514,23 @@ def latent_attn(qa, cache, meta, gate, out, H, kv_rank, rot, scale, max_ctx=0, w
     return out
 
 
-def latent_attn_expanded(q, qr, cache, portions, w_ukv, gate, out, H, dim, rot, kv_rank, scale, window=0, sink=None):
+def _expanded_launches(seen, H, room):
+    """Launches of ``latent_attn_expanded`` (csrc/latent_attn_mma.cu) over portions that see so many latents."""
+    n, count, latents = 0, 0, 0
+    for s in seen + [None]:
+        if count and (s is None or count == 16 or (latents + s) * H > room):
+            n += 2 if latents * H <= room else 3 * -(-H // (room // latents))
+            count, latents = 0, 0
+        count, latents = count + 1, latents + (s or 0)
+    return n
+
+
+def latent_attn_expanded(q, qr, cache, portions, w_ukv, gate, out, H, dim, rot, kv_rank, scale, window=0, sink=None, room=1 << 18):
     """Attention of the rows of ``portions`` -- (slot, first position, first row, rows) each, host numbers -- over the latents they see, keys and values
     expanded per head (csrc/latent_attn_mma.cu).  ``q`` [M, H * (dim + rot)] bf16; ``qr``: the turned query parts, a view [M, H, rot] of fp32;
     ``cache`` [slots, capacity, kv_rank + rot] bf16; ``w_ukv`` [2 H dim, kv_rank]: Wuk above Wuv.  ``out`` [M, H * dim] bf16 or fp32: only the
-    portions' rows are written."""
+    portions' rows are written.  At most ``room`` (latent, head) pairs are expanded at a time (12 ``dim`` bytes each; fewer where memory is short), which changes
+    no bit of the result."""
     _dev(q, "q", BF16); _req(cache, "cache"); _req(w_ukv, "w_ukv")
     M = q.shape[0]
     for t, m in ((gate, "gate"), (sink, "sink")):
@@ -533,13 +545,20 @@ def latent_attn_expanded(q, qr, cache, portions, w_ukv, gate, out, H, dim, rot, 
         if not (0 <= slot < cache.shape[0] and 0 <= p0 and n > 0 and p0 + n <= cache.shape[1] and 0 <= row and row + n <= M):
             raise _lib.LiaError(f"latent_attn_expanded: portion {(slot, p0, row, n)} outside {M} rows or the cache {tuple(cache.shape)}")
         seen.append(p0 + n - (max(0, p0 - window + 1) if window > 0 else 0))
-    lib = _lib.load()
-    groups = range(0, len(seen), 16)
-    ws = torch.empty(lib.lia_latent_expanded_workspace_bytes(max(sum(seen[g:g + 16]) for g in groups), H, dim), dtype=torch.uint8, device=q.device)
+    lib, longest = _lib.load(), max(seen)
+    room = max(longest, min(room, H * max(sum(seen[g:g + 16]) for g in range(0, len(seen), 16))))
+    while True:
+        try:
+            ws = torch.empty(lib.lia_latent_expanded_workspace_bytes(room, 1, dim), dtype=torch.uint8, device=q.device)
+            break
+        except torch.OutOfMemoryError:
+            if room == longest:
+                raise
+            room = max(longest, room // 4)
     table = (ctypes.c_int * (4 * len(portions)))(*[int(x) for p in portions for x in p])
-    check(lib.lia_latent_attn_expanded(_p(q), _rowmajor(q, "q"), _p(qr), qr.stride(1), _p(cache), cache.stride(0), table, len(portions), _p(w_ukv), _p(gate),
-                                       _p(sink), _p(out), _f32(out), _p(ws), H, dim, rot, kv_rank, int(window), float(scale), _stream()), "lia_latent_attn_expanded")
-    count_launches(2 * len(groups))
+    check(lib.lia_latent_attn_expanded_in(_p(q), _rowmajor(q, "q"), _p(qr), qr.stride(1), _p(cache), cache.stride(0), table, len(portions), _p(w_ukv), _p(gate),
+                                          _p(sink), _p(out), _f32(out), _p(ws), ws.numel(), H, dim, rot, kv_rank, int(window), float(scale), _stream()), "lia_latent_attn_expanded")
+    count_launches(_expanded_launches(seen, H, room))
     return out
 
 

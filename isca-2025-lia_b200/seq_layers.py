@@ -146,8 +146,10 @@ class LatentAttentionMixer:
     EXPAND_ROWS = 64          # portions of at least this many rows may expand the latents they see ...
     EXPAND_RATIO = 4          # ... if these are at most this many times the rows
     # The tensor-core form, which keeps expanded keys and values as exact as fp32 (csrc/latent_attn_mma.cu), for designs with a rotated part or a gate:
-    EXPAND_ROWS_EXACT = 16             # from here on expanding costs less than attention in the latent space on the CUDA cores
-    EXPAND_KEYS_EXACT = 1 << 20        # keys x heads whose expansion (1.5 KB each at 128 channels) a step may hold at a time
+    # The portion alone decides (``_expands_exactly``), whatever else is in the step.
+    EXPAND_ROWS_EXACT = 16             # fewer rows never
+    EXPAND_ROWS_ALWAYS = 64            # a block's rows: from here on whatever the history; below, its cost is that of 64 rows
+    EXPAND_KEYS_EXACT = 1 << 18        # keys x heads that are held expanded at a time (1.5 KB each at 128 channels)
 
     def __init__(self, w, heads, dim, rot_dim, vdim, kv_rank, rot_dims, rot_base, scale, norm_eps, dtype, device, q_rank=None, rot_pairs=False,
                  rot_scaling=None, gate="head", window=0, sink=False, own_latent=True):
@@ -228,7 +230,7 @@ class LatentAttentionMixer:
         exact = self._expands_exactly(q, portions, H)
         if exact:
             ops.latent_attn_expanded(q, qa.view(M, H, D)[:, :, self.rank:], cache, [portions[i] for i in exact], self.w_ukv, gate, o, H, self.dim, self.rot,
-                                     self.rank, self.scale, window=self.window, sink=self.sink)
+                                     self.rank, self.scale, window=self.window, sink=self.sink, room=self.EXPAND_KEYS_EXACT)
         for i, (slot, p0, row, n) in enumerate(portions if exact or self.up_k is not None else ()):
             if i in exact:
                 self._in_latent_space(q, qa, cache, gate, batch, o, done, row)
@@ -246,15 +248,20 @@ class LatentAttentionMixer:
         return self.out(o)
 
     def _expands_exactly(self, q, portions, H):
-        """The portions (by number) whose latents are expanded to keys and values as exact as fp32: of some length, within the workspace's bound."""
+        """The portions (by number) whose latents are expanded to keys and values as exact as fp32.  A block walks a portion's keys for 64 rows of one head
+        whether it has them or not, while the kernel in the latent space takes as long as rows x groups of 8 heads and splits few rows' keys over the GPU.  Time
+        of the mixer's kernels, latent space | expanded, in us: 16 heads, 16 rows that see 256 keys 93 | 85, 1024 keys 119 | 177, 33 rows that see 1024 keys 220 | 186,
+        64 rows that see 8192 keys 1842 | 1296; 4 heads, 24 rows that see 256 keys 83 | 78, 1024 keys 100 | 157.  Heads that do not fit EXPAND_KEYS_EXACT go in turn,
+        which needs enough blocks each time."""
         if self.w_ukv is None or q.data_ptr() % 16 or q.stride(0) % 8:
             return ()
-        found, seen = [], 0
+        found = []
         for i, (_, p0, _, n) in enumerate(portions):
             ctx = p0 + n - (max(0, p0 - self.window + 1) if self.window else 0)
-            if n >= self.EXPAND_ROWS_EXACT and (seen + ctx) * H <= self.EXPAND_KEYS_EXACT:
+            pays = n >= self.EXPAND_ROWS_ALWAYS or 5 * ctx <= 2 * n * n * ((H + 7) // 8)
+            heads = min(H, self.EXPAND_KEYS_EXACT // ctx)
+            if n >= self.EXPAND_ROWS_EXACT and pays and (heads == H or heads * -(-n // 64) >= 128):
                 found.append(i)
-                seen += ctx
         return found
 
     def _in_latent_space(self, q, qa, cache, gate, batch, o, r0, r1):

@@ -124,3 +124,23 @@ def test_linear_plain_with_numbers_that_are_not_finite(w_dt, M, N, K):
     bound = torch.nan_to_num(a.to(F64).abs() @ w.to(F64).abs().T, nan=inf) * K * 2.0 ** -24
     assert bool(((got - want).abs()[fin] <= bound[fin]).all())
     assert not bool(fin[3].any()) and bool((~torch.isnan(want[3])).all()) and bool(fin[7, :2].all())
+
+
+@pytest.mark.parametrize("window", [0, 70])
+@pytest.mark.parametrize("dim", [64, 128])
+def test_latent_workspace_of_any_size(window, dim):
+    """Portions in as many launches as the workspace asks for, a large one by groups of heads: the same bits."""
+    H, rank, rot = 5, 72, 64
+    portions = [(0, 0, 0, 30), (2, 100, 30, 65), (1, 31, 95, 40), (3, 250, 135, 16)] + [(4 + i, i, 151 + i, 1) for i in range(17)]
+    M, g = 168, torch.Generator().manual_seed(dim)
+    q, qr = torch.randn(M, H * (dim + rot), generator=g).to(BF16).to(DEV), torch.randn(M, H, rot, generator=g).to(DEV)
+    lat = torch.randn(21, 280, rank + rot, generator=g).to(BF16).to(DEV)
+    w = (torch.randn(2 * H * dim, rank, generator=g) * rank ** -0.5).to(BF16).to(DEV)
+    gate, sink = torch.rand(M, H, generator=g).to(DEV), torch.linspace(-1.0, 1.0, H, device=DEV)
+    want = None
+    for room in (1 << 20, 3000, 1100, 400, 1):                  # everything; some portions; one at a time; 2 heads; one head
+        out = torch.full((M, H * dim), float("nan"), dtype=F32, device=DEV)
+        ops.latent_attn_expanded(q, qr, lat, portions, w, gate, out, H, dim, rot, rank, 0.1, window=window, sink=sink, room=room)
+        assert bool(torch.isfinite(out).all())
+        want = out if want is None else want
+        assert torch.equal(out, want)
