@@ -164,8 +164,9 @@ __global__ void __launch_bounds__(128, 2) latent_expanded_kernel(const __grid_co
     const bool on = warp_on && j0 <= wpos + 15 && j0 + BK - 1 >= wpos - a.window + 1;
     cp_async_wait<1>();
     __syncthreads();                                     // the keys (and, at first, the queries) are there
-    // Two sums per score: the unrotated channels' high products, and all the rest -- its small parts first, then the rotated channels' high
-    // products.  The tensor cores cut sums off below the 24th bit, so chains are kept short.
+    // Two sums per score: the unrotated channels' high products, 16 channels at a time added in fp32, and all the rest -- its small parts first, then the
+    // rotated channels' high products.  The tensor cores cut sums off below the 24th bit: with the high products of all channels in one chain the output of 16 to
+    // 64 rows behind up to 1500 positions was off by 0.9 to 1.15 times what the latent space gives, now by 0.75 to 0.90 (2048 tokens: 490 -> 504 us).
     float S[NT][4], S2[NT][4];
 #pragma unroll
     for (int n = 0; n < NT; ++n)
@@ -182,8 +183,19 @@ __global__ void __launch_bounds__(128, 2) latent_expanded_kernel(const __grid_co
           for (int p = 2; p >= 0; --p) {
             uint32_t b[4];
             ldsm_x4(at_chunk<QC>(kn + p * BK * DN * 2, n * 8 + (lane & 7) + ((lane >> 4) << 3), 2 * kk + ((lane >> 3) & 1)), b);
-            mma_bf16(p ? S2[n] : S[n], af, b[0], b[1]);
-            mma_bf16(p ? S2[n + 1] : S[n + 1], af, b[2], b[3]);
+            if (p > 0) {
+              mma_bf16(S2[n], af, b[0], b[1]);
+              mma_bf16(S2[n + 1], af, b[2], b[3]);
+            } else {
+              float f[2][4];
+              mma_bf16_first(f[0], af, b[0], b[1]);
+              mma_bf16_first(f[1], af, b[2], b[3]);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                S[n][i] += f[0][i];
+                S[n + 1][i] += f[1][i];
+              }
+            }
           }
       }
 #pragma unroll

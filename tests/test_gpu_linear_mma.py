@@ -144,3 +144,31 @@ def test_latent_workspace_of_any_size(window, dim):
         assert bool(torch.isfinite(out).all())
         want = out if want is None else want
         assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("H,n,past", [(4, 16, 100), (4, 33, 300), (16, 20, 200), (16, 64, 100)])
+def test_latent_portions_are_as_close_to_64_bits_as_in_the_latent_space(H, n, past):
+    """Mean over inputs of the two forms' errors: a measured 0.75 to 0.90."""
+    dim, rank, rot, ctx, ratio = 128, 512, 64, past + n, []
+    i32 = dict(dtype=torch.int32, device=DEV)
+    meta = torch.tensor([(0, past + i) for i in range(n)], **i32)
+    for seed in range(4):
+        g = torch.Generator().manual_seed(seed)
+        q = torch.randn(n, H * (dim + rot), generator=g).to(BF16).to(DEV)
+        lat, qr = torch.randn(1, ctx, rank + rot, generator=g).to(BF16).to(DEV), torch.randn(n, H, rot, generator=g).to(DEV)
+        w = (torch.randn(2 * H * dim, rank, generator=g) * rank ** -0.5).to(BF16).to(DEV)
+        scale, D = (dim + rot) ** -0.5, rank + rot
+        new = torch.empty(n, H * dim, dtype=F32, device=DEV)
+        ops.latent_attn_expanded(q, qr, lat, [(0, past, 0, n)], w, None, new, H, dim, rot, rank, scale)
+        wk, wv = w.view(2, H, dim, rank)
+        qa, oa, old = torch.empty(n, H * D, dtype=F32, device=DEV), torch.empty(n, H * rank, dtype=F32, device=DEV), torch.empty(n, H * dim, dtype=F32, device=DEV)
+        ops.linear_plain(q, wk.transpose(1, 2).contiguous(), qa, batch=H, a_batch_stride=dim + rot, w_batch_stride=rank * dim, out_batch_stride=D, n=rank, k=dim)
+        qa.view(n, H, D)[:, :, rank:] = qr
+        ops.latent_attn(qa, lat, meta, None, oa, H, rank, rot, scale, max_ctx=ctx)
+        ops.linear_plain(oa, wv, old, batch=H, a_batch_stride=rank, w_batch_stride=dim * rank, out_batch_stride=dim, n=dim, k=rank)
+        kv = (lat[0, :, :rank].to(F64) @ w.to(F64).T).view(ctx, 2, H, dim)
+        sc = (torch.einsum("nhd,shd->hns", q.to(F64).view(n, H, dim + rot)[..., :dim], kv[:, 0]) + torch.einsum("nhd,sd->hns", qr.to(F64), lat[0, :, rank:].to(F64))) * scale
+        sc = sc.masked_fill(torch.arange(ctx, device=DEV)[None, :] > torch.arange(past, ctx, device=DEV)[:, None], -math.inf)
+        want = torch.einsum("hns,shd->nhd", torch.softmax(sc, -1), kv[:, 1]).reshape(n, -1)
+        ratio.append(float((new.to(F64) - want).norm() / (old.to(F64) - want).norm()))
+    assert sum(ratio) / len(ratio) <= 1.0, ratio
