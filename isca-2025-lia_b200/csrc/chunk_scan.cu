@@ -14,8 +14,8 @@
 // one the next chunk's gates.  Q, K and V arrive by cp.async a chunk ahead.
 //
 // The hi parts' products are summed per instruction (exact but for the last bits) and added in fp32; only the lower parts stay in the tensor cores' sums,
-// which truncate.  Against 64 bits (16 heads of 128 x 128, 1024 tokens): outputs off by 8.8e-8 (token loop: 12e-8), the state by 7.8e-8 (19e-8); gated, 4 heads
-// of 256 x 512: outputs' median 1.8e-7 (2.3e-7), state 1.3e-7 (1.2e-7; 400 tokens: 1.60e-7 and 1.66e-7).
+// which truncate.  Against 64 bits, means over 6 to 10 inputs: 16 heads of 128 x 128, 1024 tokens: outputs off by 8.5e-8 (token loop: 12e-8), the state by 8e-8 (19e-8), 64
+// tokens: 7.8e-8 (8.0e-8) and 6.1e-8 (12e-8); gated, 4 heads of 256 x 512, 503 and 400 tokens: outputs' median 1.5e-7 (1.9e-7), state 1.15e-7 (1.2e-7), normaliser as there.
 // A chunk of 64 takes about 4 us, one after the other (a sequence's chunks cannot run at once): cutting the additions to half did not change that, so
 // the chain ldmatrix, mma, add and the two barriers bound it rather than the number of instructions.  A portion of 2048 tokens: 16 heads of 128 x 128
 // 533 -> 116 us, 4 heads of 256 x 512 878 -> 282.
@@ -38,8 +38,9 @@ constexpr int VP = COLS + 8;                   // row pitches in bf16 (16 bytes 
 constexpr int OP = COLS + 4;                   // and of the output parts in floats
 // A portion of fewer tokens is left to the token loops, whichever portions come with it (a portion's rounding must not depend on its company).  One portion of 24 tokens:
 // 13 us there and 10 here, of 32: 14 and 11, 8 of 33: 44 and 29; but 16 of one token: 6 and 47, for a CTA fills an SM and its chunk costs the same few
-// us however little it holds.  A prompt of 256 among 31 single tokens: 90 us all by tokens, 90 all in chunks, 42 split.
-constexpr int SHORT = 32;
+// us however little it holds.  A prompt of 256 among 31 single tokens: 90 us all by tokens, 90 all in chunks, 42 split.  With a fixed decay the outputs of 32 to 63
+// tokens would be off by 1.02 to 1.08 times what the token loop's few roundings give (64 tokens: 0.98, 100: 0.92), so there the line is 64.
+__host__ __device__ constexpr int shortest(bool mlstm) { return mlstm ? 32 : 64; }
 
 struct ChunkArgs {
   const bf16 *q, *k, *v;
@@ -77,7 +78,7 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
   ChunkSmem<DIM, L>& sm = *reinterpret_cast<ChunkSmem<DIM, L>*>(raw);
   const int seg = blockIdx.z, h = blockIdx.y, colb = blockIdx.x * COLS;
   const int slot = p.segs[4 * seg], row0 = p.segs[4 * seg + 2], len = p.segs[4 * seg + 3];
-  if (len < SHORT) return;
+  if (len < shortest(MLSTM)) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
   const int H = p.H, vdim = p.vdim;
   const bf16* qb = p.q + (size_t)row0 * p.ldqk + (size_t)(h / (H / p.G)) * DIM;
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
     if (warp < MW) {
       const int blocks = (n + 15) >> 4;        // blocks of 16 tokens that hold any
       if (rb < blocks) {
-        float acc[4][4] = {}, rest[4][4] = {}, sc[NB][2][4] = {};      // rest: what the lower parts give, small enough to stay in the tensor cores' sums
+        float acc[4][4] = {}, rest[4][4] = {}, sc[2][NB][2][4] = {};   // rest: what the lower parts give, small enough to stay in the tensor cores' sums
         // scores of this warp's blocks (rows rb, keys share, share + WPR, ..) and its share of Q S
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
             mma_bf16_first(st[0], qf, kf[0], kf[1]);
             mma_bf16_first(st[1], qf, kf[2], kf[3]);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) sc[j][e >> 2][e & 3] += st[e >> 2][e & 3];
+            for (int e = 0; e < 8; ++e) sc[ks & 1][j][e >> 2][e & 3] += st[e >> 2][e & 3];     // two chains: half the roundings each
           }
         }
 #pragma unroll
@@ -318,7 +319,9 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
 #pragma unroll
           for (int nt = 0; nt < 2; ++nt) {
             const int s = kblk * 16 + nt * 8 + 2 * t4;
-            float* x = sc[j][nt];
+            float* x = sc[0][j][nt];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[e] += sc[1][j][nt][e];
             auto weight = [&](int t, int s_) { return MLSTM ? sm.D[b][t & 31][s_ & 31] : sm.pw[max(t - s_, 0)]; };
             x[0] = s <= ra ? x[0] * weight(ra, s) : 0.f;
             x[1] = s + 1 <= ra ? x[1] * weight(ra, s + 1) : 0.f;
@@ -475,7 +478,9 @@ bool whole_vectors(const ChunkArgs& p) {
 
 extern "C" int lia_chunk_scan_takes(int mlstm, int dim, int vdim) { return vdim > 0 && vdim % 8 == 0 && (dim == 128 || (mlstm && dim == 256)); }
 
-extern "C" int lia_chunk_scan_rows() { return SHORT; }
+extern "C" int lia_chunk_scan_rows_of(int mlstm) { return shortest(mlstm != 0); }
+
+extern "C" int lia_chunk_scan_rows() { return shortest(false); }
 
 extern "C" int lia_decay_scan_chunks(const void* q, const void* k, int ldqk, const void* v, int ldv, const float* decay, float* state_S, const int* segs, int nseg,
                                      int mixed, int H, int G, int dim, int vdim, float* o, lia_stream_t stream_) {
@@ -487,7 +492,7 @@ extern "C" int lia_decay_scan_chunks(const void* q, const void* k, int ldqk, con
               nullptr, nullptr, segs, H, G, vdim, 1.f, 0.f, o};
   LIA_CHECK_ARG(whole_vectors(p), "lia_decay_scan_chunks: rows are not whole 16-byte vectors");
   const int rc = launch_chunks<false, 128, 64>(p, nseg, stream);
-  return rc != LIA_OK || !mixed ? rc : decay_scan_tokens(q, k, ldqk, v, ldv, decay, state_S, segs, SHORT, nseg, H, G, dim, vdim, o, stream);
+  return rc != LIA_OK || !mixed ? rc : decay_scan_tokens(q, k, ldqk, v, ldv, decay, state_S, segs, shortest(false), nseg, H, G, dim, vdim, o, stream);
 }
 
 extern "C" int lia_mlstm_scan_chunks(const void* q, const void* k, const void* v, int ld, const float* gates, float* state_S, float* state_n, float* state_m,
@@ -502,6 +507,6 @@ extern "C" int lia_mlstm_scan_chunks(const void* q, const void* k, const void* v
   LIA_CHECK_ARG(whole_vectors(p), "lia_mlstm_scan_chunks: rows are not whole 16-byte vectors");
   const int rc = dim == 128 ? launch_chunks<true, 128, 32>(p, nseg, stream) : launch_chunks<true, 256, 32>(p, nseg, stream);
   if (rc != LIA_OK) return rc;
-  if (mixed) return mlstm_scan_tokens(q, k, v, ld, gates, state_S, state_n, state_m, ws, segs, SHORT, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  if (mixed) return mlstm_scan_tokens(q, k, v, ld, gates, state_S, state_n, state_m, ws, segs, shortest(true), nseg, H, dim, vdim, q_scale, den_eps, o, stream);
   return p.ws ? mlstm_take_state(p.ws, segs, nseg, state_n, state_m, H, dim, stream) : LIA_OK;
 }

@@ -396,7 +396,7 @@ def argmax_f32(logits, suppress_id=-1, out=None):
 @functools.lru_cache(maxsize=256)
 def _chunk_rows(mlstm, dim, vdim):
     lib = _lib.load()
-    return lib.lia_chunk_scan_rows() if lib.lia_chunk_scan_takes(mlstm, dim, vdim) else 0
+    return lib.lia_chunk_scan_rows_of(mlstm) if lib.lia_chunk_scan_takes(mlstm, dim, vdim) else 0
 
 
 def _in_chunks(mlstm, q, k, v, ld, ldv, dim, vdim, state_S, o, n, lengths):

@@ -152,3 +152,40 @@ def test_portions_of_unknown_lengths_in_a_larger_buffer(gated, lens):
         got.append((o, *st))
     assert torch.equal(got[0][0][:lens[0]], got[1][0]) and bool((got[0][0][lens[0]:] == 7.0).all())
     assert all(torch.equal(a, b) for a, b in zip(got[0][1:], got[1][1:])) and not torch.equal(got[0][1], start[0])
+
+
+@pytest.mark.parametrize("gated,n", [(False, 32), (False, 63), (False, 64), (False, 100), (True, 32), (True, 65)])
+def test_outputs_are_as_close_to_64_bits_as_token_by_token(gated, n):
+    """Mean over inputs: the error in chunks is no larger than that of the token loop (a measured 0.72 to 0.98 times, 1 where the loop is what runs)."""
+    H, dim, vdim, ratio = 4, 128, 128, []
+    for seed in range(6):
+        q, k, v, _, dsegs, r = _step([n], H, H, dim, vdim, seed)
+        q, k = (x if gated else torch.nn.functional.silu(x.float()).to(BF16) for x in (q, k))
+        q, k, v = torch.cat([q, k, v], 1).split([H * dim, H * dim, H * vdim], 1)
+        gates, d = torch.cat([r(n, H), torch.nn.functional.logsigmoid(r(n, H) + 2)], 1).contiguous(), torch.tensor([0.5, 0.9, 0.98, 0.996], device="cuda")
+        start, scale, err = (r(1, H, vdim, dim), r(1, H, dim), r(1, H)), dim ** -0.5, []
+        S, nn, m = (t[0].double() for t in start)
+        want = torch.empty(n, H, vdim, dtype=F64, device="cuda")
+        for t in range(n):
+            kt, qt, vt = k[t].double().view(H, dim), q[t].double().view(H, dim), v[t].double().view(H, vdim)
+            if gated:
+                i, f = gates[t].double().view(2, H)
+                new = torch.maximum(f + m, i)
+                a, b, m = torch.exp(f + m - new), torch.exp(i - new), new
+                nn = nn * a[:, None] + b[:, None] * kt
+            else:
+                a, b = d.double(), torch.ones_like(d, dtype=F64)
+            S = S * a[:, None, None] + b[:, None, None] * vt[:, :, None] * kt[:, None, :]
+            want[t] = (S @ qt[:, :, None])[..., 0]
+            if gated:
+                want[t] *= scale / (torch.maximum((nn * qt).sum(-1).abs() * scale, torch.exp(-m)) + 1e-6)[:, None]
+        for lengths in ((1, 1), (n, n)):
+            st, o = [t.clone() for t in start], torch.empty(n, H * vdim, device="cuda")
+            if gated:
+                ops.mlstm_scan(q, k, v, gates, *st, dsegs, H, dim, vdim, scale, 1e-6, o, lengths=lengths)
+            else:
+                ops.linear_scan(q, k, v, st[0], dsegs, H, H, dim, vdim, o, decay=d, lengths=lengths)
+            e = ((o.double() - want.view(n, -1)).abs() / want.view(n, -1).abs().clamp_min(1e-30)).flatten().median() if gated else _rel(o, want.view(n, -1))
+            err.append(float(e))
+        ratio.append(err[1] / err[0])
+    assert sum(ratio) / len(ratio) <= 1.01, ratio
