@@ -148,7 +148,7 @@ class LatentAttentionMixer:
     # The tensor-core form, which keeps expanded keys and values as exact as fp32 (csrc/latent_attn_mma.cu), for designs with a rotated part or a gate:
     # The portion alone decides (``_expands_exactly``), whatever else is in the step.
     EXPAND_ROWS_EXACT = 16             # fewer rows never
-    EXPAND_ROWS_ALWAYS = 64            # a block's rows: from here on whatever the history; below, its cost is that of 64 rows
+    EXPAND_WORK_ALWAYS = 128           # rows x groups of 8 heads: from here on whatever the history
     EXPAND_KEYS_EXACT = 1 << 18        # keys x heads that are held expanded at a time (1.5 KB each at 128 channels)
 
     def __init__(self, w, heads, dim, rot_dim, vdim, kv_rank, rot_dims, rot_base, scale, norm_eps, dtype, device, q_rank=None, rot_pairs=False,
@@ -250,15 +250,16 @@ class LatentAttentionMixer:
     def _expands_exactly(self, q, portions, H):
         """The portions (by number) whose latents are expanded to keys and values as exact as fp32.  A block walks a portion's keys for 64 rows of one head
         whether it has them or not, while the kernel in the latent space takes as long as rows x groups of 8 heads and splits few rows' keys over the GPU.  Time
-        of the mixer's kernels, latent space | expanded, in us: 16 heads, 16 rows that see 256 keys 93 | 85, 1024 keys 119 | 177, 33 rows that see 1024 keys 220 | 186,
-        64 rows that see 8192 keys 1842 | 1296; 4 heads, 24 rows that see 256 keys 83 | 78, 1024 keys 100 | 157.  Heads that do not fit EXPAND_KEYS_EXACT go in turn,
-        which needs enough blocks each time."""
+        of a mixer's kernels, latent space | expanded, in us, for rows that see 256, 1024, 8192 keys -- 8 heads: 24 rows 91 | 82, 109 | 161, 430 | 1228; 64 rows
+        145 | 101, 197 | 173, 1095 | 1285; 16 heads: 16 rows 93 | 85, 119 | 177, 548 | 1119; 33 rows 133 | 98, 220 | 186, 1077 | 1266; 64 rows 216 | 98, 374 | 193,
+        1842 | 1296.  Heads that do not fit EXPAND_KEYS_EXACT go in turn, which needs enough blocks each time."""
         if self.w_ukv is None or q.data_ptr() % 16 or q.stride(0) % 8:
             return ()
         found = []
         for i, (_, p0, _, n) in enumerate(portions):
             ctx = p0 + n - (max(0, p0 - self.window + 1) if self.window else 0)
-            pays = n >= self.EXPAND_ROWS_ALWAYS or 5 * ctx <= 2 * n * n * ((H + 7) // 8)
+            work = n * ((H + 7) // 8)
+            pays = work >= self.EXPAND_WORK_ALWAYS or 5 * ctx <= 2 * n * work
             heads = min(H, self.EXPAND_KEYS_EXACT // ctx)
             if n >= self.EXPAND_ROWS_EXACT and pays and (heads == H or heads * -(-n // 64) >= 128):
                 found.append(i)
