@@ -181,6 +181,7 @@ _PROTOTYPES = {
     "lia_moe_plan_rows": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "lia_moe_tc_rows": (c_int, []),
     "lia_moe_timeouts": (c_int, []),
+    "lia_moe_timeouts_seen": (c_int, []),
     "lia_moe_gemm_tc": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                 c_float, c_float, c_int, c_void_p]),
     "lia_qkv_prep_heads": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p,

@@ -14,9 +14,11 @@
 // feed-forward 742 us with one launch per expert and projection, each a quarter full, a host round trip and two more passes over bf16 sums
 // -> 196 us.  150 rows, whose experts' weights (277 MB) are the bound: 903 us on the CUDA cores -> 131 us.
 //
-// Every wait is bounded: a barrier that does not come within the limit raises a flag in shared memory, all roles leave, the loads in
-// flight are waited for, and lia_moe_timeouts() counts the launch.
+// Every wait is bounded: a barrier that does not come within the limit raises a flag in shared memory, all roles leave, what the CTA still owed becomes NaN, loads
+// and products in flight are waited for, and a word in host memory counts the CTA (lia_moe_timeouts_seen(), which the engine asks before and after its steps).
 #include <cuda.h>
+
+#include <mutex>
 
 #include "act.cuh"
 #include "common.cuh"
@@ -31,11 +33,9 @@ template <int COLS> struct Shape {
   static constexpr int A_BYTES = ROWS * KB * 2, B_BYTES = COLS * KB * 2, STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGING = 4 * 4096;                         // 32 rows of 128 bytes per epilogue warp
   static constexpr int BARS = STAGES * STAGE_BYTES + STAGING;
-  static constexpr int SMEM = BARS + (2 * STAGES + 4) * 8 + 16 + 1024;
+  static constexpr int SMEM = BARS + (2 * STAGES + 5) * 8 + 16 + 1024;
 };
 constexpr unsigned WAIT_LIMIT = 1u << 20;                          // try_wait itself sleeps for a while: seconds in all
-
-__device__ int g_timeouts;
 
 __device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t parity, volatile int* dead) {
   for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
@@ -60,6 +60,7 @@ struct MoeArgs {
   long long out_ld;
   int n_tiles, n_real, N, n_rows_w, k_blocks, act, weigh_in;       // N: output columns; n_rows_w: weight rows of an expert
   float p0, p1;
+  int* timeouts;                                                   // in host memory
 };
 
 enum { UP, UP_GATED, DOWN_PLAN, DOWN_PAIR };
@@ -80,8 +81,9 @@ __global__ void __launch_bounds__(256, 1) moe_tc_kernel(const __grid_constant__ 
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
   auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + a); };
   auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + 2 + a); };
-  volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(smem_gen + BARS + (2 * STAGES + 4) * 8);
-  volatile int* dead = reinterpret_cast<volatile int*>(smem_gen + BARS + (2 * STAGES + 4) * 8 + 8);
+  const uint32_t drain_bar = bar_base + 8u * (2 * STAGES + 4);
+  volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(smem_gen + BARS + (2 * STAGES + 5) * 8);
+  volatile int* dead = reinterpret_cast<volatile int*>(smem_gen + BARS + (2 * STAGES + 5) * 8 + 8);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -98,6 +100,7 @@ __global__ void __launch_bounds__(256, 1) moe_tc_kernel(const __grid_constant__ 
       mbar_init(tfull_bar(a), 1);
       mbar_init(tempty_bar(a), 4);
     }
+    mbar_init(drain_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {
@@ -116,10 +119,11 @@ __global__ void __launch_bounds__(256, 1) moe_tc_kernel(const __grid_constant__ 
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
   const int col_tiles = (p.N + OUT_COLS - 1) / OUT_COLS, total = used * col_tiles;
+  int issued = 0;                                                  // loads of the producer's lane
 
   if (warp == 0) {
     if (lane == 0) {
-      int stage = 0, issued = 0;
+      int stage = 0;
       uint32_t phase = 0;
       bool alive = true;
       for (int u = blockIdx.x; u < total && alive; u += gridDim.x) {
@@ -138,14 +142,6 @@ __global__ void __launch_bounds__(256, 1) moe_tc_kernel(const __grid_constant__ 
             stage = 0;
             phase ^= 1u;
           }
-        }
-      }
-      // after a timeout: the loads in flight land before the shared memory is given back
-      if (!alive) {
-        volatile int none = 0;
-        for (int i = 0; i < STAGES && i < issued; ++i) {
-          const int n = issued - 1 - i;
-          wait_for(full_bar(n % STAGES), (uint32_t)(n / STAGES) & 1u, &none);
         }
       }
     }
@@ -177,22 +173,29 @@ __global__ void __launch_bounds__(256, 1) moe_tc_kernel(const __grid_constant__ 
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
       }
-      // the last products are done before TMEM is freed: the epilogue has waited for each of them unless it gave up
-      if (*dead) {
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);
-      }
     }
   } else if (warp >= 4) {
     const int ew = warp - 4;
     const uint32_t stg = smem_base + STAGES * STAGE_BYTES + ew * 4096;
     int acc = 0;
     uint32_t acc_phase = 0;
+    bool alive = true;
     for (int u = blockIdx.x; u < total; u += gridDim.x) {
       const int tm = u / col_tiles, tn = u - tm * col_tiles;
       const int row0 = tm * ROWS + ew * 32;                        // of this warp
       const int pair = p.perm[row0 + lane];
       const float w = (pair >= 0 && ((MODE == DOWN_PAIR && p.wt != nullptr) || ((MODE == UP || GATED) && p.weigh_in))) ? p.wt[pair] : 1.0f;
-      if (!wait_for(tfull_bar(acc), acc_phase, dead)) break;
+      alive = __all_sync(0xffffffffu, alive && wait_for(tfull_bar(acc), acc_phase, dead));
+      if (!alive) {                                                // these outputs will not be: NaN, so that nobody takes them for some
+        for (int r = 0; r < 32; ++r) {
+          const int to = MODE == DOWN_PAIR ? __shfl_sync(0xffffffffu, pair, r) : row0 + r;
+          for (int col = tn * OUT_COLS + lane; to >= 0 && col < min(p.N, (tn + 1) * OUT_COLS); col += 32) {
+            if constexpr (MODE == DOWN_PAIR) reinterpret_cast<float*>(p.out)[(size_t)to * p.out_ld + col] = NAN;
+            else reinterpret_cast<bf16*>(p.out)[(size_t)to * p.out_ld + col] = __float2bfloat16_rn(NAN);
+          }
+        }
+        continue;
+      }
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + (uint32_t)(acc * COLS) + ((uint32_t)(ew * 32) << 16);
       constexpr int SLAB = MODE == DOWN_PAIR ? 32 : 64;            // columns of 128 bytes
@@ -253,7 +256,21 @@ __global__ void __launch_bounds__(256, 1) moe_tc_kernel(const __grid_constant__ 
 
   tcgen05_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && *dead) atomicAdd(&g_timeouts, 1);
+  if (*dead) {                                                     // loads and products in flight end before shared memory and TMEM are given back
+    volatile int none = 0;
+    if (threadIdx.x == 0) {
+      atomicAdd_system(p.timeouts, 1);
+      for (int i = 0; i < STAGES && i < issued; ++i) {
+        const int n = issued - 1 - i;
+        wait_for(full_bar(n % STAGES), (uint32_t)(n / STAGES) & 1u, &none);
+      }
+    }
+    if (warp == 1 && lane == 0) {
+      tcgen05_commit(drain_bar);
+      wait_for(drain_bar, 0u, &none);
+    }
+    __syncthreads();
+  }
   if (warp == 2) {
     tcgen05_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2u * COLS) : "memory");
@@ -284,12 +301,36 @@ template <int MODE> int launch(const void* W, uint64_t w_rows, int K, const CUte
 
 extern "C" int lia_moe_tc_rows(void) { return ROWS; }
 
-/* launches of lia_moe_gemm_tc that gave up a wait, since the library was loaded (synchronises) */
+namespace {
+// The word that counts CTAs whose wait ran out: host memory that every GPU can write, allocated with the first launch and kept.
+int* timeout_word(bool make) {
+  static std::mutex m;
+  static int* word = nullptr;
+  std::lock_guard<std::mutex> lock(m);
+  if (word == nullptr && make) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;     // the first launch may be part of a capture
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+      word = static_cast<int*>(p);
+      *word = 0;
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  }
+  return word;
+}
+}  // namespace
+
+/* CTAs of lia_moe_gemm_tc that gave up a wait, as far as launches have ended, since the library was loaded */
+extern "C" int lia_moe_timeouts_seen(void) {
+  const volatile int* word = timeout_word(false);
+  return word ? *word : 0;
+}
+
+/* the same after all launches (synchronises) */
 extern "C" int lia_moe_timeouts(void) {
-  int n = 0;
   LIA_CUDA(cudaDeviceSynchronize());
-  LIA_CUDA(cudaMemcpyFromSymbol(&n, g_timeouts, sizeof(int)));
-  return n;
+  return lia_moe_timeouts_seen();
 }
 
 extern "C" int lia_moe_gemm_tc(const void* A, const void* W, void* C, int c_f32, const int* perm, const int* tile_expert, int n_tiles, const float* wt, int N,
@@ -307,7 +348,8 @@ extern "C" int lia_moe_gemm_tc(const void* A, const void* W, void* C, int c_f32,
   const int rc = lia_make_tmap_2d(&tmA, A, (uint64_t)n_tiles * ROWS, K, K, ROWS);
   if (rc != LIA_OK) return rc;
   const uint64_t w_rows = (uint64_t)E * rows_w;
-  MoeArgs a{perm, tile_expert, wt, C, N, n_tiles, E, N, rows_w, (K + KB - 1) / KB, act, weigh_in, p0, p1};
+  MoeArgs a{perm, tile_expert, wt, C, N, n_tiles, E, N, rows_w, (K + KB - 1) / KB, act, weigh_in, p0, p1, timeout_word(true)};
+  LIA_CHECK_ARG(a.timeouts != nullptr, "lia_moe_gemm_tc: no host memory for the count of timeouts");
   if (up) return gated ? launch<UP_GATED>(W, w_rows, K, tmA, a, stream) : launch<UP>(W, w_rows, K, tmA, a, stream);
   if (!c_f32) return launch<DOWN_PLAN>(W, w_rows, K, tmA, a, stream);
   if (weigh_in) a.wt = nullptr;

@@ -22,7 +22,7 @@ step-wise models need.
 import numpy as np
 import torch
 
-from . import graphs, ops
+from . import _lib, graphs, ops
 from .seq_layers import StepBatch
 
 
@@ -44,6 +44,15 @@ class Engine:
         self.slots = model.new_state(int(max_requests), int(max_tokens))
         self.device = model.device
         self._host = self._copied = None
+        self._timeouts = ops.moe_timeouts_seen()
+
+    def check(self):
+        """Raise if a kernel of an earlier step gave up a wait: the logits of that step, and the state it left, hold NaN.  Steps ask by themselves before they begin,
+        ``generate`` also after it has read a step's tokens; a caller who reads logits may ask then."""
+        seen = ops.moe_timeouts_seen()
+        if seen != self._timeouts:
+            new, self._timeouts = seen - self._timeouts, seen
+            raise _lib.LiaError(f"{new} blocks of an experts' projection gave up waiting: results of this engine since its last check hold NaN")
 
     # ---- batch assembly: one pinned staging buffer, one H2D copy per pass
     def _upload(self, ids, segs, meta, want, static=None):
@@ -124,6 +133,7 @@ class Engine:
     def step(self, entries, end=(), trace=None):
         """entries: dicts ``{"id", "tokens", "want"}``; returns fp32 logits [wanted places, vocab] in the order of the entries
         and of their ``want`` lists (None if nothing is wanted)."""
+        self.check()
         vocab = self.model.config.vocab
         todo, restore = [], []
         for e in entries:
@@ -194,13 +204,16 @@ class Engine:
             logits = self.step(entries)
             if logits is not None:
                 picks = ops.argmax_f32(logits, suppress_id).tolist()
+                self.check()
                 for e, tok in zip([e for e in entries if e["want"]], picks):
                     nxt[e["id"]] = tok
         for i in ids:
             out[i].append(nxt[i])
         for _ in range(max_new_tokens - 1):
             logits = self.step([{"id": i, "tokens": [out[i][-1]], "want": [0]} for i in ids])
-            for i, tok in zip(ids, ops.argmax_f32(logits, suppress_id).tolist()):
+            picks = ops.argmax_f32(logits, suppress_id).tolist()
+            self.check()
+            for i, tok in zip(ids, picks):
                 out[i].append(tok)
         for i in ids:
             self.slots.free(i)

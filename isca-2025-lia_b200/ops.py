@@ -688,6 +688,11 @@ def moe_gemm_tc(a, w, out, perm, tile_expert, wt, up, act=ACT_NONE, gated=False,
     return out
 
 
+def moe_timeouts_seen():
+    """Blocks of ``moe_gemm_tc`` that gave up a wait in any launch that has ended (their results are NaN).  Does not synchronise."""
+    return _lib.load().lia_moe_timeouts_seen()
+
+
 def moe_gemm(a, w, out, idx, wt, top, up, act=ACT_NONE, perm=None, tile_expert=None, gated=False, act_params=(0.0, 0.0), weigh_in=False):
     """One projection of every expert over its own rows; ``w`` [E, N, K].  up: out[place] = act(a[token] @ w[e].T);
     down: out[pair] = wt[pair] * a[place] @ w[e].T (fp32).  Without a plan (``perm`` None) a pair's place is the pair.
