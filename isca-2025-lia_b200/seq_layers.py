@@ -811,7 +811,7 @@ class MoEFeedForward:
     # width 4096: 16 pairs 266 | 270 us, 40 pairs 541 | 276 us; width 1024, 18 pairs (78 MB): 75 | 107 us.
     FEW_BYTES = 400 << 20
     FEW_PAIRS = 48
-    TENSOR_CORE_PAIRS = 512   # from here the experts' outputs are rounded to bf16 before they are weighted and added
+    TENSOR_CORE_PAIRS = 512   # from here the experts' outputs are rounded to bf16 before they are weighted and added, but not in captured (decoding) steps
 
     def __init__(self, router_w, experts_w, top, ff, act, shared, dtype, device, correction=None, renorm=True, identity=0, act_params=(0.0, 0.0),
                  score="softmax", weigh="output", shared_gate=None, groups=None):
@@ -846,7 +846,8 @@ class MoEFeedForward:
 
     def _experts_tensor_core(self, h, idx, wt, y, shared_gate):
         """The pairs grouped by expert (tiles of 128 rows), the rows gathered into that order, then one tensor-core launch per projection
-        over all experts (csrc/moe_sm100.cu).  The experts' outputs are kept by pair in fp32, or from TENSOR_CORE_PAIRS pairs on in the plan's order in bf16."""
+        over all experts (csrc/moe_sm100.cu).  The experts' outputs are kept by pair in fp32, or in an eager step from TENSOR_CORE_PAIRS pairs on in the plan's
+        order in bf16."""
         M, W = h.shape
         R, top, ff, dev = self.R, self.top, self.ff, h.device
         pairs = M * top
@@ -861,7 +862,7 @@ class MoEFeedForward:
         ops.moe_gemm_tc(xs, self.w_up, mid, perm, tile_expert, wt, True, self.act, gated=self.gated, act_params=self.act_params, weigh_in=self.weigh_in)
         shared = self.shared(h) if self.shared is not None else None
         identity = (idx, self.E, h, wt) if self.identity else None
-        if pairs >= self.TENSOR_CORE_PAIRS:
+        if pairs >= self.TENSOR_CORE_PAIRS and not torch.cuda.is_current_stream_capturing():
             ys = torch.empty(n_tiles * tm, W, dtype=self.dtype, device=dev)
             ops.moe_gemm_tc(mid, self.w_down, ys, perm, tile_expert, wt, False)
             ops.moe_combine(ys, shared, y, top, pos_of=pos_of, wt=None if self.weigh_in else wt, identity=identity, weighted=self.weigh_in, shared_gate=shared_gate)

@@ -99,3 +99,25 @@ def test_a_plan_in_a_larger_buffer():
     assert torch.equal(plans[0], plans[1]) and torch.equal(plans[0], plans[2])
     with pytest.raises(_lib.LiaError):
         ops.moe_plan(idx, E, torch.empty(n_tiles * tm - 1, **i32), torch.empty(n_tiles, **i32), torch.empty(idx.numel(), **i32))
+
+
+def test_captured_steps_keep_the_experts_outputs_in_fp32(monkeypatch):
+    """However many pairs a captured (decoding) step has: the form that fewer pairs take, bit for bit."""
+    from lia_b200.seq_layers import MoEFeedForward
+    g = torch.Generator().manual_seed(2)
+    E, top, W, ff, M = 4, 2, 64, 72, 300
+
+    def r(*s):
+        return torch.randn(*s, generator=g) * s[-1] ** -0.5
+    experts = [{"gate": r(ff, W), "up": r(ff, W), "down": r(W, ff)} for _ in range(E)]
+    m, h = MoEFeedForward(r(E, W), experts, top, ff, ops.ACT_SILU, None, BF16, DEV), torch.randn(M, W, generator=g).to(BF16).to(DEV)
+    assert M * top >= MoEFeedForward.TENSOR_CORE_PAIRS
+    m(h)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = m(h)
+    graph.replay()
+    eager = m(h)
+    monkeypatch.setattr(MoEFeedForward, "TENSOR_CORE_PAIRS", 1 << 30)
+    want = m(h)
+    assert torch.equal(got, want) and not torch.equal(eager, want)
