@@ -118,7 +118,7 @@ template <int DK, int DV, int NQ> struct PromptShape {
 };
 
 // NQ = 1: bf16 queries; 3: fp32 queries in three parts.  segs[s] = {slot, first position, first row, rows}; null: one portion that meta's first
-// row begins.  blockIdx.y counts the portions' tiles from the last to the first: the longest histories start first.
+// row begins (tiles whose rows do not continue it are taken row by row).  blockIdx.y counts the portions' tiles from the last to the first: the longest histories start first.
 template <int DK, int DV, int NQ>
 __global__ void __launch_bounds__(128, (DV <= 128 && NQ == 1) ? 3 : 2) window_prompt_kernel(const void* __restrict__ q, int ldq, const bf16* __restrict__ kcache, long long k_slot_stride,
                                                             const bf16* __restrict__ vcache, long long v_slot_stride, const int* __restrict__ meta,
@@ -158,10 +158,30 @@ __global__ void __launch_bounds__(128, (DV <= 128 && NQ == 1) ? 3 : 2) window_pr
   row0 += tile * BM;
   pos0 += tile * BM;
   rows = min(BM, rows - tile * BM);
+  const size_t k_stride = (size_t)a.G * DK, v_stride = (size_t)Gv * DV;
+  const float mul = a.scale * (x.temp ? x.temp[h] : 1.0f), slope = x.slopes ? x.slopes[h] : 0.f;
+  auto by_itself = [&](size_t row, int slot_, int pos) {               // one row by one warp
+    const PlainRow<DV> y = plain_row<DK, DV, NQ>(q, row * ldq + (size_t)h * DK, kcache + (size_t)slot_ * k_slot_stride + (size_t)kg * DK, k_stride,
+                                                 vcache + (size_t)slot_ * v_slot_stride + (size_t)vg * DV, v_stride, first_key(a, pos), pos, pos, mul, slope, a.softcap);
+    const float invl = 1.0f / (y.l + (x.sink ? expf(x.sink[h] - y.m) : 0.f));
+#pragma unroll
+    for (int c = 0; c < DV / 32; ++c) {
+      const int ch = lane + 32 * c;
+      store_out(out, (row * a.H + h) * DV + ch, y.o[c] * invl * gate_of<bf16>(x, a, row, h, ch), a);
+    }
+  };
+  if (segs == nullptr) {                                 // what meta says counts: rows that do not continue one sequence go one by one
+    bool run = true;
+    if ((int)threadIdx.x < rows) run = meta[2 * (row0 + threadIdx.x)] == slot && meta[2 * (row0 + threadIdx.x) + 1] == pos0 + (int)threadIdx.x;
+    if (!__syncthreads_and(run)) {
+#pragma unroll 1
+      for (int r = warp; r < rows; r += 4) by_itself(row0 + r, meta[2 * (row0 + r)], meta[2 * (row0 + r) + 1]);
+      return;
+    }
+  }
   const int pos_last = pos0 + rows - 1, jb = first_key(a, pos0);
   const bf16* kc = kcache + (size_t)slot * k_slot_stride + (size_t)kg * DK;
   const bf16* vc = vcache + (size_t)slot * v_slot_stride + (size_t)vg * DV;
-  const size_t k_stride = (size_t)a.G * DK, v_stride = (size_t)Gv * DV;
   load_tile<DK, BK>(ks, kc, k_stride, jb, pos_last);
   load_tile<DV, BK>(vs, vc, v_stride, jb, pos_last);
   cp_async_commit();
@@ -192,7 +212,6 @@ __global__ void __launch_bounds__(128, (DV <= 128 && NQ == 1) ? 3 : 2) window_pr
                    "r"(part[s][2]), "r"(part[s][3]) : "memory");
   }
 
-  const float mul = a.scale * (x.temp ? x.temp[h] : 1.0f), slope = x.slopes ? x.slopes[h] : 0.f;
   const int wpos = pos0 + warp * 16;                     // position of the warp's first row
   const bool warp_on = warp * 16 < rows;
   float O[DV / 8][4], m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
@@ -326,14 +345,7 @@ __global__ void __launch_bounds__(128, (DV <= 128 && NQ == 1) ? 3 : 2) window_pr
 #pragma unroll 1
   for (int i = 0; i < 16; ++i) {
     if ((((i < 8 ? again[0] : again[1]) >> (4 * (i & 7))) & 15u) == 0u) continue;
-    const size_t row = row0 + warp * 16 + i;
-    const PlainRow<DV> y = plain_row<DK, DV, NQ>(q, row * ldq + (size_t)h * DK, kc, k_stride, vc, v_stride, first_key(a, wpos + i), wpos + i, wpos + i, mul, slope, a.softcap);
-    const float invl = 1.0f / (y.l + (x.sink ? expf(x.sink[h] - y.m) : 0.f));
-#pragma unroll
-    for (int c = 0; c < DV / 32; ++c) {
-      const int ch = (int)(threadIdx.x & 31) + 32 * c;
-      store_out(out, (row * a.H + h) * DV + ch, y.o[c] * invl * gate_of<bf16>(x, a, row, h, ch), a);
-    }
+    by_itself(row0 + warp * 16 + i, slot, wpos + i);
   }
 }
 

@@ -111,3 +111,18 @@ def test_what_the_general_kernel_keeps():
     wide[:, 4:] = q
     ops.window_attn(wide[:, 4:], kc, vc, meta, None, out, 2, 2, 128, 128, 0, 0.1, 0.0, nseg=1, max_ctx=70)
     assert float((out.cpu().to(F64) - want.reshape(out.shape)).abs().max() / want.abs().max()) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("q_f32", [False, True])
+@pytest.mark.parametrize("at", [[(0, 5), (1, 69)], [(0, 69), (0, 68), (0, 0)], None])
+def test_one_portion_announced_whose_rows_are_others(q_f32, at):
+    """Without segments `nseg` is advice: a row's slot and position come from meta alone, up to the caches' last rows."""
+    H, G, d, cap, M = 4, 2, 64, 70, 130
+    g = torch.Generator().manual_seed(4)
+    q = torch.randn(M, H * d, generator=g).to(F32 if q_f32 else BF16).to(DEV)
+    kc, vc = (torch.randn(2, cap, G * d, generator=g).to(BF16).to(DEV) for _ in range(2))
+    rows = [(at * M)[i] if at else (i % 2, (7 * i) % cap) for i in range(M)]
+    out = torch.empty(M, H * d, dtype=F32, device=DEV)
+    ops.window_attn(q, kc, vc, torch.tensor(rows, dtype=torch.int32, device=DEV), None, out, H, G, d, d, 33, 0.1, 0.0, nseg=1, max_ctx=cap)
+    want = reference(q, kc, vc, [(s, p, r, 1) for r, (s, p) in enumerate(rows)], H, G, d, d, 0.1, window=33)
+    assert float((out.cpu().to(F64) - want.reshape(out.shape)).abs().max() / want.abs().max()) < TOL
