@@ -604,53 +604,53 @@ __global__ void __launch_bounds__(128) linear_small_kernel(const TA* __restrict_
   const int row0 = blockIdx.x * R, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool va = vec_ok(a, lda), vw = vec_ok(w, K);
   for (int n0 = blockIdx.y * 8; n0 < N; n0 += gridDim.y * 8) {
-  float acc[R][8];
+    float acc[R][8];
 #pragma unroll
-  for (int r = 0; r < R; ++r)
+    for (int r = 0; r < R; ++r)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[r][j] = 0.f;
-  for (int k = threadIdx.x * 8; k < K; k += 128 * 8) {
-    float av[R][8], wv[8];
+      for (int j = 0; j < 8; ++j) acc[r][j] = 0.f;
+    for (int k = threadIdx.x * 8; k < K; k += 128 * 8) {
+      float av[R][8], wv[8];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      if (row0 + r < M) {
-        load8(a + (size_t)(row0 + r) * lda, k, K, va, av[r]);
-      } else {
+      for (int r = 0; r < R; ++r) {
+        if (row0 + r < M) {
+          load8(a + (size_t)(row0 + r) * lda, k, K, va, av[r]);
+        } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) av[r][i] = 0.f;
+          for (int i = 0; i < 8; ++i) av[r][i] = 0.f;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (n0 + j < N) {
+          load8(w + (size_t)(n0 + j) * K, k, K, vw, wv);
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[r][j] = fmaf(av[r][i], wv[i], acc[r][j]);
+        }
       }
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (n0 + j < N) {
-        load8(w + (size_t)(n0 + j) * K, k, K, vw, wv);
+    for (int r = 0; r < R; ++r)
 #pragma unroll
-        for (int r = 0; r < R; ++r)
-#pragma unroll
-          for (int i = 0; i < 8; ++i) acc[r][j] = fmaf(av[r][i], wv[i], acc[r][j]);
+      for (int j = 0; j < 8; ++j) {
+        acc[r][j] = warp_sum(acc[r][j]);
+        if (lane == 0) part[warp][r][j] = acc[r][j];
       }
+    __syncthreads();
+    const int r = threadIdx.x >> 3, n = n0 + (threadIdx.x & 7), j = threadIdx.x & 7;
+    if (r < R && row0 + r < M && n < N) {
+      float z = ((part[0][r][j] + part[1][r][j]) + (part[2][r][j] + part[3][r][j])) + (bias ? bias[n] : 0.f);
+      if (mode == 1) {
+        z = cap * tanhf(z / cap);
+        if (n >= N / 2) z = log_sigmoid(z);
+      } else if (mode == 2) {
+        z = 1.0f / (1.0f + expf(-z));
+      }
+      out[(size_t)(row0 + r) * N + n] = z;
     }
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      acc[r][j] = warp_sum(acc[r][j]);
-      if (lane == 0) part[warp][r][j] = acc[r][j];
-    }
-  __syncthreads();
-  const int r = threadIdx.x >> 3, n = n0 + (threadIdx.x & 7), j = threadIdx.x & 7;
-  if (r < R && row0 + r < M && n < N) {
-    float z = ((part[0][r][j] + part[1][r][j]) + (part[2][r][j] + part[3][r][j])) + (bias ? bias[n] : 0.f);
-    if (mode == 1) {
-      z = cap * tanhf(z / cap);
-      if (n >= N / 2) z = log_sigmoid(z);
-    } else if (mode == 2) {
-      z = 1.0f / (1.0f + expf(-z));
-    }
-    out[(size_t)(row0 + r) * N + n] = z;
-  }
-  __syncthreads();                          // `part` may be overwritten
+    __syncthreads();                          // `part` may be overwritten
   }
 }
 

@@ -798,8 +798,8 @@ extern "C" int lia_moe_gather(const void* src, int act_f32, const int* perm, voi
   return LIA_OK;
 }
 
-// The tensor-core form: every expert's contiguous rows of the gathered input through lia_gemm_bf16, one launch per expert that has
-// rows, issued from here so that the launches follow each other without a trip through the caller's interpreter.
+// For callers who know the rows per expert on the host (published interface; the feed-forward takes lia_moe_gemm_tc): every expert's contiguous rows
+// of the gathered input through lia_gemm_bf16, one launch per expert that has rows, issued back to back from here.
 extern "C" int lia_moe_expert_gemms(const void* A, const void* W, long long w_expert_stride, void* C, const int* tiles_per_expert, int E,
                                     int tile_rows, int N, int K, void* workspace, size_t workspace_bytes, lia_stream_t stream_) {
   LIA_CHECK_ARG(A && W && C && tiles_per_expert && E > 0 && tile_rows > 0 && N > 0 && K > 0, "lia_moe_expert_gemms: bad arguments");
@@ -838,7 +838,7 @@ extern "C" int lia_moe_combine_gated(const void* ypair, int ypair_f32, const int
   LIA_CHECK_ARG(!shared_gate || (shared && ldg >= 1), "lia_moe_combine: a gate without a shared expert");
   LIA_CHECK_ARG(!idx || (h && wt && n_real >= 0), "lia_moe_combine: identity experts need the routing weights and the experts' input");
   const unsigned blocks = capped_blocks((size_t)M * W);
-const uintptr_t addr = reinterpret_cast<uintptr_t>(ypair) | reinterpret_cast<uintptr_t>(shared) | reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(y);
+  const uintptr_t addr = reinterpret_cast<uintptr_t>(ypair) | reinterpret_cast<uintptr_t>(shared) | reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(y);
   if (W % 4 == 0 && addr % 16 == 0) {
 #define LIA_MCV(TY, TS) lia_launch(moe_combine_vec_kernel<TY, TS>, dim3(M), dim3(256), 0, stream, reinterpret_cast<const TY*>(ypair), pos_of, wt, reinterpret_cast<const TS*>(shared), y, W, top, idx, n_real, reinterpret_cast<const TS*>(h), weighted, shared_gate, ldg)
     if (ypair_f32 && act_f32) LIA_MCV(float, float);

@@ -121,3 +121,18 @@ def test_captured_steps_keep_the_experts_outputs_in_fp32(monkeypatch):
     monkeypatch.setattr(MoEFeedForward, "TENSOR_CORE_PAIRS", 1 << 30)
     want = m(h)
     assert torch.equal(got, want) and not torch.equal(eager, want)
+
+
+def test_expert_gemms_of_the_published_interface():
+    """lia_moe_expert_gemms, a GEMM per expert for callers who know the rows per expert on the host: the feed-forward itself takes one launch for all."""
+    g = torch.Generator().manual_seed(1)
+    E, N, K, counts, tm = 3, 72, 64, [1, 0, 3], 64
+    rows = sum(counts) * tm
+    a, w = torch.randn(rows, K, generator=g).to(BF16), (torch.randn(E, N, K, generator=g) * K ** -0.5).to(BF16)
+    out = torch.empty(rows, N, dtype=BF16, device=DEV)
+    ops.moe_expert_gemms(a.to(DEV), w.to(DEV), out, counts, tm, ops.GemmWorkspace(ops.GemmWorkspace.bytes_for([(n * tm, N, K) for n in counts if n]), DEV))
+    want, at = torch.empty(rows, N, dtype=F64), 0
+    for e, n in enumerate(counts):
+        want[at:at + n * tm] = a[at:at + n * tm].to(F64) @ w[e].to(F64).T
+        at += n * tm
+    assert bool(((out.cpu().to(F64) - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all())        # one rounding of a result made in fp32
