@@ -724,7 +724,8 @@ def moe_gather(src, perm, dst, top):
 
 
 def moe_expert_gemms(a, w, out, tiles_per_expert, tile_rows, workspace):
-    """out[rows of e] = a[rows of e] @ w[e].T on the tensor-core GEMM, expert after expert: expert e owns the next
+    """(For callers who know the rows per expert on the host; ``MoEFeedForward`` takes ``moe_gemm_tc``.)  out[rows of e] = a[rows of e] @ w[e].T on the
+    tensor-core GEMM, expert after expert: expert e owns the next
     ``tiles_per_expert[e] * tile_rows`` rows of ``a`` and ``out`` (bf16; ``tiles_per_expert`` is a host list)."""
     _req(a, "a"); _req(w, "w"); _req(out, "out")
     E, N, K = w.shape
