@@ -21,7 +21,7 @@ import time
 
 import torch
 
-from . import ops
+from . import _lib, ops
 
 BF16 = torch.bfloat16
 
@@ -30,8 +30,15 @@ def _nbytes(*ts):
     return sum(t.numel() * t.element_size() for t in ts if t is not None)
 
 
+def _in_chunks(mlstm, q, dim, vdim, lengths):
+    """Whether the longest portion of a matrix-state recurrence goes in chunks on the tensor cores (csrc/chunk_scan.cu)."""
+    lib = _lib.load()
+    return q.dtype == BF16 and bool(lib.lia_chunk_scan_takes(mlstm, dim, vdim)) and (lengths or (0, q.shape[0]))[1] >= lib.lia_chunk_scan_rows_of(mlstm)
+
+
 def _cost(name, a, kw):
-    """(flops, bytes, kind) of one call; kind: 'tc' tensor-core GEMM, 'f32' CUDA-core fp32 arithmetic, 'mem' memory-bound."""
+    """(flops, bytes, kind) of one call; kind: 'tc' tensor cores (the products of the definition, however many the form takes: fp32 operands in
+    three bf16 parts are three to six each), 'f32' CUDA-core fp32 arithmetic, 'mem' memory-bound."""
     if name == "gemm":
         x, w = a[0], a[1]
         M, K, N = x.shape[0], x.shape[1], w.shape[0]
@@ -42,7 +49,8 @@ def _cost(name, a, kw):
         K = kw.get("k") or x.shape[1]
         N = kw.get("n") or out.shape[1]
         M = x.shape[0]
-        return 2.0 * b * M * N * K, M * b * K * x.element_size() + _nbytes(w) + M * b * N * out.element_size(), "f32"
+        kind = "tc" if M > 64 and K % 8 == 0 and (x.dtype != BF16 or w.dtype == BF16) else "f32"       # csrc/linear_mma.cu
+        return 2.0 * b * M * N * K, M * b * K * x.element_size() + _nbytes(w) + M * b * N * out.element_size(), kind
     if name == "linear_small":
         x, w, out = a[0], a[1], a[3]
         return 2.0 * x.shape[0] * w.shape[0] * w.shape[1], _nbytes(x, w, out), "mem"
@@ -50,7 +58,15 @@ def _cost(name, a, kw):
         q, S, segs, H, dim, vdim, o = a[0], a[4], a[7], a[8], a[9], a[10], a[13]
         M = q.shape[0]
         state = 2.0 * segs.shape[0] * H * dim * vdim * 4
-        return 4.0 * M * H * dim * vdim, state + M * H * (2 * dim + vdim) * q.element_size() + _nbytes(o), "f32"
+        return 4.0 * M * H * dim * vdim, state + M * H * (2 * dim + vdim) * q.element_size() + _nbytes(o), "tc" if _in_chunks(1, q, dim, vdim, kw.get("lengths")) else "f32"
+    if name == "latent_attn_expanded":
+        q, portions, w, out, H, dim, rot, rank = a[0], a[3], a[4], a[6], a[7], a[8], a[9], a[10]
+        win = kw.get("window", 0) or 1 << 30
+        keys = sum(min(win, p0 + i + 1) for _, p0, _, n in portions for i in range(n))
+        latents = sum(p0 + n - max(0, p0 - win + 1) for _, p0, _, n in portions)
+        rows = sum(n for _, _, _, n in portions)
+        return (2.0 * keys * H * (2 * dim + rot) + 4.0 * latents * H * dim * rank,
+                rows * (q.shape[1] * q.element_size() + H * rot * 4 + out.shape[1] * out.element_size()) + latents * (rank + rot) * 2 + _nbytes(w), "tc")
     if name == "latent_attn":
         qa, cache, meta, out, H, rank, rot = a[0], a[1], a[2], a[4], a[5], a[6], a[7]
         win = kw.get("window", 0) > 0
@@ -67,7 +83,8 @@ def _cost(name, a, kw):
         M = q.shape[0]
         state = 2.0 * segs.shape[0] * H * dim * vdim * 4
         per_token = 8.0 if kw.get("gates") is not None else 4.0                    # delta: two dot products and two updates per cell
-        return per_token * M * H * dim * vdim, state + M * (2 * G * dim + H * vdim) * q.element_size() + _nbytes(o), "f32"
+        chunks = kw.get("decay") is not None and not kw.get("in_silu") and _in_chunks(0, q, dim, vdim, kw.get("lengths"))
+        return per_token * M * H * dim * vdim, state + M * (2 * G * dim + H * vdim) * q.element_size() + _nbytes(o), "tc" if chunks else "f32"
     if name == "forget_scan":
         q, S, segs, H, dim, vdim, o = a[0], a[3], a[4], a[5], a[6], a[7], a[8]
         M = q.shape[0]
@@ -75,7 +92,8 @@ def _cost(name, a, kw):
     if name == "window_attn":
         q, kc, out, H, G, dim, vdim = a[0], a[1], a[5], a[6], a[7], a[8], a[9]
         keys = float(kw.get("_wkeys", 0))                                          # sum over rows of keys inside the window
-        return 2.0 * keys * H * (dim + vdim), _nbytes(q, out) + kw.get("_wctx", 0) * G * (dim + vdim) * kc.element_size(), "f32"
+        kind = "tc" if kc.dtype == BF16 and dim in (64, 128) and vdim in (64, 128, 256) else "f32"             # csrc/window_attn_mma.cu
+        return 2.0 * keys * H * (dim + vdim), _nbytes(q, out) + kw.get("_wctx", 0) * G * (dim + vdim) * kc.element_size(), kind
     if name == "qkv_prep":
         y, q_out, kc, vc = a[0], a[3], a[4], a[5]
         M = y.shape[0]
@@ -118,6 +136,11 @@ def _cost(name, a, kw):
         touched = min(w.shape[0], pairs)
         kind = "tc" if x.dtype == BF16 and pairs > 64 else "mem"
         return 2.0 * pairs * N * K, pairs * (K * x.element_size() + N * out.element_size()) + touched * N * K * w.element_size(), kind
+    if name == "moe_gemm_tc":
+        w, out, wt = a[1], a[2], a[5]
+        pairs, (E, N, K) = wt.numel(), w.shape
+        n_out = N // 2 if kw.get("gated") else N
+        return 2.0 * pairs * N * K, pairs * (K * 2.0 + n_out * out.element_size()) + min(E, pairs) * N * K * 2.0, "tc"
     if name == "moe_expert_gemms":
         x, w, counts, tm = a[0], a[1], a[3], a[4]
         rows, N, K = sum(counts) * tm, w.shape[1], w.shape[2]
@@ -135,10 +158,10 @@ def _cost(name, a, kw):
 
 
 class Instrument:
-    NAMES = ("gemm", "linear_plain", "linear_small", "mlstm_scan", "headnorm_gate", "latent_prep", "latent_attn", "clamped_glu",
+    NAMES = ("gemm", "linear_plain", "linear_small", "mlstm_scan", "headnorm_gate", "latent_prep", "latent_attn", "latent_attn_expanded", "clamped_glu",
              "rms_add_norm", "embed_rmsnorm", "rms_gather", "layernorm", "attn_prefill", "attn_decode", "embed", "argmax", "argmax_f32",
              "linear_scan", "conv_prep", "conv_state_update", "kv_store", "window_attn", "ln_add_norm", "embed_rows", "ln_gather", "gated_act",
-             "router_topk", "moe_plan", "moe_gemm", "moe_gather", "moe_expert_gemms", "moe_combine", "qkv_prep", "gated_rms_add", "poly_norm",
+             "router_topk", "moe_plan", "moe_gemm", "moe_gemm_tc", "moe_gather", "moe_expert_gemms", "moe_combine", "qkv_prep", "gated_rms_add", "poly_norm",
              "embed_scale_pos", "residual_norm", "rms_norm_rows", "sigmoid_mul", "softcap", "forget_gate_prep", "forget_scan", "diff_combine",
              "latent_store", "embed_bigram_pos", "streams_update", "streams_embed", "streams_gather", "conv_act", "ssd_scan", "rglru_scan", "silu_gate_norm")
 
