@@ -8,7 +8,7 @@
 // One block per (64 rows, head), warp by 16 rows, the scores becoming the weights' operand in registers; 32 keys per stage.  Keys and values
 // are fetched in turn (the next keys while the values are taken in, the next values while the scores are made), so one stage of 52 KB
 // is enough and two blocks share an SM.  Bound: tensor cores and shared-memory reads about equally.  2048 tokens, 16 heads of 128 + 64 on latents
-// of 512: 4794 us in the latent space on the CUDA cores and 439 us for its two projections -> 329 and 67 us for the expansion.
+// of 512: 4794 us in the latent space on the CUDA cores and 439 us for its two projections -> 352 and 67 us for the expansion.
 // Rows whose sums are not finite are formed again key by key at the end, as in window_attn_mma.cu: a masked key's weight of 0 still meets its value.
 #include <limits.h>
 #include <math.h>
