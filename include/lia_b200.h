@@ -292,11 +292,11 @@ int lia_mlstm_scan_ws(const void* q, const void* k, const void* v, int act_f32, 
                       float* ws, lia_stream_t stream);
 /* the same recurrence, and that of lia_linear_scan with a fixed decay, for long portions in bf16: chunks of tokens on the tensor cores.  Takes a dim of 128 (and
  * 256 for lia_mlstm_scan_chunks), a vdim that is a multiple of 8 (lia_chunk_scan_takes) and rows of whole 16-byte vectors.  Portions of fewer than
- * lia_chunk_scan_rows_of(..) tokens go token by token, in a launch of their own that `mixed` asks for (0: there are none); lia_chunk_scan_rows() is the larger
- * of both recurrences' limits */
+ * lia_chunk_scan_rows() tokens go token by token, in a launch of their own that `mixed` asks for (0: there are none).  With a fixed decay
+ * those of fewer than lia_chunk_scan_few() tokens have a launch of their own as well; mixed & 2: there are none, mixed & 4: there are no longer ones */
 int lia_chunk_scan_takes(int mlstm, int dim, int vdim);
 int lia_chunk_scan_rows(void);
-int lia_chunk_scan_rows_of(int mlstm);
+int lia_chunk_scan_few(void);
 int lia_mlstm_scan_chunks(const void* q, const void* k, const void* v, int ld, const float* gates, float* state_S, float* state_n, float* state_m,
                           const int* segs, int nseg, int mixed, int H, int dim, int vdim, float q_scale, float den_eps, float* o, float* ws,
                           lia_stream_t stream);

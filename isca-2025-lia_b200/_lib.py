@@ -100,7 +100,7 @@ _PROTOTYPES = {
                                c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p, c_void_p]),
     "lia_chunk_scan_takes": (c_int, [c_int, c_int, c_int]),
     "lia_chunk_scan_rows": (c_int, []),
-    "lia_chunk_scan_rows_of": (c_int, [c_int]),
+    "lia_chunk_scan_few": (c_int, []),
     "lia_mlstm_scan_chunks": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                       c_int, c_int, c_float, c_float, c_void_p, c_void_p, c_void_p]),
     "lia_decay_scan_chunks": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,

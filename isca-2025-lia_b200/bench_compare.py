@@ -33,7 +33,7 @@ def _nbytes(*ts):
 def _in_chunks(mlstm, q, dim, vdim, lengths):
     """Whether the longest portion of a matrix-state recurrence goes in chunks on the tensor cores (csrc/chunk_scan.cu)."""
     lib = _lib.load()
-    return q.dtype == BF16 and bool(lib.lia_chunk_scan_takes(mlstm, dim, vdim)) and (lengths or (0, q.shape[0]))[1] >= lib.lia_chunk_scan_rows_of(mlstm)
+    return q.dtype == BF16 and bool(lib.lia_chunk_scan_takes(mlstm, dim, vdim)) and (lengths or (0, q.shape[0]))[1] >= lib.lia_chunk_scan_rows()
 
 
 def _cost(name, a, kw):

@@ -38,9 +38,12 @@ constexpr int VP = COLS + 8;                   // row pitches in bf16 (16 bytes 
 constexpr int OP = COLS + 4;                   // and of the output parts in floats
 // A portion of fewer tokens is left to the token loops, whichever portions come with it (a portion's rounding must not depend on its company).  One portion of 24 tokens:
 // 13 us there and 10 here, of 32: 14 and 11, 8 of 33: 44 and 29; but 16 of one token: 6 and 47, for a CTA fills an SM and its chunk costs the same few
-// us however little it holds.  A prompt of 256 among 31 single tokens: 90 us all by tokens, 90 all in chunks, 42 split.  With a fixed decay the outputs of 32 to 63
-// tokens would be off by 1.02 to 1.08 times what the token loop's few roundings give (64 tokens: 0.98, 100: 0.92), so there the line is 64.
-__host__ __device__ constexpr int shortest(bool mlstm) { return mlstm ? 32 : 64; }
+// us however little it holds.  A prompt of 256 among 31 single tokens: 90 us all by tokens, 90 all in chunks, 42 split.
+constexpr int SHORT = 32;
+// Below this many tokens with a fixed decay the token loop rounds so little that scores summed in two chains would leave the outputs off by 1.02 to 1.08 times its error:
+// they are summed with their rounding errors, 0.93 to 0.98 times, by a kernel of their own (from here on two chains: 0.98 at 64 tokens, 0.92 at 100; the errors kept for
+// all portions: 28 us more of 216 for 2048 tokens, both ways in one kernel: 5).
+constexpr int FEW = 64;
 
 struct ChunkArgs {
   const bf16 *q, *k, *v;
@@ -68,8 +71,8 @@ template <int DIM, int L> struct ChunkSmem {
   alignas(16) int bad[2][COLS];                            // first token whose v is not finite
 };
 
-// MLSTM: gates per token with a running-maximum stabiliser and a normaliser; else one decay per head.
-template <bool MLSTM, int DIM, int L>
+// MLSTM: gates per token with a running-maximum stabiliser and a normaliser; else one decay per head, and the portions of SHORT to FEW - 1 tokens (few) or those of FEW and more.
+template <bool MLSTM, int DIM, int L, bool few = false>
 __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(ChunkArgs p) {
   pdl_launch_dependents();
   pdl_wait();
@@ -78,7 +81,7 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
   ChunkSmem<DIM, L>& sm = *reinterpret_cast<ChunkSmem<DIM, L>*>(raw);
   const int seg = blockIdx.z, h = blockIdx.y, colb = blockIdx.x * COLS;
   const int slot = p.segs[4 * seg], row0 = p.segs[4 * seg + 2], len = p.segs[4 * seg + 3];
-  if (len < shortest(MLSTM)) return;
+  if (len < (MLSTM || few ? SHORT : FEW) || (few && len >= FEW)) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
   const int H = p.H, vdim = p.vdim;
   const bf16* qb = p.q + (size_t)row0 * p.ldqk + (size_t)(h / (H / p.G)) * DIM;
@@ -260,7 +263,7 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
       const int blocks = (n + 15) >> 4;        // blocks of 16 tokens that hold any
       if (rb < blocks) {
         float acc[4][4] = {}, rest[4][4] = {}, sc[2][NB][2][4] = {};   // rest: what the lower parts give, small enough to stay in the tensor cores' sums
-        // scores of this warp's blocks (rows rb, keys share, share + WPR, ..) and its share of Q S
+        // scores of this warp's blocks (rows rb, keys share, share + WPR, ..), and then its share of Q S
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
           uint32_t qf[4], kf[4];
@@ -274,7 +277,17 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
             mma_bf16_first(st[0], qf, kf[0], kf[1]);
             mma_bf16_first(st[1], qf, kf[2], kf[3]);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) sc[ks & 1][j][e >> 2][e & 3] += st[e >> 2][e & 3];     // two chains: half the roundings each
+            for (int e = 0; e < 8; ++e) {
+              const float x = st[e >> 2][e & 3];
+              if constexpr (few) {           // what the sum rounds off, exactly (Knuth's two-sum), in a sum of its own
+                float& sum = sc[0][j][e >> 2][e & 3];
+                const float next = sum + x, back = next - sum;
+                sc[1][j][e >> 2][e & 3] += (sum - (next - back)) + (x - back);
+                sum = next;
+              } else {                                   // two chains: half the roundings each
+                sc[ks & 1][j][e >> 2][e & 3] += x;
+              }
+            }
           }
         }
 #pragma unroll
@@ -460,11 +473,11 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
   }
 }
 
-template <bool MLSTM, int DIM, int L>
+template <bool MLSTM, int DIM, int L, bool few = false>
 int launch_chunks(const ChunkArgs& p, int nseg, cudaStream_t stream) {
   const size_t smem = sizeof(ChunkSmem<DIM, L>);
-  LIA_CUDA(cudaFuncSetAttribute(chunk_scan_kernel<MLSTM, DIM, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  lia_launch_after(chunk_scan_kernel<MLSTM, DIM, L>, dim3((p.vdim + COLS - 1) / COLS, p.H, nseg), dim3((MW + 4 + MLSTM) * 32), smem, stream, p);
+  LIA_CUDA(cudaFuncSetAttribute(chunk_scan_kernel<MLSTM, DIM, L, few>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  lia_launch_after(chunk_scan_kernel<MLSTM, DIM, L, few>, dim3((p.vdim + COLS - 1) / COLS, p.H, nseg), dim3((MW + 4 + MLSTM) * 32), smem, stream, p);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -478,9 +491,9 @@ bool whole_vectors(const ChunkArgs& p) {
 
 extern "C" int lia_chunk_scan_takes(int mlstm, int dim, int vdim) { return vdim > 0 && vdim % 8 == 0 && (dim == 128 || (mlstm && dim == 256)); }
 
-extern "C" int lia_chunk_scan_rows_of(int mlstm) { return shortest(mlstm != 0); }
+extern "C" int lia_chunk_scan_rows() { return SHORT; }
 
-extern "C" int lia_chunk_scan_rows() { return shortest(false); }
+extern "C" int lia_chunk_scan_few() { return FEW; }
 
 extern "C" int lia_decay_scan_chunks(const void* q, const void* k, int ldqk, const void* v, int ldv, const float* decay, float* state_S, const int* segs, int nseg,
                                      int mixed, int H, int G, int dim, int vdim, float* o, lia_stream_t stream_) {
@@ -491,8 +504,9 @@ extern "C" int lia_decay_scan_chunks(const void* q, const void* k, int ldqk, con
   ChunkArgs p{reinterpret_cast<const bf16*>(q), reinterpret_cast<const bf16*>(k), reinterpret_cast<const bf16*>(v), ldqk, ldv, decay, nullptr, state_S, nullptr,
               nullptr, nullptr, segs, H, G, vdim, 1.f, 0.f, o};
   LIA_CHECK_ARG(whole_vectors(p), "lia_decay_scan_chunks: rows are not whole 16-byte vectors");
-  const int rc = launch_chunks<false, 128, 64>(p, nseg, stream);
-  return rc != LIA_OK || !mixed ? rc : decay_scan_tokens(q, k, ldqk, v, ldv, decay, state_S, segs, shortest(false), nseg, H, G, dim, vdim, o, stream);
+  int rc = mixed & 4 ? LIA_OK : launch_chunks<false, 128, 64>(p, nseg, stream);
+  if (rc == LIA_OK && !(mixed & 2)) rc = launch_chunks<false, 128, 64, true>(p, nseg, stream);
+  return rc != LIA_OK || !(mixed & 1) ? rc : decay_scan_tokens(q, k, ldqk, v, ldv, decay, state_S, segs, SHORT, nseg, H, G, dim, vdim, o, stream);
 }
 
 extern "C" int lia_mlstm_scan_chunks(const void* q, const void* k, const void* v, int ld, const float* gates, float* state_S, float* state_n, float* state_m,
@@ -507,6 +521,6 @@ extern "C" int lia_mlstm_scan_chunks(const void* q, const void* k, const void* v
   LIA_CHECK_ARG(whole_vectors(p), "lia_mlstm_scan_chunks: rows are not whole 16-byte vectors");
   const int rc = dim == 128 ? launch_chunks<true, 128, 32>(p, nseg, stream) : launch_chunks<true, 256, 32>(p, nseg, stream);
   if (rc != LIA_OK) return rc;
-  if (mixed) return mlstm_scan_tokens(q, k, v, ld, gates, state_S, state_n, state_m, ws, segs, shortest(true), nseg, H, dim, vdim, q_scale, den_eps, o, stream);
+  if (mixed) return mlstm_scan_tokens(q, k, v, ld, gates, state_S, state_n, state_m, ws, segs, SHORT, nseg, H, dim, vdim, q_scale, den_eps, o, stream);
   return p.ws ? mlstm_take_state(p.ws, segs, nseg, state_n, state_m, H, dim, stream) : LIA_OK;
 }

@@ -1,5 +1,5 @@
 // Linear-attention recurrences with a matrix state per head, for prompts, portions of prompts and single decoded tokens
-// alike, and what prepares their inputs.  (DECAY with 128 dims in bf16, portions of 64 tokens and more: chunk_scan.cu.)
+// alike, and what prepares their inputs.  (DECAY with 128 dims in bf16, portions of 32 tokens and more: chunk_scan.cu.)
 //
 //   DECAY  (a fixed decay per head):     S_t = d_h S_{t-1} + k_t v_t^T                      o_t = S_t^T q_t
 //   DELTA  (gated delta rule):           S'  = g_t S_{t-1};  u_t = beta_t (v_t - S'^T k_t);  S_t = S' + k_t u_t^T;  o_t = S_t^T q_t

@@ -396,7 +396,7 @@ def argmax_f32(logits, suppress_id=-1, out=None):
 @functools.lru_cache(maxsize=256)
 def _chunk_rows(mlstm, dim, vdim):
     lib = _lib.load()
-    return lib.lia_chunk_scan_rows_of(mlstm) if lib.lia_chunk_scan_takes(mlstm, dim, vdim) else 0
+    return lib.lia_chunk_scan_rows() if lib.lia_chunk_scan_takes(mlstm, dim, vdim) else 0
 
 
 def _in_chunks(mlstm, q, k, v, ld, ldv, dim, vdim, state_S, o, n, lengths):
@@ -815,9 +815,11 @@ def linear_scan(q, k, v, state_S, segs, H, G, dim, vdim, o, decay=None, gates=No
     n = segs.shape[0]
     chunks, mixed = _in_chunks(0, q, k, v, ld, ldv, dim, vdim, state_S, o, n, lengths) if decay is not None and not in_silu else (False, False)
     if chunks:
-        check(_lib.load().lia_decay_scan_chunks(_p(q), _p(k), ld, _p(v), ldv, _p(_req(decay, "decay", F32)), _p(state_S), _p(segs), n, int(mixed), H, G, dim, vdim, _p(o),
-                                                _stream()), "lia_decay_scan_chunks")
-        count_launches(1 + mixed)
+        lib, (shortest, longest) = _lib.load(), lengths or (0, M)
+        none_few, none_long = shortest >= lib.lia_chunk_scan_few(), longest < lib.lia_chunk_scan_few()
+        check(lib.lia_decay_scan_chunks(_p(q), _p(k), ld, _p(v), ldv, _p(_req(decay, "decay", F32)), _p(state_S), _p(segs), n, mixed + 2 * none_few + 4 * none_long, H, G, dim, vdim,
+                                        _p(o), _stream()), "lia_decay_scan_chunks")
+        count_launches(2 - none_few - none_long + mixed)
         return o
     check(_lib.load().lia_linear_scan(_p(q), _p(k), ld, _p(v), ldv, _f32(q), int(in_silu), _p(_req(decay, "decay", F32) if decay is not None else None),
                                       _p(_req(gates, "gates", F32) if gates is not None else None), _p(state_S), _p(segs), segs.shape[0], H, G, dim,

@@ -156,7 +156,7 @@ def test_portions_of_unknown_lengths_in_a_larger_buffer(gated, lens):
 
 @pytest.mark.parametrize("gated,n", [(False, 32), (False, 63), (False, 64), (False, 100), (True, 32), (True, 65)])
 def test_outputs_are_as_close_to_64_bits_as_token_by_token(gated, n):
-    """Mean over inputs: the error in chunks is no larger than that of the token loop (a measured 0.72 to 0.98 times, 1 where the loop is what runs)."""
+    """Mean over inputs: the error in chunks is no larger than that of the token loop (a measured 0.72 to 0.98 times)."""
     H, dim, vdim, ratio = 4, 128, 128, []
     for seed in range(6):
         q, k, v, _, dsegs, r = _step([n], H, H, dim, vdim, seed)
