@@ -132,9 +132,10 @@ def test_latent_workspace_of_any_size(window, dim):
     """Portions in as many launches as the workspace asks for, a large one by groups of heads: the same bits."""
     H, rank, rot = 5, 72, 64
     portions = [(0, 0, 0, 30), (2, 100, 30, 65), (1, 31, 95, 40), (3, 250, 135, 16)] + [(4 + i, i, 151 + i, 1) for i in range(17)]
-    M, g = 168, torch.Generator().manual_seed(dim)
+    portions.insert(2, (21, 20, 168, 256))                        # of many rows, among those of few
+    M, g = 424, torch.Generator().manual_seed(dim)
     q, qr = torch.randn(M, H * (dim + rot), generator=g).to(BF16).to(DEV), torch.randn(M, H, rot, generator=g).to(DEV)
-    lat = torch.randn(21, 280, rank + rot, generator=g).to(BF16).to(DEV)
+    lat = torch.randn(22, 280, rank + rot, generator=g).to(BF16).to(DEV)
     w = (torch.randn(2 * H * dim, rank, generator=g) * rank ** -0.5).to(BF16).to(DEV)
     gate, sink = torch.rand(M, H, generator=g).to(DEV), torch.linspace(-1.0, 1.0, H, device=DEV)
     want = None
@@ -146,9 +147,9 @@ def test_latent_workspace_of_any_size(window, dim):
         assert torch.equal(out, want)
 
 
-@pytest.mark.parametrize("H,n,past", [(4, 16, 100), (4, 33, 300), (16, 20, 200), (16, 64, 100)])
+@pytest.mark.parametrize("H,n,past", [(4, 16, 100), (4, 33, 300), (16, 20, 200), (16, 64, 100), (4, 255, 0), (16, 256, 300)])
 def test_latent_portions_are_as_close_to_64_bits_as_in_the_latent_space(H, n, past):
-    """Mean over inputs of the two forms' errors: a measured 0.75 to 0.90."""
+    """Mean over inputs of the two forms' errors: a measured 0.60 to 0.95."""
     dim, rank, rot, ctx, ratio = 128, 512, 64, past + n, []
     i32 = dict(dtype=torch.int32, device=DEV)
     meta = torch.tensor([(0, past + i) for i in range(n)], **i32)
