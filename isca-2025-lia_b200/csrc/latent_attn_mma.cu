@@ -23,10 +23,6 @@ namespace {
 
 constexpr int BM = 64, BK = 32;
 constexpr int MAX_PORTIONS = 16;        // of one launch
-// Portions of fewer rows have their scores' high products added in fp32 every 16 channels.  With those of all channels in one chain of the tensor cores, which cut sums off
-// below the 24th bit, the output of 16 to 100 rows behind up to 1500 positions is off by 0.9 to 1.15 times what the latent space gives, so by 0.75 to 0.90; from 200
-// rows on the chain gives 0.42 to 0.99, and costs less (2048 tokens: 490 us against 504).
-constexpr int MANY_ROWS = 256;
 
 // 16-byte chunk c of row r in a tile of rows of CH (at least 8) chunks, turned by the row (window_attn_mma.cu)
 template <int CH> __device__ __forceinline__ uint32_t at_chunk(uint32_t base, int r, int c) { return base + (uint32_t)(r * CH + (c ^ (r & 7))) * 16u; }
@@ -89,7 +85,7 @@ __device__ __noinline__ PlainRow<DN> plain_row(const bf16* q, const float* qr, c
 
 template <int DN, int DR> constexpr int expanded_smem() { return (BM * DN + 3 * BM * DR + 2 * 3 * BK * DN + BK * DR) * 2; }
 
-template <int DN, int DR, bool APART>
+template <int DN, int DR>
 __global__ void __launch_bounds__(128, 2) latent_expanded_kernel(const __grid_constant__ ExpandedArgs a) {
   pdl_launch_dependents();
   pdl_wait();
@@ -168,8 +164,10 @@ __global__ void __launch_bounds__(128, 2) latent_expanded_kernel(const __grid_co
     const bool on = warp_on && j0 <= wpos + 15 && j0 + BK - 1 >= wpos - a.window + 1;
     cp_async_wait<1>();
     __syncthreads();                                     // the keys (and, at first, the queries) are there
-    // Two sums per score: the unrotated channels' high products (APART: added in fp32 every 16 channels), and all the rest -- its small parts first, then the
-    // rotated channels' high products.
+    // Two sums per score: the unrotated channels' high products, 16 channels at a time added in fp32, and all the rest -- its small parts first, then the
+    // rotated channels' high products.  The tensor cores cut sums off below the 24th bit: with the high products of all channels in one chain the output of 16 to
+    // 100 rows behind up to 1500 positions was off by 0.9 to 1.15 times what the latent space gives, now by 0.68 to 0.90 (2048 tokens: 490 -> 505 us; the chain for
+    // portions of 256 rows and more alone, where it is exact enough: 490 us again, but portions of 401 to 250 rows in two launches 210 us instead of 154).
     float S[NT][4], S2[NT][4];
 #pragma unroll
     for (int n = 0; n < NT; ++n)
@@ -186,9 +184,9 @@ __global__ void __launch_bounds__(128, 2) latent_expanded_kernel(const __grid_co
           for (int p = 2; p >= 0; --p) {
             uint32_t b[4];
             ldsm_x4(at_chunk<QC>(kn + p * BK * DN * 2, n * 8 + (lane & 7) + ((lane >> 4) << 3), 2 * kk + ((lane >> 3) & 1)), b);
-            if (p > 0 || !APART) {
-              mma_bf16(p ? S2[n] : S[n], af, b[0], b[1]);
-              mma_bf16(p ? S2[n + 1] : S[n + 1], af, b[2], b[3]);
+            if (p > 0) {
+              mma_bf16(S2[n], af, b[0], b[1]);
+              mma_bf16(S2[n + 1], af, b[2], b[3]);
             } else {
               float f[2][4];
               mma_bf16_first(f[0], af, b[0], b[1]);
@@ -341,10 +339,10 @@ __global__ void __launch_bounds__(128, 2) latent_expanded_kernel(const __grid_co
   }
 }
 
-template <int DN, int DR, bool APART> int run(const ExpandedArgs& a, int tiles, cudaStream_t stream) {
+template <int DN, int DR> int run(const ExpandedArgs& a, int tiles, cudaStream_t stream) {
   constexpr int smem = expanded_smem<DN, DR>();
-  LIA_CUDA(cudaFuncSetAttribute(latent_expanded_kernel<DN, DR, APART>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  lia_launch(latent_expanded_kernel<DN, DR, APART>, dim3(a.nh, tiles), dim3(128), smem, stream, a);
+  LIA_CUDA(cudaFuncSetAttribute(latent_expanded_kernel<DN, DR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  lia_launch(latent_expanded_kernel<DN, DR>, dim3(a.nh, tiles), dim3(128), smem, stream, a);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -384,49 +382,42 @@ extern "C" int lia_latent_attn_expanded_in(const void* q, int ldq, const float* 
   const int D = kv_rank + rot;
   const size_t room = workspace_bytes / lia_latent_expanded_workspace_bytes(1, 1, dim);          // (latent, head) pairs
   if (window <= 0) window = 1 << 30;
-  for (int apart = 0; apart < 2; ++apart)                          // the portions of many rows, then those of few
-    for (int first = 0; first < np;) {
-      ExpandedArgs a{reinterpret_cast<const bf16*>(q), qr, reinterpret_cast<const bf16*>(workspace), gate, sink, out, D, ldq, qr_stride, H, 0, 0, window, out_f32, 0, scale, {}};
-      const bf16* src[MAX_PORTIONS];
-      int rows[MAX_PORTIONS], tiles = 0;
-      long long latents = 0;
-      while (first < np && a.np < MAX_PORTIONS) {
-        const int* p = portions + 4 * first;                         // slot, first position, first row, rows
-        LIA_CHECK_ARG(p[0] >= 0 && p[1] >= 0 && p[2] >= 0 && p[3] > 0, "lia_latent_attn_expanded: bad portion");
-        if ((p[3] < MANY_ROWS) != (apart == 1)) {
-          ++first;
-          continue;
-        }
-        const int base = p[1] - window + 1 > 0 ? p[1] - window + 1 : 0, seen = p[1] + p[3] - base, i = a.np;
-        if (i > 0 && ((size_t)(latents + seen) * H > room || latents + seen > INT_MAX)) break;
-        src[i] = reinterpret_cast<const bf16*>(cache) + (size_t)p[0] * slot_stride + (size_t)base * D;
-        rows[i] = seen;
-        a.p[i] = Portion{src[i] + kv_rank, p[2], p[3], p[1] - base, (int)latents, tiles};
-        tiles += (p[3] + BM - 1) / BM;
-        latents += seen;
-        ++a.np;
-        ++first;
-      }
-      if (a.np == 0) break;
-      LIA_CHECK_ARG(tiles <= 65535, "lia_latent_attn_expanded: too many rows");
-      LIA_CHECK_ARG((size_t)latents <= room, "lia_latent_attn_expanded: a workspace of %zu bytes does not hold one head of %lld latents", workspace_bytes, latents);
-      const int most = (size_t)latents * H <= room ? H : (int)(room / latents);
-      const bf16* wk = reinterpret_cast<const bf16*>(w_ukv);
-      bf16* ws = reinterpret_cast<bf16*>(workspace);
-      for (a.h0 = 0; a.h0 < H; a.h0 += a.nh) {
-        a.nh = most < H - a.h0 ? most : H - a.h0;
-        const long long ldc = 6ll * a.nh * dim;
-        int rc;
-        if (a.nh == H) {
-          rc = linear_mma_parts(src, rows, a.np, D, wk, ws, ldc, 2 * H * dim, kv_rank, dim, stream);
-        } else {
-          rc = linear_mma_parts(src, rows, a.np, D, wk + (size_t)a.h0 * dim * kv_rank, ws, ldc, a.nh * dim, kv_rank, dim, stream);
-          if (rc == LIA_OK) rc = linear_mma_parts(src, rows, a.np, D, wk + (size_t)(H + a.h0) * dim * kv_rank, ws + (size_t)3 * a.nh * dim, ldc, a.nh * dim, kv_rank, dim, stream);
-        }
-        if (rc == LIA_OK && apart) rc = dim == 128 ? run<128, 64, true>(a, tiles, stream) : run<64, 64, true>(a, tiles, stream);
-        if (rc == LIA_OK && !apart) rc = dim == 128 ? run<128, 64, false>(a, tiles, stream) : run<64, 64, false>(a, tiles, stream);
-        if (rc != LIA_OK) return rc;
-      }
+  for (int first = 0; first < np;) {
+    ExpandedArgs a{reinterpret_cast<const bf16*>(q), qr, reinterpret_cast<const bf16*>(workspace), gate, sink, out, D, ldq, qr_stride, H, 0, 0, window, out_f32, 0, scale, {}};
+    const bf16* src[MAX_PORTIONS];
+    int rows[MAX_PORTIONS], tiles = 0;
+    long long latents = 0;
+    while (first < np && a.np < MAX_PORTIONS) {
+      const int* p = portions + 4 * first;                         // slot, first position, first row, rows
+      LIA_CHECK_ARG(p[0] >= 0 && p[1] >= 0 && p[2] >= 0 && p[3] > 0, "lia_latent_attn_expanded: bad portion");
+      const int base = p[1] - window + 1 > 0 ? p[1] - window + 1 : 0, seen = p[1] + p[3] - base, i = a.np;
+      if (i > 0 && ((size_t)(latents + seen) * H > room || latents + seen > INT_MAX)) break;
+      src[i] = reinterpret_cast<const bf16*>(cache) + (size_t)p[0] * slot_stride + (size_t)base * D;
+      rows[i] = seen;
+      a.p[i] = Portion{src[i] + kv_rank, p[2], p[3], p[1] - base, (int)latents, tiles};
+      tiles += (p[3] + BM - 1) / BM;
+      latents += seen;
+      ++a.np;
+      ++first;
     }
+    LIA_CHECK_ARG(tiles <= 65535, "lia_latent_attn_expanded: too many rows");
+    LIA_CHECK_ARG((size_t)latents <= room, "lia_latent_attn_expanded: a workspace of %zu bytes does not hold one head of %lld latents", workspace_bytes, latents);
+    const int most = (size_t)latents * H <= room ? H : (int)(room / latents);
+    const bf16* wk = reinterpret_cast<const bf16*>(w_ukv);
+    bf16* ws = reinterpret_cast<bf16*>(workspace);
+    for (a.h0 = 0; a.h0 < H; a.h0 += a.nh) {
+      a.nh = most < H - a.h0 ? most : H - a.h0;
+      const long long ldc = 6ll * a.nh * dim;
+      int rc;
+      if (a.nh == H) {
+        rc = linear_mma_parts(src, rows, a.np, D, wk, ws, ldc, 2 * H * dim, kv_rank, dim, stream);
+      } else {
+        rc = linear_mma_parts(src, rows, a.np, D, wk + (size_t)a.h0 * dim * kv_rank, ws, ldc, a.nh * dim, kv_rank, dim, stream);
+        if (rc == LIA_OK) rc = linear_mma_parts(src, rows, a.np, D, wk + (size_t)(H + a.h0) * dim * kv_rank, ws + (size_t)3 * a.nh * dim, ldc, a.nh * dim, kv_rank, dim, stream);
+      }
+      if (rc == LIA_OK) rc = dim == 128 ? run<128, 64>(a, tiles, stream) : run<64, 64>(a, tiles, stream);
+      if (rc != LIA_OK) return rc;
+    }
+  }
   return LIA_OK;
 }

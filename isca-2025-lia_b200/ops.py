@@ -514,16 +514,14 @@ def latent_attn(qa, cache, meta, gate, out, H, kv_rank, rot, scale, max_ctx=0, w
     return out
 
 
-def _expanded_launches(portions, seen, H, room, many=256):
+def _expanded_launches(seen, H, room):
     """Launches of ``latent_attn_expanded`` (csrc/latent_attn_mma.cu) over portions that see so many latents."""
-    n = 0
-    for few in (False, True):
-        count = latents = 0
-        for s in [s for p, s in zip(portions, seen) if (p[3] < many) == few] + [None]:
-            if count and (s is None or count == 16 or (latents + s) * H > room):
-                n += 2 if latents * H <= room else 3 * -(-H // (room // latents))
-                count = latents = 0
-            count, latents = count + 1, latents + (s or 0)
+    n, count, latents = 0, 0, 0
+    for s in seen + [None]:
+        if count and (s is None or count == 16 or (latents + s) * H > room):
+            n += 2 if latents * H <= room else 3 * -(-H // (room // latents))
+            count, latents = 0, 0
+        count, latents = count + 1, latents + (s or 0)
     return n
 
 
@@ -560,7 +558,7 @@ def latent_attn_expanded(q, qr, cache, portions, w_ukv, gate, out, H, dim, rot, 
     table = (ctypes.c_int * (4 * len(portions)))(*[int(x) for p in portions for x in p])
     check(lib.lia_latent_attn_expanded_in(_p(q), _rowmajor(q, "q"), _p(qr), qr.stride(1), _p(cache), cache.stride(0), table, len(portions), _p(w_ukv), _p(gate),
                                           _p(sink), _p(out), _f32(out), _p(ws), ws.numel(), H, dim, rot, kv_rank, int(window), float(scale), _stream()), "lia_latent_attn_expanded")
-    count_launches(_expanded_launches(portions, seen, H, room))
+    count_launches(_expanded_launches(seen, H, room))
     return out
 
 
