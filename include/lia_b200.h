@@ -607,6 +607,13 @@ int lia_conv_act(const void* y, int y_f32, int ld, int col0, int C, const float*
  * rows: tokens of all nseg portions together */
 int lia_ssd_scan(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* state_S, const int* segs, int nseg,
                  int rows, int H, int G, int N, int vdim, float* o, lia_stream_t stream);
+/* The same with the portions of lia_ssd_chunk_rows() tokens and more in chunks on the tensor cores, `chunks` chunks (of 128 tokens) of every portion at a time; N = 128,
+ * vdim a multiple of 64, all rows whole 16-byte vectors.  ws: lia_ssd_workspace() bytes for the same shape and chunks, which is 0 where lia_ssd_scan() is to be called.
+ * The result does not depend on `chunks`. */
+int lia_ssd_chunk_rows(void);
+long long lia_ssd_workspace(int rows, int nseg, int H, int G, int N, int vdim, int chunks);
+int lia_ssd_scan_chunks(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* state_S, const int* segs, int nseg, int rows,
+                        int H, int G, int N, int vdim, float* o, void* ws, long long ws_bytes, int chunks, lia_stream_t stream);
 /* Real-gated linear recurrent unit over every portion, channel by channel (width = blocks * n): log a = c sigmoid(r + its bias),
  * S = a S + sqrt(1 - a^2) sigmoid(i + its bias) u, out = S * gelu_tanh(y + y_bias) of y's type; z [rows][blocks][2n] = r | i,
  * z_bias [blocks][2n], state [slot][width] fp32; y has row stride ldy, y_bias may be NULL; rows as above */

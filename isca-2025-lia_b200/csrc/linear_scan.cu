@@ -554,13 +554,22 @@ constexpr int SSD_TB = 16;        // tokens per stage
 template <int NJ, int RG, int TG, bool VL>
 __global__ void __launch_bounds__(128, TG > 1 ? 1 : (NJ <= 2 ? 5 : (NJ <= 4 ? 3 : 1))) ssd_scan_kernel(const float* __restrict__ B, const float* __restrict__ C, const float* __restrict__ x, int ld,
                                                        const float* __restrict__ gates, const float* __restrict__ D, float* __restrict__ St,
-                                                       const int* __restrict__ segs, int H, int G, int N, int vdim, float* __restrict__ o) {
+                                                       const int* __restrict__ segs, int tok0, int span, int below, const int* __restrict__ flags, const float* __restrict__ after,
+                                                       int H, int G, int N, int vdim, float* __restrict__ o) {
   pdl_launch_dependents();
   pdl_wait();
   constexpr int SSD_COLS = 4 * 4 * 32 / RG, NP = NJ * 4 * RG, ROWF = 2 * NP + SSD_COLS + 4;
   extern __shared__ __align__(16) float stage[];       // [2][SSD_TB][ROWF]
   const int seg = blockIdx.z, h = blockIdx.y, colb = blockIdx.x * SSD_COLS, g = h / (H / G);
-  const int slot = segs[4 * seg], row0 = segs[4 * seg + 2], len = segs[4 * seg + 3];
+  const int slot = segs[4 * seg], row0 = segs[4 * seg + 2] + tok0, all = segs[4 * seg + 3], len = min(all - tok0, span);
+  if (all >= below && (len <= 0 || !flags[(size_t)seg * H + h])) {                  // ssd_chunk_sm100.cu had these tokens (span: some of its portion's at a time): the state
+    if (len <= 0) return;                                                            // after them is to go where it belongs
+    const size_t first = (size_t)h * vdim * N + (size_t)colb * N, all_heads = (size_t)H * vdim * N;
+    for (int e = threadIdx.x * 4; e < min(SSD_COLS, vdim - colb) * N; e += 512)
+      *reinterpret_cast<float4*>(St + slot * all_heads + first + e) = *reinterpret_cast<const float4*>(after + seg * all_heads + first + e);
+    return;
+  }
+  if (all < below && tok0 > 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rg = lane % RG;
   const int cl = warp * (SSD_COLS / 4) + (lane / RG) * 4, col0 = colb + cl;
   const int ncol = min(SSD_COLS, vdim - colb);
@@ -728,14 +737,22 @@ __global__ void __launch_bounds__(128, TG > 1 ? 1 : (NJ <= 2 ? 5 : (NJ <= 4 ? 3 
   }
 }
 
+struct SsdTokens {                             // which tokens: those of portions shorter than `below`, and tok0 .. tok0 + span - 1 of the heads that `flags` names
+  int tok0 = 0, span = INT_MAX, below = INT_MAX;
+  const int* flags = nullptr;
+  const float* after = nullptr;                // [nseg][H][vdim][N], for the other heads of the longer portions
+};
+
 template <int NJ, int RG, int TG, bool VL>
-int launch_ssd_as(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* St, const int* segs, int nseg, int H,
+int launch_ssd_as(const SsdTokens& w, const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* St, const int* segs, int nseg, int H,
                   int G, int N, int vdim, float* o, cudaStream_t stream) {
   constexpr int COLS = 16 * 32 / RG;
   const size_t smem = (size_t)2 * SSD_TB * (2 * NJ * 4 * RG + COLS + 4) * sizeof(float);
   if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(ssd_scan_kernel<NJ, RG, TG, VL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((vdim + COLS - 1) / COLS, H, nseg);
-  lia_launch_after(ssd_scan_kernel<NJ, RG, TG, VL>, dim3(grid), dim3(128), smem, stream, B, C, x, ld, gates, D, St, segs, H, G, N, vdim, o);
+  // beside the chunks there is seldom much to do, and nothing to crowd out
+  lia_launch_as(w.flags != nullptr, ssd_scan_kernel<NJ, RG, TG, VL>, dim3(grid), dim3(128), smem, stream, B, C, x, ld, gates, D, St, segs, w.tok0, w.span, w.below, w.flags, w.after, H, G, N,
+                vdim, o);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -743,13 +760,13 @@ int launch_ssd_as(const float* B, const float* C, const float* x, int ld, const 
 // 128-bit copies and state accesses: every B, C, x segment and every state column starts on a 16-byte boundary
 // single: every portion is one token (decoding) -- the variant without token groups needs fewer registers, so more blocks share an SM
 template <int NJ, int RG, int TG>
-int launch_ssd(bool single, const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* St, const int* segs,
+int launch_ssd(const SsdTokens& w, bool single, const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* St, const int* segs,
                int nseg, int H, int G, int N, int vdim, float* o, cudaStream_t stream) {
   const bool aligned = ((reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(St)) % 16 == 0) &&
                        ld % 4 == 0 && N % 4 == 0 && vdim % 4 == 0;
-  if (aligned && single) return launch_ssd_as<NJ, RG, 1, true>(B, C, x, ld, gates, D, St, segs, nseg, H, G, N, vdim, o, stream);
-  if (aligned) return launch_ssd_as<NJ, RG, TG, true>(B, C, x, ld, gates, D, St, segs, nseg, H, G, N, vdim, o, stream);
-  return launch_ssd_as<NJ, RG, TG, false>(B, C, x, ld, gates, D, St, segs, nseg, H, G, N, vdim, o, stream);
+  if (aligned && single) return launch_ssd_as<NJ, RG, 1, true>(w, B, C, x, ld, gates, D, St, segs, nseg, H, G, N, vdim, o, stream);
+  if (aligned) return launch_ssd_as<NJ, RG, TG, true>(w, B, C, x, ld, gates, D, St, segs, nseg, H, G, N, vdim, o, stream);
+  return launch_ssd_as<NJ, RG, TG, false>(w, B, C, x, ld, gates, D, St, segs, nseg, H, G, N, vdim, o, stream);
 }
 
 // ---------------------------------------------------------------------------------------------------- gated linear recurrent unit
@@ -940,6 +957,11 @@ extern "C" int lia_conv_act(const void* y, int y_f32, int ld, int col0, int C, c
   return LIA_OK;
 }
 
+int ssd_scan_tokens(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* St, const int* segs, int tok0, int span, int below,
+                    const int* flags, const float* after, int nseg, int H, int G, int N, int vdim, float* o, cudaStream_t stream) {
+  return launch_ssd<2, 16, 4>(SsdTokens{tok0, span, below, flags, after}, false, B, C, x, ld, gates, D, St, segs, nseg, H, G, N, vdim, o, stream);      // N = 128
+}
+
 extern "C" int lia_ssd_scan(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* state_S, const int* segs,
                             int nseg, int rows, int H, int G, int N, int vdim, float* o, lia_stream_t stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
@@ -948,10 +970,10 @@ extern "C" int lia_ssd_scan(const float* B, const float* C, const float* x, int 
   LIA_CHECK_ARG(B && C && x && gates && D && state_S && segs && o, "lia_ssd_scan: null pointer");
   LIA_CHECK_ARG(nseg > 0 && nseg <= 65535 && H > 0 && H <= 65535 && G > 0 && H % G == 0 && N > 0 && N <= 512 && vdim > 0,
                 "lia_ssd_scan: bad shape nseg=%d H=%d G=%d N=%d vdim=%d", nseg, H, G, N, vdim);
-  if (N <= 64) return launch_ssd<1, 16, 8>(single, B, C, x, ld, gates, D, state_S, segs, nseg, H, G, N, vdim, o, stream);
-  if (N <= 128) return launch_ssd<2, 16, 4>(single, B, C, x, ld, gates, D, state_S, segs, nseg, H, G, N, vdim, o, stream);
-  if (N <= 256) return launch_ssd<4, 16, 2>(single, B, C, x, ld, gates, D, state_S, segs, nseg, H, G, N, vdim, o, stream);
-  return launch_ssd<8, 16, 1>(single, B, C, x, ld, gates, D, state_S, segs, nseg, H, G, N, vdim, o, stream);
+  if (N <= 64) return launch_ssd<1, 16, 8>({}, single, B, C, x, ld, gates, D, state_S, segs, nseg, H, G, N, vdim, o, stream);
+  if (N <= 128) return launch_ssd<2, 16, 4>({}, single, B, C, x, ld, gates, D, state_S, segs, nseg, H, G, N, vdim, o, stream);
+  if (N <= 256) return launch_ssd<4, 16, 2>({}, single, B, C, x, ld, gates, D, state_S, segs, nseg, H, G, N, vdim, o, stream);
+  return launch_ssd<8, 16, 1>({}, single, B, C, x, ld, gates, D, state_S, segs, nseg, H, G, N, vdim, o, stream);
 }
 
 extern "C" int lia_rglru_scan(const float* u, const float* z, const float* z_bias, const float* c, const void* y, int y_f32, int ldy, const float* y_bias,

@@ -305,9 +305,8 @@ template <int MODE> int launch(const void* W, uint64_t w_rows, int K, const CUte
 
 extern "C" int lia_moe_tc_rows(void) { return ROWS; }
 
-namespace {
 // The word that counts CTAs whose wait ran out: host memory that every GPU can write, allocated with the first launch and kept.
-int* timeout_word(bool make) {
+static int* timeout_word(bool make) {
   static std::mutex m;
   static int* word = nullptr;
   std::lock_guard<std::mutex> lock(m);
@@ -323,9 +322,9 @@ int* timeout_word(bool make) {
   }
   return word;
 }
-}  // namespace
+int* lia_timeout_word() { return timeout_word(true); }             // for the kernels of other files
 
-/* CTAs of lia_moe_gemm_tc that gave up a wait, as far as launches have ended, since the library was loaded */
+/* CTAs of lia_moe_gemm_tc and lia_ssd_scan_chunks that gave up a wait, as far as launches have ended, since the library was loaded */
 extern "C" int lia_moe_timeouts_seen(void) {
   const volatile int* word = timeout_word(false);
   return word ? *word : 0;

@@ -1269,10 +1269,35 @@ def ssd_scan(xbc, gates, D, state_S, segs, H, G, N, vdim, o):
     if xbc.dtype != F32 or xbc.shape[1] != inner + 2 * G * N or tuple(gates.shape) != (M, 2 * H) or D.numel() != H or tuple(o.shape) != (M, inner) \
             or tuple(state_S.shape[1:]) != (H, vdim, N):
         raise _lib.LiaError("ssd_scan: shapes do not agree")
-    check(_lib.load().lia_ssd_scan(_p(xbc[:, inner:]), _p(xbc[:, inner + G * N:]), _p(xbc), ld, _p(gates), _p(D), _p(state_S), _p(segs), segs.shape[0], M, H, G, N,
-                                   vdim, _p(o), _stream()), "lia_ssd_scan")
-    count_launches()
+    lib, nseg = _lib.load(), segs.shape[0]
+    args = (_p(xbc[:, inner:]), _p(xbc[:, inner + G * N:]), _p(xbc), ld, _p(gates), _p(D), _p(state_S), _p(segs), nseg, M, H, G, N, vdim, _p(o))
+    chunks, ws = _ssd_workspace(lib, M, nseg, H, G, N, vdim, (xbc, state_S, o), ld, inner)
+    if ws is not None:
+        check(lib.lia_ssd_scan_chunks(*args, _p(ws), ws.numel(), chunks, _stream()), "lia_ssd_scan_chunks")
+        count_launches(4 * -(-(M - nseg + 1) // (128 * chunks)))
+    else:
+        check(lib.lia_ssd_scan(*args, _stream()), "lia_ssd_scan")
+        count_launches()
     return o
+
+
+SSD_WORKSPACE = 256 << 20                                     # bytes for the states between chunks; longer steps take some chunks of every portion at a time
+
+
+def _ssd_workspace(lib, M, nseg, H, G, N, vdim, tensors, ld, inner):
+    """How many chunks of every portion to take at a time, and their workspace; None: token by token (csrc/ssd_chunk_sm100.cu).  The result does not depend on
+    the number, so that less is taken where memory is short."""
+    one = lib.lia_ssd_workspace(M, nseg, H, G, N, vdim, 1)
+    if not one or ld % 4 or any(t.data_ptr() % 16 for t in tensors):
+        return 0, None
+    chunks = max(1, min(-(-(M - nseg + 1) // 128), SSD_WORKSPACE // one))
+    while True:
+        try:
+            return chunks, torch.empty(lib.lia_ssd_workspace(M, nseg, H, G, N, vdim, chunks), dtype=torch.uint8, device=tensors[0].device)
+        except torch.OutOfMemoryError:
+            if chunks == 1:
+                return 0, None
+            chunks = (chunks + 1) // 2
 
 
 def rglru_scan(u, z, z_bias, c, y, y_bias, state, segs, blocks, out):

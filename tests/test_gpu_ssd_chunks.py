@@ -1,0 +1,122 @@
+"""The state-space recurrence in chunks of tokens (csrc/ssd_chunk_sm100.cu) against the token loop in 64 bits, beside the kernel that goes token by token: portions that end
+around the chunks, heads of one and two slices, groups of more heads than a CTA takes, a workspace that holds some of the chunks, values that are not finite or too large."""
+import pytest
+import torch
+
+import lia_b200  # noqa: F401
+from lia_b200 import _lib, ops
+
+pytestmark = pytest.mark.gpu
+F32, F64 = torch.float32, torch.float64
+N = 128
+
+
+class Step:
+    def __init__(self, lens, H, G, vdim, rate=1.0, pad=0, seed=0):
+        g = torch.Generator(device="cuda").manual_seed(seed + sum(lens) + H)
+        r = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+        self.shape, self.lens, M = (H, G, N, vdim), lens, sum(lens)
+        self.inner = H * vdim
+        self.xbc = torch.nn.functional.silu(r(M, self.inner + 2 * G * N + pad))[:, :self.inner + 2 * G * N]
+        dt = torch.nn.functional.softplus(r(M, H) - 2)
+        self.gates = torch.cat([dt, torch.exp(-torch.exp(r(H) * 0.7) * rate * dt)], 1).contiguous()
+        self.D, self.S0 = r(H), r(len(lens) + 1, H, vdim, N)
+        self.slots = [(3 * i + 1) % (len(lens) + 1) if (len(lens) + 1) % 3 else i for i in range(len(lens))]
+        self.segs, row = [], 0
+        for s, n in zip(self.slots, lens):
+            self.segs.append((s, 0, row, n))
+            row += n
+
+    def run(self, by_tokens=False, segs=None):
+        S, o = self.S0.clone(), torch.full((self.xbc.shape[0], self.inner), 7.0, device="cuda")
+        d, (H, G, _, vdim) = torch.tensor(segs or self.segs, dtype=torch.int32, device="cuda"), self.shape
+        if by_tokens:
+            x, p = self.xbc, ops._p
+            ops.check(_lib.load().lia_ssd_scan(p(x[:, self.inner:]), p(x[:, self.inner + G * N:]), p(x), x.stride(0), p(self.gates), p(self.D), p(S), p(d), d.shape[0], x.shape[0],
+                                               H, G, N, vdim, p(o), ops._stream()), "lia_ssd_scan")
+        else:
+            ops.ssd_scan(self.xbc, self.gates, self.D, S, d, H, G, N, vdim, o)
+        return o, S
+
+    def exact(self):
+        (H, G, _, vdim), M = self.shape, self.xbc.shape[0]
+        x, B, C = torch.split(self.xbc.double(), [self.inner, G * N, G * N], -1)
+        x, (B, C) = x.view(M, H, vdim), (t.reshape(M, G, N).repeat_interleave(H // G, 1) for t in (B, C))
+        dt, a = self.gates.double().split(H, 1)
+        u, o, state = dt[:, :, None] * x, torch.empty(M, H, vdim, dtype=F64, device="cuda"), self.S0.double()
+        for slot, _, row, n in self.segs:
+            S = state[slot]
+            for t in range(row, row + n):
+                S.mul_(a[t][:, None, None]).add_(u[t][:, :, None] * B[t][:, None, :])
+                o[t] = (S @ C[t][:, :, None])[..., 0]
+        return (o + self.D.double()[:, None] * x).view(M, -1), state
+
+
+def _rel(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
+def _chunked(step):
+    H, G, _, vdim = step.shape
+    return _lib.load().lia_ssd_workspace(step.xbc.shape[0], len(step.segs), H, G, N, vdim, 1) > 0
+
+
+@pytest.mark.parametrize("lens,H,G,vdim,rate,pad", [([256], 2, 1, 64, 1.0, 0), ([257, 40, 300], 4, 4, 64, 1.0, 4), ([511, 1], 18, 2, 64, 1.0, 0), ([512], 4, 2, 128, 0.02, 8),
+                                                   ([385, 255, 640], 3, 1, 64, 20.0, 0), ([900], 8, 8, 192, 0.3, 0)])
+def test_against_the_token_loop(lens, H, G, vdim, rate, pad):
+    """Either kernel's numbers are fp32 sums of the same products in another order: this one's error is at most the other's, up to a rounding of 2^-25."""
+    step = Step(lens, H, G, vdim, rate, pad)
+    assert _chunked(step)
+    want = step.exact()
+    for new, old, w in zip(step.run(), step.run(by_tokens=True), want):
+        assert _rel(new, w) <= _rel(old, w) + 2.0 ** -25
+
+
+def test_a_workspace_for_some_of_the_chunks_changes_no_bit(monkeypatch):
+    step = Step([1000, 300], 4, 2, 64)
+    whole = step.run()
+    for size in (1, 1 << 21):
+        monkeypatch.setattr(ops, "SSD_WORKSPACE", size)
+        assert all(torch.equal(a, b) for a, b in zip(whole, step.run()))
+
+
+def test_a_portion_does_not_depend_on_its_company():
+    step = Step([300, 1, 256, 255, 700], 8, 2, 64)
+    o, S = step.run()
+    for slot, p0, row, n in step.segs:
+        alone, state = step.run(segs=[(slot, p0, row, n)])
+        assert torch.equal(alone[row:row + n], o[row:row + n]) and torch.equal(state[slot], S[slot])
+    short = step.run(by_tokens=True)
+    for slot, _, row, n in step.segs:
+        if n < 256:
+            assert torch.equal(o[row:row + n], short[0][row:row + n]) and torch.equal(S[slot], short[1][slot])
+
+
+@pytest.mark.parametrize("what,value", [("x", float("nan")), ("x", float("inf")), ("x", 3e38), ("B", float("-inf")), ("C", float("nan")), ("C", 1e30), ("dt", float("inf")), ("g", float("nan")),
+                                        ("g", 1.5), ("S", float("inf")), ("S", 1e35)])
+@pytest.mark.parametrize("at", [0, 131, 299])
+def test_values_out_of_range_go_token_by_token(what, value, at):
+    H, G, vdim = 4, 2, 64
+    step = Step([300], H, G, vdim)
+    clean = step.run()
+    if what in ("x", "B", "C"):
+        col = {"x": 2 * vdim + 5, "B": step.inner + N + 9, "C": step.inner + G * N + N + 9}[what]
+        step.xbc[at, col] = value
+        heads = [2] if what == "x" else [2, 3]
+    elif what == "S":
+        step.S0[step.slots[0], 2, 7, at % N] = value
+        heads = [2]
+    else:
+        step.gates[at, 2 + (H if what == "g" else 0)] = value
+        heads = [2]
+    got, old = step.run(), step.run(by_tokens=True)
+    for h in range(H):
+        o, p, q = (t[0].view(-1, H, vdim)[:, h] for t in (got, old, clean))
+        S, T, U = (t[1][:, h] for t in (got, old, clean))
+        same, like = (p, T) if h in heads else (q, U), (o, S)
+        assert all(torch.equal(a.nan_to_num(nan=123.0), b.nan_to_num(nan=123.0)) for a, b in zip(same, like)), h
+
+
+def test_rows_that_are_not_whole_vectors_and_other_shapes_go_token_by_token():
+    for step in (Step([300], 2, 1, 64, pad=1), Step([300], 2, 1, 40), Step([255, 200], 2, 1, 64)):
+        assert all(torch.equal(a, b) for a, b in zip(step.run(), step.run(by_tokens=True)))
