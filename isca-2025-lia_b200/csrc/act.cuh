@@ -4,10 +4,21 @@
 
 namespace {
 
+// y / d for d >= 1, without the branch of the compiler's division, so that a thread works on many quotients at once: the one from an approximate reciprocal (of d / 2^8, whose reciprocal
+// is never too small), corrected once by its remainder (P. Markstein, Computation of elementary functions on the IBM RISC System/6000, 1990).  An infinite y or d leaves no remainder to
+// correct by.  z / (1 + expf(-z)) for 2^25 numbers of N(0, 0.3^2) to N(0, 30^2): not a bit differs.  The experts' epilogue, 128 SiLUs a thread and tile, was bound by that branch: 2048 rows of 2048 channels, 16 experts, up projection 95 -> 73 us, of 1024 channels 60 -> 26.
+__device__ __forceinline__ float over(float y, float d) {
+  constexpr float S = 0.00390625f;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d * S));
+  const float q = (y * S) * r, better = fmaf(fmaf(-q, d, y) * S, r, q);
+  return better == better ? better : q;
+}
+
 __device__ __forceinline__ float act_apply(float z, int act) {
   switch (act) {
     case LIA_ACT_RELU: return fmaxf(z, 0.f);
-    case LIA_ACT_SILU: return z / (1.0f + expf(-z));
+    case LIA_ACT_SILU: return over(z, 1.0f + expf(-z));
     case LIA_ACT_GELU_ERF: return 0.5f * z * (1.0f + erff(z * 0.70710678118654752440f));
     case LIA_ACT_GELU_TANH: return 0.5f * z * (1.0f + tanhf(0.79788456080286535588f * (z + 0.044715f * z * z * z)));
     case LIA_ACT_RELU_SQUARED: return fmaxf(z, 0.f) * fmaxf(z, 0.f);
@@ -21,7 +32,7 @@ __device__ __forceinline__ float gated_apply(float g, float u, int act, float p0
   if (act == LIA_ACT_CLAMPED_SWISH) {
     g = fminf(g, p0);
     u = fminf(fmaxf(u, -p0), p0);
-    return g / (1.0f + expf(-p1 * g)) * (u + 1.0f);
+    return over(g, 1.0f + expf(-p1 * g)) * (u + 1.0f);
   }
   return act_apply(g, act) * u;
 }

@@ -289,12 +289,13 @@ template <int MODE, int COLS> int launch_as(const CUtensorMap& tmA, const CUtens
   return LIA_OK;
 }
 
-// The narrow tile where its rounds over the SMs, at half a wide tile's time and a little more, come out shorter (16 experts of 1408 gated columns on one row
-// tile each: 176 wide tiles are two rounds, 352 narrow ones one and a half: 79 -> 62 us).
+// What a tile takes is its operands' way from L2 (13 TB/s for all SMs; the tensor cores alone would take half that time): 384 rows of 128 bytes a block of K for the wide tile, 256 for the
+// narrow one, which is taken where its rounds over the SMs come out shorter or alike.  2048 rows, 16 gated experts of 1408 columns, K = 2048, at most 48 row tiles: 4 wide rounds 55 us,
+// 8 narrow ones 73; on one row tile each, 2 and 3 rounds: 79 and 62 us.
 template <int MODE> int launch(const void* W, uint64_t w_rows, int K, const CUtensorMap& tmA, const MoeArgs& a, cudaStream_t stream) {
   const int per_wide = MODE == UP_GATED ? 128 : 256, sms = lia_sm_count();
   const long long wide = (long long)a.n_tiles * ((a.N + per_wide - 1) / per_wide), narrow = (long long)a.n_tiles * ((a.N + per_wide / 2 - 1) / (per_wide / 2));
-  const bool use_narrow = ((narrow + sms - 1) / sms) * 9 < ((wide + sms - 1) / sms) * 16;
+  const bool use_narrow = ((narrow + sms - 1) / sms) * 2 <= ((wide + sms - 1) / sms) * 3;
   CUtensorMap tmB;
   const int rc = lia_make_tmap_2d(&tmB, W, w_rows, K, K, use_narrow ? 64 : 128);
   if (rc != LIA_OK) return rc;
