@@ -31,10 +31,14 @@ template <int N, typename Dist> __device__ __forceinline__ void finish_scores(fl
 #pragma unroll
   for (int i = 0; i < N; ++i) s[i] *= mul;
   if (a.softcap > 0.f) {
+    // s / softcap as the division rounds it, without its branch: the product with the reciprocal, corrected once by its remainder (P. Markstein, Computation of elementary functions
+    // on the IBM RISC System/6000, 1990); an infinite score leaves no remainder to correct by
+    const float inv = 1.0f / a.softcap;
     float top = 0.f;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      s[i] = s[i] / a.softcap;
+      const float q = s[i] * inv, better = fmaf(fmaf(-q, a.softcap, s[i]), inv, q);
+      s[i] = better == better ? better : q;
       top = fmaxf(top, fabsf(s[i]));
       if (s[i] != s[i]) top = INFINITY;
     }
