@@ -1,0 +1,219 @@
+// C[b][m][n] = sum_k A[b][m][k] W[b][n][k] on mma.sync for bf16 numbers where few rows or few columns leave the tcgen05 GEMM's tiles empty: the projections of decoded tokens,
+// logits, gates and routers.
+//
+// A step of decoded tokens is a chain of small projections, and what the tcgen05 GEMM takes for one is latency: tensor maps, barriers, TMEM, a ring that fills, partial sums that change
+// hands.  Here the weights go straight from global memory into the operands' registers, before the previous kernel has ended (they do not depend on it): 16 bytes of a weight row are two
+// operands' worth of k, and as the rows of A are read the same way the order of the k within 32 does not matter.  A block makes 16 or 32 columns of 8 to 32 rows, its 8 warps an eighth of K
+// each; they meet once, in shared memory.
+//
+// The tensor cores cut sums off below the 24th bit: those over 32 k are made apart and added in fp32.  Where the result is fp32 those over 16 are, what a warp's sum rounds off is added up apart
+// and the warps' sums meet in 64 bits; against 64 bits: K = 128, 1024, 4096: off by 4.3e-8, 4.4e-8, 4.4e-8 (FMA chains: 4.8e-8, 6.9e-8, 9.5e-8).  A row's result does not depend on the rows beside
+// it: neither the share of a warp nor the order of its sums looks at M.
+//
+// Bound: latency, then the rows' way from L2 (every block reads its rows of A whole).
+#include <math.h>
+
+#include <type_traits>
+
+#include "gemm_shared.cuh"
+#include "linear_rows_mma.cuh"
+#include "mma.cuh"
+
+namespace {
+
+constexpr int WARPS = 8;
+
+struct RowsArgs {
+  const bf16 *A, *W;
+  void* C;
+  long long lda, sA, ldw, sW, ldc, sC;
+  int M, N, K;
+  float scale;
+  const float* bias;                           // gates
+  int mode;
+  float cap;
+};
+
+enum { OUT_EPILOGUE, OUT_FP32, OUT_ROUNDED, OUT_GATES };
+
+__device__ __forceinline__ uint4 ldg_once(const bf16* p) {
+  uint4 r;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+  return r;
+}
+
+// A block: 8 NT rows times 16 MT columns.  CB: blocks of 32 k in registers at a time
+template <int NT, int MT, int CB> struct Form {
+  static constexpr int ROWS = 8 * NT, COLS = 16 * MT, PITCH = COLS + 4, SMEM = WARPS * ROWS * PITCH * 4;
+  static constexpr int REGS = 4 * NT * MT + CB * 4 * (2 * MT + NT);                  // of the sums and operands
+};
+template <int NT, int MT, int CB, int OUT>
+__global__ void __launch_bounds__(WARPS * 32, Form<NT, MT, CB>::REGS + (OUT == OUT_EPILOGUE ? 0 : 4 * NT * MT) <= 112 ? 2 : 1) linear_rows_kernel(const RowsArgs p, const EpiParams ep) {
+  using F = Form<NT, MT, CB>;
+  extern __shared__ __align__(16) float red[];                     // [WARPS][ROWS][PITCH]
+  pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int n0 = blockIdx.x * F::COLS, m0 = blockIdx.z * F::ROWS, blocks = (p.K + 31) >> 5;
+  const int first = (int)((long long)blocks * warp / WARPS), last = (int)((long long)blocks * (warp + 1) / WARPS);
+  const bf16* A = p.A + (size_t)blockIdx.y * p.sA + t * 8;
+  const bf16* W = p.W + (size_t)blockIdx.y * p.sW + t * 8;
+  uint4 w[CB][MT][2], x[CB][NT];
+  auto weights = [&](int b0) {
+#pragma unroll
+    for (int b = 0; b < CB; ++b) {
+      const int k = (b0 + b) * 32;
+      const bool live = b0 + b < last && k + t * 8 < p.K;
+#pragma unroll
+      for (int i = 0; i < 2 * MT; ++i) w[b][i >> 1][i & 1] = live ? ldg_once(W + (size_t)min(n0 + g + 8 * i, p.N - 1) * p.ldw + k) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  weights(first);
+  pdl_wait();
+  float acc[NT][MT][4] = {}, left[OUT == OUT_EPILOGUE ? 1 : NT][MT][4] = {};
+  auto add = [&](const float* c, int nt, int mt) {                 // what the sum rounds off is kept, exactly (Knuth's two-sum), in a sum of its own
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float& sum = acc[nt][mt][e];
+      const float next = sum + c[e], back = next - sum;
+      left[OUT == OUT_EPILOGUE ? 0 : nt][mt][e] += (sum - (next - back)) + (c[e] - back);
+      sum = next;
+    }
+  };
+#pragma unroll 1
+  for (int b0 = first; b0 < last; b0 += CB) {
+#pragma unroll
+    for (int b = 0; b < CB; ++b) {
+      const int k = (b0 + b) * 32;
+      const bool live = b0 + b < last && k + t * 8 < p.K;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) x[b][nt] = live ? ldg_act(A + (size_t)min(m0 + nt * 8 + g, p.M - 1) * p.lda + k) : make_uint4(0, 0, 0, 0);
+    }
+    if (b0 > first) weights(b0);
+#pragma unroll
+    for (int b = 0; b < CB; ++b) {
+      if (b0 + b >= last) break;
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        const uint4 u = w[b][mt][0], d = w[b][mt][1];
+        const uint32_t lo[4] = {u.x, d.x, u.y, d.y}, hi[4] = {u.z, d.z, u.w, d.w};
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          float c[4];
+          mma_bf16_first(c, lo, x[b][nt].x, x[b][nt].y);
+          if constexpr (OUT == OUT_EPILOGUE) {
+            mma_bf16(c, hi, x[b][nt].z, x[b][nt].w);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[nt][mt][e] += c[e];
+          } else {
+            float c2[4];
+            mma_bf16_first(c2, hi, x[b][nt].z, x[b][nt].w);
+            add(c, nt, mt);
+            add(c2, nt, mt);
+          }
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) red[(warp * F::ROWS + nt * 8 + 2 * t + (e & 1)) * F::PITCH + mt * 16 + g + 8 * (e >> 1)] =
+            OUT == OUT_EPILOGUE || !(fabsf(acc[nt][mt][e]) < INFINITY) ? acc[nt][mt][e] : acc[nt][mt][e] + left[OUT == OUT_EPILOGUE ? 0 : nt][mt][e];     // (of an infinity nothing is left)
+  __syncthreads();
+  for (int i = threadIdx.x; i < F::ROWS * 2 * MT; i += WARPS * 32) {           // 8 columns of a row
+    const int r = i / (2 * MT), m = m0 + r, c0 = i % (2 * MT) * 8, n = n0 + c0;
+    if (m >= p.M || n >= p.N) continue;
+    using Sum = typename std::conditional<OUT == OUT_EPILOGUE, float, double>::type;
+    Sum sum[8] = {};
+#pragma unroll
+    for (int k = 0; k < WARPS; ++k) {
+      const float4* s = reinterpret_cast<const float4*>(red + (k * F::ROWS + r) * F::PITCH + c0);
+      const float4 a = s[0], b = s[1];
+      sum[0] += a.x, sum[1] += a.y, sum[2] += a.z, sum[3] += a.w, sum[4] += b.x, sum[5] += b.y, sum[6] += b.z, sum[7] += b.w;
+    }
+    float v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = (float)sum[e];
+    if constexpr (OUT == OUT_EPILOGUE) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = bf16r(v[e]);
+      epilogue_store8(ep, m, n, v);
+    } else {
+      const int live = min(8, p.N - n);
+      const size_t at = (size_t)blockIdx.y * p.sC + (size_t)m * p.ldc + n;
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (e < live) {
+          if constexpr (OUT == OUT_FP32) {
+            reinterpret_cast<float*>(p.C)[at + e] = v[e] * p.scale;
+          } else if constexpr (OUT == OUT_ROUNDED) {
+            reinterpret_cast<bf16*>(p.C)[at + e] = __float2bfloat16_rn(v[e] * p.scale);
+          } else {
+            float z = v[e] + (p.bias ? p.bias[n + e] : 0.f);
+            if (p.mode == 1) {
+              z = p.cap * tanhf(z / p.cap);
+              if (n + e >= p.N / 2) z = fminf(z, 0.f) - log1pf(expf(-fabsf(z)));
+            } else if (p.mode == 2) {
+              z = 1.0f / (1.0f + expf(-z));
+            }
+            reinterpret_cast<float*>(p.C)[at + e] = z;
+          }
+        }
+    }
+  }
+}
+
+template <int NT, int MT, int CB, int OUT> int launch_rows_as(const RowsArgs& p, const EpiParams& ep, int batch, cudaStream_t stream) {
+  using F = Form<NT, MT, CB>;
+  if (F::SMEM > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(linear_rows_kernel<NT, MT, CB, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM));
+  lia_launch(linear_rows_kernel<NT, MT, CB, OUT>, dim3((p.N + F::COLS - 1) / F::COLS, batch, (p.M + F::ROWS - 1) / F::ROWS), dim3(WARPS * 32), F::SMEM, stream, p, ep);
+  LIA_LAUNCH_CHECK();
+  return LIA_OK;
+}
+template <int OUT> int launch_rows(const RowsArgs& p, const EpiParams& ep, int batch, cudaStream_t stream) {
+  const int sms = lia_sm_count();
+  const long long narrow = (long long)((p.N + 15) / 16) * batch;
+  constexpr bool fp32 = OUT != OUT_EPILOGUE;                       // twice the sums' registers
+  if (p.M <= 16) {                                                 // all of a warp's share of K at once, as long as its registers leave every block an SM
+    const bool deep = p.K > 8 * 32 * WARPS && narrow <= sms;
+    if (p.M <= 8) return deep ? launch_rows_as<1, 1, 12, OUT>(p, ep, batch, stream) : launch_rows_as<1, 1, fp32 ? 6 : 8, OUT>(p, ep, batch, stream);
+    return deep ? launch_rows_as<2, 1, 12, OUT>(p, ep, batch, stream) : launch_rows_as<2, 1, 4, OUT>(p, ep, batch, stream);
+  }
+  // few columns a block and much in flight while the blocks have an SM each, then two blocks an SM, then more columns a block, which read the rows less often: 2048 x 2048, 32 rows: 5.3 | 6.6 |
+  // 8.8 us, 64: 9.7 | 6.6 | 8.6, 128: 18.4 | 12.0 | 9.2
+  const long long blocks = narrow * ((p.M + 31) / 32);
+  if (blocks <= sms) return launch_rows_as<4, 1, 6, OUT>(p, ep, batch, stream);
+  if constexpr (fp32) return launch_rows_as<4, 1, 2, OUT>(p, ep, batch, stream);
+  else if (blocks <= 2 * sms) return launch_rows_as<4, 1, 3, OUT>(p, ep, batch, stream);
+  else return launch_rows_as<4, 2, 2, OUT>(p, ep, batch, stream);
+}
+
+}  // namespace
+
+// Weights up to 24 MB in up to 4096 rows; the line looks at the weights alone, for the other side's sums are other ones.  In a chain of projections over 300 MB of weights, 1 | 16 | 64 | 128 rows:
+// 1024 x 1024 5.7 | 5.9 | 7.8 | 10.6 us on the other side and 1.8 | 2.2 | 3.0 | 4.1 here, 2048 x 5632 8.3 | 9.0 | 14.4 | 26 and 5.8 | 7.7 | 14.3 | 21.5; beyond: 6144 x 2048 8.7 | 9.0 | 11.9 | 17
+// and 6.4 | 10.2 | 17 | 25, 5632 x 1024 5.8 | 6.1 | 8.2 | 11.9 and 4.3 | 5.4 | 9.2 | 14.
+bool gemm_rows_takes(int M, int N, int K) { return M <= 128 && N <= 4096 && (long long)N * K <= 12 << 20; }
+
+int gemm_rows(const void* A, const void* W, const void* ep, int M, int N, int K, cudaStream_t stream) {
+  const RowsArgs p{reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(W), nullptr, K, 0, K, 0, 0, 0, M, N, K, 1.f};
+  return launch_rows<OUT_EPILOGUE>(p, *reinterpret_cast<const EpiParams*>(ep), 1, stream);
+}
+
+bool linear_rows_takes(const void* A, long long lda, long long sA, const void* W, long long ldw, long long sW, int M, int K) {
+  return (M + 7) / 8 <= 65535 && K % 8 == 0 && lda % 8 == 0 && sA % 8 == 0 && ldw % 8 == 0 && sW % 8 == 0 &&
+         (reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) % 16 == 0;
+}
+
+int linear_rows(const void* A, long long lda, long long sA, const void* W, long long ldw, long long sW, void* C, int c_f32, long long ldc, long long sC, int M, int N, int K,
+                int batch, float scale, cudaStream_t stream) {
+  const RowsArgs p{reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(W), C, lda, sA, ldw, sW, ldc, sC, M, N, K, scale};
+  return c_f32 ? launch_rows<OUT_FP32>(p, EpiParams{}, batch, stream) : launch_rows<OUT_ROUNDED>(p, EpiParams{}, batch, stream);
+}
+
+int linear_rows_gates(const void* A, long long lda, const void* W, const float* bias, float* out, int M, int N, int K, int mode, float cap, cudaStream_t stream) {
+  const RowsArgs p{reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(W), out, lda, 0, K, 0, N, 0, M, N, K, 1.f, bias, mode, cap};
+  return launch_rows<OUT_GATES>(p, EpiParams{}, 1, stream);
+}

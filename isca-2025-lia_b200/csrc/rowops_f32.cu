@@ -9,7 +9,10 @@
 // Activations are bf16 or fp32 (`act_f32`); everything a norm, a gate or the residual sum computes is fp32 either way.
 #include <math.h>
 
+#include <type_traits>
+
 #include "common.cuh"
+#include "linear_rows_mma.cuh"
 
 // linear_mma.cu
 bool linear_mma_takes(const void* A, int a_f32, long long lda, long long sA, const void* W, int w_f32, long long ldw, long long sW, int M, int K, int batch);
@@ -777,6 +780,8 @@ __global__ void __launch_bounds__(256) argmax_f32_kernel(const float* __restrict
 template <typename TA, typename TW>
 int launch_plain(const void* A, long long lda, long long sA, const void* W, long long ldw, long long sW, void* C, long long ldc, long long sC,
                  int M, int N, int K, int batch, float scale, int c_f32, cudaStream_t stream) {
+  if (std::is_same<TA, bf16>::value && std::is_same<TW, bf16>::value && M <= 64 && linear_rows_takes(A, lda, sA, W, ldw, sW, M, K))
+    return linear_rows(A, lda, sA, W, ldw, sW, C, c_f32, ldc, sC, M, N, K, batch, scale, stream);
   if (M <= 64) {
     dim3 g2((N + 3) / 4, batch);
     if (c_f32)
@@ -903,6 +908,7 @@ extern "C" int lia_linear_small(const void* a, int a_f32, int lda, const void* w
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LIA_CHECK_ARG(a && w && out && M > 0 && N > 0 && K > 0 && lda >= K, "lia_linear_small: bad arguments");
   LIA_CHECK_ARG(mode >= 0 && mode <= 2 && (mode != 1 || (N % 2 == 0 && cap > 0.f)), "lia_linear_small: bad mode %d (N=%d cap=%f)", mode, N, cap);
+  if (!a_f32 && !w_f32 && linear_rows_takes(a, lda, 0, w, K, 0, M, K)) return linear_rows_gates(a, lda, w, bias, out, M, N, K, mode, cap, stream);
   const bool four = M >= 8 * lia_sm_count();
   const dim3 grid(four ? (M + 3) / 4 : M, (N + 7) / 8 < 65535 ? (N + 7) / 8 : 65535);
 #define LIA_LS(TA, TW)                                                                                                                                      \

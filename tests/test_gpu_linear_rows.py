@@ -1,0 +1,72 @@
+"""Projections of few rows or to few columns on mma.sync (csrc/linear_rows_mma.cu): around the lines of its forms, in every epilogue, strided and batched, and as gates."""
+import pytest
+import torch
+
+import lia_b200  # noqa: F401
+from lia_b200 import ops
+
+pytestmark = pytest.mark.gpu
+BF16, F32 = torch.bfloat16, torch.float32
+
+
+def _rand(*s, seed=0, std=1.0):
+    g = torch.Generator(device="cuda").manual_seed(seed + sum(s))
+    return (torch.randn(*s, generator=g, device="cuda") * std).to(BF16)
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32, 33, 128])
+@pytest.mark.parametrize("N,K", [(8, 8), (24, 40), (1000, 264), (2376, 2080), (4096, 3072)])
+@pytest.mark.parametrize("epilogue", [ops.EPI_BIAS, ops.EPI_BIAS_RELU, ops.EPI_BIAS_RESIDUAL])
+def test_epilogues(M, N, K, epilogue):
+    a, w, bias, res = _rand(M, K), _rand(N, K, std=K ** -0.5), _rand(N), _rand(M, N, seed=1)
+    r = res if epilogue == ops.EPI_BIAS_RESIDUAL else None
+    out = ops.gemm(a, w, bias, epilogue=epilogue, residual=r)
+    y = ((a.double() @ w.double().T).to(BF16).double() + bias.double()).to(BF16).double()
+    y = torch.relu(y) if epilogue == ops.EPI_BIAS_RELU else (y + res.double()).to(BF16).double() if r is not None else y
+    # bf16 after the sums, the bias and the residual; a sum that lies next to a rounding's middle may go the other way: one step of 2^-8 of sums up to 8, twice
+    assert float((out.double() - y).abs().max()) <= 0.0625 and float((out.double() != y).double().mean()) < 2e-3
+
+
+@pytest.mark.parametrize("M,N,K,batch", [(1, 5, 8, 3), (7, 16, 136, 2), (16, 33, 2088, 1), (40, 130, 512, 4), (64, 4800, 96, 1), (33, 2400, 128, 1)])
+@pytest.mark.parametrize("dtype", [F32, BF16])
+def test_plain(M, N, K, batch, dtype):
+    """A sum of 16 products is cut off at the 24th bit and what the sums of these round off is kept: at most 2^-23 of the sum of the magnitudes."""
+    a, w = _rand(M, batch * K + 8), _rand(batch, N, K + 8, std=K ** -0.5)
+    out = torch.full((M, batch * N + 3), 9.0, device="cuda").to(dtype)
+    ops.linear_plain(a, w[0], out, scale=0.5, batch=batch, a_batch_stride=K, w_batch_stride=w.stride(0), out_batch_stride=N, n=N, k=K)
+    for b in range(batch):
+        x, y = a[:, b * K:(b + 1) * K].double(), w[b, :, :K].double()
+        want, size = 0.5 * x @ y.T, 0.5 * x.abs() @ y.abs().T
+        err = (out[:, b * N:(b + 1) * N].double() - want).abs()
+        assert bool((err <= 2.0 ** -23 * size + (2.0 ** -8 * want.abs() if dtype == BF16 else 0.0)).all())
+    assert bool((out[:, batch * N:] == 9.0).all())
+
+
+@pytest.mark.parametrize("M", [1, 9, 40, 300])
+@pytest.mark.parametrize("N,K", [(2, 64), (16, 2048), (34, 136)])
+@pytest.mark.parametrize("mode", [ops.GATE_NONE, ops.GATE_LOG_INPUT_FORGET, ops.GATE_SIGMOID])
+def test_gates(M, N, K, mode):
+    a, w, bias = _rand(M, K + 8)[:, :K], _rand(N, K, std=K ** -0.5), _rand(N).float()
+    out = torch.empty(M, N, device="cuda")
+    ops.linear_small(a, w, bias, out, mode, 15.0)
+    z = a.double() @ w.double().T + bias.double()
+    if mode == ops.GATE_LOG_INPUT_FORGET:
+        z = 15.0 * torch.tanh(z / 15.0)
+        z[:, N // 2:] = torch.nn.functional.logsigmoid(z[:, N // 2:])
+    elif mode == ops.GATE_SIGMOID:
+        z = torch.sigmoid(z)
+    assert float((out.double() - z).abs().max()) < 3e-6        # sums up to 8 rounded at 2^-24 of their terms, then functions of slope 1 at most
+    few = torch.empty(1, N, device="cuda")
+    ops.linear_small(a[:1], w, bias, few, mode, 15.0)
+    assert torch.equal(few, out[:1])
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_a_bad_number_stays_in_its_row(bad):
+    a, w = _rand(20, 256), _rand(48, 256, std=0.06)
+    clean, out = torch.empty(20, 48, device="cuda"), torch.empty(20, 48, device="cuda")
+    ops.linear_plain(a, w, clean)
+    a[5, 77] = bad
+    ops.linear_plain(a, w, out)
+    rest = [r for r in range(20) if r != 5]
+    assert torch.equal(out[rest], clean[rest]) and torch.equal(out[5].isnan(), (a[5:6].float() @ w.float().T)[0].isnan())
