@@ -1,5 +1,9 @@
 // Activations of feed-forwards, shared by the row kernels and the experts' projections.
 #pragma once
+#include <math.h>
+
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace {
@@ -35,6 +39,18 @@ __device__ __forceinline__ float gated_apply(float g, float u, int act, float p0
     return over(g, 1.0f + expf(-p1 * g)) * (u + 1.0f);
   }
   return act_apply(g, act) * u;
+}
+
+// use(std::integral_constant<int, act>): the activation chosen once for a block of numbers
+template <typename F> __device__ __forceinline__ void act_chosen(int act, F use) {
+  switch (act) {
+    case LIA_ACT_RELU: return use(std::integral_constant<int, LIA_ACT_RELU>());
+    case LIA_ACT_SILU: return use(std::integral_constant<int, LIA_ACT_SILU>());
+    case LIA_ACT_GELU_ERF: return use(std::integral_constant<int, LIA_ACT_GELU_ERF>());
+    case LIA_ACT_GELU_TANH: return use(std::integral_constant<int, LIA_ACT_GELU_TANH>());
+    case LIA_ACT_RELU_SQUARED: return use(std::integral_constant<int, LIA_ACT_RELU_SQUARED>());
+    default: return use(std::integral_constant<int, LIA_ACT_NONE>());
+  }
 }
 
 }  // namespace

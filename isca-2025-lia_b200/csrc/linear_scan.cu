@@ -31,6 +31,7 @@
 #include <limits.h>
 #include <math.h>
 
+#include "act.cuh"
 #include "common.cuh"
 
 namespace {
@@ -39,7 +40,7 @@ template <typename T> __device__ __forceinline__ float ldf(const T* p);
 template <> __device__ __forceinline__ float ldf<float>(const float* p) { return *p; }
 template <> __device__ __forceinline__ float ldf<bf16>(const bf16* p) { return __bfloat162float(*p); }
 
-__device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
+__device__ __forceinline__ float silu(float z) { return over(z, 1.0f + expf(-z)); }
 
 // ---------------------------------------------------------------------------------------------------- convolution + gates
 constexpr int MAX_TAPS = 16;
@@ -51,8 +52,9 @@ struct ConvCols {          // where the q, k, v channels sit in a row of the pro
 
 // Block per token row.  meta[row] = {slot, position}; rows of one portion are consecutive and so are their positions.
 // state [slot][taps-1][C] holds the inputs of the taps - 1 positions before the portion (zero before the sequence's start).
-template <typename T>
-__global__ void __launch_bounds__(256) conv_prep_kernel(const T* __restrict__ y, int ld, ConvCols cc, const float* __restrict__ wconv,
+// TM: at least the taps, whose inputs are asked for together.  Few rows get 1024 threads each (an engine session's 16 steps of 4 rows of 2048 channels and a prompt: 201 us with 256 and one input after the other, 106 so).
+template <typename T, int TM>
+__global__ void __launch_bounds__(1024) conv_prep_kernel(const T* __restrict__ y, int ld, ConvCols cc, const float* __restrict__ wconv,
                                                         const float* __restrict__ state, const int* __restrict__ meta, float* __restrict__ gates,
                                                         const float* __restrict__ a_log, const float* __restrict__ dt_bias, float* __restrict__ qk,
                                                         float* __restrict__ v, int G, int H, int dim, int vdim, int taps, float q_scale,
@@ -66,27 +68,34 @@ __global__ void __launch_bounds__(256) conv_prep_kernel(const T* __restrict__ y,
   int inside = 1;                               // rows row-1 .. row-(inside-1) belong to this portion
   while (inside < taps && row - inside >= 0 && meta[2 * (row - inside)] == slot && meta[2 * (row - inside) + 1] == pos - inside) ++inside;
   const float* st = state + (size_t)slot * (taps - 1) * C;
-  for (int c = threadIdx.x; c < C; c += 256) {
+  for (int c = threadIdx.x; c < C; c += blockDim.x) {
     const int col = cc.col(c);
-    float acc = 0.f;
-    for (int j = 0; j < taps; ++j) {            // j tokens back
-      const float xin = j < inside ? ldf(y + (size_t)(row - j) * ld + col) : st[(size_t)(inside - 1 - j + taps - 1) * C + c];
-      acc = fmaf(wconv[(size_t)c * taps + taps - 1 - j], xin, acc);
+    float acc = 0.f, xin[TM], w[TM];
+#pragma unroll
+    for (int j = 0; j < TM; ++j) {              // j tokens back
+      xin[j] = w[j] = 0.f;
+      if (j < taps) {
+        xin[j] = j < inside ? ldf(y + (size_t)(row - j) * ld + col) : st[(size_t)(inside - 1 - j + taps - 1) * C + c];
+        w[j] = wconv[(size_t)c * taps + taps - 1 - j];
+      }
     }
+#pragma unroll
+    for (int j = 0; j < TM; ++j)
+      if (j < taps) acc = fmaf(w[j], xin[j], acc);
     acc = silu(acc);
     ch[c] = acc;
     if (c >= cc.nq + cc.nk) v[(size_t)row * cc.nv + c - cc.nq - cc.nk] = acc;
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int hd = warp; hd < 2 * G; hd += 8) {    // q heads, then k heads
+  for (int hd = warp; hd < 2 * G; hd += blockDim.x >> 5) {         // q heads, then k heads
     float ss = 0.f;
     for (int i = lane; i < dim; i += 32) ss += ch[hd * dim + i] * ch[hd * dim + i];
     ss = warp_sum(ss);
     const float inv = (hd < G ? q_scale : 1.0f) / sqrtf(ss + unit_eps);
     for (int i = lane; i < dim; i += 32) qk[(size_t)row * (cc.nq + cc.nk) + hd * dim + i] = ch[hd * dim + i] * inv;
   }
-  for (int h = threadIdx.x; h < H; h += 256) {
+  for (int h = threadIdx.x; h < H; h += blockDim.x) {
     float* gr = gates + (size_t)row * 2 * H;
     const float zb = gr[h], za = gr[H + h] + dt_bias[h];
     const float softplus = fmaxf(za, 0.f) + log1pf(expf(-fabsf(za)));
@@ -453,27 +462,10 @@ constexpr int CONV_STRIP = 8;
 __device__ __forceinline__ float silu_fast(float z) { return __fdividef(z, 1.0f + expf(-z)); }
 __device__ __forceinline__ float gelu_tanh(float z) { return 0.5f * z * (1.0f + tanhf(0.79788456080286535588f * (z + 0.044715f * z * z * z))); }
 
+// rows r0 .. r1 - 1 of channel c, wherever their portions begin
 template <typename T, int TM>
-__global__ void __launch_bounds__(256) conv_act_kernel(const T* __restrict__ y, const float* __restrict__ in_bias, const float* __restrict__ wconv,
-                                                       const float* __restrict__ bias, float* __restrict__ state, const int* __restrict__ meta,
-                                                       float* __restrict__ out, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
-                                                       float* __restrict__ gates, ConvActArgs a) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int c = blockIdx.x * 256 + threadIdx.x;
-  const int r0 = blockIdx.y * a.strip, r1 = min(a.M, r0 + a.strip);
-  if (c >= a.C + a.H) return;
-  if (c >= a.C) {
-    const int h = c - a.C;
-    const float rate = -expf(a_log[h]), b = dt_bias[h];
-    for (int r = r0; r < r1; ++r) {
-      const float z = ldf(y + (size_t)r * a.ld + a.dt_col + h) + b;
-      const float dt = fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)));
-      gates[(size_t)r * 2 * a.H + h] = dt;
-      gates[(size_t)r * 2 * a.H + a.H + h] = expf(rate * dt);
-    }
-    return;
-  }
+__device__ __forceinline__ void conv_channel(const T* __restrict__ y, const float* __restrict__ in_bias, const float* __restrict__ wconv, const float* __restrict__ bias,
+                                             float* __restrict__ state, const int* __restrict__ meta, float* __restrict__ out, const ConvActArgs& a, int c, int r0, int r1) {
   const T* col = y + a.col0 + c;
   const float ib = in_bias ? in_bias[c] : 0.f, ob = bias ? bias[c] : 0.f;
   float w[TM], win[TM];                          // by tokens back
@@ -481,24 +473,6 @@ __global__ void __launch_bounds__(256) conv_act_kernel(const T* __restrict__ y, 
   for (int j = 0; j < TM; ++j) {
     w[j] = j < a.taps ? wconv[(size_t)c * a.taps + a.taps - 1 - j] : 0.f;
     win[j] = 0.f;
-  }
-  if (r1 - r0 == CONV_STRIP && r0 >= TM - 1) {
-    // a whole strip in the middle of a portion: all its inputs are rows of y, fetched together
-    const int slot = meta[2 * r0], pos = meta[2 * r0 + 1];
-    if (meta[2 * (r1 - 1)] == slot && meta[2 * (r1 - 1) + 1] == pos + CONV_STRIP - 1 && meta[2 * (r0 - TM + 1)] == slot && meta[2 * (r0 - TM + 1) + 1] == pos - TM + 1) {
-      float in[CONV_STRIP + TM - 1];
-#pragma unroll
-      for (int i = 0; i < CONV_STRIP + TM - 1; ++i) in[i] = ldf(col + (size_t)(r0 - TM + 1 + i) * a.ld);
-#pragma unroll
-      for (int i = 0; i < CONV_STRIP; ++i) {
-        float acc = ob;
-#pragma unroll
-        for (int j = 0; j < TM; ++j) acc = fmaf(w[j], in[i + TM - 1 - j] + ib, acc);       // (weights beyond the taps are zero)
-        if (a.act == LIA_ACT_SILU) acc = silu_fast(acc);
-        out[(size_t)(r0 + i) * a.ldo + c] = acc;
-      }
-      return;
-    }
   }
   int pslot = -1, ppos = -1;
   for (int r = r0; r < r1; ++r) {
@@ -533,6 +507,80 @@ __global__ void __launch_bounds__(256) conv_act_kernel(const T* __restrict__ y, 
     pslot = slot;
     ppos = pos;
   }
+}
+
+__device__ __forceinline__ float2 ld_pair(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ float2 ld_pair(const bf16* p) {
+  float2 f;
+  unpack_bf16x2(*reinterpret_cast<const uint32_t*>(p), f.x, f.y);
+  return f;
+}
+
+// CH: channels per thread (2: rows of y, out, biases and weights are whole pairs)
+template <typename T, int TM, int CH>
+__global__ void __launch_bounds__(256) conv_act_kernel(const T* __restrict__ y, const float* __restrict__ in_bias, const float* __restrict__ wconv,
+                                                       const float* __restrict__ bias, float* __restrict__ state, const int* __restrict__ meta,
+                                                       float* __restrict__ out, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
+                                                       float* __restrict__ gates, ConvActArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int e = blockIdx.x * 256 + threadIdx.x, own = a.C / CH;
+  const int r0 = blockIdx.y * a.strip, r1 = min(a.M, r0 + a.strip);
+  if (e >= own + a.H) return;
+  if (e >= own) {
+    const int h = e - own;
+    const float rate = -expf(a_log[h]), b = dt_bias[h];
+    for (int r = r0; r < r1; ++r) {
+      const float z = ldf(y + (size_t)r * a.ld + a.dt_col + h) + b;
+      const float dt = fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)));
+      gates[(size_t)r * 2 * a.H + h] = dt;
+      gates[(size_t)r * 2 * a.H + a.H + h] = expf(rate * dt);
+    }
+    return;
+  }
+  const int c = e * CH;
+  if (r1 - r0 == CONV_STRIP && r0 >= TM - 1) {
+    // a whole strip in the middle of a portion: all its inputs are rows of y, fetched together
+    const int slot = meta[2 * r0], pos = meta[2 * r0 + 1];
+    if (meta[2 * (r1 - 1)] == slot && meta[2 * (r1 - 1) + 1] == pos + CONV_STRIP - 1 && meta[2 * (r0 - TM + 1)] == slot && meta[2 * (r0 - TM + 1) + 1] == pos - TM + 1) {
+      const T* col = y + a.col0 + c;
+      float in[CONV_STRIP + TM - 1][CH], w[TM][CH], ib[CH], ob[CH];
+#pragma unroll
+      for (int i = 0; i < CONV_STRIP + TM - 1; ++i) {
+        const T* at = col + (size_t)(r0 - TM + 1 + i) * a.ld;
+        if constexpr (CH == 2) {
+          const float2 v = ld_pair(at);
+          in[i][0] = v.x, in[i][CH - 1] = v.y;
+        } else {
+          in[i][0] = ldf(at);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < CH; ++k) {
+        ib[k] = in_bias ? in_bias[c + k] : 0.f;
+        ob[k] = bias ? bias[c + k] : 0.f;
+#pragma unroll
+        for (int j = 0; j < TM; ++j) w[j][k] = j < a.taps ? wconv[(size_t)(c + k) * a.taps + a.taps - 1 - j] : 0.f;
+      }
+#pragma unroll
+      for (int i = 0; i < CONV_STRIP; ++i) {
+        float acc[CH];
+#pragma unroll
+        for (int k = 0; k < CH; ++k) {
+          acc[k] = ob[k];
+#pragma unroll
+          for (int j = 0; j < TM; ++j) acc[k] = fmaf(w[j][k], in[i + TM - 1 - j][k] + ib[k], acc[k]);       // (weights beyond the taps are zero)
+          if (a.act == LIA_ACT_SILU) acc[k] = silu_fast(acc[k]);
+        }
+        float* to = out + (size_t)(r0 + i) * a.ldo + c;
+        if constexpr (CH == 2) *reinterpret_cast<float2*>(to) = make_float2(acc[0], acc[CH - 1]);
+        else *to = acc[0];
+      }
+      return;
+    }
+  }
+#pragma unroll 1
+  for (int k = 0; k < CH; ++k) conv_channel<T, TM>(y, in_bias, wconv, bias, state, meta, out, a, c + k, r0, r1);
 }
 
 // ---------------------------------------------------------------------------------------------------- state-space duality
@@ -858,13 +906,18 @@ extern "C" int lia_conv_prep(const void* y, int y_f32, int ld, int q_off, int k_
   ConvCols cc{q_off, k_off, v_off, G * dim, G * dim, H * vdim};
   const size_t smem = (size_t)(cc.nq + cc.nk + cc.nv) * sizeof(float);
   LIA_CHECK_ARG(smem <= 160 * 1024, "lia_conv_prep: %d channels do not fit shared memory", cc.nq + cc.nk + cc.nv);
-  if (y_f32) {
-    if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(conv_prep_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    lia_launch(conv_prep_kernel<float>, dim3(M), dim3(256), smem, stream, reinterpret_cast<const float*>(y), ld, cc, wconv, conv_state, meta, gates, a_log, dt_bias, qk, v, G, H, dim, vdim, taps, q_scale, unit_eps);
-  } else {
-    if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(conv_prep_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    lia_launch(conv_prep_kernel<bf16>, dim3(M), dim3(256), smem, stream, reinterpret_cast<const bf16*>(y), ld, cc, wconv, conv_state, meta, gates, a_log, dt_bias, qk, v, G, H, dim, vdim, taps, q_scale, unit_eps);
-  }
+  const int threads = M <= 64 ? 1024 : 256;
+#define LIA_CP(T, TM)                                                                                                                                                    \
+  do {                                                                                                                                                                   \
+    if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(conv_prep_kernel<T, TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));                               \
+    lia_launch(conv_prep_kernel<T, TM>, dim3(M), dim3(threads), smem, stream, reinterpret_cast<const T*>(y), ld, cc, wconv, conv_state, meta, gates, a_log, dt_bias, qk, v, G, H, dim, \
+               vdim, taps, q_scale, unit_eps);                                                                                                                           \
+  } while (0)
+  if (y_f32 && taps <= 4) LIA_CP(float, 4);
+  else if (y_f32) LIA_CP(float, MAX_TAPS);
+  else if (taps <= 4) LIA_CP(bf16, 4);
+  else LIA_CP(bf16, MAX_TAPS);
+#undef LIA_CP
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -935,15 +988,20 @@ extern "C" int lia_conv_act(const void* y, int y_f32, int ld, int col0, int C, c
   LIA_CHECK_ARG(H >= 0 && (H == 0 || (dt_bias && a_log && gates && dt_col >= 0 && ld >= dt_col + H)), "lia_conv_act: bad step sizes (H=%d)", H);
   const int single = nseg == M && taps > 1;      // every portion is one row
   ConvActArgs a{ld, col0, C, taps, act, single, ldo, M, M <= 64 ? 1 : CONV_STRIP, dt_col, H};
-  dim3 grid((C + H + 255) / 256, (M + a.strip - 1) / a.strip);
+  // pairs of channels where strips of rows are made and every row is whole pairs (2048 rows of 6144 channels: 25 us one by one, 22 so)
+  const bool pairs = M > 64 && taps <= 4 && C % 2 == 0 && ld % 2 == 0 && col0 % 2 == 0 && ldo % 2 == 0 && reinterpret_cast<uintptr_t>(y) % (y_f32 ? 8 : 4) == 0 &&
+                     reinterpret_cast<uintptr_t>(out) % 8 == 0;
+  dim3 grid(((pairs ? C / 2 : C) + H + 255) / 256, (M + a.strip - 1) / a.strip);
   LIA_CHECK_ARG(grid.y <= 65535, "lia_conv_act: too many rows (%d)", M);
-#define LIA_CA(T, TM) lia_launch(conv_act_kernel<T, TM>, dim3(grid), dim3(256), 0, stream, reinterpret_cast<const T*>(y), in_bias, wconv, bias, state, meta, out, dt_bias, a_log, gates, a)
+#define LIA_CA(T, TM, CH) lia_launch(conv_act_kernel<T, TM, CH>, dim3(grid), dim3(256), 0, stream, reinterpret_cast<const T*>(y), in_bias, wconv, bias, state, meta, out, dt_bias, a_log, gates, a)
   if (y_f32) {
-    if (taps <= 4) LIA_CA(float, 4);
-    else LIA_CA(float, MAX_TAPS);
+    if (pairs) LIA_CA(float, 4, 2);
+    else if (taps <= 4) LIA_CA(float, 4, 1);
+    else LIA_CA(float, MAX_TAPS, 1);
   } else {
-    if (taps <= 4) LIA_CA(bf16, 4);
-    else LIA_CA(bf16, MAX_TAPS);
+    if (pairs) LIA_CA(bf16, 4, 2);
+    else if (taps <= 4) LIA_CA(bf16, 4, 1);
+    else LIA_CA(bf16, MAX_TAPS, 1);
   }
 #undef LIA_CA
   LIA_LAUNCH_CHECK();

@@ -19,6 +19,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "act.cuh"
 #include "rowvec.cuh"
 
 int mlstm_take_state(const float* ws, const int* segs, int nseg, float* nst, float* mst, int H, int dim, cudaStream_t stream);
@@ -300,41 +301,45 @@ __global__ void __launch_bounds__(256) headnorm_gate_vec_kernel(const float* __r
   const int h = (int)(pair - row * H);
   const float* orow = o + pair * vdim;
   constexpr int KEEP = 4;                                   // vectors per thread that stay in registers between the two passes
-  float4 v[KEEP];
+  const T* grow = gate != nullptr ? gate + row * ldg + (size_t)h * vdim : nullptr;
+  const float* wrow = w + (size_t)h * vdim;
+  float4 v[KEEP], z[KEEP], g[KEEP];                         // (weights and gates are asked for before the sum is waited for)
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < KEEP; ++i) {
     const int c = (t + i * N) * 4;
     if (c < vdim) {
       v[i] = load4(orow + c);
-      ss += dot4(v[i], v[i]);
+      g[i] = load4(wrow + c);
+      if (grow != nullptr) z[i] = load4(grow + c);
     }
   }
+#pragma unroll
+  for (int i = 0; i < KEEP; ++i)
+    if ((t + i * N) * 4 < vdim) ss += dot4(v[i], v[i]);
   for (int c = (t + KEEP * N) * 4; c < vdim; c += N * 4) {
     const float4 u = load4(orow + c);
     ss += dot4(u, u);
   }
   ss = WIDE ? block_sum256(ss, red) : warp_sum(ss);
   const float inv = 1.0f / sqrtf(ss / (float)vdim + eps);
-  auto finish = [&](int c, const float4& u) {
-    const float4 g = load4(w + (size_t)h * vdim + c);
-    float4 y = make_float4(u.x * inv * g.x, u.y * inv * g.y, u.z * inv * g.z, u.w * inv * g.w);
-    if (gate != nullptr) {
-      const float4 z = load4(gate + row * ldg + (size_t)h * vdim + c);
-      const float4 s = make_float4(1.0f / (1.0f + expf(-z.x)), 1.0f / (1.0f + expf(-z.y)), 1.0f / (1.0f + expf(-z.z)), 1.0f / (1.0f + expf(-z.w)));
-      y.x *= gate_silu ? z.x * s.x : s.x;
-      y.y *= gate_silu ? z.y * s.y : s.y;
-      y.z *= gate_silu ? z.z * s.z : s.z;
-      y.w *= gate_silu ? z.w * s.w : s.w;
+  auto finish = [&](int c, const float4& u, const float4& f, const float4& q) {
+    float4 y = make_float4(u.x * inv * f.x, u.y * inv * f.y, u.z * inv * f.z, u.w * inv * f.w);
+    if (grow != nullptr) {
+      const float4 s = make_float4(over(1.0f, 1.0f + expf(-q.x)), over(1.0f, 1.0f + expf(-q.y)), over(1.0f, 1.0f + expf(-q.z)), over(1.0f, 1.0f + expf(-q.w)));
+      y.x *= gate_silu ? q.x * s.x : s.x;
+      y.y *= gate_silu ? q.y * s.y : s.y;
+      y.z *= gate_silu ? q.z * s.z : s.z;
+      y.w *= gate_silu ? q.w * s.w : s.w;
     }
     store4(out + pair * vdim + c, y);
   };
 #pragma unroll
   for (int i = 0; i < KEEP; ++i) {
     const int c = (t + i * N) * 4;
-    if (c < vdim) finish(c, v[i]);
+    if (c < vdim) finish(c, v[i], g[i], z[i]);
   }
-  for (int c = (t + KEEP * N) * 4; c < vdim; c += N * 4) finish(c, load4(orow + c));
+  for (int c = (t + KEEP * N) * 4; c < vdim; c += N * 4) finish(c, load4(orow + c), load4(wrow + c), grow != nullptr ? load4(grow + c) : make_float4(0.f, 0.f, 0.f, 0.f));
 }
 
 template <typename T, int DR, bool VL>

@@ -227,6 +227,38 @@ __global__ void __launch_bounds__(256) gated_act_vec_kernel(const T* __restrict_
   store4(out + (size_t)e * 4, v);
 }
 
+// the same, eight columns per thread (16 bytes of bf16), the activation chosen once: 1536 rows of 6144 bf16 16 -> 13.7 us
+template <typename T>
+__global__ void __launch_bounds__(256) gated_act_vec8_kernel(const T* __restrict__ in, int ld, int up_off, T* __restrict__ out, unsigned octs, int F, int act,
+                                                             const int* __restrict__ perm, const float* __restrict__ wt) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const unsigned e = blockIdx.x * 256 + threadIdx.x;
+  if (e >= octs) return;
+  const unsigned per = (unsigned)F / 8, m = e / per, f = (e - m * per) * 8;
+  float ws = 1.0f;
+  if (perm != nullptr) ws = perm[m] < 0 ? 0.f : wt[perm[m]];
+  const T* row = in + (size_t)m * ld + f;
+  const float4 a = load4(row), b = load4(row + 4);
+  float4 u = make_float4(1.f, 1.f, 1.f, 1.f), w = u;
+  if (up_off >= 0) {
+    u = load4(row + up_off);
+    w = load4(row + up_off + 4);
+  }
+  float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  const float up[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
+  act_chosen(act, [&](auto chosen) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = act_apply(ws * v[i], chosen.value);
+  });
+  if (up_off >= 0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] *= ws * up[i];
+  }
+  store4(out + (size_t)e * 8, make_float4(v[0], v[1], v[2], v[3]));
+  store4(out + (size_t)e * 8 + 4, make_float4(v[4], v[5], v[6], v[7]));
+}
+
 // ---------------------------------------------------------------------------------------------------- router
 // One warp per token: softmax over E logits (fp32), or a sigmoid of each (`sigmoid`), then `top` rounds of arg-max (lowest
 // index on ties) over the scores plus an optional per-expert correction that takes part in the choice only; a chosen expert's
@@ -660,6 +692,13 @@ extern "C" int lia_gated_act_weighted(const void* in, int ld, int up_off, void* 
   const int sz = act_f32 ? 4 : 2;
   if (F % 4 == 0 && ld % 4 == 0 && (up_off < 0 || up_off % 4 == 0) && reinterpret_cast<uintptr_t>(in) % (4 * sz) == 0 && reinterpret_cast<uintptr_t>(out) % (4 * sz) == 0 &&
       quads < (1ll << 31)) {
+    if (F % 8 == 0) {                          // (whole quads on both sides of an oct)
+      const unsigned g8 = (unsigned)((quads / 2 + 255) / 256);
+      if (act_f32) lia_launch(gated_act_vec8_kernel<float>, dim3(g8), dim3(256), 0, stream, reinterpret_cast<const float*>(in), ld, up_off, reinterpret_cast<float*>(out), (unsigned)(quads / 2), F, act, perm, wt);
+      else lia_launch(gated_act_vec8_kernel<bf16>, dim3(g8), dim3(256), 0, stream, reinterpret_cast<const bf16*>(in), ld, up_off, reinterpret_cast<bf16*>(out), (unsigned)(quads / 2), F, act, perm, wt);
+      LIA_LAUNCH_CHECK();
+      return LIA_OK;
+    }
     const unsigned g = (unsigned)((quads + 255) / 256);
     if (act_f32) lia_launch(gated_act_vec_kernel<float>, dim3(g), dim3(256), 0, stream, reinterpret_cast<const float*>(in), ld, up_off, reinterpret_cast<float*>(out), (unsigned)quads, F, act, perm, wt);
     else lia_launch(gated_act_vec_kernel<bf16>, dim3(g), dim3(256), 0, stream, reinterpret_cast<const bf16*>(in), ld, up_off, reinterpret_cast<bf16*>(out), (unsigned)quads, F, act, perm, wt);
