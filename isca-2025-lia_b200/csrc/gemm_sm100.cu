@@ -655,7 +655,7 @@ static int gemm_impl(const void* A, const void* W, const void* bias, const void*
   Plan pl;
   const int rc0 = gemm_fill_params(A, W, bias, residual, out, M, N, K, epilogue, qkv, tp, ep, pl);
   if (rc0 != LIA_OK) return rc0;
-  if (tp == nullptr && gemm_rows_takes(M, N, K)) return gemm_rows(A, W, &ep, M, N, K, stream);
+  if (tp == nullptr && epilogue == LIA_EPI_BIAS && bias == nullptr && gemm_rows_takes(M, N, K)) return gemm_rows(A, W, out, M, N, K, stream);
   float* ws = nullptr;
   int* flags = nullptr;
   if (pl.swap && pl.streamk) {

@@ -15,7 +15,6 @@
 
 #include <type_traits>
 
-#include "gemm_shared.cuh"
 #include "linear_rows_mma.cuh"
 #include "mma.cuh"
 
@@ -34,7 +33,7 @@ struct RowsArgs {
   float cap;
 };
 
-enum { OUT_EPILOGUE, OUT_FP32, OUT_ROUNDED, OUT_GATES };
+enum { OUT_GEMM, OUT_FP32, OUT_ROUNDED, OUT_GATES };              // GEMM: bf16, whole vectors, nothing kept of what the sums round off
 
 __device__ __forceinline__ uint4 ldg_once(const bf16* p) {
   uint4 r;
@@ -48,7 +47,7 @@ template <int NT, int MT, int CB> struct Form {
   static constexpr int REGS = 4 * NT * MT + CB * 4 * (2 * MT + NT);                  // of the sums and operands
 };
 template <int NT, int MT, int CB, int OUT>
-__global__ void __launch_bounds__(WARPS * 32, Form<NT, MT, CB>::REGS + (OUT == OUT_EPILOGUE ? 0 : 4 * NT * MT) <= 112 ? 2 : 1) linear_rows_kernel(const RowsArgs p, const EpiParams ep) {
+__global__ void __launch_bounds__(WARPS * 32, Form<NT, MT, CB>::REGS + (OUT == OUT_GEMM ? 0 : 4 * NT * MT) <= 112 ? 2 : 1) linear_rows_kernel(const RowsArgs p) {
   using F = Form<NT, MT, CB>;
   extern __shared__ __align__(16) float red[];                     // [WARPS][ROWS][PITCH]
   pdl_launch_dependents();
@@ -69,13 +68,13 @@ __global__ void __launch_bounds__(WARPS * 32, Form<NT, MT, CB>::REGS + (OUT == O
   };
   weights(first);
   pdl_wait();
-  float acc[NT][MT][4] = {}, left[OUT == OUT_EPILOGUE ? 1 : NT][MT][4] = {};
+  float acc[NT][MT][4] = {}, left[OUT == OUT_GEMM ? 1 : NT][MT][4] = {};
   auto add = [&](const float* c, int nt, int mt) {                 // what the sum rounds off is kept, exactly (Knuth's two-sum), in a sum of its own
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       float& sum = acc[nt][mt][e];
       const float next = sum + c[e], back = next - sum;
-      left[OUT == OUT_EPILOGUE ? 0 : nt][mt][e] += (sum - (next - back)) + (c[e] - back);
+      left[OUT == OUT_GEMM ? 0 : nt][mt][e] += (sum - (next - back)) + (c[e] - back);
       sum = next;
     }
   };
@@ -100,7 +99,7 @@ __global__ void __launch_bounds__(WARPS * 32, Form<NT, MT, CB>::REGS + (OUT == O
         for (int nt = 0; nt < NT; ++nt) {
           float c[4];
           mma_bf16_first(c, lo, x[b][nt].x, x[b][nt].y);
-          if constexpr (OUT == OUT_EPILOGUE) {
+          if constexpr (OUT == OUT_GEMM) {
             mma_bf16(c, hi, x[b][nt].z, x[b][nt].w);
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[nt][mt][e] += c[e];
@@ -120,12 +119,12 @@ __global__ void __launch_bounds__(WARPS * 32, Form<NT, MT, CB>::REGS + (OUT == O
     for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
       for (int e = 0; e < 4; ++e) red[(warp * F::ROWS + nt * 8 + 2 * t + (e & 1)) * F::PITCH + mt * 16 + g + 8 * (e >> 1)] =
-            OUT == OUT_EPILOGUE || !(fabsf(acc[nt][mt][e]) < INFINITY) ? acc[nt][mt][e] : acc[nt][mt][e] + left[OUT == OUT_EPILOGUE ? 0 : nt][mt][e];     // (of an infinity nothing is left)
+            OUT == OUT_GEMM || !(fabsf(acc[nt][mt][e]) < INFINITY) ? acc[nt][mt][e] : acc[nt][mt][e] + left[OUT == OUT_GEMM ? 0 : nt][mt][e];     // (of an infinity nothing is left)
   __syncthreads();
   for (int i = threadIdx.x; i < F::ROWS * 2 * MT; i += WARPS * 32) {           // 8 columns of a row
     const int r = i / (2 * MT), m = m0 + r, c0 = i % (2 * MT) * 8, n = n0 + c0;
     if (m >= p.M || n >= p.N) continue;
-    using Sum = typename std::conditional<OUT == OUT_EPILOGUE, float, double>::type;
+    using Sum = typename std::conditional<OUT == OUT_GEMM, float, double>::type;
     Sum sum[8] = {};
 #pragma unroll
     for (int k = 0; k < WARPS; ++k) {
@@ -136,10 +135,8 @@ __global__ void __launch_bounds__(WARPS * 32, Form<NT, MT, CB>::REGS + (OUT == O
     float v[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] = (float)sum[e];
-    if constexpr (OUT == OUT_EPILOGUE) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) v[e] = bf16r(v[e]);
-      epilogue_store8(ep, m, n, v);
+    if constexpr (OUT == OUT_GEMM) {
+      *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(p.C) + (size_t)m * p.ldc + n) = pack8(v);        // (N and ldc are multiples of 8)
     } else {
       const int live = min(8, p.N - n);
       const size_t at = (size_t)blockIdx.y * p.sC + (size_t)m * p.ldc + n;
@@ -165,29 +162,29 @@ __global__ void __launch_bounds__(WARPS * 32, Form<NT, MT, CB>::REGS + (OUT == O
   }
 }
 
-template <int NT, int MT, int CB, int OUT> int launch_rows_as(const RowsArgs& p, const EpiParams& ep, int batch, cudaStream_t stream) {
+template <int NT, int MT, int CB, int OUT> int launch_rows_as(const RowsArgs& p, int batch, cudaStream_t stream) {
   using F = Form<NT, MT, CB>;
   if (F::SMEM > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(linear_rows_kernel<NT, MT, CB, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM));
-  lia_launch(linear_rows_kernel<NT, MT, CB, OUT>, dim3((p.N + F::COLS - 1) / F::COLS, batch, (p.M + F::ROWS - 1) / F::ROWS), dim3(WARPS * 32), F::SMEM, stream, p, ep);
+  lia_launch(linear_rows_kernel<NT, MT, CB, OUT>, dim3((p.N + F::COLS - 1) / F::COLS, batch, (p.M + F::ROWS - 1) / F::ROWS), dim3(WARPS * 32), F::SMEM, stream, p);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
-template <int OUT> int launch_rows(const RowsArgs& p, const EpiParams& ep, int batch, cudaStream_t stream) {
+template <int OUT> int launch_rows(const RowsArgs& p, int batch, cudaStream_t stream) {
   const int sms = lia_sm_count();
   const long long narrow = (long long)((p.N + 15) / 16) * batch;
-  constexpr bool fp32 = OUT != OUT_EPILOGUE;                       // twice the sums' registers
+  constexpr bool fp32 = OUT != OUT_GEMM;                       // twice the sums' registers
   if (p.M <= 16) {                                                 // all of a warp's share of K at once, as long as its registers leave every block an SM
     const bool deep = p.K > 8 * 32 * WARPS && narrow <= sms;
-    if (p.M <= 8) return deep ? launch_rows_as<1, 1, 12, OUT>(p, ep, batch, stream) : launch_rows_as<1, 1, fp32 ? 6 : 8, OUT>(p, ep, batch, stream);
-    return deep ? launch_rows_as<2, 1, 12, OUT>(p, ep, batch, stream) : launch_rows_as<2, 1, 4, OUT>(p, ep, batch, stream);
+    if (p.M <= 8) return deep ? launch_rows_as<1, 1, 12, OUT>(p, batch, stream) : launch_rows_as<1, 1, fp32 ? 6 : 8, OUT>(p, batch, stream);
+    return deep ? launch_rows_as<2, 1, 12, OUT>(p, batch, stream) : launch_rows_as<2, 1, 4, OUT>(p, batch, stream);
   }
   // few columns a block and much in flight while the blocks have an SM each, then two blocks an SM, then more columns a block, which read the rows less often: 2048 x 2048, 32 rows: 5.3 | 6.6 |
   // 8.8 us, 64: 9.7 | 6.6 | 8.6, 128: 18.4 | 12.0 | 9.2
   const long long blocks = narrow * ((p.M + 31) / 32);
-  if (blocks <= sms) return launch_rows_as<4, 1, 6, OUT>(p, ep, batch, stream);
-  if constexpr (fp32) return launch_rows_as<4, 1, 2, OUT>(p, ep, batch, stream);
-  else if (blocks <= 2 * sms) return launch_rows_as<4, 1, 3, OUT>(p, ep, batch, stream);
-  else return launch_rows_as<4, 2, 2, OUT>(p, ep, batch, stream);
+  if (blocks <= sms) return launch_rows_as<4, 1, 6, OUT>(p, batch, stream);
+  if constexpr (fp32) return launch_rows_as<4, 1, 2, OUT>(p, batch, stream);
+  else if (blocks <= 2 * sms) return launch_rows_as<4, 1, 3, OUT>(p, batch, stream);
+  else return launch_rows_as<4, 2, 2, OUT>(p, batch, stream);
 }
 
 }  // namespace
@@ -195,11 +192,13 @@ template <int OUT> int launch_rows(const RowsArgs& p, const EpiParams& ep, int b
 // Weights up to 24 MB in up to 4096 rows; the line looks at the weights alone, for the other side's sums are other ones.  In a chain of projections over 300 MB of weights, 1 | 16 | 64 | 128 rows:
 // 1024 x 1024 5.7 | 5.9 | 7.8 | 10.6 us on the other side and 1.8 | 2.2 | 3.0 | 4.1 here, 2048 x 5632 8.3 | 9.0 | 14.4 | 26 and 5.8 | 7.7 | 14.3 | 21.5; beyond: 6144 x 2048 8.7 | 9.0 | 11.9 | 17
 // and 6.4 | 10.2 | 17 | 25, 5632 x 1024 5.8 | 6.1 | 8.2 | 11.9 and 4.3 | 5.4 | 9.2 | 14.
+// Only projections without a bias: OPT's all have one, and the program that chains a decoded token's operations in one launch (decode_program_sm100.cu) makes them with the GEMM's sums, which
+// its operations one by one give too.
 bool gemm_rows_takes(int M, int N, int K) { return M <= 128 && N <= 4096 && (long long)N * K <= 12 << 20; }
 
-int gemm_rows(const void* A, const void* W, const void* ep, int M, int N, int K, cudaStream_t stream) {
-  const RowsArgs p{reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(W), nullptr, K, 0, K, 0, 0, 0, M, N, K, 1.f};
-  return launch_rows<OUT_EPILOGUE>(p, *reinterpret_cast<const EpiParams*>(ep), 1, stream);
+int gemm_rows(const void* A, const void* W, void* C, int M, int N, int K, cudaStream_t stream) {
+  const RowsArgs p{reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(W), C, K, 0, K, 0, N, 0, M, N, K, 1.f};
+  return launch_rows<OUT_GEMM>(p, 1, stream);
 }
 
 bool linear_rows_takes(const void* A, long long lda, long long sA, const void* W, long long ldw, long long sW, int M, int K) {
@@ -210,10 +209,10 @@ bool linear_rows_takes(const void* A, long long lda, long long sA, const void* W
 int linear_rows(const void* A, long long lda, long long sA, const void* W, long long ldw, long long sW, void* C, int c_f32, long long ldc, long long sC, int M, int N, int K,
                 int batch, float scale, cudaStream_t stream) {
   const RowsArgs p{reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(W), C, lda, sA, ldw, sW, ldc, sC, M, N, K, scale};
-  return c_f32 ? launch_rows<OUT_FP32>(p, EpiParams{}, batch, stream) : launch_rows<OUT_ROUNDED>(p, EpiParams{}, batch, stream);
+  return c_f32 ? launch_rows<OUT_FP32>(p, batch, stream) : launch_rows<OUT_ROUNDED>(p, batch, stream);
 }
 
 int linear_rows_gates(const void* A, long long lda, const void* W, const float* bias, float* out, int M, int N, int K, int mode, float cap, cudaStream_t stream) {
   const RowsArgs p{reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(W), out, lda, 0, K, 0, N, 0, M, N, K, 1.f, bias, mode, cap};
-  return launch_rows<OUT_GATES>(p, EpiParams{}, 1, stream);
+  return launch_rows<OUT_GATES>(p, 1, stream);
 }

@@ -3,7 +3,7 @@
 #include "common.cuh"
 
 bool gemm_rows_takes(int M, int N, int K);
-int gemm_rows(const void* A, const void* W, const void* epilogue, int M, int N, int K, cudaStream_t stream);          // epilogue: an EpiParams (gemm_shared.cuh)
+int gemm_rows(const void* A, const void* W, void* C, int M, int N, int K, cudaStream_t stream);
 // rows of bf16 numbers that are whole 16-byte vectors
 bool linear_rows_takes(const void* A, long long lda, long long sA, const void* W, long long ldw, long long sW, int M, int K);
 int linear_rows(const void* A, long long lda, long long sA, const void* W, long long ldw, long long sW, void* C, int c_f32, long long ldc, long long sC, int M, int N, int K,

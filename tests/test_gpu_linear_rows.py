@@ -1,4 +1,4 @@
-"""Projections of few rows or to few columns on mma.sync (csrc/linear_rows_mma.cu): around the lines of its forms, in every epilogue, strided and batched, and as gates."""
+"""Projections of few rows or to few columns on mma.sync (csrc/linear_rows_mma.cu): around the lines of its forms, strided and batched, and as gates."""
 import pytest
 import torch
 
@@ -16,15 +16,12 @@ def _rand(*s, seed=0, std=1.0):
 
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32, 33, 128])
 @pytest.mark.parametrize("N,K", [(8, 8), (24, 40), (1000, 264), (2376, 2080), (4096, 3072)])
-@pytest.mark.parametrize("epilogue", [ops.EPI_BIAS, ops.EPI_BIAS_RELU, ops.EPI_BIAS_RESIDUAL])
-def test_epilogues(M, N, K, epilogue):
-    a, w, bias, res = _rand(M, K), _rand(N, K, std=K ** -0.5), _rand(N), _rand(M, N, seed=1)
-    r = res if epilogue == ops.EPI_BIAS_RESIDUAL else None
-    out = ops.gemm(a, w, bias, epilogue=epilogue, residual=r)
-    y = ((a.double() @ w.double().T).to(BF16).double() + bias.double()).to(BF16).double()
-    y = torch.relu(y) if epilogue == ops.EPI_BIAS_RELU else (y + res.double()).to(BF16).double() if r is not None else y
-    # bf16 after the sums, the bias and the residual; a sum that lies next to a rounding's middle may go the other way: one step of 2^-8 of sums up to 8, twice
-    assert float((out.double() - y).abs().max()) <= 0.0625 and float((out.double() != y).double().mean()) < 2e-3
+def test_projections(M, N, K):
+    """Sums rounded once to bf16; one that lies next to a rounding's middle may go the other way: one step of 2^-8 of sums up to 8."""
+    a, w = _rand(M, K), _rand(N, K, std=K ** -0.5)
+    out, y = ops.gemm(a, w, None), (a.double() @ w.double().T).to(BF16).double()
+    assert float((out.double() - y).abs().max()) <= 0.0325 and float((out.double() != y).double().mean()) < 2e-3
+    assert torch.equal(ops.gemm(a[:1], w, None), out[:1])
 
 
 @pytest.mark.parametrize("M,N,K,batch", [(1, 5, 8, 3), (7, 16, 136, 2), (16, 33, 2088, 1), (40, 130, 512, 4), (64, 4800, 96, 1), (33, 2400, 128, 1)])
