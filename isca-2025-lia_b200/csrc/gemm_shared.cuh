@@ -749,12 +749,6 @@ Plan make_plan(int M, int N, int K, bool allow_pair = false) {
     if (allow_pair) {
       const bool pairs = wide && M >= 4 * TILE_A && sms >= 2;      // as the default has it, so that one-CTA runs for comparison take the same widths
       long long best = pairs ? cost(tiles(2 * TILE_A, 256), sms / 2, 380) : cost(tiles(TILE_A, pl.bn), sms, pl.bn == 256 ? 500 : 330);
-      // between 129 and 511 rows pairs only where their rounds are the shorter ones, over a K that makes up for their start: 231 x 12288 x 4096 33.6 -> 29.6 us, 300 x 16384 x 4096 56 -> 50,
-      // 231 x 10240 x 2560 22.7 -> 21.5, 500 x 10240 x 2560 35.7 -> 31.8; 300 x 8192 x 2048 19.8 and 21.2
-      if (wide && !pairs && sms >= 2 && pl.k_blocks >= 40 && cost(tiles(2 * TILE_A, 256), sms / 2, 380) * 10 < best * 9) {
-        best = cost(tiles(2 * TILE_A, 256), sms / 2, 380);
-        pl.pair = pair_enabled();
-      }
       if (wide && cost(tiles(TILE_A, 128), sms, 330) * 10 < best * 9) {
         best = cost(tiles(TILE_A, 128), sms, 330);
         pl.bn = 128;
