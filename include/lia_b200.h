@@ -602,6 +602,9 @@ int lia_silu_gate_norm(const float* o, const void* z, int ldz, const float* w, v
 int lia_conv_act(const void* y, int y_f32, int ld, int col0, int C, const float* in_bias, const float* wconv, const float* bias, int taps, int act,
                  float* state, const int* meta, const int* segs, int nseg, float* out, int ldo, int M, int dt_col, int H, const float* dt_bias,
                  const float* a_log, float* gates, lia_stream_t stream);
+/* out[M][N] = A[M][K] W[N][K]^T in bf16: lia_gemm_bf16 without a bias, and for up to 128 rows and small weights a kernel whose sums are taken in another order; a row's result does
+ * not depend on how many rows up to 128 there are */
+int lia_linear_bf16(const void* A, const void* W, void* out, int M, int N, int K, void* workspace, size_t workspace_bytes, lia_stream_t stream);
 /* State-space dual recurrence over every portion, per head h (B and C of group h / (H / G), N <= 512 numbers; x of vdim numbers; all with
  * row stride ld):  S = g S + dt B x^T,  o = S^T C + D[h] x;  gates [rows][2H] = dt | g; state_S [slot][H][vdim][N], o [rows][H * vdim] fp32;
  * rows: tokens of all nseg portions together */

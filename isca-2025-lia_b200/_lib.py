@@ -213,6 +213,7 @@ _PROTOTYPES = {
                              c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "lia_ssd_scan": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
                              c_void_p]),
+    "lia_linear_bf16": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
     "lia_ssd_chunk_rows": (c_int, []),
     "lia_ssd_workspace": (c_longlong, [c_int, c_int, c_int, c_int, c_int, c_int, c_int]),
     "lia_ssd_scan_chunks": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,

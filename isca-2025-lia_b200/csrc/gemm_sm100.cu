@@ -655,7 +655,6 @@ static int gemm_impl(const void* A, const void* W, const void* bias, const void*
   Plan pl;
   const int rc0 = gemm_fill_params(A, W, bias, residual, out, M, N, K, epilogue, qkv, tp, ep, pl);
   if (rc0 != LIA_OK) return rc0;
-  if (tp == nullptr && epilogue == LIA_EPI_BIAS && bias == nullptr && gemm_rows_takes(M, N, K)) return gemm_rows(A, W, out, M, N, K, stream);
   float* ws = nullptr;
   int* flags = nullptr;
   if (pl.swap && pl.streamk) {
@@ -694,6 +693,16 @@ extern "C" int lia_gemm_bf16(const void* A, const void* W, const void* bias, con
   LIA_CHECK_ARG(epilogue >= LIA_EPI_BIAS && epilogue <= LIA_EPI_QKV, "lia_gemm_bf16: unknown epilogue %d", epilogue);
   return gemm_impl(A, W, bias, residual, out, M, N, K, epilogue, qkv, nullptr, workspace, workspace_bytes,
                    reinterpret_cast<cudaStream_t>(stream_));
+}
+
+/* see lia_b200.h */
+extern "C" int lia_linear_bf16(const void* A, const void* W, void* out, int M, int N, int K, void* workspace, size_t workspace_bytes, lia_stream_t stream_) {
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  if (!gemm_rows_takes(M, N, K)) return gemm_impl(A, W, nullptr, nullptr, out, M, N, K, LIA_EPI_BIAS, nullptr, nullptr, workspace, workspace_bytes, stream);
+  EpiParams ep;
+  Plan pl;
+  const int rc = gemm_fill_params(A, W, nullptr, nullptr, out, M, N, K, LIA_EPI_BIAS, nullptr, nullptr, ep, pl);         // the GEMM's checks
+  return rc != LIA_OK ? rc : gemm_rows(A, W, out, M, N, K, stream);
 }
 
 // ------------------------------------------------------------------ tensor-parallel fused projection + all-reduce

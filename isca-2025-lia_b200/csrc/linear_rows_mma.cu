@@ -192,9 +192,8 @@ template <int OUT> int launch_rows(const RowsArgs& p, int batch, cudaStream_t st
 // Weights up to 24 MB in up to 4096 rows; the line looks at the weights alone, for the other side's sums are other ones.  In a chain of projections over 300 MB of weights, 1 | 16 | 64 | 128 rows:
 // 1024 x 1024 5.7 | 5.9 | 7.8 | 10.6 us on the other side and 1.8 | 2.2 | 3.0 | 4.1 here, 2048 x 5632 8.3 | 9.0 | 14.4 | 26 and 5.8 | 7.7 | 14.3 | 21.5; beyond: 6144 x 2048 8.7 | 9.0 | 11.9 | 17
 // and 6.4 | 10.2 | 17 | 25, 5632 x 1024 5.8 | 6.1 | 8.2 | 11.9 and 4.3 | 5.4 | 9.2 | 14.
-// Only projections without a bias: OPT's all have one, and the program that chains a decoded token's operations in one launch (decode_program_sm100.cu) makes them with the GEMM's sums, which
-// its operations one by one give too.
-bool gemm_rows_takes(int M, int N, int K) { return M <= 128 && N <= 4096 && (long long)N * K <= 12 << 20; }
+// (lia_gemm_bf16 is not among its callers: OPT's operations one by one give the bits of the program that chains them in one launch, decode_program_sm100.cu, with the GEMM's sums.)
+bool gemm_rows_takes(int M, int N, int K) { return M > 0 && N > 0 && K > 0 && M <= 128 && N <= 4096 && (long long)N * K <= 12 << 20; }
 
 int gemm_rows(const void* A, const void* W, void* C, int M, int N, int K, cudaStream_t stream) {
   const RowsArgs p{reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(W), C, K, 0, K, 0, N, 0, M, N, K, 1.f};

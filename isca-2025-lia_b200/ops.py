@@ -91,6 +91,21 @@ def gemm(a, w, bias, out=None, epilogue=EPI_BIAS, residual=None, qkv=None, works
     return out
 
 
+def linear(a, w, out=None, workspace=None):
+    """out = a @ w.T in bf16 -- a [M,K], w [N,K] -- for projections without a bias; up to 128 rows with small weights take csrc/linear_rows_mma.cu, the rest the GEMM."""
+    _req(a, "a"); _req(w, "w")
+    M, K = a.shape
+    N = w.shape[0]
+    if out is None:
+        out = torch.empty(M, N, dtype=BF16, device=a.device)
+    if w.shape[1] != K or tuple(_req(out, "out").shape) != (M, N):
+        raise _lib.LiaError(f"linear: a is [{M},{K}], w {tuple(w.shape)}, out {tuple(out.shape)}")
+    ws_ptr, ws_bytes = (workspace.buf.data_ptr(), workspace.buf.numel()) if workspace is not None else (None, 0)
+    check(_lib.load().lia_linear_bf16(_p(a), _p(w), _p(out), M, N, K, ws_ptr, ws_bytes, _stream()), "lia_linear_bf16")
+    count_launches()
+    return out
+
+
 def gemm_allreduce(a, w, bias, residual, out, tp_args, workspace=None):
     """Row-parallel projection fused with its all-reduce and residual add (world > 1):
     out = residual + sum_over_ranks(a_r @ w_r.T + bias_r)  (decoder.py:60-77 + 247/317).

@@ -76,7 +76,7 @@ class Linear:
         if out is None:
             out = torch.empty(M, self.N, dtype=self.dtype, device=x.device)
         if self.tensor_core and x.is_contiguous() and x.data_ptr() % 16 == 0:
-            ops.gemm(x, self.weight, None, out=out, workspace=self._workspace(M, x.device))
+            ops.linear(x, self.weight, out=out, workspace=self._workspace(M, x.device))
         else:
             ops.linear_plain(x, self.weight, out)
         return out

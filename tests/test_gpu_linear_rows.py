@@ -19,9 +19,9 @@ def _rand(*s, seed=0, std=1.0):
 def test_projections(M, N, K):
     """Sums rounded once to bf16; one that lies next to a rounding's middle may go the other way: one step of 2^-8 of sums up to 8."""
     a, w = _rand(M, K), _rand(N, K, std=K ** -0.5)
-    out, y = ops.gemm(a, w, None), (a.double() @ w.double().T).to(BF16).double()
+    out, y = ops.linear(a, w), (a.double() @ w.double().T).to(BF16).double()
     assert float((out.double() - y).abs().max()) <= 0.0325 and float((out.double() != y).double().mean()) < 2e-3
-    assert torch.equal(ops.gemm(a[:1], w, None), out[:1])
+    assert torch.equal(ops.linear(a[:1], w), out[:1])
 
 
 @pytest.mark.parametrize("M,N,K,batch", [(1, 5, 8, 3), (7, 16, 136, 2), (16, 33, 2088, 1), (40, 130, 512, 4), (64, 4800, 96, 1), (33, 2400, 128, 1)])
