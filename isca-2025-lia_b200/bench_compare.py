@@ -39,7 +39,7 @@ def _in_chunks(mlstm, q, dim, vdim, lengths):
 def _cost(name, a, kw):
     """(flops, bytes, kind) of one call; kind: 'tc' tensor cores (the products of the definition, however many the form takes: fp32 operands in
     three bf16 parts are three to six each), 'f32' CUDA-core fp32 arithmetic, 'mem' memory-bound."""
-    if name == "gemm":
+    if name in ("gemm", "linear"):
         x, w = a[0], a[1]
         M, K, N = x.shape[0], x.shape[1], w.shape[0]
         return 2.0 * M * N * K, 2.0 * (M * K + N * K + M * N), "tc"
@@ -158,7 +158,7 @@ def _cost(name, a, kw):
 
 
 class Instrument:
-    NAMES = ("gemm", "linear_plain", "linear_small", "mlstm_scan", "headnorm_gate", "latent_prep", "latent_attn", "latent_attn_expanded", "clamped_glu",
+    NAMES = ("gemm", "linear", "linear_plain", "linear_small", "mlstm_scan", "headnorm_gate", "latent_prep", "latent_attn", "latent_attn_expanded", "clamped_glu",
              "rms_add_norm", "embed_rmsnorm", "rms_gather", "layernorm", "attn_prefill", "attn_decode", "embed", "argmax", "argmax_f32",
              "linear_scan", "conv_prep", "conv_state_update", "kv_store", "window_attn", "ln_add_norm", "embed_rows", "ln_gather", "gated_act",
              "router_topk", "moe_plan", "moe_gemm", "moe_gemm_tc", "moe_gather", "moe_expert_gemms", "moe_combine", "qkv_prep", "gated_rms_add", "poly_norm",
