@@ -609,7 +609,8 @@ __global__ void __launch_bounds__(128, TG > 1 ? 1 : (NJ <= 2 ? 5 : (NJ <= 4 ? 3 
   constexpr int SSD_COLS = 4 * 4 * 32 / RG, NP = NJ * 4 * RG, ROWF = 2 * NP + SSD_COLS + 4;
   extern __shared__ __align__(16) float stage[];       // [2][SSD_TB][ROWF]
   const int seg = blockIdx.z, h = blockIdx.y, colb = blockIdx.x * SSD_COLS, g = h / (H / G);
-  const int slot = segs[4 * seg], row0 = segs[4 * seg + 2] + tok0, all = segs[4 * seg + 3], len = min(all - tok0, span);
+  // (`span` is for the portions of `below` tokens and more: a shorter one is done whole with the first tokens of those)
+  const int slot = segs[4 * seg], row0 = segs[4 * seg + 2] + tok0, all = segs[4 * seg + 3], len = all < below ? all : min(all - tok0, span);
   if (all >= below && (len <= 0 || !flags[(size_t)seg * H + h])) {                  // ssd_chunk_sm100.cu had these tokens (span: some of its portion's at a time): the state
     if (len <= 0) return;                                                            // after them is to go where it belongs
     const size_t first = (size_t)h * vdim * N + (size_t)colb * N, all_heads = (size_t)H * vdim * N;

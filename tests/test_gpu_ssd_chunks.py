@@ -80,6 +80,37 @@ def test_a_workspace_for_some_of_the_chunks_changes_no_bit(monkeypatch):
         assert all(torch.equal(a, b) for a, b in zip(whole, step.run()))
 
 
+@pytest.mark.parametrize("lens,H", [([700, 200, 129, 255, 1], 4), ([300] + [200] * 15, 128)])
+def test_short_portions_beside_some_of_the_chunks(lens, H, monkeypatch):
+    """Portions that go token by token are done whole, however few chunks of the others are taken at a time."""
+    step = Step(lens, H, 2, 64)
+    old = step.run(by_tokens=True)
+    for size in (ops.SSD_WORKSPACE, 1):
+        monkeypatch.setattr(ops, "SSD_WORKSPACE", size)
+        o, S = step.run()
+        for slot, _, row, n in step.segs:
+            if n < 256:
+                assert torch.equal(o[row:row + n], old[0][row:row + n]) and torch.equal(S[slot], old[1][slot]), n
+
+
+@pytest.mark.parametrize("at", [40, 140, 299, 600])
+def test_heads_go_token_by_token_for_some_of_the_chunks(at, monkeypatch):
+    """A value out of range leaves its head to the token loop for the chunks that are taken together, and these begin with the state that the ones before them left."""
+    H, G, vdim = 4, 2, 64
+    step = Step([700, 130], H, G, vdim)
+    step.xbc[at, 2 * vdim + 5] = 3e30                            # of head 2
+    whole, old = step.run(), step.run(by_tokens=True)
+    monkeypatch.setattr(ops, "SSD_WORKSPACE", 1)
+    o, S = step.run()
+    first = at // 128 * 128                                      # the tokens that are taken with it
+    assert torch.equal(o.view(-1, H, vdim)[:, [0, 1, 3]], whole[0].view(-1, H, vdim)[:, [0, 1, 3]]) and torch.equal(S[:, [0, 1, 3]], whole[1][:, [0, 1, 3]])
+    want = step.exact()
+    rows = lambda t: t.view(-1, H, vdim)[:first, 2]  # noqa: E731
+    if first:
+        assert _rel(rows(o), rows(want[0])) <= _rel(rows(old[0]), rows(want[0])) + 2.0 ** -25
+    assert _rel(o.view(-1, H, vdim)[first:, 2], want[0].view(-1, H, vdim)[first:, 2]) <= 2.0 ** -20 and _rel(S[:, 2], want[1][:, 2]) <= 2.0 ** -20
+
+
 def test_a_portion_does_not_depend_on_its_company():
     step = Step([300, 1, 256, 255, 700], 8, 2, 64)
     o, S = step.run()
