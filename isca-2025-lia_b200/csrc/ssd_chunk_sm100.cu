@@ -950,8 +950,7 @@ extern "C" int lia_ssd_scan_chunks(const float* B, const float* C, const float* 
   LIA_CUDA(cudaFuncSetAttribute(ssd_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_BYTES));
   LIA_CUDA(cudaFuncSetAttribute(ssd_outputs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OUT_BYTES));
   p.span = chunks * L;
-  const int longest = rows - nseg + 1;         // the most tokens that a portion can have
-  for (int tok0 = 0; tok0 < longest; tok0 += p.span) {
+  for (int tok0 = 0; tok0 < rows; tok0 += p.span) {                 // a portion has `rows` tokens at most (the others may be empty)
     p.tok0 = tok0;
     const dim3 grid((unsigned)slots, (unsigned)(G * p.split));
     lia_launch(ssd_states_kernel, grid, dim3(ST_THREADS), ST_BYTES, stream, p);

@@ -1291,7 +1291,7 @@ def ssd_scan(xbc, gates, D, state_S, segs, H, G, N, vdim, o):
     chunks, ws = _ssd_workspace(lib, M, nseg, H, G, N, vdim, (xbc, state_S, o), ld, inner)
     if ws is not None:
         check(lib.lia_ssd_scan_chunks(*args, _p(ws), ws.numel(), chunks, _stream()), "lia_ssd_scan_chunks")
-        count_launches(4 * -(-(M - nseg + 1) // (128 * chunks)))
+        count_launches(4 * -(-M // (128 * chunks)))
     else:
         check(lib.lia_ssd_scan(*args, _stream()), "lia_ssd_scan")
         count_launches()
@@ -1307,7 +1307,7 @@ def _ssd_workspace(lib, M, nseg, H, G, N, vdim, tensors, ld, inner):
     one = lib.lia_ssd_workspace(M, nseg, H, G, N, vdim, 1)
     if not one or ld % 4 or any(t.data_ptr() % 16 for t in tensors):
         return 0, None
-    chunks = max(1, min(-(-(M - nseg + 1) // 128), SSD_WORKSPACE // one))
+    chunks = max(1, min(-(-M // 128), SSD_WORKSPACE // one))
     while True:
         try:
             return chunks, torch.empty(lib.lia_ssd_workspace(M, nseg, H, G, N, vdim, chunks), dtype=torch.uint8, device=tensors[0].device)

@@ -93,6 +93,16 @@ def test_short_portions_beside_some_of_the_chunks(lens, H, monkeypatch):
                 assert torch.equal(o[row:row + n], old[0][row:row + n]) and torch.equal(S[slot], old[1][slot]), n
 
 
+def test_an_empty_portion_takes_no_token_from_the_others(monkeypatch):
+    step = Step([0, 385, 0], 4, 2, 64)
+    whole = Step([385], 4, 2, 64)
+    whole.xbc, whole.gates, whole.D, whole.S0, whole.segs = step.xbc, step.gates, step.D, step.S0, step.segs[1:2]
+    want = whole.run()
+    for size in (ops.SSD_WORKSPACE, 1):
+        monkeypatch.setattr(ops, "SSD_WORKSPACE", size)
+        assert all(torch.equal(a, b) for a, b in zip(step.run(), want))
+
+
 @pytest.mark.parametrize("at", [40, 140, 299, 600])
 def test_heads_go_token_by_token_for_some_of_the_chunks(at, monkeypatch):
     """A value out of range leaves its head to the token loop for the chunks that are taken together, and these begin with the state that the ones before them left."""
