@@ -87,7 +87,8 @@ int lia_layernorm_bf16(const void* x, const void* w, const void* b, void* y, int
  * projections of A:376-418.  A, W, bias, residual, out are bf16 row-major and contiguous
  * (K % 8 == 0, N % 8 == 0, all base pointers 16-byte aligned).
  * `workspace` is used when the kernel splits K (small M): lia_gemm_workspace_bytes() bytes,
- * zero-initialised ONCE by the caller (the kernel leaves it zeroed again). */
+ * zero-initialised ONCE by the caller (the kernel leaves it zeroed again).
+ * No work in flight on the stream may write W: up to 128 rows it is read before the previous kernel has ended. */
 size_t lia_gemm_workspace_bytes(int M, int N, int K);
 int lia_gemm_bf16(const void* A, const void* W, const void* bias, const void* residual, void* out, int M, int N,
                   int K, int epilogue, const LiaQkvArgs* qkv, void* workspace, size_t workspace_bytes,
@@ -276,9 +277,15 @@ int lia_clamped_glu(const void* gate_up, int ld, int up_off, void* out, int act_
  * cap*tanh(z/cap), last N/2 logsigmoid(cap*tanh(z/cap)) (log input / log forget gates); 2: sigmoid */
 int lia_linear_small(const void* a, int a_f32, int lda, const void* w, int w_f32, const float* bias, float* out, int M, int N, int K,
                      int mode, float cap, lia_stream_t stream);
+/* the same for a `w` that no work in flight on the stream writes (a model's weights): it may be read before the previous kernel has ended */
+int lia_linear_small_resident(const void* a, int a_f32, int lda, const void* w, int w_f32, const float* bias, float* out, int M, int N, int K,
+                              int mode, float cap, lia_stream_t stream);
 /* C[b][m][n] = scale * sum_k A[b][m][k] W[b][n][k] on the CUDA cores, fp32 products and sums; element strides */
 int lia_linear_plain(const void* A, int a_f32, long long lda, long long sA, const void* W, int w_f32, long long ldw, long long sW,
                      void* C, int c_f32, long long ldc, long long sC, int M, int N, int K, int batch, float scale, lia_stream_t stream);
+/* the same for a W that no work in flight on the stream writes (a model's weights): it may be read before the previous kernel has ended */
+int lia_linear_plain_resident(const void* A, int a_f32, long long lda, long long sA, const void* W, int w_f32, long long ldw, long long sW,
+                              void* C, int c_f32, long long ldc, long long sC, int M, int N, int K, int batch, float scale, lia_stream_t stream);
 int lia_argmax_f32(const float* logits, int64_t* next, int B, int V, int suppress_id, lia_stream_t stream);
 /* matrix-memory recurrence over every portion of the step; q/k [rows][H*dim], v [rows][H*vdim] with row stride ld;
  * gates [rows][2H] = log input gates then log forget gates; state_S [slots][H][vdim][dim], state_n [slots][H][dim],
@@ -603,7 +610,7 @@ int lia_conv_act(const void* y, int y_f32, int ld, int col0, int C, const float*
                  float* state, const int* meta, const int* segs, int nseg, float* out, int ldo, int M, int dt_col, int H, const float* dt_bias,
                  const float* a_log, float* gates, lia_stream_t stream);
 /* out[M][N] = A[M][K] W[N][K]^T in bf16: lia_gemm_bf16 without a bias, and for up to 128 rows and small weights a kernel whose sums are taken in another order; a row's result does
- * not depend on how many rows up to 128 there are */
+ * not depend on how many rows up to 128 there are.  W as there: no work in flight on the stream may write it. */
 int lia_linear_bf16(const void* A, const void* W, void* out, int M, int N, int K, void* workspace, size_t workspace_bytes, lia_stream_t stream);
 /* State-space dual recurrence over every portion, per head h (B and C of group h / (H / G), N <= 512 numbers; x of vdim numbers; all with
  * row stride ld):  S = g S + dt B x^T,  o = S^T C + D[h] x;  gates [rows][2H] = dt | g; state_S [slot][H][vdim][N], o [rows][H * vdim] fp32;

@@ -91,8 +91,12 @@ _PROTOTYPES = {
     "lia_clamped_glu": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_float, c_float, c_void_p]),
     "lia_linear_small": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float,
                                  c_void_p]),
+    "lia_linear_small_resident": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float,
+                                          c_void_p]),
     "lia_linear_plain": (c_int, [c_void_p, c_int, c_longlong, c_longlong, c_void_p, c_int, c_longlong, c_longlong, c_void_p, c_int,
                                  c_longlong, c_longlong, c_int, c_int, c_int, c_int, c_float, c_void_p]),
+    "lia_linear_plain_resident": (c_int, [c_void_p, c_int, c_longlong, c_longlong, c_void_p, c_int, c_longlong, c_longlong, c_void_p, c_int,
+                                          c_longlong, c_longlong, c_int, c_int, c_int, c_int, c_float, c_void_p]),
     "lia_argmax_f32": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "lia_mlstm_scan": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p]),

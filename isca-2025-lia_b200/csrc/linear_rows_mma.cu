@@ -2,8 +2,9 @@
 // logits, gates and routers.
 //
 // A step of decoded tokens is a chain of small projections, and what the tcgen05 GEMM takes for one is latency: tensor maps, barriers, TMEM, a ring that fills, partial sums that change
-// hands.  Here the weights go straight from global memory into the operands' registers, before the previous kernel has ended (they do not depend on it): 16 bytes of a weight row are two
-// operands' worth of k, and as the rows of A are read the same way the order of the k within 32 does not matter.  A block makes 16 or 32 columns of 8 to 32 rows, its 8 warps an eighth of K
+// hands.  Here the weights go straight from global memory into the operands' registers: 16 bytes of a weight row are two operands' worth of k, and as the rows of A are read the same
+// way the order of the k within 32 does not matter.  Where the caller says that no work in flight on the stream writes them (`resident`: a model's weights) they are asked for before the
+// previous kernel has ended.  A block makes 16 or 32 columns of 8 to 32 rows, its 8 warps an eighth of K
 // each; they meet once, in shared memory.
 //
 // The tensor cores cut sums off below the 24th bit: those over 32 k are made apart and added in fp32.  Where the result is fp32 those over 16 are, what a warp's sum rounds off is added up apart
@@ -31,13 +32,14 @@ struct RowsArgs {
   const float* bias;                           // gates
   int mode;
   float cap;
+  int resident;
 };
 
 enum { OUT_GEMM, OUT_FP32, OUT_ROUNDED, OUT_GATES };              // GEMM: bf16, whole vectors, nothing kept of what the sums round off
 
-__device__ __forceinline__ uint4 ldg_once(const bf16* p) {
+__device__ __forceinline__ uint4 ldg_once(const bf16* p) {                        // by way of L2 alone: a weight may be what the previous kernel wrote
   uint4 r;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+  asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
   return r;
 }
 
@@ -66,6 +68,7 @@ __global__ void __launch_bounds__(WARPS * 32, Form<NT, MT, CB>::REGS + (OUT == O
       for (int i = 0; i < 2 * MT; ++i) w[b][i >> 1][i & 1] = live ? ldg_once(W + (size_t)min(n0 + g + 8 * i, p.N - 1) * p.ldw + k) : make_uint4(0, 0, 0, 0);
     }
   };
+  if (!p.resident) pdl_wait();
   weights(first);
   pdl_wait();
   float acc[NT][MT][4] = {}, left[OUT == OUT_GEMM ? 1 : NT][MT][4] = {};
@@ -196,7 +199,7 @@ template <int OUT> int launch_rows(const RowsArgs& p, int batch, cudaStream_t st
 bool gemm_rows_takes(int M, int N, int K) { return M > 0 && N > 0 && K > 0 && M <= 128 && N <= 4096 && (long long)N * K <= 12 << 20; }
 
 int gemm_rows(const void* A, const void* W, void* C, int M, int N, int K, cudaStream_t stream) {
-  const RowsArgs p{reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(W), C, K, 0, K, 0, N, 0, M, N, K, 1.f};
+  const RowsArgs p{reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(W), C, K, 0, K, 0, N, 0, M, N, K, 1.f, nullptr, 0, 0.f, 1};
   return launch_rows<OUT_GEMM>(p, 1, stream);
 }
 
@@ -206,12 +209,12 @@ bool linear_rows_takes(const void* A, long long lda, long long sA, const void* W
 }
 
 int linear_rows(const void* A, long long lda, long long sA, const void* W, long long ldw, long long sW, void* C, int c_f32, long long ldc, long long sC, int M, int N, int K,
-                int batch, float scale, cudaStream_t stream) {
-  const RowsArgs p{reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(W), C, lda, sA, ldw, sW, ldc, sC, M, N, K, scale};
+                int batch, float scale, int resident, cudaStream_t stream) {
+  const RowsArgs p{reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(W), C, lda, sA, ldw, sW, ldc, sC, M, N, K, scale, nullptr, 0, 0.f, resident};
   return c_f32 ? launch_rows<OUT_FP32>(p, batch, stream) : launch_rows<OUT_ROUNDED>(p, batch, stream);
 }
 
-int linear_rows_gates(const void* A, long long lda, const void* W, const float* bias, float* out, int M, int N, int K, int mode, float cap, cudaStream_t stream) {
-  const RowsArgs p{reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(W), out, lda, 0, K, 0, N, 0, M, N, K, 1.f, bias, mode, cap};
+int linear_rows_gates(const void* A, long long lda, const void* W, const float* bias, float* out, int M, int N, int K, int mode, float cap, int resident, cudaStream_t stream) {
+  const RowsArgs p{reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(W), out, lda, 0, K, 0, N, 0, M, N, K, 1.f, bias, mode, cap, resident};
   return launch_rows<OUT_GATES>(p, 1, stream);
 }

@@ -821,9 +821,9 @@ __global__ void __launch_bounds__(256) argmax_f32_kernel(const float* __restrict
 
 template <typename TA, typename TW>
 int launch_plain(const void* A, long long lda, long long sA, const void* W, long long ldw, long long sW, void* C, long long ldc, long long sC,
-                 int M, int N, int K, int batch, float scale, int c_f32, cudaStream_t stream) {
+                 int M, int N, int K, int batch, float scale, int c_f32, int resident, cudaStream_t stream) {
   if (std::is_same<TA, bf16>::value && std::is_same<TW, bf16>::value && M <= 64 && linear_rows_takes(A, lda, sA, W, ldw, sW, M, K))
-    return linear_rows(A, lda, sA, W, ldw, sW, C, c_f32, ldc, sC, M, N, K, batch, scale, stream);
+    return linear_rows(A, lda, sA, W, ldw, sW, C, c_f32, ldc, sC, M, N, K, batch, scale, resident, stream);
   if (M <= 64) {
     dim3 g2((N + 3) / 4, batch);
     if (c_f32)
@@ -945,12 +945,12 @@ extern "C" int lia_clamped_glu(const void* gate_up, int ld, int up_off, void* ou
   return LIA_OK;
 }
 
-extern "C" int lia_linear_small(const void* a, int a_f32, int lda, const void* w, int w_f32, const float* bias, float* out, int M, int N,
-                                int K, int mode, float cap, lia_stream_t stream_) {
+static int linear_small(const void* a, int a_f32, int lda, const void* w, int w_f32, const float* bias, float* out, int M, int N, int K, int mode, float cap, int resident,
+                        lia_stream_t stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LIA_CHECK_ARG(a && w && out && M > 0 && N > 0 && K > 0 && lda >= K, "lia_linear_small: bad arguments");
   LIA_CHECK_ARG(mode >= 0 && mode <= 2 && (mode != 1 || (N % 2 == 0 && cap > 0.f)), "lia_linear_small: bad mode %d (N=%d cap=%f)", mode, N, cap);
-  if (!a_f32 && !w_f32 && linear_rows_takes(a, lda, 0, w, K, 0, M, K)) return linear_rows_gates(a, lda, w, bias, out, M, N, K, mode, cap, stream);
+  if (!a_f32 && !w_f32 && linear_rows_takes(a, lda, 0, w, K, 0, M, K)) return linear_rows_gates(a, lda, w, bias, out, M, N, K, mode, cap, resident, stream);
   const bool four = M >= 8 * lia_sm_count();
   const dim3 grid(four ? (M + 3) / 4 : M, (N + 7) / 8 < 65535 ? (N + 7) / 8 : 65535);
 #define LIA_LS(TA, TW)                                                                                                                                      \
@@ -965,17 +965,33 @@ extern "C" int lia_linear_small(const void* a, int a_f32, int lda, const void* w
   return LIA_OK;
 }
 
-extern "C" int lia_linear_plain(const void* A, int a_f32, long long lda, long long sA, const void* W, int w_f32, long long ldw, long long sW,
-                                void* C, int c_f32, long long ldc, long long sC, int M, int N, int K, int batch, float scale,
-                                lia_stream_t stream_) {
+extern "C" int lia_linear_small(const void* a, int a_f32, int lda, const void* w, int w_f32, const float* bias, float* out, int M, int N, int K, int mode, float cap,
+                                lia_stream_t stream) {
+  return linear_small(a, a_f32, lda, w, w_f32, bias, out, M, N, K, mode, cap, 0, stream);
+}
+extern "C" int lia_linear_small_resident(const void* a, int a_f32, int lda, const void* w, int w_f32, const float* bias, float* out, int M, int N, int K, int mode, float cap,
+                                         lia_stream_t stream) {
+  return linear_small(a, a_f32, lda, w, w_f32, bias, out, M, N, K, mode, cap, 1, stream);
+}
+
+static int linear_plain(const void* A, int a_f32, long long lda, long long sA, const void* W, int w_f32, long long ldw, long long sW, void* C, int c_f32, long long ldc,
+                        long long sC, int M, int N, int K, int batch, float scale, int resident, lia_stream_t stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LIA_CHECK_ARG(A && W && C && M > 0 && N > 0 && K > 0 && batch > 0 && batch <= 65535, "lia_linear_plain: bad arguments");
   LIA_CHECK_ARG(lda >= K && ldw >= K && ldc >= N, "lia_linear_plain: leading dimensions smaller than the rows");
   LIA_CHECK_ARG((M + 63) / 64 <= 65535, "lia_linear_plain: too many rows (%d)", M);
-  if (a_f32 && w_f32) return launch_plain<float, float>(A, lda, sA, W, ldw, sW, C, ldc, sC, M, N, K, batch, scale, c_f32, stream);
-  if (a_f32) return launch_plain<float, bf16>(A, lda, sA, W, ldw, sW, C, ldc, sC, M, N, K, batch, scale, c_f32, stream);
-  if (w_f32) return launch_plain<bf16, float>(A, lda, sA, W, ldw, sW, C, ldc, sC, M, N, K, batch, scale, c_f32, stream);
-  return launch_plain<bf16, bf16>(A, lda, sA, W, ldw, sW, C, ldc, sC, M, N, K, batch, scale, c_f32, stream);
+  if (a_f32 && w_f32) return launch_plain<float, float>(A, lda, sA, W, ldw, sW, C, ldc, sC, M, N, K, batch, scale, c_f32, resident, stream);
+  if (a_f32) return launch_plain<float, bf16>(A, lda, sA, W, ldw, sW, C, ldc, sC, M, N, K, batch, scale, c_f32, resident, stream);
+  if (w_f32) return launch_plain<bf16, float>(A, lda, sA, W, ldw, sW, C, ldc, sC, M, N, K, batch, scale, c_f32, resident, stream);
+  return launch_plain<bf16, bf16>(A, lda, sA, W, ldw, sW, C, ldc, sC, M, N, K, batch, scale, c_f32, resident, stream);
+}
+extern "C" int lia_linear_plain(const void* A, int a_f32, long long lda, long long sA, const void* W, int w_f32, long long ldw, long long sW, void* C, int c_f32, long long ldc,
+                                long long sC, int M, int N, int K, int batch, float scale, lia_stream_t stream) {
+  return linear_plain(A, a_f32, lda, sA, W, w_f32, ldw, sW, C, c_f32, ldc, sC, M, N, K, batch, scale, 0, stream);
+}
+extern "C" int lia_linear_plain_resident(const void* A, int a_f32, long long lda, long long sA, const void* W, int w_f32, long long ldw, long long sW, void* C, int c_f32, long long ldc,
+                                         long long sC, int M, int N, int K, int batch, float scale, lia_stream_t stream) {
+  return linear_plain(A, a_f32, lda, sA, W, w_f32, ldw, sW, C, c_f32, ldc, sC, M, N, K, batch, scale, 1, stream);
 }
 
 extern "C" int lia_argmax_f32(const float* logits, int64_t* next, int B, int V, int suppress_id, lia_stream_t stream_) {

@@ -270,7 +270,7 @@ class BebulornForCausalLM:
         hn = torch.empty(n, W, dtype=dt, device=dev)
         ops.ln_gather(x, want, self.final_norm, hn, eps)
         logits = torch.empty(n, cfg.vocab, dtype=F32, device=dev)
-        ops.linear_plain(hn, self.head.weight, logits)
+        ops.linear_plain(hn, self.head.weight, logits, resident=True)
         return logits
 
     def graph_class(self, max_ctx):

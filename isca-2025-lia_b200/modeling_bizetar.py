@@ -288,7 +288,7 @@ class BizetarForCausalLM:
         hn = torch.empty(n, W, dtype=dt, device=dev)
         ops.rms_gather(x, want, self.final_norm, hn, eps)
         logits = torch.empty(n, cfg.vocab, dtype=F32, device=dev)
-        ops.linear_plain(hn, self.head.weight, logits)
+        ops.linear_plain(hn, self.head.weight, logits, resident=True)
         return logits
 
     def _one(self, dev):

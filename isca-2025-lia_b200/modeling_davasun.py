@@ -216,7 +216,7 @@ class DavasunForCausalLM:
         hn = torch.empty(n, W, dtype=dt, device=dev)
         ops.rms_gather(x, want, self.final_norm, hn, eps)
         logits = torch.empty(n, cfg.vocab, dtype=F32, device=dev)
-        ops.linear_plain(hn, self.head.weight, logits, scale=cfg.logit_scale)
+        ops.linear_plain(hn, self.head.weight, logits, scale=cfg.logit_scale, resident=True)
         return logits
 
     def graph_class(self, max_ctx):

@@ -233,7 +233,7 @@ class PazivikForCausalLM:
         hn = torch.empty(n, W, dtype=dt, device=dev)
         ops.rms_gather(x, want, self.final_norm, hn, eps)
         logits = torch.empty(n, cfg.vocab, dtype=F32, device=dev)
-        ops.linear_plain(hn, self.embed, logits)
+        ops.linear_plain(hn, self.embed, logits, resident=True)
         if cfg.logit_softcap > 0:
             ops.softcap(logits, cfg.logit_softcap)
         return logits

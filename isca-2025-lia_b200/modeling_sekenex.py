@@ -278,7 +278,7 @@ class SekenexForCausalLM:
         hn = torch.empty(n, W, dtype=dt, device=dev)
         ops.streams_gather(x, want, self.final_norm, hn, eps)
         logits = torch.empty(n, cfg.vocab, dtype=F32, device=dev)
-        ops.linear_plain(hn, self.head.weight, logits)
+        ops.linear_plain(hn, self.head.weight, logits, resident=True)
         return logits
 
     def _update(self, x, y, mixer, hc, nxt, h):

@@ -63,7 +63,8 @@ class GemmWorkspace:
 
 
 def gemm(a, w, bias, out=None, epilogue=EPI_BIAS, residual=None, qkv=None, workspace=None):
-    """out = epilogue(a @ w.T) -- a [M,K], w [N,K] (decoder.py:79-105, attentions.py:376-418)."""
+    """out = epilogue(a @ w.T) -- a [M,K], w [N,K] (decoder.py:79-105, attentions.py:376-418).  No work in flight on the stream may write ``w``: up to 128 rows
+    it is read before the previous kernel has ended."""
     _req(a, "a"); _req(w, "w")
     M, K = a.shape
     N = w.shape[0]
@@ -92,7 +93,8 @@ def gemm(a, w, bias, out=None, epilogue=EPI_BIAS, residual=None, qkv=None, works
 
 
 def linear(a, w, out=None, workspace=None):
-    """out = a @ w.T in bf16 -- a [M,K], w [N,K] -- for projections without a bias; up to 128 rows with small weights take csrc/linear_rows_mma.cu, the rest the GEMM."""
+    """out = a @ w.T in bf16 -- a [M,K], w [N,K] -- for projections without a bias; up to 128 rows with small weights take csrc/linear_rows_mma.cu, the rest the GEMM.
+    No work in flight on the stream may write ``w``, as for ``gemm``: it is read before the previous kernel has ended."""
     _req(a, "a"); _req(w, "w")
     M, K = a.shape
     N = w.shape[0]
@@ -365,8 +367,9 @@ def clamped_glu(gate_up, up_off, F, out, limit, alpha):
 GATE_NONE, GATE_LOG_INPUT_FORGET, GATE_SIGMOID = 0, 1, 2
 
 
-def linear_small(a, w, bias, out, mode=GATE_NONE, cap=1.0):
-    """out = act(a @ w.T + bias) for a handful of outputs (per-head gates), fp32 out."""
+def linear_small(a, w, bias, out, mode=GATE_NONE, cap=1.0, resident=False):
+    """out = act(a @ w.T + bias) for a handful of outputs (per-head gates), fp32 out.  ``resident``: no work in flight on the stream writes ``w`` (a
+    model's weights), so that it may be read before the previous kernel has ended."""
     lda = _rowmajor(a, "a")
     _dev(w, "w"); _req(out, "out", F32)
     M, K = a.shape
@@ -375,16 +378,17 @@ def linear_small(a, w, bias, out, mode=GATE_NONE, cap=1.0):
         raise _lib.LiaError(f"linear_small: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
     if bias is not None:
         _req(bias, "bias", F32)
-    check(_lib.load().lia_linear_small(_p(a), _f32(a), lda, _p(w), _f32(w), _p(bias), _p(out), M, N, K, mode, float(cap), _stream()),
+    lib = _lib.load()
+    check((lib.lia_linear_small_resident if resident else lib.lia_linear_small)(_p(a), _f32(a), lda, _p(w), _f32(w), _p(bias), _p(out), M, N, K, mode, float(cap), _stream()),
           "lia_linear_small")
     count_launches()
     return out
 
 
-def linear_plain(a, w, out, scale=1.0, batch=1, a_batch_stride=0, w_batch_stride=0, out_batch_stride=0, n=None, k=None):
+def linear_plain(a, w, out, scale=1.0, batch=1, a_batch_stride=0, w_batch_stride=0, out_batch_stride=0, n=None, k=None, resident=False):
     """out[b] = scale * a[b] @ w[b].T on the CUDA cores with fp32 products and sums.  ``a`` / ``out`` are row-major 2-D
     views (row stride free); batches are taken at element strides from their first element; ``n``, ``k`` give the
-    per-batch problem when the views are wider than one batch."""
+    per-batch problem when the views are wider than one batch.  ``resident``: as for ``linear_small``."""
     lda, ldc = _rowmajor(a, "a"), _rowmajor(out, "out")
     _dev(w, "w")
     M = a.shape[0]
@@ -393,8 +397,9 @@ def linear_plain(a, w, out, scale=1.0, batch=1, a_batch_stride=0, w_batch_stride
     ldw = w.stride(-2) if w.dim() >= 2 and w.shape[-2] > 1 else max(K, w.shape[-1])     # (a single row's stride may be anything)
     if out.shape[0] != M:
         raise _lib.LiaError("linear_plain: a and out differ in rows")
-    check(_lib.load().lia_linear_plain(_p(a), _f32(a), lda, a_batch_stride, _p(w), _f32(w), ldw, w_batch_stride, _p(out), _f32(out), ldc,
-                                       out_batch_stride, M, N, K, batch, float(scale), _stream()), "lia_linear_plain")
+    lib = _lib.load()
+    check((lib.lia_linear_plain_resident if resident else lib.lia_linear_plain)(_p(a), _f32(a), lda, a_batch_stride, _p(w), _f32(w), ldw, w_batch_stride, _p(out), _f32(out),
+                                                                                ldc, out_batch_stride, M, N, K, batch, float(scale), _stream()), "lia_linear_plain")
     count_launches()
     return out
 

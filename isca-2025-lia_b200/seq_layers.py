@@ -78,7 +78,7 @@ class Linear:
         if self.tensor_core and x.is_contiguous() and x.data_ptr() % 16 == 0:
             ops.linear(x, self.weight, out=out, workspace=self._workspace(M, x.device))
         else:
-            ops.linear_plain(x, self.weight, out)
+            ops.linear_plain(x, self.weight, out, resident=True)
         return out
 
     def part(self, y, i):
@@ -110,7 +110,7 @@ class MLSTMMixer:
         y = self.proj(h)
         q, k, v, g = (self.proj.part(y, i) for i in range(4))
         gates = torch.empty(M, 2 * H, dtype=F32, device=h.device)
-        ops.linear_small(h, self.w_gates, self.b_gates, gates, ops.GATE_LOG_INPUT_FORGET, self.cap)
+        ops.linear_small(h, self.w_gates, self.b_gates, gates, ops.GATE_LOG_INPUT_FORGET, self.cap, resident=True)
         o = torch.empty(M, H * self.vdim, dtype=F32, device=h.device)
         ops.mlstm_scan(q, k, v, gates, S, n, m, batch.segs, H, self.dim, self.vdim, self.q_scale, self.den_eps, o, lengths=batch.lengths)
         on = torch.empty(M, H * self.vdim, dtype=self.dtype, device=h.device)
@@ -215,7 +215,7 @@ class LatentAttentionMixer:
         gate = None
         if self.gate == "head":
             gate = torch.empty(M, H, dtype=F32, device=h.device)
-            ops.linear_small(h, self.w_gate, None, gate, ops.GATE_SIGMOID)
+            ops.linear_small(h, self.w_gate, None, gate, ops.GATE_SIGMOID, resident=True)
         channel = self.gate == "channel"
         o = torch.empty(M, H * self.vdim, dtype=F32 if channel else self.dtype, device=h.device)
         qa = None
@@ -275,11 +275,11 @@ class LatentAttentionMixer:
         qa = torch.empty(n, H * D, dtype=F32, device=o.device) if qa is None else qa[r0:r1]
         # q~[m, h, :rank] = Wuk_h^T q[m, h, :dim]
         ops.linear_plain(q, self.w_uk_t, qa, batch=H, a_batch_stride=self.dim + self.rot, w_batch_stride=self.rank * self.dim,
-                         out_batch_stride=D, n=self.rank, k=self.dim)
+                         out_batch_stride=D, n=self.rank, k=self.dim, resident=True)
         lat = torch.empty(n, H * self.rank, dtype=F32, device=o.device)
         ops.latent_attn(qa, cache, meta, gate, lat, H, self.rank, self.rot, self.scale, batch.max_ctx, window=self.window, sink=self.sink)
         ops.linear_plain(lat, self.w_uv, o, batch=H, a_batch_stride=self.rank, w_batch_stride=self.vdim * self.rank,
-                         out_batch_stride=self.vdim, n=self.vdim, k=self.rank)
+                         out_batch_stride=self.vdim, n=self.vdim, k=self.rank, resident=True)
 
     def _expand(self, q, latents, meta, ctx, o):
         """One portion's output rows ``o``: per-head keys and values of the ``latents`` [ctx, rank] it sees (as they are cached), then
@@ -378,7 +378,7 @@ class DeltaRuleMixer:
         M, H, G = h.shape[0], self.H, self.G
         y = self.proj(h)
         gates = torch.empty(M, 2 * H, dtype=F32, device=h.device)
-        ops.linear_small(h, self.w_gates, None, gates, ops.GATE_NONE)
+        ops.linear_small(h, self.w_gates, None, gates, ops.GATE_NONE, resident=True)
         qk = torch.empty(M, 2 * G * self.dim, dtype=F32, device=h.device)
         v = torch.empty(M, H * self.vdim, dtype=F32, device=h.device)
         offs = self.proj.offsets[:3]
@@ -616,7 +616,7 @@ class SinkAttentionMixer:
         gate = None
         if self.gate == "head":
             gate = torch.empty(M, H, dtype=F32, device=h.device)
-            ops.linear_small(h, self.w_gate, None, gate, ops.GATE_SIGMOID)
+            ops.linear_small(h, self.w_gate, None, gate, ops.GATE_SIGMOID, resident=True)
         elif self.gate == "channel":
             gate = self.proj.part(y, 3)
         v_first = None
@@ -679,7 +679,7 @@ class GatedRecurrentMixer:
         u = torch.empty(M, W, dtype=F32, device=h.device)
         ops.conv_act(x, 0, self.w_conv, u, batch, state=conv, in_bias=self.x_bias, bias=self.conv_bias)
         z = torch.empty(M, 2 * W, dtype=F32, device=h.device)
-        ops.linear_plain(u, self.w_gates, z, batch=self.blocks, a_batch_stride=n, w_batch_stride=2 * n * n, out_batch_stride=2 * n, n=2 * n, k=n)
+        ops.linear_plain(u, self.w_gates, z, batch=self.blocks, a_batch_stride=n, w_batch_stride=2 * n * n, out_batch_stride=2 * n, n=2 * n, k=n, resident=True)
         o = torch.empty(M, W, dtype=self.dtype, device=h.device)
         ops.rglru_scan(u, z, self.gate_bias, self.c, y, self.y_bias, S, batch.segs, self.blocks, o)
         return self.out(o)
@@ -878,7 +878,7 @@ class MoEFeedForward:
         M, W, dev = h.shape[0], h.shape[1], h.device
         R, top = self.R, self.top
         logits = torch.empty(M, R + self.shared_gated, dtype=F32, device=dev)
-        ops.linear_small(h if router_input is None else router_input, self.router, None, logits, ops.GATE_NONE)
+        ops.linear_small(h if router_input is None else router_input, self.router, None, logits, ops.GATE_NONE, resident=True)
         idx = torch.empty(M, top, dtype=torch.int32, device=dev)
         wt = torch.empty(M, top, dtype=F32, device=dev)
         ops.router_topk(logits[:, :R], top, idx, wt, correction=self.correction, renorm=self.renorm, sigmoid=self.sigmoid, groups=self.groups,

@@ -67,3 +67,38 @@ def test_a_bad_number_stays_in_its_row(bad):
     ops.linear_plain(a, w, out)
     rest = [r for r in range(20) if r != 5]
     assert torch.equal(out[rest], clean[rest]) and torch.equal(out[5].isnan(), (a[5:6].float() @ w.float().T)[0].isnan())
+
+
+@pytest.mark.parametrize("between", [0, 1, 2])
+def test_a_second_operand_that_the_launches_before_wrote(between):
+    """Plain projections and gates read both operands after the work before them has ended, unless told that ``w`` is resident."""
+    K, x, a = 1024, _rand(64, 2048), _rand(7, 1024, seed=1)
+    makers = [_rand(K, 2048, seed=2 + i, std=2048 ** -0.5) for i in range(2)]
+    w, other = torch.zeros(64, K, device="cuda", dtype=BF16), torch.zeros(64, K, device="cuda", dtype=BF16)
+    want = []
+    for maker in makers:
+        ops.linear_plain(x, maker, w)
+        torch.cuda.synchronize()
+        out = [torch.empty(7, 64, device="cuda") for _ in range(2)]
+        ops.linear_plain(a, w, out[0]), ops.linear_small(a, w, None, out[1])
+        want.append(out)
+    assert not torch.equal(want[0][0], want[1][0])
+    got = [[torch.empty(7, 64, device="cuda") for _ in range(2)] for _ in range(60)]
+    torch.cuda.synchronize()
+    for i, out in enumerate(got):
+        for f, o in zip((lambda o: ops.linear_plain(a, w, o), lambda o: ops.linear_small(a, w, None, o)), out):
+            ops.linear_plain(x, makers[1 - i % 2], w)            # the other number first, so that an old one shows
+            ops.linear_plain(x, makers[i % 2], w)
+            for _ in range(between):
+                ops.linear_plain(x[:8], makers[0], other[:8])
+            f(o)
+    torch.cuda.synchronize()
+    assert all(torch.equal(g, t) for i, out in enumerate(got) for g, t in zip(out, want[i % 2]))
+
+
+def test_a_resident_second_operand_gives_the_same_bits():
+    a, w, bias = _rand(20, 264), _rand(40, 264, std=0.06), _rand(40).float()
+    out = [torch.empty(20, 40, device="cuda") for _ in range(4)]
+    for i in range(2):
+        ops.linear_plain(a, w, out[i], resident=bool(i)), ops.linear_small(a, w, bias, out[2 + i], ops.GATE_SIGMOID, resident=bool(i))
+    assert torch.equal(out[0], out[1]) and torch.equal(out[2], out[3])
