@@ -7,22 +7,25 @@
 //   states   every chunk's B^T (w x), 128 x 64 per head                              -> workspace
 //   carry    the states before every chunk, element by element, and the last one     -> workspace, in place
 //   outputs  C B^T once per group of heads, then per head the two products with C and with the weights
-// A CTA takes a chunk and some heads of one group, whose B and C it splits once.  All operands are fp32 numbers and enter as three bf16 parts each, all products but lo lo, whose accumulators
-// gather them by size (hi hi | hi mid, mid hi | the rest); the parts of one operand lie side by side, so that an instruction takes several.  One kind of product after
-// the other.
-// The tensor cores cut their sums off below the 24th bit, eight instructions in a row off by 1.8e-7.  So the hi parts are whole multiples, of at most 256, of one power of two per row of A and
-// column of B: 128 products of two such numbers have a sum below 2^23 of their unit, which the accumulator holds exactly.  What is cut off the other products is 2^-8 of that.
+// A CTA takes a chunk and some heads of one group, whose B and C it splits once.  All operands are fp32 numbers and enter as three fp16 parts each, all products but lo lo, whose accumulators
+// gather them by size (hi hi | hi mid, mid hi, mid mid | the rest); the parts of one operand lie side by side, so that an instruction can take several.
+// The tensor cores cut their sums off below the 24th bit, eight instructions in a row off by 1.8e-7.  So each row of A and column of B is brought, by a power of two, to numbers below 2^15, and
+// its hi parts are whole multiples, of at most 256, of 2^7: 128 products of two such numbers have a sum below 2^23 of their unit, which the accumulator holds exactly.  The rest of a number
+// goes on in two parts of 11 bits and a sign, the second times 2^11 against fp16's smallest numbers: nothing of fp32 is lost down to 2^-26 of the row's or column's largest number
+// (and 2^-51 of that at most below), so that a token is as exact beside a large one as alone.  (Two bf16 parts for the rest kept 16 to 18 bits of a number below 2^-8 of the largest: 1e3 times the others in the last token of a
+// chunk put the tokens before it off by 1.2e-6.)  There the sums of the second accumulator are the result, and smaller products go into it first: what is cut off each of them is then
+// off a smaller sum.
 // The weights P o C B^T go from registers to TMEM and are the A operand from there.
 //
-// 2048 tokens, 64 heads of 64 in 8 groups: 267 us token by token -> 49 states + 10 carry + 73 outputs (a unit of a chunk takes 5 and 8 us: its 80 instructions of tcgen05 3.5, the rest are
-// hand-overs between the roles; 10 to 15 us go before the first unit); Mamba's mixer 405 -> 280.  Against 64 bits, same inputs: outputs off by 6.2e-8 (token loop 6.6e-8), states by 4.9e-8
-// (6.7e-8); decays near 1: 5.1e-8 (10.5e-8) and 4.6e-8 (39e-8).
+// 2048 tokens, 64 heads of 64 in 8 groups: 270 us token by token -> 150 (with bf16 parts 141); Mamba's mixer 405 -> 275.  Against 64 bits, same inputs: outputs off by 5.9e-8 (token loop
+// 6.6e-8), states by 0.95e-8 (1.5e-8); decays near 1: 4.6e-8 (11.1e-8) and 4.5e-8 (39.8e-8).
 //
 // The weights are products of decays (never quotients or differences of logarithms).  Inputs that are not finite, or so large that a chunk's sums could overflow where the token loop's
 // would not, are left to the token loop, head by head (`flags`): there a bad value reaches the tokens after it and no other.
 //
 // Every wait is bounded: a CTA of `states` that gave up hands its heads to the token loop, one of `outputs` leaves NaN and counts itself (lia_moe_timeouts_seen).
 #include <cuda.h>
+#include <cuda_fp16.h>
 
 #include <mutex>
 
@@ -110,9 +113,12 @@ __device__ __forceinline__ void st_shared16(uint32_t addr, uint32_t a, uint32_t 
 // The products of two operands in three parts each: part of A (bits 0-1), first part of B (2-3) and how many of its parts (4-5), which accumulator (6-7), whether it begins that (8).
 // (The instructions are issued by one lane from loops: unrolled they would not fit into the instruction cache beside the other warps' code.)
 constexpr int product_code(int a, int b, int parts, int to, int first) { return a | b << 2 | parts << 4 | to << 6 | first << 8; }
-__constant__ int PRODUCTS[5] = {product_code(0, 0, 3, 0, 1), product_code(1, 0, 2, 1, 0), product_code(1, 2, 1, 2, 0), product_code(2, 0, 1, 2, 0), product_code(2, 1, 1, 2, 0)};
-__constant__ int SINGLES[8] = {product_code(0, 0, 1, 0, 1), product_code(0, 1, 1, 1, 1), product_code(1, 0, 1, 1, 0), product_code(0, 2, 1, 2, 1),
-                               product_code(1, 1, 1, 2, 0), product_code(2, 0, 1, 2, 0), product_code(1, 2, 1, 2, 0), product_code(2, 1, 1, 2, 0)};
+__constant__ int PRODUCTS[7] = {product_code(2, 0, 1, 2, 1), product_code(2, 1, 1, 2, 0), product_code(1, 2, 1, 2, 0), product_code(1, 1, 1, 1, 1), product_code(1, 0, 1, 1, 0),
+                                product_code(0, 0, 1, 0, 1), product_code(0, 1, 2, 1, 0)};
+__constant__ int SINGLES[8] = {product_code(2, 0, 1, 2, 1), product_code(2, 1, 1, 2, 0), product_code(1, 2, 1, 2, 0), product_code(0, 2, 1, 2, 0),
+                               product_code(1, 1, 1, 1, 1), product_code(1, 0, 1, 1, 0), product_code(0, 1, 1, 1, 0), product_code(0, 0, 1, 0, 1)};
+constexpr float LOW = 1.f / 2048.f;            // what the third accumulator counts for
+__device__ __forceinline__ float gathered(uint32_t a, uint32_t b, uint32_t c) { return __uint_as_float(a) + fmaf(__uint_as_float(c), LOW, __uint_as_float(b)); }
 // K = 128.  Steps in 16-byte units: a part, 64 of the contracted numbers, 16 of them (A in TMEM: in columns, as is `a`); `width`: columns of one part of B, and of an accumulator.
 struct Operand {
   uint64_t at;
@@ -122,7 +128,8 @@ template <bool tmem_a> __device__ __forceinline__ void issue(const int* codes, i
 #pragma unroll 1
   for (int i = 0; i < count; ++i) {
     const int code = codes[i];
-    const uint32_t idesc = make_idesc(128, 0) | major | (uint32_t)(((code >> 4 & 3) * width) >> 3) << 17, to = d + (code >> 6 & 3) * width;
+    constexpr uint32_t bf16_operands = 1u << 7 | 1u << 10;           // fp16: neither bit
+    const uint32_t idesc = (make_idesc(128, 0) & ~bf16_operands) | major | (uint32_t)(((code >> 4 & 3) * width) >> 3) << 17, to = d + (code >> 6 & 3) * width;
     uint64_t a = A.at + (code & 3) * A.part, b = B.at + (code >> 2 & 3) * B.part;
     uint32_t accumulate = !(code >> 8 & 1);
 #pragma unroll 1
@@ -179,21 +186,27 @@ __device__ __forceinline__ void load8(const float* src, bool live, float* v) {
   }
   v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
 }
-// The number whose last bit is 2^-7 of the power of two below `most`: added and taken away again it rounds anything up to `most` to a multiple of that, 256 at most
-__device__ __forceinline__ float rounder(float most) { return __uint_as_float((__float_as_uint(most) & 0x7f800000u) + (16u << 23) | 0x400000u); }
-__device__ __forceinline__ void split3_unit(float x, float y, float rx, float ry, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  const float hx = __fsub_rn(__fadd_rn(x, rx), rx), hy = __fsub_rn(__fadd_rn(y, ry), ry), dx = x - hx, dy = y - hy;      // exact differences
-  hi = pack_bf16x2(hx, hy);
-  mid = pack_bf16x2(dx, dy);
-  float mx, my;
-  unpack_bf16x2(mid, mx, my);
-  lo = pack_bf16x2(dx - mx, dy - my);
+// The power of two that brings numbers up to `most` below 2^15 (those of a row of less than 2^-100 stay smaller), and its inverse
+__device__ __forceinline__ float scale_of(float most) { return __uint_as_float((268u << 23) - max(__float_as_uint(most) & 0x7f800000u, 27u << 23)); }
+__device__ __forceinline__ float inverse_of(float scale) { return __uint_as_float((254u << 23) - __float_as_uint(scale)); }
+__device__ __forceinline__ uint32_t pack_half2(float x, float y) {
+  const __half2 h = __floats2half2_rn(x, y);
+  return *reinterpret_cast<const uint32_t*>(&h);
 }
-// 8 neighbouring numbers as 16 bytes in each of three tiles `stride` bytes apart, with a rounder each (or one: each = 0)
-template <int each> __device__ __forceinline__ void put_parts(uint32_t addr, uint32_t stride, const float* v, const float* r) {
+__device__ __forceinline__ void split3(float x, float y, float sx, float sy, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  constexpr float R = 1610612736.f;            // its last bit is 2^7: added and taken away again it rounds to a multiple of that
+  x *= sx, y *= sy;
+  const float hx = __fsub_rn(__fadd_rn(x, R), R), hy = __fsub_rn(__fadd_rn(y, R), R), dx = x - hx, dy = y - hy;          // exact differences
+  hi = pack_half2(hx, hy);
+  mid = pack_half2(dx, dy);
+  const float2 m = __half22float2(*reinterpret_cast<const __half2*>(&mid));
+  lo = pack_half2((dx - m.x) * 2048.f, (dy - m.y) * 2048.f);
+}
+// 8 neighbouring numbers as 16 bytes in each of three tiles `stride` bytes apart, with a scale each (or one: each = 0)
+template <int each> __device__ __forceinline__ void put_parts(uint32_t addr, uint32_t stride, const float* v, const float* s) {
   uint32_t h[4], m[4], l[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) split3_unit(v[2 * i], v[2 * i + 1], r[each * 2 * i], r[each * (2 * i + 1)], h[i], m[i], l[i]);
+  for (int i = 0; i < 4; ++i) split3(v[2 * i], v[2 * i + 1], s[each * 2 * i], s[each * (2 * i + 1)], h[i], m[i], l[i]);
   st_shared16(addr, h[0], h[1], h[2], h[3]);
   st_shared16(addr + stride, m[0], m[1], m[2], m[3]);
   st_shared16(addr + 2 * stride, l[0], l[1], l[2], l[3]);
@@ -201,8 +214,8 @@ template <int each> __device__ __forceinline__ void put_parts(uint32_t addr, uin
 __device__ __forceinline__ float most8(const float* v) {
   return fmaxf(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))), fmaxf(fmaxf(fabsf(v[4]), fabsf(v[5])), fmaxf(fabsf(v[6]), fabsf(v[7]))));
 }
-// The largest of 8 neighbouring columns over `rows` rows of maxima, as rounders
-template <int rows, int cols> __device__ __forceinline__ void rounders_of(const float (&m)[rows][cols], int col, float* r) {
+// The scales of 8 neighbouring columns from `rows` rows of maxima
+template <int rows, int cols> __device__ __forceinline__ void scales_of(const float (&m)[rows][cols], int col, float* r) {
 #pragma unroll
   for (int e = 0; e < 8; e += 4) {
     float4 a = *reinterpret_cast<const float4*>(&m[0][col + e]);
@@ -211,7 +224,7 @@ template <int rows, int cols> __device__ __forceinline__ void rounders_of(const 
       const float4 b = *reinterpret_cast<const float4*>(&m[k][col + e]);
       a = make_float4(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z), fmaxf(a.w, b.w));
     }
-    r[e] = rounder(a.x), r[e + 1] = rounder(a.y), r[e + 2] = rounder(a.z), r[e + 3] = rounder(a.w);
+    r[e] = scale_of(a.x), r[e + 1] = scale_of(a.y), r[e + 2] = scale_of(a.z), r[e + 3] = scale_of(a.w);
   }
 }
 // A row of 128 numbers over 16 lanes, 8 each: the largest
@@ -265,11 +278,13 @@ __device__ __forceinline__ Decays decays_of(const SsdArgs& p, const Chunk& c, in
 // TMEM: 2 x 192 columns.
 constexpr int ST_THREADS = 416;
 struct StBars {
-  uint64_t x_full[2], x_empty[2], acc_full[2], acc_empty[2], drain;
+  uint64_t x_full[2], x_empty[2], scaled[2], acc_full[2], acc_empty[2], drain;             // scaled: the scales that a unit was split by are written
 };
 struct StSmem {
   alignas(16) float w[MAX_UNITS][L];
   alignas(16) float most_b[8][N], most_x[8][P];                    // by warp
+  alignas(16) float inv_x[MAX_UNITS][P];                           // the scales' inverses
+  float inv_b[N];
   float total[MAX_UNITS], total_rest[MAX_UNITS];
   int bad[MAX_UNITS], bad_all, dead;
   uint32_t tmem;
@@ -289,6 +304,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) ssd_states_kernel(const SsdArgs
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&sm.bars.x_full[i]), 8);
       mbar_init(smem_u32(&sm.bars.x_empty[i]), 1);
+      mbar_init(smem_u32(&sm.bars.scaled[i]), 1);
       mbar_init(smem_u32(&sm.bars.acc_full[i]), 1);
       mbar_init(smem_u32(&sm.bars.acc_empty[i]), 4);
     }
@@ -326,7 +342,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) ssd_states_kernel(const SsdArgs
     }
     if (!__all_sync(0xffffffffu, fine) && lane == 0) sm.bad[j] = 1;
   }
-  if (warp >= 4 && warp < 12) {                                    // B: a thread has 8 tokens of 8 rows of the state; a unit per row of the state
+  if (warp >= 4 && warp < 12) {                                    // B: a thread has 8 tokens of 8 rows of the state; a scale per row of the state
     const int th = tid - 128, piece = th & 15;
     float v[8][8], most[8] = {};
     bool fine = true;
@@ -351,7 +367,11 @@ __global__ void __launch_bounds__(ST_THREADS, 1) ssd_states_kernel(const SsdArgs
     }
     if (!fine) sm.bad_all = 1;
     asm volatile("bar.sync 2, 256;" ::: "memory");
-    rounders_of(sm.most_b, piece * 8, most);
+    scales_of(sm.most_b, piece * 8, most);
+    if (th < 16) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) sm.inv_b[piece * 8 + e] = inverse_of(most[e]);
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int t = (th >> 4) + i * 16;
@@ -371,9 +391,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) ssd_states_kernel(const SsdArgs
         const int b = j & 1;
         const uint32_t parity = (j >> 1) & 1;
         if (!wait_for(smem_u32(&sm.bars.x_full[b]), parity, dead) || !wait_for(smem_u32(&sm.bars.acc_empty[b]), parity ^ 1u, dead)) break;
+        mbar_arrive(smem_u32(&sm.bars.scaled[b]));
         tcgen05_fence_after();
         const uint32_t d = tmem + b * 192, xb = xs + b * 3 * UNIT;
-        issue<false>(PRODUCTS, 5, d, Operand{make_smem_desc_mn(base, TILE / 2), TILE >> 4, 512, 128}, Operand{make_smem_desc_mn(xb, UNIT), UNIT >> 4, 512, 128}, 64, mn);
+        issue<false>(PRODUCTS, 7, d, Operand{make_smem_desc_mn(base, TILE / 2), TILE >> 4, 512, 128}, Operand{make_smem_desc_mn(xb, UNIT), UNIT >> 4, 512, 128}, 64, mn);
         tcgen05_commit(smem_u32(&sm.bars.x_empty[b]));
         tcgen05_commit(smem_u32(&sm.bars.acc_full[b]));
       }
@@ -420,7 +441,11 @@ __global__ void __launch_bounds__(ST_THREADS, 1) ssd_states_kernel(const SsdArgs
         for (int e = 0; e < 8; e += 4) *reinterpret_cast<float4*>(&sm.most_x[warp - 4][lane * 8 + e]) = make_float4(most[e], most[e + 1], most[e + 2], most[e + 3]);
       }
       asm volatile("bar.sync 2, 256;" ::: "memory");
-      rounders_of(sm.most_x, (lane & 7) * 8, most);
+      scales_of(sm.most_x, (lane & 7) * 8, most);
+      if (th < 8) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sm.inv_x[j][th * 8 + e] = inverse_of(most[e]);
+      }
       if (alive) alive = warp_wait(smem_u32(&sm.bars.x_empty[b]), ((j >> 1) & 1) ^ 1u, dead);
       if (!alive) continue;                                        // (the others still meet at the barriers)
 #pragma unroll
@@ -444,8 +469,9 @@ __global__ void __launch_bounds__(ST_THREADS, 1) ssd_states_kernel(const SsdArgs
     if (!fine) sm.bad_all = 1;
     for (int j = 0; j < units; ++j) {
       const int b = j & 1;
-      if (!warp_wait(smem_u32(&sm.bars.acc_full[b]), (j >> 1) & 1, dead)) break;
+      if (!warp_wait(smem_u32(&sm.bars.scaled[b]), (j >> 1) & 1, dead) || !warp_wait(smem_u32(&sm.bars.acc_full[b]), (j >> 1) & 1, dead)) break;
       tcgen05_fence_after();
+      const float inv = sm.inv_b[warp * 32 + lane];
       float* dst = p.states + ((size_t)blockIdx.x * p.U + u0 + j) * P * N + warp * 32 + lane;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
@@ -459,8 +485,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) ssd_states_kernel(const SsdArgs
           if (lane == 0) mbar_arrive(smem_u32(&sm.bars.acc_empty[b]));
         }
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-          dst[(half * 32 + i) * N] = __uint_as_float(v[0][i]) + (__uint_as_float(v[1][i]) + __uint_as_float(v[2][i]));
+        for (int i = 0; i < 32; ++i) dst[(half * 32 + i) * N] = gathered(v[0][i], v[1][i], v[2][i]) * inv * sm.inv_x[j][half * 32 + i];
       }
     }
   }
@@ -545,13 +570,14 @@ __global__ void __launch_bounds__(CARRY, 4) ssd_carry_kernel(const SsdArgs p) {
 // TMEM: weights 192 columns, accumulators 192, C B^T 128 (its parts before: 384).
 constexpr int OUT_THREADS = 512;
 struct OutBars {
-  uint64_t cb_full, cb_read, s_full, x_full, w_full, inter_full, inter_read, intra_full, intra_read, drain;
+  uint64_t cb_full, cb_read, s_full, x_full, w_full, inter_scaled, inter_full, inter_read, intra_scaled, intra_full, intra_read, drain;     // scaled: as above
 };
 struct OutSmem {
   alignas(16) float dt[MAX_UNITS][L], a[MAX_UNITS][L], pre[MAX_UNITS][L];     // pre: the decays from the chunk's start up to a token
   alignas(16) float upto[MAX_UNITS][L], after[MAX_UNITS][L], block[MAX_UNITS][4];          // within its block of 32: up to it; after it, times its dt; the blocks' own
   alignas(16) float most_x[4][P];
   float most_w[2][L];
+  alignas(16) float inv_b[L], inv_c[L], inv_w[2][L], inv_s[2][P], inv_x[P];                // the scales' inverses; [2]: one unit's while the last one's are read
   int dead;
   uint32_t tmem;
   OutBars bars;
@@ -573,6 +599,8 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
     mbar_init(smem_u32(&sm.bars.s_full), 4);
     mbar_init(smem_u32(&sm.bars.x_full), 4);
     mbar_init(smem_u32(&sm.bars.w_full), 7);
+    mbar_init(smem_u32(&sm.bars.inter_scaled), 1);
+    mbar_init(smem_u32(&sm.bars.intra_scaled), 1);
     mbar_init(smem_u32(&sm.bars.inter_full), 1);
     mbar_init(smem_u32(&sm.bars.inter_read), 4);
     mbar_init(smem_u32(&sm.bars.intra_full), 1);
@@ -603,7 +631,8 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int t = ((tid & 255) >> 4) + (i0 + i) * 16;
-        const float r = rounder(most_of_row(v[i]));
+        const float r = scale_of(most_of_row(v[i]));
+        if ((tid & 15) == 0) (warp < 8 ? sm.inv_c : sm.inv_b)[t] = inverse_of(r);
         put_parts<0>(dst + t * 128 + (((tid & 7) ^ (t & 7)) << 4), TILE, v[i], &r);
       }
     }
@@ -651,7 +680,7 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
         for (int i = 0; i < 3; ++i) tmem_ld16(tmem + i * 128 + s0 + q + lanes, v[i]);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[0][i] = __float_as_uint(__uint_as_float(v[0][i]) + (__uint_as_float(v[1][i]) + __uint_as_float(v[2][i])));
+        for (int i = 0; i < 16; ++i) v[0][i] = __float_as_uint(gathered(v[0][i], v[1][i], v[2][i]) * sm.inv_c[t] * sm.inv_b[s0 + q + i]);
         tmem_st16(cb + q, v[0]);
       }
       tmem_st_wait();
@@ -718,12 +747,14 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
         for (int j = 0; j < units; ++j) {
           const uint32_t parity = j & 1;
           if (!wait_for(smem_u32(&sm.bars.s_full), parity, dead) || !wait_for(smem_u32(&sm.bars.intra_read), parity ^ 1u, dead)) break;
+          mbar_arrive(smem_u32(&sm.bars.inter_scaled));
           tcgen05_fence_after();
-          issue<false>(PRODUCTS, 5, acc, Operand{make_smem_desc(base), TILE >> 4, TILE >> 5, 2}, Operand{make_smem_desc(ss), P * 128 >> 4, S_HALF >> 4, 2}, 64, 0u);
+          issue<false>(PRODUCTS, 7, acc, Operand{make_smem_desc(base), TILE >> 4, TILE >> 5, 2}, Operand{make_smem_desc(ss), P * 128 >> 4, S_HALF >> 4, 2}, 64, 0u);
           tcgen05_commit(smem_u32(&sm.bars.inter_full));
           if (!wait_for(smem_u32(&sm.bars.x_full), parity, dead) || !wait_for(smem_u32(&sm.bars.inter_read), parity, dead) || !wait_for(smem_u32(&sm.bars.w_full), parity, dead)) break;
+          mbar_arrive(smem_u32(&sm.bars.intra_scaled));
           tcgen05_fence_after();
-          issue<true>(PRODUCTS, 5, acc, Operand{tmem, 64, 32, 8}, Operand{make_smem_desc_mn(xs, UNIT), UNIT >> 4, 512, 128}, 64, 1u << 16);
+          issue<true>(PRODUCTS, 7, acc, Operand{tmem, 64, 32, 8}, Operand{make_smem_desc_mn(xs, UNIT), UNIT >> 4, 512, 128}, 64, 1u << 16);
           tcgen05_commit(smem_u32(&sm.bars.intra_full));
         }
       __syncwarp();
@@ -741,16 +772,17 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
         most = fmaxf(most, sm.most_w[half ^ 1][t]);
         asm volatile("bar.sync %0, 64;" ::"r"(2 + own) : "memory");  // it is read
       }
-      const float r = rounder(most);
+      const float r = scale_of(most);
       if (alive && j > 0) {
         alive = warp_wait(smem_u32(&sm.bars.intra_full), (j - 1) & 1, dead);
         tcgen05_fence_after();
       }
+      if (half == 0) sm.inv_w[j & 1][t] = inverse_of(r);           // (the outputs of the last unit but one are done: the last one's products waited for them)
       if (alive) {
         weights(j, [&](int q, const float* w) {
           uint32_t part[3][8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) split3_unit(w[2 * i], w[2 * i + 1], r, r, part[0][i], part[1][i], part[2][i]);
+          for (int i = 0; i < 8; ++i) split3(w[2 * i], w[2 * i + 1], r, r, part[0][i], part[1][i], part[2][i]);
 #pragma unroll
           for (int k = 0; k < 3; ++k) tmem_st8(tmem + k * 64 + (s0 + q) / 2 + lanes, part[k]);
         });
@@ -766,9 +798,17 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
     for (; j < units && alive; ++j) {
       const uint32_t parity = j & 1;
       float y[P];
-      if (!(alive = warp_wait(smem_u32(&sm.bars.inter_full), parity, dead))) break;
+      const float dh = p.D[(u0 + j) / p.per_head];                 // D x, of x as it is
+      const float* xrow = p.x + (size_t)(c.row0 + t) * p.ld + (u0 + j) * P;
+#pragma unroll
+      for (int q = 0; q < P; q += 8) {
+        load8(xrow + q, t < c.tokens, y + q);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) y[q + i] *= dh;
+      }
+      if (!(alive = warp_wait(smem_u32(&sm.bars.inter_scaled), parity, dead) && warp_wait(smem_u32(&sm.bars.inter_full), parity, dead))) break;
       tcgen05_fence_after();
-      const float pre = sm.pre[j][t];
+      const float pre = sm.pre[j][t], inv_c = sm.inv_c[t];
 #pragma unroll
       for (int q = 0; q < P; q += 8) {
         uint32_t v[3][8];
@@ -776,27 +816,14 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
         for (int i = 0; i < 3; ++i) tmem_ld8(acc + i * 64 + q + lanes, v[i]);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) y[q + i] = pre * (__uint_as_float(v[0][i]) + (__uint_as_float(v[1][i]) + __uint_as_float(v[2][i])));
+        for (int i = 0; i < 8; ++i) y[q + i] = fmaf(pre, gathered(v[0][i], v[1][i], v[2][i]) * inv_c * sm.inv_s[j & 1][q + i], y[q + i]);
       }
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&sm.bars.inter_read));
-      if (!(alive = warp_wait(smem_u32(&sm.bars.x_full), parity, dead))) break;
-      const float dh = p.D[(u0 + j) / p.per_head];                 // D x: the parts' sum is x
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        float f[3][8];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          uint4 u;
-          asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "r"(xs + i * UNIT + t * 128 + ((k ^ (t & 7)) << 4)));
-          unpack8(u, f[i]);
-        }
-#pragma unroll
-        for (int e = 0; e < 8; ++e) y[8 * k + e] = fmaf(dh, f[0][e] + (f[1][e] + f[2][e]), y[8 * k + e]);
-      }
-      if (!(alive = warp_wait(smem_u32(&sm.bars.intra_full), parity, dead))) break;
+      if (!(alive = warp_wait(smem_u32(&sm.bars.intra_scaled), parity, dead) && warp_wait(smem_u32(&sm.bars.intra_full), parity, dead))) break;
       tcgen05_fence_after();
+      const float inv_w = sm.inv_w[j & 1][t];
       float* dst = p.o + (size_t)(c.row0 + t) * p.U * P + (u0 + j) * P;
 #pragma unroll
       for (int q = 0; q < P; q += 8) {
@@ -804,14 +831,14 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
 #pragma unroll
         for (int i = 0; i < 3; ++i) tmem_ld8(acc + i * 64 + q + lanes, v[i]);
         tmem_ld_wait();
+        float f[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = y[q + i] + gathered(v[0][i], v[1][i], v[2][i]) * inv_w * sm.inv_x[q + i];
         if (q == P - 8) {
           tcgen05_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&sm.bars.intra_read));           // x is read, too
+          if (lane == 0) mbar_arrive(smem_u32(&sm.bars.intra_read));           // the scales are read, too
         }
-        float f[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) f[i] = y[q + i] + (__uint_as_float(v[0][i]) + (__uint_as_float(v[1][i]) + __uint_as_float(v[2][i])));
         if (t < c.tokens) {
           *reinterpret_cast<float4*>(dst + q) = make_float4(f[0], f[1], f[2], f[3]);
           *reinterpret_cast<float4*>(dst + q + 4) = make_float4(f[4], f[5], f[6], f[7]);
@@ -829,12 +856,13 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
 #pragma unroll
       for (int i = 0; i < 8; ++i) load8(src + i * 1024, true, v[i]);
     };
-    auto put_state = [&]() {
+    auto put_state = [&](int j) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int r = (th >> 4) + i * 8;
-        const float unit = rounder(most_of_row(v[i]));
-        put_parts<0>(ss + ((th & 15) >> 3) * S_HALF + r * 128 + (((th & 7) ^ (r & 7)) << 4), P * 128, v[i], &unit);
+        const float scale = scale_of(most_of_row(v[i]));
+        if ((th & 15) == 0) sm.inv_s[j & 1][r] = inverse_of(scale);
+        put_parts<0>(ss + ((th & 15) >> 3) * S_HALF + r * 128 + (((th & 7) ^ (r & 7)) << 4), P * 128, v[i], &scale);
       }
       fence_proxy_async_smem();
       __syncwarp();
@@ -849,7 +877,7 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
       }
     };
     float most[8];
-    auto units_of_x = [&]() {
+    auto scales_of_x = [&]() {
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         most[e] = 0.f;
@@ -864,17 +892,21 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
         for (int e = 0; e < 8; e += 4) *reinterpret_cast<float4*>(&sm.most_x[warp - 12][lane * 8 + e]) = make_float4(most[e], most[e + 1], most[e + 2], most[e + 3]);
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");
-      rounders_of(sm.most_x, (lane & 7) * 8, most);
+      scales_of(sm.most_x, (lane & 7) * 8, most);
     };
     get_state(0);
     alive = warp_wait(smem_u32(&sm.bars.cb_full), 0u, dead) && warp_wait(smem_u32(&sm.bars.cb_read), 0u, dead);       // B and C B^T are read
     for (int j = 0; j < units; ++j) {                              // (the four warps meet at barriers whether alive or not)
       const uint32_t parity = j & 1;
-      if (alive) put_state();                                      // C S of the last unit is done: its outputs were waited for
+      if (alive) put_state(j);                                     // C S of the last unit is done: its outputs were waited for
       get_x(j);
-      units_of_x();
+      scales_of_x();
       if (alive && j > 0) alive = warp_wait(smem_u32(&sm.bars.intra_read), parity ^ 1u, dead);       // the last unit's x is read, by its product and by its outputs
       if (alive) {
+        if (th < 8) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) sm.inv_x[th * 8 + e] = inverse_of(most[e]);
+        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int t = (th >> 3) + i * 16;

@@ -158,6 +158,49 @@ def test_values_out_of_range_go_token_by_token(what, value, at):
         assert all(torch.equal(a.nan_to_num(nan=123.0), b.nan_to_num(nan=123.0)) for a, b in zip(same, like)), h
 
 
+@pytest.mark.parametrize("what", ["x", "column", "B", "C", "channels", "x and dt", "S"])
+@pytest.mark.parametrize("size", [300.0, 3e3, 1e5])
+@pytest.mark.parametrize("at", [5, 60, 127, 200])
+def test_small_numbers_beside_large_ones(what, size, at):
+    """Tokens before and after a large number, and the state, are no further from 64 bits than the token loop's, up to one more rounding of 2^-24; and each number by
+    itself is off by no more than 2^-20 of the sum of its terms' magnitudes (at most a dozen roundings and cut sums of 2^-24 lie between the inputs and a term)."""
+    H, G, vdim = 2, 1, 64
+    step = Step([300], H, G, vdim, seed=int(size) + at)
+    x, B, C = step.xbc[:, :step.inner], step.xbc[:, step.inner:step.inner + N], step.xbc[:, step.inner + N:]
+    if what in ("x", "x and dt"):
+        x[at] *= size
+        step.gates[at, :H] /= size if what == "x and dt" else 1.0
+    elif what == "column":
+        x[at, 7::vdim] *= size
+    elif what in ("B", "C"):
+        (B if what == "B" else C)[at] *= size
+    elif what == "channels":                                      # each of the two large where the other is as ever
+        B[:, 9] *= size
+        C[:, 7] *= size
+    else:
+        step.S0[:, :, :, at % N] *= size
+    new, old, want = step.run(), step.run(by_tokens=True), step.exact()
+    part = slice(7, None, vdim) if what == "column" else slice(None)
+    for rows in (slice(0, at), slice(at + 1, None), slice(at // 128 * 128, at)):       # (the row itself is one weight's rounding many times over: by the second bound)
+        n, o, w = (t[0][rows, part] for t in (new, old, want))
+        assert _rel(n, w) <= _rel(o, w) + 2.0 ** -24, (rows, _rel(n, w), _rel(o, w))
+    for t in (step.xbc, step.D, step.S0):
+        t.abs_()
+    assert all(bool(((n - w).abs() <= 2.0 ** -20 * m).all()) for n, w, m in zip(new, want, step.exact()))
+    slot = step.slots[0]
+    assert _rel(new[1][slot], want[1][slot]) <= _rel(old[1][slot], want[1][slot]) + 2.0 ** -24
+
+
+def test_the_skip_term_is_of_x_as_it_is():
+    """Without a state the outputs are D x and C B x dt: where that vanishes, D x rounded once."""
+    step = Step([300], 2, 1, 64)
+    step.gates[:, :2] = 0.0
+    step.S0.zero_()
+    step.xbc[131, :step.inner] *= 3e4
+    o, _ = step.run()
+    assert torch.equal(o, (step.D[:, None] * step.xbc[:, :step.inner].view(300, 2, 64)).reshape(300, -1))
+
+
 def test_rows_that_are_not_whole_vectors_and_other_shapes_go_token_by_token():
     for step in (Step([300], 2, 1, 64, pad=1), Step([300], 2, 1, 40), Step([255, 200], 2, 1, 64)):
         assert all(torch.equal(a, b) for a, b in zip(step.run(), step.run(by_tokens=True)))
