@@ -602,7 +602,7 @@ constexpr int SSD_TB = 16;        // tokens per stage
 template <int NJ, int RG, int TG, bool VL>
 __global__ void __launch_bounds__(128, TG > 1 ? 1 : (NJ <= 2 ? 5 : (NJ <= 4 ? 3 : 1))) ssd_scan_kernel(const float* __restrict__ B, const float* __restrict__ C, const float* __restrict__ x, int ld,
                                                        const float* __restrict__ gates, const float* __restrict__ D, float* __restrict__ St,
-                                                       const int* __restrict__ segs, int tok0, int span, int below, const int* __restrict__ flags, const float* __restrict__ after,
+                                                       const int* __restrict__ segs, int tok0, int span, int below, int longs, const int* __restrict__ flags, const float* __restrict__ after,
                                                        int H, int G, int N, int vdim, float* __restrict__ o) {
   pdl_launch_dependents();
   pdl_wait();
@@ -611,12 +611,19 @@ __global__ void __launch_bounds__(128, TG > 1 ? 1 : (NJ <= 2 ? 5 : (NJ <= 4 ? 3 
   const int seg = blockIdx.z, h = blockIdx.y, colb = blockIdx.x * SSD_COLS, g = h / (H / G);
   // (`span` is for the portions of `below` tokens and more: a shorter one is done whole with the first tokens of those)
   const int slot = segs[4 * seg], row0 = segs[4 * seg + 2] + tok0, all = segs[4 * seg + 3], len = all < below ? all : min(all - tok0, span);
-  if (all >= below && (len <= 0 || !flags[(size_t)seg * H + h])) {                  // ssd_chunk_sm100.cu had these tokens (span: some of its portion's at a time): the state
-    if (len <= 0) return;                                                            // after them is to go where it belongs
-    const size_t first = (size_t)h * vdim * N + (size_t)colb * N, all_heads = (size_t)H * vdim * N;
-    for (int e = threadIdx.x * 4; e < min(SSD_COLS, vdim - colb) * N; e += 512)
-      *reinterpret_cast<float4*>(St + slot * all_heads + first + e) = *reinterpret_cast<const float4*>(after + seg * all_heads + first + e);
-    return;
+  if (all >= below) {                          // ssd_chunk_sm100.cu had these tokens (span: some of its portion's at a time), but for the heads in `flags`
+    if (len <= 0) return;
+    int rank = 0;                              // among the portions that it takes
+    for (int k = threadIdx.x & 31; k < seg; k += 32) rank += segs[4 * k + 3] >= below;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, off);
+    if (rank >= longs) return;
+    if (!flags[(size_t)rank * H + h]) {        // the state after them is to go where it belongs
+      const size_t first = (size_t)h * vdim * N + (size_t)colb * N, all_heads = (size_t)H * vdim * N;
+      for (int e = threadIdx.x * 4; e < min(SSD_COLS, vdim - colb) * N; e += 512)
+        *reinterpret_cast<float4*>(St + slot * all_heads + first + e) = *reinterpret_cast<const float4*>(after + rank * all_heads + first + e);
+      return;
+    }
   }
   if (all < below && tok0 > 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rg = lane % RG;
@@ -787,9 +794,9 @@ __global__ void __launch_bounds__(128, TG > 1 ? 1 : (NJ <= 2 ? 5 : (NJ <= 4 ? 3 
 }
 
 struct SsdTokens {                             // which tokens: those of portions shorter than `below`, and tok0 .. tok0 + span - 1 of the heads that `flags` names
-  int tok0 = 0, span = INT_MAX, below = INT_MAX;
-  const int* flags = nullptr;
-  const float* after = nullptr;                // [nseg][H][vdim][N], for the other heads of the longer portions
+  int tok0 = 0, span = INT_MAX, below = INT_MAX, longs = 0;
+  const int* flags = nullptr;                  // [longs][H]: the portions of `below` tokens and more, in order
+  const float* after = nullptr;                // [longs][H][vdim][N], for their other heads
 };
 
 template <int NJ, int RG, int TG, bool VL>
@@ -800,7 +807,7 @@ int launch_ssd_as(const SsdTokens& w, const float* B, const float* C, const floa
   if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(ssd_scan_kernel<NJ, RG, TG, VL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((vdim + COLS - 1) / COLS, H, nseg);
   // beside the chunks there is seldom much to do, and nothing to crowd out
-  lia_launch_as(w.flags != nullptr, ssd_scan_kernel<NJ, RG, TG, VL>, dim3(grid), dim3(128), smem, stream, B, C, x, ld, gates, D, St, segs, w.tok0, w.span, w.below, w.flags, w.after, H, G, N,
+  lia_launch_as(w.flags != nullptr, ssd_scan_kernel<NJ, RG, TG, VL>, dim3(grid), dim3(128), smem, stream, B, C, x, ld, gates, D, St, segs, w.tok0, w.span, w.below, w.longs, w.flags, w.after, H, G, N,
                 vdim, o);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
@@ -1016,9 +1023,9 @@ extern "C" int lia_conv_act(const void* y, int y_f32, int ld, int col0, int C, c
   return LIA_OK;
 }
 
-int ssd_scan_tokens(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* St, const int* segs, int tok0, int span, int below,
+int ssd_scan_tokens(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* St, const int* segs, int tok0, int span, int below, int longs,
                     const int* flags, const float* after, int nseg, int H, int G, int N, int vdim, float* o, cudaStream_t stream) {
-  return launch_ssd<2, 16, 4>(SsdTokens{tok0, span, below, flags, after}, false, B, C, x, ld, gates, D, St, segs, nseg, H, G, N, vdim, o, stream);      // N = 128
+  return launch_ssd<2, 16, 4>(SsdTokens{tok0, span, below, longs, flags, after}, false, B, C, x, ld, gates, D, St, segs, nseg, H, G, N, vdim, o, stream);      // N = 128
 }
 
 extern "C" int lia_ssd_scan(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* state_S, const int* segs,

@@ -27,14 +27,14 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
-#include <mutex>
+#include <algorithm>
 
 #include "common.cuh"
 #include "mma.cuh"
 #include "umma.cuh"
 
 int* lia_timeout_word();                                           // moe_sm100.cu
-int ssd_scan_tokens(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* St, const int* segs, int tok0, int span, int below,
+int ssd_scan_tokens(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* St, const int* segs, int tok0, int span, int below, int longs,
                     const int* flags, const float* after, int nseg, int H, int G, int N, int vdim, float* o, cudaStream_t stream);     // linear_scan.cu
 
 namespace {
@@ -56,9 +56,10 @@ struct SsdArgs {
   const int* segs;
   int nseg, H, G, U, per_head;                 // U: units in all; per_head: units of a head
   float* o;
-  float *states, *after;                       // [slots][U][P][N]; [nseg][U][P][N]: after the portions' tokens
+  float *states, *after;                       // [slots][U][P][N]; [longs][U][P][N]: after the tokens of the portions of SHORT tokens and more, in order
   float2* totals;                              // [slots][U]: the product of a chunk's decays, and what is left of it
-  int *bad, *flags;                            // [slots][U], [nseg][H]
+  int *bad, *flags;                            // [slots][U], [longs][H]
+  int slots, longs;
   int tok0, span, split, per_cta;              // the tokens tok0 .. tok0 + span - 1 of every portion; a group's units in `split` CTAs of `per_cta`
   int* timeouts;
 };
@@ -174,6 +175,27 @@ __device__ __forceinline__ bool locate(const SsdArgs& p, int i, Chunk& c) {
       return true;
     }
     i -= __shfl_sync(0xffffffffu, sum, 31);
+  }
+  return false;
+}
+
+// The rank-th portion of SHORT tokens and more, and the chunks before it (a whole warp asks)
+__device__ __forceinline__ bool nth_long(const SsdArgs& p, int rank, int& seg, int& before) {
+  const int lane = threadIdx.x & 31;
+  before = 0;
+  for (int k0 = 0; k0 < p.nseg; k0 += 32) {
+    const int k = k0 + lane;
+    const unsigned taken = __ballot_sync(0xffffffffu, k < p.nseg && p.segs[4 * k + 3] >= SHORT);
+    const int found = __popc(taken), at = rank < found ? (int)__fns(taken, 0, rank + 1) : 32;
+    int n = k < p.nseg && lane < at ? (window_tokens(p, k) + L - 1) / L : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    before += n;
+    if (rank < found) {
+      seg = k0 + at;
+      return true;
+    }
+    rank -= found;
   }
   return false;
 }
@@ -515,16 +537,11 @@ constexpr int CARRY = 256;
 __global__ void __launch_bounds__(CARRY, 4) ssd_carry_kernel(const SsdArgs p) {
   pdl_launch_dependents();
   pdl_wait();
-  const int u = blockIdx.x >> 3, seg = blockIdx.y, lane = threadIdx.x & 31;
-  const int tokens = window_tokens(p, seg), n = (tokens + L - 1) / L;
-  if (n == 0) {
-    if ((blockIdx.x & 7) == 0 && threadIdx.x == 0) p.flags[(size_t)seg * p.H + u / p.per_head] = 0;
-    return;
-  }
-  int before = 0;
-  for (int k = lane; k < seg; k += 32) before += (window_tokens(p, k) + L - 1) / L;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  const int u = blockIdx.x >> 3, rank = blockIdx.y;
+  int seg, before;
+  if (!nth_long(p, rank, seg, before)) return;
+  const int n = (window_tokens(p, seg) + L - 1) / L;
+  if (n == 0 || before + n > p.slots) return;
   const int head0 = u / p.per_head * p.per_head;
   int bad = 0;
   for (int e = threadIdx.x; e < n * p.per_head; e += CARRY) bad |= p.bad[(size_t)(before + e / p.per_head) * p.U + head0 + e % p.per_head];
@@ -537,7 +554,7 @@ __global__ void __launch_bounds__(CARRY, 4) ssd_carry_kernel(const SsdArgs p) {
     for (int i = 0; i < 8; ++i) bad |= !(fabsf(v[i].x) < BIG_STATE && fabsf(v[i].y) < BIG_STATE && fabsf(v[i].z) < BIG_STATE && fabsf(v[i].w) < BIG_STATE);
   }
   bad = __syncthreads_or(bad);
-  if ((blockIdx.x & 7) == 0 && threadIdx.x == 0) p.flags[(size_t)seg * p.H + u / p.per_head] = bad;
+  if ((blockIdx.x & 7) == 0 && threadIdx.x == 0) p.flags[(size_t)rank * p.H + u / p.per_head] = bad;
   const size_t at = (size_t)u * (P * N / 4) + (blockIdx.x & 7) * CARRY + threadIdx.x, step = (size_t)p.U * (P * N / 4);
   float4* st = reinterpret_cast<float4*>(p.states) + (size_t)before * step + at;
   const float2* total = p.totals + (size_t)before * p.U + u;
@@ -561,7 +578,7 @@ __global__ void __launch_bounds__(CARRY, 4) ssd_carry_kernel(const SsdArgs p) {
         S.w = fmaf(f[i].x, S.w, fmaf(f[i].y, S.w, local[i].w));
       }
   }
-  reinterpret_cast<float4*>(p.after)[(size_t)seg * step + at] = S;     // (the token loop may still need what is in St)
+  reinterpret_cast<float4*>(p.after)[(size_t)rank * step + at] = S;     // (the token loop may still need what is in St)
 }
 
 // ------------------------------------------------------------------------------------------------ outputs
@@ -938,8 +955,10 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
 }
 
 long long round16(long long n) { return (n + 15) / 16 * 16; }
-long long slots_of(long long rows, long long nseg, long long chunks) { return nseg * chunks < (rows + nseg * (L - 1)) / L ? nseg * chunks : (rows + nseg * (L - 1)) / L; }
-long long bytes_of(long long slots, long long nseg, int H, long long U) { return slots * U * (P * N * 4 + 12) + nseg * U * P * N * 4 + round16(4 * nseg * H) + 16; }
+// of `longs` portions of SHORT tokens and more, `rows` tokens together
+long long slots_of(long long rows, long long longs, long long chunks) { return std::min(longs * chunks, (rows + longs * (L - 1)) / L); }
+long long bytes_of(long long slots, long long longs, int H, long long U) { return slots * U * (P * N * 4 + 12) + longs * U * P * N * 4 + round16(4 * longs * H) + 16; }
+int longs_of(int rows, int nseg) { return std::max(1, std::min(nseg, rows / SHORT)); }         // at most
 
 }  // namespace
 
@@ -950,26 +969,28 @@ extern "C" long long lia_ssd_workspace(int rows, int nseg, int H, int G, int Ns,
   if (Ns != N || vdim <= 0 || vdim % P || nseg <= 0 || nseg > 65535 || H <= 0 || G <= 0 || H % G || chunks <= 0 || rows - nseg + 1 < SHORT) return 0;
   const long long U = (long long)H * (vdim / P);
   if (U > 8191) return 0;
-  return bytes_of(slots_of(rows, nseg, chunks), nseg, H, U);
+  const int longs = longs_of(rows, nseg);
+  return bytes_of(slots_of(rows, longs, chunks), longs, H, U);
 }
 
-extern "C" int lia_ssd_scan_chunks(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* state_S, const int* segs, int nseg,
-                                   int rows, int H, int G, int Ns, int vdim, float* o, void* ws, long long ws_bytes, int chunks, lia_stream_t stream_) {
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-  LIA_CHECK_ARG(B && C && x && gates && D && state_S && segs && o && ws, "lia_ssd_scan_chunks: null pointer");
-  const long long need = lia_ssd_workspace(rows, nseg, H, G, Ns, vdim, chunks);
-  LIA_CHECK_ARG(need > 0, "lia_ssd_scan_chunks: bad shape nseg=%d rows=%d H=%d G=%d N=%d vdim=%d", nseg, rows, H, G, Ns, vdim);
+// `longs` portions of SHORT tokens and more, `long_rows` tokens together and `longest` at most
+static int scan_chunks(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* state_S, const int* segs, int nseg, int longs, int long_rows,
+                       int longest, int H, int G, int Ns, int vdim, float* o, void* ws, long long ws_bytes, int chunks, cudaStream_t stream) {
+  const long long need = lia_ssd_workspace(long_rows, longs, H, G, Ns, vdim, chunks);
+  LIA_CHECK_ARG(need > 0 && nseg > 0 && nseg <= 65535, "lia_ssd_scan_chunks: bad shape nseg=%d rows=%d H=%d G=%d N=%d vdim=%d", nseg, long_rows, H, G, Ns, vdim);
   LIA_CHECK_ARG(ws_bytes >= need, "lia_ssd_scan_chunks: the workspace holds %lld of %lld bytes", ws_bytes, need);
   const uintptr_t all = reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(state_S) |
                         reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(ws);
   LIA_CHECK_ARG(all % 16 == 0 && ld % 4 == 0, "lia_ssd_scan_chunks: rows are not whole 16-byte vectors");
   const int U = H * (vdim / P), per_group = U / G, sms = lia_sm_count();
-  const long long slots = slots_of(rows, nseg, chunks);
+  const long long slots = slots_of(long_rows, longs, chunks);
   LIA_CHECK_ARG(slots < (1ll << 31), "lia_ssd_scan_chunks: too many rows");
   SsdArgs p{B, C, x, ld, gates, D, state_S, segs, nseg, H, G, U, vdim / P, o};
   p.states = reinterpret_cast<float*>(ws);
   p.after = p.states + slots * U * P * N;
-  p.totals = reinterpret_cast<float2*>(p.after + (long long)nseg * U * P * N);
+  p.slots = (int)slots;
+  p.longs = longs;
+  p.totals = reinterpret_cast<float2*>(p.after + (long long)longs * U * P * N);
   p.bad = reinterpret_cast<int*>(p.totals + slots * U);
   p.flags = p.bad + slots * U;
   p.timeouts = lia_timeout_word();
@@ -982,17 +1003,32 @@ extern "C" int lia_ssd_scan_chunks(const float* B, const float* C, const float* 
   LIA_CUDA(cudaFuncSetAttribute(ssd_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_BYTES));
   LIA_CUDA(cudaFuncSetAttribute(ssd_outputs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OUT_BYTES));
   p.span = chunks * L;
-  for (int tok0 = 0; tok0 < rows; tok0 += p.span) {                 // a portion has `rows` tokens at most (the others may be empty)
+  for (int tok0 = 0; tok0 < longest; tok0 += p.span) {
     p.tok0 = tok0;
     const dim3 grid((unsigned)slots, (unsigned)(G * p.split));
     lia_launch(ssd_states_kernel, grid, dim3(ST_THREADS), ST_BYTES, stream, p);
     LIA_LAUNCH_CHECK();
-    lia_launch(ssd_carry_kernel, dim3((unsigned)U * 8, (unsigned)nseg), dim3(CARRY), 0, stream, p);
+    lia_launch(ssd_carry_kernel, dim3((unsigned)U * 8, (unsigned)longs), dim3(CARRY), 0, stream, p);
     LIA_LAUNCH_CHECK();
     lia_launch(ssd_outputs_kernel, grid, dim3(OUT_THREADS), OUT_BYTES, stream, p);
     LIA_LAUNCH_CHECK();
-    const int rc = ssd_scan_tokens(B, C, x, ld, gates, D, state_S, segs, tok0, p.span, SHORT, p.flags, p.after, nseg, H, G, Ns, vdim, o, stream);
+    const int rc = ssd_scan_tokens(B, C, x, ld, gates, D, state_S, segs, tok0, p.span, SHORT, longs, p.flags, p.after, nseg, H, G, Ns, vdim, o, stream);
     if (rc != LIA_OK) return rc;
   }
   return LIA_OK;
+}
+
+/* see lia_b200.h */
+extern "C" int lia_ssd_scan_chunks(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* state_S, const int* segs, int nseg,
+                                   int rows, int H, int G, int Ns, int vdim, float* o, void* ws, long long ws_bytes, int chunks, lia_stream_t stream) {
+  LIA_CHECK_ARG(B && C && x && gates && D && state_S && segs && o && ws, "lia_ssd_scan_chunks: null pointer");
+  LIA_CHECK_ARG(lia_ssd_workspace(rows, nseg, H, G, Ns, vdim, chunks) > 0, "lia_ssd_scan_chunks: bad shape nseg=%d rows=%d H=%d G=%d N=%d vdim=%d", nseg, rows, H, G, Ns, vdim);
+  return scan_chunks(B, C, x, ld, gates, D, state_S, segs, nseg, longs_of(rows, nseg), rows, rows, H, G, Ns, vdim, o, ws, ws_bytes, chunks, reinterpret_cast<cudaStream_t>(stream));
+}
+extern "C" int lia_ssd_scan_long(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* state_S, const int* segs, int nseg,
+                                 int longs, int long_rows, int longest, int H, int G, int Ns, int vdim, float* o, void* ws, long long ws_bytes, int chunks, lia_stream_t stream) {
+  LIA_CHECK_ARG(B && C && x && gates && D && state_S && segs && o && ws, "lia_ssd_scan_long: null pointer");
+  LIA_CHECK_ARG(longs > 0 && longs <= nseg && longest >= SHORT && longest <= long_rows && (long long)longs * SHORT <= long_rows && chunks > 0,
+                "lia_ssd_scan_long: %d portions of %d tokens, the longest one's %d", longs, long_rows, longest);
+  return scan_chunks(B, C, x, ld, gates, D, state_S, segs, nseg, longs, long_rows, longest, H, G, Ns, vdim, o, ws, ws_bytes, chunks, reinterpret_cast<cudaStream_t>(stream));
 }

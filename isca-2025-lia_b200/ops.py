@@ -1280,9 +1280,9 @@ def conv_act(y, col0, wconv, out, batch, state=None, in_bias=None, bias=None, ac
     return out
 
 
-def ssd_scan(xbc, gates, D, state_S, segs, H, G, N, vdim, o):
-    """State-space dual recurrence S = g S + dt B x^T, o = S^T C + D x over every portion of the step (csrc/linear_scan.cu).  ``xbc`` fp32
-    [M, H vdim + 2 G N] = x | B | C; gates [M, 2H] = dt | g; state_S [slots, H, vdim, N]."""
+def ssd_scan(xbc, gates, D, state_S, segs, H, G, N, vdim, o, portions=None):
+    """State-space dual recurrence S = g S + dt B x^T, o = S^T C + D x over every portion of the step (csrc/linear_scan.cu; long portions csrc/ssd_chunk_sm100.cu).
+    ``xbc`` fp32 [M, H vdim + 2 G N] = x | B | C; gates [M, 2H] = dt | g; state_S [slots, H, vdim, N].  ``portions``: the numbers of ``segs`` on the host, if known."""
     ld = _rowmajor(xbc, "xbc")
     M, inner = xbc.shape[0], H * vdim
     for t, n in ((gates, "gates"), (D, "D"), (state_S, "state_S"), (o, "o")):
@@ -1292,33 +1292,48 @@ def ssd_scan(xbc, gates, D, state_S, segs, H, G, N, vdim, o):
             or tuple(state_S.shape[1:]) != (H, vdim, N):
         raise _lib.LiaError("ssd_scan: shapes do not agree")
     lib, nseg = _lib.load(), segs.shape[0]
-    args = (_p(xbc[:, inner:]), _p(xbc[:, inner + G * N:]), _p(xbc), ld, _p(gates), _p(D), _p(state_S), _p(segs), nseg, M, H, G, N, vdim, _p(o))
-    chunks, ws = _ssd_workspace(lib, M, nseg, H, G, N, vdim, (xbc, state_S, o), ld, inner)
-    if ws is not None:
-        check(lib.lia_ssd_scan_chunks(*args, _p(ws), ws.numel(), chunks, _stream()), "lia_ssd_scan_chunks")
-        count_launches(4 * -(-M // (128 * chunks)))
-    else:
-        check(lib.lia_ssd_scan(*args, _stream()), "lia_ssd_scan")
+    first, shape = (_p(xbc[:, inner:]), _p(xbc[:, inner + G * N:]), _p(xbc), ld, _p(gates), _p(D), _p(state_S), _p(segs), nseg), (H, G, N, vdim)
+    longs, long_rows, longest, chunks, ws = _ssd_chunks(lib, M, nseg, shape, portions, (xbc, state_S, o), ld)
+    if ws is None:
+        check(lib.lia_ssd_scan(*first, M, *shape, _p(o), _stream()), "lia_ssd_scan")
         count_launches()
+    else:
+        if portions is None:
+            check(lib.lia_ssd_scan_chunks(*first, M, *shape, _p(o), _p(ws), ws.numel(), chunks, _stream()), "lia_ssd_scan_chunks")
+        else:
+            check(lib.lia_ssd_scan_long(*first, longs, long_rows, longest, *shape, _p(o), _p(ws), ws.numel(), chunks, _stream()), "lia_ssd_scan_long")
+        count_launches(4 * -(-longest // (128 * chunks)))
     return o
 
 
 SSD_WORKSPACE = 256 << 20                                     # bytes for the states between chunks; longer steps take some chunks of every portion at a time
 
 
-def _ssd_workspace(lib, M, nseg, H, G, N, vdim, tensors, ld, inner):
-    """How many chunks of every portion to take at a time, and their workspace; None: token by token (csrc/ssd_chunk_sm100.cu).  The result does not depend on
-    the number, so that less is taken where memory is short."""
-    one = lib.lia_ssd_workspace(M, nseg, H, G, N, vdim, 1)
-    if not one or ld % 4 or any(t.data_ptr() % 16 for t in tensors):
-        return 0, None
-    chunks = max(1, min(-(-M // 128), SSD_WORKSPACE // one))
+def _ssd_chunks(lib, M, nseg, shape, portions, tensors, ld):
+    """The portions that go in chunks (csrc/ssd_chunk_sm100.cu) -- how many, their tokens together, the longest one's; unknown: what there can be --, how many chunks of each to
+    take at a time, and the workspace (None: all go token by token).  The result does not depend on the number, so that less is taken where memory is short."""
+    line, none = lib.lia_ssd_chunk_rows(), (0, 0, 0, 0, None)
+    if portions is not None:
+        lens = [n for _, _, _, n in portions if n >= line]
+        if not lens:
+            return none
+        longs, long_rows, longest = len(lens), sum(lens), max(lens)
+    elif M < line:
+        return none
+    else:
+        longs, long_rows, longest = nseg, M, M
+    size = lambda chunks: lib.lia_ssd_workspace(long_rows, longs, *shape, chunks)  # noqa: E731
+    if ld % 4 or any(t.data_ptr() % 16 for t in tensors) or not size(1):
+        return none
+    chunks = -(-longest // 128)
+    while chunks > 1 and size(chunks) > SSD_WORKSPACE:
+        chunks -= -(-chunks // 8)
     while True:
         try:
-            return chunks, torch.empty(lib.lia_ssd_workspace(M, nseg, H, G, N, vdim, chunks), dtype=torch.uint8, device=tensors[0].device)
+            return longs, long_rows, longest, chunks, torch.empty(size(chunks), dtype=torch.uint8, device=tensors[0].device)
         except torch.OutOfMemoryError:
             if chunks == 1:
-                return 0, None
+                return none
             chunks = (chunks + 1) // 2
 
 

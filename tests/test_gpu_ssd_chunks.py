@@ -201,6 +201,27 @@ def test_the_skip_term_is_of_x_as_it_is():
     assert torch.equal(o, (step.D[:, None] * step.xbc[:, :step.inner].view(300, 2, 64)).reshape(300, -1))
 
 
+@pytest.mark.parametrize("lens,H,known,unknown", [([128] * 16, 8, 1, 4), ([100] * 4, 8, 1, 4), ([1] * 300, 8, 1, 4), ([2048] + [1] * 63, 64, 4, 4), ([300] + [1] * 256, 64, 4, 4),
+                                                  ([300, 1, 600] + [7] * 40, 4, 4, 4)])
+def test_passes_by_the_portions(lens, H, known, unknown):
+    """The form is chosen from the portions and the passes from the long ones among them: single tokens beside a prompt add neither passes nor workspace."""
+    step = Step(lens, H, 2, 64)
+    S, o, d = step.S0.clone(), torch.empty(step.xbc.shape[0], step.inner, device="cuda"), torch.tensor(step.segs, dtype=torch.int32, device="cuda")
+    before = _lib.launch_count
+    ops.ssd_scan(step.xbc, step.gates, step.D, S, d, H, 2, N, 64, o, portions=step.segs)
+    mid = _lib.launch_count
+    other = step.run()
+    assert mid - before == known and _lib.launch_count - mid <= unknown
+    assert torch.equal(o, other[0]) and torch.equal(S, other[1])
+    want = step.exact() if sum(lens) < 1000 else step.run(by_tokens=True)
+    for a, w in zip((o, S), want):
+        assert _rel(a, w.double()) <= 2.0 ** -21                 # (the sums of either side are tested above)
+    long = [n for n in lens if n >= _lib.load().lia_ssd_chunk_rows()]
+    if long:
+        few, whole = (_lib.load().lia_ssd_workspace(m, n, H, 2, N, 64, -(-max(long) // 128)) for m, n in ((sum(long), len(long)), (sum(lens), len(lens))))
+        assert few <= whole <= 2 * few
+
+
 def test_rows_that_are_not_whole_vectors_and_other_shapes_go_token_by_token():
     for step in (Step([300], 2, 1, 64, pad=1), Step([300], 2, 1, 40), Step([255, 200], 2, 1, 64)):
         assert all(torch.equal(a, b) for a, b in zip(step.run(), step.run(by_tokens=True)))
