@@ -620,13 +620,13 @@ int lia_ssd_scan(const float* B, const float* C, const float* x, int ld, const f
 /* The same with the portions of lia_ssd_chunk_rows() tokens and more in chunks on the tensor cores, `chunks` chunks (of 128 tokens) of every portion at a time; N = 128,
  * vdim a multiple of 64, all rows whole 16-byte vectors.  ws: lia_ssd_workspace() bytes for the same shape and chunks, which is 0 where lia_ssd_scan() is to be called.
  * The result does not depend on `chunks`.  lia_ssd_scan_long() is for callers who know these portions: `longs` of them, `long_rows` tokens together, the longest one's
- * `longest`, ws of lia_ssd_workspace(long_rows, longs, ...) bytes; without any, lia_ssd_scan() is to be called */
+ * `longest`, the longest one's of the others `others`, ws of lia_ssd_workspace(long_rows, longs, ...) bytes; without any, lia_ssd_scan() is to be called */
 int lia_ssd_chunk_rows(void);
 long long lia_ssd_workspace(int rows, int nseg, int H, int G, int N, int vdim, int chunks);
 int lia_ssd_scan_chunks(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* state_S, const int* segs, int nseg, int rows,
                         int H, int G, int N, int vdim, float* o, void* ws, long long ws_bytes, int chunks, lia_stream_t stream);
 int lia_ssd_scan_long(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* state_S, const int* segs, int nseg, int longs,
-                      int long_rows, int longest, int H, int G, int N, int vdim, float* o, void* ws, long long ws_bytes, int chunks, lia_stream_t stream);
+                      int long_rows, int longest, int others, int H, int G, int N, int vdim, float* o, void* ws, long long ws_bytes, int chunks, lia_stream_t stream);
 /* Real-gated linear recurrent unit over every portion, channel by channel (width = blocks * n): log a = c sigmoid(r + its bias),
  * S = a S + sqrt(1 - a^2) sigmoid(i + its bias) u, out = S * gelu_tanh(y + y_bias) of y's type; z [rows][blocks][2n] = r | i,
  * z_bias [blocks][2n], state [slot][width] fp32; y has row stride ldy, y_bias may be NULL; rows as above */

@@ -223,7 +223,7 @@ _PROTOTYPES = {
     "lia_ssd_scan_chunks": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
                                     c_void_p, c_longlong, c_int, c_void_p]),
     "lia_ssd_scan_long": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                                  c_void_p, c_void_p, c_longlong, c_int, c_void_p]),
+                                  c_int, c_void_p, c_void_p, c_longlong, c_int, c_void_p]),
     "lia_rglru_scan": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                c_void_p, c_void_p]),
     "lia_router_topk_grouped": (c_int, [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),

@@ -1024,8 +1024,8 @@ extern "C" int lia_conv_act(const void* y, int y_f32, int ld, int col0, int C, c
 }
 
 int ssd_scan_tokens(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* St, const int* segs, int tok0, int span, int below, int longs,
-                    const int* flags, const float* after, int nseg, int H, int G, int N, int vdim, float* o, cudaStream_t stream) {
-  return launch_ssd<2, 16, 4>(SsdTokens{tok0, span, below, longs, flags, after}, false, B, C, x, ld, gates, D, St, segs, nseg, H, G, N, vdim, o, stream);      // N = 128
+                    const int* flags, const float* after, bool single, int nseg, int H, int G, int N, int vdim, float* o, cudaStream_t stream) {
+  return launch_ssd<2, 16, 4>(SsdTokens{tok0, span, below, longs, flags, after}, single, B, C, x, ld, gates, D, St, segs, nseg, H, G, N, vdim, o, stream);      // N = 128
 }
 
 extern "C" int lia_ssd_scan(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* state_S, const int* segs,

@@ -35,7 +35,7 @@
 
 int* lia_timeout_word();                                           // moe_sm100.cu
 int ssd_scan_tokens(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* St, const int* segs, int tok0, int span, int below, int longs,
-                    const int* flags, const float* after, int nseg, int H, int G, int N, int vdim, float* o, cudaStream_t stream);     // linear_scan.cu
+                    const int* flags, const float* after, bool single, int nseg, int H, int G, int N, int vdim, float* o, cudaStream_t stream);      // linear_scan.cu
 
 namespace {
 
@@ -973,9 +973,9 @@ extern "C" long long lia_ssd_workspace(int rows, int nseg, int H, int G, int Ns,
   return bytes_of(slots_of(rows, longs, chunks), longs, H, U);
 }
 
-// `longs` portions of SHORT tokens and more, `long_rows` tokens together and `longest` at most
+// `longs` portions of SHORT tokens and more, `long_rows` tokens together and `longest` at most; the others `others`
 static int scan_chunks(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* state_S, const int* segs, int nseg, int longs, int long_rows,
-                       int longest, int H, int G, int Ns, int vdim, float* o, void* ws, long long ws_bytes, int chunks, cudaStream_t stream) {
+                       int longest, int others, int H, int G, int Ns, int vdim, float* o, void* ws, long long ws_bytes, int chunks, cudaStream_t stream) {
   const long long need = lia_ssd_workspace(long_rows, longs, H, G, Ns, vdim, chunks);
   LIA_CHECK_ARG(need > 0 && nseg > 0 && nseg <= 65535, "lia_ssd_scan_chunks: bad shape nseg=%d rows=%d H=%d G=%d N=%d vdim=%d", nseg, long_rows, H, G, Ns, vdim);
   LIA_CHECK_ARG(ws_bytes >= need, "lia_ssd_scan_chunks: the workspace holds %lld of %lld bytes", ws_bytes, need);
@@ -1012,7 +1012,7 @@ static int scan_chunks(const float* B, const float* C, const float* x, int ld, c
     LIA_LAUNCH_CHECK();
     lia_launch(ssd_outputs_kernel, grid, dim3(OUT_THREADS), OUT_BYTES, stream, p);
     LIA_LAUNCH_CHECK();
-    const int rc = ssd_scan_tokens(B, C, x, ld, gates, D, state_S, segs, tok0, p.span, SHORT, longs, p.flags, p.after, nseg, H, G, Ns, vdim, o, stream);
+    const int rc = ssd_scan_tokens(B, C, x, ld, gates, D, state_S, segs, tok0, p.span, SHORT, longs, p.flags, p.after, others == 1, nseg, H, G, Ns, vdim, o, stream);
     if (rc != LIA_OK) return rc;
   }
   return LIA_OK;
@@ -1023,12 +1023,13 @@ extern "C" int lia_ssd_scan_chunks(const float* B, const float* C, const float* 
                                    int rows, int H, int G, int Ns, int vdim, float* o, void* ws, long long ws_bytes, int chunks, lia_stream_t stream) {
   LIA_CHECK_ARG(B && C && x && gates && D && state_S && segs && o && ws, "lia_ssd_scan_chunks: null pointer");
   LIA_CHECK_ARG(lia_ssd_workspace(rows, nseg, H, G, Ns, vdim, chunks) > 0, "lia_ssd_scan_chunks: bad shape nseg=%d rows=%d H=%d G=%d N=%d vdim=%d", nseg, rows, H, G, Ns, vdim);
-  return scan_chunks(B, C, x, ld, gates, D, state_S, segs, nseg, longs_of(rows, nseg), rows, rows, H, G, Ns, vdim, o, ws, ws_bytes, chunks, reinterpret_cast<cudaStream_t>(stream));
+  return scan_chunks(B, C, x, ld, gates, D, state_S, segs, nseg, longs_of(rows, nseg), rows, rows, SHORT - 1, H, G, Ns, vdim, o, ws, ws_bytes, chunks, reinterpret_cast<cudaStream_t>(stream));
 }
 extern "C" int lia_ssd_scan_long(const float* B, const float* C, const float* x, int ld, const float* gates, const float* D, float* state_S, const int* segs, int nseg,
-                                 int longs, int long_rows, int longest, int H, int G, int Ns, int vdim, float* o, void* ws, long long ws_bytes, int chunks, lia_stream_t stream) {
+                                 int longs, int long_rows, int longest, int others, int H, int G, int Ns, int vdim, float* o, void* ws, long long ws_bytes, int chunks,
+                                 lia_stream_t stream) {
   LIA_CHECK_ARG(B && C && x && gates && D && state_S && segs && o && ws, "lia_ssd_scan_long: null pointer");
-  LIA_CHECK_ARG(longs > 0 && longs <= nseg && longest >= SHORT && longest <= long_rows && (long long)longs * SHORT <= long_rows && chunks > 0,
+  LIA_CHECK_ARG(longs > 0 && longs <= nseg && longest >= SHORT && longest <= long_rows && (long long)longs * SHORT <= long_rows && others >= 0 && others < SHORT && chunks > 0,
                 "lia_ssd_scan_long: %d portions of %d tokens, the longest one's %d", longs, long_rows, longest);
-  return scan_chunks(B, C, x, ld, gates, D, state_S, segs, nseg, longs, long_rows, longest, H, G, Ns, vdim, o, ws, ws_bytes, chunks, reinterpret_cast<cudaStream_t>(stream));
+  return scan_chunks(B, C, x, ld, gates, D, state_S, segs, nseg, longs, long_rows, longest, others, H, G, Ns, vdim, o, ws, ws_bytes, chunks, reinterpret_cast<cudaStream_t>(stream));
 }

@@ -1293,7 +1293,7 @@ def ssd_scan(xbc, gates, D, state_S, segs, H, G, N, vdim, o, portions=None):
         raise _lib.LiaError("ssd_scan: shapes do not agree")
     lib, nseg = _lib.load(), segs.shape[0]
     first, shape = (_p(xbc[:, inner:]), _p(xbc[:, inner + G * N:]), _p(xbc), ld, _p(gates), _p(D), _p(state_S), _p(segs), nseg), (H, G, N, vdim)
-    longs, long_rows, longest, chunks, ws = _ssd_chunks(lib, M, nseg, shape, portions, (xbc, state_S, o), ld)
+    longs, long_rows, longest, others, chunks, ws = _ssd_chunks(lib, M, nseg, shape, portions, (xbc, state_S, o), ld)
     if ws is None:
         check(lib.lia_ssd_scan(*first, M, *shape, _p(o), _stream()), "lia_ssd_scan")
         count_launches()
@@ -1301,7 +1301,7 @@ def ssd_scan(xbc, gates, D, state_S, segs, H, G, N, vdim, o, portions=None):
         if portions is None:
             check(lib.lia_ssd_scan_chunks(*first, M, *shape, _p(o), _p(ws), ws.numel(), chunks, _stream()), "lia_ssd_scan_chunks")
         else:
-            check(lib.lia_ssd_scan_long(*first, longs, long_rows, longest, *shape, _p(o), _p(ws), ws.numel(), chunks, _stream()), "lia_ssd_scan_long")
+            check(lib.lia_ssd_scan_long(*first, longs, long_rows, longest, others, *shape, _p(o), _p(ws), ws.numel(), chunks, _stream()), "lia_ssd_scan_long")
         count_launches(4 * -(-longest // (128 * chunks)))
     return o
 
@@ -1310,18 +1310,19 @@ SSD_WORKSPACE = 256 << 20                                     # bytes for the st
 
 
 def _ssd_chunks(lib, M, nseg, shape, portions, tensors, ld):
-    """The portions that go in chunks (csrc/ssd_chunk_sm100.cu) -- how many, their tokens together, the longest one's; unknown: what there can be --, how many chunks of each to
-    take at a time, and the workspace (None: all go token by token).  The result does not depend on the number, so that less is taken where memory is short."""
-    line, none = lib.lia_ssd_chunk_rows(), (0, 0, 0, 0, None)
+    """The portions that go in chunks (csrc/ssd_chunk_sm100.cu) -- how many, their tokens together, the longest one's, the longest one's of the others; unknown: what there can be --, how many
+    chunks of each to take at a time, and the workspace (None: all go token by token).  The result does not depend on the number, so that less is taken where memory is short."""
+    line, none = lib.lia_ssd_chunk_rows(), (0, 0, 0, 0, 0, None)
     if portions is not None:
         lens = [n for _, _, _, n in portions if n >= line]
         if not lens:
             return none
         longs, long_rows, longest = len(lens), sum(lens), max(lens)
+        others = max((n for _, _, _, n in portions if n < line), default=0)
     elif M < line:
         return none
     else:
-        longs, long_rows, longest = nseg, M, M
+        longs, long_rows, longest, others = nseg, M, M, line - 1
     size = lambda chunks: lib.lia_ssd_workspace(long_rows, longs, *shape, chunks)  # noqa: E731
     if ld % 4 or any(t.data_ptr() % 16 for t in tensors) or not size(1):
         return none
@@ -1330,7 +1331,7 @@ def _ssd_chunks(lib, M, nseg, shape, portions, tensors, ld):
         chunks -= -(-chunks // 8)
     while True:
         try:
-            return longs, long_rows, longest, chunks, torch.empty(size(chunks), dtype=torch.uint8, device=tensors[0].device)
+            return longs, long_rows, longest, others, chunks, torch.empty(size(chunks), dtype=torch.uint8, device=tensors[0].device)
         except torch.OutOfMemoryError:
             if chunks == 1:
                 return none

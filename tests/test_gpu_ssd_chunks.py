@@ -201,8 +201,8 @@ def test_the_skip_term_is_of_x_as_it_is():
     assert torch.equal(o, (step.D[:, None] * step.xbc[:, :step.inner].view(300, 2, 64)).reshape(300, -1))
 
 
-@pytest.mark.parametrize("lens,H,known,unknown", [([128] * 16, 8, 1, 4), ([100] * 4, 8, 1, 4), ([1] * 300, 8, 1, 4), ([2048] + [1] * 63, 64, 4, 4), ([300] + [1] * 256, 64, 4, 4),
-                                                  ([300, 1, 600] + [7] * 40, 4, 4, 4)])
+@pytest.mark.parametrize("lens,H,known,unknown", [([128] * 16, 8, 1, 4), ([100] * 4, 8, 1, 4), ([1] * 300, 8, 1, 4), ([2048] + [1] * 63, 64, 4, 4), ([500] + [1] * 256, 64, 4, 4),
+                                                  ([500, 1, 600] + [7] * 40, 4, 4, 4)])
 def test_passes_by_the_portions(lens, H, known, unknown):
     """The form is chosen from the portions and the passes from the long ones among them: single tokens beside a prompt add neither passes nor workspace."""
     step = Step(lens, H, 2, 64)
