@@ -41,8 +41,10 @@ namespace {
 
 constexpr int L = 128, N = 128, P = 64;        // tokens of a chunk, rows of the state, columns of a unit (a head, or 64 columns of one)
 constexpr int MAX_UNITS = 8;                   // per CTA
-// Portions of fewer tokens go token by token: 64 heads, one portion of 128: 20 us there and 39 here, 256: 37 and 41, 512: 70 and 48, 2048: 267 and 131; 32 heads, 300: 42 and 37.
-constexpr int SHORT = 256;
+// Portions of fewer tokens go token by token.  One portion of 256 | 384 | 448 | 512 | 2048 tokens, 64 heads: 37 | 54 | 62 | 70 | 269 us there and 47 | 55 | 55 | 57 | 152 here; 16 heads: 37 | 54 |
+// 62 | 70 | 266 and 42 | 43 | 45 | 47 | 65; 64 heads beside 32 single tokens: 56 | 82 | 95 | 108 and 78 | 90 | 92 | 95.  (Where the chunks of several portions are little more than the SMs a longer one
+// can still lose: four of 640, 32 heads, 134 and 159.)
+constexpr int SHORT = 448;
 constexpr int TILE = 2 * L * 128;              // one part of B or C: two slabs of 64 rows of the state, 128 bytes a token
 constexpr int UNIT = L * 128;                  // one part of a unit's x, or of half its state
 constexpr float BIG = 1073741824.f, BIG_STATE = 1.2e30f;           // 2^30, 2^100
@@ -966,7 +968,7 @@ extern "C" int lia_ssd_chunk_rows() { return SHORT; }
 
 /* Bytes of workspace for taking `chunks` chunks of every portion at a time (see lia_b200.h); 0: the step goes token by token */
 extern "C" long long lia_ssd_workspace(int rows, int nseg, int H, int G, int Ns, int vdim, int chunks) {
-  if (Ns != N || vdim <= 0 || vdim % P || nseg <= 0 || nseg > 65535 || H <= 0 || G <= 0 || H % G || chunks <= 0 || rows - nseg + 1 < SHORT) return 0;
+  if (Ns != N || vdim <= 0 || vdim % P || nseg <= 0 || nseg > 65535 || H <= 0 || G <= 0 || H % G || chunks <= 0 || rows - nseg + 1 < 2 * L) return 0;
   const long long U = (long long)H * (vdim / P);
   if (U > 8191) return 0;
   const int longs = longs_of(rows, nseg);

@@ -62,7 +62,8 @@ def _chunked(step):
 
 
 @pytest.mark.parametrize("lens,H,G,vdim,rate,pad", [([256], 2, 1, 64, 1.0, 0), ([257, 40, 300], 4, 4, 64, 1.0, 4), ([511, 1], 18, 2, 64, 1.0, 0), ([512], 4, 2, 128, 0.02, 8),
-                                                   ([385, 255, 640], 3, 1, 64, 20.0, 0), ([900], 8, 8, 192, 0.3, 0)])
+                                                   ([385, 255, 640], 3, 1, 64, 20.0, 0), ([900], 8, 8, 192, 0.3, 0),
+                                                   ([448], 2, 1, 64, 1.0, 0), ([449, 40, 500], 4, 4, 64, 1.0, 4), ([447, 513], 18, 2, 64, 1.0, 0)])
 def test_against_the_token_loop(lens, H, G, vdim, rate, pad):
     """Either kernel's numbers are fp32 sums of the same products in another order: this one's error is at most the other's, up to a rounding of 2^-25."""
     step = Step(lens, H, G, vdim, rate, pad)
@@ -80,7 +81,7 @@ def test_a_workspace_for_some_of_the_chunks_changes_no_bit(monkeypatch):
         assert all(torch.equal(a, b) for a, b in zip(whole, step.run()))
 
 
-@pytest.mark.parametrize("lens,H", [([700, 200, 129, 255, 1], 4), ([300] + [200] * 15, 128)])
+@pytest.mark.parametrize("lens,H", [([700, 200, 129, 255, 447, 1], 4), ([500] + [200] * 15, 128)])
 def test_short_portions_beside_some_of_the_chunks(lens, H, monkeypatch):
     """Portions that go token by token are done whole, however few chunks of the others are taken at a time."""
     step = Step(lens, H, 2, 64)
@@ -89,13 +90,13 @@ def test_short_portions_beside_some_of_the_chunks(lens, H, monkeypatch):
         monkeypatch.setattr(ops, "SSD_WORKSPACE", size)
         o, S = step.run()
         for slot, _, row, n in step.segs:
-            if n < 256:
+            if n < 448:
                 assert torch.equal(o[row:row + n], old[0][row:row + n]) and torch.equal(S[slot], old[1][slot]), n
 
 
 def test_an_empty_portion_takes_no_token_from_the_others(monkeypatch):
-    step = Step([0, 385, 0], 4, 2, 64)
-    whole = Step([385], 4, 2, 64)
+    step = Step([0, 513, 0], 4, 2, 64)
+    whole = Step([513], 4, 2, 64)
     whole.xbc, whole.gates, whole.D, whole.S0, whole.segs = step.xbc, step.gates, step.D, step.S0, step.segs[1:2]
     want = whole.run()
     for size in (ops.SSD_WORKSPACE, 1):
@@ -121,24 +122,26 @@ def test_heads_go_token_by_token_for_some_of_the_chunks(at, monkeypatch):
     assert _rel(o.view(-1, H, vdim)[first:, 2], want[0].view(-1, H, vdim)[first:, 2]) <= 2.0 ** -20 and _rel(S[:, 2], want[1][:, 2]) <= 2.0 ** -20
 
 
-def test_a_portion_does_not_depend_on_its_company():
-    step = Step([300, 1, 256, 255, 700], 8, 2, 64)
+@pytest.mark.parametrize("lens", [[300, 1, 256, 255, 700], [500, 1, 448, 447, 700]])
+def test_a_portion_does_not_depend_on_its_company(lens):
+    step = Step(lens, 8, 2, 64)
     o, S = step.run()
     for slot, p0, row, n in step.segs:
         alone, state = step.run(segs=[(slot, p0, row, n)])
         assert torch.equal(alone[row:row + n], o[row:row + n]) and torch.equal(state[slot], S[slot])
     short = step.run(by_tokens=True)
     for slot, _, row, n in step.segs:
-        if n < 256:
+        if n < 448:
             assert torch.equal(o[row:row + n], short[0][row:row + n]) and torch.equal(S[slot], short[1][slot])
 
 
 @pytest.mark.parametrize("what,value", [("x", float("nan")), ("x", float("inf")), ("x", 3e38), ("B", float("-inf")), ("C", float("nan")), ("C", 1e30), ("dt", float("inf")), ("g", float("nan")),
                                         ("g", 1.5), ("S", float("inf")), ("S", 1e35)])
 @pytest.mark.parametrize("at", [0, 131, 299])
-def test_values_out_of_range_go_token_by_token(what, value, at):
+@pytest.mark.parametrize("tokens", [300, 460])
+def test_values_out_of_range_go_token_by_token(what, value, at, tokens):
     H, G, vdim = 4, 2, 64
-    step = Step([300], H, G, vdim)
+    step = Step([tokens], H, G, vdim)
     clean = step.run()
     if what in ("x", "B", "C"):
         col = {"x": 2 * vdim + 5, "B": step.inner + N + 9, "C": step.inner + G * N + N + 9}[what]
@@ -165,7 +168,7 @@ def test_small_numbers_beside_large_ones(what, size, at):
     """Tokens before and after a large number, and the state, are no further from 64 bits than the token loop's, up to one more rounding of 2^-24; and each number by
     itself is off by no more than 2^-20 of the sum of its terms' magnitudes (at most a dozen roundings and cut sums of 2^-24 lie between the inputs and a term)."""
     H, G, vdim = 2, 1, 64
-    step = Step([300], H, G, vdim, seed=int(size) + at)
+    step = Step([450], H, G, vdim, seed=int(size) + at)
     x, B, C = step.xbc[:, :step.inner], step.xbc[:, step.inner:step.inner + N], step.xbc[:, step.inner + N:]
     if what in ("x", "x and dt"):
         x[at] *= size
@@ -193,12 +196,12 @@ def test_small_numbers_beside_large_ones(what, size, at):
 
 def test_the_skip_term_is_of_x_as_it_is():
     """Without a state the outputs are D x and C B x dt: where that vanishes, D x rounded once."""
-    step = Step([300], 2, 1, 64)
+    step = Step([450], 2, 1, 64)
     step.gates[:, :2] = 0.0
     step.S0.zero_()
     step.xbc[131, :step.inner] *= 3e4
     o, _ = step.run()
-    assert torch.equal(o, (step.D[:, None] * step.xbc[:, :step.inner].view(300, 2, 64)).reshape(300, -1))
+    assert torch.equal(o, (step.D[:, None] * step.xbc[:, :step.inner].view(450, 2, 64)).reshape(450, -1))
 
 
 @pytest.mark.parametrize("lens,H,known,unknown", [([128] * 16, 8, 1, 4), ([100] * 4, 8, 1, 4), ([1] * 300, 8, 1, 4), ([2048] + [1] * 63, 64, 4, 4), ([500] + [1] * 256, 64, 4, 4),
@@ -223,5 +226,5 @@ def test_passes_by_the_portions(lens, H, known, unknown):
 
 
 def test_rows_that_are_not_whole_vectors_and_other_shapes_go_token_by_token():
-    for step in (Step([300], 2, 1, 64, pad=1), Step([300], 2, 1, 40), Step([255, 200], 2, 1, 64)):
+    for step in (Step([300], 2, 1, 64, pad=1), Step([300], 2, 1, 40), Step([255, 200], 2, 1, 64), Step([500], 2, 1, 64, pad=1), Step([500], 2, 1, 40), Step([447, 200], 2, 1, 64)):
         assert all(torch.equal(a, b) for a, b in zip(step.run(), step.run(by_tokens=True)))
