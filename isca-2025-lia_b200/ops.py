@@ -1280,9 +1280,10 @@ def conv_act(y, col0, wconv, out, batch, state=None, in_bias=None, bias=None, ac
     return out
 
 
-def ssd_scan(xbc, gates, D, state_S, segs, H, G, N, vdim, o, portions=None):
+def ssd_scan(xbc, gates, D, state_S, segs, H, G, N, vdim, o, portions=None, lengths=None):
     """State-space dual recurrence S = g S + dt B x^T, o = S^T C + D x over every portion of the step (csrc/linear_scan.cu; long portions csrc/ssd_chunk_sm100.cu).
-    ``xbc`` fp32 [M, H vdim + 2 G N] = x | B | C; gates [M, 2H] = dt | g; state_S [slots, H, vdim, N].  ``portions``: the numbers of ``segs`` on the host, if known."""
+    ``xbc`` fp32 [M, H vdim + 2 G N] = x | B | C; gates [M, 2H] = dt | g; state_S [slots, H, vdim, N].  ``portions``: the numbers of ``segs`` on the host, if known;
+    ``lengths``: tokens of the shortest and of the longest of them."""
     ld = _rowmajor(xbc, "xbc")
     M, inner = xbc.shape[0], H * vdim
     for t, n in ((gates, "gates"), (D, "D"), (state_S, "state_S"), (o, "o")):
@@ -1293,7 +1294,7 @@ def ssd_scan(xbc, gates, D, state_S, segs, H, G, N, vdim, o, portions=None):
         raise _lib.LiaError("ssd_scan: shapes do not agree")
     lib, nseg = _lib.load(), segs.shape[0]
     first, shape = (_p(xbc[:, inner:]), _p(xbc[:, inner + G * N:]), _p(xbc), ld, _p(gates), _p(D), _p(state_S), _p(segs), nseg), (H, G, N, vdim)
-    longs, long_rows, longest, others, chunks, ws = _ssd_chunks(lib, M, nseg, shape, portions, (xbc, state_S, o), ld)
+    longs, long_rows, longest, others, chunks, ws = _ssd_chunks(lib, M, nseg, shape, portions, lengths, (xbc, state_S, o), ld)
     if ws is None:
         check(lib.lia_ssd_scan(*first, M, *shape, _p(o), _stream()), "lia_ssd_scan")
         count_launches()
@@ -1309,10 +1310,12 @@ def ssd_scan(xbc, gates, D, state_S, segs, H, G, N, vdim, o, portions=None):
 SSD_WORKSPACE = 256 << 20                                     # bytes for the states between chunks; longer steps take some chunks of every portion at a time
 
 
-def _ssd_chunks(lib, M, nseg, shape, portions, tensors, ld):
+def _ssd_chunks(lib, M, nseg, shape, portions, lengths, tensors, ld):
     """The portions that go in chunks (csrc/ssd_chunk_sm100.cu) -- how many, their tokens together, the longest one's, the longest one's of the others; unknown: what there can be --, how many
     chunks of each to take at a time, and the workspace (None: all go token by token).  The result does not depend on the number, so that less is taken where memory is short."""
     line, none = lib.lia_ssd_chunk_rows(), (0, 0, 0, 0, 0, None)
+    if lengths is not None and lengths[1] < line:
+        return none
     if portions is not None:
         lens = [n for _, _, _, n in portions if n >= line]
         if not lens:

@@ -736,7 +736,7 @@ class StateSpaceMixer:
         ops.conv_act(y, self.proj.offsets[1], self.w_conv, xbc, batch, state=conv, bias=self.conv_bias, act=ops.ACT_SILU, dt_col=self.proj.offsets[2],
                      dt_bias=self.dt_bias, a_log=self.a_log, gates=gates)
         o = torch.empty(M, self.inner, dtype=F32, device=dev)
-        ops.ssd_scan(xbc, gates, self.D, S, batch.segs, self.H, self.G, self.N, self.vdim, o, portions=batch.portions)
+        ops.ssd_scan(xbc, gates, self.D, S, batch.segs, self.H, self.G, self.N, self.vdim, o, portions=batch.portions, lengths=batch.lengths)
         on = torch.empty(M, self.inner, dtype=self.dtype, device=dev)
         ops.silu_gate_norm(o, self.proj.part(y, 0), self.norm_w, on, self.norm_groups, self.eps)
         return self.out(on)

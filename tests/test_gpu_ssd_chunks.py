@@ -211,7 +211,7 @@ def test_passes_by_the_portions(lens, H, known, unknown):
     step = Step(lens, H, 2, 64)
     S, o, d = step.S0.clone(), torch.empty(step.xbc.shape[0], step.inner, device="cuda"), torch.tensor(step.segs, dtype=torch.int32, device="cuda")
     before = _lib.launch_count
-    ops.ssd_scan(step.xbc, step.gates, step.D, S, d, H, 2, N, 64, o, portions=step.segs)
+    ops.ssd_scan(step.xbc, step.gates, step.D, S, d, H, 2, N, 64, o, portions=step.segs, lengths=(min(lens), max(lens)))
     mid = _lib.launch_count
     other = step.run()
     assert mid - before == known and _lib.launch_count - mid <= unknown
