@@ -32,3 +32,14 @@ def test_silu_where_the_exponential_overflows_and_of_numbers_that_are_not_finite
     want = z / (1.0 + torch.exp(-z))
     assert torch.equal(torch.isnan(out[0]), torch.isnan(want))
     assert torch.allclose(out[0].nan_to_num(nan=1.0), want.nan_to_num(nan=1.0), rtol=2.0 ** -21, atol=1e-42)
+
+
+@pytest.mark.parametrize("size", [1e-28, 1e-33, 1e-36, 1e-38, 1e-41])
+def test_silu_of_the_smallest_numbers(size):
+    """Where 1 + exp(-z) is 2 the quotient is half of z, rounded once, subnormal numbers too."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    ff = 512
+    z = torch.randn(40, ff, generator=g, device="cuda").double().mul(size).float()
+    out = torch.empty(40, ff, device="cuda")
+    ops.gated_act(torch.cat([z, torch.ones_like(z)], 1).contiguous(), ff, out, ops.ACT_SILU, up_off=ff)
+    assert torch.equal(out, (z.double() / 2).float())
