@@ -172,31 +172,48 @@ template <int NT, int MT, int CB, int OUT> int launch_rows_as(const RowsArgs& p,
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
+// Few rows a block, and all of a warp's share of K at once, as long as every block has an SM; then more rows, two blocks an SM, and more columns, which read the rows less often.  No form
+// changes a number.  Gates of 16 x 2048, 8 | 200 | 2048 | 4096 rows: blocks of 8 rows 4.0 | 4.4 | 8.8 us, of 16 4.7 | 5.4 | 5.7 | 8.1 (with less at a time), of 32 7.5 | 8.3 | 8.8 | 8.9;
+// 1024 x 2816 in bf16, 16 | 32 | 128 rows: 3.1 | 5.2, 3.1 | 3.5 | 9.5, 5.9 | 5.9 | 7.8; 2048 x 2048, 128 rows, 16 columns a block 11.5, 32 9.0.  Blocks of 24 rows where no more of them are needed:
+// 2048 x 5632, 48 rows 14.1 -> 11.8, 1024 x 8192, 40 rows 13.8 -> 12.2.
 template <int OUT> int launch_rows(const RowsArgs& p, int batch, cudaStream_t stream) {
-  const int sms = lia_sm_count();
-  const long long narrow = (long long)((p.N + 15) / 16) * batch;
-  constexpr bool fp32 = OUT != OUT_GEMM;                       // twice the sums' registers
-  if (p.M <= 16) {                                                 // all of a warp's share of K at once, as long as its registers leave every block an SM
-    const bool deep = p.K > 8 * 32 * WARPS && narrow <= sms;
-    if (p.M <= 8) return deep ? launch_rows_as<1, 1, 12, OUT>(p, batch, stream) : launch_rows_as<1, 1, fp32 ? 6 : 8, OUT>(p, batch, stream);
-    return deep ? launch_rows_as<2, 1, 12, OUT>(p, batch, stream) : launch_rows_as<2, 1, 4, OUT>(p, batch, stream);
+  const long long sms = lia_sm_count(), narrow = (long long)((p.N + 15) / 16) * batch, by8 = narrow * ((p.M + 7) / 8), by16 = narrow * ((p.M + 15) / 16), by32 = narrow * ((p.M + 31) / 32);
+  constexpr bool fp32 = OUT != OUT_GEMM;                           // twice the sums' registers
+  constexpr int SOME = fp32 ? 6 : 8;
+  const bool deep = p.K > SOME * 32 * WARPS;
+  if (by8 <= sms) return deep ? launch_rows_as<1, 1, 12, OUT>(p, batch, stream) : launch_rows_as<1, 1, SOME, OUT>(p, batch, stream);
+  if (p.M <= 8) return launch_rows_as<1, 1, SOME, OUT>(p, batch, stream);
+  if (by16 <= sms) {
+    if constexpr (!fp32)
+      if (deep) return launch_rows_as<2, 1, 12, OUT>(p, batch, stream);
+    return launch_rows_as<2, 1, 8, OUT>(p, batch, stream);
   }
-  // few columns a block and much in flight while the blocks have an SM each, then two blocks an SM, then more columns a block, which read the rows less often: 2048 x 2048, 32 rows: 5.3 | 6.6 |
-  // 8.8 us, 64: 9.7 | 6.6 | 8.6, 128: 18.4 | 12.0 | 9.2
-  const long long blocks = narrow * ((p.M + 31) / 32);
-  if (blocks <= sms) return launch_rows_as<4, 1, 6, OUT>(p, batch, stream);
-  if constexpr (fp32) return launch_rows_as<4, 1, 2, OUT>(p, batch, stream);
-  else if (blocks <= 2 * sms) return launch_rows_as<4, 1, 3, OUT>(p, batch, stream);
-  else return launch_rows_as<4, 2, 2, OUT>(p, batch, stream);
+  if (p.M <= 16) return launch_rows_as<2, 1, 4, OUT>(p, batch, stream);
+  if constexpr (fp32) {
+    if (by16 <= 2 * sms) return launch_rows_as<2, 1, 4, OUT>(p, batch, stream);
+    return launch_rows_as<4, 1, 2, OUT>(p, batch, stream);
+  } else {
+    const bool by24 = (p.M + 23) / 24 == (p.M + 31) / 32;
+    if (by32 <= sms) return by24 ? launch_rows_as<3, 1, 6, OUT>(p, batch, stream) : launch_rows_as<4, 1, 6, OUT>(p, batch, stream);
+    if (by32 <= 2 * sms) return by24 ? launch_rows_as<3, 1, 4, OUT>(p, batch, stream) : launch_rows_as<4, 1, 3, OUT>(p, batch, stream);
+    return by24 ? launch_rows_as<3, 2, 2, OUT>(p, batch, stream) : launch_rows_as<4, 2, 2, OUT>(p, batch, stream);
+  }
 }
 
 }  // namespace
 
-// Weights up to 24 MB in up to 4096 rows; the line looks at the weights alone, for the other side's sums are other ones.  In a chain of projections over 300 MB of weights, 1 | 16 | 64 | 128 rows:
-// 1024 x 1024 5.7 | 5.9 | 7.8 | 10.6 us on the other side and 1.8 | 2.2 | 3.0 | 4.1 here, 2048 x 5632 8.3 | 9.0 | 14.4 | 26 and 5.8 | 7.7 | 14.3 | 21.5; beyond: 6144 x 2048 8.7 | 9.0 | 11.9 | 17
-// and 6.4 | 10.2 | 17 | 25, 5632 x 1024 5.8 | 6.1 | 8.2 | 11.9 and 4.3 | 5.4 | 9.2 | 14.
+// The line looks at the weights alone, for the other side's sums are other ones: where no number of rows up to 128 is the slower one here.  In a chain of projections over 300 MB of weights,
+// 1 | 16 | 32 | 48 | 64 | 128 rows: 1024 x 1024 5.7 | 5.9 | 6.6 | 7.6 | 7.8 | 10.9 us on the other side and 1.7 | 2.1 | 2.1 | 2.6 | 3.0 | 4.0 here, 1024 x 8192 9.2 | 10.0 | 11.8 | 14.2 | 15.2 |
+// 26.7 and 7.0 | 7.5 | 9.4 | 12.5 | 14.7 | 18.3, 2048 x 5632 8.3 | 9.0 | 11.0 | 13.4 | 14.4 | 25.8 and 5.7 | 7.7 | 11.2 | 11.8 | 14.4 | 21.2, 4096 x 2048 7.7 | 8.1 | 9.3 | 10.6 | 11.4 | 18.7 and
+// 3.6 | 5.4 | 6.6 | 7.8 | 9.3 | 16.8; beyond: 512 x 16384 10.7 | 11.9 and 13.2 | 17.5, 3072 x 4096 8.2 | 8.5 | 11.2 | 13.1 | 14.3 and 5.3 | 8.9 | 11.7 | 13.5 | 16.8, 4096 x 3072, 96 rows, 18.7 and
+// 22.7, and, with 32 rows in blocks of 32, 1024 x 8192 11.8 and 15.0 (so that deep ones are taken where those of 16 have an SM each: 1184 columns).
 // (lia_gemm_bf16 is not among its callers: OPT's operations one by one give the bits of the program that chains them in one launch, decode_program_sm100.cu, with the GEMM's sums.)
-bool gemm_rows_takes(int M, int N, int K) { return M > 0 && N > 0 && K > 0 && M <= 128 && N <= 4096 && (long long)N * K <= 12 << 20; }
+bool gemm_rows_takes(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || K <= 0 || M > 128) return false;
+  if (N <= 1184) return K <= 8192;
+  if (N <= 2368) return K <= 5632 && (long long)N * K <= 11 << 20;
+  return N <= 4096 && (long long)N * K <= 8 << 20;
+}
 
 int gemm_rows(const void* A, const void* W, void* C, int M, int N, int K, cudaStream_t stream) {
   const RowsArgs p{reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(W), C, K, 0, K, 0, N, 0, M, N, K, 1.f, nullptr, 0, 0.f, 1};

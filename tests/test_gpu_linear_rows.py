@@ -24,6 +24,29 @@ def test_projections(M, N, K):
     assert torch.equal(ops.linear(a[:1], w), out[:1])
 
 
+@pytest.mark.parametrize("N,K", [(2048, 520), (1184, 1032), (2368, 264), (2376, 264), (4096, 136), (64, 8192), (1184, 8192), (2048, 5632), (2560, 3272)])
+def test_a_row_does_not_depend_on_how_many_there_are(N, K):
+    """Blocks of 8, 16, 24 and 32 rows and of 16 and 32 columns give the same bits, at the edges of the weights that are taken and of the SMs."""
+    a, w = _rand(128, K), _rand(N, K, std=K ** -0.5)
+    whole = ops.linear(a, w)
+    y = (a.double() @ w.double().T).to(BF16).double()
+    assert float((whole.double() - y).abs().max()) <= 0.0325 and float((whole.double() != y).double().mean()) < 2e-3
+    for M in (1, 7, 8, 9, 15, 16, 17, 24, 25, 33, 40, 48, 49, 64, 65, 72, 73, 96, 97, 127):
+        assert torch.equal(ops.linear(a[:M], w), whole[:M]), M
+
+
+@pytest.mark.parametrize("N,K", [(8, 1024), (16, 2056), (34, 136), (128, 520)])
+def test_a_row_of_gates_does_not_depend_on_how_many_there_are(N, K):
+    a, w = _rand(5000, K), _rand(N, K, std=K ** -0.5)
+    whole = torch.empty(5000, N, device="cuda")
+    ops.linear_small(a, w, None, whole)
+    assert float((whole.double() - a.double() @ w.double().T).abs().max()) < 3e-6
+    for M in (1, 8, 9, 16, 17, 148, 149, 300, 1184, 1185, 2368, 2369, 4736, 4737):
+        out = torch.empty(M, N, device="cuda")
+        ops.linear_small(a[:M], w, None, out)
+        assert torch.equal(out, whole[:M]), M
+
+
 @pytest.mark.parametrize("M,N,K,batch", [(1, 5, 8, 3), (7, 16, 136, 2), (16, 33, 2088, 1), (40, 130, 512, 4), (64, 4800, 96, 1), (33, 2400, 128, 1)])
 @pytest.mark.parametrize("dtype", [F32, BF16])
 def test_plain(M, N, K, batch, dtype):
