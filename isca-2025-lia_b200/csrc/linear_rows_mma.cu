@@ -4,7 +4,7 @@
 // A step of decoded tokens is a chain of small projections, and what the tcgen05 GEMM takes for one is latency: tensor maps, barriers, TMEM, a ring that fills, partial sums that change
 // hands.  Here the weights go straight from global memory into the operands' registers: 16 bytes of a weight row are two operands' worth of k, and as the rows of A are read the same
 // way the order of the k within 32 does not matter.  Where the caller says that no work in flight on the stream writes them (`resident`: a model's weights) they are asked for before the
-// previous kernel has ended.  A block makes 16 or 32 columns of 8 to 32 rows, its 8 warps an eighth of K
+// previous kernel has ended.  (Non-coherent loads; by ld.global.cg an engine session of four requests takes 3335 us in place of 3220.)  A block makes 16 or 32 columns of 8 to 32 rows, its 8 warps an eighth of K
 // each; they meet once, in shared memory.
 //
 // The tensor cores cut sums off below the 24th bit: those over 32 k are made apart and added in fp32.  Where the result is fp32 those over 16 are, what a warp's sum rounds off is added up apart
@@ -37,12 +37,6 @@ struct RowsArgs {
 
 enum { OUT_GEMM, OUT_FP32, OUT_ROUNDED, OUT_GATES };              // GEMM: bf16, whole vectors, nothing kept of what the sums round off
 
-__device__ __forceinline__ uint4 ldg_once(const bf16* p) {                        // by way of L2 alone: a weight may be what the previous kernel wrote
-  uint4 r;
-  asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
-  return r;
-}
-
 // A block: 8 NT rows times 16 MT columns.  CB: blocks of 32 k in registers at a time
 template <int NT, int MT, int CB> struct Form {
   static constexpr int ROWS = 8 * NT, COLS = 16 * MT, PITCH = COLS + 4, SMEM = WARPS * ROWS * PITCH * 4;
@@ -65,7 +59,7 @@ __global__ void __launch_bounds__(WARPS * 32, Form<NT, MT, CB>::REGS + (OUT == O
       const int k = (b0 + b) * 32;
       const bool live = b0 + b < last && k + t * 8 < p.K;
 #pragma unroll
-      for (int i = 0; i < 2 * MT; ++i) w[b][i >> 1][i & 1] = live ? ldg_once(W + (size_t)min(n0 + g + 8 * i, p.N - 1) * p.ldw + k) : make_uint4(0, 0, 0, 0);
+      for (int i = 0; i < 2 * MT; ++i) w[b][i >> 1][i & 1] = live ? ldg_stream(W + (size_t)min(n0 + g + 8 * i, p.N - 1) * p.ldw + k) : make_uint4(0, 0, 0, 0);
     }
   };
   if (!p.resident) pdl_wait();
