@@ -79,3 +79,20 @@ def test_linear_small(M, N, K, a_dt, w_dt):
     out = torch.empty(M, N, device=DEV)
     ops.linear_small(a.to(DEV), w.to(DEV), b.to(DEV), out, ops.GATE_SIGMOID)
     assert float((out.cpu().to(F64) - torch.sigmoid(a.to(F64) @ w.to(F64).T + b.to(F64))).abs().max()) < 2e-5
+
+
+@pytest.mark.parametrize("F,groups", [(64, 1), (128, 1), (132, 1), (512, 1), (1536, 3), (2000, 5)])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_a_row_of_a_gated_norm_does_not_depend_on_how_many_there_are(F, groups, dt):
+    g = torch.Generator(device=DEV).manual_seed(F)
+    M = 2200
+    o, z, w = torch.randn(M, F, generator=g, device=DEV), torch.randn(M, F, generator=g, device=DEV).to(dt), torch.randn(F, generator=g, device=DEV)
+    whole = torch.empty(M, F, dtype=dt, device=DEV)
+    ops.silu_gate_norm(o, z, w, whole, groups, 1e-6)
+    for m in (1, 7, 2047 // groups, -(-2048 // groups)):
+        out = torch.empty(m, F, dtype=dt, device=DEV)
+        ops.silu_gate_norm(o[:m], z[:m], w, out, groups, 1e-6)
+        assert torch.equal(out, whole[:m]), m
+    u = (o.double() * z.double() * torch.sigmoid(z.double())).view(M, groups, -1)
+    want = (u / torch.sqrt((u * u).mean(-1, keepdim=True) + 1e-6)).view(M, F) * w.double()
+    assert float((whole.double() - want).abs().max() / want.abs().max()) < (2.0 ** -20 if dt == torch.float32 else 2.0 ** -8)
