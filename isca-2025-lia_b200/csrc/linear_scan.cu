@@ -462,17 +462,21 @@ constexpr int CONV_STRIP = 8;
 __device__ __forceinline__ float silu_fast(float z) { return __fdividef(z, 1.0f + expf(-z)); }
 __device__ __forceinline__ float gelu_tanh(float z) { return 0.5f * z * (1.0f + tanhf(0.79788456080286535588f * (z + 0.044715f * z * z * z))); }
 
-// rows r0 .. r1 - 1 of channel c, wherever their portions begin
-template <typename T, int TM>
-__device__ __forceinline__ void conv_channel(const T* __restrict__ y, const float* __restrict__ in_bias, const float* __restrict__ wconv, const float* __restrict__ bias,
-                                             float* __restrict__ state, const int* __restrict__ meta, float* __restrict__ out, const ConvActArgs& a, int c, int r0, int r1) {
+// rows r0 .. r1 - 1 of the channels c .. c + CH - 1, wherever their portions begin
+template <typename T, int TM, int CH>
+__device__ __forceinline__ void conv_channels(const T* __restrict__ y, const float* __restrict__ in_bias, const float* __restrict__ wconv, const float* __restrict__ bias,
+                                              float* __restrict__ state, const int* __restrict__ meta, float* __restrict__ out, const ConvActArgs& a, int c, int r0, int r1) {
   const T* col = y + a.col0 + c;
-  const float ib = in_bias ? in_bias[c] : 0.f, ob = bias ? bias[c] : 0.f;
-  float w[TM], win[TM];                          // by tokens back
+  float ib[CH], ob[CH], w[TM][CH], win[TM][CH];  // by tokens back
 #pragma unroll
-  for (int j = 0; j < TM; ++j) {
-    w[j] = j < a.taps ? wconv[(size_t)c * a.taps + a.taps - 1 - j] : 0.f;
-    win[j] = 0.f;
+  for (int k = 0; k < CH; ++k) {
+    ib[k] = in_bias ? in_bias[c + k] : 0.f;
+    ob[k] = bias ? bias[c + k] : 0.f;
+#pragma unroll
+    for (int j = 0; j < TM; ++j) {
+      w[j][k] = j < a.taps ? wconv[(size_t)(c + k) * a.taps + a.taps - 1 - j] : 0.f;
+      win[j][k] = 0.f;
+    }
   }
   int pslot = -1, ppos = -1;
   for (int r = r0; r < r1; ++r) {
@@ -480,29 +484,38 @@ __device__ __forceinline__ void conv_channel(const T* __restrict__ y, const floa
     float* st = state ? state + (size_t)slot * (a.taps - 1) * a.C + c : nullptr;
     if (r > r0 && slot == pslot && pos == ppos + 1) {
 #pragma unroll
-      for (int j = TM - 1; j > 0; --j) win[j] = win[j - 1];
+      for (int j = TM - 1; j > 0; --j)
+#pragma unroll
+        for (int k = 0; k < CH; ++k) win[j][k] = win[j - 1][k];
     } else {
       int inside = 1;                            // rows r-1 .. r-(inside-1) belong to this portion
       while (inside < a.taps && r - inside >= 0 && meta[2 * (r - inside)] == slot && meta[2 * (r - inside) + 1] == pos - inside) ++inside;
 #pragma unroll
-      for (int j = 1; j < TM; ++j) {
-        win[j] = 0.f;
-        if (j < a.taps && j <= pos)
-          win[j] = j < inside ? ldf(col + (size_t)(r - j) * a.ld) : st[(size_t)(inside - 1 - j + a.taps - 1) * a.C];
-      }
-    }
-    win[0] = ldf(col + (size_t)r * a.ld);
-    float acc = 0.f;
+      for (int j = 1; j < TM; ++j)
 #pragma unroll
-    for (int j = 0; j < TM; ++j)
-      if (j < a.taps && j <= pos) acc = fmaf(w[j], win[j] + ib, acc);
-    acc += ob;
-    if (a.act == LIA_ACT_SILU) acc = silu_fast(acc);
-    out[(size_t)r * a.ldo + c] = acc;
+        for (int k = 0; k < CH; ++k) {
+          win[j][k] = 0.f;
+          if (j < a.taps && j <= pos) win[j][k] = j < inside ? ldf(col + k + (size_t)(r - j) * a.ld) : st[(size_t)(inside - 1 - j + a.taps - 1) * a.C + k];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < CH; ++k) win[0][k] = ldf(col + k + (size_t)r * a.ld);
+#pragma unroll
+    for (int k = 0; k < CH; ++k) {
+      float acc = 0.f;
+#pragma unroll
+      for (int j = 0; j < TM; ++j)
+        if (j < a.taps && j <= pos) acc = fmaf(w[j][k], win[j][k] + ib[k], acc);
+      acc += ob[k];
+      if (a.act == LIA_ACT_SILU) acc = silu_fast(acc);
+      out[(size_t)r * a.ldo + c + k] = acc;
+    }
     if (a.single) {
 #pragma unroll
       for (int j = 0; j < TM - 1; ++j)
-        if (j < a.taps - 1) st[(size_t)(a.taps - 2 - j) * a.C] = win[j];
+#pragma unroll
+        for (int k = 0; k < CH; ++k)
+          if (j < a.taps - 1) st[(size_t)(a.taps - 2 - j) * a.C + k] = win[j][k];
     }
     pslot = slot;
     ppos = pos;
@@ -579,8 +592,7 @@ __global__ void __launch_bounds__(256) conv_act_kernel(const T* __restrict__ y, 
       return;
     }
   }
-#pragma unroll 1
-  for (int k = 0; k < CH; ++k) conv_channel<T, TM>(y, in_bias, wconv, bias, state, meta, out, a, c + k, r0, r1);
+  conv_channels<T, TM, CH>(y, in_bias, wconv, bias, state, meta, out, a, c, r0, r1);
 }
 
 // ---------------------------------------------------------------------------------------------------- state-space duality
@@ -996,8 +1008,9 @@ extern "C" int lia_conv_act(const void* y, int y_f32, int ld, int col0, int C, c
   LIA_CHECK_ARG(H >= 0 && (H == 0 || (dt_bias && a_log && gates && dt_col >= 0 && ld >= dt_col + H)), "lia_conv_act: bad step sizes (H=%d)", H);
   const int single = nseg == M && taps > 1;      // every portion is one row
   ConvActArgs a{ld, col0, C, taps, act, single, ldo, M, M <= 64 ? 1 : CONV_STRIP, dt_col, H};
-  // pairs of channels where strips of rows are made and every row is whole pairs (2048 rows of 6144 channels: 25 us one by one, 22 so)
-  const bool pairs = M > 64 && taps <= 4 && C % 2 == 0 && ld % 2 == 0 && col0 % 2 == 0 && ldo % 2 == 0 && reinterpret_cast<uintptr_t>(y) % (y_f32 ? 8 : 4) == 0 &&
+  // pairs of channels where strips of rows are made, a block's worth of them, and every row is whole pairs (2048 | 300 rows of 6144 channels in bf16: 25.4 | 9.8 us one by one, 22.2 | 9.3 so;
+  // 300 of 96 in 300 portions 8.1 and 8.8)
+  const bool pairs = M > 64 && taps <= 4 && C >= 512 && C % 2 == 0 && ld % 2 == 0 && col0 % 2 == 0 && ldo % 2 == 0 && reinterpret_cast<uintptr_t>(y) % (y_f32 ? 8 : 4) == 0 &&
                      reinterpret_cast<uintptr_t>(out) % 8 == 0;
   dim3 grid(((pairs ? C / 2 : C) + H + 255) / 256, (M + a.strip - 1) / a.strip);
   LIA_CHECK_ARG(grid.y <= 65535, "lia_conv_act: too many rows (%d)", M);

@@ -96,3 +96,27 @@ def test_a_row_of_a_gated_norm_does_not_depend_on_how_many_there_are(F, groups, 
     u = (o.double() * z.double() * torch.sigmoid(z.double())).view(M, groups, -1)
     want = (u / torch.sqrt((u * u).mean(-1, keepdim=True) + 1e-6)).view(M, F) * w.double()
     assert float((whole.double() - want).abs().max() / want.abs().max()) < (2.0 ** -20 if dt == torch.float32 else 2.0 ** -8)
+
+
+@pytest.mark.parametrize("lens", [[65], [72, 1, 7], [300], [2] * 40, [1] * 70 + [9]])
+@pytest.mark.parametrize("taps,act", [(4, ops.ACT_SILU), (3, ops.ACT_NONE), (1, ops.ACT_NONE)])
+@pytest.mark.parametrize("dt", [F32, BF16])
+def test_convolution_by_pairs_of_channels(lens, taps, act, dt):
+    """Two channels a thread and one, chosen by the output's row stride, give the same bits, wherever portions begin."""
+    from lia_b200.seq_layers import StepBatch
+    C, M, n = 512, sum(lens), len(lens)
+    g = torch.Generator(device=DEV).manual_seed(M + taps)
+    r = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    y, w, bias, in_bias, state = r(M, C + 8).to(dt), r(C, taps), r(C), r(C), r(n, max(taps - 1, 1), C)
+    segs, meta, row = [], [], 0
+    for i, k in enumerate(lens):
+        segs.append((i, 2 * (i % 3), row, k))
+        meta += [(i, 2 * (i % 3) + j) for j in range(k)]
+        row += k
+    batch = StepBatch(M, torch.tensor(segs, dtype=torch.int32, device=DEV), torch.tensor(meta, dtype=torch.int32, device=DEV), portions=segs)
+    got = []
+    for ld in (C + 2, C + 1):
+        out, st = torch.zeros(M, ld, device=DEV)[:, :C], state.clone()
+        ops.conv_act(y, 4, w, out, batch, state=st if taps > 1 else None, in_bias=in_bias, bias=bias, act=act)
+        got.append((out.clone(), st))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
