@@ -489,6 +489,7 @@ __global__ void __launch_bounds__(128) silu_gate_norm_kernel(const float* __rest
   const float* orow = o + row * F + first;
   const T* zrow = z + row * ldz + first;
   float ss = 0.f;
+#pragma unroll 4
   for (int i = threadIdx.x * VEC; i < n; i += 128 * VEC) {
     float ov[VEC], zv[VEC];
     ld_vec<VEC>(orow + i, ov);
