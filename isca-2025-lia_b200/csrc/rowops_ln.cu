@@ -692,7 +692,9 @@ extern "C" int lia_gated_act_weighted(const void* in, int ld, int up_off, void* 
   const int sz = act_f32 ? 4 : 2;
   if (F % 4 == 0 && ld % 4 == 0 && (up_off < 0 || up_off % 4 == 0) && reinterpret_cast<uintptr_t>(in) % (4 * sz) == 0 && reinterpret_cast<uintptr_t>(out) % (4 * sz) == 0 &&
       quads < (1ll << 31)) {
-    if (F % 8 == 0) {                          // (whole quads on both sides of an oct)
+    // Octs (whole quads on both sides) where there are many.  Quads and octs, gated in bf16, 300 x 2816 | 2048 x 1408 | 2048 x 6144: SiLU 2.96 | 5.4 | 19.1 us and 2.90 | 4.4 | 14.4, GELU by tanh
+    // 2.85 | 5.5 | 19.4 and 3.25 | 5.0 | 17.0; in fp32 a squared ReLU's cost more, 300 x 6144 | 2048 x 2816 | 2048 x 6144: 3.2 | 7.6 | 25.5 and 4.1 | 8.5 | 21.7.
+    if (F % 8 == 0 && quads >= (act_f32 ? 1 << 21 : 1 << 19)) {
       const unsigned g8 = (unsigned)((quads / 2 + 255) / 256);
       if (act_f32) lia_launch(gated_act_vec8_kernel<float>, dim3(g8), dim3(256), 0, stream, reinterpret_cast<const float*>(in), ld, up_off, reinterpret_cast<float*>(out), (unsigned)(quads / 2), F, act, perm, wt);
       else lia_launch(gated_act_vec8_kernel<bf16>, dim3(g8), dim3(256), 0, stream, reinterpret_cast<const bf16*>(in), ld, up_off, reinterpret_cast<bf16*>(out), (unsigned)(quads / 2), F, act, perm, wt);

@@ -43,3 +43,20 @@ def test_silu_of_the_smallest_numbers(size):
     out = torch.empty(40, ff, device="cuda")
     ops.gated_act(torch.cat([z, torch.ones_like(z)], 1).contiguous(), ff, out, ops.ACT_SILU, up_off=ff)
     assert torch.equal(out, (z.double() / 2).float())
+
+
+@pytest.mark.parametrize("dt,rows", [(torch.bfloat16, 2048), (torch.float32, 8192)])
+@pytest.mark.parametrize("act", [ops.ACT_NONE, ops.ACT_RELU, ops.ACT_SILU, ops.ACT_GELU_ERF, ops.ACT_GELU_TANH, ops.ACT_RELU_SQUARED])
+@pytest.mark.parametrize("up", [True, False])
+def test_many_rows_give_what_few_give(dt, rows, act, up):
+    """Eight columns a thread from ``rows`` rows of 1024 on, four below: the same bits, routing weights among the factors too."""
+    g = torch.Generator(device="cuda").manual_seed(act)
+    ff = 1024
+    x = torch.randn(rows + 2, 2 * ff, generator=g, device="cuda").to(dt)
+    perm = torch.arange(rows + 2, dtype=torch.int32, device="cuda")
+    perm[5::7] = -1
+    for kw in ({}, dict(perm=perm, wt=torch.rand(rows + 2, generator=g, device="cuda"))):
+        whole, few = torch.empty(rows + 2, ff, device="cuda", dtype=dt), torch.empty(rows - 1, ff, device="cuda", dtype=dt)
+        ops.gated_act(x, ff, whole, act, up_off=ff if up else -1, **kw)
+        ops.gated_act(x[:rows - 1], ff, few, act, up_off=ff if up else -1, **kw)
+        assert torch.equal(whole[:rows - 1], few)
