@@ -36,7 +36,7 @@ def test_ln_add_norm(W, y_dt, h_dt):
             assert float((h.cpu().to(F64) - ln(want, pre)).abs().max()) < (2e-5 if h_dt == F32 else 0.03)
 
 
-@pytest.mark.parametrize("H,vdim", [(3, 4), (2, 128), (1, 512), (1, 516), (2, 1024), (1, 4100), (3, 30)])
+@pytest.mark.parametrize("H,vdim", [(3, 4), (2, 128), (1, 512), (1, 516), (2, 1024), (1, 4100), (3, 30), (2, 132), (1, 256), (2, 260), (1, 1028), (1, 2048), (1, 2052)])
 @pytest.mark.parametrize("dt", [F32, BF16])
 def test_headnorm_gate(H, vdim, dt):
     g = torch.Generator().manual_seed(vdim)
