@@ -52,9 +52,10 @@ struct ConvCols {          // where the q, k, v channels sit in a row of the pro
 
 // Block per token row.  meta[row] = {slot, position}; rows of one portion are consecutive and so are their positions.
 // state [slot][taps-1][C] holds the inputs of the taps - 1 positions before the portion (zero before the sequence's start).
-// TM: at least the taps, whose inputs are asked for together.  Few rows get 1024 threads each (an engine session's 16 steps of 4 rows of 2048 channels and a prompt: 201 us with 256 and one input after the other, 106 so).
+// TM: 0, and 256 threads, or at least the taps, whose inputs are asked for together by 1024 threads: for few rows, of more channels than 256 (1 | 33 rows of 4096 in bf16: 12.5 | 13.4 us and
+// 6.3 | 8.1; many rows fill the SMs by themselves: 300 | 2048 16.2 | 57 and 19.6 | 72).
 template <typename T, int TM>
-__global__ void __launch_bounds__(1024) conv_prep_kernel(const T* __restrict__ y, int ld, ConvCols cc, const float* __restrict__ wconv,
+__global__ void __launch_bounds__(TM ? 1024 : 256, TM ? 1 : 6) conv_prep_kernel(const T* __restrict__ y, int ld, ConvCols cc, const float* __restrict__ wconv,
                                                         const float* __restrict__ state, const int* __restrict__ meta, float* __restrict__ gates,
                                                         const float* __restrict__ a_log, const float* __restrict__ dt_bias, float* __restrict__ qk,
                                                         float* __restrict__ v, int G, int H, int dim, int vdim, int taps, float q_scale,
@@ -68,34 +69,43 @@ __global__ void __launch_bounds__(1024) conv_prep_kernel(const T* __restrict__ y
   int inside = 1;                               // rows row-1 .. row-(inside-1) belong to this portion
   while (inside < taps && row - inside >= 0 && meta[2 * (row - inside)] == slot && meta[2 * (row - inside) + 1] == pos - inside) ++inside;
   const float* st = state + (size_t)slot * (taps - 1) * C;
-  for (int c = threadIdx.x; c < C; c += blockDim.x) {
+  constexpr int THREADS = TM ? 1024 : 256;
+  for (int c = threadIdx.x; c < C; c += THREADS) {
     const int col = cc.col(c);
-    float acc = 0.f, xin[TM], w[TM];
-#pragma unroll
-    for (int j = 0; j < TM; ++j) {              // j tokens back
-      xin[j] = w[j] = 0.f;
-      if (j < taps) {
-        xin[j] = j < inside ? ldf(y + (size_t)(row - j) * ld + col) : st[(size_t)(inside - 1 - j + taps - 1) * C + c];
-        w[j] = wconv[(size_t)c * taps + taps - 1 - j];
+    float acc = 0.f;
+    if constexpr (TM == 0) {
+      for (int j = 0; j < taps; ++j) {          // j tokens back
+        const float xin = j < inside ? ldf(y + (size_t)(row - j) * ld + col) : st[(size_t)(inside - 1 - j + taps - 1) * C + c];
+        acc = fmaf(wconv[(size_t)c * taps + taps - 1 - j], xin, acc);
       }
-    }
+    } else {
+      float xin[TM], w[TM];
 #pragma unroll
-    for (int j = 0; j < TM; ++j)
-      if (j < taps) acc = fmaf(w[j], xin[j], acc);
+      for (int j = 0; j < TM; ++j) {
+        xin[j] = w[j] = 0.f;
+        if (j < taps) {
+          xin[j] = j < inside ? ldf(y + (size_t)(row - j) * ld + col) : st[(size_t)(inside - 1 - j + taps - 1) * C + c];
+          w[j] = wconv[(size_t)c * taps + taps - 1 - j];
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < TM; ++j)
+        if (j < taps) acc = fmaf(w[j], xin[j], acc);
+    }
     acc = silu(acc);
     ch[c] = acc;
     if (c >= cc.nq + cc.nk) v[(size_t)row * cc.nv + c - cc.nq - cc.nk] = acc;
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int hd = warp; hd < 2 * G; hd += blockDim.x >> 5) {         // q heads, then k heads
+  for (int hd = warp; hd < 2 * G; hd += THREADS >> 5) {            // q heads, then k heads
     float ss = 0.f;
     for (int i = lane; i < dim; i += 32) ss += ch[hd * dim + i] * ch[hd * dim + i];
     ss = warp_sum(ss);
     const float inv = (hd < G ? q_scale : 1.0f) / sqrtf(ss + unit_eps);
     for (int i = lane; i < dim; i += 32) qk[(size_t)row * (cc.nq + cc.nk) + hd * dim + i] = ch[hd * dim + i] * inv;
   }
-  for (int h = threadIdx.x; h < H; h += blockDim.x) {
+  for (int h = threadIdx.x; h < H; h += THREADS) {
     float* gr = gates + (size_t)row * 2 * H;
     const float zb = gr[h], za = gr[H + h] + dt_bias[h];
     const float softplus = fmaxf(za, 0.f) + log1pf(expf(-fabsf(za)));
@@ -926,15 +936,17 @@ extern "C" int lia_conv_prep(const void* y, int y_f32, int ld, int q_off, int k_
   ConvCols cc{q_off, k_off, v_off, G * dim, G * dim, H * vdim};
   const size_t smem = (size_t)(cc.nq + cc.nk + cc.nv) * sizeof(float);
   LIA_CHECK_ARG(smem <= 160 * 1024, "lia_conv_prep: %d channels do not fit shared memory", cc.nq + cc.nk + cc.nv);
-  const int threads = M <= 64 ? 1024 : 256;
+  const bool few = M <= 64 && cc.nq + cc.nk + cc.nv > 256;
 #define LIA_CP(T, TM)                                                                                                                                                    \
   do {                                                                                                                                                                   \
     if (smem > 48 * 1024) LIA_CUDA(cudaFuncSetAttribute(conv_prep_kernel<T, TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));                               \
-    lia_launch(conv_prep_kernel<T, TM>, dim3(M), dim3(threads), smem, stream, reinterpret_cast<const T*>(y), ld, cc, wconv, conv_state, meta, gates, a_log, dt_bias, qk, v, G, H, dim, \
+    lia_launch(conv_prep_kernel<T, TM>, dim3(M), dim3(TM ? 1024 : 256), smem, stream, reinterpret_cast<const T*>(y), ld, cc, wconv, conv_state, meta, gates, a_log, dt_bias, qk, v, G, H, dim, \
                vdim, taps, q_scale, unit_eps);                                                                                                                           \
   } while (0)
-  if (y_f32 && taps <= 4) LIA_CP(float, 4);
+  if (y_f32 && !few) LIA_CP(float, 0);
+  else if (y_f32 && taps <= 4) LIA_CP(float, 4);
   else if (y_f32) LIA_CP(float, MAX_TAPS);
+  else if (!few) LIA_CP(bf16, 0);
   else if (taps <= 4) LIA_CP(bf16, 4);
   else LIA_CP(bf16, MAX_TAPS);
 #undef LIA_CP

@@ -120,3 +120,23 @@ def test_convolution_by_pairs_of_channels(lens, taps, act, dt):
         ops.conv_act(y, 4, w, out, batch, state=st if taps > 1 else None, in_bias=in_bias, bias=bias, act=act)
         got.append((out.clone(), st))
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("G,H,dim,taps", [(1, 1, 32, 4), (2, 4, 64, 4), (2, 4, 64, 7), (1, 2, 128, 1)])
+@pytest.mark.parametrize("dt", [F32, BF16])
+def test_a_row_of_the_delta_rules_convolution_does_not_depend_on_how_many_there_are(G, H, dim, taps, dt):
+    g = torch.Generator(device=DEV).manual_seed(taps + dim)
+    r = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    M, C = 70, (2 * G + H) * dim
+    y, w, state, gates = r(M, C + 8).to(dt), r(C, taps), r(1, max(taps - 1, 1), C), r(M, 2 * H)
+    a_log, dt_bias = r(H), r(H)
+    meta = torch.tensor([(0, 3 + i) for i in range(M)], dtype=torch.int32, device=DEV)
+
+    def run(m):
+        ga, qk, v = gates[:m].clone(), torch.empty(m, 2 * G * dim, device=DEV), torch.empty(m, H * dim, device=DEV)
+        ops.conv_prep(y[:m], (0, G * dim, 2 * G * dim), w, state, meta[:m], ga, a_log, dt_bias, qk, v, G, H, dim, dim, taps, 0.25)
+        return qk, v, ga
+
+    whole = run(M)
+    for m in (1, 33, 64, 65):
+        assert all(torch.equal(a, b[:m]) for a, b in zip(run(m), whole)), m
