@@ -280,7 +280,8 @@ int lia_linear_small(const void* a, int a_f32, int lda, const void* w, int w_f32
 /* the same for a `w` that no work in flight on the stream writes (a model's weights): it may be read before the previous kernel has ended */
 int lia_linear_small_resident(const void* a, int a_f32, int lda, const void* w, int w_f32, const float* bias, float* out, int M, int N, int K,
                               int mode, float cap, lia_stream_t stream);
-/* C[b][m][n] = scale * sum_k A[b][m][k] W[b][n][k] on the CUDA cores, fp32 products and sums; element strides */
+/* C[b][m][n] = scale * sum_k A[b][m][k] W[b][n][k], products and sums as exact as fp32's; element strides.  On the tensor cores for bf16 operands of up to 64 rows, and from 65
+ * rows on but for bf16 rows times fp32 weights, where rows and addresses are whole 16 bytes (fp32 numbers in three bf16 parts), on the CUDA cores else */
 int lia_linear_plain(const void* A, int a_f32, long long lda, long long sA, const void* W, int w_f32, long long ldw, long long sW,
                      void* C, int c_f32, long long ldc, long long sC, int M, int N, int K, int batch, float scale, lia_stream_t stream);
 /* the same for a W that no work in flight on the stream writes (a model's weights): it may be read before the previous kernel has ended */

@@ -49,7 +49,7 @@ def _cost(name, a, kw):
         K = kw.get("k") or x.shape[1]
         N = kw.get("n") or out.shape[1]
         M = x.shape[0]
-        kind = "tc" if M > 64 and K % 8 == 0 and (x.dtype != BF16 or w.dtype == BF16) else "f32"       # csrc/linear_mma.cu
+        kind = "tc" if K % 8 == 0 and ((x.dtype != BF16 or w.dtype == BF16) if M > 64 else x.dtype == w.dtype == BF16) else "f32"     # csrc/linear_mma.cu, csrc/linear_rows_mma.cu
         return 2.0 * b * M * N * K, M * b * K * x.element_size() + _nbytes(w) + M * b * N * out.element_size(), kind
     if name == "linear_small":
         x, w, out = a[0], a[1], a[3]
@@ -123,7 +123,8 @@ def _cost(name, a, kw):
     if name == "ssd_scan":
         xbc, gates, S, segs, o = a[0], a[1], a[3], a[4], a[9]
         H, N, vdim = a[5], a[7], a[8]
-        return 4.0 * xbc.shape[0] * H * N * vdim, 2.0 * segs.shape[0] * H * N * vdim * 4 + xbc.shape[0] * xbc.shape[1] * 4.0 + _nbytes(gates, o), "f32"
+        return 4.0 * xbc.shape[0] * H * N * vdim, 2.0 * segs.shape[0] * H * N * vdim * 4 + xbc.shape[0] * xbc.shape[1] * 4.0 + _nbytes(gates, o), \
+            "tc" if N == 128 and vdim % 64 == 0 and (kw.get("lengths") or (0, xbc.shape[0]))[1] >= _lib.load().lia_ssd_chunk_rows() else "f32"       # csrc/ssd_chunk_sm100.cu
     if name == "rglru_scan":
         u, z, y, out = a[0], a[1], a[4], a[9]
         return 0.0, _nbytes(u, z, out) + u.numel() * y.element_size() + 2.0 * a[7].shape[0] * u.shape[1] * 4, "mem"

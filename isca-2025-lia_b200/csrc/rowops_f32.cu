@@ -3,8 +3,8 @@
 // embedding with its norm, with learned or wave positions and with a bigram table, the gated, normed residual update with a weighted mix of all earlier layers' results, the
 // residual kept as several streams that learned weights read, mix and write, a gate product under a norm in groups, the
 // polynomial activation between norms, a gated feed-forward activation with clamps, a projection onto a handful of outputs with the
-// gate non-linearities in its epilogue, a plain strided-batched projection on the CUDA cores (true 32-bit products and
-// sums: the exact path, and the carrier of shapes the tensor-core GEMM does not take), and a 32-bit argmax.
+// gate non-linearities in its epilogue, a plain strided-batched projection (true 32-bit products and sums: the exact path, and the carrier of shapes the
+// tensor-core GEMM does not take; on the CUDA cores where neither linear_rows_mma.cu nor linear_mma.cu takes it), and a 32-bit argmax.
 //
 // Activations are bf16 or fp32 (`act_f32`); everything a norm, a gate or the residual sum computes is fp32 either way.
 #include <math.h>

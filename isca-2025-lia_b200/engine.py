@@ -52,7 +52,7 @@ class Engine:
         seen = ops.moe_timeouts_seen()
         if seen != self._timeouts:
             new, self._timeouts = seen - self._timeouts, seen
-            raise _lib.LiaError(f"{new} blocks of an experts' projection gave up waiting: what was computed since the last check holds NaN")
+            raise _lib.LiaError(f"{new} blocks of an experts' projection or of a state-space scan gave up waiting: what was computed since the last check holds NaN")
 
     # ---- batch assembly: one pinned staging buffer, one H2D copy per pass
     def _upload(self, ids, segs, meta, want, static=None):

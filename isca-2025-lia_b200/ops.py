@@ -386,7 +386,8 @@ def linear_small(a, w, bias, out, mode=GATE_NONE, cap=1.0, resident=False):
 
 
 def linear_plain(a, w, out, scale=1.0, batch=1, a_batch_stride=0, w_batch_stride=0, out_batch_stride=0, n=None, k=None, resident=False):
-    """out[b] = scale * a[b] @ w[b].T on the CUDA cores with fp32 products and sums.  ``a`` / ``out`` are row-major 2-D
+    """out[b] = scale * a[b] @ w[b].T with products and sums as exact as fp32's: on the tensor cores for bf16 operands of up to 64 rows
+    (csrc/linear_rows_mma.cu) and from 65 rows on (csrc/linear_mma.cu) where rows are whole 16-byte vectors, on the CUDA cores else.  ``a`` / ``out`` are row-major 2-D
     views (row stride free); batches are taken at element strides from their first element; ``n``, ``k`` give the
     per-batch problem when the views are wider than one batch.  ``resident``: as for ``linear_small``."""
     lda, ldc = _rowmajor(a, "a"), _rowmajor(out, "out")

@@ -12,8 +12,8 @@ shared expert with or without a gate, experts that hand the token back).  Each o
 registers its per-sequence state with a ``seq_state.SlotState`` and runs one step over a batch of portions
 (``StepBatch``) through the kernels of ``ops``.
 
-Projections go through ``Linear``: the tensor-core GEMM of the OPT path (csrc/gemm_sm100.cu) for bf16 activations, the
-plain CUDA-core kernel for fp32 activations and for shapes the tensor-core kernel does not take.
+Projections go through ``Linear``: for bf16 activations the tensor-core GEMM of the OPT path (csrc/gemm_sm100.cu) and, for few rows and small
+weights, csrc/linear_rows_mma.cu; ``ops.linear_plain`` for fp32 activations and for shapes that these do not take.
 """
 import os
 
@@ -707,7 +707,7 @@ class ParallelMixer:
 
 class StateSpaceMixer:
     """Mamba-2's mixer (state-space duality): Win h = z | x | B | C | dt; x, B and C pass a short causal convolution with a bias per channel and
-    SiLU; dt = softplus(dt + dt_bias); per head S = exp(-exp(A_log) dt) S + dt B x^T, y = S^T C + D x (csrc/linear_scan.cu; the heads share
+    SiLU; dt = softplus(dt + dt_bias); per head S = exp(-exp(A_log) dt) S + dt B x^T, y = S^T C + D x (csrc/linear_scan.cu, long portions csrc/ssd_chunk_sm100.cu; the heads share
     B and C in ``groups``); N(y * silu(z)), the norm's mean taken over each of ``norm_groups`` stretches of the heads, then Wo.  Step sizes, decays, state and
     sums are fp32."""
 

@@ -40,4 +40,8 @@ def test_costs_of_the_tensor_core_forms():
     assert scan(e(64, 512), decay=d, lengths=(64, 64)) == "tc" and scan(e(64, 512), decay=d, lengths=(1, 31)) == "f32"
     assert scan(e(64, 512), gates=d, lengths=(64, 64)) == "f32" and scan(e(64, 512, dt=F32), decay=d, lengths=(64, 64)) == "f32"
     plain = lambda x, w: bench_compare._cost("linear_plain", (x, w, e(x.shape[0], w.shape[0], dt=F32)), {})[2]  # noqa: E731
-    assert plain(e(65, 64), e(8, 64)) == "tc" and plain(e(64, 64), e(8, 64)) == "f32" and plain(e(65, 64), e(8, 64, dt=F32)) == "f32" and plain(e(65, 60), e(8, 60)) == "f32"
+    assert plain(e(65, 64), e(8, 64)) == "tc" and plain(e(64, 64), e(8, 64)) == "tc" and plain(e(65, 64), e(8, 64, dt=F32)) == "f32" and plain(e(65, 60), e(8, 60)) == "f32"
+    assert plain(e(64, 64, dt=F32), e(8, 64)) == "f32" and plain(e(65, 64, dt=F32), e(8, 64)) == "tc" and plain(e(64, 60), e(8, 60)) == "f32"
+    ssd = lambda M, N, vdim, **kw: bench_compare._cost("ssd_scan", (e(M, 4 * vdim + 2 * N, dt=F32), e(M, 8, dt=F32), None, None, e(1, 4, dt=torch.int32), 4, 1, N, vdim,  # noqa: E731
+                                                                    e(M, 4 * vdim, dt=F32)), kw)[2]
+    assert ssd(448, 128, 64) == "tc" and ssd(447, 128, 64) == "f32" and ssd(600, 128, 64, lengths=(1, 300)) == "f32" and ssd(600, 64, 64) == "f32" and ssd(600, 128, 40) == "f32"
