@@ -39,23 +39,6 @@ template <int COLS> struct Shape {
   static constexpr int BARS = STAGES * STAGE_BYTES + STAGING;
   static constexpr int SMEM = BARS + (2 * STAGES + 5) * 8 + 16 + 1024;
 };
-constexpr unsigned WAIT_LIMIT = 1u << 20;                          // try_wait itself sleeps for a while: seconds in all
-
-__device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t parity, volatile int* dead) {
-  for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if ((i & 255u) == 255u && *dead) return false;
-  }
-  *dead = 1;
-  return false;
-}
-
 struct MoeArgs {
   const int* perm;
   const int* tile_expert;

@@ -48,7 +48,6 @@ constexpr int SHORT = 448;
 constexpr int TILE = 2 * L * 128;              // one part of B or C: two slabs of 64 rows of the state, 128 bytes a token
 constexpr int UNIT = L * 128;                  // one part of a unit's x, or of half its state
 constexpr float BIG = 1073741824.f, BIG_STATE = 1.2e30f;           // 2^30, 2^100
-constexpr unsigned WAIT_LIMIT = 1u << 20;      // try_wait itself sleeps for a while: seconds in all
 
 struct SsdArgs {
   const float *B, *C, *x;
@@ -65,23 +64,6 @@ struct SsdArgs {
   int tok0, span, split, per_cta;              // the tokens tok0 .. tok0 + span - 1 of every portion; a group's units in `split` CTAs of `per_cta`
   int* timeouts;
 };
-
-__device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t parity, volatile int* dead) {
-  for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if ((i & 255u) == 255u && *dead) return false;
-  }
-  *dead = 1;
-  return false;
-}
-// the same for a whole warp
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* dead) { return __all_sync(0xffffffffu, wait_for(bar, parity, dead)); }
 
 __device__ __forceinline__ void mma_tmem_a(uint32_t d, uint32_t a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(

@@ -31,6 +31,25 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
       "r"(parity)
       : "memory");
 }
+// A wait with a limit (try_wait itself sleeps for a while: seconds in all), after which it and all later ones of the block that share `dead` give up
+constexpr unsigned WAIT_LIMIT = 1u << 20;
+__device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t parity, volatile int* dead) {
+  for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if ((i & 255u) == 255u && *dead) return false;
+  }
+  *dead = 1;
+  return false;
+}
+// the same for a whole warp
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* dead) { return __all_sync(0xffffffffu, wait_for(bar, parity, dead)); }
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
