@@ -2,11 +2,11 @@
 // channels.  Nothing is held in fewer bits than on the CUDA cores: the caches are bf16 as they are, fp32 queries and the softmax's
 // weights enter as three bf16 parts (mma.cuh), scores and sums are fp32.
 //
-//   prompt:  one block per (64 rows of one portion, query head).  Bound: tensor cores and the softmax's instructions about equally -- mma.sync
+//   prompt:  (heads of 128 + 128 channels: window_attn_sm100.cu) one block per (64 rows of one portion, query head).  Bound: tensor cores and the softmax's instructions about equally -- mma.sync
 //            m16n8k16, one product for q . k (three for fp32 queries) and three for the weights times the values.  A warp owns 16 rows: its
 //            16 x 32 scores become the weights' operand in registers, so nothing but keys and values passes through shared memory; those come
 //            by cp.async, two stages of 32 keys (64 keys need 255 registers: two blocks per SM instead of three, 185 instead of 159 us).
-//            2048 tokens, 16 heads of 128 on 8 key heads, window 1024, soft cap: 1183 -> 155 us; the whole history, fp32 queries: 1713 -> 207 us.
+//            2048 tokens, 16 heads of 128 on 8 key heads, window 1024, soft cap: 1183 -> 136 us; the whole history, fp32 queries: 1713 -> 182 us (such heads: 66 and 64 us there).
 //   decode:  one block per (row, up to 8 query heads of one key/value head, range of keys).  Bound: HBM.  The heads of a group are the rows of
 //            the matrix instruction and a warp reads every cached row once for all of them, straight from global memory into operand
 //            registers: channels and value columns may be taken in any order as long as q and the output follow it, so a lane's 16
@@ -17,48 +17,14 @@
 // running ones in fp32: the error against 64 bits is 0.4 to 0.8 times that of the FMA chains (one running sum over 1700 keys: 5 times).
 // Numbers that are not finite do not survive this: a masked key of the stage has weight 0 and still meets its value, and a part of a split weight is 0 or has
 // the other sign.  Sums that are not finite stay so to the end, so it is there that such rows are found and formed again key by key (plain_row).
-#include "mma.cuh"
-#include "window_attn.cuh"
+#include "window_attn_rows.cuh"
+
+int window_prompt_tc(const void* q, int ldq, const bf16* kcache, long long kss, const bf16* vcache, long long vss, const int* meta, const int* segs, int nseg, const WindowExtras& x, bf16* out,
+                     int M, const WindowArgs& a, cudaStream_t stream);      // window_attn_sm100.cu
 
 namespace {
 
 constexpr int BM = 64;                 // rows of a prompt block
-
-// scores of one thread, in place: dot products * mul -> soft-capped, less the distance's cost.  dist(i) = query position - key position of score i.
-// tanh of small arguments (real scores are far below the cap) is its Taylor series up to the 9th power: below 0.3 the rest is under 6e-8 of
-// the value, one rounding, at a third of the instructions of tanhf, which with exp bounds this kernel as much as the products do.
-template <int N, typename Dist> __device__ __forceinline__ void finish_scores(float (&s)[N], float mul, const WindowArgs& a, float slope, const Dist& dist) {
-#pragma unroll
-  for (int i = 0; i < N; ++i) s[i] *= mul;
-  if (a.softcap > 0.f) {
-    // s / softcap as the division rounds it, without its branch: the product with the reciprocal, corrected once by its remainder (P. Markstein, Computation of elementary functions
-    // on the IBM RISC System/6000, 1990); an infinite score leaves no remainder to correct by
-    const float inv = 1.0f / a.softcap;
-    float top = 0.f;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      const float q = s[i] * inv, better = fmaf(fmaf(-q, a.softcap, s[i]), inv, q);
-      s[i] = better == better ? better : q;
-      top = fmaxf(top, fabsf(s[i]));
-      if (s[i] != s[i]) top = INFINITY;
-    }
-    if (top <= 0.3f) {
-#pragma unroll
-      for (int i = 0; i < N; ++i) {
-        const float z = s[i] * s[i];
-        const float p = z * fmaf(z, fmaf(z, fmaf(z, 62.f / 2835.f, -17.f / 315.f), 2.f / 15.f), -1.f / 3.f);
-        s[i] = a.softcap * fmaf(s[i], p, s[i]);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < N; ++i) s[i] = a.softcap * tanhf(s[i]);
-    }
-  }
-  if (slope != 0.f) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) s[i] -= slope * (float)dist(i);
-  }
-}
 
 // 16-byte chunk c of row r in a tile of rows of CH chunks: the chunk's place is turned by the row, so that ldmatrix (8 rows, one chunk)
 // touches all banks
@@ -72,48 +38,6 @@ template <int D, int BK> __device__ __forceinline__ void load_tile(uint32_t dst,
     const bool in = j0 + j <= last;
     cp_async16(at_chunk<CH>(dst, j, c), rows + (size_t)(in ? j0 + j : last) * stride + c * 8, in ? 16 : 0);
   }
-}
-
-// One row and head over the keys [lo, hi] of its sequence, all of which it sees, by one warp on the CUDA cores: lane j scores every 32nd key, lane l owns the
-// value columns l, l + 32, ...  For the rows whose sums were not finite, so it is never worth being fast.
-template <int DV> struct PlainRow {
-  float m, l, o[DV / 32];
-};
-template <int DK, int DV, int NQ>
-__device__ __noinline__ PlainRow<DV> plain_row(const void* q, size_t q_at, const bf16* kc, size_t k_stride, const bf16* vc, size_t v_stride, int lo, int hi, int pos, float mul,
-                                               float slope, float softcap) {
-  const int lane = threadIdx.x & 31;
-  PlainRow<DV> y;
-  y.m = -INFINITY;
-  y.l = 0.f;
-#pragma unroll
-  for (int c = 0; c < DV / 32; ++c) y.o[c] = 0.f;
-  for (int j0 = lo; j0 <= hi; j0 += 32) {
-    const int nk = min(32, hi + 1 - j0);
-    float s = 0.f;
-    if (lane < nk) {
-      for (int d = 0; d < DK; ++d) {
-        const float x = NQ == 1 ? __bfloat162float(reinterpret_cast<const bf16*>(q)[q_at + d]) : reinterpret_cast<const float*>(q)[q_at + d];
-        s = fmaf(x, __bfloat162float(kc[(size_t)(j0 + lane) * k_stride + d]), s);
-      }
-      s *= mul;
-      if (softcap > 0.f) s = softcap * tanhf(s / softcap);
-      if (slope != 0.f) s -= slope * (float)(pos - j0 - lane);
-    } else {
-      s = -INFINITY;
-    }
-    const float m = fmaxf(y.m, warp_max(s)), base = m == -INFINITY ? 0.f : m, p = expf(s - base), al = expf(y.m - base);
-    y.m = m;
-    y.l = fmaf(y.l, al, warp_sum(p));
-#pragma unroll
-    for (int c = 0; c < DV / 32; ++c) y.o[c] *= al;
-    for (int j = 0; j < nk; ++j) {
-      const float w = __shfl_sync(0xffffffffu, p, j);
-#pragma unroll
-      for (int c = 0; c < DV / 32; ++c) y.o[c] = fmaf(w, __bfloat162float(vc[(size_t)(j0 + j) * v_stride + lane + 32 * c]), y.o[c]);
-    }
-  }
-  return y;
 }
 
 template <int DK, int DV, int NQ> struct PromptShape {
@@ -138,23 +62,7 @@ __global__ void __launch_bounds__(128, (DV <= 128 && NQ == 1) ? 3 : 2) window_pr
     slot = meta[0]; pos0 = meta[1]; row0 = 0; rows = M;
     if (tile * BM >= rows) return;
   } else {
-    int found = -1;
-    for (int base = 0; base < nseg && found < 0; base += 32) {           // the portion that holds this tile: 32 portions at a time
-      const int n = base + lane < nseg ? (segs[4 * (base + lane) + 3] + BM - 1) / BM : 0;
-      int upto = n;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, upto, o);
-        if (lane >= o) upto += v;
-      }
-      const unsigned hit = __ballot_sync(0xffffffffu, tile < upto);
-      if (hit) {
-        found = base + __ffs(hit) - 1;
-        tile -= __shfl_sync(0xffffffffu, upto - n, __ffs(hit) - 1);
-      } else {
-        tile -= __shfl_sync(0xffffffffu, upto, 31);
-      }
-    }
+    const int found = portion_of<BM>(segs, nseg, tile);
     if (found < 0) return;
     slot = segs[4 * found]; pos0 = segs[4 * found + 1]; row0 = segs[4 * found + 2]; rows = segs[4 * found + 3];
   }
@@ -590,7 +498,10 @@ template <int DK, int DV, int NQ> int decode_as(const Call& c) {
 }
 
 template <int DK, int DV> int run_as(const Call& c, bool prompt) {
-  if (prompt) return c.a.q_f32 ? prompt_as<DK, DV, 3>(c) : prompt_as<DK, DV, 1>(c);
+  if (prompt) {
+    if constexpr (DK == 128 && DV == 128) return window_prompt_tc(c.q, c.ldq, c.kcache, c.kss, c.vcache, c.vss, c.meta, c.segs, c.nseg, c.x, c.out, c.M, c.a, c.stream);
+    else return c.a.q_f32 ? prompt_as<DK, DV, 3>(c) : prompt_as<DK, DV, 1>(c);
+  }
   return c.a.q_f32 ? decode_as<DK, DV, 3>(c) : decode_as<DK, DV, 1>(c);
 }
 

@@ -1,0 +1,44 @@
+"""Prompts through window attention on tcgen05 (csrc/window_attn_sm100.cu) against a float64 softmax, where its tiles can go wrong: portions of 1 to 300 rows behind 0 to 700
+positions (blocks of 64 keys to the second turn of the ring, tiles of 128 rows), windows and chunks that hide whole blocks from some warps, scores beyond and below the soft cap's short form,
+gates whose rows are whole 16-byte vectors and not, bf16 and fp32 outputs."""
+import pytest
+import torch
+
+import lia_b200  # noqa: F401
+from lia_b200 import ops
+from test_gpu_attn_mma import BF16, DEV, F32, F64, TOL, inputs, reference
+
+pytestmark = pytest.mark.gpu
+PORTIONS = [(0, 0, 300), (1, 700, 129), (2, 255, 1), (3, 63, 128), (4, 0, 2), (5, 129, 191)]
+
+
+@pytest.mark.parametrize("q_f32", [False, True])
+@pytest.mark.parametrize("H,G,v_div", [(4, 2, 1), (3, 3, 3), (8, 1, 1)])
+@pytest.mark.parametrize("opt", [dict(), dict(window=33), dict(window=200, softcap=30.0, temp=True), dict(softcap=1.5), dict(chunk=100, sink=True, slopes=True)], ids=str)
+def test_portions(q_f32, H, G, v_div, opt):
+    opt, d = dict(opt), 128
+    q, kc, vc, segs, d_segs, meta = inputs(PORTIONS, H, G, d, d, q_f32, 3, v_div)
+    g = torch.Generator().manual_seed(1)
+    for n in ("temp", "sink", "slopes"):
+        if opt.get(n):
+            opt[n] = 0.5 + torch.rand(H, generator=g)
+    want = reference(q, kc, vc, segs, H, G, d, d, 0.1, v_div=v_div, **opt).reshape(q.shape[0], -1)
+    dev = {n: opt[n].to(DEV) if opt.get(n) is not None else None for n in ("temp", "sink", "slopes")}
+
+    def run(dtype, gate=None):
+        out = torch.full((q.shape[0], H * d), 7.0, dtype=dtype, device=DEV)
+        ops.window_attn(q, kc, vc, meta, dev["temp"], out, H, G, d, d, opt.get("window", 0), 0.1, opt.get("softcap", 0.0), nseg=len(segs), segs=d_segs, max_ctx=830,
+                        slopes=dev["slopes"], sink=dev["sink"], chunk=opt.get("chunk", 0), v_div=v_div, gate=gate)
+        return out
+    out = run(F32)
+    assert float((out.cpu().to(F64) - want).abs().max() / want.abs().max()) < TOL
+    for i, (slot, p0, r0, n) in enumerate(segs):                    # a portion does not depend on its company
+        alone = torch.empty(n, H * d, dtype=F32, device=DEV)
+        ops.window_attn(q[r0:r0 + n].contiguous(), kc, vc, meta[r0:r0 + n].contiguous(), dev["temp"], alone, H, G, d, d, opt.get("window", 0), 0.1, opt.get("softcap", 0.0), nseg=1,
+                        segs=torch.tensor([(slot, p0, 0, n)], dtype=torch.int32, device=DEV), max_ctx=p0 + n, slopes=dev["slopes"], sink=dev["sink"], chunk=opt.get("chunk", 0), v_div=v_div)
+        assert n == 1 or torch.equal(alone, out[r0:r0 + n])
+    for pad in (0, 4):                                              # one rounding to bf16 of numbers up to the largest
+        wide = torch.randn(q.shape[0], H * d + 8 + pad, generator=g).to(BF16).to(DEV)
+        gate = wide[:, 8:8 + H * d]
+        got = want * torch.sigmoid(gate.cpu().to(F64))
+        assert float((run(BF16, gate).cpu().to(F64) - got).abs().max() / got.abs().max()) < 2.0 ** -8
