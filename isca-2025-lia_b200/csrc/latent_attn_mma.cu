@@ -5,16 +5,18 @@
 // and values are kept as three bf16 parts of their fp32 sums, and so are the rotated query parts and the softmax's weights (mma.cuh).  With bf16
 // queries and bf16 rotated keys a score is three products of each part, a weighted value six (of the nine).
 //
-// One block per (64 rows, head), warp by 16 rows, the scores becoming the weights' operand in registers; 32 keys per stage.  Keys and values
-// are fetched in turn (the next keys while the values are taken in, the next values while the scores are made), so one stage of 52 KB
-// is enough and two blocks share an SM.  Bound: tensor cores and shared-memory reads about equally.  2048 tokens, 16 heads of 128 + 64 on latents
-// of 512: 4794 us in the latent space on the CUDA cores and 439 us for its two projections -> 352 and 67 us for the expansion.
+// Heads of 128 + 64 channels are latent_attn_sm100.cu's.  Here, for heads of 64 + 64, one block per (64 rows, head), warp by 16 rows, the scores becoming the weights' operand in registers; 32 keys
+// per stage.  Keys and values are fetched in turn (the next keys while the values are taken in, the next values while the scores are made), so one stage is enough and several blocks share an SM.
+// Bound: tensor cores and shared-memory reads about equally.  2048 tokens, 16 heads of 128 + 64 on latents of 512: 4794 us in the latent space on the CUDA cores and 439 us for its two projections ->
+// 352 here (104 there) and 67 us for the expansion.
 // Rows whose sums are not finite are formed again key by key at the end, as in window_attn_mma.cu: a masked key's weight of 0 still meets its value.
 #include <limits.h>
 #include <math.h>
 #include <stdint.h>
 
-#include "mma.cuh"
+#include "latent_attn_rows.cuh"
+
+int latent_expanded_tc(const ExpandedArgs& a, int tiles, long long latents, cudaStream_t stream);      // latent_attn_sm100.cu
 
 // linear_mma.cu
 int linear_mma_parts(const bf16* const* src, const int* rows, int n, long long lda, const bf16* W, bf16* C, long long ldc, int N, int K, int part, cudaStream_t stream);
@@ -22,66 +24,9 @@ int linear_mma_parts(const bf16* const* src, const int* rows, int n, long long l
 namespace {
 
 constexpr int BM = 64, BK = 32;
-constexpr int MAX_PORTIONS = 16;        // of one launch
 
 // 16-byte chunk c of row r in a tile of rows of CH (at least 8) chunks, turned by the row (window_attn_mma.cu)
 template <int CH> __device__ __forceinline__ uint32_t at_chunk(uint32_t base, int r, int c) { return base + (uint32_t)(r * CH + (c ^ (r & 7))) * 16u; }
-
-struct Portion {
-  const bf16* kr;       // the shared rotated key part of the first latent it sees
-  int row0, n, pos0;    // its rows, and the position of the first among the latents it sees
-  int part0, tile0;     // its first expanded row and its first 64-row tile
-};
-
-struct ExpandedArgs {
-  const bf16* q;        // rows of H heads of DN + DR channels, the first DN unrotated
-  const float* qr;      // [row][H][qr_stride]: the rotated DR channels
-  const bf16* parts;    // [latent][2 nh][3][DN]: keys of the heads h0 .. h0 + nh - 1, then values
-  const float* gate;    // [row][H] or null
-  const float* sink;    // [H] or null
-  void* out;            // [row][H * DN]
-  long long kr_stride;
-  int ldq, qr_stride, H, h0, nh, window, out_f32, np;
-  float scale;
-  Portion p[MAX_PORTIONS];
-};
-
-// One row and head over the latents [lo, hi] by one warp on the CUDA cores: lane j scores every 32nd key, lane l owns the value columns l, l + 32, ...
-template <int DN> struct PlainRow {
-  float m, l, o[DN / 32];
-};
-template <int DN, int DR>
-__device__ __noinline__ PlainRow<DN> plain_row(const bf16* q, const float* qr, const bf16* keys, const bf16* vals, size_t stride, const bf16* key_rot, long long rot_stride, int lo,
-                                               int hi, float scale) {
-  const int lane = threadIdx.x & 31;
-  auto whole = [](const bf16* p) { return __bfloat162float(p[0]) + (__bfloat162float(p[DN]) + __bfloat162float(p[2 * DN])); };
-  PlainRow<DN> y;
-  y.m = -INFINITY;
-  y.l = 0.f;
-#pragma unroll
-  for (int c = 0; c < DN / 32; ++c) y.o[c] = 0.f;
-  for (int j0 = lo; j0 <= hi; j0 += 32) {
-    const int nk = min(32, hi + 1 - j0);
-    float s = -INFINITY;
-    if (lane < nk) {
-      s = 0.f;
-      for (int d = 0; d < DN; ++d) s = fmaf(__bfloat162float(q[d]), whole(keys + (size_t)(j0 + lane) * stride + d), s);
-      for (int d = 0; d < DR; ++d) s = fmaf(qr[d], __bfloat162float(key_rot[(size_t)(j0 + lane) * rot_stride + d]), s);
-      s *= scale;
-    }
-    const float m = fmaxf(y.m, warp_max(s)), base = m == -INFINITY ? 0.f : m, p = expf(s - base), al = expf(y.m - base);
-    y.m = m;
-    y.l = fmaf(y.l, al, warp_sum(p));
-#pragma unroll
-    for (int c = 0; c < DN / 32; ++c) y.o[c] *= al;
-    for (int j = 0; j < nk; ++j) {
-      const float w = __shfl_sync(0xffffffffu, p, j);
-#pragma unroll
-      for (int c = 0; c < DN / 32; ++c) y.o[c] = fmaf(w, whole(vals + (size_t)(j0 + j) * stride + lane + 32 * c), y.o[c]);
-    }
-  }
-  return y;
-}
 
 template <int DN, int DR> constexpr int expanded_smem() { return (BM * DN + 3 * BM * DR + 2 * 3 * BK * DN + BK * DR) * 2; }
 
@@ -379,7 +324,7 @@ extern "C" int lia_latent_attn_expanded_in(const void* q, int ldq, const float* 
   const uintptr_t addr = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(qr) | reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(w_ukv) |
                          reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(workspace);
   LIA_CHECK_ARG(addr % 16 == 0 && ldq % 8 == 0 && ldq >= H * (dim + rot) && qr_stride % 4 == 0 && slot_stride % 8 == 0, "lia_latent_attn_expanded: addresses and rows must be whole 16 bytes");
-  const int D = kv_rank + rot;
+  const int D = kv_rank + rot, tile_rows = dim == 128 ? 128 : BM;
   const size_t room = workspace_bytes / lia_latent_expanded_workspace_bytes(1, 1, dim);          // (latent, head) pairs
   if (window <= 0) window = 1 << 30;
   for (int first = 0; first < np;) {
@@ -395,7 +340,7 @@ extern "C" int lia_latent_attn_expanded_in(const void* q, int ldq, const float* 
       src[i] = reinterpret_cast<const bf16*>(cache) + (size_t)p[0] * slot_stride + (size_t)base * D;
       rows[i] = seen;
       a.p[i] = Portion{src[i] + kv_rank, p[2], p[3], p[1] - base, (int)latents, tiles};
-      tiles += (p[3] + BM - 1) / BM;
+      tiles += (p[3] + tile_rows - 1) / tile_rows;
       latents += seen;
       ++a.np;
       ++first;
@@ -415,7 +360,7 @@ extern "C" int lia_latent_attn_expanded_in(const void* q, int ldq, const float* 
         rc = linear_mma_parts(src, rows, a.np, D, wk + (size_t)a.h0 * dim * kv_rank, ws, ldc, a.nh * dim, kv_rank, dim, stream);
         if (rc == LIA_OK) rc = linear_mma_parts(src, rows, a.np, D, wk + (size_t)(H + a.h0) * dim * kv_rank, ws + (size_t)3 * a.nh * dim, ldc, a.nh * dim, kv_rank, dim, stream);
       }
-      if (rc == LIA_OK) rc = dim == 128 ? run<128, 64>(a, tiles, stream) : run<64, 64>(a, tiles, stream);
+      if (rc == LIA_OK) rc = dim == 128 ? latent_expanded_tc(a, tiles, latents, stream) : run<64, 64>(a, tiles, stream);
       if (rc != LIA_OK) return rc;
     }
   }

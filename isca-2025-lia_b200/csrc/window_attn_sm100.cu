@@ -1,12 +1,7 @@
 // Window attention (window_attn.cu) of prompts on tcgen05, for bf16 caches with heads of 128 channels.  Nothing is held in fewer bits than on the CUDA cores: bf16 queries, keys and values
 // enter as they are, fp32 queries and the softmax's weights as three bf16 parts (mma.cuh), scores and sums are fp32.
 //
-// One CTA per (128 rows of one portion, query head), 64 keys at a time.  The blocks of keys go in turn to two groups of four warps; a thread owns one row (= one lane of TMEM), so that
-// nothing of the softmax crosses threads but the running maximum, which goes from group to group by block.
-//   warps 0-3, 4-7   scores from TMEM -> finished scores, back to TMEM -> weights, as three parts, to TMEM in the scores' place (the A operand of the products with the values)
-//   warps 8-11       a block's weighted values from TMEM, added to the row's 128 sums in registers; at the end the sums' way out
-//   warps 12-14      keys and values, each warp a third of a block
-//   warp 15          issues the products, all lanes together (issued by one lane of a diverged warp an instruction took 115 clocks, now 65)
+// One CTA per (128 rows of one portion, query head), 64 keys at a time; who does what: attn_sm100.cuh.
 // Bound: the softmax's latencies and its some 25 instructions a score, two scores an instruction where they come in pairs: a block takes 2 x 2000 clocks of a group; the products
 // (512 multiply-adds a score, 896 for fp32 queries) 1300 to 2400 of the tensor cores.  Loops over 32 scores with small bodies, for unrolled over 64 they miss the instruction cache.
 //
@@ -15,76 +10,21 @@
 // Sums that are not finite stay so to the end, where such rows are formed again key by key (window_attn_rows.cuh): a masked key's weight of 0 still meets its value.
 // Waits are bounded: a CTA that gives up leaves NaN and counts itself (lia_moe_timeouts_seen()).
 //
-// 8 key heads of 128; on mma.sync -> here, us, and the error against 64 bits in 1e-7: 2048 rows, 16 heads, window of 1024 and soft cap 136 (1.87) -> 66 (1.70), the whole history and fp32 queries
-// 182 (2.42) -> 64 (1.73); 700 rows behind 300 91 (2.43) -> 36 (2.19); portions of 300, 250, 200 31 (1.54) -> 17 (1.49); 64 rows 9.3 (1.37) -> 9.2 (1.19).
+// 8 key heads of 128; on mma.sync -> here, us, and the error against 64 bits in 1e-7: 2048 rows, 16 heads, window of 1024 and soft cap 136 (1.87) -> 66 (1.68), the whole history and fp32 queries
+// 182 (2.42) -> 63 (1.69); 700 rows behind 300 91 (2.43) -> 35 (2.16); portions of 300, 250, 200 31 (1.54) -> 17 (1.49); 64 rows 9.3 (1.37) -> 9.4 (1.19).
+#include "attn_sm100.cuh"
 #include "window_attn_rows.cuh"
-#include "umma.cuh"
-
-int* lia_timeout_word();                                           // moe_sm100.cu
 
 namespace {
 
-constexpr int ROWS = 128, KEYS = 64, D = 128;
-constexpr int THREADS = 512, LOADERS = 3;
-constexpr int SOFTMAX_REGS = 144, SUM_REGS = 184, OTHER_REGS = 40;  // of a thread, by what its four warps do (setmaxnreg: multiples of 8)
+constexpr int KEYS = 64, CH = 32;                                  // of a block; scores that a thread has at a time
 constexpr int Q_BYTES = ROWS * D * 2, KV_BYTES = KEYS * D * 2;     // two slabs of 64 channels each, 128 bytes a row, 16-byte pieces turned by the row
-
-struct Bars {
-  uint64_t q_full, kv_full[4], kv_empty[4], s_full[2], p_full[2], m_full[2][4], o_full, o_empty, drain;
-};
-struct Tail {
-  float top[2][ROWS];                                              // the running maximum after a block
-  float2 add[4][ROWS];                                             // of a block: what the sums before it count for, the sum of its weights
-  Bars bars;
-  uint32_t tmem;
-  int dead;
+struct Tail : AttnTail {
+  uint64_t kv_full[4], kv_empty[4];
 };
 template <int NQ> __host__ __device__ constexpr int stages() { return NQ == 1 ? 4 : 3; }
 template <int NQ> __host__ __device__ constexpr int smem_bytes() { return NQ * Q_BYTES + stages<NQ>() * 2 * KV_BYTES + (int)sizeof(Tail) + 1024; }
-// TMEM: group s has its scores (three accumulators of 64 columns; the first becomes the finished scores, the others' place the weights in three parts of 32) at GROUP s; the products with the
-// values, two halves of 64 columns, at SUMS, for both groups in turn
-constexpr uint32_t GROUP = 192, WEIGHTS = 64, SUMS = 384;
-constexpr int CH = 32;                                             // scores that a thread has at a time
 
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float x, float y) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ f32x2 both(float x) { return pack2(x, x); }
-
-// exp(x) for x <= 0 as 2^(x log2 e): the power of the rounded product, corrected to first order by what the rounding of the product and of log2 e left out.  A NaN stays one; below 2^-126
-// it is 0.
-__device__ __forceinline__ f32x2 exp_pair(f32x2 v) {
-  constexpr float L2E = 1.44269502162933349609f, L2E_REST = 1.92596299e-8f, LN2 = 0.693147180559945f;
-  float x, y;
-  unpack2(v, x, y);
-  asm("max.NaN.f32 %0, %0, 0fC3160000;" : "+f"(x));                // -150: no infinity less itself below
-  asm("max.NaN.f32 %0, %0, 0fC3160000;" : "+f"(y));
-  const f32x2 z = pack2(x, y), t = mul2(z, both(L2E)), over = fma2(z, both(-L2E_REST), fma2(z, both(-L2E), t));
-  unpack2(t, x, y);
-  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(x));
-  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(y));
-  const f32x2 r = pack2(x, y);
-  return fma2(mul2(r, both(-LN2)), over, r);
-}
 // finish_scores (window_attn_rows.cuh) two at a time; `far`: query position - key position of the first
 __device__ __forceinline__ void finish_pairs(f32x2 (&s)[CH / 2], float mul, const WindowArgs& a, float slope, int far) {
 #pragma unroll
@@ -124,23 +64,87 @@ __device__ __forceinline__ void finish_pairs(f32x2 (&s)[CH / 2], float mul, cons
   }
 }
 
-__device__ __forceinline__ uint32_t elect_one() {
-  uint32_t one;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
-  return one;
-}
-__device__ __forceinline__ void mma_if(uint32_t one, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc),
-               "r"(accumulate), "r"(one)
-               : "memory");
-}
-__device__ __forceinline__ void mma_tmem_a_if(uint32_t one, uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc),
-               "r"(accumulate), "r"(one)
-               : "memory");
-}
-__device__ __forceinline__ void commit_if(uint32_t one, uint32_t bar) {
-  if (one) tcgen05_commit(bar);
+// A group's blocks s, s + 2, ... of n.  A thread's row is at position `pos` and sees the keys lo .. pos; its warp's first row is at wpos and sees keys from w_lo on, its last from w_all on; the
+// first key is jb.  finish(pairs, j): what becomes of the sums of products with the keys j, j + 1, ...
+template <class Finish>
+__device__ __forceinline__ void softmax_blocks(AttnTail& sm, uint32_t tmem, int s, int n, int jb, int pos, int lo, int wpos, int w_lo, int w_all, const Finish& finish) {
+  volatile int* dead = &sm.dead;
+  const int w = group_warp(), lane = threadIdx.x & 31, r = w * 32 + lane;
+  const uint32_t ts = tmem + s * GROUP + ((uint32_t)(w * 32) << 16);
+#pragma unroll 1
+  for (int it = s; it < n; it += 2) {
+    const int j0 = jb + it * KEYS;
+    if (!warp_wait(smem_u32(&sm.s_full[s]), (it >> 1) & 1, dead)) break;
+    tcgen05_fence_after();
+    const bool seen = j0 <= wpos + 31 && j0 + KEYS - 1 >= w_lo, partly = j0 + KEYS - 1 > wpos || j0 < w_all;         // by some row of the warp; not by every row, not every key
+    float top = -INFINITY;
+    if (seen) {
+#pragma unroll 1
+      for (int c = 0; c < KEYS; c += CH) {
+        uint32_t u[3][CH];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) tmem_ld32(ts + k * KEYS + c, u[k]);
+        tmem_ld_wait();
+        f32x2 sc[CH / 2];
+#pragma unroll
+        for (int i = 0; i < CH / 2; ++i) {
+          f32x2 v[3];
+#pragma unroll
+          for (int k = 0; k < 3; ++k) v[k] = pack2(__uint_as_float(u[k][2 * i]), __uint_as_float(u[k][2 * i + 1]));
+          sc[i] = add2(add2(v[0], v[1]), v[2]);
+        }
+        finish(sc, j0 + c);
+#pragma unroll
+        for (int i = 0; i < CH / 2; ++i) {
+          float x, y;
+          unpack2(sc[i], x, y);
+          u[0][2 * i] = __float_as_uint(x), u[0][2 * i + 1] = __float_as_uint(y);
+        }
+        if (partly) {
+#pragma unroll
+          for (int e = 0; e < CH; ++e)
+            if (j0 + c + e > pos || j0 + c + e < lo) u[0][e] = 0xff800000u;
+        }
+        float t[4] = {top, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int e = 0; e < CH; ++e) t[e & 3] = fmaxf(t[e & 3], __uint_as_float(u[0][e]));
+        top = fmaxf(fmaxf(t[0], t[1]), fmaxf(t[2], t[3]));
+        tmem_st32(ts + c, u[0]);
+      }
+      tmem_st_wait();
+    }
+    float before;
+    if (!hand_over_top(sm, s, it, top, before)) break;
+    const float from = top == -INFINITY ? 0.f : top;             // no key seen so far
+    f32x2 sum[2] = {0ull, 0ull};
+    if (seen) {
+#pragma unroll 1
+      for (int c = 0; c < KEYS; c += CH) {
+        uint32_t u[CH], p[3][CH / 2];
+        tmem_ld32(ts + c, u);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < CH / 2; ++i) {
+          const f32x2 w = exp_pair(add2(pack2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1])), both(-from)));
+          sum[i & 1] = add2(sum[i & 1], w);
+          split_pair(w, p[0][i], p[1][i], p[2][i]);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) tmem_st16(ts + WEIGHTS + k * 32 + c / 2, p[k]);
+      }
+    } else {
+      const uint32_t none[16] = {};
+#pragma unroll
+      for (int c = 0; c < 96; c += 16) tmem_st16(ts + WEIGHTS + c, none);
+    }
+    float x, y;
+    unpack2(add2(sum[0], sum[1]), x, y);
+    sm.add[it & 3][r] = make_float2(expf(before - from), x + y);
+    tmem_st_wait();
+    tcgen05_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&sm.p_full[s]));
+  }
 }
 
 template <int NQ>
@@ -154,47 +158,23 @@ __global__ void __launch_bounds__(THREADS, 1) window_prompt_tc_kernel(const void
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   volatile int* dead = &sm.dead;
   if (tid == 0) {
-    sm.dead = 0;
-    mbar_init(smem_u32(&sm.bars.q_full), 8);
+    init_hand_overs(sm);
     for (int i = 0; i < ST; ++i) {
-      mbar_init(smem_u32(&sm.bars.kv_full[i]), LOADERS);
-      mbar_init(smem_u32(&sm.bars.kv_empty[i]), 1);
+      mbar_init(smem_u32(&sm.kv_full[i]), LOADERS);
+      mbar_init(smem_u32(&sm.kv_empty[i]), 1);
     }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&sm.bars.s_full[i]), 1);
-      mbar_init(smem_u32(&sm.bars.p_full[i]), 4);
-      for (int w = 0; w < 4; ++w) mbar_init(smem_u32(&sm.bars.m_full[i][w]), 1);
-    }
-    mbar_init(smem_u32(&sm.bars.o_full), 1);
-    mbar_init(smem_u32(&sm.bars.o_empty), 4);
-    mbar_init(smem_u32(&sm.bars.drain), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 15) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem)), "r"(512u) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  tcgen05_fence_before();
-  __syncthreads();
-  tcgen05_fence_after();
-  const uint32_t tmem = sm.tmem;
-  auto leave = [&] {
-    tcgen05_fence_before();
-    __syncthreads();
-    if (warp == 15) {
-      tcgen05_fence_after();
-      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
-    }
-  };
+  const uint32_t tmem = take_tmem(sm, warp);
   pdl_launch_dependents();
   pdl_wait();
   int tile = gridDim.y - 1 - blockIdx.y, slot, pos0, row0, rows;
   if (segs == nullptr) {
     slot = meta[0]; pos0 = meta[1]; row0 = 0; rows = M;
-    if (tile * ROWS >= rows) return leave();
+    if (tile * ROWS >= rows) return give_tmem_back(tmem, warp);
   } else {
     const int found = portion_of<ROWS>(segs, nseg, tile);
-    if (found < 0) return leave();
+    if (found < 0) return give_tmem_back(tmem, warp);
     slot = segs[4 * found]; pos0 = segs[4 * found + 1]; row0 = segs[4 * found + 2]; rows = segs[4 * found + 3];
   }
   const int h = blockIdx.x, kg = h / (a.H / a.G), vg = kg / a.v_div, Gv = a.G / a.v_div;
@@ -219,35 +199,36 @@ __global__ void __launch_bounds__(THREADS, 1) window_prompt_tc_kernel(const void
     if (!__syncthreads_and(run)) {
 #pragma unroll 1
       for (int r = warp; r < rows; r += THREADS / 32) by_itself(row0 + r, meta[2 * (row0 + r)], meta[2 * (row0 + r) + 1]);
-      return leave();
+      return give_tmem_back(tmem, warp);
     }
   }
+  slot = __shfl_sync(0xffffffffu, slot, 0), pos0 = __shfl_sync(0xffffffffu, pos0, 0), row0 = __shfl_sync(0xffffffffu, row0, 0), rows = __shfl_sync(0xffffffffu, rows, 0);      // known to be the same in all lanes
   const int pos_last = pos0 + rows - 1, jb = first_key(a, pos0), n = (pos_last - jb) / KEYS + 1;
 
-  if (warp >= 12) {
+  if (warp >= LOADER0) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(OTHER_REGS));
-    if (warp < 12 + LOADERS) {
-      const int piece = lane & 15;
+    if (warp < ISSUER) {
+      const int piece = lane & 15;                                 // a piece of 16 bytes a lane and row, of keys and of values
       const bf16* kc = kcache + (size_t)slot * k_slot_stride + (size_t)kg * D + piece * 8;
       const bf16* vc = vcache + (size_t)slot * v_slot_stride + (size_t)vg * D + piece * 8;
       int under_way = -1;                                          // the block that was asked for last
       auto arrived = [&] {
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sm.bars.kv_full[under_way % ST]));
+        if (lane == 0) mbar_arrive(smem_u32(&sm.kv_full[under_way % ST]));
       };
 #pragma unroll 1
       for (int it = 0; it < n; ++it) {
         const int st = it % ST, j0 = jb + it * KEYS;
-        if (under_way >= 0 && !mbar_test(smem_u32(&sm.bars.kv_empty[st]), ((it / ST) & 1) ^ 1u)) {          // no place yet: first see the last one home
+        if (under_way >= 0 && !mbar_test(smem_u32(&sm.kv_empty[st]), ((it / ST) & 1) ^ 1u)) {          // no place yet: first see the last one home
           cp_async_wait<0>();
           arrived();
           under_way = -1;
         }
-        if (!warp_wait(smem_u32(&sm.bars.kv_empty[st]), ((it / ST) & 1) ^ 1u, dead)) break;
+        if (!warp_wait(smem_u32(&sm.kv_empty[st]), ((it / ST) & 1) ^ 1u, dead)) break;
         const uint32_t dst = ks + st * 2 * KV_BYTES + (piece >> 3) * (KV_BYTES / 2);
 #pragma unroll 4
-        for (int i = 2 * (warp - 12) + (lane >> 4); i < KEYS; i += 2 * LOADERS) {
+        for (int i = 2 * (warp - LOADER0) + (lane >> 4); i < KEYS; i += 2 * LOADERS) {
           const bool in = j0 + i <= pos_last;
           const size_t row = (size_t)(in ? j0 + i : pos_last);
           const uint32_t at = dst + i * 128 + (((piece & 7) ^ (i & 7)) << 4);
@@ -265,7 +246,7 @@ __global__ void __launch_bounds__(THREADS, 1) window_prompt_tc_kernel(const void
       if (under_way >= 0) arrived();
     } else {
       const uint32_t one = elect_one();
-      constexpr uint32_t idesc_s = make_idesc(ROWS, KEYS), idesc_o = make_idesc(ROWS, D) | (1u << 16);         // the values lie with the keys as rows
+      constexpr uint32_t idesc_s = make_idesc(ROWS, KEYS);
       // (from loops: unrolled, these instructions would not stay in the instruction cache beside the other warps' code)
       const uint64_t q_desc = make_smem_desc(base), k_desc = make_smem_desc(ks), v_desc = make_smem_desc_mn(ks + KV_BYTES, KV_BYTES / 2);
       auto scores = [&](int it) {
@@ -283,30 +264,26 @@ __global__ void __launch_bounds__(THREADS, 1) window_prompt_tc_kernel(const void
               to = to == d + 2 * KEYS ? d : to + KEYS;
             }
         }
-        commit_if(one, smem_u32(&sm.bars.s_full[it & 1]));
+        commit_if(one, smem_u32(&sm.s_full[it & 1]));
       };
-      bool alive = warp_wait(smem_u32(&sm.bars.q_full), 0u, dead);
+      bool alive = warp_wait(smem_u32(&sm.q_full), 0u, dead);
       for (int it = 0; alive && it < 2 && it < n; ++it) {
-        alive = warp_wait(smem_u32(&sm.bars.kv_full[it]), 0u, dead);
+        alive = warp_wait(smem_u32(&sm.kv_full[it]), 0u, dead);
         tcgen05_fence_after();
         if (alive) scores(it);
       }
 #pragma unroll 1
       for (int it = 0; alive && it < n; ++it) {
         const int s = it & 1;
-        if (!(alive = warp_wait(smem_u32(&sm.bars.p_full[s]), (it >> 1) & 1, dead))) break;
-        tcgen05_fence_after();
-        if (it > 0 && !(alive = warp_wait(smem_u32(&sm.bars.o_empty), (it - 1) & 1, dead))) break;
+        if (!(alive = warp_wait(smem_u32(&sm.p_full[s]), (it >> 1) & 1, dead))) break;
         tcgen05_fence_after();
         const uint64_t vb = v_desc + (uint32_t)(it % ST) * (2 * KV_BYTES >> 4);
 #pragma unroll 1
-        for (int part = 2; part >= 0; --part)
-#pragma unroll
-          for (int k = 0; k < KEYS / 16; ++k) mma_tmem_a_if(one, tmem + SUMS, tmem + s * GROUP + WEIGHTS + part * 32 + k * 8, vb + k * 128, idesc_o, part < 2 || k > 0);
-        commit_if(one, smem_u32(&sm.bars.kv_empty[it % ST]));
-        commit_if(one, smem_u32(&sm.bars.o_full));
+        for (int part = 2; part >= 0; --part) issue_values<KEYS>(one, tmem, s, part, vb, part == 2);
+        commit_if(one, smem_u32(&sm.kv_empty[it % ST]));
+        commit_if(one, smem_u32(&sm.o_full));
         if (it + 2 < n) {
-          if (!(alive = warp_wait(smem_u32(&sm.bars.kv_full[(it + 2) % ST]), ((it + 2) / ST) & 1, dead))) break;
+          if (!(alive = warp_wait(smem_u32(&sm.kv_full[(it + 2) % ST]), ((it + 2) / ST) & 1, dead))) break;
           tcgen05_fence_after();
           scores(it + 2);
         }
@@ -347,191 +324,37 @@ __global__ void __launch_bounds__(THREADS, 1) window_prompt_tc_kernel(const void
     }
     fence_proxy_async_smem();
     __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&sm.bars.q_full));
+    if (lane == 0) mbar_arrive(smem_u32(&sm.q_full));
 
     const int s = warp >> 2, r = (warp & 3) * 32 + lane, pos = pos0 + r, wpos = pos0 + (warp & 3) * 32, lo = first_key(a, pos);
     const int w_lo = first_key(a, wpos), w_all = first_key(a, wpos + 31);
-    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16, ts = tmem + s * GROUP + lanes;
-#pragma unroll 1
-    for (int it = s; it < n; it += 2) {
-      const int j0 = jb + it * KEYS;
-      if (!warp_wait(smem_u32(&sm.bars.s_full[s]), (it >> 1) & 1, dead)) break;
-      tcgen05_fence_after();
-      const bool seen = j0 <= wpos + 31 && j0 + KEYS - 1 >= w_lo, partly = j0 + KEYS - 1 > wpos || j0 < w_all;         // by some row of the warp; not by every row, not every key
-      float top = -INFINITY;
-      if (seen) {
-#pragma unroll 1
-        for (int c = 0; c < KEYS; c += CH) {
-          uint32_t u[3][CH];
-#pragma unroll
-          for (int k = 0; k < 3; ++k) tmem_ld32(ts + k * KEYS + c, u[k]);
-          tmem_ld_wait();
-          f32x2 sc[CH / 2];
-#pragma unroll
-          for (int i = 0; i < CH / 2; ++i) {
-            f32x2 v[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) v[k] = pack2(__uint_as_float(u[k][2 * i]), __uint_as_float(u[k][2 * i + 1]));
-            sc[i] = add2(add2(v[0], v[1]), v[2]);
-          }
-          finish_pairs(sc, mul, a, slope, pos - j0 - c);
-#pragma unroll
-          for (int i = 0; i < CH / 2; ++i) {
-            float x, y;
-            unpack2(sc[i], x, y);
-            u[0][2 * i] = __float_as_uint(x), u[0][2 * i + 1] = __float_as_uint(y);
-          }
-          if (partly) {
-#pragma unroll
-            for (int e = 0; e < CH; ++e)
-              if (j0 + c + e > pos || j0 + c + e < lo) u[0][e] = 0xff800000u;
-          }
-          float t[4] = {top, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-          for (int e = 0; e < CH; ++e) t[e & 3] = fmaxf(t[e & 3], __uint_as_float(u[0][e]));
-          top = fmaxf(fmaxf(t[0], t[1]), fmaxf(t[2], t[3]));
-          tmem_st32(ts + c, u[0]);
-        }
-        tmem_st_wait();
-      }
-      float before = -INFINITY;
-      if (it > 0) {
-        if (!warp_wait(smem_u32(&sm.bars.m_full[s ^ 1][warp & 3]), ((it - 1) >> 1) & 1, dead)) break;
-        before = sm.top[s ^ 1][r];
-      }
-      top = fmaxf(top, before);
-      sm.top[s][r] = top;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&sm.bars.m_full[s][warp & 3]));
-      const float from = top == -INFINITY ? 0.f : top;             // no key seen so far
-      f32x2 sum[2] = {0ull, 0ull};
-      if (seen) {
-#pragma unroll 1
-        for (int c = 0; c < KEYS; c += CH) {
-          uint32_t u[CH], p[3][CH / 2];
-          tmem_ld32(ts + c, u);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < CH / 2; ++i) {
-            const f32x2 w = exp_pair(add2(pack2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1])), both(-from)));
-            sum[i & 1] = add2(sum[i & 1], w);
-            float x, y;
-            unpack2(w, x, y);
-            p[0][i] = pack_bf16x2(x, y);                           // split3_finite (mma.cuh)
-            unpack_bf16x2(p[0][i], x, y);
-            const f32x2 rest = fma2(pack2(x, y), both(-1.f), w);
-            unpack2(rest, x, y);
-            p[1][i] = pack_bf16x2(x, y);
-            unpack_bf16x2(p[1][i], x, y);
-            unpack2(fma2(pack2(x, y), both(-1.f), rest), x, y);
-            p[2][i] = pack_bf16x2(x, y);
-          }
-#pragma unroll
-          for (int k = 0; k < 3; ++k) tmem_st16(ts + WEIGHTS + k * 32 + c / 2, p[k]);
-        }
-      } else {
-        const uint32_t none[16] = {};
-#pragma unroll
-        for (int c = 0; c < 96; c += 16) tmem_st16(ts + WEIGHTS + c, none);
-      }
-      float x, y;
-      unpack2(add2(sum[0], sum[1]), x, y);
-      sm.add[it & 3][r] = make_float2(expf(before - from), x + y);
-      tmem_st_wait();
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&sm.bars.p_full[s]));
-    }
+    softmax_blocks(sm, tmem, s, n, jb, pos, lo, wpos, w_lo, w_all, [&](f32x2 (&sc)[CH / 2], int j) { finish_pairs(sc, mul, a, slope, pos - j); });
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SUM_REGS));
-    const int r = (warp & 3) * 32 + lane;
-    const uint32_t to = tmem + SUMS + ((uint32_t)((warp & 3) * 32) << 16);
+    const int r0 = (warp & 3) * 32;
     f32x2 O[D / 2];
-    float l = 0.f;
-    bool alive = true;
+    double l;
+    const bool alive = sum_blocks(sm, tmem, n, O, l);
+    const float inv = alive ? 1.0f / ((float)l + (x.sink ? expf(x.sink[h] - sm.top[(n - 1) & 1][r0 + lane]) : 0.f)) : NAN;
+    // (the keys' and values' place: every product is done)
+    const unsigned again = rows_out(raw + (ks - smem_u32(raw)) + (warp & 3) * (32 * D * 4), O, inv, rows - r0, [&](int i, float4 y) {
+      const size_t row = row0 + r0 + i, at = (row * a.H + h) * D + lane * 4;
+      if (a.gate_mode != 0) {
+        float g[4];
 #pragma unroll
-    for (int c = 0; c < D / 2; ++c) O[c] = 0ull;
-#pragma unroll 1
-    for (int it = 0; it < n; ++it) {
-      if (!(alive = warp_wait(smem_u32(&sm.bars.o_full), it & 1, dead))) break;
-      tcgen05_fence_after();
-      const float2 add = sm.add[it & 3][r];
-      l = fmaf(l, add.x, add.y);
-#pragma unroll
-      for (int c = 0; c < D; c += 32) {
-        uint32_t v[32];
-        tmem_ld32(to + c, v);
-        tmem_ld_wait();
-        if (c == D - 32) {
-          tcgen05_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&sm.bars.o_empty));
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) O[c / 2 + i] = fma2(O[c / 2 + i], both(add.x), pack2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));
+        for (int k = 0; k < 4; ++k) g[k] = gate_of<bf16>(x, a, row, h, lane * 4 + k);
+        y = make_float4(y.x * g[0], y.y * g[1], y.z * g[2], y.w * g[3]);
       }
-    }
-    // A warp's 32 rows by way of shared memory (the keys' and values' place: every product is done), so that neighbouring lanes write neighbouring columns; little code, for it is run once.
-    uint8_t* place = raw + (ks - smem_u32(raw)) + (warp & 3) * (32 * D * 4);
-#pragma unroll
-    for (int c = 0; c < D; c += 4) {
-      float4 y;
-      unpack2(O[c / 2], y.x, y.y);
-      unpack2(O[c / 2 + 1], y.z, y.w);
-      reinterpret_cast<float4*>(place)[lane * (D / 4) + ((c / 4) ^ (lane & 7))] = y;
-    }
-    f32x2 probe[4] = {0ull, 0ull, 0ull, 0ull};                     // NaN if a sum is not finite
-#pragma unroll
-    for (int c = 0; c < D / 2; ++c) probe[c & 3] = fma2(O[c], 0ull, probe[c & 3]);
-    float p0, p1;
-    unpack2(add2(add2(probe[0], probe[1]), add2(probe[2], probe[3])), p0, p1);
-    const unsigned again = __ballot_sync(0xffffffffu, r < rows && alive && p0 + p1 != 0.f);
-    const float inv = alive ? 1.0f / (l + (x.sink ? expf(x.sink[h] - sm.top[(n - 1) & 1][r]) : 0.f)) : NAN;
-    __syncwarp();
-    const int last = rows - (warp & 3) * 32;
-    auto put = [&](int i, float4 y) {
-      const size_t at = ((size_t)(row0 + (warp & 3) * 32 + i) * a.H + h) * D + lane * 4;
-      if (i >= last || ((again >> i) & 1u)) return;
       if (a.out_f32) *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + at) = y;
       else *reinterpret_cast<uint2*>(out + at) = make_uint2(pack_bf16x2(y.x, y.y), pack_bf16x2(y.z, y.w));
-    };
-#pragma unroll 1
-    for (int i0 = 0; i0 < 32; i0 += 8) {
-      float4 y[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        y[i] = reinterpret_cast<const float4*>(place)[(i0 + i) * (D / 4) + (lane ^ i)];
-        const float f = __shfl_sync(0xffffffffu, inv, i0 + i);
-        y[i] = make_float4(y[i].x * f, y[i].y * f, y[i].z * f, y[i].w * f);
-      }
-      if (a.gate_mode != 0) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          if (i0 + i >= last) break;
-          float g[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) g[k] = gate_of<bf16>(x, a, row0 + (warp & 3) * 32 + i0 + i, h, lane * 4 + k);
-          y[i] = make_float4(y[i].x * g[0], y[i].y * g[1], y[i].z * g[2], y[i].w * g[3]);
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) put(i0 + i, y[i]);
-    }
-    if (again) {
+    });
+    if (alive && again) {
 #pragma unroll 1
       for (int i = 0; i < 32; ++i)
-        if ((again >> i) & 1u) by_itself(row0 + (warp & 3) * 32 + i, slot, pos0 + (warp & 3) * 32 + i);
+        if ((again >> i) & 1u) by_itself(row0 + r0 + i, slot, pos0 + r0 + i);
     }
   }
-  if (__syncthreads_or(*dead)) {                                   // products in flight end before shared memory and TMEM are given back
-    if (tid == 0) atomicAdd_system(timeouts, 1);
-    if (warp == 15 && lane == 0) {
-      volatile int none = 0;
-      tcgen05_commit(smem_u32(&sm.bars.drain));
-      wait_for(smem_u32(&sm.bars.drain), 0u, &none);
-    }
-  }
-  leave();
+  leave(sm, tmem, warp, timeouts);
 }
 
 template <int NQ>
@@ -540,10 +363,7 @@ int launch(const void* q, int ldq, const bf16* kcache, long long kss, const bf16
   constexpr int smem = smem_bytes<NQ>();
   static_assert(smem <= 232448, "shared memory budget exceeded");
   LIA_CUDA(cudaFuncSetAttribute(window_prompt_tc_kernel<NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  static const bool split_fits = [] {                              // the registers that the warps trade must be those that the block gets
-    cudaFuncAttributes at{};
-    return cudaFuncGetAttributes(&at, window_prompt_tc_kernel<NQ>) == cudaSuccess && at.numRegs * THREADS >= 128 * (2 * SOFTMAX_REGS + SUM_REGS + OTHER_REGS);
-  }();
+  static const bool split_fits = registers_suffice(window_prompt_tc_kernel<NQ>);
   LIA_CHECK_ARG(split_fits, "lia_window_attn_mma: built with another number of registers");
   int* timeouts = lia_timeout_word();
   LIA_CHECK_ARG(timeouts != nullptr, "lia_window_attn_mma: no host memory for the count of timeouts");

@@ -1,0 +1,55 @@
+"""Latent portions over expanded keys on tcgen05 (csrc/latent_attn_sm100.cu) against a float64 softmax: portions of 1 to 300 rows beside each other behind 0 to 500 positions (blocks of 32 keys to
+the third turn of the ring, tiles of 128 rows, a portion's last block beside the next portion's rows), windows, sinks, gates, scales of either sign and near 0, both outputs, and a workspace
+that holds a group of heads."""
+import math
+
+import pytest
+import torch
+
+import lia_b200  # noqa: F401
+from lia_b200 import ops
+
+pytestmark = pytest.mark.gpu
+BF16, F32, F64 = torch.bfloat16, torch.float32, torch.float64
+DIM, ROT, RANK = 128, 64, 64
+PORTIONS = [(1, 0, 0, 300), (0, 500, 300, 129), (2, 31, 429, 1), (3, 0, 430, 33)]        # slot, first position, first row, rows
+# scores of size 5 carry about 5 * 2^-23 * sqrt(192) of relative error through exp: below 1e-5 of the largest value with room to spare
+TOL = 1e-5
+
+
+def reference(q, qr, lat, w, H, scale, window, sink, gate):
+    out = torch.zeros(q.shape[0], H, DIM, dtype=F64, device="cuda")
+    for slot, p0, r0, n in PORTIONS:
+        c, pos, j = lat[slot, :p0 + n].to(F64), torch.arange(p0, p0 + n, device="cuda")[:, None], torch.arange(p0 + n, device="cuda")[None, :]
+        seen = (j <= pos) & ((pos - j < window) if window else True)
+        for h in range(H):
+            k, v = (c[:, :RANK] @ w[(t * H + h) * DIM:(t * H + h + 1) * DIM].to(F64).T for t in (0, 1))
+            s = (q[r0:r0 + n].view(n, H, DIM + ROT)[:, h, :DIM].to(F64) @ k.T + qr[r0:r0 + n, h].to(F64) @ c[:, RANK:].T) * scale
+            s = s.masked_fill(~seen, -math.inf)
+            if sink is not None:
+                s = torch.cat([s, sink[h].to(F64).expand(n, 1)], 1)
+            out[r0:r0 + n, h] = torch.softmax(s, -1)[:, :p0 + n] @ v
+    return (out * gate[:, :, None].to(F64) if gate is not None else out).reshape(q.shape[0], -1)
+
+
+@pytest.mark.parametrize("H,window,scale,sink,gate", [(2, 0, 0.1, False, False), (5, 40, 0.1, True, True), (3, 200, -0.1, False, True), (1, 0, 0.0, True, False), (2, 33, 1e-9, False, False)])
+def test_portions(H, window, scale, sink, gate):
+    g = torch.Generator().manual_seed(H)
+    rnd = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    M = PORTIONS[-1][2] + PORTIONS[-1][3]
+    q, qr = rnd(M, H * (DIM + ROT)).to(BF16).cuda(), rnd(M, H, ROT).cuda()
+    lat, w = rnd(4, 640, RANK + ROT).to(BF16).cuda(), (rnd(2 * H * DIM, RANK) * RANK ** -0.5).to(BF16).cuda()
+    for slot, p0, _, n in PORTIONS:
+        lat[slot, p0 + n:] = float("nan")                           # what lies behind a sequence's last position is never read
+    sk, gt = (rnd(H).cuda() if sink else None), (torch.rand(M, H, generator=g).cuda() if gate else None)
+    want = reference(q, qr, lat, w, H, scale, window, sk, gt)
+
+    def run(dtype, portions=PORTIONS, **kw):
+        out = torch.full((M, H * DIM), 7.0, dtype=dtype, device="cuda")
+        return ops.latent_attn_expanded(q, qr, lat, portions, w, gt, out, H, DIM, ROT, RANK, scale, window=window, sink=sk, **kw)
+    out = run(F32)
+    assert float((out.to(F64) - want).abs().max() / want.abs().max()) < TOL
+    assert float((run(BF16).to(F64) - want).abs().max() / want.abs().max()) < 2.0 ** -8
+    assert torch.equal(run(F32, room=700), out)                     # heads in turn: the same sums
+    for slot, p0, r0, n in PORTIONS:                                # a portion does not depend on its company
+        assert torch.equal(run(F32, [(slot, p0, r0, n)])[r0:r0 + n], out[r0:r0 + n])
