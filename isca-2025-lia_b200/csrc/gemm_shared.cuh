@@ -682,7 +682,6 @@ struct Plan {
   int grid;      // CTAs
   int streamk;   // SWAP: split tiles across CTAs at k-block granularity
   int tiles_a, tiles_b, k_blocks;
-  int split;     // NORMAL: CTAs of a cluster that share a tile's K (gemm_split_sm100.cuh)
 };
 
 // CTAs available to one GEMM launch: the SM count, or LIA_GEMM_MAX_CTAS when set (lets two launches that
@@ -707,7 +706,6 @@ bool pair_enabled() {
 Plan make_plan(int M, int N, int K, bool allow_pair = false) {
   Plan pl;
   pl.pair = false;
-  pl.split = 1;
   const int sms = gemm_cta_budget();
   pl.k_blocks = (K + BLOCK_K - 1) / BLOCK_K;
   pl.swap = (M <= 128);
@@ -738,7 +736,7 @@ Plan make_plan(int M, int N, int K, bool allow_pair = false) {
     if (env && atoi(env) == 0) pl.streamk = 0;
     if (!pl.streamk && pl.grid > pl.tiles_a) pl.grid = pl.tiles_a;
   } else {
-    // Whole tiles along K whatever the width, with the same bits, but where a few rows leave most SMs idle (below).  256-wide tiles, by CTA
+    // Whole tiles along K whatever the width, so that a row's result does not depend on how many rows are computed with it.  256-wide tiles, by CTA
     // pairs from 512 rows on, leave SMs idle where a prompt is short or the matrix narrow; a CTA's time per k-block is what its ring of stages
     // takes to refill (192 KB in flight), so narrower tiles cost less each: measured 0.50 / 0.33 / 0.25 us per k-block for 256 / 128 / 64 columns,
     // 0.38 us for a pair.  The width with the shortest rounds is taken (231 x 2560 x 10240: 20 tiles of 256 in 63 us, 80 of 64 in 37; 231 x
@@ -765,32 +763,12 @@ Plan make_plan(int M, int N, int K, bool allow_pair = false) {
         pl.bn = atoi(env);
         pl.pair = pl.pair && pl.bn == 256;
       }
-      // Tiles that leave SMs idle: their K in 2 to 8 parts (gemm_split_sm100.cuh), where one round of that is shorter by a tenth.  Estimates in ns from a sweep of 14 shapes at 129 to 1000 rows:
-      // a tile's parts cost 250 | 380 a k-block (128 | 256 columns) and 8000 | 10000 for the fill, the meeting and the end, whole tiles 215 | 245 | 500 (64 | 128 | 256; a pair 380)
-      // and 3300.  us, whole -> parts: 231 x 2560 x 10240 38 -> 22, 231 x 2048 x 8192 31 -> 16, 231 x 4096 x 16384 56 -> 38, 231 x 768 x 3072 14 -> 8, 512 x 2560 x 10240 42 -> 29;
-      // whole stays 231 x 2048 x 2048 (11.6, 9.9 in 4 parts), 640 x 2048 x 2048 (13.8, 13.9), 640 x 2560 x 10240 (42, 37).  A row's sums depend on the parts, and so on how many rows are computed with it.
-      const bool as_pair = pairs && pl.bn == 256;
-      const long long whole = as_pair ? cost(tiles(2 * TILE_A, 256), sms / 2, 380) : cost(tiles(TILE_A, pl.bn), sms, pl.bn == 256 ? 500 : pl.bn == 128 ? 245 : 215);
-      long long least = (whole * pl.k_blocks + 3300) * 9 / 10;
-      const char* e2 = getenv("LIA_GEMM_SPLIT");                   // tuning/debug override: parts; 1 = whole tiles
-      for (int bn = 128; bn <= 256; bn += 128)
-        for (int parts = 2; parts <= (bn == 256 ? 4 : 8); ++parts) {
-          const long long ctas = tiles(TILE_A, bn) * parts, part = (pl.k_blocks + parts - 1) / parts;
-          const long long took = part * (bn == 256 ? 380 : 250) + (bn == 256 ? 10000 : 8000);
-          const bool fits = pl.k_blocks >= 4 * parts && ctas <= sms * (parts == 2 || parts == 4 ? 14 : parts == 3 ? 13 : 12) / 16;       // clusters that are resident together
-          if (e2 ? atoi(e2) == parts && pl.k_blocks >= parts && (env ? atoi(env) == bn : pl.split == 1) : !env && fits && took < least) {
-            least = took;
-            pl.split = parts;
-            pl.bn = bn;
-            pl.pair = false;
-          }
-        }
     }
     pl.tiles_a = pl.pair ? (M + 2 * TILE_A - 1) / (2 * TILE_A) : (M + TILE_A - 1) / TILE_A;
     pl.tiles_b = (N + pl.bn - 1) / pl.bn;
     const int units = pl.tiles_a * pl.tiles_b;
     if (pl.pair) pl.grid = 2 * (units < sms / 2 ? units : sms / 2);
-    else pl.grid = pl.split > 1 ? units * pl.split : units < sms ? units : sms;
+    else pl.grid = units < sms ? units : sms;
   }
   return pl;
 }

@@ -33,7 +33,6 @@
 #include "common.cuh"
 #include "umma.cuh"
 #include "gemm_shared.cuh"
-#include "gemm_split_sm100.cuh"
 #include "linear_rows_mma.cuh"
 
 namespace {
@@ -681,7 +680,6 @@ static int gemm_impl(const void* A, const void* W, const void* bias, const void*
   } else {
     if ((rc = make_tmap(&tmA, A, M, K, TILE_A)) != LIA_OK) return rc;
     if ((rc = make_tmap(&tmB, W, N, K, pl.pair ? pl.bn / 2 : pl.bn)) != LIA_OK) return rc;
-    if (pl.split > 1) return pl.bn == 256 ? launch_split<256, 4>(pl, tmA, tmB, ep, stream) : launch_split<128, 6>(pl, tmA, tmB, ep, stream);
     if (pl.pair) return launch_pair<256>(pl, tmA, tmB, ep, stream);
     if (pl.bn == 256) return launch<false, 256, 4>(pl, tmA, tmB, ep, ws, flags, stream);
     if (pl.bn == 64) return launch_tp<false, 64, 8, false>(pl, tmA, tmB, ep, ws, flags, stream);

@@ -308,7 +308,7 @@ static int* timeout_word(bool make) {
 }
 int* lia_timeout_word() { return timeout_word(true); }             // for the kernels of other files
 
-/* CTAs of the tcgen05 kernels with bounded waits (lia_moe_gemm_tc, lia_ssd_scan_chunks, prompts of lia_window_attn_mma, lia_gemm_bf16 by parts of K) that gave up one, as far as launches have ended, since the library was loaded */
+/* CTAs of the tcgen05 kernels with bounded waits (lia_moe_gemm_tc, lia_ssd_scan_chunks, prompts of lia_window_attn_mma and lia_latent_attn_expanded) that gave up one, as far as launches have ended, since the library was loaded */
 extern "C" int lia_moe_timeouts_seen(void) {
   const volatile int* word = timeout_word(false);
   return word ? *word : 0;
