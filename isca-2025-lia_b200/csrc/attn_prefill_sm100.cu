@@ -101,7 +101,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                  o_full = bar_base + 144, o_empty = bar_base + 152;
   volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(smem_gen + L::BAR_OFF + L::NUM_BARS * 8);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
 
   if (warp == QK_PRODUCER_WARP && lane == 0) {
@@ -133,7 +133,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_ptr_smem;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_smem, 0);
   pdl_launch_dependents();
 
   auto load_tile = [&](const CUtensorMap* map, uint32_t dst, int col0, int row0, uint32_t bar) {
@@ -179,7 +179,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // Q.K^T jobs run ahead of the softmax as far as the three score buffers allow (also into the NEXT item); P.V jobs are
     // issued the moment the softmax warps have published a P tile.  Neither stream ever blocks the other: the thread
     // probes the barriers (mbarrier.test_wait) instead of waiting on them.
-    if (lane == 0) {
+    {
+      const uint32_t one = elect_one();
+      auto ready = [&](uint32_t bar, uint32_t parity) { return __shfl_sync(0xffffffffu, mbar_test(bar, parity) ? 1 : 0, 0) != 0; };      // the same answer for all lanes
       constexpr uint32_t idesc_qk = make_idesc(BM, BN);                   // A = Q (K-major), B = K (K-major)
       constexpr uint32_t idesc_pv = make_idesc(BM, D) | (1u << 16);       // A = P (K-major), B = V (MN-major)
       int q_idx = blockIdx.x, p_idx = blockIdx.x;
@@ -191,22 +193,22 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         bool progressed = false;
         if (!q_done) {
           const int ks = kc & 1, sb = sc % S_BUFS, qb = qn & 1;
-          if ((q_job > 0 || mbar_test(q_full(qb), (qn >> 1) & 1)) && mbar_test(k_full(ks), (kc >> 1) & 1) &&
-              mbar_test(s_empty(sb), ((sc / S_BUFS) & 1) ^ 1u)) {
+          if ((q_job > 0 || ready(q_full(qb), (qn >> 1) & 1)) && ready(k_full(ks), (kc >> 1) & 1) &&
+              ready(s_empty(sb), ((sc / S_BUFS) & 1) ^ 1u)) {
             tcgen05_fence_after();
             const uint32_t qa = smem_base + L::Q_OFF + qb * L::TILE_BYTES, ka = smem_base + L::K_OFF + ks * L::TILE_BYTES;
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk) {
               const uint32_t off = (kk >> 2) * L::SLAB_BYTES + (kk & 3) * 32;   // 64-element slab; 16 elements = 32 bytes inside the swizzle row
-              tcgen05_mma_f16(tmem_base + sb * BN, make_smem_desc(qa + off), make_smem_desc(ka + off), idesc_qk, kk > 0 ? 1u : 0u);
+              mma_if(one, tmem_base + sb * BN, make_smem_desc(qa + off), make_smem_desc(ka + off), idesc_qk, kk > 0 ? 1u : 0u);
             }
-            tcgen05_commit(k_empty(ks));
-            tcgen05_commit(s_full(sb));
+            commit_if(one, k_empty(ks));
+            commit_if(one, s_full(sb));
             ++kc;
             ++sc;
             progressed = true;
             if (++q_job == qit.qk_jobs) {
-              tcgen05_commit(q_empty(qb));            // the Q buffer is free once this item's last Q.K^T has read it
+              commit_if(one, q_empty(qb));            // the Q buffer is free once this item's last Q.K^T has read it
               q_job = 0;
               ++qn;
               q_idx += gridDim.x;
@@ -216,22 +218,22 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           }
         }
         if (!p_done) {
-          if (mbar_test(p_full, pc & 1) && mbar_test(v_full, vc & 1) && (p_blk > 0 || mbar_test(o_empty, (pn & 1) ^ 1u))) {
+          if (ready(p_full, pc & 1) && ready(v_full, vc & 1) && (p_blk > 0 || ready(o_empty, (pn & 1) ^ 1u))) {
             tcgen05_fence_after();
             const uint32_t pa = smem_base + L::P_OFF, va = smem_base + L::V_OFF;
 #pragma unroll
             for (int kk = 0; kk < BN / 16; ++kk) {
               const uint64_t dp = make_smem_desc(pa + (kk >> 2) * L::SLAB_BYTES + (kk & 3) * 32);
               const uint64_t dv = make_smem_desc_mn(va + kk * 16 * 128, L::SLAB_BYTES);   // 16 keys = 16 rows of 128 bytes
-              tcgen05_mma_f16(tmem_base + L::O_COL, dp, dv, idesc_pv, (p_blk > 0 || kk > 0) ? 1u : 0u);
+              mma_if(one, tmem_base + L::O_COL, dp, dv, idesc_pv, (p_blk > 0 || kk > 0) ? 1u : 0u);
             }
-            tcgen05_commit(v_empty);
-            tcgen05_commit(p_empty);
+            commit_if(one, v_empty);
+            commit_if(one, p_empty);
             ++vc;
             ++pc;
             progressed = true;
             if (++p_blk == pit.nblk) {
-              tcgen05_commit(o_full);
+              commit_if(one, o_full);
               p_blk = 0;
               ++pn;
               p_idx += gridDim.x;

@@ -69,25 +69,6 @@ __device__ __forceinline__ f32x2 pow2_pair(f32x2 v, float c, float c_rest, float
 }
 __device__ __forceinline__ f32x2 exp_pair(f32x2 x) { return pow2_pair(x, 1.44269502162933349609f, 1.92596299e-8f, -150.f); }
 
-__device__ __forceinline__ uint32_t elect_one() {
-  uint32_t one;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
-  return one;
-}
-__device__ __forceinline__ void mma_if(uint32_t one, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc),
-               "r"(accumulate), "r"(one)
-               : "memory");
-}
-__device__ __forceinline__ void mma_tmem_a_if(uint32_t one, uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc),
-               "r"(accumulate), "r"(one)
-               : "memory");
-}
-__device__ __forceinline__ void commit_if(uint32_t one, uint32_t bar) {
-  if (one) tcgen05_commit(bar);
-}
-
 // The warp's number in its group of four, known to be the same in all lanes (addresses in TMEM are the warp's)
 __device__ __forceinline__ int group_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5) & 3, 0); }
 // by one thread

@@ -736,33 +736,31 @@ Plan make_plan(int M, int N, int K, bool allow_pair = false) {
     if (env && atoi(env) == 0) pl.streamk = 0;
     if (!pl.streamk && pl.grid > pl.tiles_a) pl.grid = pl.tiles_a;
   } else {
-    // Whole tiles along K whatever the width, so that a row's result does not depend on how many rows are computed with it.  256-wide tiles, by CTA
-    // pairs from 512 rows on, leave SMs idle where a prompt is short or the matrix narrow; a CTA's time per k-block is what its ring of stages
-    // takes to refill (192 KB in flight), so narrower tiles cost less each: measured 0.50 / 0.33 / 0.25 us per k-block for 256 / 128 / 64 columns,
-    // 0.38 us for a pair.  The width with the shortest rounds is taken (231 x 2560 x 10240: 20 tiles of 256 in 63 us, 80 of 64 in 37; 231 x
-    // 4096 x 16384: 99 and 56 us; 500 x 7680 x 2560 stays at 256: 22 us, 23 with 128, 37 with 64).
+    // Whole tiles along K whatever the width, so that a row's result does not depend on how many rows are computed with it (a prompt's tokens not on the minibatches it is taken in).  256-wide
+    // tiles, by CTA pairs from 512 rows on, leave SMs idle where a prompt is short or the matrix narrow: 128 or 64 columns, by the shortest estimate.  A round takes 130 | 190 | 320 ns a k-block (64 |
+    // 128 | 256 columns; a pair 290) and 200 | 1800 | 5900 (6200) once: fitted to a sweep of 38 matrices from 1024 x 1024 to 20480 x 5120 at 150 to 4096 rows (299 points), in which the choice never
+    // lost 4 % to the best width and 0.08 % on average.  us, 256 wide | 128 | 64: 256 rows of 2560 x 10240 64 | 37 | 27; 2048 x 2048 15 | 11 | 9; 12288 x 2560 26 | 24 | 37; 7168 x 7168 52 | 33 | 40;
+    // 1792 rows of 8192 x 2048 48 | 53 | 68, of 2048 x 2048 21 | 19 | 23.
     auto tiles = [&](int rows, int cols) { return (long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols); };
-    auto cost = [&](long long n, int workers, int ns) { return (n + workers - 1) / workers * ns; };
+    auto rounds = [&](long long n, int workers) { return (n + workers - 1) / workers; };
     const bool wide = N % 256 == 0 || N >= 2048;
+    const bool pairs = allow_pair && wide && M >= 4 * TILE_A && sms >= 2;          // as the default has it, so that one-CTA runs for comparison take the same widths
     pl.bn = wide ? 256 : 128;
-    pl.pair = allow_pair && wide && M >= 4 * TILE_A && sms >= 2 && pair_enabled();
+    pl.pair = pairs && pair_enabled();
     if (allow_pair) {
-      const bool pairs = wide && M >= 4 * TILE_A && sms >= 2;      // as the default has it, so that one-CTA runs for comparison take the same widths
-      long long best = pairs ? cost(tiles(2 * TILE_A, 256), sms / 2, 380) : cost(tiles(TILE_A, pl.bn), sms, pl.bn == 256 ? 500 : 330);
-      if (wide && cost(tiles(TILE_A, 128), sms, 330) * 10 < best * 9) {
-        best = cost(tiles(TILE_A, 128), sms, 330);
-        pl.bn = 128;
-        pl.pair = false;
-      }
-      if (cost(tiles(TILE_A, 64), sms, 250) * 10 < best * 9) {
-        pl.bn = 64;
-        pl.pair = false;
-      }
       const char* env = getenv("LIA_GEMM_BN");                     // tuning/debug override
-      if (env && (atoi(env) == 64 || atoi(env) == 128 || atoi(env) == 256)) {
-        pl.bn = atoi(env);
-        pl.pair = pl.pair && pl.bn == 256;
-      }
+      const int only = env && (atoi(env) == 64 || atoi(env) == 128 || atoi(env) == 256) ? atoi(env) : 0;
+      long long least = -1;
+      auto offer = [&](int bn, bool pair, long long ns) {
+        if ((only && bn != only) || (least >= 0 && ns >= least)) return;
+        least = ns;
+        pl.bn = bn;
+        pl.pair = pair && pair_enabled();
+      };
+      if (pairs) offer(256, true, rounds(tiles(2 * TILE_A, 256), sms / 2) * pl.k_blocks * 290 + 6200);
+      else if (wide || only == 256) offer(256, false, rounds(tiles(TILE_A, 256), sms) * pl.k_blocks * 320 + 5900);
+      offer(128, false, rounds(tiles(TILE_A, 128), sms) * pl.k_blocks * 190 + 1800);
+      offer(64, false, rounds(tiles(TILE_A, 64), sms) * pl.k_blocks * 130 + 200);
     }
     pl.tiles_a = pl.pair ? (M + 2 * TILE_A - 1) / (2 * TILE_A) : (M + TILE_A - 1) / TILE_A;
     pl.tiles_b = (N + pl.bn - 1) / pl.bn;

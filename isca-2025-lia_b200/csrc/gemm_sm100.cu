@@ -58,7 +58,7 @@ lia_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
   auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + 2 + a); };
   volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(smem_gen + L::BAR_OFFSET + (2 * STAGES + 4) * 8);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) stamp(trace, 0);
 
@@ -94,7 +94,7 @@ lia_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
   __syncthreads();
   if (PAIR) cluster_sync_all();   // the peer's barriers are initialised before anything arrives on them
   tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_ptr_smem;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_smem, 0);
   if (threadIdx.x == 0) stamp(trace, 1);
   // PDL: from here on the next kernel in the stream may become resident; this kernel touches nothing a
   // predecessor produced until pdl_wait() (only weight tiles are fetched before it, see the producer)
@@ -156,7 +156,8 @@ lia_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     }
   } else if (warp == 1) {
     // ===================== MMA issuer =====================
-    if (lane == 0 && cta_rank == 0) {
+    if (cta_rank == 0) {
+      const uint32_t one = elect_one();
       constexpr uint32_t idesc = make_idesc(PAIR ? 2 * TILE_A : TILE_A, BN);
       int stage = 0;
       uint32_t phase = 0;
@@ -172,7 +173,7 @@ lia_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         for (int kb = w.kb0; kb < w.kb1; ++kb) {
           mbar_wait(full_bar(stage), phase);
           if (first_full) {
-            stamp(trace, 3);
+            if (one) stamp(trace, 3);
             first_full = false;
           }
           tcgen05_fence_after();
@@ -182,19 +183,21 @@ lia_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
 #pragma unroll
           for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
             // advance 16 elements = 32 bytes along K inside the 128-byte swizzle row: +2 in the >>4 address field
-            if (PAIR) tcgen05_mma_f16_pair(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > w.kb0 || k > 0) ? 1u : 0u);
-            else tcgen05_mma_f16(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > w.kb0 || k > 0) ? 1u : 0u);
+            if (PAIR) mma_pair_if(one, d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > w.kb0 || k > 0) ? 1u : 0u);
+            else mma_if(one, d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > w.kb0 || k > 0) ? 1u : 0u);
           }
-          if (PAIR) tcgen05_commit_pair(empty_bar(stage));   // frees the stage in BOTH CTAs
-          else tcgen05_commit(empty_bar(stage));   // frees the smem stage when these MMAs have read it
+          if (PAIR) {
+            if (one) tcgen05_commit_pair(empty_bar(stage));   // frees the stage in BOTH CTAs
+          } else commit_if(one, empty_bar(stage));   // frees the smem stage when these MMAs have read it
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        if (PAIR) tcgen05_commit_pair(tfull_bar(acc));   // each CTA's epilogue drains its own 128 rows
-        else tcgen05_commit(tfull_bar(acc));       // accumulator complete -> epilogue
-        stamp(trace, 4);
+        if (PAIR) {
+          if (one) tcgen05_commit_pair(tfull_bar(acc));   // each CTA's epilogue drains its own 128 rows
+        } else commit_if(one, tfull_bar(acc));       // accumulator complete -> epilogue
+        if (one) stamp(trace, 4);
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
       }

@@ -70,7 +70,7 @@ __device__ __forceinline__ void st_shared16(uint32_t addr, uint32_t a, uint32_t 
 }
 
 // The products of two operands in three parts each: part of A (bits 0-1), first part of B (2-3) and how many of its parts (4-5), which accumulator (6-7), whether it begins that (8).
-// (The instructions are issued by one lane from loops: unrolled they would not fit into the instruction cache beside the other warps' code.)
+// (The instructions are issued from loops: unrolled they would not fit into the instruction cache beside the other warps' code.)
 constexpr int product_code(int a, int b, int parts, int to, int first) { return a | b << 2 | parts << 4 | to << 6 | first << 8; }
 __constant__ int PRODUCTS[7] = {product_code(2, 0, 1, 2, 1), product_code(2, 1, 1, 2, 0), product_code(1, 2, 1, 2, 0), product_code(1, 1, 1, 1, 1), product_code(1, 0, 1, 1, 0),
                                 product_code(0, 0, 1, 0, 1), product_code(0, 1, 2, 1, 0)};
@@ -83,7 +83,7 @@ struct Operand {
   uint64_t at;
   uint32_t part, slab, step;
 };
-template <bool tmem_a> __device__ __forceinline__ void issue(const int* codes, int count, uint32_t d, const Operand& A, const Operand& B, int width, uint32_t major) {
+template <bool tmem_a> __device__ __forceinline__ void issue(uint32_t one, const int* codes, int count, uint32_t d, const Operand& A, const Operand& B, int width, uint32_t major) {
 #pragma unroll 1
   for (int i = 0; i < count; ++i) {
     const int code = codes[i];
@@ -95,8 +95,8 @@ template <bool tmem_a> __device__ __forceinline__ void issue(const int* codes, i
     for (int half = 0; half < 2; ++half, a += A.slab, b += B.slab) {
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        if constexpr (tmem_a) mma_tmem_a(to, (uint32_t)a + k * A.step, b + k * B.step, idesc, accumulate);
-        else tcgen05_mma_f16(to, a + k * A.step, b + k * B.step, idesc, accumulate);
+        if constexpr (tmem_a) mma_tmem_a_if(one, to, (uint32_t)a + k * A.step, b + k * B.step, idesc, accumulate);
+        else mma_if(one, to, a + k * A.step, b + k * B.step, idesc, accumulate);
         accumulate = 1u;
       }
     }
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) ssd_states_kernel(const SsdArgs
   extern __shared__ uint8_t raw[];
   const uint32_t base = (smem_u32(raw) + 1023u) & ~1023u, xs = base + 3 * TILE;
   StSmem& sm = *reinterpret_cast<StSmem*>(raw + (base - smem_u32(raw)) + 3 * TILE + 6 * UNIT);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   volatile int* dead = &sm.dead;
   if (tid == 0) {
     sm.dead = sm.bad_all = 0;
@@ -362,22 +362,22 @@ __global__ void __launch_bounds__(ST_THREADS, 1) ssd_states_kernel(const SsdArgs
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem = sm.tmem;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem, 0);
 
   if (warp == 12) {
-    if (lane == 0) {
-      constexpr uint32_t mn = (1u << 15) | (1u << 16);             // both operands lie with the contracted tokens as rows
-      for (int j = 0; j < units; ++j) {
-        const int b = j & 1;
-        const uint32_t parity = (j >> 1) & 1;
-        if (!wait_for(smem_u32(&sm.bars.x_full[b]), parity, dead) || !wait_for(smem_u32(&sm.bars.acc_empty[b]), parity ^ 1u, dead)) break;
-        mbar_arrive(smem_u32(&sm.bars.scaled[b]));
-        tcgen05_fence_after();
-        const uint32_t d = tmem + b * 192, xb = xs + b * 3 * UNIT;
-        issue<false>(PRODUCTS, 7, d, Operand{make_smem_desc_mn(base, TILE / 2), TILE >> 4, 512, 128}, Operand{make_smem_desc_mn(xb, UNIT), UNIT >> 4, 512, 128}, 64, mn);
-        tcgen05_commit(smem_u32(&sm.bars.x_empty[b]));
-        tcgen05_commit(smem_u32(&sm.bars.acc_full[b]));
-      }
+    const uint32_t one = elect_one();
+    constexpr uint32_t mn = (1u << 15) | (1u << 16);               // both operands lie with the contracted tokens as rows
+#pragma unroll 1
+    for (int j = 0; j < units; ++j) {
+      const int b = j & 1;
+      const uint32_t parity = (j >> 1) & 1;
+      if (!warp_wait(smem_u32(&sm.bars.x_full[b]), parity, dead) || !warp_wait(smem_u32(&sm.bars.acc_empty[b]), parity ^ 1u, dead)) break;
+      if (one) mbar_arrive(smem_u32(&sm.bars.scaled[b]));
+      tcgen05_fence_after();
+      const uint32_t d = tmem + b * 192, xb = xs + b * 3 * UNIT;
+      issue<false>(one, PRODUCTS, 7, d, Operand{make_smem_desc_mn(base, TILE / 2), TILE >> 4, 512, 128}, Operand{make_smem_desc_mn(xb, UNIT), UNIT >> 4, 512, 128}, 64, mn);
+      commit_if(one, smem_u32(&sm.bars.x_empty[b]));
+      commit_if(one, smem_u32(&sm.bars.acc_full[b]));
     }
   } else if (warp >= 4) {
     const int th = tid - 128;
@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
   extern __shared__ uint8_t raw[];
   const uint32_t base = (smem_u32(raw) + 1023u) & ~1023u, second = base + 3 * TILE, ss = second, xs = second + 2 * S_HALF;
   OutSmem& sm = *reinterpret_cast<OutSmem*>(raw + (base - smem_u32(raw)) + 6 * TILE);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   volatile int* dead = &sm.dead;
   if (tid == 0) {
     sm.dead = 0;
@@ -616,13 +616,14 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem = sm.tmem, acc = tmem + 192;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem, 0), acc = tmem + 192;
   const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
   bool alive = true;
 
-  if (warp == 4 && lane == 0) {
-    issue<false>(SINGLES, 8, tmem, Operand{make_smem_desc(base), TILE >> 4, TILE >> 5, 2}, Operand{make_smem_desc(second), TILE >> 4, TILE >> 5, 2}, 128, 0u);
-    tcgen05_commit(smem_u32(&sm.bars.cb_full));
+  const uint32_t one = elect_one();
+  if (warp == 4) {
+    issue<false>(one, SINGLES, 8, tmem, Operand{make_smem_desc(base), TILE >> 4, TILE >> 5, 2}, Operand{make_smem_desc(second), TILE >> 4, TILE >> 5, 2}, 128, 0u);
+    commit_if(one, smem_u32(&sm.bars.cb_full));
   }
   __syncwarp();
   for (int j = warp - 8; warp >= 8 && j < units; j += 8) {       // while C B^T is made
@@ -718,20 +719,20 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
       tmem_st_wait();
       tcgen05_fence_before();
       __syncwarp();
-      if (lane == 0 && alive)
-        for (int j = 0; j < units; ++j) {
-          const uint32_t parity = j & 1;
-          if (!wait_for(smem_u32(&sm.bars.s_full), parity, dead) || !wait_for(smem_u32(&sm.bars.intra_read), parity ^ 1u, dead)) break;
-          mbar_arrive(smem_u32(&sm.bars.inter_scaled));
-          tcgen05_fence_after();
-          issue<false>(PRODUCTS, 7, acc, Operand{make_smem_desc(base), TILE >> 4, TILE >> 5, 2}, Operand{make_smem_desc(ss), P * 128 >> 4, S_HALF >> 4, 2}, 64, 0u);
-          tcgen05_commit(smem_u32(&sm.bars.inter_full));
-          if (!wait_for(smem_u32(&sm.bars.x_full), parity, dead) || !wait_for(smem_u32(&sm.bars.inter_read), parity, dead) || !wait_for(smem_u32(&sm.bars.w_full), parity, dead)) break;
-          mbar_arrive(smem_u32(&sm.bars.intra_scaled));
-          tcgen05_fence_after();
-          issue<true>(PRODUCTS, 7, acc, Operand{tmem, 64, 32, 8}, Operand{make_smem_desc_mn(xs, UNIT), UNIT >> 4, 512, 128}, 64, 1u << 16);
-          tcgen05_commit(smem_u32(&sm.bars.intra_full));
-        }
+#pragma unroll 1
+      for (int j = 0; alive && j < units; ++j) {
+        const uint32_t parity = j & 1;
+        if (!warp_wait(smem_u32(&sm.bars.s_full), parity, dead) || !warp_wait(smem_u32(&sm.bars.intra_read), parity ^ 1u, dead)) break;
+        if (one) mbar_arrive(smem_u32(&sm.bars.inter_scaled));
+        tcgen05_fence_after();
+        issue<false>(one, PRODUCTS, 7, acc, Operand{make_smem_desc(base), TILE >> 4, TILE >> 5, 2}, Operand{make_smem_desc(ss), P * 128 >> 4, S_HALF >> 4, 2}, 64, 0u);
+        commit_if(one, smem_u32(&sm.bars.inter_full));
+        if (!warp_wait(smem_u32(&sm.bars.x_full), parity, dead) || !warp_wait(smem_u32(&sm.bars.inter_read), parity, dead) || !warp_wait(smem_u32(&sm.bars.w_full), parity, dead)) break;
+        if (one) mbar_arrive(smem_u32(&sm.bars.intra_scaled));
+        tcgen05_fence_after();
+        issue<true>(one, PRODUCTS, 7, acc, Operand{tmem, 64, 32, 8}, Operand{make_smem_desc_mn(xs, UNIT), UNIT >> 4, 512, 128}, 64, 1u << 16);
+        commit_if(one, smem_u32(&sm.bars.intra_full));
+      }
       __syncwarp();
     } else
     for (int j = 0; j < units; ++j) {                              // (the two warps of a row meet at barriers whether alive or not)

@@ -184,6 +184,32 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* v) {
       "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
       : "memory");
 }
+// Products issued by a whole warp, of whose lanes one has `one` set.  With warp numbers and addresses that are known to be the same in all lanes (__shfl_sync) an instruction takes 50 to 65 clocks;
+// from a lane by itself, whose operands are moved to uniform registers one after the other, 115.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one;
+}
+__device__ __forceinline__ void mma_if(uint32_t one, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc),
+               "r"(accumulate), "r"(one)
+               : "memory");
+}
+__device__ __forceinline__ void mma_tmem_a_if(uint32_t one, uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc),
+               "r"(accumulate), "r"(one)
+               : "memory");
+}
+__device__ __forceinline__ void commit_if(uint32_t one, uint32_t bar) {
+  if (one) tcgen05_commit(bar);
+}
+
+__device__ __forceinline__ void mma_pair_if(uint32_t one, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc),
+               "r"(accumulate), "r"(one)
+               : "memory");
+}
 __device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // K-major SWIZZLE_128B shared-memory matrix descriptor (UMMA SmemDescriptor):
