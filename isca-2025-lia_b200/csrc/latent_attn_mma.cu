@@ -1,5 +1,5 @@
 // Latent attention (latent_attn.cu) of portions of sequences on the tensor cores.  The rows of a portion share their keys, so the other
-// order of the two projections is less work: Wuk and Wuv are applied once to the latents the portion sees (linear_mma.cu), and the rows attend to
+// order of the two projections is less work: Wuk and Wuv are applied once to the latents the portion sees (latent_expand_sm100.cu; latents of more than 512 or no whole 64 numbers: linear_mma.cu), and the rows attend to
 // per-head keys and values -- 320 instead of 1088 multiply-adds per (row, key, head) at heads of 128 + 64 channels and latents of 512.  Nothing
 // is held in fewer bits than in the latent space, where the carried queries, the weights and the weighted latents are fp32: the expanded keys
 // and values are kept as three bf16 parts of their fp32 sums, and so are the rotated query parts and the softmax's weights (mma.cuh).  With bf16
@@ -8,7 +8,7 @@
 // Heads of 128 + 64 channels are latent_attn_sm100.cu's.  Here, for heads of 64 + 64, one block per (64 rows, head), warp by 16 rows, the scores becoming the weights' operand in registers; 32 keys
 // per stage.  Keys and values are fetched in turn (the next keys while the values are taken in, the next values while the scores are made), so one stage is enough and several blocks share an SM.
 // Bound: tensor cores and shared-memory reads about equally.  2048 tokens, 16 heads of 128 + 64 on latents of 512: 4794 us in the latent space on the CUDA cores and 439 us for its two projections ->
-// 352 here (104 there) and 67 us for the expansion.
+// 352 here (104 there) and 67 us for the expansion (29: latent_expand_sm100.cu).
 // Rows whose sums are not finite are formed again key by key at the end, as in window_attn_mma.cu: a masked key's weight of 0 still meets its value.
 #include <limits.h>
 #include <math.h>
@@ -18,6 +18,9 @@
 
 int latent_expanded_tc(const ExpandedArgs& a, int tiles, long long latents, cudaStream_t stream);      // latent_attn_sm100.cu
 
+// latent_expand_sm100.cu
+bool latent_expand_takes(long long slot_stride, int D, int K, int N, int part);
+int latent_expand(const bf16* cache, int D, const long long* first, const int* rows, int n, const bf16* W, bf16* C, long long ldc, int N, int K, int part, cudaStream_t stream);
 // linear_mma.cu
 int linear_mma_parts(const bf16* const* src, const int* rows, int n, long long lda, const bf16* W, bf16* C, long long ldc, int N, int K, int part, cudaStream_t stream);
 
@@ -330,6 +333,7 @@ extern "C" int lia_latent_attn_expanded_in(const void* q, int ldq, const float* 
   for (int first = 0; first < np;) {
     ExpandedArgs a{reinterpret_cast<const bf16*>(q), qr, reinterpret_cast<const bf16*>(workspace), gate, sink, out, D, ldq, qr_stride, H, 0, 0, window, out_f32, 0, scale, {}};
     const bf16* src[MAX_PORTIONS];
+    long long at[MAX_PORTIONS];                                    // the same as rows of the cache
     int rows[MAX_PORTIONS], tiles = 0;
     long long latents = 0;
     while (first < np && a.np < MAX_PORTIONS) {
@@ -339,6 +343,7 @@ extern "C" int lia_latent_attn_expanded_in(const void* q, int ldq, const float* 
       if (i > 0 && ((size_t)(latents + seen) * H > room || latents + seen > INT_MAX)) break;
       src[i] = reinterpret_cast<const bf16*>(cache) + (size_t)p[0] * slot_stride + (size_t)base * D;
       rows[i] = seen;
+      at[i] = (long long)p[0] * (slot_stride / D) + base;
       a.p[i] = Portion{src[i] + kv_rank, p[2], p[3], p[1] - base, (int)latents, tiles};
       tiles += (p[3] + tile_rows - 1) / tile_rows;
       latents += seen;
@@ -353,12 +358,16 @@ extern "C" int lia_latent_attn_expanded_in(const void* q, int ldq, const float* 
     for (a.h0 = 0; a.h0 < H; a.h0 += a.nh) {
       a.nh = most < H - a.h0 ? most : H - a.h0;
       const long long ldc = 6ll * a.nh * dim;
+      const bool tc = latent_expand_takes(slot_stride, D, kv_rank, a.nh * dim, dim);
+      auto expand = [&](const bf16* w, bf16* to, int N) {
+        return tc ? latent_expand(reinterpret_cast<const bf16*>(cache), D, at, rows, a.np, w, to, ldc, N, kv_rank, dim, stream) : linear_mma_parts(src, rows, a.np, D, w, to, ldc, N, kv_rank, dim, stream);
+      };
       int rc;
       if (a.nh == H) {
-        rc = linear_mma_parts(src, rows, a.np, D, wk, ws, ldc, 2 * H * dim, kv_rank, dim, stream);
+        rc = expand(wk, ws, 2 * H * dim);
       } else {
-        rc = linear_mma_parts(src, rows, a.np, D, wk + (size_t)a.h0 * dim * kv_rank, ws, ldc, a.nh * dim, kv_rank, dim, stream);
-        if (rc == LIA_OK) rc = linear_mma_parts(src, rows, a.np, D, wk + (size_t)(H + a.h0) * dim * kv_rank, ws + (size_t)3 * a.nh * dim, ldc, a.nh * dim, kv_rank, dim, stream);
+        rc = expand(wk + (size_t)a.h0 * dim * kv_rank, ws, a.nh * dim);
+        if (rc == LIA_OK) rc = expand(wk + (size_t)(H + a.h0) * dim * kv_rank, ws + (size_t)3 * a.nh * dim, a.nh * dim);
       }
       if (rc == LIA_OK) rc = dim == 128 ? latent_expanded_tc(a, tiles, latents, stream) : run<64, 64>(a, tiles, stream);
       if (rc != LIA_OK) return rc;

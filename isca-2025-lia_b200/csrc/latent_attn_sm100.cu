@@ -12,8 +12,9 @@
 // Sums that are not finite stay so to the end, where such rows are formed again key by key: a masked key's weight of 0 still meets its value.
 // Waits are bounded: a CTA that gives up leaves NaN and counts itself (lia_moe_timeouts_seen()).
 //
-// Latents of 512, with their expansion; on mma.sync -> here, us, and the error against 64 bits in 1e-7: 2048 rows, 16 heads 419 (1.97) -> 171 (1.93); 700 rows behind 300, 32 heads 251 (2.21) -> 135
-// (2.15); portions of 300, 250 and 200, 16 heads 89 (1.75) -> 54 (1.74); 64 rows 29 (1.61) -> 25 (1.52); 100 rows behind 1500, 32 heads 377 (2.31) -> 178 (2.41), 8 heads 210 (2.31) -> 111 (2.30).
+// Latents of 512, with their expansion (latent_expand_sm100.cu); on mma.sync -> here, us, and the error against 64 bits in 1e-7: 2048 rows, 16 heads 419 (1.97) -> 132 (1.84); 700 rows behind 300,
+// 32 heads 251 (2.21) -> 98 (2.07); portions of 300, 250 and 200, 16 heads 89 (1.75) -> 38 (1.61); 64 rows 29 (1.61) -> 15 (1.42); 100 rows behind 1500, 32 heads 377 (2.31) -> 123 (2.35), 8 heads 210
+// (2.31) -> 90 (2.26).
 #include "attn_sm100.cuh"
 #include "latent_attn_rows.cuh"
 
@@ -94,8 +95,9 @@ __global__ void __launch_bounds__(THREADS, 1) latent_expanded_tc_kernel(const __
         const uint32_t one = elect_one();
         const bool of_keys = warp == LOADER0;
         const int col = (of_keys ? 0 : a.nh * 3 * DN) + blockIdx.x * 3 * DN, row = pt.part0 + jb;
+        int it = 0;
 #pragma unroll 1
-        for (int it = 0; it < n; ++it) {
+        for (; it < n; ++it) {
           const uint32_t full = smem_u32(of_keys ? &sm.k_full[it & 1] : &sm.v_full[it & 1]), empty = smem_u32(of_keys ? &sm.k_empty[it & 1] : &sm.v_empty[it & 1]);
           if (!warp_wait(empty, ((it >> 1) & 1) ^ 1u, dead)) break;
           if (!one) continue;
@@ -107,6 +109,10 @@ __global__ void __launch_bounds__(THREADS, 1) latent_expanded_tc_kernel(const __
 #pragma unroll
             for (int k = 0; k < 2; ++k) tma_load_2d(at + k * slab, &map, col + part * DN + k * 64, row + it * KEYS, full);
           }
+        }
+        if (*dead && one) {                                        // loads in flight end before shared memory is given back
+          volatile int none = 0;
+          for (int t = max(0, it - 2); t < it; ++t) wait_for(smem_u32(of_keys ? &sm.k_full[t & 1] : &sm.v_full[t & 1]), (t >> 1) & 1, &none);
         }
       }
     } else {

@@ -1,6 +1,6 @@
 """Latent portions over expanded keys on tcgen05 (csrc/latent_attn_sm100.cu) against a float64 softmax: portions of 1 to 300 rows beside each other behind 0 to 500 positions (blocks of 32 keys to
 the third turn of the ring, tiles of 128 rows, a portion's last block beside the next portion's rows), windows, sinks, gates, scales of either sign and near 0, both outputs, and a workspace
-that holds a group of heads."""
+that holds a group of heads; and the expansion (csrc/latent_expand_sm100.cu) of latents of 64 to 512 numbers, beside those it leaves to mma.sync."""
 import math
 
 import pytest
@@ -53,3 +53,18 @@ def test_portions(H, window, scale, sink, gate):
     assert torch.equal(run(F32, room=700), out)                     # heads in turn: the same sums
     for slot, p0, r0, n in PORTIONS:                                # a portion does not depend on its company
         assert torch.equal(run(F32, [(slot, p0, r0, n)])[r0:r0 + n], out[r0:r0 + n])
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("rank", [64, 128, 192, 448, 512, 576, 72])
+def test_expansion(dim, rank):
+    """One row that sees one latent gives back its value, the sum of its three parts."""
+    H, slots, cap = 3, 2, 140
+    g = torch.Generator().manual_seed(rank)
+    lat = torch.randn(slots, cap, rank + ROT, generator=g).to(BF16).cuda()
+    w = (torch.randn(2 * H * dim, rank, generator=g) * rank ** -0.5).to(BF16).cuda()
+    q, qr = torch.zeros(cap, H * (dim + ROT), dtype=BF16, device="cuda"), torch.zeros(cap, H, ROT, device="cuda")
+    out = torch.empty(cap, H * dim, dtype=F32, device="cuda")
+    ops.latent_attn_expanded(q, qr, lat, [(1, 0, 0, cap)], w, None, out, H, dim, ROT, rank, 1.0, window=1)
+    want = lat[1, :, :rank].to(F64) @ w[H * dim:].to(F64).T
+    assert float((out.to(F64) - want).abs().max()) < 2.0 ** -20      # sums of size up to 5: a few last places of 2^-21
