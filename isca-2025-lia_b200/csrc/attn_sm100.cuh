@@ -185,8 +185,10 @@ __device__ __forceinline__ bool sum_blocks(AttnTail& sm, uint32_t tmem, int n, f
 }
 
 // A warp's 32 rows by way of 16 KB of shared memory at `place`, times `inv` of their threads: put(i, y) for row i and columns 4 lane .. 4 lane + 3, for neighbouring lanes to write neighbouring
-// columns.  Returns the rows among the first `rows` whose sums are not finite.  (Little code: it is run once, and instructions come slowly then.)
-template <class Put> __device__ __forceinline__ unsigned rows_out(uint8_t* place, const f32x2 (&O)[D / 2], float inv, int rows, const Put& put) {
+// columns.  `gated`: get(i) asks for a row's gates, of eight rows together, and gate(y, g) applies them.  Returns the rows among the first `rows` whose sums are not finite.  (Little code, and what
+// is not needed in one piece to skip: it is run once, and instructions come slowly then.)
+template <class Get, class Gate, class Put>
+__device__ __forceinline__ unsigned rows_out(uint8_t* place, const f32x2 (&O)[D / 2], float inv, int rows, bool gated, const Get& get, const Gate& gate, const Put& put) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int c = 0; c < D; c += 4) {
@@ -210,6 +212,13 @@ template <class Put> __device__ __forceinline__ unsigned rows_out(uint8_t* place
       y[i] = reinterpret_cast<const float4*>(place)[(i0 + i) * (D / 4) + (lane ^ i)];
       const float f = __shfl_sync(0xffffffffu, inv, i0 + i);
       y[i] = make_float4(y[i].x * f, y[i].y * f, y[i].z * f, y[i].w * f);
+    }
+    if (gated) {
+      uint2 g[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) g[i] = i0 + i < rows ? get(i0 + i) : make_uint2(0u, 0u);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) gate(y[i], g[i]);
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i)

@@ -11,7 +11,8 @@
 // Waits are bounded: a CTA that gives up leaves NaN and counts itself (lia_moe_timeouts_seen()).
 //
 // 8 key heads of 128; on mma.sync -> here, us, and the error against 64 bits in 1e-7: 2048 rows, 16 heads, window of 1024 and soft cap 136 (1.87) -> 66 (1.68), the whole history and fp32 queries
-// 182 (2.42) -> 63 (1.69); 700 rows behind 300 91 (2.43) -> 35 (2.16); portions of 300, 250, 200 31 (1.54) -> 17 (1.49); 64 rows 9.3 (1.37) -> 9.4 (1.19).
+// 182 (2.42) -> 63 (1.69); 700 rows behind 300 91 (2.43) -> 35 (2.16); portions of 300, 250, 200 31 (1.54) -> 17 (1.49); 64 rows 9.3 (1.37) -> 9.1 (1.19);
+// 33 rows 8.7 (1.18) -> 9.0 (0.97).  Four portions of 117, 100, 87, 73 behind a gate per channel: 24 -> 15 (33 with the gates asked for row by row).
 #include "attn_sm100.cuh"
 #include "window_attn_rows.cuh"
 
@@ -337,14 +338,26 @@ __global__ void __launch_bounds__(THREADS, 1) window_prompt_tc_kernel(const void
     const bool alive = sum_blocks(sm, tmem, n, O, l);
     const float inv = alive ? 1.0f / ((float)l + (x.sink ? expf(x.sink[h] - sm.top[(n - 1) & 1][r0 + lane]) : 0.f)) : NAN;
     // (the keys' and values' place: every product is done)
-    const unsigned again = rows_out(raw + (ks - smem_u32(raw)) + (warp & 3) * (32 * D * 4), O, inv, rows - r0, [&](int i, float4 y) {
-      const size_t row = row0 + r0 + i, at = (row * a.H + h) * D + lane * 4;
-      if (a.gate_mode != 0) {
-        float g[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) g[k] = gate_of<bf16>(x, a, row, h, lane * 4 + k);
-        y = make_float4(y.x * g[0], y.y * g[1], y.z * g[2], y.w * g[3]);
+    const bool gate_pairs = a.gate_mode == 2 && (reinterpret_cast<uintptr_t>(x.gate) | (uintptr_t)(a.ldg * 2)) % 8 == 0;
+    auto gates = [&](int i) {                                      // four of a row's gates before their sigmoid, or the head's
+      const size_t row = row0 + r0 + i;
+      if (a.gate_mode == 1) return make_uint2(__float_as_uint(reinterpret_cast<const float*>(x.gate)[row * a.H + h]), 0u);
+      const unsigned short* g = reinterpret_cast<const unsigned short*>(x.gate) + row * a.ldg + (size_t)h * D + lane * 4;
+      return gate_pairs ? *reinterpret_cast<const uint2*>(g) : make_uint2(g[0] | (uint32_t)g[1] << 16, g[2] | (uint32_t)g[3] << 16);
+    };
+    auto gate = [&](float4& y, uint2 u) {
+      float4 g;
+      if (a.gate_mode == 1) {
+        g.x = g.y = g.z = g.w = __uint_as_float(u.x);
+      } else {
+        unpack_bf16x2(u.x, g.x, g.y);
+        unpack_bf16x2(u.y, g.z, g.w);
+        g = make_float4(1.0f / (1.0f + expf(-g.x)), 1.0f / (1.0f + expf(-g.y)), 1.0f / (1.0f + expf(-g.z)), 1.0f / (1.0f + expf(-g.w)));
       }
+      y = make_float4(y.x * g.x, y.y * g.y, y.z * g.z, y.w * g.w);
+    };
+    const unsigned again = rows_out(raw + (ks - smem_u32(raw)) + (warp & 3) * (32 * D * 4), O, inv, rows - r0, a.gate_mode != 0, gates, gate, [&](int i, float4 y) {
+      const size_t at = ((size_t)(row0 + r0 + i) * a.H + h) * D + lane * 4;
       if (a.out_f32) *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + at) = y;
       else *reinterpret_cast<uint2*>(out + at) = make_uint2(pack_bf16x2(y.x, y.y), pack_bf16x2(y.z, y.w));
     });
