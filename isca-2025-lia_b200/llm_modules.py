@@ -49,14 +49,18 @@ class _LinearFusionCUDA:
         return self._ws[m]
 
     def _rows(self, x):
-        return x.reshape(-1, x.shape[-1]).contiguous()
+        # (rows as they are go through without views of them: two of those and one of the result were 4 of a token's 15 us)
+        return x if x.dim() == 2 and x.is_contiguous() else x.reshape(-1, x.shape[-1]).contiguous()
+
+    def _shaped(self, o, x):
+        return o if x.dim() == 2 else o.view(*x.shape[:-1], self.weight.shape[0])
 
 
 class LinearReluCUDA(_LinearFusionCUDA):
     def __call__(self, x):
         r = self._rows(x)
         y = ops.gemm(r, self.weight, self.bias, epilogue=EPI_BIAS_RELU, workspace=self._workspace(r.shape[0]))
-        return y.view(*x.shape[:-1], self.weight.shape[0])
+        return self._shaped(y, x)
 
 
 class LinearAddCUDA(_LinearFusionCUDA):
@@ -64,7 +68,7 @@ class LinearAddCUDA(_LinearFusionCUDA):
         r = self._rows(x)
         o = ops.gemm(r, self.weight, self.bias, epilogue=EPI_BIAS_RESIDUAL, residual=self._rows(y),
                      workspace=self._workspace(r.shape[0]))
-        return o.view(*x.shape[:-1], self.weight.shape[0])
+        return self._shaped(o, x)
 
 
 class FastLayerNormCUDA:

@@ -180,7 +180,7 @@ _SM_COUNT = {}
 
 
 def _sm_count(device):
-    key = torch.device(device).index or 0
+    key = (device if isinstance(device, torch.device) else torch.device(device)).index or 0
     if key not in _SM_COUNT:
         _SM_COUNT[key] = torch.cuda.get_device_properties(key).multi_processor_count
     return _SM_COUNT[key]

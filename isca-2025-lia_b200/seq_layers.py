@@ -60,12 +60,17 @@ class Linear:
         self.weight = torch.zeros(n, self.K, dtype=dtype, device=device)
         for o, w in zip(self.offsets, ws):
             self.weight[o:o + w.shape[0]] = w
+        self._ws_bytes = {}
         self.dtype = dtype
         self.tensor_core = (dtype == BF16 and self.K % 8 == 0 and self.N % 8 == 0 and os.environ.get("LIA_PLAIN_LINEAR", "0") == "0")
 
     def _workspace(self, M, device):
+        # what a launch needs follows from the weights and from which width of token tiles M takes (csrc/gemm_shared.cuh); beyond 128 rows nothing: asked for once each
+        rows = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128 if M <= 128 else 129
+        need = self._ws_bytes.get(rows)
+        if need is None:
+            need = self._ws_bytes[rows] = ops.GemmWorkspace.bytes_for([(rows, self.N, self.K)])
         key = (device, M <= 128)
-        need = ops.GemmWorkspace.bytes_for([(M, self.N, self.K)])
         ws = Linear._gemm_ws.get(key)
         if ws is None or ws.buf.numel() < need:
             ws = Linear._gemm_ws[key] = ops.GemmWorkspace(need, device)
