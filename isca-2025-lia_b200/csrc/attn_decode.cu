@@ -27,7 +27,12 @@ __global__ void __launch_bounds__(THREADS) attn_decode_kernel(const bf16* __rest
   pdl_wait();
   constexpr int LPR = D / 8;        // lanes per cached row (each lane owns 8 dims = 16 bytes)
   constexpr int RPW = 32 / LPR;     // rows per warp iteration
-  constexpr int UNROLL = 4;
+  // Rows in flight per lane.  Ten take 72 registers, seven CTAs an SM and 143 KB in flight there.  B=64 H=56 d=128 T=289:
+  // 77.8 us (6.8 TB/s); with 4, 6, 8, 12: 80.7, 77.8, 82.3, 84.6.  B=16 H=32 d=64 T=300, where few CTAs leave each its own
+  // latency to wait for: 9.7 us; with 4, 6, 8, 12: 15.4, 15.6, 13.8, 11.0.  B=96 H=32 d=128: 68 us; 79, 74, 70, 85.
+  // Four at a time with a wait for all of them before the next four, and nothing in flight during the softmax, took 90.9, 18.0
+  // and 89.9 us.  Which row a lane adds, and in which order, does not depend on this number.
+  constexpr int UNROLL = 10;
   extern __shared__ float sc[];     // [t_chunk] scores -> probabilities
   __shared__ float red[4];
   __shared__ float accs[4][D];
@@ -48,27 +53,36 @@ __global__ void __launch_bounds__(THREADS) attn_decode_kernel(const bf16* __rest
   const size_t row_stride = (size_t)cache_batch * H * D;
   const size_t base = ((size_t)(b0 + b) * H + hh) * D + chunk * 8 + (size_t)t0 * row_stride;
 
+  // One list of rows, K's and then V's: a register is asked for again as soon as its row is used, so that UNROLL loads a lane
+  // are on their way at all times, during the softmax between the passes too.
+  constexpr int BATCH = 4 * RPW * UNROLL;
+  uint4 row[UNROLL];
+#pragma unroll
+  for (int j = 0; j < UNROLL; ++j) {
+    const int r = (j * 4 + warp) * RPW + rsub;
+    if (r < n) row[j] = ldg_stream(kc + base + (size_t)r * row_stride);
+  }
+
   // ---- phase A: s_t = bf16(q . k_t)
-  for (int i = 0; i < n; i += 4 * RPW * UNROLL) {
-    uint4 kv[UNROLL];
-    int r[UNROLL];
+  for (int i = 0; i < n; i += BATCH) {
+    const bool more = i + BATCH < n;
+    const bf16* next = more ? kc + base : vc + base;
 #pragma unroll
     for (int j = 0; j < UNROLL; ++j) {
-      r[j] = i + (j * 4 + warp) * RPW + rsub;
-      if (r[j] < n) kv[j] = ldg_stream(kc + base + (size_t)r[j] * row_stride);
-    }
-#pragma unroll
-    for (int j = 0; j < UNROLL; ++j) {
+      const int place = (j * 4 + warp) * RPW + rsub;
+      const int r = i + place;
       float dot = 0.f;
-      if (r[j] < n) {
+      if (r < n) {
         float kf[8];
-        unpack8(kv[j], kf);
+        unpack8(row[j], kf);
 #pragma unroll
         for (int e = 0; e < 8; ++e) dot = fmaf(qf[e], kf[e], dot);
       }
+      const int rn = more ? r + BATCH : place;
+      if (rn < n) row[j] = ldg_stream(next + (size_t)rn * row_stride);
 #pragma unroll
       for (int o = LPR / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-      if (chunk == 0 && r[j] < n) sc[r[j]] = bf16r(dot);
+      if (chunk == 0 && r < n) sc[r] = bf16r(dot);
     }
   }
   __syncthreads();
@@ -100,23 +114,18 @@ __global__ void __launch_bounds__(THREADS) attn_decode_kernel(const bf16* __rest
   float acc[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-  for (int i = 0; i < n; i += 4 * RPW * UNROLL) {
-    uint4 vv[UNROLL];
-    int r[UNROLL];
+  for (int i = 0; i < n; i += BATCH) {
 #pragma unroll
     for (int j = 0; j < UNROLL; ++j) {
-      r[j] = i + (j * 4 + warp) * RPW + rsub;
-      if (r[j] < n) vv[j] = ldg_stream(vc + base + (size_t)r[j] * row_stride);
-    }
-#pragma unroll
-    for (int j = 0; j < UNROLL; ++j) {
-      if (r[j] < n) {
-        const float pj = sc[r[j]];
+      const int r = i + (j * 4 + warp) * RPW + rsub;
+      if (r < n) {
+        const float pj = sc[r];
         float vf[8];
-        unpack8(vv[j], vf);
+        unpack8(row[j], vf);
 #pragma unroll
         for (int e = 0; e < 8; ++e) acc[e] = fmaf(pj, vf[e], acc[e]);
       }
+      if (r + BATCH < n) row[j] = ldg_stream(vc + base + (size_t)(r + BATCH) * row_stride);
     }
   }
 #pragma unroll
