@@ -16,9 +16,9 @@
 // The hi parts' products are summed per instruction (exact but for the last bits) and added in fp32; only the lower parts stay in the tensor cores' sums,
 // which truncate.  Against 64 bits, means over 6 to 10 inputs: 16 heads of 128 x 128, 1024 tokens: outputs off by 8.5e-8 (token loop: 12e-8), the state by 8e-8 (19e-8), 64
 // tokens: 7.8e-8 (8.0e-8) and 6.1e-8 (12e-8); gated, 4 heads of 256 x 512, 503 and 400 tokens: outputs' median 1.5e-7 (1.9e-7), state 1.15e-7 (1.2e-7), normaliser as there.
-// A chunk of 64 takes about 4 us, one after the other (a sequence's chunks cannot run at once): cutting the additions to half did not change that, so
-// the chain ldmatrix, mma, add and the two barriers bound it rather than the number of instructions.  A portion of 2048 tokens: 16 heads of 128 x 128
-// 533 -> 116 us, 4 heads of 256 x 512 878 -> 282.
+// A chunk of 64 takes about 3.5 us, one of 32 at 256 dims 4.1, one after the other (a sequence's chunks cannot run at once): cutting the additions to half did not
+// change that; the chain ldmatrix, mma, add, the two barriers and the instructions themselves bound it (thirteen warps run three programs; see the loops' unrolling).
+// A portion of 2048 tokens: 16 heads of 128 x 128 533 us by tokens, 111 here, 4 heads of 256 x 512 878 and 260.
 #include <math.h>
 
 #include "common.cuh"
@@ -71,6 +71,26 @@ template <int DIM, int L> struct ChunkSmem {
   alignas(16) int bad[2][COLS];                            // first token whose v is not finite
 };
 
+// Where a contracting warp's rows of the state begin in Q S, in steps of 16: a step is 12 instructions, a block of scores 2 KS and 12 more for its values, and
+// the warps of a row block that have fewer blocks of scores take more rows.
+template <int RB, int WPR, int KS> struct Shares {
+  int from[RB][WPR + 1];
+  constexpr Shares() : from{} {
+    for (int rb = 0; rb < RB; ++rb) {
+      int load[WPR] = {}, steps[WPR] = {};
+      for (int blk = 0; blk <= rb; ++blk) load[blk % WPR] += 2 * KS + 12;
+      for (int ks = 0; ks < KS; ++ks) {
+        int least = 0;
+        for (int i = 1; i < WPR; ++i)
+          if (load[i] < load[least]) least = i;
+        load[least] += 12, ++steps[least];
+      }
+      for (int i = 0; i < WPR; ++i) from[rb][i + 1] = from[rb][i] + steps[i];
+    }
+  }
+};
+template <int RB, int WPR, int KS> __constant__ Shares<RB, WPR, KS> shares_of{};
+
 // MLSTM: gates per token with a running-maximum stabiliser and a normaliser; else one decay per head, and the portions of SHORT to FEW - 1 tokens (few) or those of FEW and more.
 template <bool MLSTM, int DIM, int L, bool few = false>
 __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(ChunkArgs p) {
@@ -90,24 +110,20 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
   const int chunks = (len + L - 1) / L;
 
   const int aux = tid - MW * 32;
-  auto fetch = [&](int c) {                    // rows beyond the portion and columns beyond vdim are zero
+  constexpr int QC = DIM / 8, PIECES = 2 * L * QC / (MW * 32);
+  auto fetch_qk = [&](int c, int piece) {      // rows beyond the portion and columns beyond vdim are zero
+    const int b = c & 1, e = tid + piece * MW * 32, r = e / (2 * QC), j = e % (2 * QC), tok = c * L + r;
+    const bool live = tok < len;
+    const bf16* src = (j < QC ? qb + j * 8 : kb + (j - QC) * 8) + (live ? (size_t)tok * p.ldqk : 0);
+    cp_async16(smem_u32(j < QC ? &sm.q[b][r][j * 8] : &sm.k[b][r][(j - QC) * 8]), src, live ? 16 : 0);
+  };
+  auto fetch_v = [&](int c) {                  // the helping warps read V before the others do
     const int b = c & 1;
-    if (warp < MW) {
-      constexpr int QC = DIM / 8;
 #pragma unroll
-      for (int e = tid; e < 2 * L * QC; e += MW * 32) {
-        const int r = e / (2 * QC), j = e % (2 * QC), tok = c * L + r;
-        const bool live = tok < len;
-        const bf16* src = (j < QC ? qb + j * 8 : kb + (j - QC) * 8) + (live ? (size_t)tok * p.ldqk : 0);
-        cp_async16(smem_u32(j < QC ? &sm.q[b][r][j * 8] : &sm.k[b][r][(j - QC) * 8]), src, live ? 16 : 0);
-      }
-    } else if (aux < 128) {                    // the helping warps read V before the others do
-#pragma unroll
-      for (int e = aux; e < L * COLS / 8; e += 128) {
-        const int r = e / (COLS / 8), col = e % (COLS / 8) * 8, tok = c * L + r;
-        const bool live = tok < len && colb + col < vdim;
-        cp_async16(smem_u32(&sm.v[b][r][col]), live ? vb + (size_t)tok * p.ldv + col : p.v, live ? 16 : 0);
-      }
+    for (int e = aux; e < L * COLS / 8; e += 128) {
+      const int r = e / (COLS / 8), col = e % (COLS / 8) * 8, tok = c * L + r;
+      const bool live = tok < len && colb + col < vdim;
+      cp_async16(smem_u32(&sm.v[b][r][col]), live ? vb + (size_t)tok * p.ldv + col : p.v, live ? 16 : 0);
     }
     cp_async_commit();
   };
@@ -126,8 +142,8 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
     const float ig = next_i, fg = next_f;
     read_gates(c + 1);
     float before = m, after = m;
-#pragma unroll
-    for (int t = 0; t < 32; ++t) {
+#pragma unroll 4                               // (like the scores' loop: whole, these loops push each other's instructions out of the cache; 143 us for two
+    for (int t = 0; t < 32; ++t) {             // portions of 1003 tokens, 4 heads of 256 x 512, 132 so; by two and one at a time 136)
       const float f = __shfl_sync(0xffffffffu, fg, t), i = __shfl_sync(0xffffffffu, ig, t);
       const float next = t < n ? fmaxf(f + m, i) : m;
       if (lane == t) before = m, after = next;
@@ -136,7 +152,7 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
     if (c > 0) asm volatile("bar.sync 2, 160;" ::: "memory");           // the chunk before the last has left this chunk's buffers
     const float a = lane < n ? expf(fg + before - after) : 1.f, w = lane < n ? expf(ig - after) : 0.f;
     float prod = 0.f, all = 1.f, mine = 1.f;
-#pragma unroll
+#pragma unroll 4
     for (int t = 0; t < 32; ++t) {
       const float at = __shfl_sync(0xffffffffu, a, t);
       all *= at;
@@ -219,7 +235,13 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
           for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(&sm.s[i][mt * 16 + g + 8 * e][d0 + nt * 8 + 2 * t4]) = part[i];
         }
   };
-  fetch(0);
+  if (warp < MW) {
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) fetch_qk(0, i);
+    cp_async_commit();
+  } else if (aux < 128) {
+    fetch_v(0);
+  }
   if (warp < MW) {
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt)
@@ -254,19 +276,21 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
   if (warp >= MW && warp < MW + 4) weigh(0);
   __syncthreads();
 
-  const int rb = warp / WPR, share = warp % WPR;                 // (contracting warps) row block, and which part of its work
+  const int rb = warp < MW / 2 ? warp / WPR : RB - 1 - (warp - MW / 2) / WPR, share = warp % WPR;   // (contracting warps) row block, and which part of its work
+  const int ks0 = warp < MW ? shares_of<RB, WPR, KS>.from[rb][share] : 0, ks1 = warp < MW ? shares_of<RB, WPR, KS>.from[rb][share + 1] : 0;
   const int la = lane & 7, i0 = (lane >> 3) & 1, i1 = lane >> 4;  // ldmatrix: row within a matrix, and the matrix's place in two directions
   for (int c = 0; c < chunks; ++c) {
     const int b = c & 1, n = min(L, len - c * L);
-    if (c + 1 < chunks) fetch(c + 1);
+    const bool more = c + 1 < chunks;
     if (warp < MW) {
       const int blocks = (n + 15) >> 4;        // blocks of 16 tokens that hold any
       if (rb < blocks) {
         float acc[4][4] = {}, rest[4][4] = {}, sc[2][NB][2][4] = {};   // rest: what the lower parts give, small enough to stay in the tensor cores' sums
         // scores of this warp's blocks (rows rb, keys share, share + WPR, ..), and then its share of Q S
-#pragma unroll
+#pragma unroll 4
         for (int ks = 0; ks < KS; ++ks) {
           uint32_t qf[4], kf[4];
+          if (more && ks % (KS / PIECES) == 0) fetch_qk(c + 1, ks / (KS / PIECES));    // (then this chunk is a whole one: every warp comes by)
           ldsm_x4(smem_u32(&sm.q[b][rb * 16 + i0 * 8 + la][ks * 16 + i1 * 8]), qf);
 #pragma unroll
           for (int j = 0; j < NB; ++j) {
@@ -290,9 +314,9 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
             }
           }
         }
-#pragma unroll
-        for (int kk = 0; kk < KS / WPR; ++kk) {
-          const int ks = share * (KS / WPR) + kk;
+cp_async_commit();
+#pragma unroll 2
+        for (int ks = ks0; ks < ks1; ++ks) {
           uint32_t qf[4];
           ldsm_x4(smem_u32(&sm.q[b][rb * 16 + i0 * 8 + la][ks * 16 + i1 * 8]), qf);
 #pragma unroll
@@ -407,11 +431,12 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
 #pragma unroll
       for (int e = 0; e < 2 * NTU * 4; ++e) S[e / (NTU * 4)][e / 4 % NTU][e & 3] += low[e / (NTU * 4)][e / 4 % NTU][e & 3];
     } else if (MLSTM && warp == MW + 4) {
-      if (c + 1 < chunks) gates(c + 1);
+      if (more) gates(c + 1);
     } else {
+      if (more) fetch_v(c + 1);
       if (c > 0) output(c - 1);
-      if (MLSTM && c + 1 < chunks) asm volatile("bar.sync 2, 160;" ::: "memory");
-      else asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (MLSTM && more) asm volatile("bar.arrive 2, 160;" ::: "memory");
+      asm volatile("bar.sync 1, 128;" ::: "memory");
       if (aux < COLS) sm.bad[b ^ 1][aux] = L;
       if (MLSTM) {                             // q . n before the chunk, then n after it
         const int t = aux >> 2;
@@ -440,7 +465,7 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
           sm.n[2 * aux + 1] = fmaf(sm.total[b], sm.n[2 * aux + 1], x1);
         }
       }
-      if (c + 1 < chunks) {
+      if (more) {
         cp_async_wait<0>();                    // the helping warps' own copies: V
         if (MLSTM) asm volatile("bar.sync 3, 160;" ::: "memory");
         else asm volatile("bar.sync 1, 128;" ::: "memory");
