@@ -576,7 +576,8 @@ int lia_moe_plan_rows(const int* idx, int pairs, int E, int tile_rows, int n_til
  * lia_moe_tc_rows() rows; A [n_tiles * rows][K]: the rows in the plan's order.  up: C [n_tiles * rows][N] bf16 = act(sum), or gated (weights [E][2N][K], gate
  * rows before up rows): act(gate) * up, both sums in fp32; weigh_in: the sums are first multiplied by their pair's wt.  down: C bf16 in the plan's
  * order, unweighted, or (c_f32) C [pairs][N] fp32 by pair, times wt unless weigh_in.  Tiles of experts >= E are skipped.  K, N multiples of 8.
- * A wait inside that does not end within seconds ends its CTA, which leaves NaN where its results should be and is counted: lia_moe_timeouts_seen() reads the count
+ * A wait inside that does not end within seconds ends its CTA, which leaves NaN where its results should be and is counted, as are those of the state-space scan and of prompt
+ * attention over windows and expanded latents: lia_moe_timeouts_seen() reads the count
  * as far as launches have ended, lia_moe_timeouts() synchronises first. */
 int lia_moe_tc_rows(void);
 int lia_moe_timeouts(void);

@@ -20,7 +20,7 @@
 //   and row sum need no shuffles; warps w and w+4 share a lane quarter and split each score block by columns
 //   (keys 0-63 | 64-127), which doubles the issue slots available to the softmax; their partial (m, l) meet in shared
 //   memory once per item.  warp 8: TMA producer (Q once per item, K tiles for both passes, V tiles for pass 2; 2-stage
-//   rings).  warp 9: TMEM allocator + MMA issuer (one lane): scores are double-buffered in TMEM (2 x 128 columns) so
+//   rings).  warp 9: TMEM allocator + MMA issuer: scores are double-buffered in TMEM (2 x 128 columns) so
 //   Q K_{j+1}^T runs while the softmax warps work on block j; O takes `d` more columns.
 #include <stdlib.h>
 

@@ -8,7 +8,7 @@
 // Design (B200-first, not a translation of anything in the reference -- it has no GPU kernels):
 //   * one persistent CTA per SM, 256 threads, warp-specialised:
 //       warp 0  TMA producer   (cp.async.bulk.tensor, SWIZZLE_128B, mbarrier complete_tx)
-//       warp 1  MMA issuer     (one elected lane issues tcgen05.mma.cta_group::1.kind::f16)
+//       warp 1  MMA issuer     (the whole warp issues tcgen05.mma.cta_group::1.kind::f16 under an elected predicate)
 //       warp 2  TMEM allocator
 //       warps 4-7 epilogue     (tcgen05.ld -> regs -> smem staging -> coalesced 16-byte global I/O)
 //   * accumulators live in TMEM, double-buffered (2 x BN columns) so the epilogue of tile i

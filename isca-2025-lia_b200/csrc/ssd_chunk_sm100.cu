@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(CARRY, 4) ssd_carry_kernel(const SsdArgs p) {
 }
 
 // ------------------------------------------------------------------------------------------------ outputs
-// 512 threads.  Warps 0-7 but 4 make the weights (lane = token t; warps 0-3 the first 64 tokens s, 5-7 the others) from C B^T, one lane of warp 4, whose weights are all zero, issues,
+// 512 threads.  Warps 0-7 but 4 make the weights (lane = token t; warps 0-3 the first 64 tokens s, 5-7 the others) from C B^T, warp 4, whose weights are all zero, issues,
 // warps 8-11 put the outputs together, warps 12-15 split the units' states and x.  Shared memory: C | B, whose place the states and x take.
 // TMEM: weights 192 columns, accumulators 192, C B^T 128 (its parts before: 384).
 constexpr int OUT_THREADS = 512;

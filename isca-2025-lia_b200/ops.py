@@ -538,7 +538,7 @@ def latent_attn(qa, cache, meta, gate, out, H, kv_rank, rot, scale, max_ctx=0, w
 
 
 def _expanded_launches(seen, H, room):
-    """Launches of ``latent_attn_expanded`` (csrc/latent_attn_mma.cu) over portions that see so many latents."""
+    """Launches of ``latent_attn_expanded`` (csrc/latent_attn_mma.cu, csrc/latent_attn_sm100.cu) over portions that see so many latents."""
     n, count, latents = 0, 0, 0
     for s in seen + [None]:
         if count and (s is None or count == 16 or (latents + s) * H > room):
@@ -550,7 +550,7 @@ def _expanded_launches(seen, H, room):
 
 def latent_attn_expanded(q, qr, cache, portions, w_ukv, gate, out, H, dim, rot, kv_rank, scale, window=0, sink=None, room=1 << 18):
     """Attention of the rows of ``portions`` -- (slot, first position, first row, rows) each, host numbers -- over the latents they see, keys and values
-    expanded per head (csrc/latent_attn_mma.cu).  ``q`` [M, H * (dim + rot)] bf16; ``qr``: the turned query parts, a view [M, H, rot] of fp32;
+    expanded per head (csrc/latent_attn_sm100.cu for heads of 128 channels, csrc/latent_attn_mma.cu).  ``q`` [M, H * (dim + rot)] bf16; ``qr``: the turned query parts, a view [M, H, rot] of fp32;
     ``cache`` [slots, capacity, kv_rank + rot] bf16; ``w_ukv`` [2 H dim, kv_rank]: Wuk above Wuv.  ``out`` [M, H * dim] bf16 or fp32: only the
     portions' rows are written.  At most ``room`` (latent, head) pairs are expanded at a time (12 ``dim`` bytes each; fewer where memory is short), which changes
     no bit of the result."""
@@ -911,7 +911,7 @@ def window_attn(q, kcache, vcache, meta, temp, out, H, G, dim, vdim, window, sca
     block of ``chunk`` positions (blocks counted from the sequence's start).  ``v_div``: key head g reads value head g // v_div
     (the value cache holds G // v_div heads: several attention maps over one set of values).  ``segs`` int32 [nseg, 4] on the device
     (slot, first position, first row, rows): the portions whose rows these are; with them, or with one portion, a step of prompts on
-    bf16 caches runs on the tensor cores (csrc/window_attn_mma.cu), and so does a step of single tokens."""
+    bf16 caches runs on the tensor cores (csrc/window_attn_sm100.cu for heads of 128 channels, csrc/window_attn_mma.cu), and so does a step of single tokens."""
     ldq = _rowmajor(q, "q")
     _req(meta, "meta", I32)
     for t, n in ((temp, "temp"), (slopes, "slopes"), (sink, "sink")):
