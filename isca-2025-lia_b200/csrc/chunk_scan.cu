@@ -16,9 +16,9 @@
 // The hi parts' products are summed per instruction (exact but for the last bits) and added in fp32; only the lower parts stay in the tensor cores' sums,
 // which truncate.  Against 64 bits, means over 6 to 10 inputs: 16 heads of 128 x 128, 1024 tokens: outputs off by 8.5e-8 (token loop: 12e-8), the state by 8e-8 (19e-8), 64
 // tokens: 7.8e-8 (8.0e-8) and 6.1e-8 (12e-8); gated, 4 heads of 256 x 512, 503 and 400 tokens: outputs' median 1.5e-7 (1.9e-7), state 1.15e-7 (1.2e-7), normaliser as there.
-// A chunk of 64 takes about 3.5 us, one of 32 at 256 dims 4.1, one after the other (a sequence's chunks cannot run at once): cutting the additions to half did not
+// A chunk of 64 takes about 3.3 us, one of 32 at 256 dims 3.8, one after the other (a sequence's chunks cannot run at once): cutting the additions to half did not
 // change that; the chain ldmatrix, mma, add, the two barriers and the instructions themselves bound it (thirteen warps run three programs; see the loops' unrolling).
-// A portion of 2048 tokens: 16 heads of 128 x 128 533 us by tokens, 111 here, 4 heads of 256 x 512 878 and 260.
+// A portion of 2048 tokens: 16 heads of 128 x 128 533 us by tokens, 102 here, 4 heads of 256 x 512 878 and 241.
 #include <math.h>
 
 #include "common.cuh"
@@ -71,18 +71,20 @@ template <int DIM, int L> struct ChunkSmem {
   alignas(16) int bad[2][COLS];                            // first token whose v is not finite
 };
 
-// Where a contracting warp's rows of the state begin in Q S, in steps of 16: a step is 12 instructions, a block of scores 2 KS and 12 more for its values, and
-// the warps of a row block that have fewer blocks of scores take more rows.
+// Where a contracting warp's rows of the state begin in Q S, in steps of 16.  A step takes a warp some 330 clocks, a block of scores and its values 8 times that at 256 dims (the warps without one
+// have the inputs to ask for all the same), and the warps of a row block that have fewer blocks of scores take more steps: the chain of two portions of 1003 tokens, 4 heads of 256 x 512, 143 us
+// with four steps each, 140 with a block counted by its instructions (2 KS + 12, a step 12), 126 so.  Where two warps share a row block, six steps of one of them are a longer
+// chain of fp32 additions and put outputs off by 1.006 times as much: five at most.
 template <int RB, int WPR, int KS> struct Shares {
   int from[RB][WPR + 1];
   constexpr Shares() : from{} {
     for (int rb = 0; rb < RB; ++rb) {
       int load[WPR] = {}, steps[WPR] = {};
-      for (int blk = 0; blk <= rb; ++blk) load[blk % WPR] += 2 * KS + 12;
+      for (int blk = 0; blk <= rb; ++blk) load[blk % WPR] += 6 * KS + 12;
       for (int ks = 0; ks < KS; ++ks) {
-        int least = 0;
-        for (int i = 1; i < WPR; ++i)
-          if (load[i] < load[least]) least = i;
+        int least = -1;
+        for (int i = 0; i < WPR; ++i)
+          if ((WPR > 2 || steps[i] < 5) && (least < 0 || load[i] < load[least])) least = i;
         load[least] += 12, ++steps[least];
       }
       for (int i = 0; i < WPR; ++i) from[rb][i + 1] = from[rb][i] + steps[i];
@@ -142,8 +144,10 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
     const float ig = next_i, fg = next_f;
     read_gates(c + 1);
     float before = m, after = m;
-#pragma unroll 4                               // (like the scores' loop: whole, these loops push each other's instructions out of the cache; 143 us for two
-    for (int t = 0; t < 32; ++t) {             // portions of 1003 tokens, 4 heads of 256 x 512, 132 so; by two and one at a time 136)
+    // (like the scores' loop by four: whole, these loops push each other's instructions out of the cache.  Two portions of 1003 tokens, 4 heads of 256 x 512, before the warps' shares were as
+    // they are now: 139 us whole, 132 by four, 136 by two and one at a time)
+#pragma unroll 4
+    for (int t = 0; t < 32; ++t) {
       const float f = __shfl_sync(0xffffffffu, fg, t), i = __shfl_sync(0xffffffffu, ig, t);
       const float next = t < n ? fmaxf(f + m, i) : m;
       if (lane == t) before = m, after = next;
@@ -170,7 +174,7 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
   // the tile, and the column's outputs are NaN from its token on
   auto weigh = [&](int c) {
     const int b = c & 1, n = min(L, len - c * L);
-#pragma unroll 2
+#pragma unroll 4
     for (int e = aux; e < L * COLS / 2; e += 128) {
       const int s = e / (COLS / 2), col = (e - s * (COLS / 2)) * 2;
       uint32_t* src = reinterpret_cast<uint32_t*>(&sm.v[b][s][col]);
@@ -287,34 +291,39 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
       if (rb < blocks) {
         float acc[4][4] = {}, rest[4][4] = {}, sc[2][NB][2][4] = {};   // rest: what the lower parts give, small enough to stay in the tensor cores' sums
         // scores of this warp's blocks (rows rb, keys share, share + WPR, ..), and then its share of Q S
+        if (share <= rb) {
 #pragma unroll 4
-        for (int ks = 0; ks < KS; ++ks) {
-          uint32_t qf[4], kf[4];
-          if (more && ks % (KS / PIECES) == 0) fetch_qk(c + 1, ks / (KS / PIECES));    // (then this chunk is a whole one: every warp comes by)
-          ldsm_x4(smem_u32(&sm.q[b][rb * 16 + i0 * 8 + la][ks * 16 + i1 * 8]), qf);
+          for (int ks = 0; ks < KS; ++ks) {
+            uint32_t qf[4], kf[4];
+            if (more && ks % (KS / PIECES) == 0) fetch_qk(c + 1, ks / (KS / PIECES));    // (then this chunk is a whole one: every warp comes by)
+            ldsm_x4(smem_u32(&sm.q[b][rb * 16 + i0 * 8 + la][ks * 16 + i1 * 8]), qf);
 #pragma unroll
-          for (int j = 0; j < NB; ++j) {
-            const int kblk = share + j * WPR;
-            if (kblk > rb) continue;
-            ldsm_x4(smem_u32(&sm.k[b][kblk * 16 + i1 * 8 + la][ks * 16 + i0 * 8]), kf);
-            float st[2][4];
-            mma_bf16_first(st[0], qf, kf[0], kf[1]);
-            mma_bf16_first(st[1], qf, kf[2], kf[3]);
+            for (int j = 0; j < NB; ++j) {
+              const int kblk = share + j * WPR;
+              if (kblk > rb) continue;
+              ldsm_x4(smem_u32(&sm.k[b][kblk * 16 + i1 * 8 + la][ks * 16 + i0 * 8]), kf);
+              float st[2][4];
+              mma_bf16_first(st[0], qf, kf[0], kf[1]);
+              mma_bf16_first(st[1], qf, kf[2], kf[3]);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const float x = st[e >> 2][e & 3];
-              if constexpr (few) {           // what the sum rounds off, exactly (Knuth's two-sum), in a sum of its own
-                float& sum = sc[0][j][e >> 2][e & 3];
-                const float next = sum + x, back = next - sum;
-                sc[1][j][e >> 2][e & 3] += (sum - (next - back)) + (x - back);
-                sum = next;
-              } else {                                   // two chains: half the roundings each
-                sc[ks & 1][j][e >> 2][e & 3] += x;
+              for (int e = 0; e < 8; ++e) {
+                const float x = st[e >> 2][e & 3];
+                if constexpr (few) {           // what the sum rounds off, exactly (Knuth's two-sum), in a sum of its own
+                  float& sum = sc[0][j][e >> 2][e & 3];
+                  const float next = sum + x, back = next - sum;
+                  sc[1][j][e >> 2][e & 3] += (sum - (next - back)) + (x - back);
+                  sum = next;
+                } else {                                   // two chains: half the roundings each
+                  sc[ks & 1][j][e >> 2][e & 3] += x;
+                }
               }
             }
           }
+        } else if (more) {                       // no scores for this warp
+#pragma unroll 1
+          for (int i = 0; i < PIECES; ++i) fetch_qk(c + 1, i);
         }
-cp_async_commit();
+        cp_async_commit();
 #pragma unroll 2
         for (int ks = ks0; ks < ks1; ++ks) {
           uint32_t qf[4];
