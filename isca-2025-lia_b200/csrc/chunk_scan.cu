@@ -16,9 +16,9 @@
 // The hi parts' products are summed per instruction (exact but for the last bits) and added in fp32; only the lower parts stay in the tensor cores' sums,
 // which truncate.  Against 64 bits, means over 6 to 10 inputs: 16 heads of 128 x 128, 1024 tokens: outputs off by 8.5e-8 (token loop: 12e-8), the state by 8e-8 (19e-8), 64
 // tokens: 7.8e-8 (8.0e-8) and 6.1e-8 (12e-8); gated, 4 heads of 256 x 512, 503 and 400 tokens: outputs' median 1.5e-7 (1.9e-7), state 1.15e-7 (1.2e-7), normaliser as there.
-// A chunk of 64 takes about 3.3 us, one of 32 at 256 dims 3.8, one after the other (a sequence's chunks cannot run at once): cutting the additions to half did not
+// A chunk of 64 takes about 3.3 us, one of 32 at 256 dims 3.6, one after the other (a sequence's chunks cannot run at once): cutting the additions to half did not
 // change that; the chain ldmatrix, mma, add, the two barriers and the instructions themselves bound it (thirteen warps run three programs; see the loops' unrolling).
-// A portion of 2048 tokens: 16 heads of 128 x 128 533 us by tokens, 102 here, 4 heads of 256 x 512 878 and 241.
+// A portion of 2048 tokens: 16 heads of 128 x 128 533 us by tokens, 102 here, 4 heads of 256 x 512 878 and 227.
 #include <math.h>
 
 #include "common.cuh"
@@ -63,7 +63,7 @@ template <int DIM, int L> struct ChunkSmem {
   bf16 s[3][COLS][QP];                         // parts of the state before the chunk
   alignas(16) float part[2][WPR][L][OP];         // of the output
   float D[2][32][33];                          // mLSTM
-  float a[2][L], w[2][L], em[2][L];
+  alignas(16) float a[2][L], w[2][L], em[2][L];
   float rs[2][WPR][L], nq[2][L];               // row sums of the scores; q . n
   alignas(16) float n[DIM];
   float pw[L + 1];                             // powers of a fixed decay
@@ -71,16 +71,16 @@ template <int DIM, int L> struct ChunkSmem {
   alignas(16) int bad[2][COLS];                            // first token whose v is not finite
 };
 
-// Where a contracting warp's rows of the state begin in Q S, in steps of 16.  A step takes a warp some 330 clocks, a block of scores and its values 8 times that at 256 dims (the warps without one
-// have the inputs to ask for all the same), and the warps of a row block that have fewer blocks of scores take more steps: the chain of two portions of 1003 tokens, 4 heads of 256 x 512, 143 us
-// with four steps each, 140 with a block counted by its instructions (2 KS + 12, a step 12), 126 so.  Where two warps share a row block, six steps of one of them are a longer
-// chain of fp32 additions and put outputs off by 1.006 times as much: five at most.
+// Where a contracting warp's rows of the state begin in Q S, in steps of 16.  A step takes a warp some 470 clocks at 256 dims, a block of scores and its values five times that (more than its
+// instructions, 2 KS + 12 beside a step's 12, for a step's are less of a chain), and the warps of a row block that have fewer blocks of scores take more steps.  The chain of two portions of 1003 tokens,
+// 4 heads of 256 x 512: 132 us with a block counted by its instructions and all warps in the scores' loop, 125 without those that have none there and a block for nine steps, 118 for five.  Where
+// two warps share a row block, six steps of one of them are a longer chain of fp32 additions and put outputs off by 1.006 times as much: five at most.
 template <int RB, int WPR, int KS> struct Shares {
   int from[RB][WPR + 1];
   constexpr Shares() : from{} {
     for (int rb = 0; rb < RB; ++rb) {
       int load[WPR] = {}, steps[WPR] = {};
-      for (int blk = 0; blk <= rb; ++blk) load[blk % WPR] += 6 * KS + 12;
+      for (int blk = 0; blk <= rb; ++blk) load[blk % WPR] += 3 * KS + 12;
       for (int ks = 0; ks < KS; ++ks) {
         int least = -1;
         for (int i = 0; i < WPR; ++i)
@@ -463,12 +463,17 @@ __global__ void __launch_bounds__((MW + 4 + MLSTM) * 32, 1) chunk_scan_kernel(Ch
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (2 * aux < DIM) {
           float x0 = 0.f, x1 = 0.f;
-#pragma unroll 8
-          for (int s = 0; s < L; ++s) {
-            float k0, k1;
-            unpack_bf16x2(*reinterpret_cast<const uint32_t*>(&sm.k[b][s][2 * aux]), k0, k1);
-            x0 = fmaf(sm.w[b][s], k0, x0);
-            x1 = fmaf(sm.w[b][s], k1, x1);
+#pragma unroll 4
+          for (int s = 0; s < L; s += 4) {
+            const float4 w = *reinterpret_cast<const float4*>(&sm.w[b][s]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float ws = i == 0 ? w.x : i == 1 ? w.y : i == 2 ? w.z : w.w;
+              float k0, k1;
+              unpack_bf16x2(*reinterpret_cast<const uint32_t*>(&sm.k[b][s + i][2 * aux]), k0, k1);
+              x0 = fmaf(ws, k0, x0);
+              x1 = fmaf(ws, k1, x1);
+            }
           }
           sm.n[2 * aux] = fmaf(sm.total[b], sm.n[2 * aux], x0);
           sm.n[2 * aux + 1] = fmaf(sm.total[b], sm.n[2 * aux + 1], x1);
