@@ -178,10 +178,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // ===================== MMA issuer: two independent job streams served by one thread =====================
     // Q.K^T jobs run ahead of the softmax as far as the three score buffers allow (also into the NEXT item); P.V jobs are
     // issued the moment the softmax warps have published a P tile.  Neither stream ever blocks the other: the thread
-    // probes the barriers (mbarrier.test_wait) instead of waiting on them.
+    // probes the barriers (warp_test) instead of waiting on them.
     {
       const uint32_t one = elect_one();
-      auto ready = [&](uint32_t bar, uint32_t parity) { return __shfl_sync(0xffffffffu, mbar_test(bar, parity) ? 1 : 0, 0) != 0; };      // the same answer for all lanes
       constexpr uint32_t idesc_qk = make_idesc(BM, BN);                   // A = Q (K-major), B = K (K-major)
       constexpr uint32_t idesc_pv = make_idesc(BM, D) | (1u << 16);       // A = P (K-major), B = V (MN-major)
       int q_idx = blockIdx.x, p_idx = blockIdx.x;
@@ -193,8 +192,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         bool progressed = false;
         if (!q_done) {
           const int ks = kc & 1, sb = sc % S_BUFS, qb = qn & 1;
-          if ((q_job > 0 || ready(q_full(qb), (qn >> 1) & 1)) && ready(k_full(ks), (kc >> 1) & 1) &&
-              ready(s_empty(sb), ((sc / S_BUFS) & 1) ^ 1u)) {
+          if ((q_job > 0 || warp_test(q_full(qb), (qn >> 1) & 1)) && warp_test(k_full(ks), (kc >> 1) & 1) &&
+              warp_test(s_empty(sb), ((sc / S_BUFS) & 1) ^ 1u)) {
             tcgen05_fence_after();
             const uint32_t qa = smem_base + L::Q_OFF + qb * L::TILE_BYTES, ka = smem_base + L::K_OFF + ks * L::TILE_BYTES;
 #pragma unroll
@@ -218,7 +217,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           }
         }
         if (!p_done) {
-          if (ready(p_full, pc & 1) && ready(v_full, vc & 1) && (p_blk > 0 || ready(o_empty, (pn & 1) ^ 1u))) {
+          if (warp_test(p_full, pc & 1) && warp_test(v_full, vc & 1) && (p_blk > 0 || warp_test(o_empty, (pn & 1) ^ 1u))) {
             tcgen05_fence_after();
             const uint32_t pa = smem_base + L::P_OFF, va = smem_base + L::V_OFF;
 #pragma unroll

@@ -31,7 +31,7 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
       "r"(parity)
       : "memory");
 }
-// non-blocking probe of an mbarrier phase
+// non-blocking probe of an mbarrier phase, by one thread: its lanes may see different answers (warp_test is for warps)
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -45,6 +45,8 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// the same answer for all lanes of a warp that probes together: the phase is over for every one of them
+__device__ __forceinline__ bool warp_test(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_test(bar, parity)); }
 // A wait with a limit (try_wait itself sleeps for a while: seconds in all), after which it and all later ones of the block that share `dead` give up
 constexpr unsigned WAIT_LIMIT = 1u << 20;
 __device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t parity, volatile int* dead) {

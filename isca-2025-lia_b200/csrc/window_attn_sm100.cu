@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(THREADS, 1) window_prompt_tc_kernel(const void
 #pragma unroll 1
       for (int it = 0; it < n; ++it) {
         const int st = it % ST, j0 = jb + it * KEYS;
-        if (under_way >= 0 && !mbar_test(smem_u32(&sm.kv_empty[st]), ((it / ST) & 1) ^ 1u)) {          // no place yet: first see the last one home
+        if (under_way >= 0 && !warp_test(smem_u32(&sm.kv_empty[st]), ((it / ST) & 1) ^ 1u)) {          // no place yet: first see the last one home
           cp_async_wait<0>();
           arrived();
           under_way = -1;

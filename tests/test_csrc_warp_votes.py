@@ -1,0 +1,15 @@
+"""Control flow of warps in the kernels' sources, as far as it can be read off them: a branch that a whole warp takes must not hang on what one lane sees."""
+import pathlib
+import re
+
+CSRC = pathlib.Path(__file__).parents[1] / "isca-2025-lia_b200" / "csrc"
+SOURCES = {p.name: re.sub(r"//[^\n]*", "", p.read_text()) for p in sorted(CSRC.glob("*.cu*"))}
+
+
+def test_probes_of_barriers_are_votes():
+    """Lanes that probe a barrier one after the other may see it before and after its phase ends, so only a vote may decide where the warp goes."""
+    calls = [(name, line.strip()) for name, text in SOURCES.items() for line in text.splitlines() if re.search(r"\bmbar_test\(", line)]
+    assert len(calls) >= 2                                          # the probe and the vote
+    for name, line in calls:
+        assert re.match(r"__device__ __forceinline__ bool mbar_test\(uint32_t bar, uint32_t parity\) \{", line) or "__all_sync(0xffffffffu, mbar_test(" in line, (name, line)
+    assert [name for name, text in SOURCES.items() if "mbarrier.test_wait" in text] == ["umma.cuh"]
