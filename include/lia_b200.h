@@ -499,9 +499,12 @@ int lia_window_attn_masked(const void* q, int ldq, int q_f32, int act_f32, const
  * and strides (elements; whole 16 bytes) */
 int lia_window_attn_mma_takes(const void* q, int ldq, int q_f32, const void* kcache, long long k_slot_stride, const void* vcache,
                               long long v_slot_stride, const void* out, int H, int G, int v_div, int dim, int vdim);
+/* Which of two kernels of lia_window_attn_mma take a step's portions of prompts with heads of 128 + 128 channels, by the time that either is expected to need.  `portions`: the numbers of `segs` on the host; NULL: not known there,
+ * as with prompt = 1.  window, chunk as in lia_window_attn_mma. */
+int lia_window_prompt_form(const int* portions, int nseg, int M, int H, int window, int chunk);
 /* lia_window_attn_masked on the tensor cores, for bf16 caches.  prompt != 0: the rows belong to nseg portions, segs[s] = {slot, first position,
  * first row, rows} on the device (NULL: all rows are one portion that continues from meta's first row); prompt == 0: every row by itself,
- * its keys in nsplit ranges (workspace as for lia_window_attn). */
+ * its keys in nsplit ranges (workspace as for lia_window_attn).  prompt is 1 or, with heads of 128 + 128 channels, lia_window_prompt_form() of the same portions. */
 int lia_window_attn_mma(const void* q, int ldq, int q_f32, const void* kcache, long long k_slot_stride, const void* vcache,
                         long long v_slot_stride, const int* meta, const int* segs, int nseg, const float* temp, const float* slopes,
                         const float* sink, const void* gate, int gate_mode, int ldg, void* out, int out_f32, float* workspace, int M, int H, int G,

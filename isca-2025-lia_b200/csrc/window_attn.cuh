@@ -33,9 +33,9 @@ template <> __device__ __forceinline__ void stf<float>(float* p, float v) { *p =
 template <> __device__ __forceinline__ void stf<bf16>(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
 
 // first position a query at `pos` sees: the window's start, and the start of its chunk if the mask is chunked
-__device__ __forceinline__ int first_key(const WindowArgs& a, int pos) {
-  int lo = max(0, pos - a.window + 1);
-  if (a.chunk > 0) lo = max(lo, pos - pos % a.chunk);
+__host__ __device__ __forceinline__ int first_key(const WindowArgs& a, int pos) {
+  int lo = pos - a.window + 1 > 0 ? pos - a.window + 1 : 0;
+  if (a.chunk > 0 && pos - pos % a.chunk > lo) lo = pos - pos % a.chunk;
   return lo;
 }
 

@@ -2,8 +2,8 @@
 // channels.  Nothing is held in fewer bits than on the CUDA cores: the caches are bf16 as they are, fp32 queries and the softmax's
 // weights enter as three bf16 parts (mma.cuh), scores and sums are fp32.
 //
-//   prompt:  (heads of 128 + 128 channels: window_attn_sm100.cu) one block per (64 rows of one portion, query head).  Bound: tensor cores and the softmax's instructions about equally -- mma.sync
-//            m16n8k16, one product for q . k (three for fp32 queries) and three for the weights times the values.  A warp owns 16 rows: its
+//   prompt:  one block per (64 rows of one portion, query head); with heads of 128 + 128 channels only for many short portions (lia_window_prompt_form), the others are
+//            window_attn_sm100.cu's.  Bound: tensor cores and the softmax's instructions about equally -- mma.sync m16n8k16, one product for q . k (three for fp32 queries) and three for the weights times the values.  A warp owns 16 rows: its
 //            16 x 32 scores become the weights' operand in registers, so nothing but keys and values passes through shared memory; those come
 //            by cp.async, two stages of 32 keys (64 keys need 255 registers: two blocks per SM instead of three, 185 instead of 159 us).
 //            2048 tokens, 16 heads of 128 on 8 key heads, window 1024, soft cap: 1183 -> 136 us; the whole history, fp32 queries: 1713 -> 182 us (such heads: 66 and 64 us there).
@@ -17,10 +17,12 @@
 // running ones in fp32: the error against 64 bits is 0.4 to 0.8 times that of the FMA chains (one running sum over 1700 keys: 5 times).
 // Numbers that are not finite do not survive this: a masked key of the stage has weight 0 and still meets its value, and a part of a split weight is 0 or has
 // the other sign.  Sums that are not finite stay so to the end, so it is there that such rows are found and formed again key by key (plain_row).
+#include <limits.h>
+
 #include "window_attn_rows.cuh"
 
 int window_prompt_tc(const void* q, int ldq, const bf16* kcache, long long kss, const bf16* vcache, long long vss, const int* meta, const int* segs, int nseg, const WindowExtras& x, bf16* out,
-                     int M, const WindowArgs& a, cudaStream_t stream);      // window_attn_sm100.cu
+                     int M, const WindowArgs& a, int least, int tiles, cudaStream_t stream);      // window_attn_sm100.cu
 
 namespace {
 
@@ -46,11 +48,12 @@ template <int DK, int DV, int NQ> struct PromptShape {
 };
 
 // NQ = 1: bf16 queries; 3: fp32 queries in three parts.  segs[s] = {slot, first position, first row, rows}; null: one portion that meta's first
-// row begins (tiles whose rows do not continue it are taken row by row).  blockIdx.y counts the portions' tiles from the last to the first: the longest histories start first.
+// row begins (tiles whose rows do not continue it are taken row by row).  Portions of more than `most` rows are another kernel's.  blockIdx.y counts the portions' tiles from the last to the
+// first: the longest histories start first.
 template <int DK, int DV, int NQ>
 __global__ void __launch_bounds__(128, (DV <= 128 && NQ == 1) ? 3 : 2) window_prompt_kernel(const void* __restrict__ q, int ldq, const bf16* __restrict__ kcache, long long k_slot_stride,
                                                             const bf16* __restrict__ vcache, long long v_slot_stride, const int* __restrict__ meta,
-                                                            const int* __restrict__ segs, int nseg, WindowExtras x, bf16* __restrict__ out, int M, WindowArgs a) {
+                                                            const int* __restrict__ segs, int nseg, int most, WindowExtras x, bf16* __restrict__ out, int M, WindowArgs a) {
   pdl_launch_dependents();
   pdl_wait();
   constexpr int BK = PromptShape<DK, DV, NQ>::BK, QC = DK / 8, VC = DV / 8, NT = BK / 8;
@@ -62,7 +65,7 @@ __global__ void __launch_bounds__(128, (DV <= 128 && NQ == 1) ? 3 : 2) window_pr
     slot = meta[0]; pos0 = meta[1]; row0 = 0; rows = M;
     if (tile * BM >= rows) return;
   } else {
-    const int found = portion_of<BM>(segs, nseg, tile);
+    const int found = portion_of<BM>(segs, nseg, tile, 1, most);
     if (found < 0) return;
     slot = segs[4 * found]; pos0 = segs[4 * found + 1]; row0 = segs[4 * found + 2]; rows = segs[4 * found + 3];
   }
@@ -477,11 +480,11 @@ struct Call {
   cudaStream_t stream;
 };
 
-template <int DK, int DV, int NQ> int prompt_as(const Call& c) {
+template <int DK, int DV, int NQ> int prompt_as(const Call& c, int most = INT_MAX, int tiles = 0) {
   constexpr int smem = PromptShape<DK, DV, NQ>::SMEM;
   LIA_CUDA(cudaFuncSetAttribute(window_prompt_kernel<DK, DV, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  const dim3 grid(c.a.H, (c.M + BM - 1) / BM + (c.segs ? c.nseg - 1 : 0));     // at least as many tiles as the portions have
-  lia_launch(window_prompt_kernel<DK, DV, NQ>, dim3(grid), dim3(128), smem, c.stream, c.q, c.ldq, c.kcache, c.kss, c.vcache, c.vss, c.meta, c.segs, c.nseg, c.x, c.out, c.M, c.a);
+  const dim3 grid(c.a.H, tiles > 0 ? tiles : (c.M + BM - 1) / BM + (c.segs ? c.nseg - 1 : 0));     // at least as many tiles as the portions have
+  lia_launch(window_prompt_kernel<DK, DV, NQ>, dim3(grid), dim3(128), smem, c.stream, c.q, c.ldq, c.kcache, c.kss, c.vcache, c.vss, c.meta, c.segs, c.nseg, most, c.x, c.out, c.M, c.a);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
@@ -497,10 +500,24 @@ template <int DK, int DV, int NQ> int decode_as(const Call& c) {
   return LIA_OK;
 }
 
-template <int DK, int DV> int run_as(const Call& c, bool prompt) {
+// What lia_window_prompt_form returns: one kernel for all portions or, by their rows, both; above these bits, in 14 each, the tiles of either (0: not known)
+enum { TCGEN05 = 2, MMA_SYNC = 3, BOTH = 4 };
+constexpr int TILE_BITS = 14, TILE_MASK = (1 << TILE_BITS) - 1;
+
+template <int DK, int DV> int run_as(const Call& c, int prompt) {
   if (prompt) {
-    if constexpr (DK == 128 && DV == 128) return window_prompt_tc(c.q, c.ldq, c.kcache, c.kss, c.vcache, c.vss, c.meta, c.segs, c.nseg, c.x, c.out, c.M, c.a, c.stream);
-    else return c.a.q_f32 ? prompt_as<DK, DV, 3>(c) : prompt_as<DK, DV, 1>(c);
+    if constexpr (DK == 128 && DV == 128) {
+      if (prompt == 1) prompt = lia_window_prompt_form(nullptr, c.segs ? c.nseg : 1, c.M, c.a.H, c.a.window, c.a.chunk);
+      const int kernels = prompt & 7, tc_tiles = prompt >> 3 & TILE_MASK, tiles = prompt >> (3 + TILE_BITS) & TILE_MASK;
+      if (kernels != MMA_SYNC) {
+        const int rc = window_prompt_tc(c.q, c.ldq, c.kcache, c.kss, c.vcache, c.vss, c.meta, c.segs, c.nseg, c.x, c.out, c.M, c.a, kernels == BOTH ? SHORT_ROWS + 1 : 1, tc_tiles, c.stream);
+        if (rc != LIA_OK || kernels == TCGEN05) return rc;
+      }
+      const int most = kernels == BOTH ? SHORT_ROWS : INT_MAX;
+      return c.a.q_f32 ? prompt_as<DK, DV, 3>(c, most, tiles) : prompt_as<DK, DV, 1>(c, most, tiles);
+    } else {
+      return c.a.q_f32 ? prompt_as<DK, DV, 3>(c) : prompt_as<DK, DV, 1>(c);
+    }
   }
   return c.a.q_f32 ? decode_as<DK, DV, 3>(c) : decode_as<DK, DV, 1>(c);
 }
@@ -508,6 +525,51 @@ template <int DK, int DV> int run_as(const Call& c, bool prompt) {
 bool head_sizes_ok(int dim, int vdim) { return (dim == 64 || dim == 128) && (vdim == 64 || vdim == 128 || vdim == 256); }
 
 }  // namespace
+
+// A tile of 128 rows has its SM to itself on tcgen05, however few of the rows are there; one of 64 on mma.sync shares it with two others.  So the first is ahead where tiles are few or histories
+// long, the second with many portions of few rows.  What a step takes is estimated, in us, from the times of 1500 steps of 1 to 64 portions of 1 to 2048 rows behind 0 to 2000 positions, 8 to 32
+// heads, both types of queries (tcgen05: 6.4 a tile and 1.1 for 64 keys; mma.sync: 1.2 a tile of throughput and, with up to 16, 32 or 64 rows, 0.76, 1.1 or 1.3 for 32 keys, of which one
+// tile alone takes 2.75 and 1.8): the kernel with the smaller estimate is the slower one by 3 % or more in 47 of them, by 13 and 22 % at most.
+// us, mma.sync | tcgen05, 32 heads on 8 key heads, rows @ positions before them: 2 @ 0 5.5 | 8.4; 64 @ 256 25 | 14; 32 portions of 16 @ 0 17 | 58, @ 500 118 | 132, @ 1000 210 | 193; of 40 @ 0
+// 29 | 62, @ 256 92 | 99, @ 500 153 | 136; of 96 @ 0 60 | 76, @ 64 92 | 86; of 128 @ 0 80 | 77.
+// A portion of more than 128 rows is always tcgen05's, so that its bits do not depend on its company; a shorter one's may, as those of its projections do (128 rows and fewer in a step are
+// multiplied another way).  Where portions are not known on the host, mma.sync has the steps of more tiles than SMs whose portions have 128 rows or fewer on average.
+extern "C" int lia_window_prompt_form(const int* portions, int nseg, int M, int H, int window, int chunk) {
+  if (nseg <= 0 || M <= 0 || H <= 0) return TCGEN05;
+  const int sms = lia_sm_count();
+  if (!portions) return nseg > 1 && M <= 128ll * nseg && ((M + 127ll) / 128 + nseg - 1) * H > sms ? MMA_SYNC : TCGEN05;
+  WindowArgs a{};
+  a.window = window > 0 ? window : 1 << 30;
+  a.chunk = chunk;
+  struct Sums {
+    long long tiles = 0;
+    double longest = 0, all = 0;
+    void take(double alone, double shared) { ++tiles, longest = alone > longest ? alone : longest, all += shared; }
+  } tc[2], mma[2];                                                 // of the long portions, of the short ones
+  for (int i = 0; i < nseg; ++i) {
+    const int pos = portions[4 * i + 1], rows = portions[4 * i + 3], is_short = rows <= SHORT_ROWS;
+    auto keys = [&](int r, int of) { return pos + (r + of < rows ? r + of : rows) - first_key(a, pos + r); };
+    for (int r = 0; r < rows; r += 128) {
+      const double t = 6.4 + 1.1 * ((keys(r, 128) + 63) / 64);
+      tc[is_short].take(t, t);
+    }
+    for (int r = 0; r < rows && is_short; r += 64) {
+      const int n = (keys(r, 64) + 31) / 32, here = rows - r;
+      mma[1].take(2.75 + 1.8 * n, 1.2 + (here <= 16 ? 0.76 : here <= 32 ? 1.1 : 1.3) * n);
+    }
+  }
+  auto tc_time = [&](long long tiles, double longest, double all) {
+    if (tiles == 0) return 0.0;
+    const long long items = tiles * H, waves = (items + sms - 1) / sms;
+    const double shared = items > 4ll * sms ? all * H / sms : all / tiles * waves;
+    return shared > longest ? shared : longest;
+  };
+  const double shared = mma[1].all * H / sms, both = shared < mma[1].longest ? mma[1].longest + 0.15 * shared : shared + 0.15 * mma[1].longest;
+  const double one = tc_time(tc[0].tiles + tc[1].tiles, tc[0].longest > tc[1].longest ? tc[0].longest : tc[1].longest, tc[0].all + tc[1].all);
+  if (mma[1].tiles == 0 || one <= tc_time(tc[0].tiles, tc[0].longest, tc[0].all) + both) return TCGEN05;
+  if (tc[0].tiles == 0) return MMA_SYNC;
+  return BOTH | (tc[0].tiles <= TILE_MASK && mma[1].tiles <= TILE_MASK ? (int)tc[0].tiles << 3 | (int)mma[1].tiles << (3 + TILE_BITS) : 0);
+}
 
 // 1 if the tensor-core kernels take bf16 caches of these head sizes, addresses and strides (elements); everything else is window_attn.cu's
 extern "C" int lia_window_attn_mma_takes(const void* q, int ldq, int q_f32, const void* kcache, long long k_slot_stride, const void* vcache,
@@ -517,7 +579,7 @@ extern "C" int lia_window_attn_mma_takes(const void* q, int ldq, int q_f32, cons
          H % G == 0 && v_div > 0 && G % v_div == 0;
 }
 
-// The tensor-core form of lia_window_attn_masked for bf16 caches.  `prompt`: rows in portions `segs` [nseg][4] on the device (null: all rows are one
+// The tensor-core form of lia_window_attn_masked for bf16 caches.  `prompt` (1, or what lia_window_prompt_form says): rows in portions `segs` [nseg][4] on the device (null: all rows are one
 // portion that continues from meta[0]); otherwise every row by itself, its keys in nsplit ranges.
 extern "C" int lia_window_attn_mma(const void* q, int ldq, int q_f32, const void* kcache, long long k_slot_stride, const void* vcache,
                                    long long v_slot_stride, const int* meta, const int* segs, int nseg, const float* temp, const float* slopes,
@@ -529,7 +591,8 @@ extern "C" int lia_window_attn_mma(const void* q, int ldq, int q_f32, const void
                 "lia_window_attn_mma: heads of %d + %d channels, these addresses or strides are not for the tensor-core kernels", dim, vdim);
   LIA_CHECK_ARG(gate_mode >= 0 && gate_mode <= 2 && (gate_mode == 0) == (gate == nullptr) && (gate_mode != 2 || ldg >= H * vdim),
                 "lia_window_attn_mma: bad output gate (mode %d, row stride %d)", gate_mode, ldg);
-  LIA_CHECK_ARG(nsplit >= 1 && nsplit <= 64 && (nsplit == 1 || (workspace && !prompt)), "lia_window_attn_mma: bad number of key ranges (%d)", nsplit);
+  LIA_CHECK_ARG(prompt >= 0 && (prompt & 7) <= BOTH && (prompt <= BOTH || (prompt & 7) == BOTH), "lia_window_attn_mma: no such form of prompts (%d)", prompt);
+  LIA_CHECK_ARG(nsplit >= 1 && nsplit <= 64 && (nsplit == 1 || (workspace && prompt == 0)), "lia_window_attn_mma: bad number of key ranges (%d)", nsplit);
   LIA_CHECK_ARG(!prompt || (segs ? nseg > 0 && (M + BM - 1) / BM + nseg - 1 <= 65535 : (M + BM - 1) / BM <= 65535), "lia_window_attn_mma: bad portions");
   const int rep = H / G;
   int HB = rep < 8 ? rep : 8;

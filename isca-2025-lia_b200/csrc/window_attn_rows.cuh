@@ -6,6 +6,9 @@
 
 namespace {
 
+// Of the prompts with heads of 128 + 128 channels, portions of up to so many rows may go to mma.sync (lia_window_prompt_form)
+constexpr int SHORT_ROWS = 128;
+
 // scores of one thread, in place: dot products * mul -> soft-capped, less the distance's cost.  dist(i) = query position - key position of score i.
 // tanh of small arguments (real scores are far below the cap) is its Taylor series up to the 9th power: below 0.3 the rest is under 6e-8 of
 // the value, one rounding, at a third of the instructions of tanhf, which with exp bounds this kernel as much as the products do.
@@ -84,12 +87,12 @@ __device__ __noinline__ PlainRow<DV> plain_row(const void* q, size_t q_at, const
   return y;
 }
 
-// The portion that holds the tile-th tile of ROWS rows, and the tile within it (a whole warp asks); < 0: there are fewer tiles
-template <int ROWS> __device__ __forceinline__ int portion_of(const int* __restrict__ segs, int nseg, int& tile) {
+// The portion that holds the tile-th tile of ROWS rows, and the tile within it, among the portions of `least` to `most` rows (a whole warp asks); < 0: there are fewer tiles
+template <int ROWS> __device__ __forceinline__ int portion_of(const int* __restrict__ segs, int nseg, int& tile, int least, int most) {
   const int lane = threadIdx.x & 31;
   int found = -1;
   for (int base = 0; base < nseg && found < 0; base += 32) {             // 32 portions at a time
-    const int n = base + lane < nseg ? (segs[4 * (base + lane) + 3] + ROWS - 1) / ROWS : 0;
+    const int rows = base + lane < nseg ? segs[4 * (base + lane) + 3] : 0, n = rows >= least && rows <= most ? (rows + ROWS - 1) / ROWS : 0;
     int upto = n;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {

@@ -13,6 +13,8 @@
 // 8 key heads of 128; on mma.sync -> here, us, and the error against 64 bits in 1e-7: 2048 rows, 16 heads, window of 1024 and soft cap 136 (1.87) -> 66 (1.68), the whole history and fp32 queries
 // 182 (2.42) -> 63 (1.69); 700 rows behind 300 91 (2.43) -> 35 (2.16); portions of 300, 250, 200 31 (1.54) -> 17 (1.49); 64 rows 9.3 (1.37) -> 9.1 (1.19);
 // 33 rows 8.7 (1.18) -> 9.0 (0.97).  Four portions of 117, 100, 87, 73 behind a gate per channel: 24 -> 15 (33 with the gates asked for row by row).
+#include <limits.h>
+
 #include "attn_sm100.cuh"
 #include "window_attn_rows.cuh"
 
@@ -151,7 +153,7 @@ __device__ __forceinline__ void softmax_blocks(AttnTail& sm, uint32_t tmem, int 
 template <int NQ>
 __global__ void __launch_bounds__(THREADS, 1) window_prompt_tc_kernel(const void* __restrict__ q, int ldq, const bf16* __restrict__ kcache, long long k_slot_stride,
                                                                       const bf16* __restrict__ vcache, long long v_slot_stride, const int* __restrict__ meta, const int* __restrict__ segs,
-                                                                      int nseg, WindowExtras x, bf16* __restrict__ out, int M, WindowArgs a, int* timeouts) {
+                                                                      int nseg, int least, WindowExtras x, bf16* __restrict__ out, int M, WindowArgs a, int* timeouts) {
   constexpr int ST = stages<NQ>();
   extern __shared__ uint8_t raw[];
   const uint32_t base = (smem_u32(raw) + 1023u) & ~1023u, ks = base + NQ * Q_BYTES;          // a stage: keys, values
@@ -174,7 +176,7 @@ __global__ void __launch_bounds__(THREADS, 1) window_prompt_tc_kernel(const void
     slot = meta[0]; pos0 = meta[1]; row0 = 0; rows = M;
     if (tile * ROWS >= rows) return give_tmem_back(tmem, warp);
   } else {
-    const int found = portion_of<ROWS>(segs, nseg, tile);
+    const int found = portion_of<ROWS>(segs, nseg, tile, least, INT_MAX);
     if (found < 0) return give_tmem_back(tmem, warp);
     slot = segs[4 * found]; pos0 = segs[4 * found + 1]; row0 = segs[4 * found + 2]; rows = segs[4 * found + 3];
   }
@@ -372,7 +374,7 @@ __global__ void __launch_bounds__(THREADS, 1) window_prompt_tc_kernel(const void
 
 template <int NQ>
 int launch(const void* q, int ldq, const bf16* kcache, long long kss, const bf16* vcache, long long vss, const int* meta, const int* segs, int nseg, const WindowExtras& x, bf16* out, int M,
-           const WindowArgs& a, cudaStream_t stream) {
+           const WindowArgs& a, int least, int tiles, cudaStream_t stream) {
   constexpr int smem = smem_bytes<NQ>();
   static_assert(smem <= 232448, "shared memory budget exceeded");
   LIA_CUDA(cudaFuncSetAttribute(window_prompt_tc_kernel<NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
@@ -380,16 +382,17 @@ int launch(const void* q, int ldq, const bf16* kcache, long long kss, const bf16
   LIA_CHECK_ARG(split_fits, "lia_window_attn_mma: built with another number of registers");
   int* timeouts = lia_timeout_word();
   LIA_CHECK_ARG(timeouts != nullptr, "lia_window_attn_mma: no host memory for the count of timeouts");
-  const dim3 grid(a.H, (M + ROWS - 1) / ROWS + (segs ? nseg - 1 : 0));                       // at least as many tiles as the portions have
-  lia_launch(window_prompt_tc_kernel<NQ>, grid, dim3(THREADS), smem, stream, q, ldq, kcache, kss, vcache, vss, meta, segs, nseg, x, out, M, a, timeouts);
+  const dim3 grid(a.H, tiles > 0 ? tiles : (M + ROWS - 1) / ROWS + (segs ? nseg - 1 : 0));   // at least as many tiles as the portions have
+  lia_launch(window_prompt_tc_kernel<NQ>, grid, dim3(THREADS), smem, stream, q, ldq, kcache, kss, vcache, vss, meta, segs, nseg, least, x, out, M, a, timeouts);
   LIA_LAUNCH_CHECK();
   return LIA_OK;
 }
 
 }  // namespace
 
-// The prompt form of lia_window_attn_mma for heads of 128 + 128 channels
+// The prompt form of lia_window_attn_mma for heads of 128 + 128 channels, for the portions of `least` rows and more; `tiles`: of 128 rows, that these have (0: not known)
 int window_prompt_tc(const void* q, int ldq, const bf16* kcache, long long kss, const bf16* vcache, long long vss, const int* meta, const int* segs, int nseg, const WindowExtras& x, bf16* out,
-                     int M, const WindowArgs& a, cudaStream_t stream) {
-  return a.q_f32 ? launch<3>(q, ldq, kcache, kss, vcache, vss, meta, segs, nseg, x, out, M, a, stream) : launch<1>(q, ldq, kcache, kss, vcache, vss, meta, segs, nseg, x, out, M, a, stream);
+                     int M, const WindowArgs& a, int least, int tiles, cudaStream_t stream) {
+  return a.q_f32 ? launch<3>(q, ldq, kcache, kss, vcache, vss, meta, segs, nseg, x, out, M, a, least, tiles, stream)
+                 : launch<1>(q, ldq, kcache, kss, vcache, vss, meta, segs, nseg, x, out, M, a, least, tiles, stream);
 }

@@ -900,8 +900,14 @@ def window_decode_splits(M, H, G, span, max_ctx, sms):
     return max(1, min(2 * sms // blocks, window_attn_split_class(max_ctx, span))) if max_ctx > 0 else 1
 
 
+def window_prompt_form(portions, nseg, M, H, window, chunk=0):
+    """Which of two kernels take a step of ``nseg`` portions of prompts (csrc/window_attn_mma.cu); ``portions``: (slot, first position, first row, rows) each on the host, or None."""
+    host = None if portions is None else (ctypes.c_int * (4 * nseg))(*(int(x) for p in portions for x in p))
+    return _lib.load().lia_window_prompt_form(host, nseg, M, H, min(int(window), 1 << 30), int(chunk))
+
+
 def window_attn(q, kcache, vcache, meta, temp, out, H, G, dim, vdim, window, scale, softcap, nseg=None, max_ctx=0, slopes=None, sink=None,
-                gate=None, gate_per_head=False, chunk=0, v_div=1, segs=None):
+                gate=None, gate_per_head=False, chunk=0, v_div=1, segs=None, form=None):
     """Softmax attention of every row over the last ``window`` cached positions of its sequence (csrc/window_attn.cu);
     ``window`` <= 0: over its whole history.  ``nseg``: portions in the step (None: one row each); ``max_ctx``: an upper
     bound of the rows' history lengths (0: unknown, no split of the keys).  ``temp`` [H] multiplies the scores, ``slopes``
@@ -911,7 +917,8 @@ def window_attn(q, kcache, vcache, meta, temp, out, H, G, dim, vdim, window, sca
     block of ``chunk`` positions (blocks counted from the sequence's start).  ``v_div``: key head g reads value head g // v_div
     (the value cache holds G // v_div heads: several attention maps over one set of values).  ``segs`` int32 [nseg, 4] on the device
     (slot, first position, first row, rows): the portions whose rows these are; with them, or with one portion, a step of prompts on
-    bf16 caches runs on the tensor cores (csrc/window_attn_sm100.cu for heads of 128 channels, csrc/window_attn_mma.cu), and so does a step of single tokens."""
+    bf16 caches runs on the tensor cores (csrc/window_attn_sm100.cu for heads of 128 channels, csrc/window_attn_mma.cu), and so does a step of single tokens.
+    ``form``: ``window_prompt_form`` of the portions, where the host knows them."""
     ldq = _rowmajor(q, "q")
     _req(meta, "meta", I32)
     for t, n in ((temp, "temp"), (slopes, "slopes"), (sink, "sink")):
@@ -943,13 +950,16 @@ def window_attn(q, kcache, vcache, meta, temp, out, H, G, dim, vdim, window, sca
     if kcache.dtype == BF16 and (by_rows or segs is not None or portions == 1) and _lib.load().lia_window_attn_mma_takes(
             _p(q), ldq, _f32(q), _p(kcache), kcache.stride(0), _p(vcache), vcache.stride(0), _p(out), H, G, int(v_div), dim, vdim):
         nsplit = window_decode_splits(M, H, G, span, max_ctx, _sm_count(q.device)) if by_rows else 1
+        prompt = 0 if by_rows else 1
+        if prompt and dim == vdim == 128:
+            prompt = window_prompt_form(None, portions, M, H, window, chunk) if form is None else form
         ws = None
         if nsplit > 1:
             ws = torch.empty(_lib.load().lia_window_attn_workspace_floats(M, H, vdim, nsplit), dtype=F32, device=q.device)
         check(_lib.load().lia_window_attn_mma(_p(q), ldq, _f32(q), _p(kcache), kcache.stride(0), _p(vcache), vcache.stride(0), _p(meta), _p(segs), portions,
                                               _p(temp), _p(slopes), _p(sink), _p(gate), gate_mode, ldg, _p(out), _f32(out), _p(ws), M, H, G, int(v_div),
-                                              dim, vdim, window, int(chunk), float(scale), float(softcap), int(not by_rows), nsplit, _stream()), "lia_window_attn_mma")
-        count_launches(2 if nsplit > 1 else 1)
+                                              dim, vdim, window, int(chunk), float(scale), float(softcap), prompt, nsplit, _stream()), "lia_window_attn_mma")
+        count_launches(2 if nsplit > 1 or prompt > 3 else 1)
         return out
     hb, qr, nsplit = window_attn_plan(M, portions, H, G, dim, vdim, span, max_ctx, _sm_count(q.device))
     ws = None

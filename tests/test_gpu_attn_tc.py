@@ -42,3 +42,62 @@ def test_portions(q_f32, H, G, v_div, opt):
         gate = wide[:, 8:8 + H * d]
         got = want * torch.sigmoid(gate.cpu().to(F64))
         assert float((run(BF16, gate).cpu().to(F64) - got).abs().max() / got.abs().max()) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("spec,form", [([(0, 40)] * 40, 3), ([(0, 16), (0, 17), (40, 5), (0, 64)], 3), ([(0, 200)] + [(30, 1)] * 40, 4), ([(300, 90)] + [(100, 16)] * 70 + [(0, 97)], 5),
+                                       ([(0, 96), (33, 64)] * 100, 6), ([(0, 130)] * 20, 2), ([(0, 60), (10, 60)], 2)], ids=str)
+@pytest.mark.parametrize("q_f32,opt", [(False, dict()), (True, dict(window=24, sink=True))], ids=str)
+def test_short_portions(spec, form, q_f32, opt):
+    """Steps whose portions go to mma.sync, to tcgen05 or to both (on 148 SMs): every row is written once, known or not on the host, and a long portion's bits are those it has alone."""
+    H, G, d = 8, 4, 128
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the forms are those of 148 SMs")
+    portions = [(i, p, n) for i, (p, n) in enumerate(spec)]
+    q, kc, vc, segs, d_segs, meta = inputs(portions, H, G, d, d, q_f32, 5, 1)
+    sink = torch.full((H,), 0.5) if opt.get("sink") else None
+    want = reference(q, kc, vc, segs, H, G, d, d, 0.1, window=opt.get("window", 0), sink=sink).reshape(q.shape[0], -1)
+    sink = sink.to(DEV) if sink is not None else None
+
+    def run(segs, d_segs, rows, form):
+        out = torch.full((len(rows), H * d), 7.0, dtype=F32, device=DEV)
+        return ops.window_attn(q[rows].contiguous(), kc, vc, meta[rows].contiguous(), None, out, H, G, d, d, opt.get("window", 0), 0.1, 0.0, nseg=len(segs), segs=d_segs, max_ctx=400, sink=sink,
+                               form=form)
+    known = ops.window_prompt_form(segs, len(segs), q.shape[0], H, opt.get("window", 0))
+    assert known == form or (opt and form != 2)                     # a window leaves fewer keys to see: more portions are short ones
+    rows = list(range(q.shape[0]))
+    for f in (known, None, 2, 3):
+        assert float((run(segs, d_segs, rows, f).cpu().to(F64) - want).abs().max() / want.abs().max()) < TOL
+    out = run(segs, d_segs, rows, known)
+    for slot, p0, r0, n in segs:
+        if n > 96 and known != 3:
+            alone = torch.tensor([(slot, p0, 0, n)], dtype=torch.int32, device=DEV)
+            assert torch.equal(run([(slot, p0, 0, n)], alone, list(range(r0, r0 + n)), None), out[r0:r0 + n])
+
+
+STEPS = {"40 of 40 rows": ([(0, 40)] * 40, 3), "few tiles": ([(0, 16), (0, 17), (40, 5), (0, 64)], 3), "a prompt and 40 tokens": ([(0, 200)] + [(30, 1)] * 40, 4),
+         "two prompts and 70 of 16 rows": ([(300, 190)] + [(100, 16)] * 70 + [(0, 129)], 4), "200 of 64 and 96 rows": ([(0, 96), (33, 64)] * 100, 3), "20 of 130 rows": ([(0, 130)] * 20, 2)}
+
+
+@pytest.mark.parametrize("step", STEPS)
+@pytest.mark.parametrize("q_f32,opt", [(False, dict()), (True, dict(window=24, sink=True))], ids=str)
+def test_short_portions(step, q_f32, opt):
+    """Steps whose portions go to mma.sync, to tcgen05 or to both (on 148 SMs): every row is written, known or not on the host, and a long portion's bits are those it has alone."""
+    H, G, d = 8, 4, 128
+    spec, kernels = STEPS[step]
+    q, kc, vc, segs, d_segs, meta = inputs([(i, p, n) for i, (p, n) in enumerate(spec)], H, G, d, d, q_f32, 5, 1)
+    sink = torch.full((H,), 0.5) if opt.get("sink") else None
+    want = reference(q, kc, vc, segs, H, G, d, d, 0.1, window=opt.get("window", 0), sink=sink).reshape(q.shape[0], -1)
+    sink = sink.to(DEV) if sink is not None else None
+
+    def run(segs, rows, form):
+        out = torch.full((rows.stop - rows.start, H * d), float("nan"), dtype=F32, device=DEV)
+        return ops.window_attn(q[rows].contiguous(), kc, vc, meta[rows].contiguous(), None, out, H, G, d, d, opt.get("window", 0), 0.1, 0.0, nseg=len(segs), max_ctx=600, sink=sink, form=form,
+                               segs=torch.tensor(segs, dtype=torch.int32, device=DEV))
+    form = ops.window_prompt_form(segs, len(segs), q.shape[0], H, opt.get("window", 0))
+    assert form & 7 == kernels or torch.cuda.get_device_properties(0).multi_processor_count != 148
+    whole = slice(0, q.shape[0])
+    for f in (form, 4, None, 2, 3):
+        assert float((run(segs, whole, f).cpu().to(F64) - want).abs().max() / want.abs().max()) < TOL
+    for slot, p0, r0, n in segs:
+        if n > 128:
+            assert torch.equal(run([(slot, p0, 0, n)], slice(r0, r0 + n), None), run(segs, whole, form)[r0:r0 + n])
