@@ -108,9 +108,8 @@ __device__ __forceinline__ void leave(AttnTail& sm, uint32_t tmem, int warp, int
   if (__syncthreads_or(*dead)) {
     if (threadIdx.x == 0) atomicAdd_system(timeouts, 1);
     if (warp == ISSUER && (threadIdx.x & 31) == 0) {
-      volatile int none = 0;
       tcgen05_commit(smem_u32(&sm.drain));
-      wait_for(smem_u32(&sm.drain), 0u, &none);
+      wait_in_flight(smem_u32(&sm.drain), 0u);
     }
   }
   give_tmem_back(tmem, warp);

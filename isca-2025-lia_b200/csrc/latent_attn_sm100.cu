@@ -111,8 +111,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_expanded_tc_kernel(const __
           }
         }
         if (*dead && one) {                                        // loads in flight end before shared memory is given back
-          volatile int none = 0;
-          for (int t = max(0, it - 2); t < it; ++t) wait_for(smem_u32(of_keys ? &sm.k_full[t & 1] : &sm.v_full[t & 1]), (t >> 1) & 1, &none);
+          for (int t = max(0, it - 2); t < it; ++t) wait_in_flight(smem_u32(of_keys ? &sm.k_full[t & 1] : &sm.v_full[t & 1]), (t >> 1) & 1);
         }
       }
     } else {

@@ -113,10 +113,10 @@ __global__ void __launch_bounds__(THREADS, 1) latent_expand_kernel(const __grid_
     const bool live = skip + r < p.rows[i];
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
     bf16* row = p.C + (size_t)(p.out0[i] + skip + r) * p.ldc;
+    bool alive = true;                                             // (the whole warp's, as the waits are: a lane without a row goes round with the others)
 #pragma unroll 1
     for (int c = c0 + group_of_four; c < c1; c += 2) {
       const int n = c - c0;
-      bool alive = true;
       float sum[COLS];
 #pragma unroll
       for (int e = 0; e < COLS; ++e) sum[e] = 0.f;
@@ -141,10 +141,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_expand_kernel(const __grid_
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&sm.acc_empty[half]));
       }
-      if (!live) {
-        if (!alive) break;
-        continue;
-      }
+      if (!live) continue;
       const int col = c * COLS;
       bf16* out = row + (size_t)(col / p.part) * 3 * p.part + col % p.part;
 #pragma unroll
@@ -164,11 +161,10 @@ __global__ void __launch_bounds__(THREADS, 1) latent_expand_kernel(const __grid_
   if (__syncthreads_or(*dead)) {                                   // products and loads in flight end before shared memory and TMEM are given back
     if (tid == 0) atomicAdd_system(timeouts, 1);
     if (warp == 9 && lane == 0) {
-      volatile int none = 0;
       tcgen05_commit(smem_u32(&sm.drain));
-      wait_for(smem_u32(&sm.drain), 0u, &none);
-      wait_for(smem_u32(&sm.a_full), 0u, &none);
-      for (int n = max(0, sm.issued - STAGES); n < sm.issued; ++n) wait_for(smem_u32(&sm.w_full[n % STAGES]), n / STAGES & 1, &none);
+      wait_in_flight(smem_u32(&sm.drain), 0u);
+      wait_in_flight(smem_u32(&sm.a_full), 0u);
+      for (int n = max(0, sm.issued - STAGES); n < sm.issued; ++n) wait_in_flight(smem_u32(&sm.w_full[n % STAGES]), n / STAGES & 1);
     }
     __syncthreads();
   }

@@ -244,17 +244,16 @@ __global__ void __launch_bounds__(256, 1) moe_tc_kernel(const __grid_constant__ 
   tcgen05_fence_before();
   __syncthreads();
   if (*dead) {                                                     // loads and products in flight end before shared memory and TMEM are given back
-    volatile int none = 0;
     if (threadIdx.x == 0) {
       atomicAdd_system(p.timeouts, 1);
       for (int i = 0; i < STAGES && i < issued; ++i) {
         const int n = issued - 1 - i;
-        wait_for(full_bar(n % STAGES), (uint32_t)(n / STAGES) & 1u, &none);
+        wait_in_flight(full_bar(n % STAGES), (uint32_t)(n / STAGES) & 1u);
       }
     }
     if (warp == 1 && lane == 0) {
       tcgen05_commit(drain_bar);
-      wait_for(drain_bar, 0u, &none);
+      wait_in_flight(drain_bar, 0u);
     }
     __syncthreads();
   }

@@ -477,9 +477,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) ssd_states_kernel(const SsdArgs
   }
   if (*dead) {
     if (warp == 12 && lane == 0) {                                 // products in flight end before shared memory and TMEM are given back
-      volatile int none = 0;
       tcgen05_commit(smem_u32(&sm.bars.drain));
-      wait_for(smem_u32(&sm.bars.drain), 0u, &none);
+      wait_in_flight(smem_u32(&sm.bars.drain), 0u);
     }
     __syncthreads();
   }
@@ -900,10 +899,9 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
   __syncthreads();
   if (*dead) {
     if (warp == 4 && lane == 0) {                                  // products in flight end before shared memory and TMEM are given back
-      volatile int none = 0;
       atomicAdd_system(p.timeouts, 1);
       tcgen05_commit(smem_u32(&sm.bars.drain));
-      wait_for(smem_u32(&sm.bars.drain), 0u, &none);
+      wait_in_flight(smem_u32(&sm.bars.drain), 0u);
     }
     __syncthreads();
   }

@@ -47,10 +47,14 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 }
 // the same answer for all lanes of a warp that probes together: the phase is over for every one of them
 __device__ __forceinline__ bool warp_test(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_test(bar, parity)); }
-// A wait with a limit (try_wait itself sleeps for a while: seconds in all), after which it and all later ones of the block that share `dead` give up
-constexpr unsigned WAIT_LIMIT = 1u << 20;
-__device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t parity, volatile int* dead) {
-  for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
+// A wait with a limit (try_wait itself sleeps for a while: seconds in all), after which it and all later ones of the block that share `dead` give up.  Built with a limit of 0 (make nowait) every
+// wait gives up at once, but for those for what is in flight.
+#ifndef LIA_WAIT_LIMIT
+#define LIA_WAIT_LIMIT (1u << 20)
+#endif
+constexpr unsigned WAIT_LIMIT = LIA_WAIT_LIMIT, FLIGHT_LIMIT = 1u << 20;
+__device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t parity, volatile int* dead, unsigned limit = WAIT_LIMIT) {
+  for (unsigned i = 0; i < limit; ++i) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -63,7 +67,12 @@ __device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t parity, volatile
   *dead = 1;
   return false;
 }
-// the same for a whole warp
+// after a wait has run out, for loads and products under way: they end before the memory that they use is given back
+__device__ __forceinline__ void wait_in_flight(uint32_t bar, uint32_t parity) {
+  volatile int none = 0;
+  wait_for(bar, parity, &none, FLIGHT_LIMIT);
+}
+// wait_for by a whole warp
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* dead) { return __all_sync(0xffffffffu, wait_for(bar, parity, dead)); }
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
