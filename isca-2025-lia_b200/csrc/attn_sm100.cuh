@@ -107,8 +107,8 @@ __device__ __forceinline__ void leave(AttnTail& sm, uint32_t tmem, int warp, int
   volatile int* dead = &sm.dead;
   if (__syncthreads_or(*dead)) {
     if (threadIdx.x == 0) atomicAdd_system(timeouts, 1);
-    if (warp == ISSUER && (threadIdx.x & 31) == 0) {
-      tcgen05_commit(smem_u32(&sm.drain));
+    if (warp == ISSUER) {
+      commit_if(elect_one(), smem_u32(&sm.drain));
       wait_in_flight(smem_u32(&sm.drain), 0u);
     }
   }

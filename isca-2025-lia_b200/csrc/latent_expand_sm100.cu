@@ -160,8 +160,8 @@ __global__ void __launch_bounds__(THREADS, 1) latent_expand_kernel(const __grid_
   tcgen05_fence_before();
   if (__syncthreads_or(*dead)) {                                   // products and loads in flight end before shared memory and TMEM are given back
     if (tid == 0) atomicAdd_system(timeouts, 1);
-    if (warp == 9 && lane == 0) {
-      tcgen05_commit(smem_u32(&sm.drain));
+    if (warp == 9) {
+      commit_if(elect_one(), smem_u32(&sm.drain));
       wait_in_flight(smem_u32(&sm.drain), 0u);
       wait_in_flight(smem_u32(&sm.a_full), 0u);
       for (int n = max(0, sm.issued - STAGES); n < sm.issued; ++n) wait_in_flight(smem_u32(&sm.w_full[n % STAGES]), n / STAGES & 1);

@@ -364,8 +364,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) ssd_states_kernel(const SsdArgs
   tcgen05_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem, 0);
 
+  const uint32_t one = elect_one();
   if (warp == 12) {
-    const uint32_t one = elect_one();
     constexpr uint32_t mn = (1u << 15) | (1u << 16);               // both operands lie with the contracted tokens as rows
 #pragma unroll 1
     for (int j = 0; j < units; ++j) {
@@ -476,8 +476,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) ssd_states_kernel(const SsdArgs
     p.totals[(size_t)blockIdx.x * p.U + u0 + tid] = make_float2(sm.total[tid], sm.total_rest[tid]);
   }
   if (*dead) {
-    if (warp == 12 && lane == 0) {                                 // products in flight end before shared memory and TMEM are given back
-      tcgen05_commit(smem_u32(&sm.bars.drain));
+    if (warp == 12) {                                              // products in flight end before shared memory and TMEM are given back
+      commit_if(one, smem_u32(&sm.bars.drain));
       wait_in_flight(smem_u32(&sm.bars.drain), 0u);
     }
     __syncthreads();
@@ -898,9 +898,9 @@ __global__ void __launch_bounds__(OUT_THREADS, 1) ssd_outputs_kernel(const SsdAr
   tcgen05_fence_before();
   __syncthreads();
   if (*dead) {
-    if (warp == 4 && lane == 0) {                                  // products in flight end before shared memory and TMEM are given back
-      atomicAdd_system(p.timeouts, 1);
-      tcgen05_commit(smem_u32(&sm.bars.drain));
+    if (warp == 4) {                                               // products in flight end before shared memory and TMEM are given back
+      if (one) atomicAdd_system(p.timeouts, 1);
+      commit_if(one, smem_u32(&sm.bars.drain));
       wait_in_flight(smem_u32(&sm.bars.drain), 0u);
     }
     __syncthreads();

@@ -195,7 +195,7 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* v) {
       "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
       : "memory");
 }
-// Products issued by a whole warp, of whose lanes one has `one` set.  With warp numbers and addresses that are known to be the same in all lanes (__shfl_sync) an instruction takes 50 to 65 clocks;
+// Products issued by a whole warp, of whose lanes one has `one` set (the same one each time; a commit follows its own lane's products alone).  With warp numbers and addresses that are known to be the same in all lanes (__shfl_sync) an instruction takes 50 to 65 clocks;
 // from a lane by itself, whose operands are moved to uniform registers one after the other, 115.
 __device__ __forceinline__ uint32_t elect_one() {
   uint32_t one;

@@ -13,3 +13,15 @@ def test_probes_of_barriers_are_votes():
     for name, line in calls:
         assert re.match(r"__device__ __forceinline__ bool mbar_test\(uint32_t bar, uint32_t parity\) \{", line) or "__all_sync(0xffffffffu, mbar_test(" in line, (name, line)
     assert [name for name, text in SOURCES.items() if "mbarrier.test_wait" in text] == ["umma.cuh"]
+
+
+def test_commits_follow_the_lane_that_issues():
+    """A commit follows the products of its own thread alone: where the elected lane issues them, it commits them too, those that are drained after a wait has run out among them."""
+    seen = 0
+    for name, text in SOURCES.items():
+        if not re.search(r"\b(elect_one|mma_\w*if)\(", text) or name == "umma.cuh":
+            continue
+        for line in text.splitlines():
+            seen += "commit_if(" in line
+            assert not re.search(r"\btcgen05_commit(_pair)?\(", line) or "if (one)" in line, (name, line.strip())
+    assert seen >= 10
