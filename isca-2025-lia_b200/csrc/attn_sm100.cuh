@@ -184,10 +184,11 @@ __device__ __forceinline__ bool sum_blocks(AttnTail& sm, uint32_t tmem, int n, f
 }
 
 // A warp's 32 rows by way of 16 KB of shared memory at `place`, times `inv` of their threads: put(i, y) for row i and columns 4 lane .. 4 lane + 3, for neighbouring lanes to write neighbouring
-// columns.  `gated`: get(i) asks for a row's gates, of eight rows together, and gate(y, g) applies them.  Returns the rows among the first `rows` whose sums are not finite.  (Little code, and what
-// is not needed in one piece to skip: it is run once, and instructions come slowly then.)
+// columns.  `gated`: get(i) asks for a row's gates, of eight rows together, and gate(y, g) applies them.  Returns the rows among the first `rows` whose sums are not finite, which are not put: they
+// are for the caller to form again.  With sums of a wait that ran out (`alive` false; `inv` is NaN) there are none, and every row is put.  (Little code, and what is not needed in one piece to skip: it
+// is run once, and instructions come slowly then.)
 template <class Get, class Gate, class Put>
-__device__ __forceinline__ unsigned rows_out(uint8_t* place, const f32x2 (&O)[D / 2], float inv, int rows, bool gated, const Get& get, const Gate& gate, const Put& put) {
+__device__ __forceinline__ unsigned rows_out(uint8_t* place, const f32x2 (&O)[D / 2], float inv, bool alive, int rows, bool gated, const Get& get, const Gate& gate, const Put& put) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int c = 0; c < D; c += 4) {
@@ -201,7 +202,7 @@ __device__ __forceinline__ unsigned rows_out(uint8_t* place, const f32x2 (&O)[D 
   for (int c = 0; c < D / 2; ++c) probe[c & 3] = fma2(O[c], 0ull, probe[c & 3]);
   float p0, p1;
   unpack2(add2(add2(probe[0], probe[1]), add2(probe[2], probe[3])), p0, p1);
-  const unsigned again = __ballot_sync(0xffffffffu, lane < rows && p0 + p1 != 0.f);
+  const unsigned again = __ballot_sync(0xffffffffu, alive && lane < rows && p0 + p1 != 0.f);
   __syncwarp();
 #pragma unroll 1
   for (int i0 = 0; i0 < 32; i0 += 8) {

@@ -358,12 +358,12 @@ __global__ void __launch_bounds__(THREADS, 1) window_prompt_tc_kernel(const void
       }
       y = make_float4(y.x * g.x, y.y * g.y, y.z * g.z, y.w * g.w);
     };
-    const unsigned again = rows_out(raw + (ks - smem_u32(raw)) + (warp & 3) * (32 * D * 4), O, inv, rows - r0, a.gate_mode != 0, gates, gate, [&](int i, float4 y) {
+    const unsigned again = rows_out(raw + (ks - smem_u32(raw)) + (warp & 3) * (32 * D * 4), O, inv, alive, rows - r0, a.gate_mode != 0, gates, gate, [&](int i, float4 y) {
       const size_t at = ((size_t)(row0 + r0 + i) * a.H + h) * D + lane * 4;
       if (a.out_f32) *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + at) = y;
       else *reinterpret_cast<uint2*>(out + at) = make_uint2(pack_bf16x2(y.x, y.y), pack_bf16x2(y.z, y.w));
     });
-    if (alive && again) {
+    if (again) {
 #pragma unroll 1
       for (int i = 0; i < 32; ++i)
         if ((again >> i) & 1u) by_itself(row0 + r0 + i, slot, pos0 + r0 + i);

@@ -25,3 +25,12 @@ def test_commits_follow_the_lane_that_issues():
             seen += "commit_if(" in line
             assert not re.search(r"\btcgen05_commit(_pair)?\(", line) or "if (one)" in line, (name, line.strip())
     assert seen >= 10
+
+
+def test_rows_that_are_not_put_are_formed_again():
+    """Attention's rows whose sums are not finite are left out when rows are written: only where sums are complete, and whoever leaves them out forms them again without a further condition."""
+    assert re.search(r"again = __ballot_sync\(0xffffffffu, alive && ", SOURCES["attn_sm100.cuh"])
+    callers = [name for name, text in SOURCES.items() if re.search(r"= rows_out\(", text)]
+    assert callers == ["latent_attn_sm100.cu", "window_attn_sm100.cu"]
+    for name in callers:
+        assert re.search(r"rows_out\([^;]*?O, inv, alive, ", SOURCES[name]) and "    if (again) {" in SOURCES[name], name
