@@ -102,14 +102,15 @@ __device__ __forceinline__ void give_tmem_back(uint32_t tmem, int warp) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
 }
-// by all threads, at the end: products in flight end before shared memory and TMEM are given back
-__device__ __forceinline__ void leave(AttnTail& sm, uint32_t tmem, int warp, int* timeouts) {
+// by all threads, at the end: products and loads in flight (loads(): by one thread) end before shared memory and TMEM are given back
+template <class Loads> __device__ __forceinline__ void leave(AttnTail& sm, uint32_t tmem, int warp, int* timeouts, const Loads& loads) {
   volatile int* dead = &sm.dead;
   if (__syncthreads_or(*dead)) {
     if (threadIdx.x == 0) atomicAdd_system(timeouts, 1);
     if (warp == ISSUER) {
       commit_if(elect_one(), smem_u32(&sm.drain));
       wait_in_flight(smem_u32(&sm.drain), 0u);
+      if ((threadIdx.x & 31) == 0) loads();
     }
   }
   give_tmem_back(tmem, warp);

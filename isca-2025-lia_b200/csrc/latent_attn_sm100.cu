@@ -27,6 +27,7 @@ constexpr int QN = 0, QR = QN + ROWS * DN * 2, K_SMALL = QR + 3 * ROWS * DR * 2,
               V_HIGH = V_MID + 2 * SLAB, STAGE = V_HIGH + 2 * SLAB - K_SMALL, TAIL = K_SMALL + 2 * STAGE;
 struct Tail : AttnTail {
   uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2];
+  int issued[2];                                                   // blocks of keys, of values that were asked for by TMA
 };
 constexpr int SMEM = TAIL + (int)sizeof(Tail) + 1024;
 static_assert(SMEM <= 232448 && TAIL - K_SMALL >= 4 * 32 * D * 4, "shared memory budget exceeded, or no place for the sums' way out");
@@ -52,6 +53,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_expanded_tc_kernel(const __
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map) : "memory");
     init_hand_overs(sm);
     for (int i = 0; i < 2; ++i) {
+      sm.issued[i] = 0;
       mbar_init(smem_u32(&sm.k_full[i]), 2);
       mbar_init(smem_u32(&sm.v_full[i]), 1);
       mbar_init(smem_u32(&sm.k_empty[i]), 1);
@@ -95,12 +97,12 @@ __global__ void __launch_bounds__(THREADS, 1) latent_expanded_tc_kernel(const __
         const uint32_t one = elect_one();
         const bool of_keys = warp == LOADER0;
         const int col = (of_keys ? 0 : a.nh * 3 * DN) + blockIdx.x * 3 * DN, row = pt.part0 + jb;
-        int it = 0;
 #pragma unroll 1
-        for (; it < n; ++it) {
+        for (int it = 0; it < n; ++it) {
           const uint32_t full = smem_u32(of_keys ? &sm.k_full[it & 1] : &sm.v_full[it & 1]), empty = smem_u32(of_keys ? &sm.k_empty[it & 1] : &sm.v_empty[it & 1]);
           if (!warp_wait(empty, ((it >> 1) & 1) ^ 1u, dead)) break;
           if (!one) continue;
+          sm.issued[of_keys ? 0 : 1] = it + 1;
           mbar_expect_tx(full, 6 * SLAB);
 #pragma unroll
           for (int part = 2; part >= 0; --part) {
@@ -109,9 +111,6 @@ __global__ void __launch_bounds__(THREADS, 1) latent_expanded_tc_kernel(const __
 #pragma unroll
             for (int k = 0; k < 2; ++k) tma_load_2d(at + k * slab, &map, col + part * DN + k * 64, row + it * KEYS, full);
           }
-        }
-        if (*dead && one) {                                        // loads in flight end before shared memory is given back
-          for (int t = max(0, it - 2); t < it; ++t) wait_in_flight(smem_u32(of_keys ? &sm.k_full[t & 1] : &sm.v_full[t & 1]), (t >> 1) & 1);
         }
       }
     } else {
@@ -307,7 +306,10 @@ __global__ void __launch_bounds__(THREADS, 1) latent_expanded_tc_kernel(const __
       }
     }
   }
-  leave(sm, tmem, warp, timeouts);
+  leave(sm, tmem, warp, timeouts, [&] {
+    for (int i = 0; i < 2; ++i)
+      for (int t = max(0, sm.issued[i] - 2); t < sm.issued[i]; ++t) wait_in_flight(smem_u32(i ? &sm.v_full[t & 1] : &sm.k_full[t & 1]), (t >> 1) & 1);
+  });
 }
 
 }  // namespace

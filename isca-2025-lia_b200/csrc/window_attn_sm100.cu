@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(THREADS, 1) window_prompt_tc_kernel(const void
         if ((again >> i) & 1u) by_itself(row0 + r0 + i, slot, pos0 + r0 + i);
     }
   }
-  leave(sm, tmem, warp, timeouts);
+  leave(sm, tmem, warp, timeouts, [] {});                          // (each loading thread has waited for its own)
 }
 
 template <int NQ>

@@ -34,3 +34,15 @@ def test_rows_that_are_not_put_are_formed_again():
     assert callers == ["latent_attn_sm100.cu", "window_attn_sm100.cu"]
     for name in callers:
         assert re.search(r"rows_out\([^;]*?O, inv, alive, ", SOURCES[name]) and "    if (again) {" in SOURCES[name], name
+
+
+def test_loads_under_way_are_waited_for_after_the_last_wait():
+    """A warp that has asked for all its loads may be done before another's wait runs out: what is under way is waited for behind the block's last barrier, when no wait is left to run out."""
+    found = 0
+    for name, text in SOURCES.items():
+        if "wait_in_flight(" not in text or name == "umma.cuh":
+            continue
+        last = max(text.rfind(s) for s in ("wait_for(", "warp_wait("))
+        assert text.index("wait_in_flight(") > last or name in ("attn_sm100.cuh", "ssd_chunk_sm100.cu"), name      # (one holds functions, the other several kernels without such loads)
+        found += "tma_load_2d(" in text
+    assert found == 3
