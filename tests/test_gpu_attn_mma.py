@@ -115,9 +115,10 @@ def test_what_the_general_kernel_keeps():
 
 @pytest.mark.parametrize("q_f32", [False, True])
 @pytest.mark.parametrize("at", [[(0, 5), (1, 69)], [(0, 69), (0, 68), (0, 0)], None])
-def test_one_portion_announced_whose_rows_are_others(q_f32, at):
+@pytest.mark.parametrize("d", [64, 128])                            # heads of 128: csrc/window_attn_sm100.cu
+def test_one_portion_announced_whose_rows_are_others(q_f32, at, d):
     """Without segments `nseg` is advice: a row's slot and position come from meta alone, up to the caches' last rows."""
-    H, G, d, cap, M = 4, 2, 64, 70, 130
+    H, G, cap, M = 4, 2, 70, 130
     g = torch.Generator().manual_seed(4)
     q = torch.randn(M, H * d, generator=g).to(F32 if q_f32 else BF16).to(DEV)
     kc, vc = (torch.randn(2, cap, G * d, generator=g).to(BF16).to(DEV) for _ in range(2))

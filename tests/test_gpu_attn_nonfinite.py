@@ -1,5 +1,5 @@
-"""Numbers that are not finite in the keys and values of the tensor-core attention kernels (csrc/window_attn_mma.cu, csrc/latent_attn_mma.cu): a row that
-sees them says so, and no other row does."""
+"""Numbers that are not finite in the keys and values of the tensor-core attention kernels (csrc/window_attn_mma.cu and csrc/window_attn_sm100.cu, csrc/latent_attn_mma.cu and
+csrc/latent_attn_sm100.cu): a row that sees them says so, and no other row does."""
 import pytest
 import torch
 

@@ -1,6 +1,6 @@
 """Prompts through window attention on tcgen05 (csrc/window_attn_sm100.cu) against a float64 softmax, where its tiles can go wrong: portions of 1 to 300 rows behind 0 to 700
 positions (blocks of 64 keys to the second turn of the ring, tiles of 128 rows), windows and chunks that hide whole blocks from some warps, scores beyond and below the soft cap's short form,
-gates whose rows are whole 16-byte vectors and not, bf16 and fp32 outputs."""
+gates whose rows are whole vectors and not, bf16 and fp32 outputs."""
 import pytest
 import torch
 
@@ -37,9 +37,10 @@ def test_portions(q_f32, H, G, v_div, opt):
         ops.window_attn(q[r0:r0 + n].contiguous(), kc, vc, meta[r0:r0 + n].contiguous(), dev["temp"], alone, H, G, d, d, opt.get("window", 0), 0.1, opt.get("softcap", 0.0), nseg=1,
                         segs=torch.tensor([(slot, p0, 0, n)], dtype=torch.int32, device=DEV), max_ctx=p0 + n, slopes=dev["slopes"], sink=dev["sink"], chunk=opt.get("chunk", 0), v_div=v_div)
         assert n == 1 or torch.equal(alone, out[r0:r0 + n])
-    for pad in (0, 4):                                              # one rounding to bf16 of numbers up to the largest
-        wide = torch.randn(q.shape[0], H * d + 8 + pad, generator=g).to(BF16).to(DEV)
-        gate = wide[:, 8:8 + H * d]
+    for first, pad in ((8, 0), (8, 4), (8, 1), (1, 7)):             # rows of whole 16 and 8 bytes, rows and a first one at 2; one rounding to bf16 of numbers up to the largest
+        wide = torch.randn(q.shape[0], first + H * d + pad, generator=g).to(BF16).to(DEV)
+        gate = wide[:, first:first + H * d]
+        assert (gate.data_ptr() | 2 * gate.stride(0)) % 8 == (0 if first == 8 and pad != 1 else 2)
         got = want * torch.sigmoid(gate.cpu().to(F64))
         assert float((run(BF16, gate).cpu().to(F64) - got).abs().max() / got.abs().max()) < 2.0 ** -8
 
