@@ -18,7 +18,12 @@ namespace {
 constexpr int THREADS = 128;
 constexpr int MAX_CHUNK = 4096;   // keys per CTA (scores kept in smem)
 
-template <int D>
+// UNROLL: rows in flight per lane.  Ten take 72 registers, seven CTAs an SM and 143 KB in flight there.  B=64 H=56 d=128 T=289:
+// 77.8 us (6.8 TB/s); with 4, 6, 8, 12: 80.7, 77.8, 82.3, 84.6.  B=16 H=32 d=64 T=300, where few CTAs leave each its own
+// latency to wait for: 9.7 us; with 4, 6, 8, 12: 15.4, 15.6, 13.8, 11.0.  B=96 H=32 d=128: 68 us; 79, 74, 70, 85.
+// Four at a time with a wait for all of them before the next four, and nothing in flight during the softmax, took 90.9, 18.0
+// and 89.9 us.  Which row a lane adds, and in which order, does not depend on this number.
+template <int D, int UNROLL>
 __global__ void __launch_bounds__(THREADS) attn_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kc,
                                                               const bf16* __restrict__ vc, bf16* __restrict__ out,
                                                               float* __restrict__ ws, int T, int H, int cache_batch,
@@ -27,12 +32,6 @@ __global__ void __launch_bounds__(THREADS) attn_decode_kernel(const bf16* __rest
   pdl_wait();
   constexpr int LPR = D / 8;        // lanes per cached row (each lane owns 8 dims = 16 bytes)
   constexpr int RPW = 32 / LPR;     // rows per warp iteration
-  // Rows in flight per lane.  Ten take 72 registers, seven CTAs an SM and 143 KB in flight there.  B=64 H=56 d=128 T=289:
-  // 77.8 us (6.8 TB/s); with 4, 6, 8, 12: 80.7, 77.8, 82.3, 84.6.  B=16 H=32 d=64 T=300, where few CTAs leave each its own
-  // latency to wait for: 9.7 us; with 4, 6, 8, 12: 15.4, 15.6, 13.8, 11.0.  B=96 H=32 d=128: 68 us; 79, 74, 70, 85.
-  // Four at a time with a wait for all of them before the next four, and nothing in flight during the softmax, took 90.9, 18.0
-  // and 89.9 us.  Which row a lane adds, and in which order, does not depend on this number.
-  constexpr int UNROLL = 10;
   extern __shared__ float sc[];     // [t_chunk] scores -> probabilities
   __shared__ float red[4];
   __shared__ float accs[4][D];
@@ -154,6 +153,14 @@ __global__ void __launch_bounds__(THREADS) attn_decode_kernel(const bf16* __rest
   }
 }
 
+// A short range's rows are all in flight from the start, and every lane goes through the places of those that are not there: the fewest of 2, 4 and 10 that hold the range.  With 2, 4, 10, and
+// four at a time as above, us: B=96 H=56 d=128 T=8 9.6, 13.6, 23.7 (14.6), T=32 17.1, 16.3, 25.7 (19.5), T=48 23.1, 24.2, 27.9 (28.2); B=64 H=32 d=64 T=32 6.4, 7.0, 9.9 (8.2), T=64 9.7, 8.2, 11.3
+// (11.3), T=80 12.2, 11.1, 11.9 (14.8).
+template <int D> auto kernel_for(int range) {
+  constexpr int STEP = 4 * 256 / D;          // rows of a CTA's lanes
+  return range <= 2 * STEP ? attn_decode_kernel<D, 2> : range <= 4 * STEP ? attn_decode_kernel<D, 4> : attn_decode_kernel<D, 10>;
+}
+
 template <int D>
 __global__ void attn_decode_combine_kernel(const float* __restrict__ ws, bf16* __restrict__ out, int splits) {
   pdl_launch_dependents();
@@ -226,11 +233,11 @@ extern "C" int lia_attn_decode_bf16(const void* q, const void* k_cache, const vo
   bf16* op = reinterpret_cast<bf16*>(out);
   float* wsp = reinterpret_cast<float*>(workspace);
   if (d == 128) {
-    lia_launch(attn_decode_kernel<128>, dim3(grid), dim3(THREADS), smem, stream, qp, kp, vp, op, wsp, T, H, cache_batch, b0, t_chunk, splits);
+    lia_launch(kernel_for<128>(t_chunk), dim3(grid), dim3(THREADS), smem, stream, qp, kp, vp, op, wsp, T, H, cache_batch, b0, t_chunk, splits);
     LIA_LAUNCH_CHECK();
     if (splits > 1) lia_launch(attn_decode_combine_kernel<128>, dim3(B * H), dim3(128), 0, stream, wsp, op, splits);
   } else {
-    lia_launch(attn_decode_kernel<64>, dim3(grid), dim3(THREADS), smem, stream, qp, kp, vp, op, wsp, T, H, cache_batch, b0, t_chunk, splits);
+    lia_launch(kernel_for<64>(t_chunk), dim3(grid), dim3(THREADS), smem, stream, qp, kp, vp, op, wsp, T, H, cache_batch, b0, t_chunk, splits);
     LIA_LAUNCH_CHECK();
     if (splits > 1) lia_launch(attn_decode_combine_kernel<64>, dim3(B * H), dim3(64), 0, stream, wsp, op, splits);
   }

@@ -1,5 +1,5 @@
-"""Decode attention around the edges of its stream of row loads: a CTA's four warps keep ten rows a lane on their way, K's and
-then V's, so that histories just below, at and above whole batches (80 rows of 128 values, 160 of 64) take every mixture of
+"""Decode attention around the edges of its stream of row loads: a CTA's four warps keep ten rows a lane on their way, two or four where those are all, K's and
+then V's, so that histories just below, at and above whole batches (16, 32 and 80 rows of 128 values, 32, 64 and 160 of 64) take every mixture of
 "the next row is K's", "is V's" and "is not there"."""
 import pytest
 import torch
@@ -9,8 +9,9 @@ from test_gpu_kernels import attn_ref, close_bf16, ops, rnd  # noqa: F401  (ops 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("d,T,splits", [(128, t, 1) for t in (2, 7, 8, 9, 79, 80, 81, 160, 161)] +
-                         [(64, t, 1) for t in (15, 17, 159, 160, 161, 321)] + [(128, 167, 2), (64, 331, 3)])
+@pytest.mark.parametrize("d,T,splits", [(128, t, 1) for t in (1, 2, 7, 8, 9, 15, 16, 17, 31, 32, 33, 79, 80, 81, 160, 161)] +
+                         [(64, t, 1) for t in (1, 15, 17, 31, 32, 33, 63, 64, 65, 159, 160, 161, 321)] +
+                         [(128, 167, 2), (64, 331, 3), (128, 64, 2), (128, 31, 2), (64, 130, 2)])
 def test_histories_around_whole_batches(ops, d, T, splits):  # noqa: F811
     B, H, Bc, b0 = 2, 3, 4, 1
     q = rnd(B, H, d, std=0.3, seed=4)
