@@ -1,6 +1,8 @@
 """Prompts through window attention on tcgen05 (csrc/window_attn_sm100.cu) against a float64 softmax, where its tiles can go wrong: portions of 1 to 300 rows behind 0 to 700
 positions (blocks of 64 keys to the second turn of the ring, tiles of 128 rows), windows and chunks that hide whole blocks from some warps, scores beyond and below the soft cap's short form,
 gates whose rows are whole vectors and not, bf16 and fp32 outputs."""
+import math
+
 import pytest
 import torch
 
@@ -102,3 +104,15 @@ def test_short_portions(step, q_f32, opt):
     for slot, p0, r0, n in segs:
         if n > 128:
             assert torch.equal(run([(slot, p0, 0, n)], slice(r0, r0 + n), None), run(segs, whole, form)[r0:r0 + n])
+
+
+@pytest.mark.parametrize("q_f32", [False, True])
+def test_weights_below_the_smallest_normal_number(q_f32):
+    """A weight of exp(-88.5) = 2^-127.7, as three parts of which the first has five bits left, times a value of 2^127."""
+    H, d = 2, 128
+    q, kc, vc = torch.zeros(2, H * d, device=DEV), torch.zeros(1, 2, H * d, device=DEV), torch.zeros(1, 2, H * d, device=DEV)
+    q[:, ::d], kc[0, 1, ::d], vc[0, 1, 5] = 1.0, -88.5, 2.0 ** 127
+    out = torch.empty(2, H * d, device=DEV)
+    ops.window_attn(q if q_f32 else q.to(BF16), kc.to(BF16), vc.to(BF16), torch.tensor([(0, 0), (0, 1)], dtype=torch.int32, device=DEV), None, out, H, H, d, d, 0, 1.0, 0.0, nseg=1, form=2)
+    want = math.exp(-88.5) * 2.0 ** 127
+    assert abs(float(out[1, 5]) / want - 1) < 2.0 ** -5 and float(out.abs().sum() - out[1, 5].abs()) == 0.0

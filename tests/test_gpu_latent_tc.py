@@ -68,3 +68,13 @@ def test_expansion(dim, rank):
     ops.latent_attn_expanded(q, qr, lat, [(1, 0, 0, cap)], w, None, out, H, dim, ROT, rank, 1.0, window=1)
     want = lat[1, :, :rank].to(F64) @ w[H * dim:].to(F64).T
     assert float((out.to(F64) - want).abs().max()) < 2.0 ** -20      # sums of size up to 5: a few last places of 2^-21
+
+
+def test_weights_below_the_smallest_normal_number():
+    """A weight of exp(-88.5) = 2^-127.7, as three parts of which the first has five bits left, times a value of 2^127."""
+    H = 2
+    q, qr, lat, w = (torch.zeros(*s, device="cuda") for s in ((2, H * (DIM + ROT)), (2, H, ROT), (1, 2, RANK + ROT), (2 * H * DIM, RANK)))
+    qr[:, :, 3], lat[0, 1, RANK + 3], lat[0, 1, 7], w[H * DIM + 5, 7] = 1.0, -88.5, 2.0 ** 100, 2.0 ** 27
+    out = torch.empty(2, H * DIM, device="cuda")
+    ops.latent_attn_expanded(q.to(BF16), qr, lat.to(BF16), [(0, 0, 0, 2)], w.to(BF16), None, out, H, DIM, ROT, RANK, 1.0)
+    assert abs(float(out[1, 5]) / (math.exp(-88.5) * 2.0 ** 127) - 1) < 2.0 ** -5 and float(out.abs().sum() - out[1, 5].abs()) == 0.0
