@@ -5,10 +5,10 @@
 // and values are kept as three bf16 parts of their fp32 sums, and so are the rotated query parts and the softmax's weights (mma.cuh).  With bf16
 // queries and bf16 rotated keys a score is three products of each part, a weighted value six (of the nine).
 //
-// Heads of 128 + 64 channels are latent_attn_sm100.cu's.  Here, for heads of 64 + 64, one block per (64 rows, head), warp by 16 rows, the scores becoming the weights' operand in registers; 32 keys
-// per stage.  Keys and values are fetched in turn (the next keys while the values are taken in, the next values while the scores are made), so one stage is enough and several blocks share an SM.
-// Bound: tensor cores and shared-memory reads about equally.  2048 tokens, 16 heads of 128 + 64 on latents of 512: 4794 us in the latent space on the CUDA cores and 439 us for its two projections ->
-// 352 here (104 there) and 67 us for the expansion (29: latent_expand_sm100.cu).
+// Heads of 128 + 64 channels are latent_attn_sm100.cu's (2048 tokens, 16 heads on latents of 512: 4794 us in the latent space on the CUDA cores and 439 us for its two projections; 130 there with the
+// expansion).  Here, for heads of 64 + 64, one block per (64 rows, head), warp by 16 rows, the scores becoming the weights' operand in registers; 32 keys per stage.  Keys and values are fetched in turn
+// (the next keys while the values are taken in, the next values while the scores are made), so one stage is enough and several blocks share an SM.  Bound: tensor cores and shared-memory reads about
+// equally.  With the expansion, latents of 512: 2048 tokens, 16 heads 252 us; 700 rows behind 300, 32 heads 141; 64 rows, 16 heads 14.
 // Rows whose sums are not finite are formed again key by key at the end, as in window_attn_mma.cu: a masked key's weight of 0 still meets its value.
 #include <limits.h>
 #include <math.h>

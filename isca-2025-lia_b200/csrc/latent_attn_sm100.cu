@@ -12,9 +12,9 @@
 // Sums that are not finite stay so to the end, where such rows are formed again key by key: a masked key's weight of 0 still meets its value.
 // Waits are bounded: a CTA that gives up leaves NaN and counts itself (lia_moe_timeouts_seen()).
 //
-// Latents of 512, with their expansion (latent_expand_sm100.cu); on mma.sync -> here, us, and the error against 64 bits in 1e-7: 2048 rows, 16 heads 419 (1.97) -> 132 (1.84); 700 rows behind 300,
-// 32 heads 251 (2.21) -> 98 (2.07); portions of 300, 250 and 200, 16 heads 89 (1.75) -> 38 (1.61); 64 rows 29 (1.61) -> 15 (1.42); 100 rows behind 1500, 32 heads 377 (2.31) -> 123 (2.35), 8 heads 210
-// (2.31) -> 90 (2.26).
+// Latents of 512, with their expansion (latent_expand_sm100.cu); on mma.sync -> here, us, and the error against 64 bits in 1e-7, means over 16 inputs: 2048 rows, 16 heads 413 (1.97) -> 130 (1.83); 700
+// rows behind 300, 32 heads 250 (2.22) -> 96 (2.08); portions of 300, 250 and 200, 16 heads 88 (1.75) -> 36 (1.60); 64 rows 28 (1.55) -> 14 (1.41); 100 rows behind 1500, 32 heads 376 (2.30) -> 122
+// (2.22), 8 heads 210 (2.30) -> 89 (2.23).
 #include "attn_sm100.cuh"
 #include "latent_attn_rows.cuh"
 

@@ -1,5 +1,5 @@
-// tcgen05 / TMEM / TMA / mbarrier PTX wrappers and the tensor-map encoder shared by the sm_100a kernels of libliab200
-// (gemm_sm100.cu, attn_prefill_sm100.cu).  Everything here is a thin inline wrapper: no policy, no state.
+// tcgen05 / TMEM / TMA / mbarrier PTX wrappers and the tensor-map encoder shared by the sm_100a kernels of libliab200 (*_sm100.cu).
+// Everything here is a thin inline wrapper: no state, and no policy but the limit of a wait.
 #pragma once
 #include <cuda.h>
 
@@ -112,17 +112,6 @@ __device__ __forceinline__ void tcgen05_commit_pair(uint32_t bar) {   // arrives
                "h"((uint16_t)3)
                : "memory");
 }
-__device__ __forceinline__ void tcgen05_mma_f16_pair(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                                     uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}" ::"r"(d_tmem),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 __device__ __forceinline__ void tcgen05_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tcgen05_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tcgen05_commit(uint32_t bar) {
@@ -159,17 +148,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* v) {
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// A from TMEM (16 numbers of a row in 8 columns)
-__device__ __forceinline__ void mma_tmem_a(uint32_t d, uint32_t a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "}" ::"r"(d),
-      "r"(a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* v) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
@@ -207,6 +185,7 @@ __device__ __forceinline__ void mma_if(uint32_t one, uint32_t d, uint64_t a, uin
                "r"(accumulate), "r"(one)
                : "memory");
 }
+// A from TMEM (16 numbers of a row in 8 columns)
 __device__ __forceinline__ void mma_tmem_a_if(uint32_t one, uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
   asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc),
                "r"(accumulate), "r"(one)

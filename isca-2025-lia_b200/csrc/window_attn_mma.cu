@@ -3,10 +3,10 @@
 // weights enter as three bf16 parts (mma.cuh), scores and sums are fp32.
 //
 //   prompt:  one block per (64 rows of one portion, query head); with heads of 128 + 128 channels only for many short portions (lia_window_prompt_form), the others are
-//            window_attn_sm100.cu's.  Bound: tensor cores and the softmax's instructions about equally -- mma.sync m16n8k16, one product for q . k (three for fp32 queries) and three for the weights times the values.  A warp owns 16 rows: its
-//            16 x 32 scores become the weights' operand in registers, so nothing but keys and values passes through shared memory; those come
-//            by cp.async, two stages of 32 keys (64 keys need 255 registers: two blocks per SM instead of three, 185 instead of 159 us).
-//            2048 tokens, 16 heads of 128 on 8 key heads, window 1024, soft cap: 1183 -> 136 us; the whole history, fp32 queries: 1713 -> 182 us (such heads: 66 and 64 us there).
+//            window_attn_sm100.cu's.  Bound: tensor cores and the softmax's instructions about equally -- mma.sync m16n8k16, one product for
+//            q . k (three for fp32 queries) and three for the weights times the values.  A warp owns 16 rows: its 16 x 32 scores become the
+//            weights' operand in registers, so nothing but keys and values passes through shared memory; those come by cp.async, two stages of 32 keys (64 keys need 255 registers: two blocks per SM instead of three, 185 instead of 159 us).
+//            2048 tokens, 16 heads of 128 on 8 key heads, window 1024, soft cap: 1183 -> 136 us; the whole history, fp32 queries: 1713 -> 182 us (66 and 63 us there).
 //   decode:  one block per (row, up to 8 query heads of one key/value head, range of keys).  Bound: HBM.  The heads of a group are the rows of
 //            the matrix instruction and a warp reads every cached row once for all of them, straight from global memory into operand
 //            registers: channels and value columns may be taken in any order as long as q and the output follow it, so a lane's 16

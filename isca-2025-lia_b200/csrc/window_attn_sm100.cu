@@ -10,9 +10,9 @@
 // Sums that are not finite stay so to the end, where such rows are formed again key by key (window_attn_rows.cuh): a masked key's weight of 0 still meets its value.
 // Waits are bounded: a CTA that gives up leaves NaN and counts itself (lia_moe_timeouts_seen()).
 //
-// 8 key heads of 128; on mma.sync -> here, us, and the error against 64 bits in 1e-7: 2048 rows, 16 heads, window of 1024 and soft cap 136 (1.87) -> 66 (1.68), the whole history and fp32 queries
-// 182 (2.42) -> 63 (1.69); 700 rows behind 300 91 (2.43) -> 35 (2.16); portions of 300, 250, 200 31 (1.54) -> 17 (1.49); 64 rows 9.3 (1.37) -> 9.1 (1.19);
-// 33 rows 8.7 (1.18) -> 9.0 (0.97).  Four portions of 117, 100, 87, 73 behind a gate per channel: 24 -> 15 (33 with the gates asked for row by row).
+// 16 heads on 8 key heads of 128; on mma.sync -> here, us, and the error against 64 bits in 1e-7, means over 16 inputs: 2048 rows, window of 1024 and soft cap 136 (1.91) -> 66 (1.72), the whole history
+// and fp32 queries 182 (2.32) -> 63 (1.62); 700 rows behind 300 89 (2.22) -> 29 (1.88); portions of 300, 250, 200 29 (1.35) -> 14 (1.26); 100 rows behind 2000 130 -> 50 (behind
+// 1500 2.71 -> 2.05); four portions of 117, 100, 87, 73 14 -> 10, behind a gate per channel 23 -> 20.  Where mma.sync is the faster one: lia_window_prompt_form.
 #include <limits.h>
 
 #include "attn_sm100.cuh"

@@ -712,7 +712,8 @@ def moe_gemm_tc(a, w, out, perm, tile_expert, wt, up, act=ACT_NONE, gated=False,
 
 
 def moe_timeouts_seen():
-    """Blocks of ``moe_gemm_tc`` that gave up a wait in any launch that has ended (their results are NaN).  Does not synchronise."""
+    """Blocks of ``moe_gemm_tc``, of the state-space scan and of prompt attention over windows and latents that gave up a wait in any launch that has ended (their
+    results are NaN).  Does not synchronise."""
     return _lib.load().lia_moe_timeouts_seen()
 
 

@@ -160,7 +160,7 @@ class LatentAttentionMixer:
 
     EXPAND_ROWS = 64          # portions of at least this many rows may expand the latents they see ...
     EXPAND_RATIO = 4          # ... if these are at most this many times the rows
-    # The tensor-core form, which keeps expanded keys and values as exact as fp32 (csrc/latent_attn_mma.cu), for designs with a rotated part or a gate:
+    # The tensor-core form, which keeps expanded keys and values as exact as fp32 (csrc/latent_attn_sm100.cu, csrc/latent_attn_mma.cu), for designs with a rotated part or a gate:
     # The portion alone decides (``_expands_exactly``), whatever else is in the step.
     EXPAND_ROWS_EXACT = 16             # fewer rows never
     EXPAND_WORK_ALWAYS = 128           # rows x groups of 8 heads: from here on whatever the history
@@ -263,11 +263,13 @@ class LatentAttentionMixer:
         return self.out(o)
 
     def _expands_exactly(self, q, portions, H):
-        """The portions (by number) whose latents are expanded to keys and values as exact as fp32.  A block walks a portion's keys for 64 rows of one head
-        whether it has them or not, while the kernel in the latent space takes as long as rows x groups of 8 heads and splits few rows' keys over the GPU.  Time
-        of a mixer's kernels, latent space | expanded, in us, for rows that see 256, 1024, 8192 keys -- 8 heads: 24 rows 91 | 82, 109 | 161, 430 | 1228; 64 rows
-        145 | 101, 197 | 173, 1095 | 1285; 16 heads: 16 rows 93 | 85, 119 | 177, 548 | 1119; 33 rows 133 | 98, 220 | 186, 1077 | 1266; 64 rows 216 | 98, 374 | 193,
-        1842 | 1296.  Heads that do not fit EXPAND_KEYS_EXACT go in turn, which needs enough blocks each time."""
+        """The portions (by number) whose latents are expanded to keys and values as exact as fp32.  A block walks a portion's keys for 64 (heads of 64 channels) or 128
+        rows of one head whether it has them or not, while the kernel in the latent space takes as long as rows x groups of 8 heads and splits few rows' keys over the
+        GPU.  The line was drawn with expanded keys on mma.sync, as heads of 64 channels still have them; heads of 128 would be faster expanded on its other side too.
+        Time of such a mixer's kernels, latent space | expanded on mma.sync | on tcgen05, in us, for rows that see 256, 1024, 8192 keys -- 8 heads: 24 rows 66 | 69 | 41,
+        86 | 149 | 75, 390 | 1128 | 437; 64 rows 104 | 74 | 42, 156 | 176 | 79, 1030 | 1175 | 442; 16 heads: 16 rows 69 | 73 | 46, 97 | 166 | 90, 505 | 1128 | 523; 33 rows
+        98 | 80 | 52, 184 | 174 | 97, 1044 | 1152 | 526; 64 rows 155 | 87 | 56, 313 | 182 | 99, 1780 | 1179 | 534.  Heads that do not fit EXPAND_KEYS_EXACT go in turn, which
+        needs enough blocks each time: 16 heads, 20000 keys, 256 rows 12.7 | 6.3 | 2.2 ms, 640 rows 30.6 | 6.3 | 2.3."""
         if self.w_ukv is None or q.data_ptr() % 16 or q.stride(0) % 8:
             return ()
         found = []
