@@ -75,8 +75,8 @@ template <int DIM, int L> struct ChunkSmem {
 // instructions, 2 KS + 12 beside a step's 12, for a step's are less of a chain), and the warps of a row block that have fewer blocks of scores take more steps.  The chain of two portions of 1003 tokens,
 // 4 heads of 256 x 512: 132 us with a block counted by its instructions and all warps in the scores' loop, 125 without those that have none there and a block for nine steps, 118 for five.  Where
 // two warps share a row block, six steps of one of them are a longer chain of fp32 additions and put outputs off by 1.006 times as much: five at most.  As many steps for each warp as before -- as
-shared now, outputs off by, in 1e-7, means over 24 inputs: four warps (256 x 512, up to six steps) 120 tokens 2.407 -- 2.408, 503 2.480 -- 2.478, 1003 2.773 -- 2.772; two (128 x 128, up to five)
-64 tokens 0.776 -- 0.776, 200 0.829 -- 0.828, 1024 1.027 -- 1.028.
+// shared now, outputs off by, in 1e-7, means over 24 inputs: four warps (256 x 512, up to six steps) 120 tokens 2.407 -- 2.408, 503 2.480 -- 2.478, 1003 2.773 -- 2.772; two (128 x 128, up to five)
+// 64 tokens 0.776 -- 0.776, 200 0.829 -- 0.828, 1024 1.027 -- 1.028.
 template <int RB, int WPR, int KS> struct Shares {
   int from[RB][WPR + 1];
   constexpr Shares() : from{} {
