@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_expanded_tc_kernel(const __
     };
     const float inv = !alive ? NAN : r0 + lane < rows ? factor(row0 + r0 + lane, sm.top[(n - 1) & 1][r0 + lane] * unit, (float)l) : 0.f;
     // (the keys' and values' place: every product is done)
-    const unsigned again = rows_out(gen + K_SMALL + (warp & 3) * (32 * D * 4), O, inv, alive, rows - r0, false, [](int) { return make_uint2(0u, 0u); }, [](float4&, uint2) {}, [&](int i, float4 y) {
+    const unsigned again = rows_out(gen + K_SMALL + (warp & 3) * (32 * D * 4), O, inv, alive, rows - r0, false, [](int, float4&) {}, [&](int i, float4 y) {
       const size_t at = ((size_t)(row0 + r0 + i) * a.H + h) * DN + lane * 4;
       if (a.out_f32) *reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + at) = y;
       else *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(a.out) + at) = make_uint2(pack_bf16x2(y.x, y.y), pack_bf16x2(y.z, y.w));

@@ -15,6 +15,7 @@
 // 1500 2.71 -> 2.05); four portions of 117, 100, 87, 73 14 -> 10, behind a gate per channel 23 -> 20.  Where mma.sync is the faster one: lia_window_prompt_form.
 #include <limits.h>
 
+#include "act.cuh"
 #include "attn_sm100.cuh"
 #include "window_attn_rows.cuh"
 
@@ -339,26 +340,36 @@ __global__ void __launch_bounds__(THREADS, 1) window_prompt_tc_kernel(const void
     double l;
     const bool alive = sum_blocks(sm, tmem, n, O, l);
     const float inv = alive ? 1.0f / ((float)l + (x.sink ? expf(x.sink[h] - sm.top[(n - 1) & 1][r0 + lane]) : 0.f)) : NAN;
-    // (the keys' and values' place: every product is done)
-    const bool gate_pairs = a.gate_mode == 2 && (reinterpret_cast<uintptr_t>(x.gate) | (uintptr_t)(a.ldg * 2)) % 8 == 0;
-    auto gates = [&](int i) {                                      // four of a row's gates before their sigmoid, or the head's
-      const size_t row = row0 + r0 + i;
-      if (a.gate_mode == 1) return make_uint2(__float_as_uint(reinterpret_cast<const float*>(x.gate)[row * a.H + h]), 0u);
-      const unsigned short* g = reinterpret_cast<const unsigned short*>(x.gate) + row * a.ldg + (size_t)h * D + lane * 4;
-      return gate_pairs ? *reinterpret_cast<const uint2*>(g) : make_uint2(g[0] | (uint32_t)g[1] << 16, g[2] | (uint32_t)g[3] << 16);
-    };
-    auto gate = [&](float4& y, uint2 u) {
+    // Every product is done: the sums' way out takes the keys' and values' place, the gates, before their sigmoid, the queries'.  By way of shared memory they are under way while the sums are written,
+    // and a loop of four rows is enough; eight rows' in registers, with the compiler's division, took a tile 10 us for 2.8 (mma.sync: 4.5 to 8.5).
+    uint8_t* gates = raw + (base - smem_u32(raw)) + (warp & 3) * (32 * D * 2);
+    float head_gate = 0.f;
+    if (a.gate_mode == 1 && r0 + lane < rows) head_gate = reinterpret_cast<const float*>(x.gate)[(size_t)(row0 + r0 + lane) * a.H + h];
+    if (a.gate_mode == 2) {
+      const unsigned short* g = reinterpret_cast<const unsigned short*>(x.gate) + (size_t)(row0 + r0) * a.ldg + (size_t)h * D + lane * 4;
+      const int n = min(32, rows - r0);
+      if ((reinterpret_cast<uintptr_t>(x.gate) | (uintptr_t)(a.ldg * 2)) % 8 == 0) {
+#pragma unroll 4
+        for (int i = 0; i < n; ++i) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(gates) + i * (D * 2) + lane * 8), "l"(g + (size_t)i * a.ldg) : "memory");
+      } else {
+#pragma unroll 1
+        for (int i = 0; i < n; ++i, g += a.ldg) reinterpret_cast<uint2*>(gates)[i * 32 + lane] = make_uint2(g[0] | (uint32_t)g[1] << 16, g[2] | (uint32_t)g[3] << 16);
+      }
+      cp_async_commit();
+    }
+    auto gate = [&](int i, float4& y) {
       float4 g;
       if (a.gate_mode == 1) {
-        g.x = g.y = g.z = g.w = __uint_as_float(u.x);
+        g.x = g.y = g.z = g.w = __shfl_sync(0xffffffffu, head_gate, i);
       } else {
+        const uint2 u = reinterpret_cast<const uint2*>(gates)[i * 32 + lane];
         unpack_bf16x2(u.x, g.x, g.y);
         unpack_bf16x2(u.y, g.z, g.w);
-        g = make_float4(1.0f / (1.0f + expf(-g.x)), 1.0f / (1.0f + expf(-g.y)), 1.0f / (1.0f + expf(-g.z)), 1.0f / (1.0f + expf(-g.w)));
+        g = make_float4(over(1.0f, 1.0f + expf(-g.x)), over(1.0f, 1.0f + expf(-g.y)), over(1.0f, 1.0f + expf(-g.z)), over(1.0f, 1.0f + expf(-g.w)));
       }
       y = make_float4(y.x * g.x, y.y * g.y, y.z * g.z, y.w * g.w);
     };
-    const unsigned again = rows_out(raw + (ks - smem_u32(raw)) + (warp & 3) * (32 * D * 4), O, inv, alive, rows - r0, a.gate_mode != 0, gates, gate, [&](int i, float4 y) {
+    const unsigned again = rows_out(raw + (ks - smem_u32(raw)) + (warp & 3) * (32 * D * 4), O, inv, alive, rows - r0, a.gate_mode != 0, gate, [&](int i, float4 y) {
       const size_t at = ((size_t)(row0 + r0 + i) * a.H + h) * D + lane * 4;
       if (a.out_f32) *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + at) = y;
       else *reinterpret_cast<uint2*>(out + at) = make_uint2(pack_bf16x2(y.x, y.y), pack_bf16x2(y.z, y.w));
