@@ -500,8 +500,8 @@ int lia_window_attn_masked(const void* q, int ldq, int q_f32, int act_f32, const
 int lia_window_attn_mma_takes(const void* q, int ldq, int q_f32, const void* kcache, long long k_slot_stride, const void* vcache,
                               long long v_slot_stride, const void* out, int H, int G, int v_div, int dim, int vdim);
 /* Which of two kernels of lia_window_attn_mma take a step's portions of prompts with heads of 128 + 128 channels, by the time that either is expected to need.  `portions`: the numbers of `segs` on the host; NULL: not known there,
- * as with prompt = 1.  window, chunk as in lia_window_attn_mma. */
-int lia_window_prompt_form(const int* portions, int nseg, int M, int H, int window, int chunk);
+ * as with prompt = 1.  window, chunk as in lia_window_attn_mma; gated: with a gate per channel. */
+int lia_window_prompt_form(const int* portions, int nseg, int M, int H, int window, int chunk, int gated);
 /* lia_window_attn_masked on the tensor cores, for bf16 caches.  prompt != 0: the rows belong to nseg portions, segs[s] = {slot, first position,
  * first row, rows} on the device (NULL: all rows are one portion that continues from meta's first row); prompt == 0: every row by itself,
  * its keys in nsplit ranges (workspace as for lia_window_attn).  prompt is 1 or, with heads of 128 + 128 channels, lia_window_prompt_form() of the same portions. */

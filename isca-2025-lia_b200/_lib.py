@@ -174,7 +174,7 @@ _PROTOTYPES = {
                                        c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                        c_int, c_int, c_float, c_float, c_int, c_int, c_int, c_void_p]),
     "lia_window_attn_mma_takes": (c_int, [c_void_p, c_int, c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int]),
-    "lia_window_prompt_form": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int]),
+    "lia_window_prompt_form": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int]),
     "lia_window_attn_mma": (c_int, [c_void_p, c_int, c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                     c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                     c_int, c_float, c_float, c_int, c_int, c_void_p]),

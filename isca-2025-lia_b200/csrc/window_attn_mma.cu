@@ -507,7 +507,7 @@ constexpr int TILE_BITS = 14, TILE_MASK = (1 << TILE_BITS) - 1;
 template <int DK, int DV> int run_as(const Call& c, int prompt) {
   if (prompt) {
     if constexpr (DK == 128 && DV == 128) {
-      if (prompt == 1) prompt = lia_window_prompt_form(nullptr, c.segs ? c.nseg : 1, c.M, c.a.H, c.a.window, c.a.chunk);
+      if (prompt == 1) prompt = lia_window_prompt_form(nullptr, c.segs ? c.nseg : 1, c.M, c.a.H, c.a.window, c.a.chunk, c.a.gate_mode == 2);
       const int kernels = prompt & 7, tc_tiles = prompt >> 3 & TILE_MASK, tiles = prompt >> (3 + TILE_BITS) & TILE_MASK;
       if (kernels != MMA_SYNC) {
         const int rc = window_prompt_tc(c.q, c.ldq, c.kcache, c.kss, c.vcache, c.vss, c.meta, c.segs, c.nseg, c.x, c.out, c.M, c.a, kernels == BOTH ? SHORT_ROWS + 1 : 1, tc_tiles, c.stream);
@@ -529,12 +529,12 @@ bool head_sizes_ok(int dim, int vdim) { return (dim == 64 || dim == 128) && (vdi
 // A tile of 128 rows has its SM to itself on tcgen05, however few of the rows are there; one of 64 on mma.sync shares it with two others.  So the first is ahead where tiles are few or histories
 // long, the second with many portions of few rows.  What a step takes is estimated, in us, from the times of 1500 steps of 1 to 64 portions of 1 to 2048 rows behind 0 to 2000 positions, 8 to 32
 // heads, both types of queries (tcgen05: 6.4 a tile and 1.1 for 64 keys; mma.sync: 1.2 a tile of throughput and, with up to 16, 32 or 64 rows, 0.76, 1.1 or 1.3 for 32 keys, of which one
-// tile alone takes 2.75 and 1.8): the kernel with the smaller estimate is the slower one by 3 % or more in 47 of them, by 13 and 22 % at most.
+// tile alone takes 2.75 and 1.8; a gate per channel 2.8 and 4.3 to 8.5 a tile): the kernel with the smaller estimate is the slower one by 3 % or more in 47 of them, by 13 and 22 % at most.
 // us, mma.sync | tcgen05, 32 heads on 8 key heads, rows @ positions before them: 2 @ 0 5.5 | 8.4; 64 @ 256 25 | 14; 32 portions of 16 @ 0 17 | 58, @ 500 118 | 132, @ 1000 210 | 193; of 40 @ 0
 // 29 | 62, @ 256 92 | 99, @ 500 153 | 136; of 96 @ 0 60 | 76, @ 64 92 | 86; of 128 @ 0 80 | 77.
 // A portion of more than 128 rows is always tcgen05's, so that its bits do not depend on its company; a shorter one's may, as those of its projections do (128 rows and fewer in a step are
 // multiplied another way).  Where portions are not known on the host, mma.sync has the steps of more tiles than SMs whose portions have 128 rows or fewer on average.
-extern "C" int lia_window_prompt_form(const int* portions, int nseg, int M, int H, int window, int chunk) {
+extern "C" int lia_window_prompt_form(const int* portions, int nseg, int M, int H, int window, int chunk, int gated) {
   if (nseg <= 0 || M <= 0 || H <= 0) return TCGEN05;
   const int sms = lia_sm_count();
   if (!portions) return nseg > 1 && M <= 128ll * nseg && ((M + 127ll) / 128 + nseg - 1) * H > sms ? MMA_SYNC : TCGEN05;
@@ -550,12 +550,12 @@ extern "C" int lia_window_prompt_form(const int* portions, int nseg, int M, int 
     const int pos = portions[4 * i + 1], rows = portions[4 * i + 3], is_short = rows <= SHORT_ROWS;
     auto keys = [&](int r, int of) { return pos + (r + of < rows ? r + of : rows) - first_key(a, pos + r); };
     for (int r = 0; r < rows; r += 128) {
-      const double t = 6.4 + 1.1 * ((keys(r, 128) + 63) / 64);
+      const double t = 6.4 + 1.1 * ((keys(r, 128) + 63) / 64) + (!gated ? 0 : rows - r <= 16 ? 0.6 : 2.8);
       tc[is_short].take(t, t);
     }
     for (int r = 0; r < rows && is_short; r += 64) {
       const int n = (keys(r, 64) + 31) / 32, here = rows - r;
-      mma[1].take(2.75 + 1.8 * n, 1.2 + (here <= 16 ? 0.76 : here <= 32 ? 1.1 : 1.3) * n);
+      mma[1].take(2.75 + 1.8 * n + (!gated ? 0 : here <= 16 ? 4.5 : here <= 32 ? 6.5 : 8.5), 1.2 + (here <= 16 ? 0.76 : here <= 32 ? 1.1 : 1.3) * n + (!gated ? 0 : here <= 16 ? 4.3 : 5.3));
     }
   }
   auto tc_time = [&](long long tiles, double longest, double all) {

@@ -4,8 +4,10 @@ PyTorch is plumbing here: it owns device memory and streams; every op below is o
 call into libliab200.so on ``torch.cuda.current_stream()``.  No op has a PyTorch
 fallback -- a missing library or a non-CUDA tensor raises.
 """
+import array
 import ctypes
 import functools
+import itertools
 import os
 
 import torch
@@ -901,10 +903,24 @@ def window_decode_splits(M, H, G, span, max_ctx, sms):
     return max(1, min(2 * sms // blocks, window_attn_split_class(max_ctx, span))) if max_ctx > 0 else 1
 
 
-def window_prompt_form(portions, nseg, M, H, window, chunk=0):
-    """Which of two kernels take a step of ``nseg`` portions of prompts (csrc/window_attn_mma.cu); ``portions``: (slot, first position, first row, rows) each on the host, or None."""
-    host = None if portions is None else (ctypes.c_int * (4 * nseg))(*(int(x) for p in portions for x in p))
-    return _lib.load().lia_window_prompt_form(host, nseg, M, H, min(int(window), 1 << 30), int(chunk))
+def window_prompt_form(portions, nseg, M, H, window, chunk=0, gated=False):
+    """Which of two kernels take a step of ``nseg`` portions of prompts (csrc/window_attn_mma.cu); ``portions``: (slot, first position, first row, rows) each on the host, or None;
+    ``gated``: a gate per channel."""
+    host = None if portions is None else array.array("i", itertools.chain.from_iterable(portions))
+    return _lib.load().lia_window_prompt_form(host and host.buffer_info()[0], nseg, M, H, window, chunk, gated)
+
+
+def window_step_form(portions, lengths, M, max_ctx, H, window, chunk, gated, sms):
+    """``window_prompt_form`` of a step whose ``lengths`` (of its shortest and longest portion) and longest history may be enough to tell: with no portion of up to 128 rows it is tcgen05
+    for all, and so it is with no more tiles than SMs where there is a gate or a row sees more than 96 keys; with so few tiles and no row that sees more than 64 it is mma.sync."""
+    if lengths[0] > 128:
+        return 2
+    if ((M + 127) // 128 + len(portions) - 1) * H <= sms:
+        if gated or (max_ctx > 96 and not chunk and (window <= 0 or window > 96)):
+            return 2
+        if 0 < max_ctx <= 64:
+            return 3
+    return window_prompt_form(portions, len(portions), M, H, window, chunk, gated)
 
 
 def window_attn(q, kcache, vcache, meta, temp, out, H, G, dim, vdim, window, scale, softcap, nseg=None, max_ctx=0, slopes=None, sink=None,
@@ -953,7 +969,7 @@ def window_attn(q, kcache, vcache, meta, temp, out, H, G, dim, vdim, window, sca
         nsplit = window_decode_splits(M, H, G, span, max_ctx, _sm_count(q.device)) if by_rows else 1
         prompt = 0 if by_rows else 1
         if prompt and dim == vdim == 128:
-            prompt = window_prompt_form(None, portions, M, H, window, chunk) if form is None else form
+            prompt = window_prompt_form(None, portions, M, H, window, chunk, gate_mode == 2) if form is None else form
         ws = None
         if nsplit > 1:
             ws = torch.empty(_lib.load().lia_window_attn_workspace_floats(M, H, vdim, nsplit), dtype=F32, device=q.device)

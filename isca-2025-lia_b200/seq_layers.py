@@ -20,7 +20,7 @@ import os
 import torch
 
 from . import ops
-from .ops import window_prompt_form
+from .ops import _sm_count as sm_count, window_step_form
 
 BF16, F32 = torch.bfloat16, torch.float32
 
@@ -41,14 +41,15 @@ class StepBatch:
         self.max_ctx = max_ctx              # longest history (tokens cached after this step) among the step's sequences
         self.scratch = {}                   # what one layer of this step leaves for later layers (per-token tensors)
 
-    def window_form(self, H, window, chunk=0):
-        """``window_prompt_form`` of the step's portions, worked out by the first of its layers that asks; None: they are not known on the host, or every row goes by itself."""
+    def window_form(self, H, window, chunk=0, gated=False):
+        """``window_step_form`` of the step's portions, worked out by the first of its layers that asks; None: they are not known on the host, or every row goes by itself."""
         if self.portions is None or self.rows < 2 * len(self.portions):
             return None
-        key = ("window form", H, window, chunk)
-        if key not in self.scratch:
-            self.scratch[key] = window_prompt_form(self.portions, len(self.portions), self.rows, H, window, chunk)
-        return self.scratch[key]
+        key = ("window form", H, window, chunk, gated)
+        form = self.scratch.get(key)
+        if form is None:
+            form = self.scratch[key] = window_step_form(self.portions, self.lengths, self.rows, self.max_ctx, H, window, chunk, gated, sm_count(self.meta.device))
+        return form
 
 
 class Linear:
@@ -654,7 +655,7 @@ class SinkAttentionMixer:
         o = torch.empty(M, H * self.vdim, dtype=self.dtype, device=h.device)
         ops.window_attn(q, kc, vc, batch.meta, None, o, H, G, self.dim, self.vdim, 0, self.scale, 0.0, nseg=batch.segs.shape[0], segs=batch.segs,
                         max_ctx=batch.max_ctx, slopes=self.slopes, sink=self.sink, gate=gate, gate_per_head=self.gate == "head",
-                        form=batch.window_form(H, 0))
+                        form=batch.window_form(H, 0, gated=self.gate == "channel"))
         return self.out(o)
 
 
