@@ -12,7 +12,7 @@
 //
 // 16 heads on 8 key heads of 128; on mma.sync -> here, us, and the error against 64 bits in 1e-7, means over 16 inputs: 2048 rows, window of 1024 and soft cap 136 (1.91) -> 66 (1.72), the whole history
 // and fp32 queries 182 (2.32) -> 63 (1.62); 700 rows behind 300 89 (2.22) -> 29 (1.88); portions of 300, 250, 200 29 (1.35) -> 14 (1.26); 100 rows behind 2000 130 -> 50 (behind
-// 1500 2.71 -> 2.05); four portions of 117, 100, 87, 73 14 -> 10, behind a gate per channel 23 -> 20.  Where mma.sync is the faster one: lia_window_prompt_form.
+// 1500 2.71 -> 2.05); four portions of 117, 100, 87, 73 14 -> 10, behind a gate per channel 23 -> 13.  Where mma.sync is the faster one: lia_window_prompt_form.
 #include <limits.h>
 
 #include "act.cuh"
