@@ -507,7 +507,7 @@ constexpr int TILE_BITS = 14, TILE_MASK = (1 << TILE_BITS) - 1;
 template <int DK, int DV> int run_as(const Call& c, int prompt) {
   if (prompt) {
     if constexpr (DK == 128 && DV == 128) {
-      if (prompt == 1) prompt = lia_window_prompt_form(nullptr, c.segs ? c.nseg : 1, c.M, c.a.H, c.a.window, c.a.chunk, c.a.gate_mode == 2);
+      if (prompt == 1 || (!c.segs && prompt != MMA_SYNC)) prompt = lia_window_prompt_form(nullptr, c.segs ? c.nseg : 1, c.M, c.a.H, c.a.window, c.a.chunk, c.a.gate_mode == 2);      // (without segments there is one portion)
       const int kernels = prompt & 7, tc_tiles = prompt >> 3 & TILE_MASK, tiles = prompt >> (3 + TILE_BITS) & TILE_MASK;
       if (kernels != MMA_SYNC) {
         const int rc = window_prompt_tc(c.q, c.ldq, c.kcache, c.kss, c.vcache, c.vss, c.meta, c.segs, c.nseg, c.x, c.out, c.M, c.a, kernels == BOTH ? SHORT_ROWS + 1 : 1, tc_tiles, c.stream);
