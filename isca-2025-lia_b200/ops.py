@@ -935,7 +935,7 @@ def window_attn(q, kcache, vcache, meta, temp, out, H, G, dim, vdim, window, sca
     (the value cache holds G // v_div heads: several attention maps over one set of values).  ``segs`` int32 [nseg, 4] on the device
     (slot, first position, first row, rows): the portions whose rows these are; with them, or with one portion, a step of prompts on
     bf16 caches runs on the tensor cores (csrc/window_attn_sm100.cu for heads of 128 channels, csrc/window_attn_mma.cu), and so does a step of single tokens.
-    ``form``: ``window_prompt_form`` of the portions, where the host knows them."""
+    ``form``: ``window_prompt_form`` of the portions, where the host knows them, or what gives it when asked for (H, window, chunk, gated)."""
     ldq = _rowmajor(q, "q")
     _req(meta, "meta", I32)
     for t, n in ((temp, "temp"), (slopes, "slopes"), (sink, "sink")):
@@ -969,7 +969,9 @@ def window_attn(q, kcache, vcache, meta, temp, out, H, G, dim, vdim, window, sca
         nsplit = window_decode_splits(M, H, G, span, max_ctx, _sm_count(q.device)) if by_rows else 1
         prompt = 0 if by_rows else 1
         if prompt and dim == vdim == 128:
-            prompt = window_prompt_form(None, portions, M, H, window, chunk, gate_mode == 2) if form is None else form
+            prompt = form(H, window, chunk, gate_mode == 2) if callable(form) else form
+            if prompt is None:
+                prompt = window_prompt_form(None, portions, M, H, window, chunk, gate_mode == 2)
         ws = None
         if nsplit > 1:
             ws = torch.empty(_lib.load().lia_window_attn_workspace_floats(M, H, vdim, nsplit), dtype=F32, device=q.device)

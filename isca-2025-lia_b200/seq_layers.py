@@ -41,9 +41,9 @@ class StepBatch:
         self.max_ctx = max_ctx              # longest history (tokens cached after this step) among the step's sequences
         self.scratch = {}                   # what one layer of this step leaves for later layers (per-token tensors)
 
-    def window_form(self, H, window, chunk=0, gated=False):
-        """``window_step_form`` of the step's portions, worked out by the first of its layers that asks; None: they are not known on the host, or every row goes by itself."""
-        if self.portions is None or self.rows < 2 * len(self.portions):
+    def window_form(self, H, window, chunk, gated):
+        """``window_step_form`` of the step's portions, worked out by the first of its layers whose operator asks; None: they are not known on the host."""
+        if self.portions is None:
             return None
         key = ("window form", H, window, chunk, gated)
         form = self.scratch.get(key)
@@ -436,7 +436,7 @@ class WindowAttentionMixer:
         ops.kv_store(k, v, batch.meta, kc, vc, self.G, self.dim, self.vdim, self.eps, self.norm_values)
         o = torch.empty(M, self.H * self.vdim, dtype=self.dtype, device=h.device)
         ops.window_attn(q, kc, vc, batch.meta, self.temp, o, self.H, self.G, self.dim, self.vdim, self.window, self.scale, self.softcap,
-                        nseg=batch.segs.shape[0], segs=batch.segs, max_ctx=batch.max_ctx, form=batch.window_form(self.H, self.window))
+                        nseg=batch.segs.shape[0], segs=batch.segs, max_ctx=batch.max_ctx, form=batch.window_form)
         return self.out(o)
 
 
@@ -535,7 +535,7 @@ class DifferentialAttentionMixer:
                      v_heads=self.G)
         a = torch.empty(M, H2 * self.vdim, dtype=F32, device=h.device)
         ops.window_attn(q, kc, vc, batch.meta, None, a, H2, G2, self.dim, self.vdim, self.window, self.scale, 0.0, nseg=batch.segs.shape[0], segs=batch.segs,
-                        max_ctx=batch.max_ctx, chunk=self.chunk, v_div=2, form=batch.window_form(H2, self.window, self.chunk))
+                        max_ctx=batch.max_ctx, chunk=self.chunk, v_div=2, form=batch.window_form)
         o = torch.empty(M, self.H * self.vdim, dtype=self.dtype, device=h.device)
         ops.diff_combine(a, o, self.H, self.G, self.vdim, self.lam, 1.0 - self.diff, self.eps)
         return self.out(o)
@@ -655,7 +655,7 @@ class SinkAttentionMixer:
         o = torch.empty(M, H * self.vdim, dtype=self.dtype, device=h.device)
         ops.window_attn(q, kc, vc, batch.meta, None, o, H, G, self.dim, self.vdim, 0, self.scale, 0.0, nseg=batch.segs.shape[0], segs=batch.segs,
                         max_ctx=batch.max_ctx, slopes=self.slopes, sink=self.sink, gate=gate, gate_per_head=self.gate == "head",
-                        form=batch.window_form(H, 0, gated=self.gate == "channel"))
+                        form=batch.window_form)
         return self.out(o)
 
 
